@@ -11,7 +11,9 @@
 #include "ssd_mamba3.cuh"
 #include "ssd_elementwise.cuh"
 
+#include <algorithm>
 #include <atomic>
+#include <initializer_list>
 #include <vector>
 
 namespace ssd {
@@ -125,6 +127,24 @@ int resolve_path(const ssd_b200_shape& s) {
     if (s.path == SSD_B200_PATH_AUTO && tc) return SSD_B200_PATH_TC;
     if (!simt_supported(s, &why)) return fail(SSD_B200_EUNSUPPORTED, "%s", why);
     return SSD_B200_PATH_SIMT;
+}
+
+// The tensor-core kernels move whole tiles by TMA, which wants 16-byte aligned tensors; the SIMT kernels take any address.
+// Where the library chose the path itself, a call with an unaligned tensor runs on the SIMT kernels if they cover the shape
+// (and the caller keeps no tile states, which only the tensor-core kernels know); the workspace of such a shape fits both.
+// Shapes that fill whole tiles have always been refused with an unaligned tensor, and still are.
+bool whole_tiles(const ssd_b200_shape& s) {
+    return s.headdim == ssd::tc::HP && s.dstate == ssd::tc::DN && s.seqlen % ssd::tc::LT == 0 &&
+           (s.chunk % ssd::tc::LT == 0 || ssd::tc::LT % s.chunk == 0);
+}
+bool simt_takes_unaligned(const ssd_b200_shape& s, int path) {
+    const char* why = "";
+    return path == SSD_B200_PATH_TC && s.path == SSD_B200_PATH_AUTO && !whole_tiles(s) && simt_supported(s, &why);
+}
+bool any_unaligned(std::initializer_list<const void*> ps) {
+    for (const void* p : ps)
+        if ((uintptr_t)p & 15) return true;
+    return false;
 }
 
 // Workspace layout of the SIMT path (all fp32, each block 256-byte aligned).
@@ -535,8 +555,9 @@ size_t ssd_b200_workspace_bytes(const ssd_b200_shape* shape, int pass) {
     int path = resolve_path(*shape);
     if (path < 0) return 0;
     ssd::Dims d = dims_of(*shape);
-    if (path == SSD_B200_PATH_TC) return ssd::tc::workspace_bytes(d, pass);
-    return simt_ws(d, pass).total;
+    if (path == SSD_B200_PATH_SIMT) return simt_ws(d, pass).total;
+    const size_t tc = ssd::tc::workspace_bytes(d, pass);
+    return simt_takes_unaligned(*shape, path) ? std::max(tc, simt_ws(d, pass).total) : tc;
 }
 
 size_t ssd_b200_states_bytes(const ssd_b200_shape* shape) {
@@ -560,6 +581,8 @@ int ssd_b200_fwd(const ssd_b200_fwd_args* a, void* stream) {
     if (a->states && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`states` is only used by the tensor-core path");
     if (a->ysq && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`ysq` is only written by the tensor-core path");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
+    if (!a->states && !a->ysq && form != 3 && any_unaligned({a->x, a->B, a->C, a->y}) && simt_takes_unaligned(a->shape, path))
+        path = SSD_B200_PATH_SIMT;
     if (path == SSD_B200_PATH_TC) return ssd::tc::forward(a, dims_of(a->shape), st, g_err, sizeof(g_err));
     return a->shape.dtype == SSD_B200_BF16 ? simt_fwd<__nv_bfloat16>(a, st) : simt_fwd<float>(a, st);
 }
@@ -588,6 +611,9 @@ int ssd_b200_bwd(const ssd_b200_bwd_args* a, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (a->states && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`states` is only used by the tensor-core path");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
+    if (!a->states && form != 3 && any_unaligned({a->x, a->B, a->C, a->dy, a->dx, a->dB, a->dC}) &&
+        simt_takes_unaligned(a->shape, path))
+        path = SSD_B200_PATH_SIMT;
     if (path == SSD_B200_PATH_TC) return ssd::tc::backward(a, dims_of(a->shape), st, g_err, sizeof(g_err));
     return a->shape.dtype == SSD_B200_BF16 ? simt_bwd<__nv_bfloat16>(a, st) : simt_bwd<float>(a, st);
 }

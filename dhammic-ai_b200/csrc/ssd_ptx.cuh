@@ -111,12 +111,27 @@ __device__ __forceinline__ void fence_async_smem() {  // generic-proxy smem writ
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// ---------------------------------------------------------------- TMA (tiled, 2D, no multicast)
+// ---------------------------------------------------------------- TMA (tiled, no multicast)
+// [rows][64] tensors (the saved states)
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
+}
+// [batch][position][head][column] tensors: a box is 64 columns of one head and 128 positions of one sequence; positions
+// behind the end of the sequence and columns behind the head's last read as zero.
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int col, int head, int pos, int batch) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(col), "r"(head), "r"(pos), "r"(batch)
+        : "memory");
+}
+// The store of such a box; what lies outside the tensor is not written.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* smem_src, int col, int head, int pos, int batch) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map),
+                 "r"(smem_u32(smem_src)), "r"(col), "r"(head), "r"(pos), "r"(batch)
+                 : "memory");
 }
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),

@@ -1,14 +1,13 @@
 // Tensor-core path of the SSD chunked scan for sm_100a: tcgen05.mma with TMEM accumulators,
 // operands staged in 128-byte-swizzled shared memory by TMA (no cluster multicast).
 //
-// Covered shapes: bf16 storage, headdim 64, d_state 128, sequence a multiple of 128, chunk a
-// multiple or a divisor of 128.  The kernels work on tiles of 128 positions whatever the chunk
-// size (the recurrence does not depend on where chunk boundaries fall); `tcum` is the inclusive
+// Covered shapes: bf16 storage, headdim up to 64, d_state up to 128 (see supported()), sequences and chunks of any
+// length.  The kernels work on tiles of 128 positions whatever the chunk size (the recurrence does not depend on where chunk boundaries fall); `tcum` is the inclusive
 // cumulative log-decay inside each 128-tile.
 //
 // Kernels
 //   tile_cumsum_kernel  a_cumsum (b,h,c,l) -> tcum (b,h,T), dt (b,T,h) -> dtT (b,h,T)
-//   cumsum_tile_fused_kernel  the same together with the cumulative sums themselves, for chunk = 128
+//   cumsum_tile_fused_kernel  the same together with the cumulative sums themselves
 //   fwd_walk_kernel     one CTA per (batch, head) walks the tiles with the state (64 x 128 fp32) in registers:
 //                       Y = ((C B^T) o L) X + diag(e) C H^T (+ D x);  H <- e^{S} H + X^T diag(d) B
 //   states_walk_kernel  only the recurrence; stores H_k (state entering tile k) as bf16
@@ -44,57 +43,66 @@ constexpr int PANEL = 16384;  // bytes of one [128 rows][64 bf16] swizzled panel
 // of the call exceeds it, and the kernels that build the mask carry two bodies: the factorised one, and one that
 // evaluates diagonal blocks entry by entry (one exp2 per entry); the flag selects the body on the device.
 constexpr float kMaskSafeLog2 = 100.f;
+constexpr int kFusedChunkMax = 1024;  // see cumsum_tile_fused_kernel
 
+// Shapes below the tile's own size are padded on chip: TMA fills what lies behind the end of a sequence, or behind a head's
+// last column, with zeros, and does not write it.  (A row of p or n bf16 values has to be a multiple of 16 bytes for
+// that.)  Half-empty tiles still beat the fp32 kernels down to about a quarter of the tile's columns.
 inline bool supported(int dtype, int T, int h, int p, int n, int g, int l) {
-    (void)h;
+    (void)T;
     (void)g;
-    return dtype == 1 && p == HP && n == DN && T % LT == 0 && (l % LT == 0 || LT % l == 0);
+    return dtype == 1 && p > HP / 2 && p <= HP && p % 8 == 0 && n > DN / 4 && n <= DN && n % 8 == 0 &&
+           (l <= kFusedChunkMax || (long long)l * (h + 1) * 4 <= 227 * 1024);
 }
+inline int tiles_of(int T) { return (T + LT - 1) / LT; }
 
 // ------------------------------------------------------------------------------------------
-// Tile-cumulative log2 decay and dt in (b,h,T) order, one block per (128-tile, 32 heads, batch): dt arrives in the
-// caller's (b,T,h) order and goes through a shared-memory transpose, so reads and writes are both 128-byte rows.
+// Per-position arrays of the tile kernels from a given a_cumsum: the tile-cumulative log2 decay, dt and the skip coefficient in
+// (b,h,Tp) order, Tp = T rounded up to whole tiles (behind the end of the sequence the decay stays at its last value and
+// dt and skip are zero).  One block per (128-tile, 32 heads, batch): dt arrives in the caller's (b,T,h) order and goes
+// through a shared-memory transpose, so reads and writes are both 128-byte rows.  Chunks of any length: the cumulative
+// decay from the tile's start is a difference inside the tile's first chunk plus the totals of the chunks that end in
+// the tile.
 __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restrict__ cum, const float* __restrict__ dt,
                                                           float* __restrict__ tcum, float* __restrict__ dtT,
                                                           const float* __restrict__ skip, float* __restrict__ skipT,
-                                                          int* __restrict__ extreme, int b, int T, int h, int l) {
+                                                          int* __restrict__ extreme, int T, int Tp, int h, int l) {
     __shared__ float sdt[LT][33];
     __shared__ float ssk[LT][33];
     const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h0 = hg * 32;
-    (void)b;
+    const int t0 = kt * LT, rows = min(LT, T - t0);
+    const bool head_ok = h0 + lane < h;
     if (dt) {
-        const bool head_ok = h0 + lane < h;
 #pragma unroll
         for (int t = warp; t < LT; t += 8)
-            sdt[t][lane] = head_ok ? dt[((size_t)bb * T + (size_t)kt * LT + t) * h + h0 + lane] : 0.f;
+            sdt[t][lane] = (head_ok && t < rows) ? dt[((size_t)bb * T + t0 + t) * h + h0 + lane] : 0.f;
     }
     if (skip) {  // per-position skip coefficient of the scaled operator form, same transpose
-        const bool head_ok = h0 + lane < h;
 #pragma unroll
         for (int t = warp; t < LT; t += 8)
-            ssk[t][lane] = head_ok ? skip[((size_t)bb * T + (size_t)kt * LT + t) * h + h0 + lane] : 0.f;
+            ssk[t][lane] = (head_ok && t < rows) ? skip[((size_t)bb * T + t0 + t) * h + h0 + lane] : 0.f;
     }
     __syncthreads();
-    const int c = T / l;
+    const int k0 = t0 / l, i0 = t0 - k0 * l;  // chunk of the tile's first position, position in it
 #pragma unroll
     for (int i4 = 0; i4 < 4; ++i4) {
         const int hl = warp * 4 + i4, hh = h0 + hl;
         if (hh >= h) break;  // warp-uniform
-        const float* cu = cum + ((size_t)((size_t)bb * h + hh) * c) * l;
-        const size_t o = ((size_t)bb * h + hh) * T + (size_t)kt * LT;
+        const float* cu = cum + ((size_t)bb * h + hh) * T;  // (b,h,c,l): position t of the sequence at t
+        const size_t o = ((size_t)bb * h + hh) * Tp + t0;
+        const float before = i0 > 0 ? cu[t0 - 1] : 0.f;
 #pragma unroll
         for (int s4 = 0; s4 < 4; ++s4) {
-            const int tt = s4 * 32 + lane, t = kt * LT + tt;
-            const int k = t / l, i = t - k * l;
-            float v = cu[(size_t)k * l + i];
-            if (l >= LT) {
-                const int i0 = (i / LT) * LT;
-                if (i0 > 0) v -= cu[(size_t)k * l + i0 - 1];
+            const int tt = s4 * 32 + lane, t = t0 + min(tt, rows - 1);
+            const int k = t / l;
+            float v = cu[t];
+            if (k == k0) {
+                v -= before;
             } else {
-                const int k0 = kt * (LT / l);
-                for (int kk = k0; kk < k; ++kk) v += cu[(size_t)kk * l + l - 1];
+                v += cu[(size_t)(k0 + 1) * l - 1] - before;
+                for (int kk = k0 + 1; kk < k; ++kk) v += cu[(size_t)(kk + 1) * l - 1];
             }
             v *= 1.4426950408889634f;  // stored in log2 units: every consumer uses exp2
             tcum[o + tt] = v;
@@ -108,68 +116,120 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
 }
 
 // ------------------------------------------------------------------------------------------
-// The two kernels above in one, for chunk size = tile size (128): reads the per-position log-decay once (dt * A_head,
-// or `a` as given, fp32 or bf16) in the caller's (b,T,h) layout through a shared-memory transpose, scans it inside each
-// 128-tile (warp per head, four 32-lane segments) and writes a_cumsum (b,h,c,l) in natural-log units, the same in
-// log2 units (tcum), dt and skip in (b,h,T) order, and the extreme-decay flag.
-// CH positions per pass: 128 (one pass) when there is no skip array to transpose, 64 (two passes, the running sums
-// carried over) with it — three [CH][33] arrays must fit the 48 KB of static shared memory.
-template <int CH, bool SKIP>
+// The same from the per-position log-decay itself (dt * A_head, or `a` as given, fp32 or bf16), which is read once in the
+// caller's (b,T,h) layout through a shared-memory transpose and scanned inside each 128-tile (warp per head, four 32-lane
+// segments, scanned side by side); also writes a_cumsum (b,h,c,l) in natural-log units.  Chunks of any length: where one
+// ends inside the tile its sums come from a second, segmented scan of the same values (CUT), so that they carry no
+// rounding of the positions before the chunk; where a chunk began in an earlier tile, the block adds up the positions
+// between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
+// kernels this replaces: 28 -> 7 us at (8, 2048, 24) with chunks of 64).  The skip array is transposed in a second round
+// through the panel of the log-decay.
+template <bool CUT>
 __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __restrict__ a, int a_is_bf16,
                                                                 const float* __restrict__ dt, const float* __restrict__ A_head,
                                                                 float* __restrict__ cum, float* __restrict__ tcum,
                                                                 float* __restrict__ dtT, const float* __restrict__ skip,
-                                                                float* __restrict__ skipT, int* __restrict__ extreme, int T, int h) {
-    __shared__ float sa[CH][33];
-    __shared__ float sdt[CH][33];
-    __shared__ float ssk[SKIP ? CH : 1][33];
+                                                                float* __restrict__ skipT, int* __restrict__ extreme, int T, int Tp,
+                                                                int h, int l) {
+    __shared__ float sa[LT][33];
+    __shared__ float sdt[LT][33];
+    __shared__ float sbef[8][33];
     const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h0 = hg * 32;
+    const int t0 = kt * LT, rows = min(LT, T - t0);
     const bool head_ok = h0 + lane < h;
     const float Ah = (!a && head_ok) ? A_head[h0 + lane] : 0.f;
-    float carry[4] = {0.f, 0.f, 0.f, 0.f};
+    auto log_decay = [&](size_t i, float d) {
+        if (!a) return d * Ah;
+        return a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[i]) : ((const float*)a)[i];
+    };
+    const size_t row0 = (size_t)bb * T;
 #pragma unroll
-    for (int part = 0; part < LT / CH; ++part) {
-        if (part) __syncthreads();
-#pragma unroll
-        for (int t = warp; t < CH; t += 8) {
-            const size_t i = ((size_t)bb * T + (size_t)kt * LT + part * CH + t) * h + h0 + lane;
-            float d = 0.f, av = 0.f;
-            if (head_ok) {
-                if (dt) d = dt[i];
-                if (a) av = a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[i]) : ((const float*)a)[i];
-                else av = d * Ah;
-                if (SKIP) ssk[t][lane] = skip[i];
-            }
-            sa[t][lane] = av;
-            sdt[t][lane] = d;
+    for (int t = warp; t < LT; t += 8) {
+        const size_t i = (row0 + t0 + t) * h + h0 + lane;
+        float d = 0.f, av = 0.f;
+        if (head_ok && t < rows) {
+            if (dt) d = dt[i];
+            av = log_decay(i, d);
         }
+        sa[t][lane] = av;
+        sdt[t][lane] = d;
+    }
+    const int i0 = t0 % l;  // positions of the tile's first chunk that lie in earlier tiles
+    if (i0) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int t = warp; t < i0; t += 8) {
+            const size_t i = (row0 + t0 - i0 + t) * h + h0 + lane;
+            if (head_ok) s += log_decay(i, dt && !a ? dt[i] : 0.f);
+        }
+        sbef[warp][lane] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {
+        const int hl = warp * 4 + i4, hh = h0 + hl;
+        if (hh >= h) break;  // warp-uniform
+        const size_t o = ((size_t)bb * h + hh) * Tp + t0, oc = ((size_t)bb * h + hh) * T + t0;
+        float before = 0.f;
+        if (i0) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) before += sbef[w][hl];
+        }
+        float v[4], c[4];
+#pragma unroll
+        for (int s4 = 0; s4 < 4; ++s4) v[s4] = c[s4] = sa[s4 * 32 + lane][hl];
+        int pos[4];  // position inside its chunk
+        if (CUT) {
+#pragma unroll
+            for (int s4 = 0; s4 < 4; ++s4) pos[s4] = (t0 + s4 * 32 + lane) % l;
+        }
+#pragma unroll
+        for (int of = 1; of < 32; of <<= 1) {
+#pragma unroll
+            for (int s4 = 0; s4 < 4; ++s4) {
+                const float u = __shfl_up_sync(0xffffffffu, v[s4], of);
+                if (lane >= of) v[s4] += u;
+                if (CUT) {
+                    const float w = __shfl_up_sync(0xffffffffu, c[s4], of);
+                    if (lane >= of && pos[s4] >= of) c[s4] += w;
+                }
+            }
+        }
+        float run = 0.f, runc = before;
+#pragma unroll
+        for (int s4 = 0; s4 < 4; ++s4) {
+            const int tt = s4 * 32 + lane;
+            v[s4] += run;
+            run = __shfl_sync(0xffffffffu, v[s4], 31);
+            if (CUT) {
+                if (pos[s4] > lane) c[s4] += runc;  // the chunk began before this segment
+                runc = __shfl_sync(0xffffffffu, c[s4], 31);
+            } else {
+                c[s4] = v[s4] + before;
+            }
+            if (tt < rows) cum[oc + tt] = c[s4];
+            const float w = v[s4] * 1.4426950408889634f;
+            tcum[o + tt] = w;
+            const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);
+            if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
+            if (dt) dtT[o + tt] = sdt[tt][hl];
+        }
+    }
+    if (skip) {
+        __syncthreads();
+#pragma unroll
+        for (int t = warp; t < LT; t += 8)
+            sa[t][lane] = (head_ok && t < rows) ? skip[(row0 + t0 + t) * h + h0 + lane] : 0.f;
         __syncthreads();
 #pragma unroll
         for (int i4 = 0; i4 < 4; ++i4) {
             const int hl = warp * 4 + i4, hh = h0 + hl;
-            if (hh >= h) break;  // warp-uniform
-            const size_t o = ((size_t)bb * h + hh) * T + (size_t)kt * LT + part * CH;  // (b,h,T) = (b,h,c,l), l = 128
+            if (hh >= h) break;
+            const size_t o = ((size_t)bb * h + hh) * Tp + t0;
 #pragma unroll
-            for (int s2 = 0; s2 < CH / 32; ++s2) {
-                const int tt = s2 * 32 + lane;
-                float incl = sa[tt][hl];
-#pragma unroll
-                for (int of = 1; of < 32; of <<= 1) {
-                    const float u = __shfl_up_sync(0xffffffffu, incl, of);
-                    if (lane >= of) incl += u;
-                }
-                incl += carry[i4];
-                carry[i4] = __shfl_sync(0xffffffffu, incl, 31);
-                cum[o + tt] = incl;
-                const float v = incl * 1.4426950408889634f;
-                tcum[o + tt] = v;
-                const float span = __shfl_sync(0xffffffffu, v, 0) - __shfl_sync(0xffffffffu, v, 31);
-                if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
-                if (dt) dtT[o + tt] = sdt[tt][hl];
-                if (SKIP) skipT[o + tt] = ssk[tt][hl];
-            }
+            for (int s4 = 0; s4 < 4; ++s4) skipT[o + s4 * 32 + lane] = sa[s4 * 32 + lane][hl];
         }
     }
 }
@@ -193,7 +253,7 @@ struct DecayTileParams {
     float* dskip;        // (b,T,h) or null (scaled operator form)
     float* dAh_part;     // (b*nt, h)
     float* dD_part;      // (b*nt, h) or null
-    int b, T, h, nt;
+    int b, T, Tp, h, nt;  // Tp = nt * 128: stride of g, ddtx and dyx
 };
 
 __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
@@ -203,10 +263,11 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h0 = hg * 32;
     const bool head_ok = h0 + lane < P.h;
+    const int rows = min(LT, P.T - k * LT);
     if (P.dt) {
 #pragma unroll
         for (int t = warp; t < LT; t += 8)
-            sdt[t][lane] = head_ok ? P.dt[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + lane] : 0.f;
+            sdt[t][lane] = (head_ok && t < rows) ? P.dt[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + lane] : 0.f;
     }
     // every load of the warp's four heads is issued before any of them is used
     const bool scaled = P.dt && !P.A_head;  // scaled operator form: three per-position outputs
@@ -218,7 +279,7 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
 #pragma unroll
         for (int s4 = 0; s4 < 4; ++s4) va[i][s4] = dxa[i][s4] = yxp[i][s4] = 0.f;
         if (hh < P.h) {
-            const size_t base = ((size_t)bb * P.h + hh) * P.T + (size_t)k * LT;
+            const size_t base = ((size_t)bb * P.h + hh) * P.Tp + (size_t)k * LT;
 #pragma unroll
             for (int s4 = 0; s4 < 4; ++s4) {
                 const int t = s4 * 32 + lane;
@@ -307,7 +368,7 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
         __syncthreads();
         if (head_ok) {
 #pragma unroll
-            for (int t = warp; t < LT; t += 8) out[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + lane] = sout[t][lane];
+            for (int t = warp; t < rows; t += 8) out[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + lane] = sout[t][lane];
         }
     }
 }
@@ -350,9 +411,9 @@ __global__ void __launch_bounds__(32) bounded_wait_selftest_kernel(int* status, 
 
 // ------------------------------------------------------------------------------------------
 struct WalkParams {
-    CUtensorMap mU;   // x (modes 0,1) or dy (reverse walks): 2D [b*T][h*64]
-    CUtensorMap mV;   // B (modes 0,1) or C (reverse walks):  2D [b*T][g*128]
-    CUtensorMap mC;   // C (mode 0)
+    CUtensorMap mU;   // x, or dy (reverse walks): (b,T,h,p)
+    CUtensorMap mV;   // B, or C (reverse walks): (b,T,g,n)
+    CUtensorMap mC;   // C (forward)
     const float* tcum;
     const float* dtT;
     const float* D;
@@ -365,7 +426,8 @@ struct WalkParams {
     const int* extreme;  // see kMaskSafeLog2 (forward only)
     float* ysq;          // (b, T/128, h, 2, 128) per half row sum_p y^2 (forward only), or null
     int* status;
-    int T, h, hpg, nt;
+    int Tp, h, hpg, nt;  // Tp = nt * 128: stride of the per-position arrays
+    int p, n;            // headdim and d_state of the tensors (at most 64 and 128)
 };
 
 constexpr uint32_t kIdescS = instr_desc(128, 128, false, false);    // K-major x K-major, N = 128

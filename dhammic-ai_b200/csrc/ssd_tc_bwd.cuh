@@ -40,7 +40,7 @@ namespace ssd {
 namespace tc {
 
 struct BwdParams {
-    CUtensorMap mX, mdY, mB, mC;   // loads: [b*T][h*64] and [b*T][g*128]
+    CUtensorMap mX, mdY, mB, mC;   // loads: (b,T,h,p) and (b,T,g,n)
     CUtensorMap mH, mQ;            // loads: states [b*nt*h*128][64]
     CUtensorMap mdX, mdB, mdC;     // stores
     const float* tcum;             // (b,h,T) tile-cumulative log2-decay
@@ -53,7 +53,8 @@ struct BwdParams {
     float* gS;                     // (b,h,nt,8): the terms that act through S = cum[127] of the tile
     const int* extreme;            // nonzero: the decay across some 32-position block is beyond the factorised mask
     int* status;
-    int T, h, hpg, nt, b;
+    int Tp, h, hpg, nt, b;         // Tp = nt * 128: stride of the per-position arrays
+    int n;                         // d_state (columns 64 .. of B, C, dB, dC exist only beyond 64)
     int items;                     // nt * groups * b work items (tile, group, batch), tile fastest
 };
 
@@ -150,7 +151,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         sD[row] = 0.f;
         sD[LT + row] = 0.f;
         __syncwarp();
-        fetch_scalars(0, ((size_t)bb0 * P.h + gg0 * hpg) * P.T + (size_t)k0 * LT, gg0 * hpg);
+        fetch_scalars(0, ((size_t)bb0 * P.h + gg0 * hpg) * P.Tp + (size_t)k0 * LT, gg0 * hpg);
         finish_scalars(0);
     }
     tc_fence_before();
@@ -282,14 +283,13 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
     } else if (warp == 17 && lane == 0) {
         // ---------------- TMA loads and stores
         int item = item0, k = k0, gg = gg0, bb = bb0;
-        int row0 = bb * P.T + k * LT;
         uint32_t hc = 0, ic = 0;
-        auto load_xy_at = [&](int hh, int r0, int xb) {
+        auto load_xy_at = [&](int hh, int kk, int b_, int xb) {
             mbar_expect_tx(&bar_xy[xb], 2 * PANEL);
-            tma_load_2d(sXY + (2 * xb) * PANEL, &P.mX, &bar_xy[xb], hh * HP, r0);
-            tma_load_2d(sXY + (2 * xb + 1) * PANEL, &P.mdY, &bar_xy[xb], hh * HP, r0);
+            tma_load_4d(sXY + (2 * xb) * PANEL, &P.mX, &bar_xy[xb], 0, hh, kk * LT, b_);
+            tma_load_4d(sXY + (2 * xb + 1) * PANEL, &P.mdY, &bar_xy[xb], 0, hh, kk * LT, b_);
         };
-        auto load_xy = [&](int hl) { load_xy_at(gg * hpg + hl, row0, (hc + hl) & 1); };
+        auto load_xy = [&](int hl) { load_xy_at(gg * hpg + hl, k, bb, (hc + hl) & 1); };
         auto load_hq = [&](int hl) {
             const int hh = gg * hpg + hl;
             const int srow = (int)((((size_t)bb * P.nt + k) * P.h + hh) * DN);
@@ -299,10 +299,10 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         };
         auto load_item = [&]() {  // C and B of the item, H / Q of its first head
             mbar_expect_tx(&bar_cb, 4 * PANEL);
-            tma_load_2d(sC, &P.mC, &bar_cb, gg * DN, row0);
-            tma_load_2d(sC + PANEL, &P.mC, &bar_cb, gg * DN + 64, row0);
-            tma_load_2d(sB, &P.mB, &bar_cb, gg * DN, row0);
-            tma_load_2d(sB + PANEL, &P.mB, &bar_cb, gg * DN + 64, row0);
+            tma_load_4d(sC, &P.mC, &bar_cb, 0, gg, k * LT, bb);
+            tma_load_4d(sC + PANEL, &P.mC, &bar_cb, 64, gg, k * LT, bb);
+            tma_load_4d(sB, &P.mB, &bar_cb, 0, gg, k * LT, bb);
+            tma_load_4d(sB + PANEL, &P.mB, &bar_cb, 64, gg, k * LT, bb);
             load_hq(0);
         };
         prefetch_tmap(&P.mX);
@@ -330,10 +330,10 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                 } else if (more) {
                     // x / dy of the next item's first head into the buffer of the head before this one (this head's
                     // buffer stages dB at the end of the item)
-                    load_xy_at(ngg * hpg, nbb * P.T + nk * LT, (hcur + 1) & 1);
+                    load_xy_at(ngg * hpg, nk, nbb, (hcur + 1) & 1);
                 }
                 mbar_wait_spin(&bar_c, ph, &failed);    // dx staged
-                tma_store_2d(&P.mdX, sdX, hh * HP, row0);
+                tma_store_4d(&P.mdX, sdX, 0, hh, k * LT, bb);
                 tma_store_commit();
                 tma_store_wait_read();
                 mbar_arrive(&bar_sr);  // the dx staging panel may be rewritten
@@ -341,7 +341,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             mbar_wait(&bar_m3, ic & 1, &failed);
             // C, B, H, Q are free now: the next item's loads go out before this item's group terms are stored
             const uint32_t hlast = hc + hpg - 1;
-            const int st_gg = gg, st_row0 = row0;
+            const int st_gg = gg, st_pos = k * LT, st_bb = bb;
             uint8_t* sdBst = sXY + (2 * (hlast & 1)) * PANEL;  // dB staging: the last head's x / dy buffer
             const uint32_t ic_done = ic;
             item = nitem;
@@ -351,14 +351,15 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                 k = nk;
                 gg = ngg;
                 bb = nbb;
-                row0 = bb * P.T + k * LT;
                 load_item();
             }
             mbar_wait_spin(&bar_g2, ic_done & 1, &failed);  // dC and dB staged
-            tma_store_2d(&P.mdC, sG, st_gg * DN, st_row0);
-            tma_store_2d(&P.mdC, sG + PANEL, st_gg * DN + 64, st_row0);
-            tma_store_2d(&P.mdB, sdBst, st_gg * DN, st_row0);
-            tma_store_2d(&P.mdB, sdBst + PANEL, st_gg * DN + 64, st_row0);
+            tma_store_4d(&P.mdC, sG, 0, st_gg, st_pos, st_bb);
+            tma_store_4d(&P.mdB, sdBst, 0, st_gg, st_pos, st_bb);
+            if (P.n > 64) {
+                tma_store_4d(&P.mdC, sG + PANEL, 64, st_gg, st_pos, st_bb);
+                tma_store_4d(&P.mdB, sdBst + PANEL, 64, st_gg, st_pos, st_bb);
+            }
             tma_store_commit();
             tma_store_wait_read();  // shared memory must outlive the reads only (the writes complete with the kernel)
             if (!more) break;
@@ -372,7 +373,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
     setmaxnreg_inc<kBwdRegsRow>();
     int item = item0, k = k0, gg = gg0, bb = bb0;
     uint32_t hc = 0, ic = 0;
-    auto pos_of = [&](int hl) { return ((size_t)bb * P.h + gg * hpg + hl) * P.T + (size_t)k * LT; };
+    auto pos_of = [&](int hl) { return ((size_t)bb * P.h + gg * hpg + hl) * P.Tp + (size_t)k * LT; };
     const int rb = row >> 5;                   // row block, warp-uniform
     const bool active = qc <= rb, diag = qc == rb;
     const uint32_t lanes = lane_base(warp);
@@ -401,7 +402,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             const size_t tpos = pos_of(hl) + row;
             if (qc == 0) {
                 if (hl + 1 < hpg) fetch_scalars((hcur + 1) & 1, pos_of(hl + 1), hh + 1);
-                else if (more) fetch_scalars((hcur + 1) & 1, ((size_t)nbb * P.h + ngg * hpg) * P.T + (size_t)nk * LT, ngg * hpg);
+                else if (more) fetch_scalars((hcur + 1) & 1, ((size_t)nbb * P.h + ngg * hpg) * P.Tp + (size_t)nk * LT, ngg * hpg);
             }
             const float c_i = scum2[buf * LT + row], dtv = sdt[buf * LT + row], Dh = sD[buf * LT + row];
             mbar_wait(&bar_xy[xb], (hcur >> 1) & 1, &failed);

@@ -103,14 +103,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     // state row of this thread: n = row, p in [16 q, 16 q + 16)
     float H[16];
     if (warp < 16) {
-        if (P.seed) {
-            const float* s = P.seed + bh * (size_t)HP * DN;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) H[j] = s[(size_t)(q * 16 + j) * DN + row];
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) H[j] = 0.f;
-        }
+        load_state_row(P.seed, bh, P.p, P.n, row, q * 16, H);
         store_quarter_row(sH, row, q * 2, H);
         fence_async_smem();
     }
@@ -186,13 +179,12 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             auto issue_loads = [&](int it) {
                 const int s = it % NST;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
-                const int grow = bb * P.T + it * LT;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_2d(st, &P.mV, &bar_ld[s], gg * DN, grow);
-                tma_load_2d(st + PANEL, &P.mV, &bar_ld[s], gg * DN + 64, grow);
-                tma_load_2d(st + 2 * PANEL, &P.mU, &bar_ld[s], hh * HP, grow);
-                tma_load_2d(st + 3 * PANEL, &P.mC, &bar_ld[s], gg * DN, grow);
-                tma_load_2d(st + 4 * PANEL, &P.mC, &bar_ld[s], gg * DN + 64, grow);
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, it * LT, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, it * LT, bb);
+                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, it * LT, bb);
+                tma_load_4d(st + 3 * PANEL, &P.mC, &bar_ld[s], 0, gg, it * LT, bb);
+                tma_load_4d(st + 4 * PANEL, &P.mC, &bar_ld[s], 64, gg, it * LT, bb);
             };
             for (int it = 0; it < NST - 1 && it < nt; ++it) issue_loads(it);
             if (P.save_states) {  // the seed is the state entering the first tile
@@ -207,7 +199,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 }
                 if (it > 0) {
                     mbar_wait_spin(&bar_h, (it - 1) & 1, &failed);  // new state in sH, y staged
-                    tma_store_2d(&P.mY, sY, hh * HP, bb * P.T + (it - 1) * LT);
+                    tma_store_4d(&P.mY, sY, 0, hh, (it - 1) * LT, bb);
                     if (P.save_states) tma_store_2d(&P.mS, sH, 0, state_row(it));
                     tma_store_commit();
                 }
@@ -215,7 +207,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 mbar_arrive(&bar_sr);  // sH and sY may be rewritten
             }
             mbar_wait_spin(&bar_h, (nt - 1) & 1, &failed);
-            tma_store_2d(&P.mY, sY, hh * HP, bb * P.T + (nt - 1) * LT);
+            tma_store_4d(&P.mY, sY, 0, hh, (nt - 1) * LT, bb);
             tma_store_commit();
             tma_store_wait_all();
         }
@@ -225,11 +217,11 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         setmaxnreg_inc<kFwdRegsRow>();
         const int rb = row >> 5;  // row block, warp-uniform
         const bool active = q <= rb, diag = q == rb;
-        const float* tcum = P.tcum + bh * P.T;
-        const float* dtT = P.dtT ? P.dtT + bh * P.T : nullptr;
+        const float* tcum = P.tcum + bh * P.Tp;
+        const float* dtT = P.dtT ? P.dtT + bh * P.Tp : nullptr;
         const uint32_t lanes = lane_base(warp);
         const float Dhead = P.D ? P.D[hh] : 0.f;
-        const float* skipT = P.skipT ? P.skipT + bh * P.T : nullptr;  // per-position skip instead of D
+        const float* skipT = P.skipT ? P.skipT + bh * P.Tp : nullptr;  // per-position skip instead of D
         const bool has_skip = P.D || P.skipT;
         const int c0 = q * 32;  // this thread's 32 columns of S
         // per-tile scalars are fetched one tile ahead
@@ -386,11 +378,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 P.ysq[((((size_t)bb * nt + (nt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((nt - 1) & 1) * 2 + (q >> 1)) * LT + row];
         }
-        if (P.out_state) {
-            float* o = P.out_state + bh * (size_t)HP * DN;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[(size_t)(q * 16 + j) * DN + row] = H[j];
-        }
+        store_state_row(P.out_state, bh, P.p, P.n, row, q * 16, H);
     }
     tc_fence_before();
     __syncthreads();

@@ -25,7 +25,7 @@ inline EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2D bf16 tensor [rows][cols] (cols contiguous), box 64 columns x 128 rows, 128-byte swizzle.
+// 2D bf16 tensor [rows][cols] (the saved states), box 64 columns x 128 rows, 128-byte swizzle.
 inline bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
@@ -34,6 +34,21 @@ inline bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t c
     cuuint32_t box[2] = {64, 128};
     cuuint32_t es[2] = {1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// A (b, T, heads, inner) bf16 tensor as the tile kernels see it: boxes of 64 columns of one head x 128 positions of one
+// sequence.  Keeping the dimensions apart is what makes a box that reaches behind the end of a sequence, or behind a head's
+// last column, read zeros instead of the neighbour's values.
+inline bool make_map4(CUtensorMap* m, const void* base, const Dims& d, int heads, int inner) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return false;
+    cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)heads, (cuuint64_t)d.T, (cuuint64_t)d.b};
+    cuuint64_t strides[3] = {(cuuint64_t)inner * 2, (cuuint64_t)heads * inner * 2, (cuuint64_t)d.T * heads * inner * 2};
+    cuuint32_t box[4] = {64, 1, 128, 1};
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -50,9 +65,10 @@ inline Ws ws_layout(const Dims& d, int pass) {
         off += (bytes + 255) / 256 * 256;
         return o;
     };
-    const size_t bht = (size_t)d.b * d.h * d.T * 4;
+    const int nt = tiles_of(d.T);
+    const size_t bht = (size_t)d.b * d.h * nt * LT * 4;
     const size_t bhpn = (size_t)d.b * d.h * d.p * d.n * 4;
-    const size_t st = (size_t)d.b * (d.T / LT) * d.h * DN * HP * 2;
+    const size_t st = (size_t)d.b * tiles_of(d.T) * d.h * DN * HP * 2;
     w.status = take(256);
     w.tcum = take(bht);
     w.dtT = take(bht);
@@ -65,9 +81,9 @@ inline Ws ws_layout(const Dims& d, int pass) {
         w.g = take(bht);
         w.ddtx = take(bht);
         w.dyx = take(bht);
-        w.gS = take((size_t)d.b * d.h * (d.T / LT) * 8 * 4);
-        w.dAh_part = take((size_t)d.b * (d.T / LT) * d.h * 4);
-        w.dD_part = take((size_t)d.b * (d.T / LT) * d.h * 4);
+        w.gS = take((size_t)d.b * d.h * nt * 8 * 4);
+        w.dAh_part = take((size_t)d.b * nt * d.h * 4);
+        w.dD_part = take((size_t)d.b * nt * d.h * 4);
     }
     w.total = off;
     return w;
@@ -75,11 +91,11 @@ inline Ws ws_layout(const Dims& d, int pass) {
 
 inline size_t workspace_bytes(const Dims& d, int pass) { return ws_layout(d, pass).total; }
 // The `states` buffer a forward call may fill for the backward call of the same inputs: the bf16 state entering
-// every tile, followed by the three (b,h,T) fp32 arrays the tile kernels read (tile-cumulative log2 decay, dt and
+// every tile, followed by the three (b,h,Tp) fp32 arrays the tile kernels read (tile-cumulative log2 decay, dt and
 // the per-position skip coefficient in (b,h,T) order) and the extreme-decay flag of tile_cumsum_kernel, so that the backward neither walks the states
 // nor rebuilds those arrays.
-inline size_t tile_states_bytes(const Dims& d) { return (size_t)d.b * (d.T / LT) * d.h * DN * HP * 2; }
-inline size_t states_bytes(const Dims& d) { return tile_states_bytes(d) + 3 * ((size_t)d.b * d.h * d.T * 4) + 256; }
+inline size_t tile_states_bytes(const Dims& d) { return (size_t)d.b * tiles_of(d.T) * d.h * DN * HP * 2; }
+inline size_t states_bytes(const Dims& d) { return tile_states_bytes(d) + 3 * ((size_t)d.b * d.h * tiles_of(d.T) * LT * 4) + 256; }
 
 #define SSD_TC_FAIL(code, ...)              \
     do {                                    \
@@ -127,8 +143,9 @@ inline int set_walk_attrs(char* err, size_t errn) {
 
 inline int launch_tile_cumsum(const Dims& d, const float* cum, const float* dt, float* tcum, float* dtT, const float* skip,
                               float* skipT, int* extreme, cudaStream_t st, char* err, size_t errn) {
-    dim3 g(d.T / LT, (d.h + 31) / 32, d.b);
-    SSD_LAUNCH(prof::K_TC_AUX, st, tile_cumsum_kernel<<<g, 256, 0, st>>>(cum, dt, tcum, dtT, skip, skipT, extreme, d.b, d.T, d.h, d.l));
+    const int nt = tiles_of(d.T);
+    dim3 g(nt, (d.h + 31) / 32, d.b);
+    SSD_LAUNCH(prof::K_TC_AUX, st, tile_cumsum_kernel<<<g, 256, 0, st>>>(cum, dt, tcum, dtT, skip, skipT, extreme, d.T, nt * LT, d.h, d.l));
     SSD_TC_CHECK("tile_cumsum");
     return 0;
 }
@@ -140,6 +157,8 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     const bool states_only = (a->flags & SSD_B200_FWD_STATES_ONLY) != 0;
     for (const void* p : {a->x, a->B, a->C, (const void*)a->y})
         if ((uintptr_t)p & 15) SSD_TC_FAIL(SSD_B200_EINVAL, "tensor-core path needs 16-byte aligned tensors");
+    const int nt = tiles_of(d.T), Tp = nt * LT;
+    const size_t bht = (size_t)d.b * d.h * Tp;
     char* ws = (char*)a->workspace;
     int* status = (int*)(ws + w.status);
     float* tcum = (float*)(ws + w.tcum);
@@ -150,21 +169,18 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     if (aux_valid && !a->states) SSD_TC_FAIL(SSD_B200_EINVAL, "SSD_B200_FWD_AUX_VALID needs the `states` buffer that holds the arrays");
     if (a->states) {  // the per-position arrays live behind the tile states, kept for later calls on the same inputs
         tcum = (float*)((char*)a->states + tile_states_bytes(d));
-        if (a->dt) dtT = tcum + (size_t)d.b * d.h * d.T;
-        if (a->skip) skipT = tcum + 2 * (size_t)d.b * d.h * d.T;
-        extreme = (int*)(tcum + 3 * (size_t)d.b * d.h * d.T);
+        if (a->dt) dtT = tcum + bht;
+        if (a->skip) skipT = tcum + 2 * bht;
+        extreme = (int*)(tcum + 3 * bht);
         if (!aux_valid && cudaMemsetAsync(extreme, 0, 4, st) != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "memset failed");
     }
     if (cudaMemsetAsync(status, 0, 8, st) != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "memset failed");
-    if (!a->cumsum_is_input && !aux_valid && d.l == LT) {
-        // chunk = tile: the within-chunk cumulative sums, their log2 copies, the transposes and the flag in one kernel
-        dim3 g(d.T / LT, (d.h + 31) / 32, d.b);
-        if (a->skip)
-            SSD_LAUNCH(prof::K_CUMSUM, st, (cumsum_tile_fused_kernel<64, true><<<g, 256, 0, st>>>(
-                a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, tcum, dtT, a->skip, skipT, extreme, d.T, d.h)));
-        else
-            SSD_LAUNCH(prof::K_CUMSUM, st, (cumsum_tile_fused_kernel<128, false><<<g, 256, 0, st>>>(
-                a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, tcum, dtT, nullptr, nullptr, extreme, d.T, d.h)));
+    if (!a->cumsum_is_input && !aux_valid && d.l <= kFusedChunkMax) {
+        // the within-chunk cumulative sums, the tile-cumulative log2 copies, the transposes and the flag in one kernel
+        const dim3 g(nt, (d.h + 31) / 32, d.b);
+        const bool cut = d.l % LT != 0;  // a chunk ends inside a tile
+        SSD_LAUNCH(prof::K_CUMSUM, st, ((cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>)<<<g, 256, 0, st>>>(
+            a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, tcum, dtT, a->skip, skipT, extreme, d.T, Tp, d.h, d.l)));
         SSD_TC_CHECK("cumsum_tile_fused");
     } else {
         if (!a->cumsum_is_input) {
@@ -186,24 +202,23 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     P.skipT = skipT;
     P.extreme = extreme;
     P.ysq = a->ysq;
-    const uint64_t rows = (uint64_t)d.b * d.T;
-    bool ok = make_map(&P.mU, a->x, rows, (uint64_t)d.h * HP) && make_map(&P.mV, a->B, rows, (uint64_t)d.g * DN) &&
-              make_map(&P.mC, a->C, rows, (uint64_t)d.g * DN) &&
-              make_map(&P.mY, states_only ? a->x : (const void*)a->y, rows, (uint64_t)d.h * HP);
+    bool ok = make_map4(&P.mU, a->x, d, d.h, d.p) && make_map4(&P.mV, a->B, d, d.g, d.n) && make_map4(&P.mC, a->C, d, d.g, d.n) &&
+              make_map4(&P.mY, states_only ? a->x : (const void*)a->y, d, d.h, d.p);
     if (a->states && ((uintptr_t)a->states & 15)) SSD_TC_FAIL(SSD_B200_EINVAL, "`states` must be 16-byte aligned");
     if (ok && a->states && !states_only) {
-        ok = make_map(&P.mS, a->states, (uint64_t)d.b * (d.T / LT) * d.h * DN, HP);
+        ok = make_map(&P.mS, a->states, (uint64_t)d.b * nt * d.h * DN, HP);
         P.save_states = 1;
     } else {
         P.mS = P.mY;
     }
     if (!ok) SSD_TC_FAIL(SSD_B200_ECUDA, "tensor map encoding failed");
     P.tcum = tcum; P.dtT = dtT; P.D = a->D; P.seed = a->init; P.out_state = a->final_state; P.status = status;
-    P.T = d.T; P.h = d.h; P.hpg = d.hpg; P.nt = d.T / LT;
+    P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
     if (states_only) {  // what this piece of the sequence adds to the state after it (plus the decayed seed)
         SummaryParams S{};
         S.mU = P.mU; S.mV = P.mV; S.tcum = tcum; S.dtT = dtT; S.seed = a->init; S.out = a->final_state;
-        S.logdecay = a->logdecay_total; S.status = status; S.T = d.T; S.h = d.h; S.hpg = d.hpg; S.nt = d.T / LT;
+        S.logdecay = a->logdecay_total; S.status = status; S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = nt;
+        S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)  // two heads of a group per CTA share the group's panels
             SSD_LAUNCH(prof::K_TC_SUMMARY, st, (summary_kernel<false, 2><<<dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st>>>(S)));
         else
@@ -227,6 +242,8 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
     if (!encode_fn()) SSD_TC_FAIL(SSD_B200_ECUDA, "cuTensorMapEncodeTiled is not available");
     for (const void* p : {a->x, a->B, a->C, a->dy, (const void*)a->dx, (const void*)a->dB, (const void*)a->dC})
         if ((uintptr_t)p & 15) SSD_TC_FAIL(SSD_B200_EINVAL, "tensor-core path needs 16-byte aligned tensors");
+    const int nt = tiles_of(d.T), Tp = nt * LT;
+    const size_t bht = (size_t)d.b * d.h * Tp;
     char* ws = (char*)a->workspace;
     int* status = (int*)(ws + w.status);
     float* tcum = (float*)(ws + w.tcum);
@@ -241,21 +258,20 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
     float* skipT = a->skip ? (float*)(ws + w.skipT) : nullptr;
     if (a->states) {  // the forward left the arrays and the flag behind the tile states
         tcum = (float*)((uintptr_t)a->states + tile_states_bytes(d));
-        dtT = a->dt ? tcum + (size_t)d.b * d.h * d.T : nullptr;
-        skipT = a->skip ? tcum + 2 * (size_t)d.b * d.h * d.T : nullptr;
-        extreme = (int*)(tcum + 3 * (size_t)d.b * d.h * d.T);
+        dtT = a->dt ? tcum + bht : nullptr;
+        skipT = a->skip ? tcum + 2 * bht : nullptr;
+        extreme = (int*)(tcum + 3 * bht);
     } else if (int rc = launch_tile_cumsum(d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn)) {
         return rc;
     }
     if (int rc = set_walk_attrs(err, errn)) return rc;
-    const int nt = d.T / LT;
-    const uint64_t rows = (uint64_t)d.b * d.T, srows = (uint64_t)d.b * nt * d.h * DN;
+    const uint64_t srows = (uint64_t)d.b * nt * d.h * DN;
     if (a->flags & SSD_B200_BWD_DINIT_ONLY) {  // d(initial state) of this piece for the given (or a zero) dfinal
         SummaryParams S{};
-        if (!(make_map(&S.mU, a->dy, rows, (uint64_t)d.h * HP) && make_map(&S.mV, a->C, rows, (uint64_t)d.g * DN)))
+        if (!(make_map4(&S.mU, a->dy, d, d.h, d.p) && make_map4(&S.mV, a->C, d, d.g, d.n)))
             SSD_TC_FAIL(SSD_B200_ECUDA, "tensor map encoding failed");
         S.tcum = tcum; S.dtT = nullptr; S.seed = a->dfinal; S.out = a->dinit; S.logdecay = nullptr; S.status = status;
-        S.T = d.T; S.h = d.h; S.hpg = d.hpg; S.nt = nt;
+        S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = nt; S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)
             SSD_LAUNCH(prof::K_TC_SUMMARY, st, (summary_kernel<true, 2><<<dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st>>>(S)));
         else
@@ -264,17 +280,15 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         return 0;
     }
     CUtensorMap mX, mdY, mB, mC, mH, mQ, mdX, mdB, mdC;
-    bool ok = make_map(&mX, a->x, rows, (uint64_t)d.h * HP) && make_map(&mdY, a->dy, rows, (uint64_t)d.h * HP) &&
-              make_map(&mB, a->B, rows, (uint64_t)d.g * DN) && make_map(&mC, a->C, rows, (uint64_t)d.g * DN) &&
-              make_map(&mH, Hst, srows, HP) && make_map(&mQ, Qst, srows, HP) &&
-              make_map(&mdX, a->dx, rows, (uint64_t)d.h * HP) && make_map(&mdB, a->dB, rows, (uint64_t)d.g * DN) &&
-              make_map(&mdC, a->dC, rows, (uint64_t)d.g * DN);
+    bool ok = make_map4(&mX, a->x, d, d.h, d.p) && make_map4(&mdY, a->dy, d, d.h, d.p) && make_map4(&mB, a->B, d, d.g, d.n) &&
+              make_map4(&mC, a->C, d, d.g, d.n) && make_map(&mH, Hst, srows, HP) && make_map(&mQ, Qst, srows, HP) &&
+              make_map4(&mdX, a->dx, d, d.h, d.p) && make_map4(&mdB, a->dB, d, d.g, d.n) && make_map4(&mdC, a->dC, d, d.g, d.n);
     if (!ok) SSD_TC_FAIL(SSD_B200_ECUDA, "tensor map encoding failed");
     if (!a->states) {  // states entering every tile (skipped when the forward saved them)
         WalkParams P{};
         P.mU = mX; P.mV = mB; P.mC = mC; P.mY = mdX; P.mS = mH; P.save_states = 1;
         P.tcum = tcum; P.dtT = dtT; P.D = nullptr; P.seed = a->init; P.out_state = fin; P.status = status;
-        P.T = d.T; P.h = d.h; P.hpg = d.hpg; P.nt = nt;
+        P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (states_walk_kernel<<<dim3(d.h, d.b), kWalkThreads, WalkCfg<1>::SMEM, st>>>(P)));
         SSD_TC_CHECK("tc_bwd_state");
     }
@@ -282,7 +296,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         WalkParams P{};
         P.mU = mdY; P.mV = mC; P.mC = mC; P.mY = mdX; P.mS = mQ; P.save_states = 1;
         P.tcum = tcum; P.dtT = nullptr; P.D = nullptr; P.seed = a->dfinal; P.out_state = dinit; P.status = status;
-        P.T = d.T; P.h = d.h; P.hpg = d.hpg; P.nt = nt;
+        P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         if (d.hpg % 2 == 0)  // two heads of a group per CTA: shared C panels, one N = 128 product per tile
             SSD_LAUNCH(prof::K_TC_BWD_STATE, st, rev_walk_kernel<2><<<dim3(d.h / 2, d.b), RevCfg<2>::THREADS, RevCfg<2>::SMEM, st>>>(P));
         else
@@ -293,7 +307,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         BwdParams P{};
         P.mX = mX; P.mdY = mdY; P.mB = mB; P.mC = mC; P.mH = mH; P.mQ = mQ; P.mdX = mdX; P.mdB = mdB; P.mdC = mdC;
         P.tcum = tcum; P.dtT = dtT; P.D = a->D; P.skipT = skipT; P.g = (float*)(ws + w.g); P.ddtx = (float*)(ws + w.ddtx);
-        P.dyx = (float*)(ws + w.dyx); P.status = status; P.T = d.T; P.h = d.h;
+        P.dyx = (float*)(ws + w.dyx); P.status = status; P.Tp = Tp; P.h = d.h; P.n = d.n;
         P.hpg = d.hpg; P.nt = nt; P.b = d.b; P.gS = (float*)(ws + w.gS);
         P.items = nt * d.g * d.b;
         P.extreme = extreme;
@@ -309,7 +323,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.dt = a->dt; P.A_head = a->A_head; P.ddt = a->ddt; P.da = a->cumsum_is_input ? nullptr : a->da;
         P.dskip = a->skip ? a->dskip : nullptr;
         P.dAh_part = (float*)(ws + w.dAh_part); P.dD_part = P.dyx ? (float*)(ws + w.dD_part) : nullptr;
-        P.b = d.b; P.T = d.T; P.h = d.h; P.nt = nt;
+        P.b = d.b; P.T = d.T; P.Tp = Tp; P.h = d.h; P.nt = nt;
         SSD_LAUNCH(prof::K_DECAY, st, decay_tile_kernel<<<dim3(nt, (d.h + 31) / 32, d.b), 256, 0, st>>>(P));
         SSD_TC_CHECK("decay_grad");
         if (a->dt && a->A_head) {

@@ -85,12 +85,11 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
                 const int k = nt - 1 - it;
                 const int s = it % kRevStages;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
-                const int grow = bb * P.T + k * LT;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_2d(st, &P.mV, &bar_ld[s], gg * DN, grow);
-                tma_load_2d(st + PANEL, &P.mV, &bar_ld[s], gg * DN + 64, grow);
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, k * LT, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, k * LT, bb);
 #pragma unroll
-                for (int hs = 0; hs < NH; ++hs) tma_load_2d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], (hh0 + hs) * HP, grow);
+                for (int hs = 0; hs < NH; ++hs) tma_load_4d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], 0, hh0 + hs, k * LT, bb);
             };
             for (int it = 0; it < kRevStages && it < nt; ++it) issue_loads(it);
             for (int it = 0; it < nt; ++it) {
@@ -121,18 +120,11 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
         const int hh = hh0 + hs;
         const int ht = tid & 255, row = ht & 127, hf = ht >> 7;
         const size_t bh = (size_t)bb * P.h + hh;
-        const float* tcum = P.tcum + bh * P.T;
+        const float* tcum = P.tcum + bh * P.Tp;
         const uint32_t lanes = lane_base(warp);
         uint8_t* sQ = sQ0 + (size_t)hs * PANEL;
         float H[32];  // state gradient row n = row, p in [hf*32, hf*32+32)
-        if (P.seed) {
-            const float* s = P.seed + bh * (size_t)HP * DN;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) H[q] = s[(size_t)(hf * 32 + q) * DN + row];
-        } else {
-#pragma unroll
-            for (int q = 0; q < 32; ++q) H[q] = 0.f;
-        }
+        load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, H);
         // Store the state gradient leaving tile nt-1-it: staged in the head's sQ panel, written by one TMA store of the
         // head's first thread, which waits until its previous store has read the panel; the first barrier (the head's
         // 256 threads) releases the panel to the writers, the second hands the written panel to the store.
@@ -203,11 +195,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
             c_i = c_n;
             Sk = Sk_n;
         }
-        if (P.out_state) {
-            float* o = P.out_state + bh * (size_t)HP * DN;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) o[(size_t)(hf * 32 + q) * DN + row] = H[q];
-        }
+        store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
         if (ht == 0) tma_store_wait_all();
     }
     tc_fence_before();

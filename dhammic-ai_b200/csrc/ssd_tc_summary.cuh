@@ -40,7 +40,8 @@ struct SummaryParams {
     float* out;            // (b,h,p,n) fp32
     float* logdecay;       // (b,h) total log-decay of the piece in natural-log units, or null
     int* status;
-    int T, h, hpg, nt;
+    int Tp, h, hpg, nt;   // Tp = nt * 128: stride of the per-position arrays
+    int p, n;
 };
 
 template <bool REV, int NH>
@@ -86,12 +87,12 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
             auto issue_loads = [&](int it) {
                 const int s = it % NS;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
-                const int grow = bb * P.T + tile_of(it) * LT;
+                const int pos = tile_of(it) * LT;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_2d(st, &P.mV, &bar_ld[s], gg * DN, grow);
-                tma_load_2d(st + PANEL, &P.mV, &bar_ld[s], gg * DN + 64, grow);
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
 #pragma unroll
-                for (int hs = 0; hs < NH; ++hs) tma_load_2d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], (hh0 + hs) * HP, grow);
+                for (int hs = 0; hs < NH; ++hs) tma_load_4d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], 0, hh0 + hs, pos, bb);
             };
             for (int it = 0; it < NS && it < nt; ++it) issue_loads(it);
             for (int it = 0; it < nt; ++it) {
@@ -116,8 +117,8 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         const int hh = hh0 + hs;
         const size_t bh = (size_t)bb * P.h + hh;
         const int ht = tid & 255, row = ht & 127, hf = ht >> 7;  // scaling: position `row`, columns [32 hf, 32 hf + 32) of the panel
-        const float* tcum = P.tcum + bh * P.T;
-        const float* dtT = (!REV && P.dtT) ? P.dtT + bh * P.T : nullptr;
+        const float* tcum = P.tcum + bh * P.Tp;
+        const float* dtT = (!REV && P.dtT) ? P.dtT + bh * P.Tp : nullptr;
         float run = 0.f;  // forward: log2-decay of the tiles after this one; reverse: of the tiles before it
         float c_n = tcum[(size_t)tile_of(0) * LT + row];
         float S_n = tcum[(size_t)tile_of(0) * LT + LT - 1];
@@ -159,15 +160,11 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         tmem_ld32(tm + lane_base(warp) + hs * 64 + hf * 32, r);
         tmem_ld_wait();
         const float dec = exp2f(run);
-        float* o = P.out + bh * (size_t)HP * DN;  // accumulator row = n, columns = p
-        const float* sd = P.seed ? P.seed + bh * (size_t)HP * DN : nullptr;
+        float v[32];  // accumulator row = n, columns = p
+        load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, v);
 #pragma unroll
-        for (int q = 0; q < 32; ++q) {
-            const size_t idx = (size_t)(hf * 32 + q) * DN + row;
-            float v = __uint_as_float(r[q]);
-            if (sd) v = fmaf(dec, sd[idx], v);
-            o[idx] = v;
-        }
+        for (int q = 0; q < 32; ++q) v[q] = fmaf(dec, v[q], __uint_as_float(r[q]));
+        store_state_row(P.out, bh, P.p, P.n, row, hf * 32, v);
         if (P.logdecay && ht == 0) P.logdecay[bh] = run * 0.6931471805599453f;
     }
     tc_fence_before();

@@ -39,18 +39,26 @@ __device__ __forceinline__ void store_half_row(uint8_t* panel, int row, int chun
     }
 }
 
-// 32 fp32 state values of (row n, half hf) as 64 contiguous bytes of the [n][p] bf16 state tile `slot`.
-__device__ __forceinline__ void store_state_slot(__nv_bfloat16* slot, int row, int hf, const float (&H)[32]) {
-    uint4* o = reinterpret_cast<uint4*>(slot + (size_t)row * HP + hf * 32);
+// N values p0 .. p0+N-1 of row n of a (b,h,p,n) fp32 state, n and p below the tile's 128 x 64: what lies beyond the state's own
+// size reads as zero and is not written.
+template <int N>
+__device__ __forceinline__ void load_state_row(const float* base, size_t bh, int p, int n, int row, int p0, float (&H)[N]) {
+    const float* s = base ? base + bh * (size_t)p * n + (size_t)p0 * n + row : nullptr;
+    if (s && p == HP && row < n) {
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-        uint4 v;
-        v.x = pack_bf16(H[ch * 8 + 0], H[ch * 8 + 1]);
-        v.y = pack_bf16(H[ch * 8 + 2], H[ch * 8 + 3]);
-        v.z = pack_bf16(H[ch * 8 + 4], H[ch * 8 + 5]);
-        v.w = pack_bf16(H[ch * 8 + 6], H[ch * 8 + 7]);
-        o[ch] = v;
+        for (int q = 0; q < N; ++q) H[q] = s[(size_t)q * n];
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; ++q) H[q] = (s && row < n && p0 + q < p) ? s[(size_t)q * n] : 0.f;
     }
+}
+template <int N>
+__device__ __forceinline__ void store_state_row(float* base, size_t bh, int p, int n, int row, int p0, const float (&H)[N]) {
+    if (!base || row >= n) return;
+    float* o = base + bh * (size_t)p * n + (size_t)p0 * n + row;
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+        if (p == HP || p0 + q < p) o[(size_t)q * n] = H[q];
 }
 
 template <int MODE>
@@ -101,14 +109,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     // state row of this thread: n = row, p in [hf*32, hf*32+32)
     float H[32];
     if (warp < 8) {
-        if (P.seed) {
-            const float* s = P.seed + bh * (size_t)HP * DN;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) H[q] = s[(size_t)(hf * 32 + q) * DN + row];
-        } else {
-#pragma unroll
-            for (int q = 0; q < 32; ++q) H[q] = 0.f;
-        }
+        load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, H);
         store_half_row(sH, row, hf * 4, H);
         fence_async_smem();
     }
@@ -148,11 +149,10 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
             auto issue_loads = [&](int it) {
                 const int s = it % NST;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
-                const int grow = bb * P.T + it * LT;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_2d(st, &P.mV, &bar_ld[s], gg * DN, grow);
-                tma_load_2d(st + PANEL, &P.mV, &bar_ld[s], gg * DN + 64, grow);
-                tma_load_2d(st + 2 * PANEL, &P.mU, &bar_ld[s], hh * HP, grow);
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, it * LT, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, it * LT, bb);
+                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, it * LT, bb);
             };
             for (int it = 0; it < NST - 1 && it < nt; ++it) issue_loads(it);
             tma_store_2d(&P.mS, sH, 0, state_row(0));  // the seed is the state entering the first tile
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ row warps
-        const float* tcum = P.tcum + bh * P.T;
-        const float* dtT = P.dtT ? P.dtT + bh * P.T : nullptr;
+        const float* tcum = P.tcum + bh * P.Tp;
+        const float* dtT = P.dtT ? P.dtT + bh * P.Tp : nullptr;
         const uint32_t lanes = lane_base(warp);
         // per-tile scalars are fetched one tile ahead
         float c_n = tcum[row], S_n = tcum[LT - 1];
@@ -230,11 +230,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
             fence_async_smem();
             mbar_arrive_warp(&bar_h);
         }
-        if (P.out_state) {
-            float* o = P.out_state + bh * (size_t)HP * DN;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) o[(size_t)(hf * 32 + q) * DN + row] = H[q];
-        }
+        store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
     }
     tc_fence_before();
     __syncthreads();

@@ -31,7 +31,7 @@ import torch
 from torch import Tensor
 
 from . import _cabi
-from .ssd_scan import _dt_code, _ptr, _run_bwd_operator, _run_bwd_scaled, _run_fwd, _stream
+from .ssd_scan import _dense, _dt_code, _ptr, _run_bwd_operator, _run_bwd_scaled, _run_fwd, _stream
 
 
 def _shape(x: Tensor, B: Tensor) -> _cabi.Shape:
@@ -45,7 +45,7 @@ class _SSDMamba3(torch.autograd.Function):
         assert x.is_cuda, "ssd_b200 runs on CUDA tensors only (no CPU fallback)"
         lib = _cabi.load()
         chunk = int(chunk_size)
-        xc, Bc, Cc = x.contiguous(), B.contiguous(), C_.contiguous()
+        xc, Bc, Cc = _dense(x), _dense(B), _dense(C_)
         # angles keep their own precision: fp32 angles (the reference's dt * theta product) are summed as given
         ang = raw_angles.contiguous() if raw_angles.dtype in (torch.float32, x.dtype) else raw_angles.contiguous().float()
         dtc, lamc, Ah = dt.float().contiguous(), lam.float().contiguous(), A_head.float().contiguous()
@@ -99,7 +99,7 @@ class _SSDMamba3(torch.autograd.Function):
         g, n = B.shape[2], B.shape[3]
         dev = x.device
         with torch.cuda.device(dev):
-            dy = dY.contiguous().to(x.dtype)
+            dy = _dense(dY).to(x.dtype)
             if ctx.fused:  # dx is complete; dw = <dX, x> and dyx = <dy, x> come from the scan's own row sums
                 dx, da, dw, dyx, dBr, dCr = _run_bwd_scaled(ctx.scan_shape, x, dA, w, skip, Br, Cr, a_cumsum, dy, ctx.states)
                 dxw = None

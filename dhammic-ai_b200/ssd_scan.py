@@ -86,6 +86,12 @@ def _ptr(t: Tensor | None):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+def _dense(t: Tensor) -> Tensor:
+    """Contiguous and, where the storage starts between two 16-byte boundaries, copied to a fresh one (TMA needs them)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _stream(dev) -> C.c_void_p:
     return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
 
@@ -205,7 +211,7 @@ def _run_bwd_operator(shape, x, A, B, Cm, cum, dY, states, init4=None, dfinal_st
     dev = x.device
     b, T, h, p = x.shape
     with torch.cuda.device(dev):
-        dy = dY.contiguous()
+        dy = _dense(dY)
         if dy.dtype != x.dtype:
             dy = dy.to(x.dtype)
         dfin = None if dfinal_state is None else dfinal_state.float().contiguous()
@@ -234,7 +240,7 @@ class FusedSSDScan(torch.autograd.Function):
         _check_inputs(x, B, C_)
         assert A.is_cuda
         chunk = int(chunk_size)
-        xc, Ac, Bc, Cc = x.contiguous(), A.contiguous(), B.contiguous(), C_.contiguous()
+        xc, Ac, Bc, Cc = _dense(x), A.contiguous(), _dense(B), _dense(C_)
         b, T, h, p = xc.shape
         n = Bc.shape[3]
         init4 = None
@@ -306,7 +312,7 @@ class _SSDMamba2(torch.autograd.Function):
         _check_inputs(x, B, C_)
         ctx.set_materialize_grads(False)  # an unused final state must not cost a zero tensor and a seeded reverse walk
         chunk = int(chunk_size)
-        xc, Bc, Cc = x.contiguous(), B.contiguous(), C_.contiguous()
+        xc, Bc, Cc = _dense(x), _dense(B), _dense(C_)
         dtc = dt.float().contiguous()
         Ah = A_head.float().contiguous()
         Dc = None if D is None else D.float().contiguous()
@@ -336,7 +342,7 @@ class _SSDMamba2(torch.autograd.Function):
         dev = x.device
         b, T, h, p = x.shape
         with torch.cuda.device(dev):
-            dy = dY.contiguous().to(x.dtype)
+            dy = _dense(dY).to(x.dtype)
             dfin = None if dfinal is None else dfinal.float().contiguous()
             dx = torch.empty_like(x)
             dB = torch.empty_like(B)
@@ -375,7 +381,7 @@ def _run_bwd_scaled(shape, x, a, w, skip, B, Cm, cum, dY, states):
     dev = x.device
     b, T, h, p = x.shape
     with torch.cuda.device(dev):
-        dy = dY.contiguous().to(x.dtype)
+        dy = _dense(dY).to(x.dtype)
         dx, dB, dC = torch.empty_like(x), torch.empty_like(B), torch.empty_like(Cm)
         da = torch.empty(b, T, h, dtype=torch.float32, device=dev)
         dw, dskip = torch.empty_like(da), torch.empty_like(da)
@@ -395,7 +401,7 @@ def _mamba2_backward(ctx_shape, x, dt, Ah, B, Cm, cum, D, init4, states, dY, dfi
     dev = x.device
     b, T, h, p = x.shape
     with torch.cuda.device(dev):
-        dy = dY.contiguous().to(x.dtype)
+        dy = _dense(dY).to(x.dtype)
         dfin = None if dfinal is None else dfinal.float().contiguous()
         dx = torch.empty_like(x)
         dB = torch.empty_like(B)
@@ -425,7 +431,7 @@ class _SSDMamba2Gated(torch.autograd.Function):
         ctx.set_materialize_grads(False)
         lib = _cabi.load()
         chunk = int(chunk_size)
-        xc, Bc, Cc = x.contiguous(), B.contiguous(), C_.contiguous()
+        xc, Bc, Cc = _dense(x), _dense(B), _dense(C_)
         dtc = dt.float().contiguous()
         Ah = A_head.float().contiguous()
         Dc = None if D is None else D.float().contiguous()
@@ -440,7 +446,7 @@ class _SSDMamba2Gated(torch.autograd.Function):
         _cabi.check(path)
         with torch.cuda.device(dev):
             ysq = None
-            if path == _cabi.PATH_TC:
+            if path == _cabi.PATH_TC and T % 128 == 0:
                 ysq = torch.empty(b * (T // 128) * h * 2 * 128, dtype=torch.float32, device=dev)
             y, final, cum, shape, states = _run_fwd(xc, None, dtc, Ah, Dc, Bc, Cc, chunk, init4, None,
                                                     want_states=any(ctx.needs_input_grad), ysq=ysq)

@@ -166,6 +166,42 @@ def test_tensor_core_path_edge_shapes(pkg, cabi, oracle, batch, seqlen, heads, g
     check_mamba2(pkg, oracle, cfg, TOL_BF16, init=states, dfinal=states, seed=33)
 
 
+@pytest.mark.parametrize("b,T,h,p,n,g,l", [(1, 1, 2, 64, 128, 1, 1), (2, 127, 3, 64, 128, 1, 127), (2, 129, 2, 64, 128, 2, 43),
+                                           (2, 200, 3, 64, 128, 1, 100), (3, 320, 4, 64, 64, 2, 80), (1, 256, 2, 40, 72, 1, 64),
+                                           (2, 480, 5, 56, 40, 5, 96), (1, 1300, 2, 64, 128, 1, 650)])
+@pytest.mark.parametrize("states", [False, True])
+def test_tensor_core_path_partial_tiles(pkg, cabi, oracle, b, T, h, p, n, g, l, states):
+    """Sequences that end inside a tile, chunks that end anywhere, and heads narrower than the tile's 64 x 128 (bar as for
+    whole tiles: the rounding of the operands is the same)."""
+    cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, headdim=p, d_state=n, ngroups=g, chunk=l)
+    assert pkg.resolved_path_name(cfg) == "tc"
+    # (one position and no state: the decay acts on nothing, dA_head is 0 and an error relative to it is 0 / 0)
+    check_mamba2(pkg, oracle, cfg, TOL_BF16, init=states or T == 1, dfinal=states, seed=77)
+    inp = pkg.make_inputs(cfg, seed=78)
+    a = (inp["dt"] * inp["A_head"]).to(DEV)
+    args = [inp[k].to(DEV) for k in ("x", "B", "C")]
+    _, _, cache = pkg.fused_ssd_scan(args[0], a, args[1], args[2], l)
+    want = a.cpu().double().view(b, T // l, l, h).cumsum(2).permute(0, 3, 1, 2)
+    assert rel_err(cache["A_cumsum"], want) < TOL_FP32
+    y0, f0, _ = pkg.fused_ssd_scan(args[0], a, args[1], args[2], l)
+    y1, f1, _ = pkg.fused_ssd_scan(args[0], a, args[1], args[2], l, None, cache)  # from the cached sums
+    assert rel_err(y1, y0) < TOL_BF16 and rel_err(f1, f0) < TOL_BF16
+
+
+def test_unaligned_inputs(pkg, cabi, oracle):
+    """Tensors that start between two 16-byte boundaries."""
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=192, nheads=2, ngroups=1, chunk=64)
+    inp = pkg.make_inputs(cfg, seed=5)
+    def shifted(t):
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        buf[1:] = t.to(DEV).flatten()
+        return buf[1:].view(t.shape)
+    got = pkg.ssd_mamba2(shifted(inp["x"]), inp["dt"].to(DEV), inp["A_head"].to(DEV), shifted(inp["B"]), shifted(inp["C"]),
+                         inp["D"].to(DEV), cfg.chunk)
+    want = pkg.ssd_mamba2(*[inp[k].to(DEV) for k in ("x", "dt", "A_head", "B", "C", "D")], cfg.chunk)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 @pytest.mark.parametrize("h,p,n,g,l,T", [(3, 24, 12, 1, 32, 96), (4, 80, 40, 2, 48, 96), (6, 16, 72, 3, 100, 200),
                                          (2, 128, 130, 1, 64, 64), (2, 8, 8, 2, 16, 16)])
 def test_ragged_shapes_fp32(pkg, cabi, oracle, h, p, n, g, l, T):
