@@ -147,36 +147,53 @@ bool any_unaligned(std::initializer_list<const void*> ps) {
     return false;
 }
 
+// Blocks that share the heads of a group in the SIMT kernels: as many (a divisor of the heads per group) as it takes to have two
+// blocks per SM of the target, because below that the time of a call is one block's walk over its heads.  More would only
+// add partial sums of dB and dC (each split writes its own, which bounds them at about 300 blocks' worth).
+int simt_splits(const ssd::Dims& d) {
+    const long long base = (long long)d.c * ((d.l + ssd::simt::TS - 1) / ssd::simt::TS) * d.b * d.g;
+    int s = 1;
+    while (s < d.hpg && (base * s < 2 * 148 || d.hpg % s)) ++s;
+    return s;
+}
+
 // Workspace layout of the SIMT path (all fp32, each block 256-byte aligned).
 struct SimtWs {
-    size_t states, dstates, final_state, g_row, g_col, ddtx, dAh_part, dD_part, dinit, total;
+    size_t states, final_state, dstates, g_row, g_col, ddtx, dyx, dAh_part, dD_part, dB_part, dC_part, total;
 };
+size_t simt_states_elems(const ssd::Dims& d) { return (size_t)d.b * d.c * d.h * d.p * d.n; }
 
 SimtWs simt_ws(const ssd::Dims& d, int pass) {
     SimtWs w{};
     size_t off = 0;
-    const size_t st = (size_t)d.b * d.c * d.h * d.p * d.n * 4;
-    const size_t bhpn = (size_t)d.b * d.h * d.p * d.n * 4;
-    const size_t bht = (size_t)d.b * d.h * d.T * 4;
-    const size_t bh = (size_t)d.b * d.h * 4;
-    auto take = [&](size_t bytes) {
+    auto take = [&](size_t elems) {
         size_t o = off;
-        off += align_up(bytes);
+        off += align_up(elems * 4);
         return o;
     };
-    w.states = take(st);
+    w.states = take(simt_states_elems(d));
     if (pass == SSD_B200_PASS_BWD) {
-        w.dstates = take(st);
-        w.final_state = take(bhpn);
-        w.dinit = take(bhpn);
+        const size_t bht = (size_t)d.b * d.h * d.T, splits = simt_splits(d);
+        const size_t bc = splits > 1 ? (size_t)d.b * d.T * d.g * splits * d.n : 0;
+        w.dstates = take(simt_states_elems(d));
+        w.final_state = take((size_t)d.b * d.h * d.p * d.n);
         w.g_row = take(bht);
         w.g_col = take(bht);
         w.ddtx = take(bht);
-        w.dAh_part = take(bh);
-        w.dD_part = take(bh);
+        w.dyx = take(bht);
+        w.dAh_part = take((size_t)d.b * d.h);
+        w.dD_part = take((size_t)d.b * d.h);
+        w.dB_part = take(bc);
+        w.dC_part = take(bc);
     }
     w.total = off;
     return w;
+}
+// The `states` buffer of the SIMT path: what a forward keeps for the backward of the same inputs, the state entering every chunk
+// and the final state.  Beyond a gigabyte recomputing them is the better bargain.
+size_t simt_states_bytes(const ssd::Dims& d) {
+    const size_t bytes = align_up(simt_states_elems(d) * 4) + (size_t)d.b * d.h * d.p * d.n * 4;
+    return bytes <= ((size_t)1 << 30) ? bytes : 0;
 }
 
 #define CUDA_LAUNCH_CHECK(what)                                                              \
@@ -185,152 +202,135 @@ SimtWs simt_ws(const ssd::Dims& d, int pass) {
         if (e_ != cudaSuccess) return fail(SSD_B200_ECUDA, "%s: %s", what, cudaGetErrorString(e_)); \
     } while (0)
 
-template <class K>
-int set_smem(K kernel, size_t bytes, const char* name) {
+// Opt-in shared-memory size of one kernel, raised when a call needs more than any before it did (a function attribute lives as
+// long as the device's context).
+template <auto KERNEL>
+int set_smem(size_t bytes, const char* name) {
     if (bytes > 227 * 1024) return fail(SSD_B200_EUNSUPPORTED, "%s needs %zu bytes of shared memory", name, bytes);
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return fail(SSD_B200_ECUDA, "%s: set smem: %s", name, cudaGetErrorString(e));
-    }
+    if (bytes <= 48 * 1024) return 0;
+    static std::atomic<size_t> granted[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+    if (granted[dev & 63].load(std::memory_order_acquire) >= bytes) return 0;
+    cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return fail(SSD_B200_ECUDA, "%s: set smem: %s", name, cudaGetErrorString(e));
+    granted[dev & 63].store(227 * 1024, std::memory_order_release);
     return 0;
 }
 
+ssd::simt::Params simt_params(const ssd::Dims& d) {
+    ssd::simt::Params P{};
+    P.d = d;
+    P.lb = (d.l + ssd::simt::TS - 1) / ssd::simt::TS;
+    P.splits = simt_splits(d);
+    return P;
+}
+
+// Local states (mode 0) or local state gradients (mode 1) of every chunk, and the recurrence over the chunks.
 template <class T>
-int simt_forward_states(const ssd::simt::Params& P, cudaStream_t st) {
+int simt_chunk_states(const ssd::simt::Params& P, int mode, cudaStream_t st) {
     using namespace ssd::simt;
     const ssd::Dims& d = P.d;
-    dim3 gs((d.n + TS - 1) / TS, (d.p + TS - 1) / TS, d.b * d.c * d.h);
-    SSD_LAUNCH(ssd::prof::K_CHUNK_STATE, st, chunk_state_kernel<T><<<gs, NTHR, 0, st>>>(P, 0));
+    const dim3 g(d.c * d.b, d.h, ((d.p + TS - 1) / TS) * ((d.n + TS - 1) / TS));
+    SSD_LAUNCH(mode ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, (chunk_state_kernel<T><<<g, NTHR, 0, st>>>(P, mode)));
     CUDA_LAUNCH_CHECK("chunk_state");
     const size_t pn = (size_t)d.p * d.n;
-    dim3 gp((unsigned)((pn + NTHR - 1) / NTHR), d.h, d.b);
-    SSD_LAUNCH(ssd::prof::K_STATE_PASS, st, state_passing_kernel<<<gp, NTHR, 0, st>>>(P, 0));
+    const dim3 gp((unsigned)((pn + NTHR - 1) / NTHR), d.h, d.b);
+    SSD_LAUNCH(mode ? ssd::prof::K_STATE_PASS_REV : ssd::prof::K_STATE_PASS, st, state_passing_kernel<<<gp, NTHR, 0, st>>>(P, mode));
     CUDA_LAUNCH_CHECK("state_passing");
     return 0;
 }
 
-int launch_cumsum(const ssd::simt::Params& P, cudaStream_t st) {
+template <class T, int PT>
+int launch_chunk_scan(const ssd::simt::Params& P, cudaStream_t st) {
     using namespace ssd::simt;
-    const ssd::Dims& d = P.d;
-    size_t sm = (size_t)d.l * (d.h + 1) * 4;
-    if (int rc = set_smem(chunk_cumsum_kernel, sm, "chunk_cumsum")) return rc;
-    SSD_LAUNCH(ssd::prof::K_CUMSUM, st, chunk_cumsum_kernel<<<dim3(d.c, d.b), NTHR, sm, st>>>(P));
-    CUDA_LAUNCH_CHECK("chunk_cumsum");
+    const size_t sm = chunk_scan_smem(P.d, PT);
+    if (int rc = set_smem<chunk_scan_kernel<T, PT>>(sm, "chunk_scan")) return rc;
+    SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, (chunk_scan_kernel<T, PT><<<dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits), NTHR, sm, st>>>(P)));
+    CUDA_LAUNCH_CHECK("chunk_scan");
     return 0;
 }
 
 template <class T>
 int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
     using namespace ssd::simt;
-    Params P{};
-    P.d = dims_of(a->shape);
+    using namespace ssd::cum;
+    Params P = simt_params(dims_of(a->shape));
     const ssd::Dims& d = P.d;
     SimtWs w = simt_ws(d, SSD_B200_PASS_FWD);
     if (a->workspace_bytes < w.total) return fail(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
-    char* ws = (char*)a->workspace;
-    P.x = a->x; P.a = a->a; P.dt = a->dt; P.A_head = a->A_head; P.D = a->D; P.B = a->B; P.C = a->C;
-    P.init = a->init; P.cum = a->a_cumsum; P.states = (float*)(ws + w.states);
-    P.final_state = a->final_state; P.y = a->y; P.a_is_bf16 = a->shape.a_dtype == SSD_B200_BF16;
-    if (!a->cumsum_is_input)
-        if (int rc = launch_cumsum(P, st)) return rc;
-    if (int rc = simt_forward_states<T>(P, st)) return rc;
+    P.x = a->x; P.dt = a->dt; P.A_head = a->A_head; P.D = a->D; P.B = a->B; P.C = a->C;
+    P.init = a->init; P.cum = a->a_cumsum; P.final_state = a->final_state; P.y = a->y;
+    P.states = a->states ? (float*)a->states : (float*)((char*)a->workspace + w.states);
+    if (a->states) P.final_keep = (float*)((char*)a->states + align_up(simt_states_elems(d) * 4));
+    if (!a->cumsum_is_input) {
+        const size_t sm = (size_t)d.l * (d.h + 1) * 4;
+        if (int rc = set_smem<chunk_cumsum_kernel>(sm, "chunk_cumsum")) return rc;
+        SSD_LAUNCH(ssd::prof::K_CUMSUM, st, chunk_cumsum_kernel<<<dim3(d.c, d.b), NTHR, sm, st>>>(
+            a->dt ? nullptr : a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, d.T, d.h, d.l));
+        CUDA_LAUNCH_CHECK("chunk_cumsum");
+    }
+    if (int rc = simt_chunk_states<T>(P, 0, st)) return rc;
     if (a->logdecay_total) {
         SSD_LAUNCH(ssd::prof::K_CUMSUM, st, logdecay_total_kernel<<<(d.b * d.h + 127) / 128, 128, 0, st>>>(a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
         CUDA_LAUNCH_CHECK("logdecay_total");
     }
     if (a->flags & SSD_B200_FWD_STATES_ONLY) return 0;
-    const int PT = (d.p + TS - 1) / TS;
-    const int hrows = d.p > TS ? d.p : TS;
-    size_t sm = ((size_t)TS * (d.n + 1) + (size_t)hrows * (d.n + 1) + (size_t)TS * (PT * TS + 1) + TS * (TS + 1) + 2 * TS) * 4;
-    dim3 g((d.l + TS - 1) / TS, d.h, d.b * d.c);
-    if (PT == 1) {
-        if (int rc = set_smem(chunk_scan_kernel<T, 1>, sm, "chunk_scan")) return rc;
-        SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, chunk_scan_kernel<T, 1><<<g, NTHR, sm, st>>>(P));
-    } else {
-        if (int rc = set_smem(chunk_scan_kernel<T, 2>, sm, "chunk_scan")) return rc;
-        SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, chunk_scan_kernel<T, 2><<<g, NTHR, sm, st>>>(P));
-    }
-    CUDA_LAUNCH_CHECK("chunk_scan");
-    return 0;
+    return d.p <= TS ? launch_chunk_scan<T, 1>(P, st) : launch_chunk_scan<T, 2>(P, st);
 }
 
-template <class T, int NTN>
-int launch_bwd_row(const ssd::simt::Params& P, cudaStream_t st) {
+template <class T, int PT, int NTN>
+int launch_chunk_bwd(ssd::simt::Params P, cudaStream_t st) {
     using namespace ssd::simt;
-    const ssd::Dims& d = P.d;
-    const int hrows = d.p > TS ? d.p : TS;
-    const int pp_pad = (d.p + 3) / 4 * 4;
-    size_t sm = ((size_t)TS * (d.n + 1) + (size_t)hrows * (d.n + 1) + 2 * (size_t)TS * (pp_pad + 1) + TS * (TS + 1) + 2 * TS) * 4;
-    if (int rc = set_smem(bwd_row_kernel<T, NTN>, sm, "bwd_row")) return rc;
-    SSD_LAUNCH(ssd::prof::K_BWD_ROW, st, bwd_row_kernel<T, NTN><<<dim3((d.l + TS - 1) / TS, d.g, d.b * d.c), NTHR, sm, st>>>(P));
-    CUDA_LAUNCH_CHECK("bwd_row");
+    // one panel less where that makes the kernel fit at all, or (headdim and d_state up to 64) fit twice on an SM
+    P.share_ws = chunk_bwd_smem(P.d, PT, false) > (PT * NTN == 1 ? 113 : 227) * 1024;
+    const size_t sm = chunk_bwd_smem(P.d, PT, P.share_ws);
+    if (int rc = set_smem<chunk_bwd_kernel<T, PT, NTN>>(sm, "chunk_bwd")) return rc;
+    SSD_LAUNCH(ssd::prof::K_BWD_COL, st, (chunk_bwd_kernel<T, PT, NTN><<<dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st>>>(P)));
+    CUDA_LAUNCH_CHECK("chunk_bwd");
     return 0;
 }
-
-template <class T, int NTN, int PT>
-int launch_bwd_col(const ssd::simt::Params& P, cudaStream_t st) {
-    using namespace ssd::simt;
-    const ssd::Dims& d = P.d;
-    const int hrows = d.p > TS ? d.p : TS;
-    size_t sm = ((size_t)TS * (d.n + 1) + (size_t)hrows * (d.n + 1) + 2 * (size_t)TS * (PT * TS + 1) + 2 * TS * (TS + 1) + 3 * TS) * 4;
-    if (int rc = set_smem(bwd_col_kernel<T, NTN, PT>, sm, "bwd_col")) return rc;
-    SSD_LAUNCH(ssd::prof::K_BWD_COL, st, bwd_col_kernel<T, NTN, PT><<<dim3((d.l + TS - 1) / TS, d.g, d.b * d.c), NTHR, sm, st>>>(P));
-    CUDA_LAUNCH_CHECK("bwd_col");
-    return 0;
+template <class T, int PT>
+int dispatch_chunk_bwd(const ssd::simt::Params& P, cudaStream_t st) {
+    if (P.d.n <= 64) return launch_chunk_bwd<T, PT, 1>(P, st);
+    if (P.d.n <= 128) return launch_chunk_bwd<T, PT, 2>(P, st);
+    return launch_chunk_bwd<T, PT, 4>(P, st);
 }
 
 template <class T>
 int simt_bwd(const ssd_b200_bwd_args* a, cudaStream_t st) {
     using namespace ssd::simt;
-    Params P{};
-    P.d = dims_of(a->shape);
+    Params P = simt_params(dims_of(a->shape));
     const ssd::Dims& d = P.d;
     SimtWs w = simt_ws(d, SSD_B200_PASS_BWD);
     if (a->workspace_bytes < w.total) return fail(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
     char* ws = (char*)a->workspace;
-    P.x = a->x; P.a = a->a; P.dt = a->dt; P.A_head = a->A_head; P.D = a->D; P.B = a->B; P.C = a->C;
-    P.dy = a->dy; P.init = a->init; P.dfinal = a->dfinal; P.cum = (float*)a->a_cumsum;
-    P.states = (float*)(ws + w.states); P.dstates = (float*)(ws + w.dstates);
-    P.final_state = (float*)(ws + w.final_state);
-    P.dinit = a->dinit ? a->dinit : (float*)(ws + w.dinit);
+    P.x = a->x; P.dt = a->dt; P.A_head = a->A_head; P.D = a->D; P.B = a->B; P.C = a->C;
+    P.dy = a->dy; P.init = a->init; P.dfinal = a->dfinal; P.dinit = a->dinit; P.cum = a->a_cumsum;
+    P.states = a->states ? (float*)const_cast<void*>(a->states) : (float*)(ws + w.states);
+    P.final_state = a->states ? (float*)((char*)const_cast<void*>(a->states) + align_up(simt_states_elems(d) * 4)) : (float*)(ws + w.final_state);
+    P.dstates = (float*)(ws + w.dstates);
     P.dx = a->dx; P.dB = a->dB; P.dC = a->dC;
     P.g_row = (float*)(ws + w.g_row); P.g_col = (float*)(ws + w.g_col); P.ddtx = (float*)(ws + w.ddtx);
+    P.dyx = (a->dt && a->D) ? (float*)(ws + w.dyx) : nullptr;
     P.da = a->cumsum_is_input ? nullptr : a->da;
     P.ddt = a->ddt; P.dAh_part = (float*)(ws + w.dAh_part); P.dD_part = (float*)(ws + w.dD_part);
-    P.a_is_bf16 = a->shape.a_dtype == SSD_B200_BF16;
-    const bool dinit_only = (a->flags & SSD_B200_BWD_DINIT_ONLY) != 0;
-    // states entering each chunk (recomputed) and the final state
-    if (!dinit_only)
-        if (int rc = simt_forward_states<T>(P, st)) return rc;
-    // local state gradients and the reverse recurrence
-    dim3 gs((d.n + TS - 1) / TS, (d.p + TS - 1) / TS, d.b * d.c * d.h);
-    SSD_LAUNCH(ssd::prof::K_CHUNK_DSTATE, st, chunk_state_kernel<T><<<gs, NTHR, 0, st>>>(P, 1));
-    CUDA_LAUNCH_CHECK("chunk_dstate");
-    const size_t pn = (size_t)d.p * d.n;
-    SSD_LAUNCH(ssd::prof::K_STATE_PASS_REV, st, state_passing_kernel<<<dim3((unsigned)((pn + NTHR - 1) / NTHR), d.h, d.b), NTHR, 0, st>>>(P, 1));
-    CUDA_LAUNCH_CHECK("state_passing_rev");
-    if (dinit_only) return 0;
-    const int NTN = (d.n + TS - 1) / TS, PT = (d.p + TS - 1) / TS;
-    int rc = 0;
-    if (NTN <= 1) rc = launch_bwd_row<T, 1>(P, st);
-    else if (NTN == 2) rc = launch_bwd_row<T, 2>(P, st);
-    else rc = launch_bwd_row<T, 4>(P, st);
-    if (rc) return rc;
-    if (PT == 1) {
-        if (NTN <= 1) rc = launch_bwd_col<T, 1, 1>(P, st);
-        else if (NTN == 2) rc = launch_bwd_col<T, 2, 1>(P, st);
-        else rc = launch_bwd_col<T, 4, 1>(P, st);
-    } else {
-        if (NTN <= 1) rc = launch_bwd_col<T, 1, 2>(P, st);
-        else if (NTN == 2) rc = launch_bwd_col<T, 2, 2>(P, st);
-        else rc = launch_bwd_col<T, 4, 2>(P, st);
+    if (P.splits > 1) {
+        P.dB_part = (float*)(ws + w.dB_part);
+        P.dC_part = (float*)(ws + w.dC_part);
     }
-    if (rc) return rc;
-    SSD_LAUNCH(ssd::prof::K_DECAY, st, decay_grad_kernel<T><<<dim3(d.h, d.b), NTHR, 0, st>>>(P));
+    const bool dinit_only = (a->flags & SSD_B200_BWD_DINIT_ONLY) != 0;
+    if (!dinit_only && !a->states)  // states entering each chunk and the final state, if the forward did not keep them
+        if (int rc = simt_chunk_states<T>(P, 0, st)) return rc;
+    if (int rc = simt_chunk_states<T>(P, 1, st)) return rc;  // local state gradients and the reverse recurrence
+    if (dinit_only) return 0;
+    if (int rc = d.p <= TS ? dispatch_chunk_bwd<T, 1>(P, st) : dispatch_chunk_bwd<T, 2>(P, st)) return rc;
+    const size_t total = P.splits > 1 ? (size_t)d.b * d.T * d.g * d.n : 0;
+    SSD_LAUNCH(ssd::prof::K_DECAY, st, decay_grad_kernel<T><<<(unsigned)(d.b * d.h + (total + NTHR - 1) / NTHR), NTHR, 0, st>>>(P));
     CUDA_LAUNCH_CHECK("decay_grad");
     if (a->dt) {
-        SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_batch_kernel<<<(d.h + 127) / 128, 128, 0, st>>>(P.dAh_part, a->dA_head, d.b, d.h));
-        if (a->D) SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_batch_kernel<<<(d.h + 127) / 128, 128, 0, st>>>(P.dD_part, a->dD, d.b, d.h));
+        SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_batch_kernel<<<dim3((d.h + 127) / 128, a->D ? 2 : 1), 128, 0, st>>>(
+            P.dAh_part, a->dA_head, P.dD_part, a->dD, d.b, d.h));
         CUDA_LAUNCH_CHECK("reduce_batch");
     }
     return 0;
@@ -562,8 +562,9 @@ size_t ssd_b200_workspace_bytes(const ssd_b200_shape* shape, int pass) {
 
 size_t ssd_b200_states_bytes(const ssd_b200_shape* shape) {
     if (check_shape(shape)) return 0;
-    if (resolve_path(*shape) != SSD_B200_PATH_TC) return 0;
-    return ssd::tc::states_bytes(dims_of(*shape));
+    const int path = resolve_path(*shape);
+    if (path < 0) return 0;
+    return path == SSD_B200_PATH_TC ? ssd::tc::states_bytes(dims_of(*shape)) : simt_states_bytes(dims_of(*shape));
 }
 
 int ssd_b200_fwd(const ssd_b200_fwd_args* a, void* stream) {
@@ -578,7 +579,7 @@ int ssd_b200_fwd(const ssd_b200_fwd_args* a, void* stream) {
     if (path < 0) return path;
     if (!a->workspace || ((uintptr_t)a->workspace & 255)) return fail(SSD_B200_EWORKSPACE, "workspace null or not 256-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    if (a->states && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`states` is only used by the tensor-core path");
+    if ((uintptr_t)a->states & 15) return fail(SSD_B200_EINVAL, "`states` must be 16-byte aligned");
     if (a->ysq && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`ysq` is only written by the tensor-core path");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
     if (!a->states && !a->ysq && form != 3 && any_unaligned({a->x, a->B, a->C, a->y}) && simt_takes_unaligned(a->shape, path))
@@ -609,7 +610,7 @@ int ssd_b200_bwd(const ssd_b200_bwd_args* a, void* stream) {
     if (path < 0) return path;
     if (!a->workspace || ((uintptr_t)a->workspace & 255)) return fail(SSD_B200_EWORKSPACE, "workspace null or not 256-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    if (a->states && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`states` is only used by the tensor-core path");
+    if ((uintptr_t)a->states & 15) return fail(SSD_B200_EINVAL, "`states` must be 16-byte aligned");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
     if (!a->states && form != 3 && any_unaligned({a->x, a->B, a->C, a->dy, a->dx, a->dB, a->dC}) &&
         simt_takes_unaligned(a->shape, path))

@@ -1,0 +1,246 @@
+// Cumulative log-decays: within the caller's chunks (an output of the operator) and within the 128-position tiles
+// the tensor-core kernels work on.
+#pragma once
+#include "ssd_common.cuh"
+
+namespace ssd {
+namespace cum {
+
+constexpr int LT = 128;  // tile length
+
+// The decay mask of a 32-column block is the product of a per-row and a per-column factor taken relative to the
+// block's last column.  Below the diagonal both are <= 1.  Inside the diagonal block the row factor is
+// 2^(decay from the row to the block end) >= 1 and the column factor its inverse scale; beyond this many log2
+// units across a block one of them would leave the fp32 range.  tile_cumsum_kernel raises a flag when any block
+// of the call exceeds it, and the kernels that build the mask carry two bodies: the factorised one, and one that
+// evaluates diagonal blocks entry by entry (one exp2 per entry); the flag selects the body on the device.
+constexpr float kMaskSafeLog2 = 100.f;
+constexpr int kFusedChunkMax = 1024;  // see cumsum_tile_fused_kernel
+
+
+// ------------------------------------------------------------------------------------------
+// Per-position arrays of the tile kernels from a given a_cumsum: the tile-cumulative log2 decay, dt and the skip coefficient in
+// (b,h,Tp) order, Tp = T rounded up to whole tiles (behind the end of the sequence the decay stays at its last value and
+// dt and skip are zero).  One block per (tile, 32 heads, batch): dt arrives in the caller's (b,T,h) order and goes
+// through a shared-memory transpose, so reads and writes are both 128-byte rows.  Chunks of any length: the cumulative
+// decay from the tile's start is a difference inside the tile's first chunk plus the totals of the chunks that end in
+// the tile.
+__global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restrict__ cum, const float* __restrict__ dt,
+                                                          float* __restrict__ tcum, float* __restrict__ dtT,
+                                                          const float* __restrict__ skip, float* __restrict__ skipT,
+                                                          int* __restrict__ extreme, int T, int Tp, int h, int l) {
+    __shared__ float sdt[LT][33];
+    __shared__ float ssk[LT][33];
+    const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h0 = hg * 32;
+    const int t0 = kt * LT, rows = min(LT, T - t0);
+    const bool head_ok = h0 + lane < h;
+    if (dt) {
+#pragma unroll
+        for (int t = warp; t < LT; t += 8)
+            sdt[t][lane] = (head_ok && t < rows) ? dt[((size_t)bb * T + t0 + t) * h + h0 + lane] : 0.f;
+    }
+    if (skip) {  // per-position skip coefficient of the scaled operator form, same transpose
+#pragma unroll
+        for (int t = warp; t < LT; t += 8)
+            ssk[t][lane] = (head_ok && t < rows) ? skip[((size_t)bb * T + t0 + t) * h + h0 + lane] : 0.f;
+    }
+    __syncthreads();
+    const int k0 = t0 / l, i0 = t0 - k0 * l;  // chunk of the tile's first position, position in it
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {
+        const int hl = warp * 4 + i4, hh = h0 + hl;
+        if (hh >= h) break;  // warp-uniform
+        const float* cu = cum + ((size_t)bb * h + hh) * T;  // (b,h,c,l): position t of the sequence at t
+        const size_t o = ((size_t)bb * h + hh) * Tp + t0;
+        const float before = i0 > 0 ? cu[t0 - 1] : 0.f;
+#pragma unroll
+        for (int s4 = 0; s4 < LT / 32; ++s4) {
+            const int tt = s4 * 32 + lane, t = t0 + min(tt, rows - 1);
+            const int k = t / l;
+            float v = cu[t];
+            if (k == k0) {
+                v -= before;
+            } else {
+                v += cu[(size_t)(k0 + 1) * l - 1] - before;
+                for (int kk = k0 + 1; kk < k; ++kk) v += cu[(size_t)(kk + 1) * l - 1];
+            }
+            v *= 1.4426950408889634f;  // stored in log2 units: every consumer uses exp2
+            tcum[o + tt] = v;
+            // decay across this 32-position block (lane 0 to lane 31)
+            const float span = __shfl_sync(0xffffffffu, v, 0) - __shfl_sync(0xffffffffu, v, 31);
+            if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
+            if (dtT) dtT[o + tt] = sdt[tt][hl];
+            if (skipT) skipT[o + tt] = ssk[tt][hl];
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// The same from the per-position log-decay itself (dt * A_head, or `a` as given, fp32 or bf16), which is read once in the
+// caller's (b,T,h) layout through a shared-memory transpose and scanned inside each tile (warp per head, 32-lane segments
+// scanned side by side); also writes a_cumsum (b,h,c,l) in natural-log units.  Chunks of any length: where one
+// ends inside the tile its sums come from a second, segmented scan of the same values (CUT), so that they carry no
+// rounding of the positions before the chunk; where a chunk began in an earlier tile, the block adds up the positions
+// between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
+// kernels this replaces: 28 -> 7 us at (8, 2048, 24) with chunks of 64).  The skip array is transposed in a second round
+// through the panel of the log-decay.
+template <bool CUT>
+__global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __restrict__ a, int a_is_bf16,
+                                                                const float* __restrict__ dt, const float* __restrict__ A_head,
+                                                                float* __restrict__ cum, float* __restrict__ tcum,
+                                                                float* __restrict__ dtT, const float* __restrict__ skip,
+                                                                float* __restrict__ skipT, int* __restrict__ extreme, int T, int Tp,
+                                                                int h, int l) {
+    __shared__ float sa[LT][33];
+    __shared__ float sdt[LT][33];
+    __shared__ float sbef[8][33];
+    const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h0 = hg * 32;
+    const int t0 = kt * LT, rows = min(LT, T - t0);
+    const bool head_ok = h0 + lane < h;
+    const float Ah = (!a && head_ok) ? A_head[h0 + lane] : 0.f;
+    auto log_decay = [&](size_t i, float d) {
+        if (!a) return d * Ah;
+        return a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[i]) : ((const float*)a)[i];
+    };
+    const size_t row0 = (size_t)bb * T;
+#pragma unroll
+    for (int t = warp; t < LT; t += 8) {
+        const size_t i = (row0 + t0 + t) * h + h0 + lane;
+        float d = 0.f, av = 0.f;
+        if (head_ok && t < rows) {
+            if (dt) d = dt[i];
+            av = log_decay(i, d);
+        }
+        sa[t][lane] = av;
+        sdt[t][lane] = d;
+    }
+    const int i0 = t0 % l;  // positions of the tile's first chunk that lie in earlier tiles
+    if (i0) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int t = warp; t < i0; t += 8) {
+            const size_t i = (row0 + t0 - i0 + t) * h + h0 + lane;
+            if (head_ok) s += log_decay(i, dt && !a ? dt[i] : 0.f);
+        }
+        sbef[warp][lane] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {
+        const int hl = warp * 4 + i4, hh = h0 + hl;
+        if (hh >= h) break;  // warp-uniform
+        const size_t o = ((size_t)bb * h + hh) * Tp + t0, oc = ((size_t)bb * h + hh) * T + t0;
+        float before = 0.f;
+        if (i0) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) before += sbef[w][hl];
+        }
+        float v[LT / 32], c[LT / 32];
+#pragma unroll
+        for (int s4 = 0; s4 < LT / 32; ++s4) v[s4] = c[s4] = sa[s4 * 32 + lane][hl];
+        int pos[LT / 32];  // position inside its chunk
+        if (CUT) {
+#pragma unroll
+            for (int s4 = 0; s4 < LT / 32; ++s4) pos[s4] = (t0 + s4 * 32 + lane) % l;
+        }
+#pragma unroll
+        for (int of = 1; of < 32; of <<= 1) {
+#pragma unroll
+            for (int s4 = 0; s4 < LT / 32; ++s4) {
+                const float u = __shfl_up_sync(0xffffffffu, v[s4], of);
+                if (lane >= of) v[s4] += u;
+                if (CUT) {
+                    const float w = __shfl_up_sync(0xffffffffu, c[s4], of);
+                    if (lane >= of && pos[s4] >= of) c[s4] += w;
+                }
+            }
+        }
+        float run = 0.f, runc = before;
+#pragma unroll
+        for (int s4 = 0; s4 < LT / 32; ++s4) {
+            const int tt = s4 * 32 + lane;
+            v[s4] += run;
+            run = __shfl_sync(0xffffffffu, v[s4], 31);
+            if (CUT) {
+                if (pos[s4] > lane) c[s4] += runc;  // the chunk began before this segment
+                runc = __shfl_sync(0xffffffffu, c[s4], 31);
+            } else {
+                c[s4] = v[s4] + before;
+            }
+            if (tt < rows) cum[oc + tt] = c[s4];
+            const float w = v[s4] * 1.4426950408889634f;
+            tcum[o + tt] = w;
+            const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);
+            if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
+            if (dtT) dtT[o + tt] = sdt[tt][hl];
+        }
+    }
+    if (skip) {
+        __syncthreads();
+#pragma unroll
+        for (int t = warp; t < LT; t += 8)
+            sa[t][lane] = (head_ok && t < rows) ? skip[(row0 + t0 + t) * h + h0 + lane] : 0.f;
+        __syncthreads();
+#pragma unroll
+        for (int i4 = 0; i4 < 4; ++i4) {
+            const int hl = warp * 4 + i4, hh = h0 + hl;
+            if (hh >= h) break;
+            const size_t o = ((size_t)bb * h + hh) * Tp + t0;
+#pragma unroll
+            for (int s4 = 0; s4 < LT / 32; ++s4) skipT[o + s4 * 32 + lane] = sa[s4 * 32 + lane][hl];
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// Chunk cumsum: a (b,T,h) -> cum (b,h,c,l), inclusive within each chunk.  One block per
+// (chunk, batch); the [l][h] tile is staged through shared memory so that both the strided
+// read (h contiguous) and the transposed write (l contiguous) are coalesced; each warp scans
+// one head at a time with warp shuffles.  (SIMT path, and chunks beyond kFusedChunkMax.)
+// ------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) chunk_cumsum_kernel(const void* __restrict__ a, int a_is_bf16, const float* __restrict__ dt,
+                                                           const float* __restrict__ A_head, float* __restrict__ cum, int T, int h, int l) {
+    extern __shared__ float sm[];
+    const int k = blockIdx.x, bb = blockIdx.y;
+    const int ldh = h + 1;
+    for (int idx = threadIdx.x; idx < l * h; idx += 256) {
+        const int i = idx / h, hh = idx - i * h;
+        const size_t o = ((size_t)bb * T + (size_t)k * l + i) * h + hh;
+        sm[i * ldh + hh] = !a ? dt[o] * A_head[hh] : a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[o]) : ((const float*)a)[o];
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // lane <-> position inside a 32-position segment (coalesced stores); segments in sequence with a running carry
+    for (int hh = warp; hh < h; hh += 8) {
+        float* out = cum + ((size_t)bb * h + hh) * T + (size_t)k * l;
+        float carry = 0.f;
+        for (int i0 = 0; i0 < l; i0 += 32) {
+            const int i = i0 + lane;
+            float incl = i < l ? sm[i * ldh + hh] : 0.f;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                float v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            incl += carry;
+            if (i < l) out[i] = incl;
+            carry = __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+}
+
+// Total log-decay of every (batch, head) sequence from the within-chunk cumulative sums: sum of the chunks' last entries.
+__global__ void logdecay_total_kernel(const float* __restrict__ cum, float* __restrict__ out, int bh, int c, int l) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= bh) return;
+    float s = 0.f;
+    for (int k = 0; k < c; ++k) s += cum[((size_t)m * c + k) * l + l - 1];
+    out[m] = s;
+}
+
+}  // namespace cum
+}  // namespace ssd

@@ -22,6 +22,16 @@
 //   d a_t = sum_{s >= t} g_s                                  (reverse cumsum over the sequence)
 // This closed form replaces the reference's autograd re-run (src/kernels/ssd_scan.py:468-533)
 // and its O(l^3)-traffic segsum backward (:123-198).
+//
+// What bounds these kernels at the sizes the path is used at is the number of blocks and the chain of launches, then shared
+// memory.  So a block of the forward and of the backward takes as few heads of a group as it needs to fill the chip (dB and dC of a
+// group are then summed over its blocks), the row and the column pass of the backward are one launch, states are kept from the forward,
+// and the products read shared memory 16 bytes at a time without bank conflicts.  Forward + backward of (2, 512, 8 heads, 64,
+// d_state 64, chunk 64): 665 us of kernels with one block per group and 4-byte reads, 62 us now.
+//
+// The decay gradient is a small difference of large row and column sums; its rounding (about 1e-5 of dA_head) follows from the
+// order in which each element is summed.  That order is the same for any thread layout here: products run through k one by
+// one, row and column sums through quads of columns, then a tree over the sixteen quads.
 #pragma once
 #include "ssd_common.cuh"
 
@@ -29,12 +39,14 @@ namespace ssd {
 namespace simt {
 
 constexpr int TS = 64;    // output tile edge of every block-level product
-constexpr int NTHR = 256; // threads per block: 16 x 16, each owning a 4 x 4 micro-tile
+constexpr int NTHR = 256; // threads per block: 16 x 16, each owning a 4 x 4 micro-tile (rows 4 ty + r, columns 4 tx + c)
 
 struct Params {
     Dims d;
+    int lb;               // 64-row blocks per chunk
+    int splits;           // blocks that share the heads of a group
+    int share_ws;         // backward: the state panel takes the place of M0 and M1 (shapes that would not fit otherwise)
     const void* x;
-    const void* a;        // (b,T,h) per-position log-decay in a_dtype, or null
     const float* dt;      // (b,T,h) or null
     const float* A_head;  // (h) or null
     const float* D;       // (h) or null
@@ -43,11 +55,12 @@ struct Params {
     const void* dy;
     const float* init;    // (b,h,p,n) or null
     const float* dfinal;  // (b,h,p,n) or null
-    float* cum;           // (b,h,c,l)
+    const float* cum;     // (b,h,c,l)
     float* states;        // (b,c,h,p,n): local chunk states, then states entering each chunk
     float* dstates;       // (b,c,h,p,n): local state gradients, then dH_{k+1} per chunk
     float* final_state;   // (b,h,p,n)
-    float* dinit;         // (b,h,p,n)
+    float* final_keep;    // (b,h,p,n) second copy kept for the backward, or null
+    float* dinit;         // (b,h,p,n) or null
     void* y;
     void* dx;
     void* dB;
@@ -55,41 +68,83 @@ struct Params {
     float* g_row;         // (b,h,T)
     float* g_col;         // (b,h,T)
     float* ddtx;          // (b,h,T)  sum_p dX * x
-    const float* dyx;     // (b,h,T)  sum_p dy * x, or null (then the decay kernel reads x and dy itself)
+    float* dyx;           // (b,h,T)  sum_p dy * x, or null
     float* da;            // (b,T,h)
     float* ddt;           // (b,T,h)
     float* dAh_part;      // (b,h)
     float* dD_part;       // (b,h)
-    int a_is_bf16;
-    const float* g_row2;  // tile form only: second partial of g / ddtx / dyx (column halves), or null
-    const float* ddtx2;
-    const float* dyx2;
-    const float* gS;      // tile form only: (b,h,T/128,8) terms added to the last row of every tile, or null
-    int scan_len;         // decay gradient: 0 = reverse cumsum over the whole sequence (g holds the
-                          // row-minus-column terms), 128 = reverse cumsum inside each 128-tile (g holds the
-                          // gradient with respect to the tile-cumulative log-decay)
+    float* dB_part;       // (b,T,g*splits,n) fp32 when splits > 1, else null
+    float* dC_part;
 };
 
-__device__ __forceinline__ float load_a(const Params& P, int bb, int t, int hh) {
-    size_t i = ((size_t)bb * P.d.T + t) * P.d.h + hh;
-    if (P.dt) return P.dt[i] * P.A_head[hh];
-    return P.a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)P.a)[i]) : ((const float*)P.a)[i];
-}
+// ------------------------------------------------------------------------------------------
+// Shared-memory tiles: rows of `ld` floats, ld a multiple of 32, in units of four floats; unit q of row r sits at q ^ ((r / 4) % 8), so
+// that sixteen threads reading the same columns of rows 4 t + c hit different banks, and so do sixteen threads reading
+// neighbouring units of one row.
+// ------------------------------------------------------------------------------------------
+__host__ __device__ __forceinline__ int ld_of(int cols) { return (cols + 31) / 32 * 32; }
+__device__ __forceinline__ int sw(int r, int q, int ld) { return r * ld + ((q ^ ((r >> 2) & 7)) << 2); }
+__device__ __forceinline__ float4 ld4(const float* t, int r, int q, int ld) { return *reinterpret_cast<const float4*>(t + sw(r, q, ld)); }
+__device__ __forceinline__ float& at(float* t, int r, int c, int ld) { return t[sw(r, c >> 2, ld) + (c & 3)]; }
 
-// acc[r][c] += sum_k a(r,k) * b(k,c); the functors read shared memory.
-template <class FA, class FB>
-__device__ __forceinline__ void tile_mma(float (&acc)[4][4], int K, FA a, FB b) {
+#define SSD_FMA4(acc, av, b)                 \
+    do {                                     \
+        (acc)[0] = fmaf(av, (b).x, (acc)[0]); \
+        (acc)[1] = fmaf(av, (b).y, (acc)[1]); \
+        (acc)[2] = fmaf(av, (b).z, (acc)[2]); \
+        (acc)[3] = fmaf(av, (b).w, (acc)[3]); \
+    } while (0)
+
+// acc[r][c] += sum_k A[a0 + r][k] B[b0 + c][k], k in [ka, ka + K) of A and [0, K) of B (multiples of 4)
+__device__ __forceinline__ void mma_nt(float (&acc)[4][4], const float* A, int a0, int lda, int ka, const float* B, int b0, int ldb, int K) {
 #pragma unroll 2
-    for (int k = 0; k < K; ++k) {
-        float av[4], bv[4];
+    for (int k = 0; k < K; k += 4) {
+        float4 a[4], b[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) av[r] = a(r, k);
+        for (int r = 0; r < 4; ++r) a[r] = ld4(A, a0 + r, (ka + k) >> 2, lda);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) bv[c] = b(k, c);
+        for (int c = 0; c < 4; ++c) b[c] = ld4(B, b0 + c, k >> 2, ldb);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
+            for (int c = 0; c < 4; ++c)
+                acc[r][c] = fmaf(a[r].w, b[c].w, fmaf(a[r].z, b[c].z, fmaf(a[r].y, b[c].y, fmaf(a[r].x, b[c].x, acc[r][c]))));
+    }
+}
+// acc[r][c] += sum_{k < K} A[a0 + r][k] B[k][4 bq + c]
+__device__ __forceinline__ void mma_nn(float (&acc)[4][4], const float* A, int a0, int lda, const float* B, int bq, int ldb, int K) {
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        float4 a[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) a[r] = ld4(A, a0 + r, k >> 2, lda);
+        const float* Bk = B + k * ldb + ((bq ^ ((k >> 2) & 7)) << 2);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 b = *reinterpret_cast<const float4*>(Bk + q * ldb);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float av = q == 0 ? a[r].x : q == 1 ? a[r].y : q == 2 ? a[r].z : a[r].w;
+                SSD_FMA4(acc[r], av, b);
+            }
+        }
+    }
+}
+// acc[r][c] += sum_{k0 <= k < K} A[k][4 aq + r] B[k][4 bq + c]   (k0 and K multiples of 4)
+__device__ __forceinline__ void mma_tn(float (&acc)[4][4], const float* A, int aq, int lda, const float* B, int bq, int ldb, int k0, int K) {
+#pragma unroll 2
+    for (int k = k0; k < K; k += 4) {
+        const int f = (k >> 2) & 7;
+        const float* Ak = A + k * lda + ((aq ^ f) << 2);
+        const float* Bk = B + k * ldb + ((bq ^ f) << 2);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 a = *reinterpret_cast<const float4*>(Ak + q * lda), b = *reinterpret_cast<const float4*>(Bk + q * ldb);
+            SSD_FMA4(acc[0], a.x, b);
+            SSD_FMA4(acc[1], a.y, b);
+            SSD_FMA4(acc[2], a.z, b);
+            SSD_FMA4(acc[3], a.w, b);
+        }
     }
 }
 
@@ -100,53 +155,69 @@ __device__ __forceinline__ void zero(float (&acc)[4][4]) {
         for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
 }
 
-// Load `rows` x `cols` (row r at src + r*stride), zero-filling rows >= valid_rows and columns
-// in [cols, cols_pad), into dst[r*ld + c].
+// Four consecutive elements as floats (one wide access).
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    uint2 u;
+    u.x = *reinterpret_cast<const uint32_t*>(&a);
+    u.y = *reinterpret_cast<const uint32_t*>(&b);
+    *reinterpret_cast<uint2*>(p) = u;
+}
+// Whether rows of `cols` values (at a pitch of `stride`) can be moved four at a time.
 template <class T>
-__device__ __forceinline__ void load_tile(float* dst, int ld, const T* src, size_t stride, int rows, int valid_rows,
-                                          int cols, int cols_pad) {
-    for (int idx = threadIdx.x; idx < rows * cols_pad; idx += NTHR) {
-        int r = idx / cols_pad, c = idx - r * cols_pad;
-        float v = 0.f;
-        if (r < valid_rows && c < cols) v = to_f(src[(size_t)r * stride + c]);
-        dst[r * ld + c] = v;
+__device__ __forceinline__ bool wide(const T* base, int cols, size_t stride) {
+    return cols % 4 == 0 && stride % 4 == 0 && ((uintptr_t)base & (4 * sizeof(T) - 1)) == 0;
+}
+// Up to `n` of the four values v to o[0..3].
+template <class T>
+__device__ __forceinline__ void store_upto4(T* o, const float (&v)[4], int n, bool vec) {
+    if (vec) {
+        store4(o, v);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (c < n) o[c] = from_f<T>(v[c]);
+    }
+}
+template <class T>
+__device__ __forceinline__ float4 load_upto4(const T* p, int n, bool vec) {
+    if (vec) return load4(p);
+    return make_float4(n > 0 ? to_f(p[0]) : 0.f, n > 1 ? to_f(p[1]) : 0.f, n > 2 ? to_f(p[2]) : 0.f, n > 3 ? to_f(p[3]) : 0.f);
+}
+
+// `rows` rows of `cols` values (row r at src + r * stride, times scale[r] where given) into a shared tile; rows >= valid and the
+// columns up to the next multiple of 4 become zero.
+template <class T>
+__device__ __forceinline__ void load_tile(float* dst, int ld, const T* src, size_t stride, int rows, int valid, int cols,
+                                          const float* scale = nullptr) {
+    const int q4 = (cols + 3) / 4;
+    const bool vec = wide(src, cols, stride);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < rows * q4; i += NTHR) {
+        const int r = i / q4, q = i - r * q4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < valid) v = load_upto4(src + (size_t)r * stride + q * 4, cols - q * 4, vec);
+        if (scale) {
+            const float w = scale[r];
+            v.x *= w; v.y *= w; v.z *= w; v.w *= w;
+        }
+        *reinterpret_cast<float4*>(dst + sw(r, q, ld)) = v;
     }
 }
 
-// ------------------------------------------------------------------------------------------
-// Chunk cumsum: a (b,T,h) -> cum (b,h,c,l), inclusive within each chunk.  One block per
-// (chunk, batch); the [l][h] tile is staged through shared memory so that both the strided
-// read (h contiguous) and the transposed write (l contiguous) are coalesced; each warp scans
-// one head at a time with warp shuffles.
-// ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHR) chunk_cumsum_kernel(Params P) {
-    extern __shared__ float sm[];
-    const Dims& d = P.d;
-    const int k = blockIdx.x, bb = blockIdx.y;
-    const int ldh = d.h + 1;
-    for (int idx = threadIdx.x; idx < d.l * d.h; idx += NTHR) {
-        int i = idx / d.h, hh = idx - i * d.h;
-        sm[i * ldh + hh] = load_a(P, bb, k * d.l + i, hh);
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // lane <-> position inside a 32-position segment (coalesced stores); segments in sequence with a running carry
-    for (int hh = warp; hh < d.h; hh += NTHR / 32) {
-        float* out = P.cum + cum_off(d, bb, hh, k);
-        float carry = 0.f;
-        for (int i0 = 0; i0 < d.l; i0 += 32) {
-            const int i = i0 + lane;
-            float incl = i < d.l ? sm[i * ldh + hh] : 0.f;
+// Sum over the 16 threads (tx) that share a row; result valid in every lane of the group.
+__device__ __forceinline__ float row_reduce16(float v) {
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                float v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            incl += carry;
-            if (i < d.l) out[i] = incl;
-            carry = __shfl_sync(0xffffffffu, incl, 31);
-        }
-    }
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -157,15 +228,13 @@ __global__ void __launch_bounds__(NTHR) chunk_cumsum_kernel(Params P) {
 // ------------------------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(NTHR) chunk_state_kernel(Params P, int mode) {
-    __shared__ float Us[TS][TS + 4];
-    __shared__ float Vs[TS][TS + 4];
+    __shared__ __align__(16) float Us[TS * TS];
+    __shared__ __align__(16) float Vs[TS * TS];
     __shared__ float w[TS];
     const Dims& d = P.d;
-    const int nt = blockIdx.x, pt = blockIdx.y;
-    int z = blockIdx.z;
-    const int hh = z % d.h;
-    z /= d.h;
-    const int k = z % d.c, bb = z / d.c;
+    const int ntn = (d.n + TS - 1) / TS;
+    const int k = blockIdx.x % d.c, bb = blockIdx.x / d.c, hh = blockIdx.y;
+    const int p0 = (blockIdx.z / ntn) * TS, n0 = (blockIdx.z % ntn) * TS;
     const int gg = hh / d.hpg;
     const T* U = (const T*)(mode == 0 ? P.x : P.dy);
     const T* V = (const T*)(mode == 0 ? P.B : P.C);
@@ -175,9 +244,10 @@ __global__ void __launch_bounds__(NTHR) chunk_state_kernel(Params P, int mode) {
     float acc[4][4];
     zero(acc);
     for (int j0 = 0; j0 < d.l; j0 += TS) {
-        const int rows = min(TS, d.l - j0);
+        const int rows = min(TS, d.l - j0), t0 = k * d.l + j0;
+        if (j0) __syncthreads();
         if (threadIdx.x < TS) {
-            int j = j0 + threadIdx.x;
+            const int j = j0 + threadIdx.x;
             float wv = 0.f;
             if (j < d.l) {
                 if (mode == 0) {
@@ -189,36 +259,25 @@ __global__ void __launch_bounds__(NTHR) chunk_state_kernel(Params P, int mode) {
             }
             w[threadIdx.x] = wv;
         }
+        load_tile(Vs, TS, V + bc_off(d, bb, t0, gg) + n0, (size_t)d.g * d.n, TS, rows, min(TS, d.n - n0));
         __syncthreads();
-        const int t0 = k * d.l + j0;
-        for (int idx = threadIdx.x; idx < TS * TS; idx += NTHR) {
-            int r = idx >> 6, cc = idx & 63;
-            float u = 0.f, v = 0.f;
-            if (r < rows) {
-                int pp = pt * TS + cc, nn = nt * TS + cc;
-                if (pp < d.p) u = to_f(U[x_off(d, bb, t0 + r, hh) + pp]) * w[r];
-                if (nn < d.n) v = to_f(V[bc_off(d, bb, t0 + r, gg) + nn]);
-            }
-            Us[r][cc] = u;
-            Vs[r][cc] = v;
-        }
+        load_tile(Us, TS, U + x_off(d, bb, t0, hh) + p0, (size_t)d.h * d.p, TS, rows, min(TS, d.p - p0), w);
         __syncthreads();
-        tile_mma(acc, TS, [&](int r, int kk) { return Us[kk][ty * 4 + r]; },
-                 [&](int kk, int cc) { return Vs[kk][tx * 4 + cc]; });
-        __syncthreads();
+        mma_tn(acc, Us, ty, TS, Vs, tx, TS, 0, (rows + 3) / 4 * 4);
     }
     float* out = (mode == 0 ? P.states : P.dstates) + st_off(d, bb, k, hh);
+    const int nn = n0 + tx * 4;
+    const bool vec = d.n % 4 == 0;
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            int pp = pt * TS + ty * 4 + r, nn = nt * TS + tx * 4 + cc;
-            if (pp < d.p && nn < d.n) out[(size_t)pp * d.n + nn] = acc[r][cc];
-        }
+    for (int r = 0; r < 4; ++r) {
+        const int pp = p0 + ty * 4 + r;
+        if (pp < d.p && nn < d.n) store_upto4(out + (size_t)pp * d.n + nn, acc[r], d.n - nn, vec);
+    }
 }
 
 // ------------------------------------------------------------------------------------------
-// Inter-chunk state passing, one thread per state element, sequential over chunks.
+// Inter-chunk state passing, one thread per state element, sequential over chunks; eight chunks' values are fetched ahead
+// of the chain of multiply-adds.
 // forward : slot k <- H_k (state entering chunk k), H_{k+1} = exp(S_k) H_k + local_k ; final = H_c
 // reverse : slot k <- Q_k = dH_{k+1},               dH_k   = exp(S_k) Q_k + local_k ; dinit = dH_0
 // ------------------------------------------------------------------------------------------
@@ -228,427 +287,438 @@ __global__ void __launch_bounds__(NTHR) state_passing_kernel(Params P, int rever
     const size_t e = (size_t)blockIdx.x * NTHR + threadIdx.x;
     if (e >= pn) return;
     const int hh = blockIdx.y, bb = blockIdx.z;
-    float* buf = reverse ? P.dstates : P.states;
+    float* buf = (reverse ? P.dstates : P.states) + e;
     const float* seed = reverse ? P.dfinal : P.init;
-    float H = seed ? seed[((size_t)bb * d.h + hh) * pn + e] : 0.f;
-    for (int s = 0; s < d.c; ++s) {
-        const int k = reverse ? d.c - 1 - s : s;
-        const float S = P.cum[cum_off(d, bb, hh, k) + d.l - 1];
-        float* slot = buf + st_off(d, bb, k, hh) + e;
-        const float loc = *slot;
-        *slot = H;
-        H = __expf(S) * H + loc;
+    const size_t o = ((size_t)bb * d.h + hh) * pn + e;
+    float H = seed ? seed[o] : 0.f;
+    constexpr int BATCH = 8;
+    for (int s0 = 0; s0 < d.c; s0 += BATCH) {
+        float loc[BATCH], S[BATCH];
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j)
+            if (s0 + j < d.c) {
+                const int k = reverse ? d.c - 1 - (s0 + j) : s0 + j;
+                loc[j] = buf[st_off(d, bb, k, hh)];
+                S[j] = P.cum[cum_off(d, bb, hh, k) + d.l - 1];
+            }
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j)
+            if (s0 + j < d.c) {
+                const int k = reverse ? d.c - 1 - (s0 + j) : s0 + j;
+                buf[st_off(d, bb, k, hh)] = H;
+                H = __expf(S[j]) * H + loc[j];
+            }
     }
     float* out = reverse ? P.dinit : P.final_state;
-    if (out) out[((size_t)bb * d.h + hh) * pn + e] = H;
+    if (out) out[o] = H;
+    if (!reverse && P.final_keep) P.final_keep[o] = H;
+}
+
+// Which rows a block of the forward or the backward works on: 64-row block `ib` of chunk k, heads h0 .. h0 + hps - 1 of group gg.
+struct Where {
+    int k, ib, bb, gg, sp, h0, hps;
+};
+__device__ __forceinline__ Where where(const Params& P) {
+    Where w;
+    int z = blockIdx.x;
+    w.ib = z % P.lb;
+    z /= P.lb;
+    w.k = z % P.d.c;
+    w.bb = z / P.d.c;
+    w.gg = blockIdx.y / P.splits;
+    w.sp = blockIdx.y % P.splits;
+    w.hps = P.d.hpg / P.splits;
+    w.h0 = w.gg * P.d.hpg + w.sp * w.hps;
+    return w;
+}
+// cum of the 64 positions from j0 of a chunk, and dt of the same positions (1 without dt, 0 behind the chunk)
+__device__ __forceinline__ void load_scalars(const Params& P, int bb, int hh, int k, int j0, float* cum64, float* dt64) {
+    const Dims& d = P.d;
+    if (threadIdx.x < TS) {
+        const int j = j0 + threadIdx.x;
+        const bool ok = j < d.l;
+        cum64[threadIdx.x] = ok ? P.cum[cum_off(d, bb, hh, k) + j] : 0.f;
+        if (dt64) dt64[threadIdx.x] = (ok && P.dt) ? P.dt[((size_t)bb * d.T + k * d.l + j) * d.h + hh] : 1.f;
+    }
 }
 
 // ------------------------------------------------------------------------------------------
-// Chunk scan output.  Block = 64 rows i of one (batch, chunk, head); loops the causal column
+// Chunk scan output.  Block = 64 rows i of one (batch, chunk, split of a group); per head it loops the causal column
 // blocks j <= i:  Y_i = sum_j ((C_i B_j^T) o L_ij) X_j  +  diag(e_i) C_i H_k^T  (+ D x_i).
 // ------------------------------------------------------------------------------------------
 template <class T, int PT>
 __global__ void __launch_bounds__(NTHR) chunk_scan_kernel(Params P) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     const Dims& d = P.d;
-    const int ib = blockIdx.x, hh = blockIdx.y;
-    const int k = blockIdx.z % d.c, bb = blockIdx.z / d.c;
-    const int gg = hh / d.hpg;
-    const int ldn = d.n + 1, ldp = PT * TS + 1, ldg = TS + 1;
-    const int hrows = max(TS, d.p);
-    float* Cs = sm;                  // [64][n+1]
-    float* Bs = Cs + TS * ldn;       // [max(64,p)][n+1]  (B_j, later H_k)
-    float* Xs = Bs + hrows * ldn;    // [64][PT*64+1]
-    float* Gs = Xs + TS * ldp;       // [64][65]
-    float* cum_i = Gs + TS * ldg;    // [64]
-    float* cum_j = cum_i + TS;       // [64]
-    const T* x = (const T*)P.x;
-    const T* Bp = (const T*)P.B;
-    const T* Cp = (const T*)P.C;
-    const float* cum = P.cum + cum_off(d, bb, hh, k);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int i0 = ib * TS, t_i0 = k * d.l + i0;
-    const int rows_i = min(TS, d.l - i0);
-
-    load_tile(Cs, ldn, Cp + bc_off(d, bb, t_i0, gg), (size_t)d.g * d.n, TS, rows_i, d.n, d.n);
-    if (threadIdx.x < TS) cum_i[threadIdx.x] = threadIdx.x < rows_i ? cum[i0 + threadIdx.x] : 0.f;
-    float accY[PT][4][4];
-#pragma unroll
-    for (int q = 0; q < PT; ++q) zero(accY[q]);
-
-    for (int jb = 0; jb <= ib; ++jb) {
-        const int j0 = jb * TS, t_j0 = k * d.l + j0;
-        const int rows_j = min(TS, d.l - j0);
-        __syncthreads();
-        load_tile(Bs, ldn, Bp + bc_off(d, bb, t_j0, gg), (size_t)d.g * d.n, TS, rows_j, d.n, d.n);
-        load_tile(Xs, ldp, x + x_off(d, bb, t_j0, hh), (size_t)d.h * d.p, TS, rows_j, d.p, PT * TS);
-        if (threadIdx.x < TS) cum_j[threadIdx.x] = threadIdx.x < rows_j ? cum[j0 + threadIdx.x] : 0.f;
-        __syncthreads();
-        if (P.dt) {  // X = x * dt
-            for (int idx = threadIdx.x; idx < rows_j * PT * TS; idx += NTHR) {
-                int r = idx / (PT * TS), cc = idx - r * (PT * TS);
-                Xs[r * ldp + cc] *= P.dt[((size_t)bb * d.T + t_j0 + r) * d.h + hh];
-            }
-        }
-        float s[4][4];
-        zero(s);
-        tile_mma(s, d.n, [&](int r, int kk) { return Cs[(ty * 4 + r) * ldn + kk]; },
-                 [&](int kk, int cc) { return Bs[(tx * 4 + cc) * ldn + kk]; });
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                int il = ty * 4 + r, jl = tx * 4 + cc;
-                bool ok = (i0 + il >= j0 + jl) && il < rows_i && jl < rows_j;
-                Gs[il * ldg + jl] = ok ? s[r][cc] * __expf(cum_i[il] - cum_j[jl]) : 0.f;
-            }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < PT; ++q)
-            tile_mma(accY[q], TS, [&](int r, int kk) { return Gs[(ty * 4 + r) * ldg + kk]; },
-                     [&](int kk, int cc) { return Xs[kk * ldp + q * TS + tx * 4 + cc]; });
-    }
-    // state -> output
-    __syncthreads();
-    load_tile(Bs, ldn, P.states + st_off(d, bb, k, hh), (size_t)d.n, hrows, d.p, d.n, d.n);
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PT; ++q) {
-        float o[4][4];
-        zero(o);
-        tile_mma(o, d.n, [&](int r, int kk) { return Cs[(ty * 4 + r) * ldn + kk]; },
-                 [&](int kk, int cc) { return Bs[min(q * TS + tx * 4 + cc, hrows - 1) * ldn + kk]; });
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float e = __expf(cum_i[ty * 4 + r]);
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) accY[q][r][cc] += e * o[r][cc];
-        }
-    }
-    T* y = (T*)P.y;
-    const float Dh = P.D ? P.D[hh] : 0.f;
-#pragma unroll
-    for (int q = 0; q < PT; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                int il = ty * 4 + r, pp = q * TS + tx * 4 + cc;
-                if (il < rows_i && pp < d.p) {
-                    size_t o = x_off(d, bb, t_i0 + il, hh) + pp;
-                    float v = accY[q][r][cc];
-                    if (P.D) v += Dh * to_f(x[o]);
-                    y[o] = from_f<T>(v);
-                }
-            }
-}
-
-// Sum over the 16 threads (tx) that share a row; result valid in every lane of the group.
-__device__ __forceinline__ float row_reduce16(float v) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// ------------------------------------------------------------------------------------------
-// Backward, row pass.  Block = 64 rows i of one (batch, chunk, group); loops the heads of the
-// group and the causal column blocks:  dC_i = sum_h [ sum_j dS_ij B_j + diag(e) dY_i H_k ],
-// g_row[i] = rowsum_i(M) + <dC_off_i, C_i> per head.
-// ------------------------------------------------------------------------------------------
-template <class T, int NTN>
-__global__ void __launch_bounds__(NTHR) bwd_row_kernel(Params P) {
-    extern __shared__ float sm[];
-    const Dims& d = P.d;
-    const int ib = blockIdx.x, gg = blockIdx.y;
-    const int k = blockIdx.z % d.c, bb = blockIdx.z / d.c;
-    const int pp_pad = ((d.p + 3) / 4) * 4;
-    const int ldn = d.n + 1, ldp = pp_pad + 1, ldg = TS + 1;
-    const int hrows = max(TS, d.p);
-    float* Cs = sm;                  // [64][n+1]      C_i
-    float* Bs = Cs + TS * ldn;       // [max(64,p)][n+1]  B_j, later H_k
-    float* dYs = Bs + hrows * ldn;   // [64][p+1]      dY_i
-    float* Xs = dYs + TS * ldp;      // [64][p+1]      X_j
-    float* dSs = Xs + TS * ldp;      // [64][65]
-    float* cum_i = dSs + TS * ldg;
+    const Where w = where(P);
+    const int bb = w.bb, k = w.k, ldn = ld_of(d.n), ldp = ld_of(d.p), n4 = (d.n + 3) / 4 * 4;
+    float* Cs = sm;                    // [64][ldn]
+    float* Bs = Cs + TS * ldn;         // [64][ldn]
+    float* Xs = Bs + TS * ldn;         // [64][ldp]
+    float* Gs = Xs + TS * ldp;         // [64][64]
+    float* Hs = Gs + TS * TS;          // [p][64]: 64 columns of the entering state
+    float* cum_i = Hs + PT * TS * TS;  // [64] each
     float* cum_j = cum_i + TS;
+    float* dt_j = cum_j + TS;
     const T* x = (const T*)P.x;
-    const T* dy = (const T*)P.dy;
-    const T* Bp = (const T*)P.B;
-    const T* Cp = (const T*)P.C;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int i0 = ib * TS, t_i0 = k * d.l + i0;
+    const int i0 = w.ib * TS, t_i0 = k * d.l + i0;
     const int rows_i = min(TS, d.l - i0);
-    float dC[NTN][4][4];
+    load_tile(Cs, ldn, (const T*)P.C + bc_off(d, bb, t_i0, w.gg), (size_t)d.g * d.n, TS, rows_i, d.n);
+    float s[4][4];
+    for (int hl = 0; hl < w.hps; ++hl) {
+        const int hh = w.h0 + hl;
+        const float* H = P.states + st_off(d, bb, k, hh);
+        float acc[PT][4][4];
 #pragma unroll
-    for (int q = 0; q < NTN; ++q) zero(dC[q]);
-    load_tile(Cs, ldn, Cp + bc_off(d, bb, t_i0, gg), (size_t)d.g * d.n, TS, rows_i, d.n, d.n);
-
-    for (int hl = 0; hl < d.hpg; ++hl) {
-        const int hh = gg * d.hpg + hl;
-        const float* cum = P.cum + cum_off(d, bb, hh, k);
-        __syncthreads();
-        load_tile(dYs, ldp, dy + x_off(d, bb, t_i0, hh), (size_t)d.h * d.p, TS, rows_i, d.p, pp_pad);
-        if (threadIdx.x < TS) cum_i[threadIdx.x] = threadIdx.x < rows_i ? cum[i0 + threadIdx.x] : 0.f;
-        float rowacc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int jb = 0; jb <= ib; ++jb) {
+        for (int q = 0; q < PT; ++q) zero(acc[q]);
+        if (hl) __syncthreads();
+        load_scalars(P, bb, hh, k, i0, cum_i, nullptr);
+        load_tile(Hs, TS, H, d.n, d.p, d.p, min(TS, d.n));
+        for (int jb = 0; jb <= w.ib; ++jb) {
             const int j0 = jb * TS, t_j0 = k * d.l + j0;
             const int rows_j = min(TS, d.l - j0);
+            if (jb) __syncthreads();
+            if (hl == 0 || w.ib) load_tile(Bs, ldn, (const T*)P.B + bc_off(d, bb, t_j0, w.gg), (size_t)d.g * d.n, TS, rows_j, d.n);
+            load_tile(Xs, ldp, x + x_off(d, bb, t_j0, hh), (size_t)d.h * d.p, TS, rows_j, d.p);
+            load_scalars(P, bb, hh, k, j0, cum_j, dt_j);
             __syncthreads();
-            load_tile(Bs, ldn, Bp + bc_off(d, bb, t_j0, gg), (size_t)d.g * d.n, TS, rows_j, d.n, d.n);
-            load_tile(Xs, ldp, x + x_off(d, bb, t_j0, hh), (size_t)d.h * d.p, TS, rows_j, d.p, pp_pad);
-            if (threadIdx.x < TS) cum_j[threadIdx.x] = threadIdx.x < rows_j ? cum[j0 + threadIdx.x] : 0.f;
-            __syncthreads();
-            if (P.dt) {
-                for (int idx = threadIdx.x; idx < rows_j * pp_pad; idx += NTHR) {
-                    int r = idx / pp_pad, cc = idx - r * pp_pad;
-                    Xs[r * ldp + cc] *= P.dt[((size_t)bb * d.T + t_j0 + r) * d.h + hh];
-                }
-                __syncthreads();
+            if (hl == 0 || w.ib) {  // a chunk of one block: C B^T serves every head of this block
+                zero(s);
+                mma_nt(s, Cs, ty * 4, ldn, 0, Bs, tx * 4, ldn, n4);
             }
-            float s[4][4], dg[4][4];
-            zero(s);
-            zero(dg);
-            tile_mma(s, d.n, [&](int r, int kk) { return Cs[(ty * 4 + r) * ldn + kk]; },
-                     [&](int kk, int cc) { return Bs[(tx * 4 + cc) * ldn + kk]; });
-            tile_mma(dg, d.p, [&](int r, int kk) { return dYs[(ty * 4 + r) * ldp + kk]; },
-                     [&](int kk, int cc) { return Xs[(tx * 4 + cc) * ldp + kk]; });
+            if (jb == 0) {  // state -> output, while the scalars of this head are fresh
+                for (int n0 = 0; n0 < d.n; n0 += TS) {
+                    if (n0) {
+                        __syncthreads();
+                        load_tile(Hs, TS, H + n0, d.n, d.p, d.p, min(TS, d.n - n0));
+                        __syncthreads();
+                    }
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    int il = ty * 4 + r, jl = tx * 4 + cc;
-                    bool ok = (i0 + il >= j0 + jl) && il < rows_i && jl < rows_j;
-                    float ds = ok ? dg[r][cc] * __expf(cum_i[il] - cum_j[jl]) : 0.f;
-                    rowacc[r] += ds * s[r][cc];
-                    dSs[il * ldg + jl] = ds;
+                    for (int q = 0; q < PT; ++q) mma_nt(acc[q], Cs, ty * 4, ldn, n0, Hs, q * TS + tx * 4, TS, min(TS, n4 - n0));
                 }
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < NTN; ++q)
-                if (q * TS < d.n)
-                    tile_mma(dC[q], TS, [&](int r, int kk) { return dSs[(ty * 4 + r) * ldg + kk]; },
-                             [&](int kk, int cc) { return Bs[kk * ldn + min(q * TS + tx * 4 + cc, d.n - 1)]; });
-        }
-        // state term: dC_off = diag(e) dY_i H_k
-        __syncthreads();
-        load_tile(Bs, ldn, P.states + st_off(d, bb, k, hh), (size_t)d.n, hrows, d.p, d.n, d.n);
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < NTN; ++q)
-            if (q * TS < d.n) {
-                float o[4][4];
-                zero(o);
-                tile_mma(o, d.p, [&](int r, int kk) { return dYs[(ty * 4 + r) * ldp + kk]; },
-                         [&](int kk, int cc) { return Bs[kk * ldn + min(q * TS + tx * 4 + cc, d.n - 1)]; });
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const float e = __expf(cum_i[ty * 4 + r]);
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) {
-                        int nn = q * TS + tx * 4 + cc;
-                        if (nn < d.n) {
-                            float v = e * o[r][cc];
-                            dC[q][r][cc] += v;
-                            rowacc[r] += v * Cs[(ty * 4 + r) * ldn + nn];
-                        }
-                    }
+                    for (int q = 0; q < PT; ++q)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) acc[q][r][c] *= e;
                 }
             }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            float v = row_reduce16(rowacc[r]);
-            int il = ty * 4 + r;
-            if (tx == 0 && il < rows_i) P.g_row[((size_t)bb * d.h + hh) * d.T + t_i0 + il] = v;
+            for (int r = 0; r < 4; ++r) {
+                float g[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int il = ty * 4 + r, jl = tx * 4 + c;
+                    const bool ok = (i0 + il >= j0 + jl) && il < rows_i && jl < rows_j;
+                    g[c] = ok ? s[r][c] * __expf(cum_i[il] - cum_j[jl]) * dt_j[jl] : 0.f;
+                }
+                *reinterpret_cast<float4*>(Gs + sw(ty * 4 + r, tx, TS)) = make_float4(g[0], g[1], g[2], g[3]);
+            }
+            __syncthreads();
+            const int kend = jb == w.ib ? ty * 4 + 4 : TS;  // on the diagonal only the columns up to the row
+#pragma unroll
+            for (int q = 0; q < PT; ++q) mma_nn(acc[q], Gs, ty * 4, TS, Xs, q * 16 + tx, ldp, kend);
+        }
+        T* y = (T*)P.y + x_off(d, bb, t_i0, hh);
+        const bool vec = wide(y, d.p, (size_t)d.h * d.p);
+        const float Dh = P.D ? P.D[hh] : 0.f;
+#pragma unroll
+        for (int q = 0; q < PT; ++q) {
+            const int pp = q * TS + tx * 4;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int il = ty * 4 + r;
+                if (il >= rows_i || pp >= d.p) continue;
+                if (P.D) {  // Xs holds the block's own rows (the last column block)
+                    const float4 xv = ld4(Xs, il, pp >> 2, ldp);
+                    SSD_FMA4(acc[q][r], Dh, xv);
+                }
+                store_upto4(y + (size_t)il * d.h * d.p + pp, acc[q][r], d.p - pp, vec);
+            }
         }
     }
-    T* dCo = (T*)P.dC;
-#pragma unroll
-    for (int q = 0; q < NTN; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                int il = ty * 4 + r, nn = q * TS + tx * 4 + cc;
-                if (il < rows_i && nn < d.n) dCo[bc_off(d, bb, t_i0 + il, gg) + nn] = from_f<T>(dC[q][r][cc]);
-            }
+}
+__host__ inline size_t chunk_scan_smem(const Dims& d, int pt) {
+    return ((size_t)2 * TS * ld_of(d.n) + TS * ld_of(d.p) + TS * TS + (size_t)pt * TS * TS + 3 * TS) * 4;
 }
 
 // ------------------------------------------------------------------------------------------
-// Backward, column pass.  Block = 64 columns j of one (batch, chunk, group); loops the heads and
-// the row blocks i >= j:  dX_j = sum_i G_ij^T dY_i + diag(d) B_j Q^T,
-// dB_j = sum_h [ sum_i dS_ij^T C_i + diag(d) X_j Q ],  g_col[j] = colsum_j(M) + <dB_st_j, B_j>,
-// dx = dX * dt + D * dy,  ddtx[j] = <dX_j, x_j>.
+// Backward of 64 positions of one (batch, chunk, split of a group); the heads in an inner loop.  blockIdx.z = 0 is the row
+// pass over the causal column blocks j <= i:
+//   dC_i = sum_h [ sum_j dS_ij B_j + diag(e) dY_i H_k ],   g_row[i] = rowsum_i(M) + <dC_off_i, C_i> per head
+// and blockIdx.z = 1 the column pass over the row blocks i >= j:
+//   dX_j = sum_i G_ij^T dY_i + diag(d) B_j Q^T,  dB_j = sum_h [ sum_i dS_ij^T C_i + diag(d) X_j Q ],
+//   g_col[j] = colsum_j(M) + <dB_st_j, B_j>,  dx = dX * dt + D * dy,  ddtx[j] = <dX_j, x_j>,  dyx[j] = <dy_j, x_j>.
+// The panel Ws holds 64 columns of H (row pass) or Q (column pass) at a time.
 // ------------------------------------------------------------------------------------------
-template <class T, int NTN, int PT>
-__global__ void __launch_bounds__(NTHR) bwd_col_kernel(Params P) {
-    extern __shared__ float sm[];
+template <int NTN, class T>
+__device__ __forceinline__ void store_bc(const Params& P, const Where& w, int t0, int rows, const float (&acc)[NTN][4][4], float* part, T* out) {
     const Dims& d = P.d;
-    const int jb = blockIdx.x, gg = blockIdx.y;
-    const int k = blockIdx.z % d.c, bb = blockIdx.z / d.c;
-    const int ldn = d.n + 1, ldp = PT * TS + 1, ldg = TS + 1;
-    const int hrows = max(TS, d.p);
-    float* Bs = sm;                   // [64][n+1]          B_j
-    float* Cs = Bs + TS * ldn;        // [max(64,p)][n+1]   C_i, later Q_k
-    float* Xs = Cs + hrows * ldn;     // [64][PT*64+1]      X_j (already scaled by dt)
-    float* dYs = Xs + TS * ldp;       // [64][PT*64+1]      dY_i
-    float* GT = dYs + TS * ldp;       // [64 j][65]         G^T
-    float* dST = GT + TS * ldg;       // [64 j][65]         dS^T
-    float* cum_j = dST + TS * ldg;
-    float* cum_i = cum_j + TS;
-    float* dt_j = cum_i + TS;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int q = 0; q < NTN; ++q) {
+        const int nn = q * TS + tx * 4;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int il = ty * 4 + r;
+            if (il >= rows || nn >= d.n) continue;
+            if (part) {
+                float* o = part + ((((size_t)w.bb * d.T + t0 + il) * d.g + w.gg) * P.splits + w.sp) * d.n + nn;
+                store_upto4(o, acc[q][r], d.n - nn, d.n % 4 == 0);
+            } else {
+                T* o = out + bc_off(d, w.bb, t0 + il, w.gg) + nn;
+                store_upto4(o, acc[q][r], d.n - nn, wide(o, d.n, 4));
+            }
+        }
+    }
+}
+
+template <class T, int PT, int NTN>
+__global__ void __launch_bounds__(NTHR, PT * NTN == 1 ? 2 : 1) chunk_bwd_kernel(Params P) {
+    extern __shared__ __align__(16) float sm[];
+    const Dims& d = P.d;
+    const Where w = where(P);
+    const int bb = w.bb, k = w.k, ldn = ld_of(d.n), ldp = ld_of(d.p), n4 = (d.n + 3) / 4 * 4, p4 = (d.p + 3) / 4 * 4;
+    float* Rn = sm;                    // [64][ldn]  C_i (row pass) or B_j (column pass): the block's own positions
+    float* On = Rn + TS * ldn;         // [64][ldn]  B_j or C_i: the positions it loops over
+    float* Rp = On + TS * ldn;         // [64][ldp]  dY_i or X_j
+    float* Op = Rp + TS * ldp;         // [64][ldp]  X_j or dY_i
+    float* M0 = Op + TS * ldp;         // [64][64]   dS (row pass), dS^T (column pass)
+    float* M1 = M0 + TS * TS;          // [64][64]   G^T (column pass)
+    float* Ws = P.share_ws ? M0 : M1 + TS * TS;  // [p4][64]
+    float* cum_r = M1 + TS * TS + (P.share_ws ? 0 : PT * TS * TS);  // [64] each: own positions, and the ones looped over
+    float* dt_r = cum_r + TS;
+    float* cum_o = dt_r + TS;
+    float* dt_o = cum_o + TS;
     const T* x = (const T*)P.x;
     const T* dy = (const T*)P.dy;
     const T* Bp = (const T*)P.B;
     const T* Cp = (const T*)P.C;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int j0 = jb * TS, t_j0 = k * d.l + j0;
-    const int rows_j = min(TS, d.l - j0);
-    const int nib = (d.l + TS - 1) / TS;
-    float dBa[NTN][4][4];
+    const int r0 = w.ib * TS, t_r0 = k * d.l + r0;
+    const int rows_r = min(TS, d.l - r0);
+    const bool row_pass = blockIdx.z == 0;
+    const size_t xs = (size_t)d.h * d.p, bs = (size_t)d.g * d.n;
+    float acc[NTN][4][4];  // dC_i or dB_j
 #pragma unroll
-    for (int q = 0; q < NTN; ++q) zero(dBa[q]);
-    load_tile(Bs, ldn, Bp + bc_off(d, bb, t_j0, gg), (size_t)d.g * d.n, TS, rows_j, d.n, d.n);
+    for (int q = 0; q < NTN; ++q) zero(acc[q]);
+    load_tile(Rn, ldn, (row_pass ? Cp : Bp) + bc_off(d, bb, t_r0, w.gg), bs, TS, rows_r, d.n);
+    float s[4][4];
 
-    for (int hl = 0; hl < d.hpg; ++hl) {
-        const int hh = gg * d.hpg + hl;
-        const float* cum = P.cum + cum_off(d, bb, hh, k);
-        const float S = cum[d.l - 1];
-        __syncthreads();
-        load_tile(Xs, ldp, x + x_off(d, bb, t_j0, hh), (size_t)d.h * d.p, TS, rows_j, d.p, PT * TS);
-        if (threadIdx.x < TS) {
-            bool ok = threadIdx.x < rows_j;
-            cum_j[threadIdx.x] = ok ? cum[j0 + threadIdx.x] : 0.f;
-            dt_j[threadIdx.x] = (ok && P.dt) ? P.dt[((size_t)bb * d.T + t_j0 + threadIdx.x) * d.h + hh] : 1.f;
-        }
-        __syncthreads();
-        if (P.dt) {
-            for (int idx = threadIdx.x; idx < rows_j * PT * TS; idx += NTHR) {
-                int r = idx / (PT * TS), cc = idx - r * (PT * TS);
-                Xs[r * ldp + cc] *= dt_j[r];
-            }
-        }
-        float accX[PT][4][4];
-#pragma unroll
-        for (int q = 0; q < PT; ++q) zero(accX[q]);
-        float colacc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int ib = jb; ib < nib; ++ib) {
-            const int i0 = ib * TS, t_i0 = k * d.l + i0;
-            const int rows_i = min(TS, d.l - i0);
-            __syncthreads();
-            load_tile(Cs, ldn, Cp + bc_off(d, bb, t_i0, gg), (size_t)d.g * d.n, TS, rows_i, d.n, d.n);
-            load_tile(dYs, ldp, dy + x_off(d, bb, t_i0, hh), (size_t)d.h * d.p, TS, rows_i, d.p, PT * TS);
-            if (threadIdx.x < TS) cum_i[threadIdx.x] = threadIdx.x < rows_i ? cum[i0 + threadIdx.x] : 0.f;
-            __syncthreads();
-            float st[4][4], dgt[4][4];  // transposed: rows j, columns i
-            zero(st);
-            zero(dgt);
-            tile_mma(st, d.n, [&](int r, int kk) { return Bs[(ty * 4 + r) * ldn + kk]; },
-                     [&](int kk, int cc) { return Cs[(tx * 4 + cc) * ldn + kk]; });
-            tile_mma(dgt, d.p, [&](int r, int kk) { return Xs[(ty * 4 + r) * ldp + kk]; },
-                     [&](int kk, int cc) { return dYs[(tx * 4 + cc) * ldp + kk]; });
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    int jl = ty * 4 + r, il = tx * 4 + cc;
-                    bool ok = (i0 + il >= j0 + jl) && il < rows_i && jl < rows_j;
-                    float Lv = ok ? __expf(cum_i[il] - cum_j[jl]) : 0.f;
-                    float ds = dgt[r][cc] * Lv;
-                    colacc[r] += ds * st[r][cc];
-                    GT[jl * ldg + il] = st[r][cc] * Lv;
-                    dST[jl * ldg + il] = ds;
+    if (row_pass) {
+        for (int hl = 0; hl < w.hps; ++hl) {
+            const int hh = w.h0 + hl;
+            const float* H = P.states + st_off(d, bb, k, hh);
+            float rowacc[4] = {0.f, 0.f, 0.f, 0.f};
+            if (hl) __syncthreads();
+            load_tile(Rp, ldp, dy + x_off(d, bb, t_r0, hh), xs, TS, rows_r, d.p);
+            if (!P.share_ws) load_tile(Ws, TS, H, d.n, p4, d.p, min(TS, d.n));
+            load_scalars(P, bb, hh, k, r0, cum_r, nullptr);
+            for (int jb = 0; jb <= w.ib; ++jb) {
+                const int j0 = jb * TS, t_j0 = k * d.l + j0;
+                const int rows_j = min(TS, d.l - j0);
+                if (jb) __syncthreads();
+                load_scalars(P, bb, hh, k, j0, cum_o, dt_o);
+                if (hl == 0 || w.ib) load_tile(On, ldn, Bp + bc_off(d, bb, t_j0, w.gg), bs, TS, rows_j, d.n);
+                __syncthreads();
+                load_tile(Op, ldp, x + x_off(d, bb, t_j0, hh), xs, TS, rows_j, d.p, P.dt ? dt_o : nullptr);
+                if (hl == 0 || w.ib) {
+                    zero(s);
+                    mma_nt(s, Rn, ty * 4, ldn, 0, On, tx * 4, ldn, n4);
                 }
-            __syncthreads();
+                __syncthreads();
+                float dg[4][4];
+                zero(dg);
+                mma_nt(dg, Rp, ty * 4, ldp, 0, Op, tx * 4, ldp, p4);
 #pragma unroll
-            for (int q = 0; q < PT; ++q)
-                tile_mma(accX[q], TS, [&](int r, int kk) { return GT[(ty * 4 + r) * ldg + kk]; },
-                         [&](int kk, int cc) { return dYs[kk * ldp + q * TS + tx * 4 + cc]; });
+                for (int r = 0; r < 4; ++r) {
+                    float v[4];
 #pragma unroll
-            for (int q = 0; q < NTN; ++q)
-                if (q * TS < d.n)
-                    tile_mma(dBa[q], TS, [&](int r, int kk) { return dST[(ty * 4 + r) * ldg + kk]; },
-                             [&](int kk, int cc) { return Cs[kk * ldn + min(q * TS + tx * 4 + cc, d.n - 1)]; });
-        }
-        // state terms with Q_k = dH_{k+1}
-        __syncthreads();
-        load_tile(Cs, ldn, P.dstates + st_off(d, bb, k, hh), (size_t)d.n, hrows, d.p, d.n, d.n);
-        __syncthreads();
-        float dj[4];
+                    for (int c = 0; c < 4; ++c) {
+                        const int il = ty * 4 + r, jl = tx * 4 + c;
+                        const bool ok = (r0 + il >= j0 + jl) && il < rows_r && jl < rows_j;
+                        v[c] = ok ? dg[r][c] * __expf(cum_r[il] - cum_o[jl]) : 0.f;
+                        rowacc[r] = fmaf(v[c], s[r][c], rowacc[r]);
+                    }
+                    *reinterpret_cast<float4*>(M0 + sw(ty * 4 + r, tx, TS)) = make_float4(v[0], v[1], v[2], v[3]);
+                }
+                __syncthreads();
+                const int kend = jb == w.ib ? ty * 4 + 4 : TS;  // on the diagonal only the columns up to the row
 #pragma unroll
-        for (int r = 0; r < 4; ++r) dj[r] = (ty * 4 + r) < rows_j ? __expf(S - cum_j[ty * 4 + r]) : 0.f;
+                for (int q = 0; q < NTN; ++q)
+                    if (q * TS < d.n) mma_nn(acc[q], M0, ty * 4, TS, On, q * 16 + tx, ldn, kend);
+            }
+            // state term: dC_off = diag(e) dY_i H_k
 #pragma unroll
-        for (int q = 0; q < PT; ++q) {
-            float o[4][4];
-            zero(o);
-            tile_mma(o, d.n, [&](int r, int kk) { return Bs[(ty * 4 + r) * ldn + kk]; },
-                     [&](int kk, int cc) { return Cs[min(q * TS + tx * 4 + cc, hrows - 1) * ldn + kk]; });
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) accX[q][r][cc] += dj[r] * o[r][cc];
-        }
-#pragma unroll
-        for (int q = 0; q < NTN; ++q)
-            if (q * TS < d.n) {
+            for (int q = 0; q < NTN; ++q) {
+                if (q * TS >= d.n) break;
+                if (q || P.share_ws) {
+                    __syncthreads();
+                    load_tile(Ws, TS, H + q * TS, d.n, p4, d.p, min(TS, d.n - q * TS));
+                    __syncthreads();
+                }
                 float o[4][4];
                 zero(o);
-                tile_mma(o, d.p, [&](int r, int kk) { return Xs[(ty * 4 + r) * ldp + kk]; },
-                         [&](int kk, int cc) { return Cs[kk * ldn + min(q * TS + tx * 4 + cc, d.n - 1)]; });
+                mma_nn(o, Rp, ty * 4, ldp, Ws, tx, TS, p4);
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+                for (int r = 0; r < 4; ++r) {
+                    const float e = __expf(cum_r[ty * 4 + r]);
+                    const float4 cv = ld4(Rn, ty * 4 + r, q * 16 + tx, ldn);
+                    const float cc[4] = {cv.x, cv.y, cv.z, cv.w};
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) {
-                        int nn = q * TS + tx * 4 + cc;
-                        if (nn < d.n) {
-                            float v = dj[r] * o[r][cc];
-                            dBa[q][r][cc] += v;
-                            colacc[r] += v * Bs[(ty * 4 + r) * ldn + nn];
+                    for (int c = 0; c < 4; ++c)
+                        if (q * TS + tx * 4 + c < d.n) {
+                            const float v = e * o[r][c];
+                            acc[q][r][c] += v;
+                            rowacc[r] = fmaf(v, cc[c], rowacc[r]);
                         }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float v = row_reduce16(rowacc[r]);
+                const int il = ty * 4 + r;
+                if (tx == 0 && il < rows_r) P.g_row[((size_t)bb * d.h + hh) * d.T + t_r0 + il] = v;
+            }
+        }
+        store_bc<NTN, T>(P, w, t_r0, rows_r, acc, P.dC_part, (T*)P.dC);
+        return;
+    }
+
+    for (int hl = 0; hl < w.hps; ++hl) {
+        const int hh = w.h0 + hl;
+        const float* Q = P.dstates + st_off(d, bb, k, hh);
+        const float S = P.cum[cum_off(d, bb, hh, k) + d.l - 1];
+        float colacc[4] = {0.f, 0.f, 0.f, 0.f};
+        float a1[PT][4][4];
+#pragma unroll
+        for (int q = 0; q < PT; ++q) zero(a1[q]);
+        if (hl) __syncthreads();
+        load_scalars(P, bb, hh, k, r0, cum_r, dt_r);
+        if (!P.share_ws) load_tile(Ws, TS, Q, d.n, p4, d.p, min(TS, d.n));
+        __syncthreads();
+        load_tile(Rp, ldp, x + x_off(d, bb, t_r0, hh), xs, TS, rows_r, d.p, P.dt ? dt_r : nullptr);
+        for (int ib = w.ib; ib < P.lb; ++ib) {
+            const int i0 = ib * TS, t_i0 = k * d.l + i0;
+            const int rows_i = min(TS, d.l - i0);
+            if (ib > w.ib) __syncthreads();
+            if (hl == 0 || P.lb > 1) load_tile(On, ldn, Cp + bc_off(d, bb, t_i0, w.gg), bs, TS, rows_i, d.n);
+            load_tile(Op, ldp, dy + x_off(d, bb, t_i0, hh), xs, TS, rows_i, d.p);
+            load_scalars(P, bb, hh, k, i0, cum_o, nullptr);
+            __syncthreads();
+            if (hl == 0 || P.lb > 1) {  // transposed: rows j, columns i
+                zero(s);
+                mma_nt(s, Rn, ty * 4, ldn, 0, On, tx * 4, ldn, n4);
+            }
+            float dg[4][4];
+            zero(dg);
+            mma_nt(dg, Rp, ty * 4, ldp, 0, Op, tx * 4, ldp, p4);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                float gv[4], v[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int jl = ty * 4 + r, il = tx * 4 + c;
+                    const bool ok = (i0 + il >= r0 + jl) && il < rows_i && jl < rows_r;
+                    const float L = ok ? __expf(cum_o[il] - cum_r[jl]) : 0.f;
+                    v[c] = dg[r][c] * L;
+                    colacc[r] = fmaf(v[c], s[r][c], colacc[r]);
+                    gv[c] = s[r][c] * L;
+                }
+                *reinterpret_cast<float4*>(M0 + sw(ty * 4 + r, tx, TS)) = make_float4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<float4*>(M1 + sw(ty * 4 + r, tx, TS)) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < PT; ++q) mma_nn(a1[q], M1, ty * 4, TS, Op, q * 16 + tx, ldp, TS);
+#pragma unroll
+            for (int q = 0; q < NTN; ++q)
+                if (q * TS < d.n) mma_nn(acc[q], M0, ty * 4, TS, On, q * 16 + tx, ldn, TS);
+        }
+        // state terms with Q_k = dH_{k+1}
+        float dj[4], a2[PT][4][4];
+#pragma unroll
+        for (int q = 0; q < PT; ++q) zero(a2[q]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) dj[r] = (ty * 4 + r) < rows_r ? __expf(S - cum_r[ty * 4 + r]) : 0.f;
+#pragma unroll
+        for (int q = 0; q < NTN; ++q) {
+            if (q * TS >= d.n) break;
+            if (q || P.share_ws) {
+                __syncthreads();
+                load_tile(Ws, TS, Q + q * TS, d.n, p4, d.p, min(TS, d.n - q * TS));
+                __syncthreads();
+            }
+#pragma unroll
+            for (int pq = 0; pq < PT; ++pq) mma_nt(a2[pq], Rn, ty * 4, ldn, q * TS, Ws, pq * TS + tx * 4, TS, min(TS, n4 - q * TS));
+            float o[4][4];
+            zero(o);
+            mma_nn(o, Rp, ty * 4, ldp, Ws, tx, TS, p4);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float4 bv = ld4(Rn, ty * 4 + r, q * 16 + tx, ldn);
+                const float bc[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (q * TS + tx * 4 + c < d.n) {
+                        const float v = dj[r] * o[r][c];
+                        acc[q][r][c] += v;
+                        colacc[r] = fmaf(v, bc[c], colacc[r]);
                     }
             }
-        // per-head outputs
-        T* dxo = (T*)P.dx;
+        }
+        // per-head outputs; x and dy come back from memory as they were given (Rp holds x dt)
+        const size_t xo = x_off(d, bb, t_r0, hh);
+        T* dxo = (T*)P.dx + xo;
         const float Dh = P.D ? P.D[hh] : 0.f;
-        float ddt_acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int q = 0; q < PT; ++q)
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    int jl = ty * 4 + r, pp = q * TS + tx * 4 + cc;
-                    if (jl < rows_j && pp < d.p) {
-                        size_t o = x_off(d, bb, t_j0 + jl, hh) + pp;
-                        float dX = accX[q][r][cc];
-                        float xv = to_f(x[o]);
-                        ddt_acc[r] += dX * xv;
-                        float v = dX * dt_j[jl];
-                        if (P.D) v += Dh * to_f(dy[o]);
-                        dxo[o] = from_f<T>(v);
-                    }
-                }
+        const bool vec = wide(dxo, d.p, xs) && wide(x + xo, d.p, xs) && wide(dy + xo, d.p, xs);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            float gc = row_reduce16(colacc[r]);
-            float dd = row_reduce16(ddt_acc[r]);
-            int jl = ty * 4 + r;
-            if (tx == 0 && jl < rows_j) {
-                size_t o = ((size_t)bb * d.h + hh) * d.T + t_j0 + jl;
+            const int jl = ty * 4 + r;
+            float ddt = 0.f, yx = 0.f;
+            const float dtj = dt_r[jl];
+#pragma unroll
+            for (int q = 0; q < PT; ++q) {
+                const int pp = q * TS + tx * 4;
+                if (jl >= rows_r || pp >= d.p) continue;
+                const size_t o = (size_t)jl * xs + pp;
+                const float4 xv = load_upto4(x + xo + o, d.p - pp, vec);
+                const float xc[4] = {xv.x, xv.y, xv.z, xv.w};
+                float yc[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
+                if (P.D) {
+                    const float4 yv = load_upto4(dy + xo + o, d.p - pp, vec);
+                    yc[0] = yv.x; yc[1] = yv.y; yc[2] = yv.z; yc[3] = yv.w;
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    v[c] = 0.f;
+                    if (pp + c < d.p) {
+                        const float e = fmaf(dj[r], a2[q][r][c], a1[q][r][c]);
+                        ddt = fmaf(e, xc[c], ddt);
+                        yx = fmaf(yc[c], xc[c], yx);
+                        v[c] = fmaf(Dh, yc[c], e * dtj);
+                    }
+                }
+                store_upto4(dxo + o, v, d.p - pp, vec);
+            }
+            const float gc = row_reduce16(colacc[r]);
+            ddt = row_reduce16(ddt);
+            yx = row_reduce16(yx);
+            if (tx == 0 && jl < rows_r) {
+                const size_t o = ((size_t)bb * d.h + hh) * d.T + t_r0 + jl;
                 P.g_col[o] = gc;
-                P.ddtx[o] = dd;
+                P.ddtx[o] = ddt;
+                if (P.dyx) P.dyx[o] = yx;
             }
         }
     }
-    T* dBo = (T*)P.dB;
-#pragma unroll
-    for (int q = 0; q < NTN; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                int jl = ty * 4 + r, nn = q * TS + tx * 4 + cc;
-                if (jl < rows_j && nn < d.n) dBo[bc_off(d, bb, t_j0 + jl, gg) + nn] = from_f<T>(dBa[q][r][cc]);
-            }
+    store_bc<NTN, T>(P, w, t_r0, rows_r, acc, P.dB_part, (T*)P.dB);
+}
+__host__ inline size_t chunk_bwd_smem(const Dims& d, int pt, bool share_ws) {
+    return ((size_t)2 * TS * ld_of(d.n) + 2 * TS * ld_of(d.p) + 2 * TS * TS + (size_t)(share_ws ? 0 : pt) * TS * TS + 4 * TS) * 4;
 }
 
 __device__ __forceinline__ float block_sum(float v, float* red) {
@@ -664,44 +734,71 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Decay gradient.  One block per (head, batch): g = g_row - g_col (+ <dfinal, final> at T-1),
-// d a_t = reverse inclusive cumsum of g over the whole sequence (tiles of 256 with a carry,
-// warp-shuffle scan inside a tile).  Operator form writes da; Mamba-2 form writes
-// ddt = ddtx + da * A_head and the per-(batch, head) partials of dA_head and dD.
+// What the backward's blocks left in parts.  Blocks [0, b h): the decay gradient of one (head, batch),
+// g = g_row - g_col (+ <dfinal, final> at T-1), d a_t = reverse inclusive cumsum of g over the whole sequence (tiles of 256
+// with a carry, warp-shuffle scan inside a tile; the next tile's values are on their way meanwhile).  Operator form writes da;
+// Mamba-2 form writes ddt = ddtx + da * A_head and the per-(batch, head) partials of dA_head and dD.  The blocks behind them:
+// dB and dC summed over the splits of a group, four elements per thread, in a fixed order.
 // ------------------------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(NTHR) decay_grad_kernel(Params P) {
     __shared__ float red[NTHR / 32];
     __shared__ float wsum[NTHR / 32];
     const Dims& d = P.d;
-    const int hh = blockIdx.x, bb = blockIdx.y;
+    if ((int)blockIdx.x >= d.b * d.h) {
+        const size_t e = ((size_t)(blockIdx.x - d.b * d.h) * NTHR + threadIdx.x), total = (size_t)d.b * d.T * d.g * d.n;
+        if (e >= total) return;
+        const size_t o = (e / d.n) * P.splits * d.n + e % d.n;
+        float sb = 0.f, sc = 0.f;
+#pragma unroll 4
+        for (int s = 0; s < P.splits; ++s) {
+            sb += P.dB_part[o + (size_t)s * d.n];
+            sc += P.dC_part[o + (size_t)s * d.n];
+        }
+        ((T*)P.dB)[e] = from_f<T>(sb);
+        ((T*)P.dC)[e] = from_f<T>(sc);
+        return;
+    }
+    const int hh = blockIdx.x % d.h, bb = blockIdx.x / d.h;
     const size_t pn = (size_t)d.p * d.n;
     float gfin = 0.f;
-    if (P.dfinal && P.scan_len != 128) {
+    if (P.dfinal) {
         const float* a = P.dfinal + ((size_t)bb * d.h + hh) * pn;
         const float* f = P.final_state + ((size_t)bb * d.h + hh) * pn;
         float v = 0.f;
+#pragma unroll 8
         for (size_t e = threadIdx.x; e < pn; e += NTHR) v += a[e] * f[e];
         gfin = block_sum(v, red);
     }
     const size_t base = ((size_t)bb * d.h + hh) * d.T;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float carry = 0.f, dAh = 0.f;
+    float carry = 0.f, dAh = 0.f, yx = 0.f;
     const float Ah = P.dt ? P.A_head[hh] : 0.f;
+    const bool form2 = P.dt != nullptr;
+    float n_row = 0.f, n_col = 0.f, n_dx = 0.f, n_dt = 0.f, n_yx = 0.f;
+    auto fetch = [&](int t) {
+        if (t < 0) return;
+        n_row = P.g_row[base + t];
+        n_col = P.g_col[base + t];
+        if (form2) {
+            n_dx = P.ddtx[base + t];
+            n_dt = P.dt[((size_t)bb * d.T + t) * d.h + hh];
+            if (P.dyx) n_yx = P.dyx[base + t];
+        }
+    };
+    fetch(d.T - 1 - (int)threadIdx.x);
     for (int hi = d.T; hi > 0; hi -= NTHR) {
         // thread q handles t = hi-1-q, so the scan runs toward smaller t
         const int t = hi - 1 - (int)threadIdx.x;
+        const float dxv = n_dx, dtv = n_dt;
         float v = 0.f;
         if (t >= 0) {
-            v = P.g_row[base + t];
-            if (P.g_col) v -= P.g_col[base + t];
-            if (P.g_row2) v += P.g_row2[base + t];
-            if (P.gS && (t & 127) == 127) {
-                const float* q = P.gS + (base / 128 + t / 128) * 8;
-                v += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
-            }
-            if (t == d.T - 1 && P.scan_len != 128) v += gfin;
+            v = n_row;
+            v -= n_col;
+            if (t == d.T - 1) v += gfin;
+            yx += n_yx;
         }
+        fetch(t - NTHR);
         float incl = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -712,49 +809,40 @@ __global__ void __launch_bounds__(NTHR) decay_grad_kernel(Params P) {
         if (lane == 31) wsum[warp] = incl;
         __syncthreads();
         float pre = 0.f, tot = 0.f;
-        const int seg_first = P.scan_len == 128 ? (warp & ~3) : 0;  // 4 warps = one 128-tile
         for (int w = 0; w < NTHR / 32; ++w) {
-            if (w >= seg_first && w < warp) pre += wsum[w];
+            if (w < warp) pre += wsum[w];
             tot += wsum[w];
         }
         const float dA = carry + pre + incl;
-        if (P.scan_len != 128) carry += tot;
+        carry += tot;
         if (t >= 0) {
             const size_t o = ((size_t)bb * d.T + t) * d.h + hh;
-            if (P.dt) {
-                P.ddt[o] = P.ddtx[base + t] + (P.ddtx2 ? P.ddtx2[base + t] : 0.f) + dA * Ah;
-                dAh += dA * P.dt[o];
+            if (form2) {
+                P.ddt[o] = dxv + dA * Ah;
+                dAh += dA * dtv;
             } else if (P.da) {
                 P.da[o] = dA;
             }
         }
     }
-    if (P.dt) {
-        float s = block_sum(dAh, red);
+    if (form2) {
+        const float s = block_sum(dAh, red);
         if (threadIdx.x == 0) P.dAh_part[(size_t)bb * d.h + hh] = s;
-        if (P.D) {
-            const T* x = (const T*)P.x;
-            const T* dy = (const T*)P.dy;
-            float v = 0.f;
-            if (P.dyx) {
-                for (int t = threadIdx.x; t < d.T; t += NTHR) v += P.dyx[base + t] + (P.dyx2 ? P.dyx2[base + t] : 0.f);
-            } else {
-                for (size_t e = threadIdx.x; e < (size_t)d.T * d.p; e += NTHR) {
-                    int t = (int)(e / d.p), pp = (int)(e - (size_t)t * d.p);
-                    size_t o = x_off(d, bb, t, hh) + pp;
-                    v += to_f(x[o]) * to_f(dy[o]);
-                }
-            }
-            float sd = block_sum(v, red);
+        if (P.dyx) {
+            const float sd = block_sum(yx, red);
             if (threadIdx.x == 0) P.dD_part[(size_t)bb * d.h + hh] = sd;
         }
     }
 }
 
-// out[hh] = sum_b part[b,hh]   (fixed order: deterministic)
-__global__ void reduce_batch_kernel(const float* part, float* out, int b, int h) {
+// out[hh] = sum_b part[b,hh]   (fixed order: deterministic); dA_head, and dD by the blocks with blockIdx.y = 1
+__global__ void reduce_batch_kernel(const float* part, float* out, const float* part2, float* out2, int b, int h) {
     int hh = blockIdx.x * blockDim.x + threadIdx.x;
     if (hh >= h) return;
+    if (blockIdx.y) {
+        part = part2;
+        out = out2;
+    }
     float s = 0.f;
     for (int bb = 0; bb < b; ++bb) s += part[(size_t)bb * h + hh];
     out[hh] = s;
@@ -901,15 +989,6 @@ __global__ void __launch_bounds__(32) exchange_arrive_kernel(unsigned int* const
     }
     if (!ok) atomicExch(status, 3);
     __threadfence_system();
-}
-
-// Total log-decay of every (batch, head) sequence from the within-chunk cumulative sums: sum of the chunks' last entries.
-__global__ void logdecay_total_kernel(const float* __restrict__ cum, float* __restrict__ out, int bh, int c, int l) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= bh) return;
-    float s = 0.f;
-    for (int k = 0; k < c; ++k) s += cum[((size_t)m * c + k) * l + l - 1];
-    out[m] = s;
 }
 
 }  // namespace simt

@@ -184,14 +184,12 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
         SSD_TC_CHECK("cumsum_tile_fused");
     } else {
         if (!a->cumsum_is_input) {
-            simt::Params P{};
-            P.d = d; P.a = a->a; P.dt = a->a ? nullptr : a->dt; P.A_head = a->A_head; P.cum = a->a_cumsum;
-            P.a_is_bf16 = a->shape.a_dtype == SSD_B200_BF16;
-            size_t sm = (size_t)d.l * (d.h + 1) * 4;
+            const size_t sm = (size_t)d.l * (d.h + 1) * 4;
             if (sm > 48 * 1024 &&
-                cudaFuncSetAttribute(simt::chunk_cumsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+                cudaFuncSetAttribute(chunk_cumsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
                 SSD_TC_FAIL(SSD_B200_ECUDA, "chunk_cumsum: set shared memory size failed");
-            SSD_LAUNCH(prof::K_CUMSUM, st, simt::chunk_cumsum_kernel<<<dim3(d.c, d.b), simt::NTHR, sm, st>>>(P));
+            SSD_LAUNCH(prof::K_CUMSUM, st, chunk_cumsum_kernel<<<dim3(d.c, d.b), 256, sm, st>>>(
+                a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, d.T, d.h, d.l));
             SSD_TC_CHECK("chunk_cumsum");
         }
         if (!aux_valid)
@@ -230,7 +228,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     SSD_LAUNCH(prof::K_TC_FWD_ALT, st, (fwd_walk_kernel<true><<<dim3(d.h, d.b), kFwdThreads, kFwdSmem, st>>>(P)));
     SSD_TC_CHECK("tc_fwd_walk");
     if (a->logdecay_total) {
-        SSD_LAUNCH(prof::K_CUMSUM, st, simt::logdecay_total_kernel<<<(d.b * d.h + 127) / 128, 128, 0, st>>>(a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
+        SSD_LAUNCH(prof::K_CUMSUM, st, logdecay_total_kernel<<<(d.b * d.h + 127) / 128, 128, 0, st>>>(a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
         SSD_TC_CHECK("logdecay_total");
     }
     return 0;

@@ -188,6 +188,15 @@ def test_tensor_core_path_partial_tiles(pkg, cabi, oracle, b, T, h, p, n, g, l, 
     assert rel_err(y1, y0) < TOL_BF16 and rel_err(f1, f0) < TOL_BF16
 
 
+@pytest.mark.parametrize("b,T,h,p,n,g,l", [(2, 3200, 6, 8, 16, 1, 64), (1, 128, 4, 100, 200, 2, 128), (1, 192, 2, 64, 256, 1, 96),
+                                           (1, 64, 8, 65, 8, 2, 16), (2, 256, 12, 40, 65, 2, 128)])
+def test_fp32_head_splits_and_wide_states(pkg, cabi, oracle, b, T, h, p, n, g, l):
+    """The heads of a group on one block, on some and on one block each; states beyond 64 x 64, up to where the backward's
+    panels have to share memory; several 64-row blocks per chunk with a partial last one."""
+    cfg = replace(pkg.CONFIGS[0], batch=b, seqlen=T, nheads=h, headdim=p, d_state=n, ngroups=g, chunk=l)
+    check_mamba2(pkg, oracle, cfg, TOL_FP32, init=True, dfinal=True, seed=99)
+
+
 def test_unaligned_inputs(pkg, cabi, oracle):
     """Tensors that start between two 16-byte boundaries."""
     cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=192, nheads=2, ngroups=1, chunk=64)
