@@ -48,28 +48,37 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
     }
     __syncthreads();
     const int k0 = t0 / l, i0 = t0 - k0 * l;  // chunk of the tile's first position, position in it
+    const bool one = i0 + rows <= l;           // the whole tile lies in that chunk
+    float v[4][4], before[4];
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {  // every load of the warp's four heads is issued before any of them is used
+        const int hh = h0 + warp * 4 + i4;
+        const float* cu = cum + ((size_t)bb * h + hh) * T;  // (b,h,c,l): position t of the sequence at t
+        before[i4] = (hh < h && i0 > 0) ? cu[t0 - 1] : 0.f;
+#pragma unroll
+        for (int s4 = 0; s4 < 4; ++s4) v[i4][s4] = hh < h ? cu[t0 + min(s4 * 32 + lane, rows - 1)] : 0.f;
+    }
 #pragma unroll
     for (int i4 = 0; i4 < 4; ++i4) {
         const int hl = warp * 4 + i4, hh = h0 + hl;
         if (hh >= h) break;  // warp-uniform
-        const float* cu = cum + ((size_t)bb * h + hh) * T;  // (b,h,c,l): position t of the sequence at t
+        const float* cu = cum + ((size_t)bb * h + hh) * T;
         const size_t o = ((size_t)bb * h + hh) * Tp + t0;
-        const float before = i0 > 0 ? cu[t0 - 1] : 0.f;
 #pragma unroll
-        for (int s4 = 0; s4 < LT / 32; ++s4) {
-            const int tt = s4 * 32 + lane, t = t0 + min(tt, rows - 1);
-            const int k = t / l;
-            float v = cu[t];
-            if (k == k0) {
-                v -= before;
-            } else {
-                v += cu[(size_t)(k0 + 1) * l - 1] - before;
-                for (int kk = k0 + 1; kk < k; ++kk) v += cu[(size_t)(kk + 1) * l - 1];
+        for (int s4 = 0; s4 < 4; ++s4) {
+            const int tt = s4 * 32 + lane;
+            float w = v[i4][s4] - before[i4];
+            if (!one) {
+                const int k = (t0 + min(tt, rows - 1)) / l;
+                if (k != k0) {
+                    w = v[i4][s4] + (cu[(size_t)(k0 + 1) * l - 1] - before[i4]);
+                    for (int kk = k0 + 1; kk < k; ++kk) w += cu[(size_t)(kk + 1) * l - 1];
+                }
             }
-            v *= 1.4426950408889634f;  // stored in log2 units: every consumer uses exp2
-            tcum[o + tt] = v;
+            w *= 1.4426950408889634f;  // stored in log2 units: every consumer uses exp2
+            tcum[o + tt] = w;
             // decay across this 32-position block (lane 0 to lane 31)
-            const float span = __shfl_sync(0xffffffffu, v, 0) - __shfl_sync(0xffffffffu, v, 31);
+            const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);
             if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
             if (dtT) dtT[o + tt] = sdt[tt][hl];
             if (skipT) skipT[o + tt] = ssk[tt][hl];

@@ -4,7 +4,8 @@
 arity, cache keys and error behaviour of the reference operator
 (src/kernels/ssd_scan.py:427-465, :468-533, :539-583) so that the only
 production caller (src/mamba_base_engine.py:170-181) runs unchanged.  All
-arithmetic happens in the CUDA library behind include/ssd_b200.h; PyTorch here
+arithmetic happens in the CUDA library behind include/ssd_b200.h, reached through the
+native host path (csrc/ssd_torch.cpp: checks, allocations, autograd nodes); PyTorch
 only owns device memory and the stream.  There is no CPU or eager fallback:
 non-CUDA tensors raise, as in the reference (src/kernels/ssd_scan.py:247).
 
@@ -34,7 +35,7 @@ import os
 import torch
 from torch import Tensor
 
-from . import _cabi
+from . import _cabi, _native
 
 _EAGER_CACHE = False
 _FORCE_PATH = _cabi.PATH_AUTO
@@ -86,12 +87,6 @@ def _ptr(t: Tensor | None):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
-def _dense(t: Tensor) -> Tensor:
-    """Contiguous and, where the storage starts between two 16-byte boundaries, copied to a fresh one (TMA needs them)."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
-
-
 def _stream(dev) -> C.c_void_p:
     return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
 
@@ -109,26 +104,19 @@ def _workspace(lib, shape: _cabi.Shape, which: int, dev) -> Tensor:
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)
 
 
-def _check_inputs(x: Tensor, B: Tensor, Cm: Tensor) -> None:
-    assert x.is_cuda and B.is_cuda and Cm.is_cuda, "ssd_b200 runs on CUDA tensors only (no CPU fallback)"
-    if x.dim() != 4 or B.dim() != 4 or Cm.dim() != 4:
-        raise ValueError("expected x (b,T,h,p) and B, C (b,T,g,n)")
-    if B.shape != Cm.shape or B.shape[:2] != x.shape[:2]:
-        raise ValueError(f"shape mismatch: x {tuple(x.shape)}, B {tuple(B.shape)}, C {tuple(Cm.shape)}")
-    if not (x.dtype == B.dtype == Cm.dtype):
-        raise RuntimeError(f"expected x, B and C to have the same dtype, got {x.dtype}, {B.dtype}, {Cm.dtype}")
-
-
 class LazySSDCache(dict):
     """The operator's cache dict.  ``A_cumsum`` is always present; ``L`` and ``decay_chunk`` are built
     by a small kernel the first time they are read (the production caller only hands the dict back)."""
 
-    def __init__(self, a_cumsum: Tensor, shape: _cabi.Shape, out_dtype: torch.dtype):
+    def __init__(self, a_cumsum: Tensor, shape, out_dtype: torch.dtype):
+        """``shape``: the call's ``_cabi.Shape``, or a function that makes it when it is first needed."""
         super().__init__(A_cumsum=a_cumsum)
         self._shape = shape
         self._dtype = out_dtype
 
     def _materialize(self, key: str) -> Tensor:
+        if callable(self._shape):
+            self._shape = self._shape()
         s = self._shape
         cum = dict.__getitem__(self, "A_cumsum")
         c = s.seqlen // s.chunk
@@ -204,81 +192,41 @@ def _run_fwd(x, a, dt, A_head, D, B, Cm, chunk, init4, a_cumsum_in, want_states=
     return y, final, cum, shape, states
 
 
-def _run_bwd_operator(shape, x, A, B, Cm, cum, dY, states, init4=None, dfinal_state=None, cached=False):
-    """Backward launcher of the operator form (log-decay A given per position).  Returns
-    (dx, dA fp32 (b,T,h) or None when ``cached``, dB, dC, d initial state fp32 or None)."""
+def _run_bwd_scaled(shape, x, a, w, skip, B, Cm, cum, dY, states):
+    """Backward launcher of the scaled operator form (X = x * w, log-decay a, y += skip * x).  Returns
+    (dx, da, dw, dskip, dB, dC): dx complete, the three (b,T,h) gradients fp32."""
     lib = _cabi.load()
     dev = x.device
     b, T, h, p = x.shape
     with torch.cuda.device(dev):
-        dy = _dense(dY)
-        if dy.dtype != x.dtype:
-            dy = dy.to(x.dtype)
-        dfin = None if dfinal_state is None else dfinal_state.float().contiguous()
-        dx = torch.empty_like(x)
-        dB = torch.empty_like(B)
-        dC = torch.empty_like(Cm)
-        da = None if cached else torch.empty(b, T, h, dtype=torch.float32, device=dev)
-        dinit = torch.empty(b, h, p, B.shape[3], dtype=torch.float32, device=dev) if init4 is not None else None
+        dy = dY.contiguous().to(x.dtype)
+        dx, dB, dC = torch.empty_like(x), torch.empty_like(B), torch.empty_like(Cm)
+        da = torch.empty(b, T, h, dtype=torch.float32, device=dev)
+        dw, dskip = torch.empty_like(da), torch.empty_like(da)
         ws = _workspace(lib, shape, _cabi.PASS_BWD, dev)
-        args = _cabi.BwdArgs(shape, _ptr(x), _ptr(A), None, None, None, _ptr(B), _ptr(Cm), _ptr(init4), _ptr(cum),
-                             _ptr(dy), _ptr(dfin), _ptr(dx), _ptr(dB), _ptr(dC), _ptr(da), None, None, None, _ptr(dinit),
-                             1 if cached else 0, 0, _ptr(ws), ws.numel(), _ptr(states))
+        args = _cabi.BwdArgs(shape, _ptr(x), _ptr(a), _ptr(w), None, None, _ptr(B), _ptr(Cm), None, _ptr(cum), _ptr(dy),
+                             None, _ptr(dx), _ptr(dB), _ptr(dC), _ptr(da), _ptr(dw), None, None, None, 0, 0, _ptr(ws),
+                             ws.numel(), _ptr(states), _ptr(skip), _ptr(dskip))
         _cabi.check(lib.ssd_b200_bwd(C.byref(args), _stream(dev)))
         _status(lib, shape, ws, dev)
-    return dx, da, dB, dC, dinit
+    return dx, da, dw, dskip, dB, dC
 
 
-class FusedSSDScan(torch.autograd.Function):
+class FusedSSDScan:
     """Same call signature as the reference's FusedSSDScan (src/kernels/ssd_scan.py:441-465)."""
 
     @staticmethod
-    def forward(ctx, x: Tensor, A: Tensor, B: Tensor, C_: Tensor, chunk_size: int,
-                initial_states: Tensor | None, L_cache_in: Tensor | None,
-                decay_chunk_cache_in: Tensor | None, A_cumsum_cache_in: Tensor | None):
-        ctx.set_materialize_grads(False)  # an unused final state must not cost a zero tensor and a seeded reverse walk
-        _check_inputs(x, B, C_)
-        assert A.is_cuda
-        chunk = int(chunk_size)
-        xc, Ac, Bc, Cc = _dense(x), A.contiguous(), _dense(B), _dense(C_)
-        b, T, h, p = xc.shape
-        n = Bc.shape[3]
-        init4 = None
-        if initial_states is not None:
-            init4 = initial_states.reshape(b, h, p, n).float().contiguous()
-        cached = A_cumsum_cache_in is not None
-        y, final, cum, shape, states = _run_fwd(xc, Ac, None, None, None, Bc, Cc, chunk, init4,
-                                                A_cumsum_cache_in if cached else None,
-                                                want_states=any(ctx.needs_input_grad))
-        ctx.states = states
-        ctx.save_for_backward(xc, Ac, Bc, Cc, init4 if init4 is not None else torch.empty(0, device=x.device), cum)
-        ctx.chunk = chunk
-        ctx.has_init = initial_states is not None
-        ctx.init_shape = None if initial_states is None else tuple(initial_states.shape)
-        ctx.init_dtype = None if initial_states is None else initial_states.dtype
-        ctx.cached = cached
-        ctx.shape_struct = shape
-        ctx.mark_non_differentiable(cum)
+    def apply(x: Tensor, A: Tensor, B: Tensor, C_: Tensor, chunk_size: int, initial_states: Tensor | None,
+              L_cache_in: Tensor | None, decay_chunk_cache_in: Tensor | None, A_cumsum_cache_in: Tensor | None):
+        """(Y, final_state, L, decay_chunk, A_cumsum); L and decay_chunk are None unless the eager cache is on."""
+        y, final, cum = _native.load().operator_scan(x, A, B, C_, int(chunk_size), initial_states, A_cumsum_cache_in,
+                                                     _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
         L = dc = None
         if _EAGER_CACHE:
-            lazy = LazySSDCache(cum, shape, x.dtype)
+            lazy = LazySSDCache(cum, _make_shape(x, _cabi.F32, B, int(chunk_size)), x.dtype)
             L = L_cache_in.detach() if L_cache_in is not None else lazy["L"]
             dc = decay_chunk_cache_in.detach() if decay_chunk_cache_in is not None else lazy["decay_chunk"]
-            ctx.mark_non_differentiable(L, dc)
-        return y, final.to(x.dtype), L, dc, cum
-
-    @staticmethod
-    def backward(ctx, dY, dfinal_state, dL_unused, ddecay_chunk_unused, dA_cumsum_unused):
-        x, A, B, Cm, init4, cum = ctx.saved_tensors
-        if dY is None:
-            dY = torch.zeros_like(x)
-        dx, da, dB, dC, dinit = _run_bwd_operator(ctx.shape_struct, x, A, B, Cm, cum, dY, ctx.states,
-                                                  init4 if ctx.has_init else None, dfinal_state, ctx.cached)
-        dA = None if da is None else da.to(A.dtype)
-        dis = None
-        if ctx.has_init:
-            dis = dinit.reshape(ctx.init_shape).to(ctx.init_dtype)
-        return dx, dA, dB, dC, None, dis, None, None, None
+        return y, final, L, dc, cum
 
 
 def fused_ssd_scan(x: Tensor, A: Tensor, B: Tensor, C: Tensor, chunk_size: int,
@@ -299,68 +247,13 @@ def fused_ssd_scan(x: Tensor, A: Tensor, B: Tensor, C: Tensor, chunk_size: int,
         L_in = dc_in = ac_in = None
     Y, final_state, L_out, dc_out, ac_out = FusedSSDScan.apply(
         x, A, B, C, int(chunk_size), initial_states, L_in, dc_in, ac_in)
-    out_cache = LazySSDCache(ac_out, _make_shape(x, _cabi.F32, B, int(chunk_size)), x.dtype)
+    dims = (*x.shape, B.shape[3], B.shape[2], int(chunk_size))  # (not the tensors: the cache must not keep them alive)
+    code, path = _dt_code(x), _FORCE_PATH
+    out_cache = LazySSDCache(ac_out, lambda: _cabi.Shape(_cabi.ABI_VERSION, code, _cabi.F32, path, *dims), x.dtype)
     for k, v in (("L", L_out if L_out is not None else L_in), ("decay_chunk", dc_out if dc_out is not None else dc_in)):
         if v is not None:
             dict.__setitem__(out_cache, k, v)
     return Y, final_state, out_cache
-
-
-class _SSDMamba2(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, dt, A_head, B, C_, D, chunk_size, initial_states):
-        _check_inputs(x, B, C_)
-        ctx.set_materialize_grads(False)  # an unused final state must not cost a zero tensor and a seeded reverse walk
-        chunk = int(chunk_size)
-        xc, Bc, Cc = _dense(x), _dense(B), _dense(C_)
-        dtc = dt.float().contiguous()
-        Ah = A_head.float().contiguous()
-        Dc = None if D is None else D.float().contiguous()
-        b, T, h, p = xc.shape
-        n = Bc.shape[3]
-        init4 = None if initial_states is None else initial_states.reshape(b, h, p, n).float().contiguous()
-        y, final, cum, shape, states = _run_fwd(xc, None, dtc, Ah, Dc, Bc, Cc, chunk, init4, None,
-                                                want_states=any(ctx.needs_input_grad))
-        ctx.states = states
-        ctx.save_for_backward(xc, dtc, Ah, Bc, Cc, cum,
-                              Dc if Dc is not None else torch.empty(0, device=x.device),
-                              init4 if init4 is not None else torch.empty(0, device=x.device))
-        ctx.has_D = D is not None
-        ctx.has_init = initial_states is not None
-        ctx.init_shape = None if initial_states is None else tuple(initial_states.shape)
-        ctx.shape_struct = shape
-        ctx.in_dtypes = (dt.dtype, A_head.dtype, None if D is None else D.dtype)
-        return y, final
-
-    @staticmethod
-    def backward(ctx, dY, dfinal):
-        x, dt, Ah, B, Cm, cum, D, init4 = ctx.saved_tensors
-        if dY is None:
-            dY = torch.zeros_like(x)
-        lib = _cabi.load()
-        shape = ctx.shape_struct
-        dev = x.device
-        b, T, h, p = x.shape
-        with torch.cuda.device(dev):
-            dy = _dense(dY).to(x.dtype)
-            dfin = None if dfinal is None else dfinal.float().contiguous()
-            dx = torch.empty_like(x)
-            dB = torch.empty_like(B)
-            dC = torch.empty_like(Cm)
-            ddt = torch.empty(b, T, h, dtype=torch.float32, device=dev)
-            dAh = torch.empty(h, dtype=torch.float32, device=dev)
-            dD = torch.empty(h, dtype=torch.float32, device=dev) if ctx.has_D else None
-            dinit = torch.empty(b, h, p, B.shape[3], dtype=torch.float32, device=dev) if ctx.has_init else None
-            ws = _workspace(lib, shape, _cabi.PASS_BWD, dev)
-            args = _cabi.BwdArgs(shape, _ptr(x), None, _ptr(dt), _ptr(Ah), _ptr(D) if ctx.has_D else None, _ptr(B),
-                                 _ptr(Cm), _ptr(init4) if ctx.has_init else None, _ptr(cum), _ptr(dy), _ptr(dfin),
-                                 _ptr(dx), _ptr(dB), _ptr(dC), None, _ptr(ddt), _ptr(dAh), _ptr(dD), _ptr(dinit),
-                                 0, 0, _ptr(ws), ws.numel(), _ptr(ctx.states))
-            _cabi.check(lib.ssd_b200_bwd(C.byref(args), _stream(dev)))
-            _status(lib, shape, ws, dev)
-        dtd, ahd, dd = ctx.in_dtypes
-        return (dx, ddt.to(dtd), dAh.to(ahd), dB, dC, None if dD is None else dD.to(dd), None,
-                None if dinit is None else dinit.reshape(ctx.init_shape))
 
 
 def ssd_mamba2(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: Tensor | None, chunk_size: int,
@@ -371,129 +264,7 @@ def ssd_mamba2(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: T
     x (b,T,h,p) bf16/fp32; dt (b,T,h); A_head (h); B, C (b,T,g,n); D (h) or None;
     initial_states (b,h,p,n) or (b,1,h,p,n).  Returns (Y, final_state fp32 (b,h,p,n)).
     """
-    return _SSDMamba2.apply(x, dt, A_head, B, C, D, int(chunk_size), initial_states)
-
-
-def _run_bwd_scaled(shape, x, a, w, skip, B, Cm, cum, dY, states):
-    """Backward launcher of the scaled operator form (X = x * w, log-decay a, y += skip * x).  Returns
-    (dx, da, dw, dskip, dB, dC): dx complete, the three (b,T,h) gradients fp32."""
-    lib = _cabi.load()
-    dev = x.device
-    b, T, h, p = x.shape
-    with torch.cuda.device(dev):
-        dy = _dense(dY).to(x.dtype)
-        dx, dB, dC = torch.empty_like(x), torch.empty_like(B), torch.empty_like(Cm)
-        da = torch.empty(b, T, h, dtype=torch.float32, device=dev)
-        dw, dskip = torch.empty_like(da), torch.empty_like(da)
-        ws = _workspace(lib, shape, _cabi.PASS_BWD, dev)
-        args = _cabi.BwdArgs(shape, _ptr(x), _ptr(a), _ptr(w), None, None, _ptr(B), _ptr(Cm), None, _ptr(cum), _ptr(dy),
-                             None, _ptr(dx), _ptr(dB), _ptr(dC), _ptr(da), _ptr(dw), None, None, None, 0, 0, _ptr(ws),
-                             ws.numel(), _ptr(states), _ptr(skip), _ptr(dskip))
-        _cabi.check(lib.ssd_b200_bwd(C.byref(args), _stream(dev)))
-        _status(lib, shape, ws, dev)
-    return dx, da, dw, dskip, dB, dC
-
-
-def _mamba2_backward(ctx_shape, x, dt, Ah, B, Cm, cum, D, init4, states, dY, dfinal, has_D, has_init):
-    """Backward launcher of the Mamba-2 form; returns (dx, ddt, dA_head, dB, dC, dD or None, dinit or None), fp32
-    for the small ones."""
-    lib = _cabi.load()
-    dev = x.device
-    b, T, h, p = x.shape
-    with torch.cuda.device(dev):
-        dy = _dense(dY).to(x.dtype)
-        dfin = None if dfinal is None else dfinal.float().contiguous()
-        dx = torch.empty_like(x)
-        dB = torch.empty_like(B)
-        dC = torch.empty_like(Cm)
-        ddt = torch.empty(b, T, h, dtype=torch.float32, device=dev)
-        dAh = torch.empty(h, dtype=torch.float32, device=dev)
-        dD = torch.empty(h, dtype=torch.float32, device=dev) if has_D else None
-        dinit = torch.empty(b, h, p, B.shape[3], dtype=torch.float32, device=dev) if has_init else None
-        ws = _workspace(lib, ctx_shape, _cabi.PASS_BWD, dev)
-        args = _cabi.BwdArgs(ctx_shape, _ptr(x), None, _ptr(dt), _ptr(Ah), _ptr(D) if has_D else None, _ptr(B),
-                             _ptr(Cm), _ptr(init4) if has_init else None, _ptr(cum), _ptr(dy), _ptr(dfin),
-                             _ptr(dx), _ptr(dB), _ptr(dC), None, _ptr(ddt), _ptr(dAh), _ptr(dD), _ptr(dinit),
-                             0, 0, _ptr(ws), ws.numel(), _ptr(states))
-        _cabi.check(lib.ssd_b200_bwd(C.byref(args), _stream(dev)))
-        _status(lib, ctx_shape, ws, dev)
-    return dx, ddt, dAh, dB, dC, dD, dinit
-
-
-class _SSDMamba2Gated(torch.autograd.Function):
-    """The scan followed by the block's output stage, out = rmsnorm(y over all heads) * silu(z)
-    (src/mamba_base_engine.py:189-191), as one operator.  The forward walk leaves the per-half-row sums of y^2
-    behind, so the norm reads y once; y itself is kept (the norm's backward needs it)."""
-
-    @staticmethod
-    def forward(ctx, x, dt, A_head, B, C_, D, z, norm_weight, eps, chunk_size, initial_states):
-        _check_inputs(x, B, C_)
-        ctx.set_materialize_grads(False)
-        lib = _cabi.load()
-        chunk = int(chunk_size)
-        xc, Bc, Cc = _dense(x), _dense(B), _dense(C_)
-        dtc = dt.float().contiguous()
-        Ah = A_head.float().contiguous()
-        Dc = None if D is None else D.float().contiguous()
-        b, T, h, p = xc.shape
-        n = Bc.shape[3]
-        dev = x.device
-        assert z.is_cuda and z.shape[:2] == x.shape[:2] and z.numel() == x.numel(), \
-            f"the gate must have the size of y: {tuple(z.shape)} vs {tuple(x.shape)}"
-        init4 = None if initial_states is None else initial_states.reshape(b, h, p, n).float().contiguous()
-        shape = _make_shape(xc, _cabi.F32, Bc, chunk)
-        path = lib.ssd_b200_resolve_path(C.byref(shape))
-        _cabi.check(path)
-        with torch.cuda.device(dev):
-            ysq = None
-            if path == _cabi.PATH_TC and T % 128 == 0:
-                ysq = torch.empty(b * (T // 128) * h * 2 * 128, dtype=torch.float32, device=dev)
-            y, final, cum, shape, states = _run_fwd(xc, None, dtc, Ah, Dc, Bc, Cc, chunk, init4, None,
-                                                    want_states=any(ctx.needs_input_grad), ysq=ysq)
-            zc = z.contiguous().to(xc.dtype).reshape(b * T, h * p)
-            w = norm_weight.contiguous().float()
-            out = torch.empty_like(y)
-            rstd = torch.empty(b * T, dtype=torch.float32, device=dev)
-            if ysq is not None:
-                _cabi.check(lib.ssd_b200_rmsnorm_fwd_presummed(_dt_code(y), b * T, h * p, float(eps), _ptr(y), _ptr(w),
-                                                               _ptr(zc), _ptr(ysq), h, _ptr(out), _ptr(rstd), _stream(dev)))
-            else:
-                _cabi.check(lib.ssd_b200_rmsnorm_fwd(_dt_code(y), b * T, h * p, float(eps), _ptr(y), _ptr(w), _ptr(zc),
-                                                     _ptr(out), _ptr(rstd), _stream(dev)))
-        ctx.states = states
-        ctx.save_for_backward(xc, dtc, Ah, Bc, Cc, cum,
-                              Dc if Dc is not None else torch.empty(0, device=dev),
-                              init4 if init4 is not None else torch.empty(0, device=dev), y, zc, w, rstd)
-        ctx.has_D = D is not None
-        ctx.has_init = initial_states is not None
-        ctx.init_shape = None if initial_states is None else tuple(initial_states.shape)
-        ctx.shape_struct = shape
-        ctx.in_dtypes = (dt.dtype, A_head.dtype, None if D is None else D.dtype, z.dtype, norm_weight.dtype)
-        ctx.z_shape = tuple(z.shape)
-        return out, final
-
-    @staticmethod
-    def backward(ctx, dout, dfinal):
-        x, dt, Ah, B, Cm, cum, D, init4, y, zc, w, rstd = ctx.saved_tensors
-        if dout is None:
-            dout = torch.zeros_like(x)
-        lib = _cabi.load()
-        dev = x.device
-        b, T, h, p = x.shape
-        rows, Dn = b * T, h * p
-        with torch.cuda.device(dev):
-            do = dout.contiguous().to(x.dtype).reshape(rows, Dn)
-            dy = torch.empty_like(y)
-            dz = torch.empty_like(zc)
-            dw = torch.empty(Dn, dtype=torch.float32, device=dev)
-            ws = torch.empty(int(lib.ssd_b200_rmsnorm_ws_floats(rows, Dn)), dtype=torch.float32, device=dev)
-            _cabi.check(lib.ssd_b200_rmsnorm_bwd(_dt_code(y), rows, Dn, _ptr(y), _ptr(w), _ptr(zc), _ptr(do), _ptr(rstd),
-                                                 _ptr(dy), _ptr(dz), _ptr(dw), _ptr(ws), _stream(dev)))
-        dx, ddt, dAh, dB, dC, dD, dinit = _mamba2_backward(ctx.shape_struct, x, dt, Ah, B, Cm, cum, D, init4, ctx.states,
-                                                           dy, dfinal, ctx.has_D, ctx.has_init)
-        dtd, ahd, dd, zd, wd = ctx.in_dtypes
-        return (dx, ddt.to(dtd), dAh.to(ahd), dB, dC, None if dD is None else dD.to(dd), dz.reshape(ctx.z_shape).to(zd),
-                dw.to(wd), None, None, None if dinit is None else dinit.reshape(ctx.init_shape))
+    return _native.load().mamba2(x, dt, A_head, B, C, D, int(chunk_size), initial_states, _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
 
 
 def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: Tensor | None, z: Tensor,
@@ -505,7 +276,8 @@ def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor
     Returns (out in x's shape, final_state fp32 (b,h,p,n)).  Gradients: x, dt, A_head, B, C, D, z, norm_weight,
     initial_states.
     """
-    return _SSDMamba2Gated.apply(x, dt, A_head, B, C, D, z, norm_weight, float(eps), int(chunk_size), initial_states)
+    return _native.load().mamba2_gated(x, dt, A_head, B, C, D, z, norm_weight, float(eps), int(chunk_size), initial_states,
+                                       _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
 
 
 def resolved_path_name(cfg) -> str:
