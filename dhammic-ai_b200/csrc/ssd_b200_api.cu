@@ -483,6 +483,33 @@ int trapezoid_impl(bool backward, size_t M, int H, const void* dt_raw, const voi
     return 0;
 }
 
+// Blocks of the norm kernels that keep a row in registers: enough of them to fill the chip, each walking many rows.
+constexpr int kNormFwdBlocks = 4 * 148, kNormBwdBlocks = 4 * 148;  // (of up to 256 threads; fewer of the larger ones)
+unsigned norm_blocks(size_t M, int rows_per_block, int most) {
+    return (unsigned)std::min<size_t>(most, (M + rows_per_block - 1) / rows_per_block);
+}
+
+// A warp per row up to 4 vectors a lane (512 fp32, 1024 bf16 columns), else the block; as few vectors a thread as the row needs.
+template <class T, bool GATED>
+void launch_norm_rows(bool backward, size_t M, int D, float eps, const T* x, const float* w, const T* z, const T* dout, T* out, T* dz, float* rstd,
+                      float* part, unsigned nb, cudaStream_t st) {
+    using namespace ssd::ew;
+    const int vecs = D / VecOf<T>::N;
+#define SSD_NORM(TPR, NV)                                                                                                                    \
+    do {                                                                                                                                     \
+        const unsigned blocks = nb;                                                                        \
+        if (backward) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<blocks, TPR < 256 ? 256 : TPR, 0, st>>>(x, w, z, dout, rstd, out, dz, part, M, D))); \
+        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_fwd_kernel<T, TPR, NV, GATED><<<blocks, TPR < 256 ? 256 : TPR, 0, st>>>(x, w, z, out, rstd, M, D, eps))); \
+    } while (0)
+    if (vecs <= 32) SSD_NORM(32, 1);
+    else if (vecs <= 64) SSD_NORM(32, 2);
+    else if (vecs <= 128) SSD_NORM(32, 4);
+    else if (vecs <= 256) SSD_NORM(256, 1);
+    else if (vecs <= 512) SSD_NORM(512, 1);
+    else SSD_NORM(1024, 1);
+#undef SSD_NORM
+}
+
 template <class T>
 int rmsnorm_impl(bool backward, size_t M, int D, float eps, const void* x, const float* w, const void* z, const void* dout,
                  void* out, void* dz, float* rstd, float* dw, float* part_ws, cudaStream_t st, const float* ysq = nullptr,
@@ -491,7 +518,13 @@ int rmsnorm_impl(bool backward, size_t M, int D, float eps, const void* x, const
     constexpr int V = VecOf<T>::N;
     const bool vec = D % V == 0;
     const unsigned blocks = (unsigned)((M + 7) / 8);
-    if (!backward) {
+    if (rms_fits<T>(D) && !ysq && !any_unaligned({x, z, dout, out, dz})) {
+        const int vecs = D / V, most = backward ? kNormBwdBlocks : kNormFwdBlocks;
+        const unsigned nb = norm_blocks(M, vecs <= 128 ? 8 : 1, vecs <= 256 ? most : vecs <= 512 ? most / 2 : most / 4);
+        if (z) launch_norm_rows<T, true>(backward, M, D, eps, (const T*)x, w, (const T*)z, (const T*)dout, (T*)out, (T*)dz, rstd, part_ws, nb, st);
+        else launch_norm_rows<T, false>(backward, M, D, eps, (const T*)x, w, nullptr, (const T*)dout, (T*)out, nullptr, rstd, part_ws, nb, st);
+        if (backward) SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_partial_rows_kernel<<<(D + 31) / 32, 256, 0, st>>>(part_ws, dw, (int)nb, D));
+    } else if (!backward) {
         if (vec) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_fwd_kernel<T, V><<<blocks, 256, 0, st>>>((const T*)x, w, (const T*)z, (T*)out, rstd, M, D, eps, ysq, ysq_heads)));
         else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_fwd_kernel<T, 1><<<blocks, 256, 0, st>>>((const T*)x, w, (const T*)z, (T*)out, rstd, M, D, eps, ysq, ysq_heads)));
     } else {
@@ -500,7 +533,7 @@ int rmsnorm_impl(bool backward, size_t M, int D, float eps, const void* x, const
         const unsigned chunks = (unsigned)((M + RMS_ROWS - 1) / RMS_ROWS);
         if (vec) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_dw_kernel<T, V><<<dim3((D + 32 * V - 1) / (32 * V), chunks), 256, 0, st>>>((const T*)x, (const T*)z, (const T*)dout, rstd, part_ws, M, D)));
         else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_dw_kernel<T, 1><<<dim3((D + 31) / 32, chunks), 256, 0, st>>>((const T*)x, (const T*)z, (const T*)dout, rstd, part_ws, M, D)));
-        SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::tc::reduce_rows_kernel<<<D, 256, 0, st>>>(part_ws, dw, (int)chunks, D));
+        SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_partial_rows_kernel<<<(D + 31) / 32, 256, 0, st>>>(part_ws, dw, (int)chunks, D));
     }
     CUDA_LAUNCH_CHECK("rmsnorm");
     return 0;
@@ -829,7 +862,8 @@ int ssd_b200_trapezoid_bwd(int32_t dtype, int64_t rows, int64_t H, const void* d
 
 size_t ssd_b200_rmsnorm_ws_floats(int64_t rows, int64_t D) {
     if (rows <= 0 || D <= 0) return 0;
-    return (size_t)((rows + ssd::ew::RMS_ROWS - 1) / ssd::ew::RMS_ROWS) * (size_t)D;
+    const int64_t chunks = (rows + ssd::ew::RMS_ROWS - 1) / ssd::ew::RMS_ROWS;
+    return (size_t)std::max<int64_t>(chunks, std::min<int64_t>(rows, kNormBwdBlocks)) * (size_t)D;
 }
 
 int ssd_b200_rmsnorm_fwd(int32_t dtype, int64_t rows, int64_t D, float eps, const void* x, const float* weight,

@@ -215,9 +215,14 @@ __global__ void __launch_bounds__(256) trapezoid_bwd_kernel(const T* __restrict_
 // ------------------------------------------------------------------------------------------
 // RMS norm over the last dimension, optionally gated:  out = x * rsqrt(mean(x^2) + eps) * w  [* silu(z)]
 // (src/kernels/rmsnorm.py:75-150; the block's closing `norm(y) * silu(z)`, src/mamba_base_engine.py:189-191).
-// One warp per row, two passes over the row (the second one hits L1 / L2); V elements per lane and step.
 //   backward:  dn = do [* silu(z)],  s = sum_j w_j x_j dn_j,  dx_i = r (w_i dn_i - x_i r^2 s / D),
-//              dz_j = do_j n_j silu'(z_j),  dw_j = sum_rows x_j r dn_j  (a separate column reduction).
+//              dz_j = do_j n_j silu'(z_j),  dw_j = sum_rows x_j r dn_j
+//
+// Two sets of kernels.  Where a row fits the registers of the threads that share it (rms_fits), every tensor is read once: a
+// row's vectors stay in registers between the statistic and the use, the next row's are on their way meanwhile, and the
+// backward keeps its columns' dw over all the rows of a block (one partial row per block, so dw costs no pass over x,
+// z and do).  HBM-bound: forward + backward of (16384, 4096) bf16 gated, 8 passes over 134 MB: 358 us with a second pass in
+// each direction and a third kernel for dw, 214 us now.  Other rows: one warp per row, two passes.
 // ------------------------------------------------------------------------------------------
 // V consecutive weights (16-byte vector loads when V is a multiple of 4: the column index then is too)
 template <int V>
@@ -237,6 +242,193 @@ __device__ __forceinline__ float silu_f(float z) { return z * sigmoid_f(z); }
 __device__ __forceinline__ float silu_grad_f(float z) {
     const float sg = sigmoid_f(z);
     return sg * (1.f + z * (1.f - sg));
+}
+
+// A row of D elements over TPR threads (a warp, or the block), NV 16-byte vectors each.  A block's row has one vector per thread: the
+// fewer registers a thread needs, the more warps hide the latency of the loads and of the gate's exponentials (with 256
+// threads and two vectors each the backward took 143 us at (16384, 4096), 133 us with 512 threads).
+template <class T>
+__host__ __device__ inline bool rms_fits(int D) {
+    return D % VecOf<T>::N == 0 && D <= 256 * 4 * VecOf<T>::N;
+}
+template <class T, int NV>
+struct RowVecs {
+    uint4 v[NV];
+    __device__ __forceinline__ void load(const T* row, int first, int step, int D) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = (first + i * step) * VecOf<T>::N;
+            v[i] = c < D ? *reinterpret_cast<const uint4*>(row + c) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    __device__ __forceinline__ float at(int i, int q) const { return to_f(reinterpret_cast<const T*>(&v[i])[q]); }
+};
+// Sum over the TPR threads of a row; `red` holds one float per warp and is used alternately (parity) by successive rows.
+template <int TPR>
+__device__ __forceinline__ float rms_sum(float v, float* red) {
+#pragma unroll
+    for (int of = 16; of > 0; of >>= 1) v += __shfl_xor_sync(0xffffffffu, v, of);
+    if constexpr (TPR > 32) {
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        const int lane = threadIdx.x & 31;  // every warp adds the warps' sums itself
+        v = lane < TPR / 32 ? red[lane] : 0.f;
+#pragma unroll
+        for (int of = TPR / 64; of > 0; of >>= 1) v += __shfl_xor_sync(0xffffffffu, v, of);
+        v = __shfl_sync(0xffffffffu, v, 0);
+    }
+    return v;
+}
+
+template <class T, int TPR, int NV, bool GATED>
+__global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR : 1) rmsnorm_rows_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const T* __restrict__ z,
+                                                               T* __restrict__ out, float* __restrict__ rstd, size_t M, int D, float eps) {
+    constexpr int V = VecOf<T>::N, RPB = TPR < 256 ? 256 / TPR : 1;
+    __shared__ float red[2][32];
+    const int sub = threadIdx.x % TPR;
+    float wv[NV * V];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = (sub + i * TPR) * V;
+#pragma unroll
+        for (int q = 0; q < V; ++q) wv[i * V + q] = c < D ? w[c + q] : 0.f;
+    }
+    const size_t step = (size_t)gridDim.x * RPB;
+    size_t row = (size_t)blockIdx.x * RPB + threadIdx.x / TPR;
+    RowVecs<T, NV> xn, zn;
+    if (row < M) {
+        xn.load(x + row * D, sub, TPR, D);
+        if (GATED) zn.load(z + row * D, sub, TPR, D);
+    }
+    for (int par = 0; row < M; row += step, par ^= 1) {  // (TPR = 256: uniform over the block; TPR = 32: over the warp)
+        const RowVecs<T, NV> xc = xn, zc = zn;
+        if (row + step < M) {
+            xn.load(x + (row + step) * D, sub, TPR, D);
+            if (GATED) zn.load(z + (row + step) * D, sub, TPR, D);
+        }
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int q = 0; q < V; ++q) ss = fmaf(xc.at(i, q), xc.at(i, q), ss);
+        ss = rms_sum<TPR>(ss, red[par]);
+        const float r = rsqrtf(ss / (float)D + eps);
+        if (sub == 0) rstd[row] = r;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = (sub + i * TPR) * V;
+            if (c >= D) continue;
+            float o[V];
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+                o[q] = xc.at(i, q) * r * wv[i * V + q];
+                if (GATED) o[q] *= silu_f(zc.at(i, q));
+            }
+            store_elems1<T, V>(out + row * D + c, o);
+        }
+    }
+}
+
+template <class T, int TPR, int NV, bool GATED>
+__global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR : 1) rmsnorm_rows_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const T* __restrict__ z,
+                                                               const T* __restrict__ dout, const float* __restrict__ rstd, T* __restrict__ dx,
+                                                               T* __restrict__ dz, float* __restrict__ part, size_t M, int D) {
+    constexpr int V = VecOf<T>::N, RPB = TPR < 256 ? 256 / TPR : 1;
+    __shared__ float red[2][32];
+    const int sub = threadIdx.x % TPR;
+    __shared__ __align__(16) float sw[TPR * NV * V];  // (the weights in registers would make the kernel spill)
+    for (int c = threadIdx.x; c < TPR * NV * V; c += TPR < 256 ? 256 : TPR) sw[c] = c < D ? w[c] : 0.f;
+    __syncthreads();
+    float dw[NV * V];
+#pragma unroll
+    for (int i = 0; i < NV * V; ++i) dw[i] = 0.f;
+    const size_t step = (size_t)gridDim.x * RPB;
+    size_t row = (size_t)blockIdx.x * RPB + threadIdx.x / TPR;
+    RowVecs<T, NV> xn, zn, gn;
+    float rn = 0.f;
+    auto fetch = [&](size_t r) {
+        if (r >= M) return;
+        xn.load(x + r * D, sub, TPR, D);
+        gn.load(dout + r * D, sub, TPR, D);
+        if (GATED) zn.load(z + r * D, sub, TPR, D);
+        rn = rstd[r];
+    };
+    fetch(row);
+    for (int par = 0; row < M; row += step, par ^= 1) {
+        const RowVecs<T, NV> xc = xn, zc = zn, gc = gn;
+        const float r = rn;
+        fetch(row + step);
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            float wv[V];
+            load_w<V>(sw + (sub + i * TPR) * V, wv);
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+                float dn = gc.at(i, q);
+                if (GATED) dn *= silu_f(zc.at(i, q));
+                const float t = xc.at(i, q) * dn;
+                s = fmaf(wv[q], t, s);
+                dw[i * V + q] = fmaf(r, t, dw[i * V + q]);
+            }
+        }
+        s = rms_sum<TPR>(s, red[par]);
+        const float k = r * r * s / (float)D;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = (sub + i * TPR) * V;
+            if (c >= D) continue;
+            float o[V], oz[V], wv[V];
+            load_w<V>(sw + c, wv);
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+                const float xv = xc.at(i, q), gv = gc.at(i, q), wq = wv[q];
+                float dn = gv;
+                if (GATED) {
+                    const float zv = zc.at(i, q), si = sigmoid_f(zv);
+                    dn *= zv * si;
+                    oz[q] = gv * (xv * r * wq) * (si * (1.f + zv * (1.f - si)));
+                }
+                o[q] = r * (wq * dn - xv * k);
+            }
+            store_elems1<T, V>(dx + row * D + c, o);
+            if (GATED) store_elems1<T, V>(dz + row * D + c, oz);
+        }
+    }
+    if constexpr (RPB == 1) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = (sub + i * TPR) * V;
+            if (c < D) m3::store_f32<V>(part + (size_t)blockIdx.x * D + c, *reinterpret_cast<const float(*)[V]>(&dw[i * V]));
+        }
+    } else {  // the rows of the block's warps, added in a fixed order
+        __shared__ float sdw[RPB][TPR * NV * V];
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int q = 0; q < V; ++q) sdw[threadIdx.x / TPR][(sub + i * TPR) * V + q] = dw[i * V + q];
+        __syncthreads();
+        for (int c = threadIdx.x; c < D; c += 256) {
+            float t = 0.f;
+#pragma unroll
+            for (int g = 0; g < RPB; ++g) t += sdw[g][c];
+            part[(size_t)blockIdx.x * D + c] = t;
+        }
+    }
+}
+
+// out[c] = sum of `rows` partial rows; block = 32 columns x 8 row lanes, a fixed order of additions
+__global__ void __launch_bounds__(256) reduce_partial_rows_kernel(const float* __restrict__ part, float* __restrict__ out, int rows, int D) {
+    __shared__ float red[8][33];
+    const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5, c = blockIdx.x * 32 + cl;
+    float s = 0.f;
+    if (c < D) {
+#pragma unroll 8
+        for (int r = rl; r < rows; r += 8) s += part[(size_t)r * D + c];
+    }
+    red[rl][cl] = s;
+    __syncthreads();
+    if (rl == 0 && c < D) out[c] = ((red[0][cl] + red[1][cl]) + (red[2][cl] + red[3][cl])) + ((red[4][cl] + red[5][cl]) + (red[6][cl] + red[7][cl]));
 }
 
 template <class T, int V>

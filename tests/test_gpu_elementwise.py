@@ -168,7 +168,8 @@ def test_rmsnorm_backward_fp32(pkg, cabi, shape):
 
 
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 5e-2)])
-@pytest.mark.parametrize("shape", [(2, 128, 4096), (2, 64, 256), (1, 33, 96)])
+@pytest.mark.parametrize("shape", [(2, 128, 4096), (2, 64, 256), (1, 33, 96), (1, 1, 8), (3, 401, 1024), (1, 601, 1032), (1, 5, 2056),
+                                   (1, 700, 8192), (1, 9, 8200)])
 def test_gate_norm_matches_block_epilogue(pkg, cabi, shape, dtype, tol):
     """norm(y) * silu(z) as the block composes it (src/mamba_base_engine.py:189-191), forward and gradients."""
     torch.manual_seed(5)
