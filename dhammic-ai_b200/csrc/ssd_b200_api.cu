@@ -687,7 +687,12 @@ int ssd_b200_fwd_static_scratch(const ssd_b200_fwd_args* a, void* stream) {
     if (int rc = check_shape(&a->shape)) return rc;
     int path = resolve_path(a->shape);
     if (path < 0) return path;
-    const size_t need = ssd_b200_workspace_bytes(&a->shape, SSD_B200_PASS_FWD);
+    size_t need = ssd_b200_workspace_bytes(&a->shape, SSD_B200_PASS_FWD);
+    if (path == SSD_B200_PATH_TC) {  // a tensor-core walk runs in one piece where the room for more is missing
+        const ssd::Dims d = dims_of(a->shape);
+        need = ssd::tc::ws_layout(d, SSD_B200_PASS_FWD).base;
+        if (simt_takes_unaligned(a->shape, path)) need = std::max(need, simt_ws(d, SSD_B200_PASS_FWD).total);
+    }
     if (need > (size_t)SSD_B200_STATIC_SCRATCH_BYTES)
         return fail(SSD_B200_EWORKSPACE,
                     "this shape needs %zu bytes of scratch but the built-in array holds %u; use ssd_b200_fwd with a "

@@ -241,6 +241,12 @@ struct WalkParams {
     int* status;
     int Tp, h, hpg, nt;  // Tp = nt * 128: stride of the per-position arrays
     int p, n;            // headdim and d_state of the tensors (at most 64 and 128)
+    // Pieces of the sequence (blockIdx.z; see Pieces): tiles of a piece, and what the parts of each piece but the last
+    // (reverse walk: but the first) add to the state behind them (to the gradient of the state before them), (piece, part,
+    // b, h, p, n), with their total log-decay (piece, part, b, h), from summary_kernel.
+    int pt, parts;
+    const float* piece_sum;
+    const float* piece_decay;
 };
 
 constexpr uint32_t kIdescS = instr_desc(128, 128, false, false);    // K-major x K-major, N = 128

@@ -1,7 +1,8 @@
 // Forward walk of the tensor-core path (included by ssd_tc.cuh).
 //
-// One CTA per (batch, head) walks the 128-position tiles in order with the recurrent state (64 x 128, fp32) in
-// registers.  Per tile k (V = B, U = x, C of the tile; H = state entering it; S_k = its total log2-decay):
+// One CTA per (batch, head, piece of the sequence) walks the 128-position tiles in order with the recurrent state
+// (64 x 128, fp32) in registers; more than one piece where (batch, head) pairs alone leave most of the chip idle (Pieces,
+// ssd_tc_host.cuh).  Per tile k (V = B, U = x, C of the tile; H = state entering it; S_k = its total log2-decay):
 //   S  = C V^T                     issued one tile ahead into a double-buffered TMEM accumulator
 //   Yo = C H^T                     the entering state's part of the output
 //   Hl = V^T (d dt o U)            the tile's contribution to the state; the weighted copy of U is made by the rows
@@ -74,16 +75,17 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     float* sysq = sdtc + 2 * LT;                           // [2][2][128] partial sums of y^2 of the odd quarters
     __shared__ uint64_t bar_ld[2], bar_s, bar_u, bar_g, bar_mh, bar_m2, bar_h, bar_sr;
     __shared__ uint32_t tmem_slot;
-    __shared__ int failed;
+    __shared__ int failed, rows_nt;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hh = blockIdx.x, bb = blockIdx.y;
     const int gg = hh / P.hpg;
     const size_t bh = (size_t)bb * P.h + hh;
-    const int nt = P.nt;
+    const int k0 = blockIdx.z * P.pt, nt = min(P.pt, P.nt - k0);  // the piece's tiles
 
     if (tid == 0) {
         failed = 0;
+        rows_nt = nt;
         mbar_init(&bar_ld[0], 1);
         mbar_init(&bar_ld[1], 1);
         mbar_init(&bar_s, 1);
@@ -103,7 +105,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     // state row of this thread: n = row, p in [16 q, 16 q + 16)
     float H[16];
     if (warp < 16) {
-        load_state_row(P.seed, bh, P.p, P.n, row, q * 16, H);
+        load_piece_row<false>(P, bh, row, q * 16, H);
         store_quarter_row(sH, row, q * 2, H);
         fence_async_smem();
     }
@@ -114,7 +116,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     // S double-buffered [0,256), masked operand (bf16 pairs) [256,320), Yd [320,384), Yo [384,448), Hl [448,512)
     const uint32_t tG = tm + 256, tYd = tm + 320, tYo = tm + 384, tHl = tm + 448;
     auto state_row = [&](int it) {  // row of tile `it` of this walk in the [b*nt*h*128][64] state tensor
-        return (int)((((size_t)bb * nt + it) * P.h + hh) * DN);
+        return (int)((((size_t)bb * P.nt + k0 + it) * P.h + hh) * DN);
     };
 
     if (warp >= 16) {
@@ -180,11 +182,12 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 const int s = it % NST;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, it * LT, bb);
-                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, it * LT, bb);
-                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, it * LT, bb);
-                tma_load_4d(st + 3 * PANEL, &P.mC, &bar_ld[s], 0, gg, it * LT, bb);
-                tma_load_4d(st + 4 * PANEL, &P.mC, &bar_ld[s], 64, gg, it * LT, bb);
+                const int pos = (k0 + it) * LT;
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
+                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, pos, bb);
+                tma_load_4d(st + 3 * PANEL, &P.mC, &bar_ld[s], 0, gg, pos, bb);
+                tma_load_4d(st + 4 * PANEL, &P.mC, &bar_ld[s], 64, gg, pos, bb);
             };
             for (int it = 0; it < NST - 1 && it < nt; ++it) issue_loads(it);
             if (P.save_states) {  // the seed is the state entering the first tile
@@ -199,7 +202,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 }
                 if (it > 0) {
                     mbar_wait_spin(&bar_h, (it - 1) & 1, &failed);  // new state in sH, y staged
-                    tma_store_4d(&P.mY, sY, 0, hh, (it - 1) * LT, bb);
+                    tma_store_4d(&P.mY, sY, 0, hh, (k0 + it - 1) * LT, bb);
                     if (P.save_states) tma_store_2d(&P.mS, sH, 0, state_row(it));
                     tma_store_commit();
                 }
@@ -207,7 +210,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 mbar_arrive(&bar_sr);  // sH and sY may be rewritten
             }
             mbar_wait_spin(&bar_h, (nt - 1) & 1, &failed);
-            tma_store_4d(&P.mY, sY, 0, hh, (nt - 1) * LT, bb);
+            tma_store_4d(&P.mY, sY, 0, hh, (k0 + nt - 1) * LT, bb);
             tma_store_commit();
             tma_store_wait_all();
         }
@@ -215,13 +218,15 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     } else {
         // ------------------------------------------------------------------ row warps: thread = (row, column quarter)
         setmaxnreg_inc<kFwdRegsRow>();
+        const volatile int& rnt = rows_nt;  // in shared memory: the row warps have no register left for it
         const int rb = row >> 5;  // row block, warp-uniform
         const bool active = q <= rb, diag = q == rb;
-        const float* tcum = P.tcum + bh * P.Tp;
-        const float* dtT = P.dtT ? P.dtT + bh * P.Tp : nullptr;
+        const size_t t0 = bh * P.Tp + (size_t)k0 * LT;
+        const float* tcum = P.tcum + t0;
+        const float* dtT = P.dtT ? P.dtT + t0 : nullptr;
         const uint32_t lanes = lane_base(warp);
         const float Dhead = P.D ? P.D[hh] : 0.f;
-        const float* skipT = P.skipT ? P.skipT + bh * P.Tp : nullptr;  // per-position skip instead of D
+        const float* skipT = P.skipT ? P.skipT + t0 : nullptr;  // per-position skip instead of D
         const bool has_skip = P.D || P.skipT;
         const int c0 = q * 32;  // this thread's 32 columns of S
         // per-tile scalars are fetched one tile ahead
@@ -231,11 +236,11 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         float sk_n = skipT ? skipT[row] : Dhead;
         float ysq_own = 0.f;  // even quarters: own partial of the tile before
 
-        for (int it = 0; it < nt; ++it) {
+        for (int it = 0; it < rnt; ++it) {
             const int s = it % NST, buf = it & 1;
             const uint32_t ph = it & 1;
             const float c_i = c_n, cend = cend_n, dtv = dt_n, Dh = sk_n;
-            if (it + 1 < nt) {
+            if (it + 1 < rnt) {
                 const size_t o = (size_t)(it + 1) * LT;
                 c_n = tcum[o + row];
                 cend_n = tcum[o + (row | 31)];
@@ -250,7 +255,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             mbar_wait(&bar_ld[s], (it / NST) & 1, &failed);
             named_barrier(1, 512);
             if (P.ysq && it > 0 && !(q & 1))  // the sum of the half row of the tile before: own quarter + the odd one's
-                P.ysq[((((size_t)bb * nt + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
+                P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((it - 1) & 1) * 2 + (q >> 1)) * LT + row];
 
             const float Sk = scum2[buf * LT + LT - 1];
@@ -375,10 +380,10 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         if (P.ysq) {
             named_barrier(1, 512);
             if (!(q & 1))
-                P.ysq[((((size_t)bb * nt + (nt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
-                    ysq_own + sysq[(((nt - 1) & 1) * 2 + (q >> 1)) * LT + row];
+                P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (rnt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
+                    ysq_own + sysq[(((rnt - 1) & 1) * 2 + (q >> 1)) * LT + row];
         }
-        store_state_row(P.out_state, bh, P.p, P.n, row, q * 16, H);
+        if (blockIdx.z * P.pt + rnt == P.nt) store_state_row(P.out_state, bh, P.p, P.n, row, q * 16, H);
     }
     tc_fence_before();
     __syncthreads();

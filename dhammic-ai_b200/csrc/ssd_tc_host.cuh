@@ -54,8 +54,37 @@ inline bool make_map4(CUtensorMap* m, const void* base, const Dims& d, int heads
 }
 
 struct Ws {
-    size_t status, tcum, dtT, skipT, Hst, Qst, final_state, dinit, g, ddtx, dyx, gS, dAh_part, dD_part, total;
+    size_t status, tcum, dtT, skipT, Hst, Qst, final_state, dinit, g, ddtx, dyx, gS, dAh_part, dD_part, piece_sum, piece_decay, base, total;
 };
+
+// The pieces that a walk over one sequence is cut into.  A walk has one CTA per (batch, head), which takes 2.15 us per tile forward
+// and 1.5 us in reverse; with few of them most SMs idle.  Pieces run side by side: every piece but the walk's last is first
+// summarised (0.8 us per tile, no chain, in parts that fill the chip), and a piece's CTA folds the summaries before its own into
+// its seed.  Only while all CTAs fit on the chip at once, and where the tiles taken off the chain outweigh the summary and its
+// launch (12 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.
+// One prompt of 16,384 positions and 64 heads (128 tiles, two pieces): 282 us in one piece, 213 with one summary, 189 with two parts.
+struct Pieces {
+    int pt, np, ps, parts;  // tiles of a piece, pieces, tiles of a summarised part, parts of a piece
+};
+constexpr int kPieceSms = 148, kMaxEntries = 16;
+inline Pieces pieces_of(const Dims& d, bool reverse) {
+    const int nt = tiles_of(d.T);
+    const long long bh = (long long)d.b * d.h;
+    const double tile = reverse ? 1.5 : 2.15;
+    Pieces best{nt, 1, nt, 1};
+    double cost = 0.9 * tile * nt;
+    for (int P = 2; P <= kMaxEntries && P * bh <= kPieceSms && P <= nt; ++P) {
+        const int pt = (nt + P - 1) / P, np = (nt + pt - 1) / pt;
+        const int want = (int)std::max(1LL, std::min({(long long)pt, kPieceSms / (bh * (np - 1)), (long long)kMaxEntries / (np - 1)}));
+        const int ps = (pt + want - 1) / want, parts = (pt + ps - 1) / ps;
+        const double c = tile * pt + 0.8 * ps + 12.0 + 0.6 * parts * (np - 1);
+        if (c < cost) {
+            cost = c;
+            best = {pt, np, ps, parts};
+        }
+    }
+    return best;
+}
 
 inline Ws ws_layout(const Dims& d, int pass) {
     Ws w{};
@@ -84,6 +113,16 @@ inline Ws ws_layout(const Dims& d, int pass) {
         w.gS = take((size_t)d.b * d.h * nt * 8 * 4);
         w.dAh_part = take((size_t)d.b * nt * d.h * 4);
         w.dD_part = take((size_t)d.b * nt * d.h * 4);
+    }
+    w.base = off;  // enough for a walk in one piece
+    auto entries = [&](bool reverse) {
+        const Pieces pc = pieces_of(d, reverse);
+        return (size_t)(pc.np - 1) * pc.parts;
+    };
+    const size_t ne = pass == SSD_B200_PASS_BWD ? std::max(entries(false), entries(true)) : entries(false);
+    if (ne > 0) {
+        w.piece_sum = take(ne * bhpn);
+        w.piece_decay = take(ne * d.b * d.h * 4);
     }
     w.total = off;
     return w;
@@ -150,9 +189,27 @@ inline int launch_tile_cumsum(const Dims& d, const float* cum, const float* dt, 
     return 0;
 }
 
+// Cuts the walk of P into pieces where that pays and the workspace has the room, and summarises them.
+template <bool REV>
+inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace, size_t bytes, int* pieces, cudaStream_t st, char* err, size_t errn) {
+    P.pt = P.nt;
+    *pieces = 1;
+    const Pieces pc = pieces_of(d, REV);
+    if (pc.np == 1 || bytes < w.total) return 0;
+    SummaryParams S{};
+    S.mU = P.mU; S.mV = P.mV; S.tcum = P.tcum; S.dtT = P.dtT; S.out = (float*)((char*)workspace + w.piece_sum);
+    S.logdecay = (float*)((char*)workspace + w.piece_decay); S.status = P.status; S.Tp = P.Tp; S.h = P.h; S.hpg = P.hpg; S.nt = P.nt;
+    S.p = P.p; S.n = P.n; S.pt = pc.pt; S.ps = pc.ps; S.parts = pc.parts; S.z0 = REV ? 1 : 0;
+    SSD_LAUNCH(prof::K_TC_SUMMARY, st, (summary_kernel<REV, 1><<<dim3(d.h, d.b, (pc.np - 1) * pc.parts), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st>>>(S)));
+    SSD_TC_CHECK("tc_summary_pieces");
+    P.pt = pc.pt; P.parts = pc.parts; P.piece_sum = S.out; P.piece_decay = S.logdecay;
+    *pieces = pc.np;
+    return 0;
+}
+
 inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, char* err, size_t errn) {
     Ws w = ws_layout(d, SSD_B200_PASS_FWD);
-    if (a->workspace_bytes < w.total) SSD_TC_FAIL(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
+    if (a->workspace_bytes < w.base) SSD_TC_FAIL(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.base);
     if (!encode_fn()) SSD_TC_FAIL(SSD_B200_ECUDA, "cuTensorMapEncodeTiled is not available");
     const bool states_only = (a->flags & SSD_B200_FWD_STATES_ONLY) != 0;
     for (const void* p : {a->x, a->B, a->C, (const void*)a->y})
@@ -215,7 +272,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     if (states_only) {  // what this piece of the sequence adds to the state after it (plus the decayed seed)
         SummaryParams S{};
         S.mU = P.mU; S.mV = P.mV; S.tcum = tcum; S.dtT = dtT; S.seed = a->init; S.out = a->final_state;
-        S.logdecay = a->logdecay_total; S.status = status; S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = nt;
+        S.logdecay = a->logdecay_total; S.status = status; S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1;
         S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)  // two heads of a group per CTA share the group's panels
             SSD_LAUNCH(prof::K_TC_SUMMARY, st, (summary_kernel<false, 2><<<dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st>>>(S)));
@@ -224,8 +281,10 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
         SSD_TC_CHECK("tc_summary_fwd");
         return 0;
     }
-    SSD_LAUNCH(prof::K_TC_FWD, st, (fwd_walk_kernel<false><<<dim3(d.h, d.b), kFwdThreads, kFwdSmem, st>>>(P)));
-    SSD_LAUNCH(prof::K_TC_FWD_ALT, st, (fwd_walk_kernel<true><<<dim3(d.h, d.b), kFwdThreads, kFwdSmem, st>>>(P)));
+    int pieces;
+    if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, st, err, errn)) return rc;
+    SSD_LAUNCH(prof::K_TC_FWD, st, (fwd_walk_kernel<false><<<dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st>>>(P)));
+    SSD_LAUNCH(prof::K_TC_FWD_ALT, st, (fwd_walk_kernel<true><<<dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st>>>(P)));
     SSD_TC_CHECK("tc_fwd_walk");
     if (a->logdecay_total) {
         SSD_LAUNCH(prof::K_CUMSUM, st, logdecay_total_kernel<<<(d.b * d.h + 127) / 128, 128, 0, st>>>(a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
@@ -236,7 +295,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
 
 inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, char* err, size_t errn) {
     Ws w = ws_layout(d, SSD_B200_PASS_BWD);
-    if (a->workspace_bytes < w.total) SSD_TC_FAIL(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
+    if (a->workspace_bytes < w.base) SSD_TC_FAIL(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.base);
     if (!encode_fn()) SSD_TC_FAIL(SSD_B200_ECUDA, "cuTensorMapEncodeTiled is not available");
     for (const void* p : {a->x, a->B, a->C, a->dy, (const void*)a->dx, (const void*)a->dB, (const void*)a->dC})
         if ((uintptr_t)p & 15) SSD_TC_FAIL(SSD_B200_EINVAL, "tensor-core path needs 16-byte aligned tensors");
@@ -269,7 +328,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         if (!(make_map4(&S.mU, a->dy, d, d.h, d.p) && make_map4(&S.mV, a->C, d, d.g, d.n)))
             SSD_TC_FAIL(SSD_B200_ECUDA, "tensor map encoding failed");
         S.tcum = tcum; S.dtT = nullptr; S.seed = a->dfinal; S.out = a->dinit; S.logdecay = nullptr; S.status = status;
-        S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = nt; S.p = d.p; S.n = d.n;
+        S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1; S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)
             SSD_LAUNCH(prof::K_TC_SUMMARY, st, (summary_kernel<true, 2><<<dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st>>>(S)));
         else
@@ -287,7 +346,9 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.mU = mX; P.mV = mB; P.mC = mC; P.mY = mdX; P.mS = mH; P.save_states = 1;
         P.tcum = tcum; P.dtT = dtT; P.D = nullptr; P.seed = a->init; P.out_state = fin; P.status = status;
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
-        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (states_walk_kernel<<<dim3(d.h, d.b), kWalkThreads, WalkCfg<1>::SMEM, st>>>(P)));
+        int pieces;  // the same as the forward's: the states have the same bits
+        if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, st, err, errn)) return rc;
+        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (states_walk_kernel<<<dim3(d.h, d.b, pieces), kWalkThreads, WalkCfg<1>::SMEM, st>>>(P)));
         SSD_TC_CHECK("tc_bwd_state");
     }
     {   // reverse walk: gradient of the state leaving every tile, and d(initial state)
@@ -295,10 +356,14 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.mU = mdY; P.mV = mC; P.mC = mC; P.mY = mdX; P.mS = mQ; P.save_states = 1;
         P.tcum = tcum; P.dtT = nullptr; P.D = nullptr; P.seed = a->dfinal; P.out_state = dinit; P.status = status;
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
-        if (d.hpg % 2 == 0)  // two heads of a group per CTA: shared C panels, one N = 128 product per tile
+        int pieces;
+        if (int rc = split_walk<true>(P, d, w, ws, a->workspace_bytes, &pieces, st, err, errn)) return rc;
+        // two heads of a group per CTA: shared C panels, one N = 128 product per tile; but a tile then takes 1.7 us instead of
+        // 1.5, so only where one head per CTA would not fit on the chip at once
+        if (d.hpg % 2 == 0 && pieces == 1 && (long long)d.b * d.h > kPieceSms)
             SSD_LAUNCH(prof::K_TC_BWD_STATE, st, rev_walk_kernel<2><<<dim3(d.h / 2, d.b), RevCfg<2>::THREADS, RevCfg<2>::SMEM, st>>>(P));
         else
-            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, rev_walk_kernel<1><<<dim3(d.h, d.b), RevCfg<1>::THREADS, RevCfg<1>::SMEM, st>>>(P));
+            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, rev_walk_kernel<1><<<dim3(d.h, d.b, pieces), RevCfg<1>::THREADS, RevCfg<1>::SMEM, st>>>(P));
         SSD_TC_CHECK("tc_bwd_dstate");
     }
     {

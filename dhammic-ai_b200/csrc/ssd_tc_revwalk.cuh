@@ -1,7 +1,7 @@
 // Reverse tile walk of the backward pass (included by ssd_tc.cuh after ssd_tc_walk.cuh).
 //
-// One CTA walks the 128-position tiles of NH heads of one group (same batch entry) from the last tile to the first,
-// with the gradient of each head's recurrent state Q (128 x 64, fp32) in the registers of that head's eight row
+// One CTA walks the 128-position tiles of NH heads of one group (same batch entry; NH = 1: or of a piece of the sequence, where
+// a whole one per CTA would leave most of the chip idle) from the last tile to the first, with the gradient of each head's recurrent state Q (128 x 64, fp32) in the registers of that head's eight row
 // warps.  Per tile k and head it
 //   * stores Q as it leaves tile k (bf16, [n][p]) for the per-tile backward kernel,
 //   * updates Q <- exp(S_k) Q + C^T (e . dY).
@@ -55,7 +55,8 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
     constexpr int CTLW = 8 * NH;  // control warp
     const int hh0 = blockIdx.x * NH, bb = blockIdx.y;
     const int gg = hh0 / P.hpg;
-    const int nt = P.nt;
+    // the piece's tiles; with two heads per CTA there is only ever one piece (and no register to spare)
+    const int k0 = NH == 1 ? (int)blockIdx.z * P.pt : 0, nt = NH == 1 ? min(P.pt, P.nt - k0) : P.nt;
 
     if (tid == 0) {
         failed = 0;
@@ -82,14 +83,14 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
             prefetch_tmap(&P.mU);
             prefetch_tmap(&P.mV);
             auto issue_loads = [&](int it) {
-                const int k = nt - 1 - it;
+                const int pos = (k0 + nt - 1 - it) * LT;
                 const int s = it % kRevStages;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, k * LT, bb);
-                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, k * LT, bb);
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
 #pragma unroll
-                for (int hs = 0; hs < NH; ++hs) tma_load_4d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], 0, hh0 + hs, k * LT, bb);
+                for (int hs = 0; hs < NH; ++hs) tma_load_4d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], 0, hh0 + hs, pos, bb);
             };
             for (int it = 0; it < kRevStages && it < nt; ++it) issue_loads(it);
             for (int it = 0; it < nt; ++it) {
@@ -120,11 +121,12 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
         const int hh = hh0 + hs;
         const int ht = tid & 255, row = ht & 127, hf = ht >> 7;
         const size_t bh = (size_t)bb * P.h + hh;
-        const float* tcum = P.tcum + bh * P.Tp;
+        const float* tcum = P.tcum + bh * P.Tp + (size_t)k0 * LT;
         const uint32_t lanes = lane_base(warp);
         uint8_t* sQ = sQ0 + (size_t)hs * PANEL;
         float H[32];  // state gradient row n = row, p in [hf*32, hf*32+32)
-        load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, H);
+        if (NH == 1) load_piece_row<true>(P, bh, row, hf * 32, H);
+        else load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, H);
         // Store the state gradient leaving tile nt-1-it: staged in the head's sQ panel, written by one TMA store of the
         // head's first thread, which waits until its previous store has read the panel; the first barrier (the head's
         // 256 threads) releases the panel to the writers, the second hands the written panel to the store.
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
             fence_async_smem();
             named_barrier(2 + 2 * hs, 256);
             if (ht == 0) {
-                tma_store_2d(&P.mS, sQ, 0, (int)((((size_t)bb * nt + (nt - 1 - it)) * P.h + hh) * DN));
+                tma_store_2d(&P.mS, sQ, 0, (int)((((size_t)bb * P.nt + k0 + (nt - 1 - it)) * P.h + hh) * DN));
                 tma_store_commit();
             }
         };
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
             c_i = c_n;
             Sk = Sk_n;
         }
-        store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
+        if (k0 == 0) store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
         if (ht == 0) tma_store_wait_all();
     }
     tc_fence_before();

@@ -14,7 +14,9 @@
 // overflows; the forward walks the tiles from the last to the first (the decay after a tile is a running sum that starts
 // at 0 where the weights are largest), the reverse from the first to the last.
 //
-// A given seed (initial state, or final-state gradient) enters as  exp(total log-decay) * seed.
+// A given seed (initial state, or final-state gradient) enters as  exp(total log-decay) * seed.  blockIdx.z =
+// (piece of `pt` tiles, part of `ps` tiles), each with its own out and logdecay (blockIdx.z, b, h, ...): the pieces of one
+// sequence that the walks run side by side.
 // mbarriers, per stage s (phase (it / stages) & 1): bar_ld[s] TMA bytes landed; bar_u[s] rows scaled, one arrival per
 // warp; bar_m[s] the products of the stage completed (the stage may be reloaded; the last one also releases the
 // accumulator to the row warps).
@@ -37,11 +39,13 @@ struct SummaryParams {
     const float* tcum;     // (b,h,T) tile-cumulative log2-decay
     const float* dtT;      // (b,h,T) dt (forward) or null
     const float* seed;     // (b,h,p,n) fp32 or null
-    float* out;            // (b,h,p,n) fp32
-    float* logdecay;       // (b,h) total log-decay of the piece in natural-log units, or null
+    float* out;            // (z,b,h,p,n) fp32
+    float* logdecay;       // (z,b,h) total log-decay of the part in natural-log units, or null
     int* status;
     int Tp, h, hpg, nt;   // Tp = nt * 128: stride of the per-position arrays
     int p, n;
+    int pt, ps, parts;    // tiles of a piece and of a part, parts per piece
+    int z0;               // piece of the blocks with blockIdx.z = 0
 };
 
 template <bool REV, int NH>
@@ -58,9 +62,10 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hh0 = blockIdx.x * NH, bb = blockIdx.y;
     const int gg = hh0 / P.hpg;
-    const int nt = P.nt;
-    // forward: tiles nt-1 .. 0; reverse: 0 .. nt-1
-    auto tile_of = [&](int it) { return REV ? it : nt - 1 - it; };
+    const int part = (int)blockIdx.z % P.parts, piece = P.z0 + (int)blockIdx.z / P.parts;
+    const int k0 = piece * P.pt + part * P.ps, nt = max(0, min(min(P.ps, P.pt - part * P.ps), P.nt - k0));  // (the last piece can be short)
+    // forward: tiles nt-1 .. 0 of the part; reverse: 0 .. nt-1
+    auto tile_of = [&](int it) { return k0 + (REV ? it : nt - 1 - it); };
 
     if (tid == 0) {
         failed = 0;
@@ -120,9 +125,10 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         const float* tcum = P.tcum + bh * P.Tp;
         const float* dtT = (!REV && P.dtT) ? P.dtT + bh * P.Tp : nullptr;
         float run = 0.f;  // forward: log2-decay of the tiles after this one; reverse: of the tiles before it
-        float c_n = tcum[(size_t)tile_of(0) * LT + row];
-        float S_n = tcum[(size_t)tile_of(0) * LT + LT - 1];
-        float dt_n = dtT ? dtT[(size_t)tile_of(0) * LT + row] : 1.f;
+        const size_t o0 = (size_t)max(0, min(tile_of(0), P.nt - 1)) * LT;
+        float c_n = tcum[o0 + row];
+        float S_n = tcum[o0 + LT - 1];
+        float dt_n = dtT ? dtT[o0 + row] : 1.f;
         for (int it = 0; it < nt; ++it) {
             const int s = it % NS;
             const float c_i = c_n, Sk = S_n, dtv = dt_n;
@@ -154,18 +160,24 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         }
         // `run` is now the total log2-decay of the piece
         const int last = nt - 1;
-        mbar_wait(&bar_m[last % NS], (last / NS) & 1, &failed);
-        tc_fence_after();
         uint32_t r[32];
-        tmem_ld32(tm + lane_base(warp) + hs * 64 + hf * 32, r);
-        tmem_ld_wait();
+        if (nt > 0) {  // (block-uniform)
+            mbar_wait(&bar_m[last % NS], (last / NS) & 1, &failed);
+            tc_fence_after();
+            tmem_ld32(tm + lane_base(warp) + hs * 64 + hf * 32, r);
+            tmem_ld_wait();
+        } else {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) r[q] = 0u;
+        }
         const float dec = exp2f(run);
         float v[32];  // accumulator row = n, columns = p
         load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, v);
 #pragma unroll
         for (int q = 0; q < 32; ++q) v[q] = fmaf(dec, v[q], __uint_as_float(r[q]));
-        store_state_row(P.out, bh, P.p, P.n, row, hf * 32, v);
-        if (P.logdecay && ht == 0) P.logdecay[bh] = run * 0.6931471805599453f;
+        const size_t zbh = (size_t)blockIdx.z * gridDim.y * P.h + bh;
+        store_state_row(P.out, zbh, P.p, P.n, row, hf * 32, v);
+        if (P.logdecay && ht == 0) P.logdecay[zbh] = run * 0.6931471805599453f;
     }
     tc_fence_before();
     __syncthreads();

@@ -1,6 +1,6 @@
 // State walk of the tensor-core path and what the walk kernels share (included by ssd_tc.cuh).
 //
-// states_walk_kernel: one CTA per (batch, head) walks the 128-position tiles in order with the recurrent state
+// states_walk_kernel: one CTA per (batch, head, piece of the sequence) walks the 128-position tiles in order with the recurrent state
 // (64 x 128, fp32) in registers and stores the state entering every tile as bf16 — the recurrence of the forward without
 // its output.  The backward uses it when the forward did not keep the states.  Ten warps:
 //   warps 0-7  "row" warps: thread (row = tid & 127, half = tid >> 7) owns TMEM lane `row` and one half of the
@@ -52,6 +52,22 @@ __device__ __forceinline__ void load_state_row(const float* base, size_t bh, int
         for (int q = 0; q < N; ++q) H[q] = (s && row < n && p0 + q < p) ? s[(size_t)q * n] : 0.f;
     }
 }
+// The same for the state entering this block's piece of a walk: the seed carried through the pieces before it (reverse walk:
+// the state gradient leaving the piece, through the pieces behind it; the entries start with piece 1).
+template <bool REV, int N>
+__device__ __forceinline__ void load_piece_row(const WalkParams& P, size_t bh, int row, int p0, float (&H)[N]) {
+    load_state_row(P.seed, bh, P.p, P.n, row, p0, H);
+    const size_t nbh = (size_t)gridDim.y * P.h;
+    const int passed = P.parts * (int)(REV ? gridDim.z - 1 - blockIdx.z : blockIdx.z), all = P.parts * (int)(gridDim.z - 1);
+    for (int i = 0; i < passed; ++i) {
+        const int j = REV ? all - 1 - i : i;
+        const float dec = expf(P.piece_decay[j * nbh + bh]);
+        float v[N];
+        load_state_row(P.piece_sum, j * nbh + bh, P.p, P.n, row, p0, v);
+#pragma unroll
+        for (int q = 0; q < N; ++q) H[q] = fmaf(dec, H[q], v[q]);
+    }
+}
 template <int N>
 __device__ __forceinline__ void store_state_row(float* base, size_t bh, int p, int n, int row, int p0, const float (&H)[N]) {
     if (!base || row >= n) return;
@@ -90,7 +106,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     const int hh = blockIdx.x, bb = blockIdx.y;
     const int gg = hh / P.hpg;
     const size_t bh = (size_t)bb * P.h + hh;
-    const int nt = P.nt;
+    const int k0 = blockIdx.z * P.pt, nt = min(P.pt, P.nt - k0);  // the piece's tiles
 
     if (tid == 0) {
         failed = 0;
@@ -109,7 +125,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     // state row of this thread: n = row, p in [hf*32, hf*32+32)
     float H[32];
     if (warp < 8) {
-        load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, H);
+        load_piece_row<false>(P, bh, row, hf * 32, H);
         store_half_row(sH, row, hf * 4, H);
         fence_async_smem();
     }
@@ -118,7 +134,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     tc_fence_after();
     const uint32_t tHl = tmem_slot;
     auto state_row = [&](int it) {  // row of tile `it` of this walk in the [b*nt*h*128][64] state tensor
-        return (int)((((size_t)bb * nt + it) * P.h + hh) * DN);
+        return (int)((((size_t)bb * P.nt + k0 + it) * P.h + hh) * DN);
     };
     if (warp == 8) {
         // ------------------------------------------------------------------ product lane
@@ -150,9 +166,10 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
                 const int s = it % NST;
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, it * LT, bb);
-                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, it * LT, bb);
-                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, it * LT, bb);
+                const int pos = (k0 + it) * LT;
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
+                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, pos, bb);
             };
             for (int it = 0; it < NST - 1 && it < nt; ++it) issue_loads(it);
             tma_store_2d(&P.mS, sH, 0, state_row(0));  // the seed is the state entering the first tile
@@ -176,8 +193,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ row warps
-        const float* tcum = P.tcum + bh * P.Tp;
-        const float* dtT = P.dtT ? P.dtT + bh * P.Tp : nullptr;
+        const float* tcum = P.tcum + bh * P.Tp + (size_t)k0 * LT;
+        const float* dtT = P.dtT ? P.dtT + bh * P.Tp + (size_t)k0 * LT : nullptr;
         const uint32_t lanes = lane_base(warp);
         // per-tile scalars are fetched one tile ahead
         float c_n = tcum[row], S_n = tcum[LT - 1];
@@ -230,7 +247,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
             fence_async_smem();
             mbar_arrive_warp(&bar_h);
         }
-        store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
+        if (k0 + nt == P.nt) store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
     }
     tc_fence_before();
     __syncthreads();

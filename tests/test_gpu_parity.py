@@ -333,6 +333,38 @@ def test_saved_states_equal_recomputed_states(pkg, cabi):
         assert torch.equal(kept[k], redone[k]), k
 
 
+@pytest.mark.parametrize("b,T,h,g,p,n,chunk", [(1, 4096, 6, 2, 64, 128, 128), (1, 3008, 30, 5, 64, 64, 64), (2, 6016, 4, 4, 48, 128, 64),
+                                               (1, 16384, 9, 1, 64, 128, 256)])
+def test_walks_in_pieces(pkg, cabi, oracle, b, T, h, g, p, n, chunk):
+    """Few (batch, head) pairs and a long sequence: the walks run in pieces side by side, seeded from summaries.  Several pieces, a
+    short last piece, summaries in parts, states in and out, columns below the tile's; against the oracle, and the same whether
+    the forward kept its states or the backward walks them again (bit for bit where a chunk is a tile; for other chunks the
+    backward rebuilds the tiles' decays from a_cumsum, which rounds differently)."""
+    gen = torch.Generator().manual_seed(T + h)
+    def randn(*s):
+        return torch.randn(*s, generator=gen)
+    bf = torch.bfloat16
+    inp = {"x": randn(b, T, h, p).to(bf), "dt": torch.nn.functional.softplus(0.5 * randn(b, T, h) - 3.9).clamp(1e-3, 0.1),
+           "A_head": -torch.exp(torch.rand(h, generator=gen) * 2.77 - 2.0), "B": (randn(b, T, g, n) / n ** 0.5).to(bf),
+           "C": (randn(b, T, g, n) / n ** 0.5).to(bf), "D": randn(h), "dy": randn(b, T, h, p).to(bf)}
+    init, dfinal = randn(b, h, p, n) * 0.5, randn(b, h, p, n)
+    got = mamba2_gpu(pkg, inp, chunk, init, dfinal)
+    want = oracle.mamba2_fwd_bwd(inp, chunk, torch.float32, init.unsqueeze(1), dfinal)
+    errs = {k: rel_err(got[k], want[k].reshape(got[k].shape)) for k in got}
+    bad = {k: v for k, v in errs.items() if not v < TOL_BF16}
+    assert not bad, errs
+    pkg.set_save_states(False)
+    try:
+        redone = mamba2_gpu(pkg, inp, chunk, init, dfinal)
+    finally:
+        pkg.set_save_states(True)
+    for k in got:
+        if chunk == 128:
+            assert torch.equal(got[k], redone[k]), k
+        else:
+            assert rel_err(redone[k], want[k].reshape(redone[k].shape)) < TOL_BF16, k
+
+
 def test_mamba3_variant_takes_fp32_angles_with_bf16_tensors(pkg, cabi, oracle):
     """Angles given in fp32 (the reference's fp32 dt * theta product) are summed at that precision although x, B and C
     are bf16; their gradient comes back in fp32."""
