@@ -386,18 +386,25 @@ int m3_fwd_impl(const ssd::Dims& d, const void* x, const float* dt, const float*
                 float* segsum, const float* D, float* wout, float* skip, cudaStream_t st) {
     using namespace ssd::m3;
     const int E = d.h * (d.n / 2), nseg = (d.T + SEG - 1) / SEG;
-    dim3 gs(nseg, (E + 255) / 256, d.b);
-    if (ang_f32) {  // angles keep their own precision whatever the storage type of x, B and C
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<float><<<gs, 256, 0, st>>>((const float*)ang, segsum, d.T, E));
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, float><<<gs, 256, 0, st>>>((const float*)ang, segsum, cum, d.T, E, 0, -1.f)));
+    if (d.n % VecOf<T>::N == 0 && !any_unaligned({B, C, ang, cum, Br, Cr})) {  // whole vectors
+        constexpr int V = VecOf<T>::N, N = V / 2;
+        const dim3 gw((d.T + WALK - 1) / WALK, (E / N + 255) / 256, d.b), gp((E + 63) / 64, d.b);
+        if (ang_f32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (angle_segsum_kernel<float, N><<<gw, 256, 0, st>>>((const float*)ang, cum, d.T, E)));
+        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (angle_segsum_kernel<T, N><<<gw, 256, 0, st>>>((const T*)ang, cum, d.T, E)));
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, angle_prefix_kernel<<<gp, 64, 0, st>>>(cum, d.T, E));
+        if (ang_f32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_walk_fwd_kernel<T, float, V><<<gw, 256, 0, st>>>((const T*)B, (const T*)C, (const float*)ang, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
+        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_walk_fwd_kernel<T, T, V><<<gw, 256, 0, st>>>((const T*)B, (const T*)C, (const T*)ang, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
     } else {
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<T><<<gs, 256, 0, st>>>((const T*)ang, segsum, d.T, E));
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<T, float><<<gs, 256, 0, st>>>((const T*)ang, segsum, cum, d.T, E, 0, -1.f)));
-    }
-    if (d.n % VecOf<T>::N == 0)
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_fwd_kernel<T, VecOf<T>::N><<<dim3(d.T, d.b), 256, 0, st>>>((const T*)B, (const T*)C, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
-    else
+        const dim3 gs(nseg, (E + 255) / 256, d.b);
+        if (ang_f32) {  // angles keep their own precision whatever the storage type of x, B and C
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<float><<<gs, 256, 0, st>>>((const float*)ang, segsum, d.T, E));
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, float><<<gs, 256, 0, st>>>((const float*)ang, segsum, cum, d.T, E, 0, -1.f)));
+        } else {
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<T><<<gs, 256, 0, st>>>((const T*)ang, segsum, d.T, E));
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<T, float><<<gs, 256, 0, st>>>((const T*)ang, segsum, cum, d.T, E, 0, -1.f)));
+        }
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_fwd_kernel<T, 2><<<dim3(d.T, d.b), 256, 0, st>>>((const T*)B, (const T*)C, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
+    }
     const size_t grows = (size_t)d.b * d.T * d.g, rows = (size_t)d.b * d.T * d.h;
     SSD_LAUNCH(ssd::prof::K_TC_AUX, st, bc_dot_kernel<T><<<(unsigned)((grows + 7) / 8), 256, 0, st>>>((const T*)B, (const T*)C, sdot, d.n, grows));
     if (xw) {
@@ -436,13 +443,19 @@ int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* 
         const size_t items = (size_t)d.b * d.T * d.g * (d.n / 2);
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_bwd_kernel<T, 2><<<(unsigned)((items + 255) / 256), 256, 0, st>>>((const T*)B, (const T*)C, cum, (const T*)dBr, (const T*)dCr, dyx, dt, lam, (T*)dB, (T*)dC, dcum, d.T, d.h, d.g, d.n, items)));
     }
-    dim3 gs(nseg, (E + 255) / 256, d.b);
-    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<float><<<gs, 256, 0, st>>>(dcum, segsum, d.T, E));
     // d raw_angles[t] = - sum_{s >= t} d cum[s]
-    if (ang_f32)
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, float><<<gs, 256, 0, st>>>(dcum, segsum, (float*)dang, d.T, E, 1, -1.f)));
-    else
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, T><<<gs, 256, 0, st>>>(dcum, segsum, (T*)dang, d.T, E, 1, -1.f)));
+    if ((long long)d.b * E >= kOnePassColumns) {
+        const dim3 go((E + 63) / 64, d.b);
+        if (ang_f32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_rev_kernel<float><<<go, 64, 0, st>>>(dcum, (float*)dang, d.T, E, -1.f));
+        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_rev_kernel<T><<<go, 64, 0, st>>>(dcum, (T*)dang, d.T, E, -1.f));
+    } else {
+        const dim3 gs(nseg, (E + 255) / 256, d.b);
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<float><<<gs, 256, 0, st>>>(dcum, segsum, d.T, E));
+        if (ang_f32)
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, float><<<gs, 256, 0, st>>>(dcum, segsum, (float*)dang, d.T, E, 1, -1.f)));
+        else
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, T><<<gs, 256, 0, st>>>(dcum, segsum, (T*)dang, d.T, E, 1, -1.f)));
+    }
     CUDA_LAUNCH_CHECK("mamba3 prologue backward");
     return 0;
 }

@@ -529,7 +529,7 @@ Tensor mamba3(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Ten
         at::NoGradGuard no_grad;
         xc = dense(x); Bc = dense(B); Cc = dense(C);
         // angles keep their own precision: fp32 angles (the reference's dt * theta product) are summed as given
-        ang = raw_angles.contiguous();
+        ang = dense(raw_angles);
         if (ang.scalar_type() != at::kFloat && ang.scalar_type() != x.scalar_type()) ang = ang.to(at::kFloat);
         dtc = f32(dt); lamc = f32(lam); Ah = f32(A_head);
         if (D.defined()) Dc = f32(D);

@@ -409,6 +409,39 @@ def test_mamba3_variant(pkg, cabi, oracle, dtype, tol):
     assert not bad, errs
 
 
+@pytest.mark.parametrize("T,h,g,n,chunk,ang32,shift", [(64, 1, 1, 40, 64, False, 0), (128, 4, 4, 128, 128, False, 0), (448, 5, 1, 64, 64, True, 0),
+                                                       (1120, 12, 2, 104, 32, False, 1), (160, 600, 1, 64, 32, False, 0)])
+def test_mamba3_angles_edges(pkg, cabi, oracle, T, h, g, n, chunk, ang32, shift):
+    """The running sum of the angles where it can go wrong: one block of positions and several, a last one that is not full,
+    columns that do not fill the blocks, angles in fp32 and at an odd address, enough columns for the one-pass reverse sum.
+    Against the oracle's two-call composition."""
+    gen = torch.Generator().manual_seed(T + h)
+    def randn(*s):
+        return torch.randn(*s, generator=gen)
+    bf = torch.bfloat16
+    inp = {"x": randn(2, T, h, 64).to(bf), "dt": torch.nn.functional.softplus(0.5 * randn(2, T, h) - 3.9).clamp(1e-3, 0.1),
+           "A_head": -torch.exp(torch.rand(h, generator=gen) * 2.77), "B": (randn(2, T, g, n) / n ** 0.5).to(bf),
+           "C": (randn(2, T, g, n) / n ** 0.5).to(bf), "D": randn(h),
+           "raw_angles": (torch.pi * (2 * torch.rand(2, T, h, n // 2, generator=gen) - 1)).to(torch.float32 if ang32 else bf),
+           "lam": torch.sigmoid(randn(2, T, h))}
+    dy = randn(2, T, h, 64).to(bf)
+    lv = {k: v.to(DEV).requires_grad_(True) for k, v in inp.items()}
+    if shift:
+        raw = torch.empty(inp["raw_angles"].numel() + shift, dtype=bf, device=DEV)[shift:].view(inp["raw_angles"].shape)
+        lv["raw_angles"] = raw.copy_(inp["raw_angles"]).requires_grad_(True)
+    y = pkg.ssd_mamba3(*lv.values(), chunk)
+    grads = torch.autograd.grad([y], list(lv.values()), [dy.to(DEV)])
+    torch.cuda.synchronize()
+    assert grads[6].dtype == inp["raw_angles"].dtype
+    ol = {k: v.float().requires_grad_(True) for k, v in inp.items()}
+    yo = oracle.mamba3_operator(*ol.values(), chunk)
+    go = torch.autograd.grad([yo], list(ol.values()), [dy.float()])
+    errs = {"y": rel_err(y, yo)}
+    errs.update({"d" + k: rel_err(a, b) for k, a, b in zip(inp, grads, go)})
+    bad = {k: v for k, v in errs.items() if not v < TOL_BF16}
+    assert not bad, errs
+
+
 def test_mamba3_against_reference_fixture(pkg, cabi):
     """The one-scan Mamba-3 form on the GPU against outputs of the reference's own two-call composition
     (tests/golden/m3_reference_block.npz: reference rotation convention, coefficients and scan), fp32."""
