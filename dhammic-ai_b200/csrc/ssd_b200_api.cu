@@ -118,29 +118,17 @@ bool simt_supported(const ssd_b200_shape& s, const char** why) {
 
 int resolve_path(const ssd_b200_shape& s) {
     const char* why = "";
-    const bool tc = ssd::tc::supported(s.dtype, (int)s.seqlen, (int)s.nheads, (int)s.headdim, (int)s.dstate,
-                                       (int)s.ngroups, (int)s.chunk);
+    const bool tc = ssd::tc::supported(s.dtype, (int)s.headdim, (int)s.dstate, (int)s.chunk, (int)s.nheads);
     if (s.path == SSD_B200_PATH_TC) {
         if (!tc) return fail(SSD_B200_EUNSUPPORTED, "tensor-core path does not cover this shape/dtype");
         return SSD_B200_PATH_TC;
     }
-    if (s.path == SSD_B200_PATH_AUTO && tc) return SSD_B200_PATH_TC;
+    if (s.path == SSD_B200_PATH_AUTO && tc && ssd::tc::whole_tiles((int)s.seqlen, (int)s.headdim, (int)s.dstate, (int)s.chunk))
+        return SSD_B200_PATH_TC;
     if (!simt_supported(s, &why)) return fail(SSD_B200_EUNSUPPORTED, "%s", why);
     return SSD_B200_PATH_SIMT;
 }
 
-// The tensor-core kernels move whole tiles by TMA, which wants 16-byte aligned tensors; the SIMT kernels take any address.
-// Where the library chose the path itself, a call with an unaligned tensor runs on the SIMT kernels if they cover the shape
-// (and the caller keeps no tile states, which only the tensor-core kernels know); the workspace of such a shape fits both.
-// Shapes that fill whole tiles have always been refused with an unaligned tensor, and still are.
-bool whole_tiles(const ssd_b200_shape& s) {
-    return s.headdim == ssd::tc::HP && s.dstate == ssd::tc::DN && s.seqlen % ssd::tc::LT == 0 &&
-           (s.chunk % ssd::tc::LT == 0 || ssd::tc::LT % s.chunk == 0);
-}
-bool simt_takes_unaligned(const ssd_b200_shape& s, int path) {
-    const char* why = "";
-    return path == SSD_B200_PATH_TC && s.path == SSD_B200_PATH_AUTO && !whole_tiles(s) && simt_supported(s, &why);
-}
 bool any_unaligned(std::initializer_list<const void*> ps) {
     for (const void* p : ps)
         if ((uintptr_t)p & 15) return true;
@@ -601,9 +589,7 @@ size_t ssd_b200_workspace_bytes(const ssd_b200_shape* shape, int pass) {
     int path = resolve_path(*shape);
     if (path < 0) return 0;
     ssd::Dims d = dims_of(*shape);
-    if (path == SSD_B200_PATH_SIMT) return simt_ws(d, pass).total;
-    const size_t tc = ssd::tc::workspace_bytes(d, pass);
-    return simt_takes_unaligned(*shape, path) ? std::max(tc, simt_ws(d, pass).total) : tc;
+    return path == SSD_B200_PATH_TC ? ssd::tc::workspace_bytes(d, pass) : simt_ws(d, pass).total;
 }
 
 size_t ssd_b200_states_bytes(const ssd_b200_shape* shape) {
@@ -628,8 +614,6 @@ int ssd_b200_fwd(const ssd_b200_fwd_args* a, void* stream) {
     if ((uintptr_t)a->states & 15) return fail(SSD_B200_EINVAL, "`states` must be 16-byte aligned");
     if (a->ysq && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`ysq` is only written by the tensor-core path");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
-    if (!a->states && !a->ysq && form != 3 && any_unaligned({a->x, a->B, a->C, a->y}) && simt_takes_unaligned(a->shape, path))
-        path = SSD_B200_PATH_SIMT;
     if (path == SSD_B200_PATH_TC) return ssd::tc::forward(a, dims_of(a->shape), st, g_err, sizeof(g_err));
     return a->shape.dtype == SSD_B200_BF16 ? simt_fwd<__nv_bfloat16>(a, st) : simt_fwd<float>(a, st);
 }
@@ -658,9 +642,6 @@ int ssd_b200_bwd(const ssd_b200_bwd_args* a, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if ((uintptr_t)a->states & 15) return fail(SSD_B200_EINVAL, "`states` must be 16-byte aligned");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
-    if (!a->states && form != 3 && any_unaligned({a->x, a->B, a->C, a->dy, a->dx, a->dB, a->dC}) &&
-        simt_takes_unaligned(a->shape, path))
-        path = SSD_B200_PATH_SIMT;
     if (path == SSD_B200_PATH_TC) return ssd::tc::backward(a, dims_of(a->shape), st, g_err, sizeof(g_err));
     return a->shape.dtype == SSD_B200_BF16 ? simt_bwd<__nv_bfloat16>(a, st) : simt_bwd<float>(a, st);
 }
@@ -700,12 +681,9 @@ int ssd_b200_fwd_static_scratch(const ssd_b200_fwd_args* a, void* stream) {
     if (int rc = check_shape(&a->shape)) return rc;
     int path = resolve_path(a->shape);
     if (path < 0) return path;
-    size_t need = ssd_b200_workspace_bytes(&a->shape, SSD_B200_PASS_FWD);
-    if (path == SSD_B200_PATH_TC) {  // a tensor-core walk runs in one piece where the room for more is missing
-        const ssd::Dims d = dims_of(a->shape);
-        need = ssd::tc::ws_layout(d, SSD_B200_PASS_FWD).base;
-        if (simt_takes_unaligned(a->shape, path)) need = std::max(need, simt_ws(d, SSD_B200_PASS_FWD).total);
-    }
+    // (a tensor-core walk runs in one piece where the room for more is missing)
+    const size_t need = path == SSD_B200_PATH_TC ? ssd::tc::ws_layout(dims_of(a->shape), SSD_B200_PASS_FWD).base
+                                                 : ssd_b200_workspace_bytes(&a->shape, SSD_B200_PASS_FWD);
     if (need > (size_t)SSD_B200_STATIC_SCRATCH_BYTES)
         return fail(SSD_B200_EWORKSPACE,
                     "this shape needs %zu bytes of scratch but the built-in array holds %u; use ssd_b200_fwd with a "

@@ -2,7 +2,8 @@
 // operands staged in 128-byte-swizzled shared memory by TMA (no cluster multicast).
 //
 // Covered shapes: bf16 storage, headdim up to 64, d_state up to 128 (see supported()), sequences and chunks of any
-// length.  The kernels work on tiles of 128 positions whatever the chunk size (the recurrence does not depend on where chunk boundaries fall); `tcum` is the inclusive
+// length; chosen without being asked for where these fill whole tiles (whole_tiles()).  The kernels work on tiles of 128
+// positions whatever the chunk size (the recurrence does not depend on where chunk boundaries fall); `tcum` is the inclusive
 // cumulative log-decay inside each 128-tile.
 //
 // Kernels
@@ -36,15 +37,19 @@ using namespace ssd::cum;
 constexpr int HP = 64;   // headdim
 constexpr int DN = 128;  // d_state
 constexpr int PANEL = 16384;  // bytes of one [128 rows][64 bf16] swizzled panel
-// Shapes below the tile's own size are padded on chip: TMA fills what lies behind the end of a sequence, or behind a head's
-// last column, with zeros, and does not write it.  (A row of p or n bf16 values has to be a multiple of 16 bytes for
-// that.)  Half-empty tiles still beat the fp32 kernels down to about a quarter of the tile's columns.
-inline bool supported(int dtype, int T, int h, int p, int n, int g, int l) {
-    (void)T;
-    (void)g;
+// What the kernels can run: shapes below the tile's own size are padded on chip, TMA fills what lies behind the end of a
+// sequence, or behind a head's last column, with zeros, and does not write it.  (A row of p or n bf16 values has to be a
+// multiple of 16 bytes for that.)
+inline bool supported(int dtype, int p, int n, int l, int h) {
     return dtype == 1 && p > HP / 2 && p <= HP && p % 8 == 0 && n > DN / 4 && n <= DN && n % 8 == 0 &&
            (l <= kFusedChunkMax || (long long)l * (h + 1) * 4 <= 227 * 1024);
 }
+// What they are chosen for.  Operands of the products (the masked scores, the weighted x, the states a tile starts from) are
+// rounded to bf16 here and are fp32 in the SIMT kernels.  Calls that fill whole tiles take that rounding; for others it is the
+// caller's choice (SSD_B200_PATH_TC): the final state of 320 positions in chunks of 80 is 2.4e-3 off the exact one on
+// these kernels, 2.5e-7 on the SIMT kernels (and forward + backward of (4, 1984, 20 heads, 64), d_state 64, chunk 64 take
+// 168 us here, 929 us there).
+inline bool whole_tiles(int T, int p, int n, int l) { return p == HP && n == DN && T % LT == 0 && (l % LT == 0 || LT % l == 0); }
 inline int tiles_of(int T) { return (T + LT - 1) / LT; }
 
 // ------------------------------------------------------------------------------------------

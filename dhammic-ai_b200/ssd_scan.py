@@ -70,7 +70,10 @@ def set_eager_cache(flag: bool) -> None:
 
 
 def set_kernel_path(path: str) -> None:
-    """'auto' (default), 'simt' (fp32 SIMT kernels) or 'tc' (tcgen05 kernels; raises if unsupported)."""
+    """'auto' (default), 'simt' (fp32 SIMT kernels) or 'tc' (tcgen05 kernels; raises if unsupported).  'auto' takes the tcgen05
+    kernels for bf16 calls that fill their tiles (headdim 64, d_state 128, whole tiles of 128 positions).  'tc' takes them for
+    others too (headdim above 32 and up to 64, d_state above 32 and up to 128, multiples of 8; any length and chunk), which is
+    faster, with the operands of the products rounded to bf16 where the fp32 kernels round nothing."""
     global _FORCE_PATH
     _FORCE_PATH = {"auto": _cabi.PATH_AUTO, "simt": _cabi.PATH_SIMT, "tc": _cabi.PATH_TC}[path]
 

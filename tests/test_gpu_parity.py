@@ -41,6 +41,14 @@ def run_operator(pkg, x, A, B, C, chunk, init=None, dY=None, dfinal=None, cache=
     return res
 
 
+@pytest.fixture
+def tensor_cores(pkg):
+    """The tensor-core kernels also for shapes that they are not chosen for."""
+    pkg.set_kernel_path("tc")
+    yield
+    pkg.set_kernel_path("auto")
+
+
 @pytest.mark.parametrize("name", REF_CASES)
 def test_fp32_against_reference_fixtures(pkg, cabi, name):
     g = load_golden(name)
@@ -170,9 +178,9 @@ def test_tensor_core_path_edge_shapes(pkg, cabi, oracle, batch, seqlen, heads, g
                                            (2, 200, 3, 64, 128, 1, 100), (3, 320, 4, 64, 64, 2, 80), (1, 256, 2, 40, 72, 1, 64),
                                            (2, 480, 5, 56, 40, 5, 96), (1, 1300, 2, 64, 128, 1, 650)])
 @pytest.mark.parametrize("states", [False, True])
-def test_tensor_core_path_partial_tiles(pkg, cabi, oracle, b, T, h, p, n, g, l, states):
-    """Sequences that end inside a tile, chunks that end anywhere, and heads narrower than the tile's 64 x 128 (bar as for
-    whole tiles: the rounding of the operands is the same)."""
+def test_tensor_core_path_partial_tiles(pkg, cabi, oracle, tensor_cores, b, T, h, p, n, g, l, states):
+    """Sequences that end inside a tile, chunks that end anywhere, and heads narrower than the tile's 64 x 128, on the
+    tensor-core kernels when they are asked for (bar as for whole tiles: the rounding of the operands is the same)."""
     cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, headdim=p, d_state=n, ngroups=g, chunk=l)
     assert pkg.resolved_path_name(cfg) == "tc"
     # (one position and no state: the decay acts on nothing, dA_head is 0 and an error relative to it is 0 / 0)
@@ -186,6 +194,22 @@ def test_tensor_core_path_partial_tiles(pkg, cabi, oracle, b, T, h, p, n, g, l, 
     y0, f0, _ = pkg.fused_ssd_scan(args[0], a, args[1], args[2], l)
     y1, f1, _ = pkg.fused_ssd_scan(args[0], a, args[1], args[2], l, None, cache)  # from the cached sums
     assert rel_err(y1, y0) < TOL_BF16 and rel_err(f1, f0) < TOL_BF16
+
+
+@pytest.mark.parametrize("b,T,h,p,n,g,l", [(2, 320, 3, 64, 128, 1, 80), (2, 127, 2, 64, 128, 2, 127), (1, 256, 4, 64, 64, 2, 64),
+                                           (2, 128, 2, 56, 128, 1, 64), (1, 384, 2, 64, 128, 1, 192)])
+def test_partial_tiles_keep_fp32_arithmetic(pkg, cabi, oracle, b, T, h, p, n, g, l):
+    """A bf16 call that does not fill whole tiles runs in fp32 unless the caller asks for the tensor cores: its fp32 outputs are
+    within the fp32 bar of the oracle in fp32 on the same inputs (bf16 operands would be 2e-3 off)."""
+    cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, headdim=p, d_state=n, ngroups=g, chunk=l)
+    assert pkg.resolved_path_name(cfg) == "simt"
+    inp = pkg.make_inputs(cfg, seed=13)
+    gen = torch.Generator().manual_seed(14)
+    init, dfinal = torch.randn(b, h, p, n, generator=gen) * 0.2, torch.randn(b, h, p, n, generator=gen)
+    got = mamba2_gpu(pkg, inp, l, init, dfinal)
+    want = oracle.mamba2_fwd_bwd(inp, l, torch.float32, init.unsqueeze(1), dfinal)
+    for k in ("final_state", "ddt", "dA_head", "dD", "dinit"):
+        assert got[k].dtype == torch.float32 and rel_err(got[k], want[k].reshape(got[k].shape)) < TOL_FP32, k
 
 
 @pytest.mark.parametrize("b,T,h,p,n,g,l", [(2, 3200, 6, 8, 16, 1, 64), (1, 128, 4, 100, 200, 2, 128), (1, 192, 2, 64, 256, 1, 96),
@@ -335,7 +359,7 @@ def test_saved_states_equal_recomputed_states(pkg, cabi):
 
 @pytest.mark.parametrize("b,T,h,g,p,n,chunk", [(1, 4096, 6, 2, 64, 128, 128), (1, 3008, 30, 5, 64, 64, 64), (2, 6016, 4, 4, 48, 128, 64),
                                                (1, 16384, 9, 1, 64, 128, 256)])
-def test_walks_in_pieces(pkg, cabi, oracle, b, T, h, g, p, n, chunk):
+def test_walks_in_pieces(pkg, cabi, oracle, tensor_cores, b, T, h, g, p, n, chunk):
     """Few (batch, head) pairs and a long sequence: the walks run in pieces side by side, seeded from summaries.  Several pieces, a
     short last piece, summaries in parts, states in and out, columns below the tile's; against the oracle, and the same whether
     the forward kept its states or the backward walks them again (bit for bit where a chunk is a tile; for other chunks the
