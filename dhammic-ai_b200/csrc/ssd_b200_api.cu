@@ -491,16 +491,21 @@ unsigned norm_blocks(size_t M, int rows_per_block, int most) {
 }
 
 // A warp per row up to 4 vectors a lane (512 fp32, 1024 bf16 columns), else the block; as few vectors a thread as the row needs.
+// `given`: the forward finds the rows' statistic in rstd.
 template <class T, bool GATED>
 void launch_norm_rows(bool backward, size_t M, int D, float eps, const T* x, const float* w, const T* z, const T* dout, T* out, T* dz, float* rstd,
-                      float* part, unsigned nb, cudaStream_t st) {
+                      float* part, bool given, unsigned nb, cudaStream_t st) {
     using namespace ssd::ew;
     const int vecs = D / VecOf<T>::N;
-#define SSD_NORM(TPR, NV)                                                                                                                    \
-    do {                                                                                                                                     \
-        const unsigned blocks = nb;                                                                        \
-        if (backward) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<blocks, TPR < 256 ? 256 : TPR, 0, st>>>(x, w, z, dout, rstd, out, dz, part, M, D))); \
-        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_fwd_kernel<T, TPR, NV, GATED><<<blocks, TPR < 256 ? 256 : TPR, 0, st>>>(x, w, z, out, rstd, M, D, eps))); \
+#define SSD_NORM(TPR, NV)                                                                                                           \
+    do {                                                                                                                            \
+        constexpr int threads = TPR < 256 ? 256 : TPR;                                                                              \
+        if (backward)                                                                                                               \
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<nb, threads, 0, st>>>(                \
+                x, w, z, dout, rstd, out, dz, part, M, D)));                                                                        \
+        else                                                                                                                        \
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_fwd_kernel<T, TPR, NV, GATED><<<nb, threads, 0, st>>>(                \
+                x, w, z, out, rstd, M, D, eps, given)));                                                                            \
     } while (0)
     if (vecs <= 32) SSD_NORM(32, 1);
     else if (vecs <= 64) SSD_NORM(32, 2);
@@ -519,11 +524,12 @@ int rmsnorm_impl(bool backward, size_t M, int D, float eps, const void* x, const
     constexpr int V = VecOf<T>::N;
     const bool vec = D % V == 0;
     const unsigned blocks = (unsigned)((M + 7) / 8);
-    if (rms_fits<T>(D) && !ysq && !any_unaligned({x, z, dout, out, dz})) {
+    if (rms_fits<T>(D) && !any_unaligned({x, z, dout, out, dz})) {
         const int vecs = D / V, most = backward ? kNormBwdBlocks : kNormFwdBlocks;
         const unsigned nb = norm_blocks(M, vecs <= 128 ? 8 : 1, vecs <= 256 ? most : vecs <= 512 ? most / 2 : most / 4);
-        if (z) launch_norm_rows<T, true>(backward, M, D, eps, (const T*)x, w, (const T*)z, (const T*)dout, (T*)out, (T*)dz, rstd, part_ws, nb, st);
-        else launch_norm_rows<T, false>(backward, M, D, eps, (const T*)x, w, nullptr, (const T*)dout, (T*)out, nullptr, rstd, part_ws, nb, st);
+        if (ysq) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, ysq_rstd_kernel<<<(unsigned)(M / 32), 256, 0, st>>>(ysq, ysq_heads, rstd, D, eps));
+        if (z) launch_norm_rows<T, true>(backward, M, D, eps, (const T*)x, w, (const T*)z, (const T*)dout, (T*)out, (T*)dz, rstd, part_ws, ysq, nb, st);
+        else launch_norm_rows<T, false>(backward, M, D, eps, (const T*)x, w, nullptr, (const T*)dout, (T*)out, nullptr, rstd, part_ws, ysq, nb, st);
         if (backward) SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_partial_rows_kernel<<<(D + 31) / 32, 256, 0, st>>>(part_ws, dw, (int)nb, D));
     } else if (!backward) {
         if (vec) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_fwd_kernel<T, V><<<blocks, 256, 0, st>>>((const T*)x, w, (const T*)z, (T*)out, rstd, M, D, eps, ysq, ysq_heads)));

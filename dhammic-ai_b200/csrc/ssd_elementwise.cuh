@@ -281,8 +281,9 @@ __device__ __forceinline__ float rms_sum(float v, float* red) {
 }
 
 template <class T, int TPR, int NV, bool GATED>
-__global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR : 1) rmsnorm_rows_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const T* __restrict__ z,
-                                                               T* __restrict__ out, float* __restrict__ rstd, size_t M, int D, float eps) {
+__global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR : 1)
+    rmsnorm_rows_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const T* __restrict__ z, T* __restrict__ out,
+                            float* __restrict__ rstd, size_t M, int D, float eps, bool given) {
     constexpr int V = VecOf<T>::N, RPB = TPR < 256 ? 256 / TPR : 1;
     __shared__ float red[2][32];
     const int sub = threadIdx.x % TPR;
@@ -296,24 +297,28 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
     const size_t step = (size_t)gridDim.x * RPB;
     size_t row = (size_t)blockIdx.x * RPB + threadIdx.x / TPR;
     RowVecs<T, NV> xn, zn;
-    if (row < M) {
-        xn.load(x + row * D, sub, TPR, D);
-        if (GATED) zn.load(z + row * D, sub, TPR, D);
-    }
+    float rn = 0.f;  // `given`: the statistic is there already (ysq_rstd_kernel)
+    auto fetch = [&](size_t r) {
+        if (r >= M) return;
+        xn.load(x + r * D, sub, TPR, D);
+        if (GATED) zn.load(z + r * D, sub, TPR, D);
+        if (given) rn = rstd[r];
+    };
+    fetch(row);
     for (int par = 0; row < M; row += step, par ^= 1) {  // (TPR = 256: uniform over the block; TPR = 32: over the warp)
         const RowVecs<T, NV> xc = xn, zc = zn;
-        if (row + step < M) {
-            xn.load(x + (row + step) * D, sub, TPR, D);
-            if (GATED) zn.load(z + (row + step) * D, sub, TPR, D);
+        float r = rn;
+        fetch(row + step);
+        if (!given) {
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+#pragma unroll
+                for (int q = 0; q < V; ++q) ss = fmaf(xc.at(i, q), xc.at(i, q), ss);
+            ss = rms_sum<TPR>(ss, red[par]);
+            r = rsqrtf(ss / (float)D + eps);
+            if (sub == 0) rstd[row] = r;
         }
-        float ss = 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i)
-#pragma unroll
-            for (int q = 0; q < V; ++q) ss = fmaf(xc.at(i, q), xc.at(i, q), ss);
-        ss = rms_sum<TPR>(ss, red[par]);
-        const float r = rsqrtf(ss / (float)D + eps);
-        if (sub == 0) rstd[row] = r;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int c = (sub + i * TPR) * V;
@@ -429,6 +434,35 @@ __global__ void __launch_bounds__(256) reduce_partial_rows_kernel(const float* _
     red[rl][cl] = s;
     __syncthreads();
     if (rl == 0 && c < D) out[c] = ((red[0][cl] + red[1][cl]) + (red[2][cl] + red[3][cl])) + ((red[4][cl] + red[5][cl]) + (red[6][cl] + red[7][cl]));
+}
+
+// The rows' statistic from the partial sums that the scan's forward leaves, [row / 128][head][half][row % 128] (sums of the fp32
+// values, before y is rounded to its storage type).  Block = 32 rows: lane = row, so that a read is 128 neighbouring bytes;
+// warp w adds the entries w, w + 8, w + 16, w + 24 modulo 32, and warp 0 the 32 sums of a row as the shuffles of
+// rmsnorm_fwd_kernel do (the threads that hold the row would read one sector per value).  Costs nothing against summing the
+// row in the norm itself: 750 and 757 us for forward + backward of the whole operator at (4, 4096, 64 heads).
+__global__ void __launch_bounds__(256) ysq_rstd_kernel(const float* __restrict__ ysq, int heads, float* __restrict__ rstd, int D, float eps) {
+    __shared__ float part[32][33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = 2 * heads;
+    const size_t row = (size_t)blockIdx.x * 32 + lane;
+    const float* p = ysq + (row >> 7) * (size_t)n * 128 + (row & 127);
+#pragma unroll
+    for (int l = warp; l < 32; l += 8) {
+        float s = 0.f;
+#pragma unroll 4
+        for (int i = l; i < n; i += 32) s += p[(size_t)i * 128];
+        part[l][lane] = s;
+    }
+    __syncthreads();
+    if (warp) return;
+    float v[32];
+#pragma unroll
+    for (int l = 0; l < 32; ++l) v[l] = part[l][lane];
+#pragma unroll
+    for (int of = 16; of > 0; of >>= 1)
+#pragma unroll
+        for (int l = 0; l < of; ++l) v[l] += v[l + of];
+    rstd[row] = rsqrtf(v[0] / (float)D + eps);
 }
 
 template <class T, int V>

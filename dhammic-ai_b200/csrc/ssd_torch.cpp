@@ -390,8 +390,8 @@ Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTenso
 
 // ---------------------------------------------------------------------------------------------------- scan + norm + gate
 // The scan followed by the block's output stage, out = rmsnorm(y over all heads) * silu(z)
-// (src/mamba_base_engine.py:189-191).  Up to 8192 columns the norm holds a row in registers and reads y once in any case; for
-// wider rows the forward walk leaves the per-half-row sums of y^2 behind, so that the norm need not read y twice.
+// (src/mamba_base_engine.py:189-191).  The forward walk leaves the per-half-row sums of y^2 behind, from its fp32 values: the
+// statistic carries no rounding of y to its storage type, and the norm reads y once however wide the row.
 struct GatedNode : ScanNode {
     SavedVariable y, z, w, rstd;
     at::ScalarType dt_type, A_type, D_type, z_type, w_type;
@@ -436,7 +436,7 @@ std::tuple<Tensor, Tensor> mamba2_gated(const Tensor& x, const Tensor& dt, const
         const int rp = ssd_b200_resolve_path(&probe);
         check(rp);
         Tensor ysq;
-        if (rp == SSD_B200_PATH_TC && T % 128 == 0 && Dn > 8192) ysq = empty_f32({rows * h * 2}, x);
+        if (rp == SSD_B200_PATH_TC && T % 128 == 0) ysq = empty_f32({rows * h * 2}, x);
         scan = scan_forward(s, chunk, o, {}, grad, ysq);
         zc = cast(z.contiguous(), x.scalar_type());
         w = f32(weight);

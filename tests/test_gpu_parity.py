@@ -557,6 +557,19 @@ def test_scan_with_gated_norm_output_stage(pkg, cabi, oracle, idx, batch, seqlen
     assert rel_err(out, o2) < (1e-2 if cfg.dtype == "bf16" else 1e-5)
 
 
+@pytest.mark.parametrize("h", [2, 24, 128, 130])
+def test_gated_norm_statistic_of_unrounded_values(pkg, cabi, h):
+    """The norm's statistic is of the scan's fp32 values: y = 1.0038 at every position rounds to 1 in bf16, its statistic does not,
+    and at silu(20) = 20 the two differ by a bf16 step (19.875 against 20).  Rows held in registers (up to 8192 columns) and not."""
+    bf, T = torch.bfloat16, 256
+    B = torch.zeros(1, T, 1, 128, dtype=bf, device=DEV)
+    x, z = torch.ones(1, T, h, 64, dtype=bf, device=DEV), torch.full((1, T, h * 64), 20.0, dtype=bf, device=DEV)
+    out, _ = pkg.ssd_mamba2_gated(x, torch.full((1, T, h), 0.01, device=DEV), torch.full((h,), -1.0, device=DEV), B, B,
+                                  torch.full((h,), 1.0038, device=DEV), z, torch.ones(h * 64, device=DEV), 1e-6, 128)
+    want = torch.nn.functional.silu(z.double()) * (1.0038 ** 2 + 1e-6) ** -0.5  # 19.924, no tie
+    assert torch.equal(out.flatten(), want.to(bf).flatten())
+
+
 def test_scaled_operator_form_matches_mamba2_form(pkg, cabi):
     """The scan's third calling form (log-decay a, input weight dt and skip coefficient all per position; what the
     one-scan Mamba-3 composition uses) against the Mamba-2 form with a = dt * A_head and skip = D on the same data:
