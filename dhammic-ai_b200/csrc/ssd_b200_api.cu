@@ -368,20 +368,30 @@ int m3_row_threads(int p) {
         }                                                                                                         \
     } while (0)
 
+// Running sums of the angles and rotation of whole vectors.
+template <class T, class TA>
+void m3_angles_and_rope(const ssd::Dims& d, int E, int nseg, const T* B, const T* C, const TA* ang, float* segsum, float* cum, T* Br, T* Cr,
+                        cudaStream_t st) {
+    using namespace ssd::m3;
+    constexpr int V = VecOf<T>::N, N = V / 2;
+    const unsigned gy = (E / N + 255) / 256;
+    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (angle_segsum_kernel<TA, N><<<dim3(nseg, gy, d.b), 256, 0, st>>>(ang, segsum, d.T, E)));
+    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, angle_prefix_kernel<<<dim3((E + 63) / 64, d.b), 64, 0, st>>>(segsum, nseg, E));
+    if (rope_walks_segments(d.b, d.T, E, N))
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_walk_fwd_kernel<T, TA, V, SEG><<<dim3(nseg, gy, d.b), 256, 0, st>>>(B, C, ang, segsum, cum, Br, Cr, d.T, d.h, d.g, d.n)));
+    else
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_walk_fwd_kernel<T, TA, V, 32><<<dim3((d.T + 31) / 32, gy, d.b), 256, 0, st>>>(B, C, ang, segsum, cum, Br, Cr, d.T, d.h, d.g, d.n)));
+}
+
 template <class T>
 int m3_fwd_impl(const ssd::Dims& d, const void* x, const float* dt, const float* lam, const float* A_head, const void* B,
                 const void* C, const void* ang, bool ang_f32, void* xw, float* dA, void* Br, void* Cr, float* sdot, float* cum,
                 float* segsum, const float* D, float* wout, float* skip, cudaStream_t st) {
     using namespace ssd::m3;
     const int E = d.h * (d.n / 2), nseg = (d.T + SEG - 1) / SEG;
-    if (d.n % VecOf<T>::N == 0 && !any_unaligned({B, C, ang, cum, Br, Cr})) {  // whole vectors
-        constexpr int V = VecOf<T>::N, N = V / 2;
-        const dim3 gw((d.T + WALK - 1) / WALK, (E / N + 255) / 256, d.b), gp((E + 63) / 64, d.b);
-        if (ang_f32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (angle_segsum_kernel<float, N><<<gw, 256, 0, st>>>((const float*)ang, cum, d.T, E)));
-        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (angle_segsum_kernel<T, N><<<gw, 256, 0, st>>>((const T*)ang, cum, d.T, E)));
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, angle_prefix_kernel<<<gp, 64, 0, st>>>(cum, d.T, E));
-        if (ang_f32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_walk_fwd_kernel<T, float, V><<<gw, 256, 0, st>>>((const T*)B, (const T*)C, (const float*)ang, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
-        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_walk_fwd_kernel<T, T, V><<<gw, 256, 0, st>>>((const T*)B, (const T*)C, (const T*)ang, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
+    if (d.n % VecOf<T>::N == 0 && !any_unaligned({B, C, ang, cum, Br, Cr, segsum})) {  // whole vectors
+        if (ang_f32) m3_angles_and_rope<T, float>(d, E, nseg, (const T*)B, (const T*)C, (const float*)ang, segsum, cum, (T*)Br, (T*)Cr, st);
+        else m3_angles_and_rope<T, T>(d, E, nseg, (const T*)B, (const T*)C, (const T*)ang, segsum, cum, (T*)Br, (T*)Cr, st);
     } else {
         const dim3 gs(nseg, (E + 255) / 256, d.b);
         if (ang_f32) {  // angles keep their own precision whatever the storage type of x, B and C

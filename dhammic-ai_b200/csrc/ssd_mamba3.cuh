@@ -126,32 +126,50 @@ __global__ void __launch_bounds__(256) scanT_apply_kernel(const TI* __restrict__
     }
 }
 
-// Both passes in one, from the last position to the first: a thread keeps one column's sum over the whole sequence, 32 loads
-// ahead of it.  Reads the input once instead of twice: 325 + 174 us -> 309 us at (16, 4096, 64 x 64) fp32 -> bf16.  Needs enough columns to
-// have the bytes in flight (kOnePassColumns); blocks of 64 threads, so that they spread evenly over the SMs.
+// Both passes in one, from the last position to the first: a thread keeps one column's sum over the segments behind (their
+// sums added one by one, as scanT_apply_kernel does: same order, same bits) and holds a segment's values, half of them in
+// registers and half in shared memory, while it adds them up in one direction and walks them in the other.  Reads the input
+// once instead of twice: 325 + 174 us -> 346 us at (16, 4096, 64 x 64) fp32 -> bf16.  Needs enough columns to have the bytes in
+// flight (kOnePassColumns); blocks of 64 threads, so that they spread evenly over the SMs and all of them are resident there.
 constexpr int kOnePassColumns = 148 * 256;
 template <class TO>
-__global__ void __launch_bounds__(64) scanT_rev_kernel(const float* __restrict__ in, TO* __restrict__ out, int Tlen, int E, float sign) {
+__global__ void __launch_bounds__(64, 8) scanT_rev_kernel(const float* __restrict__ in, TO* __restrict__ out, int Tlen, int E, float sign) {
+    constexpr int U = SEG / 2;
+    __shared__ float hi[U][64];
     const int e = blockIdx.x * 64 + threadIdx.x;
     if (e >= E) return;
     const size_t base = (size_t)blockIdx.y * Tlen * E + e;
-    constexpr int U = 32;
-    float run = 0.f, v[U];
-    auto fetch = [&](int t_hi) {  // positions t_hi - 1, t_hi - 2, ...
-#pragma unroll
-        for (int q = 0; q < U; ++q) v[q] = t_hi - 1 - q >= 0 ? in[base + (size_t)(t_hi - 1 - q) * E] : 0.f;
-    };
-    fetch(Tlen);
-    for (int t_hi = Tlen; t_hi > 0; t_hi -= U) {
-        float c[U];
-#pragma unroll
-        for (int q = 0; q < U; ++q) c[q] = v[q];
-        fetch(t_hi - U);
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-            run += c[q];
-            if (t_hi - 1 - q >= 0) out[base + (size_t)(t_hi - 1 - q) * E] = from_f<TO>(sign * run);
+    const uint32_t sh = (uint32_t)__cvta_generic_to_shared(&hi[0][threadIdx.x]);
+    float behind = 0.f;
+    for (int t0 = (Tlen - 1) / SEG * SEG; t0 >= 0; t0 -= SEG) {
+        const int rows = min(SEG, Tlen - t0);
+        const float* p = in + base + (size_t)t0 * E;
+#pragma unroll 16
+        for (int q = 0; q < U; ++q) {  // zeros behind the end
+            const int ok = U + q < rows ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sh + q * 256), "l"(p + (size_t)(ok ? U + q : 0) * E), "r"(ok) : "memory");
         }
+        float lo[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) lo[q] = q < rows ? p[(size_t)q * E] : 0.f;
+        asm volatile("cp.async.wait_all;" ::: "memory");  // (a thread reads only what it copied itself)
+        float s = 0.f, run = behind;
+#pragma unroll
+        for (int q = 0; q < U; ++q) s += lo[q];
+#pragma unroll 16
+        for (int q = 0; q < U; ++q) s += hi[q][threadIdx.x];
+        TO* o = out + base + (size_t)t0 * E;
+#pragma unroll 16
+        for (int q = U - 1; q >= 0; --q) {
+            run += hi[q][threadIdx.x];
+            if (U + q < rows) o[(size_t)(U + q) * E] = from_f<TO>(sign * run);
+        }
+#pragma unroll
+        for (int q = U - 1; q >= 0; --q) {
+            run += lo[q];
+            if (q < rows) o[(size_t)q * E] = from_f<TO>(sign * run);
+        }
+        behind += s;
     }
 }
 
@@ -240,65 +258,78 @@ __global__ void __launch_bounds__(256) rope_fwd_kernel(const T* __restrict__ B, 
 
 // The running sum of the angles and the rotation in one pass: a thread owns V columns of one head (V / 2 pairs) and walks
 // WALK positions, so that a block reads and writes 4 KB of every tensor per position (with blocks of 64-byte rows the same
-// bytes took twice as long) and the cumulative angle is written for the backward but not read back.
-// HBM-bound: at (16, 4096, 64 heads, 64 pairs) 138 + 333 + 531 us with a kernel for each step, 96 + 24 + 723 us now (5.6 TB/s).  The sum in front of
-// the positions of a block waits in the first of their rows of `cum` (angle_segsum_kernel, angle_prefix_kernel).  Needs whole vectors (n a multiple of V, 16-byte aligned angles).
-constexpr int WALK = 32;
+// bytes took twice as long) and the cumulative angle is written for the backward but not read back.  The sum starts from the
+// sums of the segments before (angle_segsum_kernel, angle_prefix_kernel) and runs through its segment one by one: the order, and
+// the bits, of scanT_segsum_kernel and scanT_apply_kernel.  Where whole segments are too few blocks (rope_walks_segments), blocks of
+// 32 positions first add up what lies before them in the segment.
+// HBM-bound: at (16, 4096, 64 heads, 64 pairs) 138 + 333 + 531 us with a kernel for each step, 87 + 5 + 722 us now.
+// Needs whole vectors (n a multiple of V, 16-byte aligned angles).
 template <class TA, int N>
 struct alignas(N * sizeof(TA)) AngleVec {
     TA v[N];
 };
 template <class TA, int N>
-__global__ void __launch_bounds__(256) angle_segsum_kernel(const TA* __restrict__ raw, float* __restrict__ cum, int Tlen, int E) {
+__global__ void __launch_bounds__(256) angle_segsum_kernel(const TA* __restrict__ raw, float* __restrict__ segsum, int Tlen, int E) {
     const int e = (blockIdx.y * 256 + threadIdx.x) * N;
     if (e >= E) return;
-    const int t0 = blockIdx.x * WALK, t1 = min(Tlen, t0 + WALK);
+    const int t0 = blockIdx.x * SEG, t1 = min(Tlen, t0 + SEG);
     const TA* p = raw + ((size_t)blockIdx.z * Tlen + t0) * E + e;
     AngleVec<float, N> s;
 #pragma unroll
     for (int q = 0; q < N; ++q) s.v[q] = 0.f;
-#pragma unroll 16
+#pragma unroll 32
     for (int t = t0; t < t1; ++t, p += E) {
         const AngleVec<TA, N> a = *reinterpret_cast<const AngleVec<TA, N>*>(p);
 #pragma unroll
         for (int q = 0; q < N; ++q) s.v[q] += to_f(a.v[q]);
     }
-    *reinterpret_cast<AngleVec<float, N>*>(cum + ((size_t)blockIdx.z * Tlen + t0) * E + e) = s;
+    store_angles<N>(segsum + ((size_t)blockIdx.z * gridDim.x + blockIdx.x) * E + e, s.v);
 }
-// In place, on the rows of the blocks' first positions: sum of all blocks before.
-__global__ void __launch_bounds__(64) angle_prefix_kernel(float* __restrict__ cum, int Tlen, int E) {
+// In place: the sum of all segments before.
+__global__ void __launch_bounds__(64) angle_prefix_kernel(float* __restrict__ segsum, int nseg, int E) {
     const int e = blockIdx.x * 64 + threadIdx.x;
     if (e >= E) return;
-    float* p = cum + (size_t)blockIdx.y * Tlen * E + e;
-    const int nseg = (Tlen + WALK - 1) / WALK;
-    const size_t step = (size_t)WALK * E;
+    float* p = segsum + (size_t)blockIdx.y * nseg * E + e;
     float run = 0.f;
     for (int s0 = 0; s0 < nseg; s0 += 16) {
         float v[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = s0 + q < nseg ? p[(size_t)(s0 + q) * step] : 0.f;
+        for (int q = 0; q < 16; ++q) v[q] = s0 + q < nseg ? p[(size_t)(s0 + q) * E] : 0.f;
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
-            if (s0 + q < nseg) p[(size_t)(s0 + q) * step] = run;
+            if (s0 + q < nseg) p[(size_t)(s0 + q) * E] = run;
             run += v[q];
         }
     }
 }
-template <class T, class TA, int V>
+// Whole segments per block from about four blocks per SM on.
+inline bool rope_walks_segments(int b, int T, int E, int N) {
+    return (long long)b * ((T + SEG - 1) / SEG) * ((E / N + 255) / 256) >= 4 * 148;
+}
+template <class T, class TA, int V, int WALK>
 __global__ void __launch_bounds__(256) rope_walk_fwd_kernel(const T* __restrict__ B, const T* __restrict__ C, const TA* __restrict__ raw,
-                                                            float* __restrict__ cum, T* __restrict__ Br, T* __restrict__ Cr,
-                                                            int Tlen, int h, int g, int n) {
+                                                            const float* __restrict__ segsum, float* __restrict__ cum, T* __restrict__ Br,
+                                                            T* __restrict__ Cr, int Tlen, int h, int g, int n) {
     constexpr int N = V / 2;
     const int upr = n / V, unit = blockIdx.y * 256 + threadIdx.x;  // vector of a position's h x n columns
     if (unit >= h * upr) return;
     const int hh = unit / upr, j0 = (unit - hh * upr) * V, E = h * n / 2;
-    const int t0 = blockIdx.x * WALK, t1 = min(Tlen, t0 + WALK);
+    const int t0 = blockIdx.x * WALK, t1 = min(Tlen, t0 + WALK), seg = t0 / SEG, nseg = (Tlen + SEG - 1) / SEG;
     const size_t bt = (size_t)blockIdx.z * Tlen + t0;
     const T* pB = B + (bt * g + hh / (h / g)) * n + j0;
     const T* pC = C + (bt * g + hh / (h / g)) * n + j0;
     const size_t a0 = bt * E + (size_t)unit * N, o0 = bt * h * n + (size_t)unit * V;
     float run[N];
-    load_angles<N>(cum + a0, run);  // left there by the prefix; overwritten below
+    load_angles<N>(segsum + ((size_t)blockIdx.z * nseg + seg) * E + (size_t)unit * N, run);
+    if (WALK < SEG) {
+        const TA* p = raw + a0 - (size_t)(t0 - seg * SEG) * E;
+#pragma unroll 16
+        for (int t = seg * SEG; t < t0; ++t, p += E) {
+            const AngleVec<TA, N> a = *reinterpret_cast<const AngleVec<TA, N>*>(p);
+#pragma unroll
+            for (int q = 0; q < N; ++q) run[q] += to_f(a.v[q]);
+        }
+    }
 #pragma unroll 4
     for (int i = 0; i < t1 - t0; ++i) {
         const AngleVec<TA, N> a = *reinterpret_cast<const AngleVec<TA, N>*>(raw + a0 + (size_t)i * E);

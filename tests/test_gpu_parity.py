@@ -466,6 +466,59 @@ def test_mamba3_angles_edges(pkg, cabi, oracle, T, h, g, n, chunk, ang32, shift)
     assert not bad, errs
 
 
+@pytest.mark.parametrize("T,h,n,b", [(300, 3, 24, 2), (1120, 40, 64, 9), (129, 5, 8, 1)])
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_mamba3_angle_sums_do_not_depend_on_the_route(pkg, cabi, T, h, n, b, dtype):
+    """The cumulative angles and the rotated B and C, from kernels that need aligned angles and from those that take any address:
+    the sums are taken in one order, so the bits are the same.  Blocks of whole segments (the second shape) and of 32 positions."""
+    import ctypes
+    lib, S = cabi.load(), pkg.ssd_scan
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    dt_ = torch.float32 if dtype == "fp32" else torch.bfloat16
+    g = 1
+    B, C = (torch.randn(b, T, g, n, generator=gen, device=DEV).to(dt_) for _ in range(2))
+    ang = (torch.randn(b, T, h, n // 2, generator=gen, device=DEV)).to(dt_)
+    shifted = torch.empty(ang.numel() + 1, dtype=dt_, device=DEV)[1:].view(ang.shape).copy_(ang)
+    assert shifted.data_ptr() % 16
+    dt, lam = torch.rand(b, T, h, generator=gen, device=DEV), torch.rand(b, T, h, generator=gen, device=DEV)
+    Ah = -torch.ones(h, device=DEV)
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.F32 if dtype == "fp32" else cabi.BF16, cabi.F32, cabi.PATH_AUTO, b, T, h, 64, n, g, T)
+    res = []
+    for a in (ang, shifted):
+        f = {k: torch.empty(b, T, h, device=DEV) for k in ("dA", "w", "skip")}
+        Br, Cr = torch.empty(b, T, h, n, dtype=dt_, device=DEV), torch.empty(b, T, h, n, dtype=dt_, device=DEV)
+        sdot, cum = torch.empty(b, T, g, device=DEV), torch.empty(b, T, h, n // 2, device=DEV)
+        seg = torch.empty(b * ((T + 127) // 128) * h * (n // 2), device=DEV)
+        P = S._ptr
+        cabi.check(lib.ssd_b200_m3_prologue_fwd(ctypes.byref(shape), P(B), P(dt), P(lam), P(Ah), P(B), P(C), P(a), shape.dtype, None, P(f["dA"]),
+                                                P(Br), P(Cr), P(sdot), P(cum), P(seg), None, P(f["w"]), P(f["skip"]), S._stream(torch.device(DEV))))
+        torch.cuda.synchronize()
+        res.append((cum, Br, Cr))
+    for x, y in zip(*res):
+        assert torch.equal(x, y)
+    want = -ang.double().cumsum(1)
+    assert rel_err(res[0][0], want) < TOL_FP32
+
+
+@pytest.mark.parametrize("T", [600, 128])
+def test_mamba3_angle_gradient_does_not_depend_on_the_batch(pkg, cabi, T):
+    """Many columns take the reverse sum of the angle gradients in one pass, few in two; the order of the sums, and so
+    the bits, are the same (a running sum over the whole sequence would round more the longer it is)."""
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    b, h, p, n = 10, 64, 8, 128  # 40,960 columns
+    def rand(*s):
+        return torch.rand(*s, generator=gen, device=DEV)
+    lv = [rand(b, T, h, p) - 0.5, 0.05 * rand(b, T, h), -rand(h), rand(b, T, 1, n) - 0.5, rand(b, T, 1, n) - 0.5, rand(h), 6 * rand(b, T, h, n // 2) - 3,
+          rand(b, T, h)]
+    dy = rand(b, T, h, p) - 0.5
+    def dang(k):
+        part = [t[:k].clone().requires_grad_(True) if t.shape[0] == b else t.clone().requires_grad_(True) for t in lv]
+        y = pkg.ssd_mamba3(*part, T // 8)
+        return y.detach(), torch.autograd.grad([y], [part[6]], [dy[:k]])[0]
+    (y0, d0), (y1, d1) = dang(b), dang(1)
+    assert torch.equal(y0[:1], y1) and torch.equal(d0[:1], d1)
+
+
 def test_mamba3_against_reference_fixture(pkg, cabi):
     """The one-scan Mamba-3 form on the GPU against outputs of the reference's own two-call composition
     (tests/golden/m3_reference_block.npz: reference rotation convention, coefficients and scan), fp32."""
