@@ -351,10 +351,11 @@ int m3_row_threads(int p) {
     const int tpr = p / V;
     return (tpr <= 32 && (tpr & (tpr - 1)) == 0) ? tpr : 0;
 }
-#define M3_ROW_DISPATCH(KERNEL, ...)                                                                              \
+// ALIGNED: whether the kernel's vectors start on 16-byte boundaries (else single elements)
+#define M3_ROW_DISPATCH(ALIGNED, KERNEL, ...)                                                                     \
     do {                                                                                                          \
         constexpr int V = ssd::m3::VecOf<T>::N;                                                                   \
-        const int tpr = m3_row_threads<T>(d.p);                                                                   \
+        const int tpr = (ALIGNED) ? m3_row_threads<T>(d.p) : 0;                                                   \
         const size_t thr = rows * (size_t)(tpr ? tpr : 32);                                                       \
         const unsigned blocks = (unsigned)((thr + 255) / 256);                                                    \
         switch (tpr) {                                                                                            \
@@ -406,7 +407,7 @@ int m3_fwd_impl(const ssd::Dims& d, const void* x, const float* dt, const float*
     const size_t grows = (size_t)d.b * d.T * d.g, rows = (size_t)d.b * d.T * d.h;
     SSD_LAUNCH(ssd::prof::K_TC_AUX, st, bc_dot_kernel<T><<<(unsigned)((grows + 7) / 8), 256, 0, st>>>((const T*)B, (const T*)C, sdot, d.n, grows));
     if (xw) {
-        M3_ROW_DISPATCH(xw_fwd_kernel, (const T*)x, dt, lam, A_head, (T*)xw, dA, d.T, d.h, d.p, rows);
+        M3_ROW_DISPATCH(!any_unaligned({x, xw}), xw_fwd_kernel, (const T*)x, dt, lam, A_head, (T*)xw, dA, d.T, d.h, d.p, rows);
     } else {  // the scan takes the weight and the skip coefficient per position: x is not touched here
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, coef_fwd_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(dt, lam, A_head, D, sdot, wout, dA, skip, d.T, d.h, d.hpg, rows));
     }
@@ -419,7 +420,7 @@ int m3_skip_impl(const ssd::Dims& d, const void* y_scan, const void* x, const fl
                  const float* sdot, void* y, cudaStream_t st) {
     using namespace ssd::m3;
     const size_t rows = (size_t)d.b * d.T * d.h;
-    M3_ROW_DISPATCH(skip_fwd_kernel, (const T*)y_scan, (const T*)x, D, dt, lam, sdot, (T*)y, d.T, d.h, d.hpg, d.p, rows);
+    M3_ROW_DISPATCH(!any_unaligned({y_scan, x, y}), skip_fwd_kernel, (const T*)y_scan, (const T*)x, D, dt, lam, sdot, (T*)y, d.T, d.h, d.hpg, d.p, rows);
     CUDA_LAUNCH_CHECK("mamba3 skip forward");
     return 0;
 }
@@ -433,8 +434,8 @@ int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* 
     const int E = d.h * (d.n / 2), nseg = (d.T + SEG - 1) / SEG;
     const size_t rows = (size_t)d.b * d.T * d.h;
     if (dxw)  // otherwise the scan's backward has already produced dx, dw and dyx (scaled operator form)
-        M3_ROW_DISPATCH(xw_bwd_kernel, (const T*)x, (const T*)dy, (const T*)dxw, dt, lam, D, sdot, (T*)dx, dw, dyx, d.T, d.h, d.hpg, d.p, rows);
-    if (d.n % VecOf<T>::N == 0) {
+        M3_ROW_DISPATCH(!any_unaligned({x, dy, dxw, dx}), xw_bwd_kernel, (const T*)x, (const T*)dy, (const T*)dxw, dt, lam, D, sdot, (T*)dx, dw, dyx, d.T, d.h, d.hpg, d.p, rows);
+    if (d.n % VecOf<T>::N == 0 && !any_unaligned({B, C, cum, dBr, dCr, dB, dC, dcum})) {
         const size_t items = (size_t)d.b * d.T * d.g * (d.n / VecOf<T>::N);
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_bwd_kernel<T, VecOf<T>::N><<<(unsigned)((items + 255) / 256), 256, 0, st>>>((const T*)B, (const T*)C, cum, (const T*)dBr, (const T*)dCr, dyx, dt, lam, (T*)dB, (T*)dC, dcum, d.T, d.h, d.g, d.n, items)));
     } else {
@@ -463,7 +464,7 @@ int rope_op_impl(bool backward, long long BT, int H, int D, int aH, const void* 
                  void* out, float* dang, cudaStream_t st) {
     using namespace ssd::ew;
     constexpr int V = VecOf<T>::N;
-    const bool vec = D % V == 0;
+    const bool vec = D % V == 0 && !any_unaligned({x, dy, out});  // (the angles are read one by one)
     if (!backward) {
         if (vec) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_op_fwd_kernel<T, V><<<(unsigned)BT, 256, 0, st>>>((const T*)x, ang, (T*)out, H, D, aH)));
         else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_op_fwd_kernel<T, 2><<<(unsigned)BT, 256, 0, st>>>((const T*)x, ang, (T*)out, H, D, aH)));
@@ -532,9 +533,9 @@ int rmsnorm_impl(bool backward, size_t M, int D, float eps, const void* x, const
                  int ysq_heads = 0) {
     using namespace ssd::ew;
     constexpr int V = VecOf<T>::N;
-    const bool vec = D % V == 0;
+    const bool aligned = !any_unaligned({x, z, dout, out, dz}), vec = D % V == 0 && aligned && !any_unaligned({w});
     const unsigned blocks = (unsigned)((M + 7) / 8);
-    if (rms_fits<T>(D) && !any_unaligned({x, z, dout, out, dz})) {
+    if (rms_fits<T>(D) && aligned && !any_unaligned({part_ws})) {  // (these read the weights one by one)
         const int vecs = D / V, most = backward ? kNormBwdBlocks : kNormFwdBlocks;
         const unsigned nb = norm_blocks(M, vecs <= 128 ? 8 : 1, vecs <= 256 ? most : vecs <= 512 ? most / 2 : most / 4);
         if (ysq) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, ysq_rstd_kernel<<<(unsigned)(M / 32), 256, 0, st>>>(ysq, ysq_heads, rstd, D, eps));

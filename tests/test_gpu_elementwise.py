@@ -204,3 +204,66 @@ def test_rmsnorm_module_swap(pkg, cabi):
     xk = x.clone().requires_grad_(True)
     pkg.FusedRMSNorm.apply(xk, mod.weight, EPS).sum().backward()
     assert xk.grad is not None and mod.weight.grad is not None
+
+
+def _shifted(t):
+    """The same values, starting one element behind a 16-byte boundary."""
+    out = torch.empty(t.numel() + 16, dtype=t.dtype, device=t.device)[1:t.numel() + 1].view(t.shape).copy_(t)
+    assert out.data_ptr() % 16 and out.is_contiguous()
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("who", ["x", "angles", "dy"])
+def test_rope_takes_any_address(pkg, cabi, dtype, who):
+    """Tensors off the 16-byte boundaries of the vector accesses: same results (single-element accesses, same arithmetic)."""
+    x, angles = _rope_inputs(2, 40, 3, 64, dtype, seed=3, per_head=True)
+    dy = torch.randn_like(x)
+    def run(*ts):
+        lv = [t.detach().requires_grad_(True) for t in ts[:2]]
+        y = pkg.fused_rope(*lv)
+        return [y.detach()] + list(torch.autograd.grad([y], lv, [ts[2]]))
+    want = run(x, angles, dy)
+    got = run(*[_shifted(t) if n == who else t for n, t in zip(("x", "angles", "dy"), (x, angles, dy))])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [256, 8200, 100])
+@pytest.mark.parametrize("who", ["x", "z", "weight", "dy"])
+def test_gate_norm_takes_any_address(pkg, cabi, dtype, D, who):
+    """The gated norm with one tensor off the 16-byte boundaries: as aligned, up to the order of the sums over a row (fp32: a few
+    1e-7 of the largest value; bf16: one step of the storage type)."""
+    g = torch.Generator(device=DEV).manual_seed(D)
+    t = {"x": torch.randn(3, 21, D, generator=g, device=DEV).to(dtype), "z": torch.randn(3, 21, D, generator=g, device=DEV).to(dtype),
+         "weight": torch.randn(D, generator=g, device=DEV) * 0.5 + 1, "dy": torch.randn(3, 21, D, generator=g, device=DEV).to(dtype)}
+    def run(t):
+        lv = [t[k].detach().requires_grad_(True) for k in ("x", "z", "weight")]
+        y = pkg.fused_gate_norm(*lv, EPS)
+        return [y.detach()] + list(torch.autograd.grad([y], lv, [t["dy"]]))
+    want = run(t)
+    got = run({k: _shifted(v) if k == who else v for k, v in t.items()})
+    tol = 2e-6 if dtype == torch.float32 else 2 ** -7
+    for a, b in zip(got, want):
+        assert float((a.float() - b.float()).abs().max()) <= tol * float(b.float().abs().max())
+
+
+@pytest.mark.parametrize("D", [256, 8200])
+def test_rmsnorm_backward_takes_any_workspace_address(pkg, cabi, D):
+    """The scratch of ssd_b200_rmsnorm_bwd needs no more than the alignment of its floats."""
+    S, lib, rows = pkg.ssd_scan, cabi.load(), 37
+    g = torch.Generator(device=DEV).manual_seed(D)
+    x, dy, w = torch.randn(rows, D, generator=g, device=DEV), torch.randn(rows, D, generator=g, device=DEV), torch.rand(D, generator=g, device=DEV) + 0.5
+    rstd = torch.rsqrt(x.pow(2).mean(1) + EPS)
+    n = int(lib.ssd_b200_rmsnorm_ws_floats(rows, D))
+    res = []
+    for off in (0, 1):
+        ws, dx, dw = torch.full((n + 2,), float("nan"), device=DEV), torch.empty_like(x), torch.empty_like(w)
+        cabi.check(lib.ssd_b200_rmsnorm_bwd(cabi.F32, rows, D, S._ptr(x), S._ptr(w), None, S._ptr(dy), S._ptr(rstd), S._ptr(dx), None, S._ptr(dw),
+                                            S._ptr(ws[off:]), S._stream(torch.device(DEV))))
+        torch.cuda.synchronize()
+        assert torch.isnan(ws[n + off:]).all()
+        res.append((dx, dw))
+    for a, b in zip(*res):
+        assert float((a - b).abs().max()) <= 2e-6 * float(b.abs().max())
