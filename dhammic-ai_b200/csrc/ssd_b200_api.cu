@@ -630,6 +630,7 @@ int ssd_b200_fwd(const ssd_b200_fwd_args* a, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if ((uintptr_t)a->states & 15) return fail(SSD_B200_EINVAL, "`states` must be 16-byte aligned");
     if (a->ysq && path != SSD_B200_PATH_TC) return fail(SSD_B200_EINVAL, "`ysq` is only written by the tensor-core path");
+    if (a->ysq && a->shape.seqlen % ssd::tc::LT) return fail(SSD_B200_EINVAL, "`ysq` needs a sequence of whole tiles of 128 positions");
     if (form == 3 && path != SSD_B200_PATH_TC) return fail(SSD_B200_EUNSUPPORTED, "the scaled operator form needs the tensor-core path");
     if (path == SSD_B200_PATH_TC) return ssd::tc::forward(a, dims_of(a->shape), st, g_err, sizeof(g_err));
     return a->shape.dtype == SSD_B200_BF16 ? simt_fwd<__nv_bfloat16>(a, st) : simt_fwd<float>(a, st);

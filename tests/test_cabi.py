@@ -7,6 +7,7 @@ import sys
 from pathlib import Path
 
 import pytest
+import torch
 
 ROOT = Path(__file__).resolve().parents[1]
 HEADER = ROOT / "include" / "ssd_b200.h"
@@ -74,8 +75,21 @@ def test_host_validation_without_gpu(cabi):
     assert lib.ssd_b200_bwd(None, None) == cabi.EINVAL
 
 
+@pytest.mark.parametrize("T,refused", [(64, True), (192, True), (128, False)])
+def test_row_sums_of_squares_need_whole_tiles(cabi, T, refused):
+    """`ysq` holds one entry per position of whole 128-position tiles; a sequence that ends inside a tile would be written past
+    it.  The call is refused on the host (and where it is not, it ends for want of a GPU, not of a check)."""
+    if torch.cuda.is_available():
+        pytest.skip("the accepted case would run with pointers that are none")
+    lib = cabi.load()
+    s = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_TC, 2, T, 2, 64, 128, 1, 64)
+    p = 4096
+    a = cabi.FwdArgs(s, p, None, p, p, p, p, p, None, p, p, p, 0, 0, p, 1 << 40, None, None, p, None)
+    rc = lib.ssd_b200_fwd(C.byref(a), None)
+    assert rc < 0 and (rc == cabi.EINVAL and "whole tiles" in cabi.last_error()) == refused
+
+
 def test_operator_rejects_cpu_tensors(pkg, cabi):
-    import torch
     x = torch.zeros(1, 64, 2, 8)
     with pytest.raises(AssertionError):
         pkg.fused_ssd_scan(x, torch.zeros(1, 64, 2), torch.zeros(1, 64, 2, 4), torch.zeros(1, 64, 2, 4), 32)
