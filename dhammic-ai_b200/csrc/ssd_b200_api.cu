@@ -118,7 +118,7 @@ bool simt_supported(const ssd_b200_shape& s, const char** why) {
 
 int resolve_path(const ssd_b200_shape& s) {
     const char* why = "";
-    const bool tc = ssd::tc::supported(s.dtype, (int)s.headdim, (int)s.dstate, (int)s.chunk, (int)s.nheads);
+    const bool tc = ssd::tc::supported(s.dtype, (int)s.headdim, (int)s.dstate);
     if (s.path == SSD_B200_PATH_TC) {
         if (!tc) return fail(SSD_B200_EUNSUPPORTED, "tensor-core path does not cover this shape/dtype");
         return SSD_B200_PATH_TC;

@@ -40,9 +40,8 @@ constexpr int PANEL = 16384;  // bytes of one [128 rows][64 bf16] swizzled panel
 // What the kernels can run: shapes below the tile's own size are padded on chip, TMA fills what lies behind the end of a
 // sequence, or behind a head's last column, with zeros, and does not write it.  (A row of p or n bf16 values has to be a
 // multiple of 16 bytes for that.)
-inline bool supported(int dtype, int p, int n, int l, int h) {
-    return dtype == 1 && p > HP / 2 && p <= HP && p % 8 == 0 && n > DN / 4 && n <= DN && n % 8 == 0 &&
-           (l <= kFusedChunkMax || (long long)l * (h + 1) * 4 <= 227 * 1024);
+inline bool supported(int dtype, int p, int n) {
+    return dtype == 1 && p > HP / 2 && p <= HP && p % 8 == 0 && n > DN / 4 && n <= DN && n % 8 == 0;
 }
 // What they are chosen for.  Operands of the products (the masked scores, the weighted x, the states a tile starts from) are
 // rounded to bf16 here and are fp32 in the SIMT kernels.  Calls that fill whole tiles take that rounding; for others it is the

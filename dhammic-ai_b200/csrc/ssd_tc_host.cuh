@@ -242,6 +242,8 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     } else {
         if (!a->cumsum_is_input) {
             const size_t sm = (size_t)d.l * (d.h + 1) * 4;
+            if (sm > 227 * 1024)  // (with a_cumsum given, a chunk can have any length)
+                SSD_TC_FAIL(SSD_B200_EUNSUPPORTED, "chunk * nheads too large for the cumsum tile");
             if (sm > 48 * 1024 &&
                 cudaFuncSetAttribute(chunk_cumsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
                 SSD_TC_FAIL(SSD_B200_ECUDA, "chunk_cumsum: set shared memory size failed");

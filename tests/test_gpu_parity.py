@@ -212,6 +212,25 @@ def test_partial_tiles_keep_fp32_arithmetic(pkg, cabi, oracle, b, T, h, p, n, g,
         assert got[k].dtype == torch.float32 and rel_err(got[k], want[k].reshape(got[k].shape)) < TOL_FP32, k
 
 
+def test_cached_call_takes_any_chunk(pkg, cabi):
+    """With the sums given, nothing bounds the chunk (2048 positions of 32 heads are too many for the kernel that makes the sums,
+    which is refused); same result as with chunks of 128."""
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=2048, nheads=32, ngroups=2, chunk=2048)
+    inp = pkg.make_inputs(cfg, seed=4)
+    a = (inp["dt"] * inp["A_head"]).to(DEV)
+    x, B, C, dy = (inp[k].to(DEV) for k in ("x", "B", "C", "dy"))
+    with pytest.raises(NotImplementedError, match="too large for the cumsum tile"):
+        pkg.fused_ssd_scan(x, a, B, C, 2048)
+    res = []
+    for l in (128, 2048):
+        cum = a.view(1, 2048 // l, l, 32).cumsum(2).permute(0, 3, 1, 2).contiguous()
+        lv = [t.detach().requires_grad_(True) for t in (x, B, C)]
+        y, fs, _ = pkg.fused_ssd_scan(lv[0], a, lv[1], lv[2], l, None, {"A_cumsum": cum})
+        res.append([y.detach(), fs] + list(torch.autograd.grad([y], lv, [dy])))
+    for u, v in zip(*res):
+        assert rel_err(u, v) < TOL_BF16
+
+
 @pytest.mark.parametrize("b,T,h,p,n,g,l", [(2, 3200, 6, 8, 16, 1, 64), (1, 128, 4, 100, 200, 2, 128), (1, 192, 2, 64, 256, 1, 96),
                                            (1, 64, 8, 65, 8, 2, 16), (2, 256, 12, 40, 65, 2, 128)])
 def test_fp32_head_splits_and_wide_states(pkg, cabi, oracle, b, T, h, p, n, g, l):
