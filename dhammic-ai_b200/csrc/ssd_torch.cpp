@@ -86,6 +86,15 @@ void check_inputs(const Tensor& x, const Tensor& B, const Tensor& C) {
                       B.sizes(), ", C ", C.sizes());
     TORCH_CHECK(x.scalar_type() == B.scalar_type() && B.scalar_type() == C.scalar_type(),
                 "expected x, B and C to have the same dtype, got ", x.scalar_type(), ", ", B.scalar_type(), ", ", C.scalar_type());
+    TORCH_CHECK_VALUE(B.device() == x.device() && C.device() == x.device(), "x, B and C are on different devices");
+}
+
+// A tensor whose values a kernel reads by x's sizes: on x's device, and with as many values as those sizes have.
+void check_like(const char* name, const Tensor& t, const Tensor& x, int64_t numel) {
+    if (!t.defined()) return;
+    SSD_ASSERT(t.is_cuda(), "ssd_b200 runs on CUDA tensors only (no CPU fallback): ", name);
+    TORCH_CHECK_VALUE(t.device() == x.device(), name, " is on ", t.device(), ", x on ", x.device());
+    TORCH_CHECK_VALUE(t.numel() == numel, name, " has shape ", t.sizes(), ": expected ", numel, " values for x ", x.sizes());
 }
 
 ssd_b200_shape make_shape(const Tensor& x, int a_dtype, const Tensor& B, int64_t chunk, int path) {
@@ -107,6 +116,14 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
     for (const Tensor* t : ts)
         if (t->defined() && t->requires_grad()) return true;
     return false;
+}
+
+// The per-position and per-head arguments of the forms with dt and A_head.
+void check_coefficients(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Tensor& D, const Tensor& init, int64_t n) {
+    check_like("dt", dt, x, x.size(0) * x.size(1) * x.size(2));
+    check_like("A_head", A_head, x, x.size(2));
+    check_like("D", D, x, x.size(2));
+    check_like("initial_states", init, x, x.size(0) * x.size(2) * x.size(3) * n);
 }
 
 // The inputs of one scan in the form the kernels read (see ssd_b200_fwd_args for the forms), and what its forward leaves.
@@ -253,6 +270,7 @@ std::tuple<Tensor, Tensor> mamba2(const Tensor& x, const Tensor& dt, const Tenso
     const Options o{path, save_states, status};
     const Tensor D = get(D_), init = get(init_);
     check_inputs(x, B, C);
+    check_coefficients(x, dt, A_head, D, init, B.size(3));
     c10::cuda::CUDAGuard guard(x.device());
     const bool grad = wants_grad({&x, &dt, &A_head, &B, &C, &D, &init});
     Scan s;
@@ -298,7 +316,9 @@ std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& 
     const Options o{path, save_states, status};
     const Tensor init = get(init_);
     check_inputs(x, B, C);
-    SSD_ASSERT(A.is_cuda(), "ssd_b200 runs on CUDA tensors only (no CPU fallback)");
+    check_like("A", A, x, x.size(0) * x.size(1) * x.size(2));
+    check_like("initial_states", init, x, x.size(0) * x.size(2) * x.size(3) * B.size(3));
+    check_like("A_cumsum", get(cum_in), x, x.size(0) * x.size(1) * x.size(2));
     c10::cuda::CUDAGuard guard(x.device());
     const bool grad = wants_grad({&x, &A, &B, &C, &init});
     Scan s;
@@ -331,7 +351,7 @@ struct NormGrads {
     Tensor dx, dz, dw;
 };
 NormGrads norm_backward(const Tensor& x, const Tensor& w, const Tensor& z, const Tensor& dout, const Tensor& rstd) {
-    const int64_t D = w.size(0), rows = x.numel() / D;
+    const int64_t D = w.numel(), rows = rstd.numel();
     NormGrads g{at::empty_like(x), z.defined() ? at::empty_like(z) : Tensor(), empty_f32({D}, x)};
     const Tensor ws = empty_f32({ws_floats(ssd_b200_rmsnorm_ws_floats(rows, D))}, x);
     check(ssd_b200_rmsnorm_bwd(dtype_code(x), rows, D, ptr(x), ptr<float>(w), ptr(z), ptr(dout), ptr<float>(rstd), ptr(g.dx), ptr(g.dz),
@@ -365,6 +385,8 @@ Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTenso
     const int64_t D = x.size(-1);
     SSD_ASSERT(weight.dim() == 1 && weight.size(0) == D, "weight shape ", weight.sizes(), " mismatches D=", D);
     if (z.defined()) SSD_ASSERT(z.is_cuda() && z.sizes() == x.sizes(), "gate shape ", z.sizes(), " vs x ", x.sizes());
+    check_like("weight", weight, x, D);
+    check_like("gate", z, x, x.numel());
     c10::cuda::CUDAGuard guard(x.device());
     Tensor xc, zc, w, out, rstd;
     {
@@ -395,7 +417,7 @@ Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTenso
 struct GatedNode : ScanNode {
     SavedVariable y, z, w, rstd;
     at::ScalarType dt_type, A_type, D_type, z_type, w_type;
-    std::vector<int64_t> init_shape, z_shape;
+    std::vector<int64_t> init_shape, z_shape, w_shape;
     std::string name() const override { return "SSDMamba2GatedBackward"; }
     void release_variables() override {
         ScanNode::release_variables();
@@ -409,7 +431,7 @@ struct GatedNode : ScanNode {
         const NormGrads n = norm_backward(y.unpack(), w.unpack(), z.unpack(), dout, rstd.unpack());
         const ScanGrads g = scan_backward(s, opt, n.dx, dfinal_of(grads[1]), false);
         return {g.dx, cast(g.ddt, dt_type), cast(g.dA_head, A_type), g.dB, g.dC, cast(g.dD, D_type), cast(n.dz.view(z_shape), z_type),
-                cast(n.dw, w_type), g.dinit.defined() ? g.dinit.view(init_shape) : Tensor()};
+                cast(n.dw.view(w_shape), w_type), g.dinit.defined() ? g.dinit.view(init_shape) : Tensor()};
     }
 };
 
@@ -419,6 +441,9 @@ std::tuple<Tensor, Tensor> mamba2_gated(const Tensor& x, const Tensor& dt, const
     const Options o{path, save_states, status};
     const Tensor D = get(D_), init = get(init_);
     check_inputs(x, B, C);
+    check_coefficients(x, dt, A_head, D, init, B.size(3));
+    check_like("norm_weight", weight, x, x.size(2) * x.size(3));
+    check_like("z", z, x, x.numel());
     SSD_ASSERT(z.is_cuda() && z.dim() >= 2 && z.size(0) == x.size(0) && z.size(1) == x.size(1) && z.numel() == x.numel(),
                "the gate must have the size of y: ", z.sizes(), " vs ", x.sizes());
     c10::cuda::CUDAGuard guard(x.device());
@@ -456,6 +481,7 @@ std::tuple<Tensor, Tensor> mamba2_gated(const Tensor& x, const Tensor& dt, const
         node->dt_type = dt.scalar_type(); node->A_type = A_head.scalar_type();
         node->z_type = z.scalar_type(); node->w_type = weight.scalar_type();
         node->z_shape = z.sizes().vec();
+        node->w_shape = weight.sizes().vec();
         if (D.defined()) node->D_type = D.scalar_type();
         if (init.defined()) node->init_shape = init.sizes().vec();
         torch::autograd::set_history(out, node);
@@ -516,7 +542,11 @@ Tensor mamba3(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Ten
               const Tensor& lam, int64_t chunk, int path, bool save_states, bool status) {
     const Options o{path, save_states, status};
     const Tensor D = get(D_);
-    SSD_ASSERT(x.is_cuda(), "ssd_b200 runs on CUDA tensors only (no CPU fallback)");
+    check_inputs(x, B, C);
+    check_coefficients(x, dt, A_head, D, {}, B.size(3));
+    check_like("lam", lam, x, x.size(0) * x.size(1) * x.size(2));
+    TORCH_CHECK_VALUE(B.size(3) % 2 == 0, "d_state must be even for the pairwise rotation, got ", B.size(3));
+    check_like("raw_angles", raw_angles, x, x.size(0) * x.size(1) * x.size(2) * (B.size(3) / 2));
     c10::cuda::CUDAGuard guard(x.device());
     const bool grad = wants_grad({&x, &dt, &A_head, &B, &C, &D, &raw_angles, &lam});
     const int64_t b = x.size(0), T = x.size(1), h = x.size(2), g = B.size(2), n = B.size(3);
@@ -608,6 +638,7 @@ Tensor rope(const Tensor& x, const Tensor& angles) {
     SSD_ASSERT(angles.size(0) == B && angles.size(1) == T && angles.size(3) == D / 2, "angles ", angles.sizes(), " do not fit x ", x.sizes(),
                ": want (", B, ", ", T, ", 1 or ", H, ", ", D / 2, ")");
     SSD_ASSERT(aH == 1 || aH == H, "angles carry ", aH, " heads; give 1 (shared by all heads) or ", H, " (one set per head)");
+    check_like("angles", angles, x, B * T * aH * (D / 2));
     c10::cuda::CUDAGuard guard(x.device());
     Tensor xc, ang, out;
     {
@@ -662,6 +693,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> trapezoid(const Tensor& dt_raw, const
     const int64_t H = dt_raw.size(-1);
     SSD_ASSERT(dt_bias.dim() == 1 && dt_bias.size(0) == H, "dt_bias must be (", H, ",), got ", dt_bias.sizes());
     SSD_ASSERT(A_log.dim() == 1 && A_log.size(0) == H, "A_log must be (", H, ",), got ", A_log.sizes());
+    check_like("lam_raw", lam_raw, dt_raw, dt_raw.numel());
+    check_like("dt_bias", dt_bias, dt_raw, H);
+    check_like("A_log", A_log, dt_raw, H);
     c10::cuda::CUDAGuard guard(dt_raw.device());
     Tensor d, l, bias, alog, o[4];
     {

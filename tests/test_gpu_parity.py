@@ -290,6 +290,69 @@ def test_error_behaviour_on_gpu(pkg, cabi):
         pkg.fused_ssd_scan(x[:, :64], A[:, :64], B[:, :64].bfloat16(), B[:, :64], 64)
 
 
+def _scan_args(b=2, T=128, h=2, p=64, n=128, g=1, dtype=torch.bfloat16):
+    gen = torch.Generator(device=DEV).manual_seed(b + T + h)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    return {"x": randn(b, T, h, p).to(dtype), "dt": 0.1 * torch.rand(b, T, h, generator=gen, device=DEV), "A_head": -torch.ones(h, device=DEV),
+            "B": (0.1 * randn(b, T, g, n)).to(dtype), "C": (0.1 * randn(b, T, g, n)).to(dtype), "D": randn(h)}
+
+
+def _call(pkg, op, a):
+    if op == "mamba2":
+        return pkg.ssd_mamba2(*[a[k] for k in ("x", "dt", "A_head", "B", "C", "D")], 64, a.get("init"))
+    if op == "operator":
+        cache = {"A_cumsum": a["cum"]} if "cum" in a else None
+        return pkg.fused_ssd_scan(a["x"], a["dt"], a["B"], a["C"], 64, a.get("init"), cache)[:2]
+    if op == "gated":
+        return pkg.ssd_mamba2_gated(*[a[k] for k in ("x", "dt", "A_head", "B", "C", "D", "z", "weight")], 1e-6, 64, a.get("init"))
+    return (pkg.ssd_mamba3(*[a[k] for k in ("x", "dt", "A_head", "B", "C", "D", "angles", "lam")], 64),)
+
+
+def _op_args(op, **kw):
+    a = _scan_args(**kw)
+    b, T, h, p = a["x"].shape
+    n = a["B"].shape[3]
+    if op == "gated":
+        a.update(z=torch.ones(b, T, h * p, dtype=a["x"].dtype, device=DEV), weight=torch.ones(h * p, device=DEV))
+    if op == "mamba3":
+        a.update(angles=torch.ones(b, T, h, n // 2, dtype=a["x"].dtype, device=DEV), lam=torch.full((b, T, h), 0.5, device=DEV))
+    return a
+
+
+@pytest.mark.parametrize("op,arg,bad", [
+    ("mamba2", "dt", (2, 64, 2)), ("mamba2", "A_head", (1,)), ("mamba2", "D", (1,)), ("mamba2", "init", (1, 2, 64, 128)), ("mamba2", "dt", "cpu"),
+    ("operator", "dt", (2, 128, 1)), ("operator", "init", (2, 1, 2, 64, 64)), ("operator", "cum", (2, 2, 1, 64)), ("operator", "cum", "cpu"),
+    ("gated", "weight", (64,)), ("gated", "weight", "cpu"), ("gated", "z", (2, 128, 64)), ("gated", "A_head", (1,)),
+    ("mamba3", "angles", (2, 128, 2, 32)), ("mamba3", "lam", (2, 64, 2)), ("mamba3", "D", (1,)), ("mamba3", "dt", (2, 128, 1)), ("mamba3", "angles", "cpu"),
+    ("mamba3", "C", (2, 128, 1, 64)), ("mamba3", "B", "fp32")])
+def test_arguments_that_are_too_small_are_refused(pkg, cabi, op, arg, bad):
+    """Kernels read these by x's sizes: what is shorter, of another type or on another device ends in an exception before any launch."""
+    a = _op_args(op)
+    good = a.get(arg, torch.zeros(2, 2, 2, 64, device=DEV))
+    a[arg] = good.cpu() if bad == "cpu" else good.float() if bad == "fp32" else torch.zeros(*bad, dtype=good.dtype, device=DEV)
+    before = cabi.launch_count()
+    with pytest.raises((ValueError, AssertionError, RuntimeError)):
+        _call(pkg, op, a)
+    assert cabi.launch_count() == before
+
+
+def test_gated_norm_weight_per_head(pkg, cabi):
+    """A weight of shape (heads, headdim) is the flat one, forward and backward (its gradient has its shape)."""
+    a = _op_args("gated", h=3)
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    w = torch.rand(3, 64, generator=gen, device=DEV)
+    res = []
+    for weight in (w.flatten(), w):
+        a["weight"] = weight.clone().requires_grad_(True)
+        a["x"] = a["x"].detach().requires_grad_(True)
+        out = _call(pkg, "gated", a)[0]
+        res.append([out.detach()] + list(torch.autograd.grad(out.float().square().sum(), [a["weight"], a["x"]])))
+    assert res[1][1].shape == (3, 64)
+    for u, v in zip(*res):
+        assert torch.equal(u.flatten(), v.flatten())
+
+
 def test_noncontiguous_inputs_and_determinism(pkg, cabi):
     """The caller passes products and padded views (src/mamba_base_engine.py:170-181); results are
     bitwise reproducible run to run."""
