@@ -12,8 +12,10 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 
 #include "../../include/ssd_b200.h"
 
@@ -217,18 +219,30 @@ struct SavedScan {
     }
 };
 
-// Nodes share the once-released guard: a second backward through a freed graph is reported as torch reports it.
-struct ScanNode : Node {
-    SavedScan saved;
-    Options opt{};
+// A node with saved variables.  Two threads can run backward through one graph, so unpacking and releasing take the node's lock; a
+// second backward through a freed graph is reported as torch reports it.
+struct SavingNode : Node {
     bool released = false;
+    virtual void release_saved() = 0;
     void release_variables() override {
-        saved.release();
+        std::lock_guard<std::mutex> lock(mutex_);
+        release_saved();
         released = true;
     }
-    Scan load() {
+    // What `unpack` returns: the saved tensors, taken out while nobody releases them.
+    template <class F>
+    auto unpacked(F&& unpack) {
+        std::lock_guard<std::mutex> lock(mutex_);
         TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-        return saved.load();
+        return unpack();
+    }
+};
+struct ScanNode : SavingNode {
+    SavedScan saved;
+    Options opt{};
+    void release_saved() override { saved.release(); }
+    Scan load() {
+        return unpacked([&] { return saved.load(); });
     }
 };
 
@@ -359,22 +373,19 @@ NormGrads norm_backward(const Tensor& x, const Tensor& w, const Tensor& z, const
     return g;
 }
 
-struct NormNode : Node {
+struct NormNode : SavingNode {
     SavedVariable x, w, z, rstd;
     at::ScalarType w_type, z_type;
-    bool released = false;
     std::string name() const override { return "FusedRMSNormBackward"; }
-    void release_variables() override {
+    void release_saved() override {
         for (SavedVariable* v : {&x, &w, &z, &rstd}) v->reset_data();
-        released = true;
     }
     variable_list apply(variable_list&& grads) override {
         if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         at::NoGradGuard no_grad;
-        const Tensor xv = x.unpack(), zv = z.unpack();
+        const auto [xv, wv, zv, rv] = unpacked([&] { return std::tuple(x.unpack(), w.unpack(), z.unpack(), rstd.unpack()); });
         c10::cuda::CUDAGuard guard(xv.device());
-        const NormGrads g = norm_backward(xv, w.unpack(), zv, cast(grads[0].contiguous(), xv.scalar_type()), rstd.unpack());
+        const NormGrads g = norm_backward(xv, wv, zv, cast(grads[0].contiguous(), xv.scalar_type()), rv);
         return {g.dx, cast(g.dw, w_type), cast(g.dz, z_type)};
     }
 };
@@ -419,16 +430,16 @@ struct GatedNode : ScanNode {
     at::ScalarType dt_type, A_type, D_type, z_type, w_type;
     std::vector<int64_t> init_shape, z_shape, w_shape;
     std::string name() const override { return "SSDMamba2GatedBackward"; }
-    void release_variables() override {
-        ScanNode::release_variables();
+    void release_saved() override {
+        ScanNode::release_saved();
         for (SavedVariable* v : {&y, &z, &w, &rstd}) v->reset_data();
     }
     variable_list apply(variable_list&& grads) override {
         at::NoGradGuard no_grad;
-        const Scan s = load();
+        const auto [s, yv, wv, zv, rv] = unpacked([&] { return std::tuple(saved.load(), y.unpack(), w.unpack(), z.unpack(), rstd.unpack()); });
         c10::cuda::CUDAGuard guard(s.x.device());
         const Tensor dout = grads[0].defined() ? dense_as(grads[0], s.x.scalar_type()) : at::zeros_like(s.x);
-        const NormGrads n = norm_backward(y.unpack(), w.unpack(), z.unpack(), dout, rstd.unpack());
+        const NormGrads n = norm_backward(yv, wv, zv, dout, rv);
         const ScanGrads g = scan_backward(s, opt, n.dx, dfinal_of(grads[1]), false);
         return {g.dx, cast(g.ddt, dt_type), cast(g.dA_head, A_type), g.dB, g.dC, cast(g.dD, D_type), cast(n.dz.view(z_shape), z_type),
                 cast(n.dw.view(w_shape), w_type), g.dinit.defined() ? g.dinit.view(init_shape) : Tensor()};
@@ -499,15 +510,16 @@ struct Mamba3Node : ScanNode {
     at::ScalarType ang_type, dt_type, A_type, D_type, raw_type, lam_type;
     bool fused = false;
     std::string name() const override { return "SSDMamba3Backward"; }
-    void release_variables() override {
-        ScanNode::release_variables();
+    void release_saved() override {
+        ScanNode::release_saved();
         for (SavedVariable* v : {&x, &dt, &lam, &A_head, &D, &B, &C, &cum, &sdot}) v->reset_data();
     }
     variable_list apply(variable_list&& grads) override {
         at::NoGradGuard no_grad;
-        const Scan s = load();
-        const Tensor xv = x.unpack(), dtv = dt.unpack(), lamv = lam.unpack(), Ah = A_head.unpack(), Dv = D.unpack(), Bv = B.unpack(), Cv = C.unpack(),
-                     cumv = cum.unpack(), sd = sdot.unpack();
+        const auto [s, xv, dtv, lamv, Ah, Dv, Bv, Cv, cumv, sd] = unpacked([&] {
+            return std::tuple(saved.load(), x.unpack(), dt.unpack(), lam.unpack(), A_head.unpack(), D.unpack(), B.unpack(), C.unpack(), cum.unpack(),
+                              sdot.unpack());
+        });
         c10::cuda::CUDAGuard guard(xv.device());
         const int64_t b = xv.size(0), T = xv.size(1), h = xv.size(2), n = Bv.size(3);
         const Tensor dy = grads[0].defined() ? dense_as(grads[0], xv.scalar_type()) : at::zeros_like(xv);
@@ -605,21 +617,19 @@ Tensor mamba3(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Ten
 }
 
 // ---------------------------------------------------------------------------------------------------- rotation
-struct RopeNode : Node {
+struct RopeNode : SavingNode {
     SavedVariable x, ang;
     at::ScalarType ang_type;
-    bool broadcast = false, released = false;
+    bool broadcast = false;
     std::string name() const override { return "FusedRoPEBackward"; }
-    void release_variables() override {
+    void release_saved() override {
         x.reset_data();
         ang.reset_data();
-        released = true;
     }
     variable_list apply(variable_list&& grads) override {
         if (!grads[0].defined()) return {Tensor(), Tensor()};
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         at::NoGradGuard no_grad;
-        const Tensor xv = x.unpack(), av = ang.unpack();
+        const auto [xv, av] = unpacked([&] { return std::tuple(x.unpack(), ang.unpack()); });
         c10::cuda::CUDAGuard guard(xv.device());
         const Tensor dy = cast(grads[0].contiguous(), xv.scalar_type());
         const Tensor dx = at::empty_like(xv), dang = at::empty_like(av);
@@ -660,19 +670,16 @@ Tensor rope(const Tensor& x, const Tensor& angles) {
 }
 
 // ---------------------------------------------------------------------------------------------------- coefficients
-struct TrapezoidNode : Node {
+struct TrapezoidNode : SavingNode {
     SavedVariable dt_raw, lam_raw, bias, alog;
     at::ScalarType bias_type, alog_type, lam_type;
-    bool released = false;
     std::string name() const override { return "FusedTrapezoidalBackward"; }
-    void release_variables() override {
+    void release_saved() override {
         for (SavedVariable* v : {&dt_raw, &lam_raw, &bias, &alog}) v->reset_data();
-        released = true;
     }
     variable_list apply(variable_list&& grads) override {
-        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
         at::NoGradGuard no_grad;
-        const Tensor d = dt_raw.unpack(), l = lam_raw.unpack(), bv = bias.unpack(), av = alog.unpack();
+        const auto [d, l, bv, av] = unpacked([&] { return std::tuple(dt_raw.unpack(), lam_raw.unpack(), bias.unpack(), alog.unpack()); });
         c10::cuda::CUDAGuard guard(d.device());
         const int64_t H = d.size(-1), rows = d.numel() / H;
         Tensor g[4];

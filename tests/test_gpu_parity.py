@@ -337,6 +337,66 @@ def test_arguments_that_are_too_small_are_refused(pkg, cabi, op, arg, bad):
     assert cabi.launch_count() == before
 
 
+def _graph(pkg, op):
+    """The leaves, the output and an output gradient of one call of an operator with a recorded graph."""
+    if op in ("mamba2", "operator", "gated", "mamba3"):
+        a = _op_args(op)
+        lv = [t.requires_grad_(True) for t in a.values()] if op != "operator" else [a[k].requires_grad_(True) for k in ("x", "dt", "B", "C")]
+        out = _call(pkg, op, a)[0]
+    else:
+        gen = torch.Generator(device=DEV).manual_seed(8)
+        x = torch.randn(2, 64, 4, 16, generator=gen, device=DEV)
+        lv = {"rope": [x, x[..., :8].clone()], "norm": [x, torch.ones(16, device=DEV), x.clone()],
+              "trapezoid": [x[..., 0].clone(), x[..., 1].clone(), x[0, 0, :, 2].clone(), x[0, 0, :, 3].clone()]}[op]
+        lv = [t.requires_grad_(True) for t in lv]
+        out = {"rope": lambda: pkg.fused_rope(*lv), "norm": lambda: pkg.fused_gate_norm(lv[0], lv[2], lv[1]),
+               "trapezoid": lambda: pkg.fused_trapezoidal(*lv)[2]}[op]()
+    return lv, out, torch.ones_like(out)
+
+
+ALL_OPS = ["mamba2", "operator", "gated", "mamba3", "rope", "norm", "trapezoid"]
+
+
+@pytest.mark.parametrize("op", ALL_OPS)
+def test_backward_twice_through_a_freed_graph_raises(pkg, cabi, op):
+    lv, out, g = _graph(pkg, op)
+    first = torch.autograd.grad([out], lv, [g], retain_graph=True, allow_unused=True)
+    second = torch.autograd.grad([out], lv, [g], allow_unused=True)
+    for a, b in zip(first, second):
+        assert (a is None and b is None) or torch.equal(a, b)
+    with pytest.raises(RuntimeError, match="backward through the graph a second time"):
+        torch.autograd.grad([out], lv, [g], allow_unused=True)
+
+
+@pytest.mark.parametrize("op", ALL_OPS)
+def test_two_threads_on_one_graph(pkg, cabi, op):
+    """Threads that run backward through one graph at the same time, one of them freeing it: each ends with the gradients or with
+    torch's error about a freed graph, never with anything else."""
+    import threading
+    for _ in range(5):
+        lv, out, g = _graph(pkg, op)
+        want = torch.autograd.grad([out], lv, [g], retain_graph=True, allow_unused=True)
+        got, start = {}, threading.Barrier(2)
+        def work(i):
+            start.wait()
+            try:
+                got[i] = torch.autograd.grad([out], lv, [g], retain_graph=i == 0, allow_unused=True)
+                torch.cuda.synchronize()
+            except RuntimeError as e:
+                got[i] = e
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for i, r in got.items():
+            if isinstance(r, Exception):
+                assert i == 0 and "second time" in str(r)
+            else:
+                for a, b in zip(r, want):
+                    assert (a is None and b is None) or torch.equal(a, b)
+
+
 def test_gated_norm_weight_per_head(pkg, cabi):
     """A weight of shape (heads, headdim) is the flat one, forward and backward (its gradient has its shape)."""
     a = _op_args("gated", h=3)
