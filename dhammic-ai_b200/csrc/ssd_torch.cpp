@@ -113,6 +113,14 @@ void check_status(const Options& o, const ssd_b200_shape& s, const Tensor& ws) {
     if (o.check_status) check(ssd_b200_device_status(&s, ptr(ws), stream_of(ws)));
 }
 
+// The operators have reverse-mode derivatives only.  A tangent would be dropped without a word (the kernels see values), which the
+// caller would read as a zero derivative.
+void refuse_tangents(std::initializer_list<const Tensor*> ts) {
+    for (const Tensor* t : ts)
+        TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(),
+                                    "ssd_b200 operators have no jvp: they cannot be used with forward-mode AD");
+}
+
 bool wants_grad(std::initializer_list<const Tensor*> ts) {
     if (!at::GradMode::is_enabled()) return false;
     for (const Tensor* t : ts)
@@ -283,6 +291,7 @@ std::tuple<Tensor, Tensor> mamba2(const Tensor& x, const Tensor& dt, const Tenso
                                   int64_t chunk, const OptTensor& init_, int path, bool save_states, bool status) {
     const Options o{path, save_states, status};
     const Tensor D = get(D_), init = get(init_);
+    refuse_tangents({&x, &dt, &A_head, &B, &C, &D, &init});
     check_inputs(x, B, C);
     check_coefficients(x, dt, A_head, D, init, B.size(3));
     c10::cuda::CUDAGuard guard(x.device());
@@ -328,11 +337,12 @@ struct OperatorNode : ScanNode {
 std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk,
                                                  const OptTensor& init_, const OptTensor& cum_in, int path, bool save_states, bool status) {
     const Options o{path, save_states, status};
-    const Tensor init = get(init_);
+    const Tensor init = get(init_), cached = get(cum_in);
+    refuse_tangents({&x, &A, &B, &C, &init, &cached});
     check_inputs(x, B, C);
     check_like("A", A, x, x.size(0) * x.size(1) * x.size(2));
     check_like("initial_states", init, x, x.size(0) * x.size(2) * x.size(3) * B.size(3));
-    check_like("A_cumsum", get(cum_in), x, x.size(0) * x.size(1) * x.size(2));
+    check_like("A_cumsum", cached, x, x.size(0) * x.size(1) * x.size(2));
     c10::cuda::CUDAGuard guard(x.device());
     const bool grad = wants_grad({&x, &A, &B, &C, &init});
     Scan s;
@@ -341,7 +351,7 @@ std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& 
         at::NoGradGuard no_grad;
         s.x = dense(x); s.a = A.contiguous(); s.B = dense(B); s.C = dense(C);
         if (init.defined()) s.init = f32(init.reshape({x.size(0), x.size(2), x.size(3), B.size(3)}));
-        out = scan_forward(s, chunk, o, get(cum_in), grad);
+        out = scan_forward(s, chunk, o, cached, grad);
         out.final_state = cast(out.final_state, x.scalar_type());
     }
     if (grad) {
@@ -392,6 +402,7 @@ struct NormNode : SavingNode {
 
 Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTensor& z_) {
     const Tensor z = get(z_);
+    refuse_tangents({&x, &weight, &z});
     SSD_ASSERT(x.is_cuda() && weight.is_cuda(), "FusedRMSNorm requires CUDA tensors");
     const int64_t D = x.size(-1);
     SSD_ASSERT(weight.dim() == 1 && weight.size(0) == D, "weight shape ", weight.sizes(), " mismatches D=", D);
@@ -451,6 +462,7 @@ std::tuple<Tensor, Tensor> mamba2_gated(const Tensor& x, const Tensor& dt, const
                                         bool save_states, bool status) {
     const Options o{path, save_states, status};
     const Tensor D = get(D_), init = get(init_);
+    refuse_tangents({&x, &dt, &A_head, &B, &C, &D, &z, &weight, &init});
     check_inputs(x, B, C);
     check_coefficients(x, dt, A_head, D, init, B.size(3));
     check_like("norm_weight", weight, x, x.size(2) * x.size(3));
@@ -554,6 +566,7 @@ Tensor mamba3(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Ten
               const Tensor& lam, int64_t chunk, int path, bool save_states, bool status) {
     const Options o{path, save_states, status};
     const Tensor D = get(D_);
+    refuse_tangents({&x, &dt, &A_head, &B, &C, &D, &raw_angles, &lam});
     check_inputs(x, B, C);
     check_coefficients(x, dt, A_head, D, {}, B.size(3));
     check_like("lam", lam, x, x.size(0) * x.size(1) * x.size(2));
@@ -640,6 +653,7 @@ struct RopeNode : SavingNode {
 };
 
 Tensor rope(const Tensor& x, const Tensor& angles) {
+    refuse_tangents({&x, &angles});
     SSD_ASSERT(x.is_cuda() && angles.is_cuda(), "rotation runs on the GPU only: x and angles must be CUDA tensors");
     SSD_ASSERT(x.dim() == 4 && angles.dim() == 4, "x must be (B,T,H,D) and angles (B,T,1 or H,D/2); got ", x.dim(), " and ", angles.dim(),
                " dimensions");
@@ -693,6 +707,7 @@ struct TrapezoidNode : SavingNode {
 };
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> trapezoid(const Tensor& dt_raw, const Tensor& lam_raw, const Tensor& dt_bias, const Tensor& A_log) {
+    refuse_tangents({&dt_raw, &lam_raw, &dt_bias, &A_log});
     SSD_ASSERT(dt_raw.is_cuda() && lam_raw.is_cuda() && dt_bias.is_cuda() && A_log.is_cuda(),
                "the coefficient kernel runs on the GPU only: all four arguments must be CUDA tensors");
     SSD_ASSERT(dt_raw.sizes() == lam_raw.sizes(), "dt_raw and lam_raw must have one shape, got ", dt_raw.sizes(), " and ", lam_raw.sizes());

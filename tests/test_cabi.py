@@ -95,6 +95,27 @@ def test_operator_rejects_cpu_tensors(pkg, cabi):
         pkg.fused_ssd_scan(x, torch.zeros(1, 64, 2), torch.zeros(1, 64, 2, 4), torch.zeros(1, 64, 2, 4), 32)
 
 
+def test_forward_mode_is_refused(pkg, cabi):
+    """A dual tensor ends in an exception in every operator, whichever argument it is (a dropped tangent would read as zero)."""
+    import torch.autograd.forward_ad as fwd
+    x, dt, h1, B = torch.zeros(1, 64, 2, 8), torch.zeros(1, 64, 2), torch.zeros(2), torch.zeros(1, 64, 1, 8)
+    ang, w = torch.zeros(1, 64, 2, 4), torch.ones(16)
+    init, cum = torch.zeros(1, 2, 8, 8), torch.zeros(1, 2, 2, 32)
+    calls = {
+        "mamba2": ([x, dt, h1, B, B, h1, init], lambda a: pkg.ssd_mamba2(*a[:6], 32, a[6])),
+        "operator": ([x, dt, B, B, init, cum], lambda a: pkg.fused_ssd_scan(*a[:4], 32, a[4], {"A_cumsum": a[5]})),
+        "gated": ([x, dt, h1, B, B, h1, x, w, init], lambda a: pkg.ssd_mamba2_gated(*a[:8], 1e-6, 32, a[8])),
+        "mamba3": ([x, dt, h1, B, B, h1, ang, dt], lambda a: pkg.ssd_mamba3(*a, 32)),
+        "rope": ([x, ang], lambda a: pkg.fused_rope(*a)),
+        "norm": ([x, x, torch.ones(8)], lambda a: pkg.fused_gate_norm(*a)),
+        "trapezoid": ([dt, dt, h1, h1], lambda a: pkg.fused_trapezoidal(*a)),
+    }
+    for name, (args, call) in calls.items():
+        for i in range(len(args)):
+            with fwd.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+                call([fwd.make_dual(t.clone(), torch.ones_like(t)) if j == i else t for j, t in enumerate(args)])
+
+
 def test_missing_library_fails_loudly(cabi, monkeypatch, tmp_path):
     monkeypatch.setattr(cabi, "_lib", None)
     monkeypatch.setattr(cabi, "library_path", lambda: tmp_path / "libssd_b200.so")
