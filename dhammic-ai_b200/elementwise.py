@@ -23,7 +23,7 @@ class FusedRoPE:
 
     @staticmethod
     def apply(x: Tensor, angles: Tensor) -> Tensor:
-        return _native.load().rope(x, angles)
+        return _native.call("rope", x, angles)
 
 
 def fused_rope(x: Tensor, angles: Tensor) -> Tensor:
@@ -37,7 +37,7 @@ class FusedTrapezoidal:
 
     @staticmethod
     def apply(dt_raw: Tensor, lam_raw: Tensor, dt_bias: Tensor, A_log: Tensor):
-        return _native.load().trapezoid(dt_raw, lam_raw, dt_bias, A_log)
+        return _native.call("trapezoid", dt_raw, lam_raw, dt_bias, A_log)
 
 
 def fused_trapezoidal(dt_raw: Tensor, lam_raw: Tensor, dt_bias: Tensor, A_log: Tensor):
@@ -52,7 +52,7 @@ class FusedRMSNorm:
 
     @staticmethod
     def apply(x: Tensor, weight: Tensor, eps: float, *gate: Tensor) -> Tensor:
-        return _native.load().rmsnorm(x, weight, float(eps), gate[0] if gate else None)
+        return _native.call("rmsnorm", x, weight, float(eps), gate[0] if gate else None)
 
 
 def fused_rmsnorm(x: Tensor, weight: Tensor, eps: float = 1e-6) -> Tensor:

@@ -222,7 +222,7 @@ class FusedSSDScan:
     def apply(x: Tensor, A: Tensor, B: Tensor, C_: Tensor, chunk_size: int, initial_states: Tensor | None,
               L_cache_in: Tensor | None, decay_chunk_cache_in: Tensor | None, A_cumsum_cache_in: Tensor | None):
         """(Y, final_state, L, decay_chunk, A_cumsum); L and decay_chunk are None unless the eager cache is on."""
-        y, final, cum = _native.load().operator_scan(x, A, B, C_, int(chunk_size), initial_states, A_cumsum_cache_in,
+        y, final, cum = _native.call("operator_scan", x, A, B, C_, int(chunk_size), initial_states, A_cumsum_cache_in,
                                                      _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
         L = dc = None
         if _EAGER_CACHE:
@@ -250,7 +250,8 @@ def fused_ssd_scan(x: Tensor, A: Tensor, B: Tensor, C: Tensor, chunk_size: int,
         L_in = dc_in = ac_in = None
     Y, final_state, L_out, dc_out, ac_out = FusedSSDScan.apply(
         x, A, B, C, int(chunk_size), initial_states, L_in, dc_in, ac_in)
-    dims = (*x.shape, B.shape[3], B.shape[2], int(chunk_size))  # (not the tensors: the cache must not keep them alive)
+    # (not the tensors: the cache must not keep them alive; int: while tracing, a size is a tensor)
+    dims = tuple(int(v) for v in (*x.shape, B.shape[3], B.shape[2], chunk_size))
     code, path = _dt_code(x), _FORCE_PATH
     out_cache = LazySSDCache(ac_out, lambda: _cabi.Shape(_cabi.ABI_VERSION, code, _cabi.F32, path, *dims), x.dtype)
     for k, v in (("L", L_out if L_out is not None else L_in), ("decay_chunk", dc_out if dc_out is not None else dc_in)):
@@ -267,7 +268,7 @@ def ssd_mamba2(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: T
     x (b,T,h,p) bf16/fp32; dt (b,T,h); A_head (h); B, C (b,T,g,n); D (h) or None;
     initial_states (b,h,p,n) or (b,1,h,p,n).  Returns (Y, final_state fp32 (b,h,p,n)).
     """
-    return _native.load().mamba2(x, dt, A_head, B, C, D, int(chunk_size), initial_states, _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
+    return _native.call("mamba2", x, dt, A_head, B, C, D, int(chunk_size), initial_states, _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
 
 
 def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: Tensor | None, z: Tensor,
@@ -279,7 +280,7 @@ def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor
     Returns (out in x's shape, final_state fp32 (b,h,p,n)).  Gradients: x, dt, A_head, B, C, D, z, norm_weight,
     initial_states.
     """
-    return _native.load().mamba2_gated(x, dt, A_head, B, C, D, z, norm_weight, float(eps), int(chunk_size), initial_states,
+    return _native.call("mamba2_gated", x, dt, A_head, B, C, D, z, norm_weight, float(eps), int(chunk_size), initial_states,
                                        _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
 
 

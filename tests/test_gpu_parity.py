@@ -397,6 +397,35 @@ def test_two_threads_on_one_graph(pkg, cabi, op):
                     assert (a is None and b is None) or torch.equal(a, b)
 
 
+@pytest.mark.parametrize("op", ALL_OPS)
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+@pytest.mark.filterwarnings("ignore:.*torch.jit.*:DeprecationWarning")
+def test_trace_replays_the_operator(pkg, cabi, op):
+    """A traced call gives on other inputs what the operator gives on them, with its gradients."""
+    if op in ("mamba2", "operator", "gated", "mamba3"):
+        a = _op_args(op)
+        if op == "operator":
+            a = {k: a[k] for k in ("x", "dt", "B", "C")}
+        names = list(a)
+        def fn(*t):
+            return _call(pkg, op, dict(zip(names, t)))[0]
+        args = list(a.values())
+    else:
+        lv, _, _ = _graph(pkg, op)
+        args = [t.detach() for t in lv]
+        fn = {"rope": pkg.fused_rope, "norm": lambda x, w, z: pkg.fused_gate_norm(x, z, w), "trapezoid": lambda *t: pkg.fused_trapezoidal(*t)[2]}[op]
+    traced = torch.jit.trace(fn, tuple(args))
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    other = [(t * (0.5 + torch.rand(t.shape, generator=gen, device=DEV))).to(t.dtype) for t in args]
+    res = []
+    for f in (fn, traced):
+        lv = [t.clone().requires_grad_(True) for t in other]
+        y = f(*lv)
+        res.append([y.detach()] + list(torch.autograd.grad([y], lv, [torch.ones_like(y)], allow_unused=True)))
+    for u, v in zip(*res):
+        assert (u is None and v is None) or torch.equal(u, v)
+
+
 def test_gated_norm_weight_per_head(pkg, cabi):
     """A weight of shape (heads, headdim) is the flat one, forward and backward (its gradient has its shape)."""
     a = _op_args("gated", h=3)
