@@ -112,15 +112,13 @@ class LazySSDCache(dict):
     by a small kernel the first time they are read (the production caller only hands the dict back)."""
 
     def __init__(self, a_cumsum: Tensor, shape, out_dtype: torch.dtype):
-        """``shape``: the call's ``_cabi.Shape``, or a function that makes it when it is first needed."""
+        """``shape``: the call's ``_cabi.Shape``, or its fields behind the ABI version as a tuple, which becomes one when needed."""
         super().__init__(A_cumsum=a_cumsum)
         self._shape = shape
         self._dtype = out_dtype
 
     def _materialize(self, key: str) -> Tensor:
-        if callable(self._shape):
-            self._shape = self._shape()
-        s = self._shape
+        s = _cabi.Shape(_cabi.ABI_VERSION, *self._shape) if isinstance(self._shape, tuple) else self._shape
         cum = dict.__getitem__(self, "A_cumsum")
         c = s.seqlen // s.chunk
         with torch.cuda.device(cum.device):
@@ -252,8 +250,7 @@ def fused_ssd_scan(x: Tensor, A: Tensor, B: Tensor, C: Tensor, chunk_size: int,
         x, A, B, C, int(chunk_size), initial_states, L_in, dc_in, ac_in)
     # (not the tensors: the cache must not keep them alive; int: while tracing, a size is a tensor)
     dims = tuple(int(v) for v in (*x.shape, B.shape[3], B.shape[2], chunk_size))
-    code, path = _dt_code(x), _FORCE_PATH
-    out_cache = LazySSDCache(ac_out, lambda: _cabi.Shape(_cabi.ABI_VERSION, code, _cabi.F32, path, *dims), x.dtype)
+    out_cache = LazySSDCache(ac_out, (_dt_code(x), _cabi.F32, _FORCE_PATH, *dims), x.dtype)
     for k, v in (("L", L_out if L_out is not None else L_in), ("decay_chunk", dc_out if dc_out is not None else dc_in)):
         if v is not None:
             dict.__setitem__(out_cache, k, v)

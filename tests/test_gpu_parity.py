@@ -337,6 +337,20 @@ def test_arguments_that_are_too_small_are_refused(pkg, cabi, op, arg, bad):
     assert cabi.launch_count() == before
 
 
+def test_cache_can_be_pickled_and_copied(pkg, cabi):
+    """The operator's cache goes through pickle and copy before anything was read from it, and works as the one it came from."""
+    import copy
+    import pickle
+    a = _op_args("operator", p=16, n=8, dtype=torch.float32)
+    decay = -a["dt"]
+    y0, _, cache = pkg.fused_ssd_scan(a["x"], decay, a["B"], a["C"], 64)
+    for other in (pickle.loads(pickle.dumps(cache)), copy.copy(cache), copy.deepcopy(cache)):
+        y1, _, _ = pkg.fused_ssd_scan(a["x"], decay, a["B"], a["C"], 64, None, other)
+        assert torch.equal(y0, y1)
+        for k in ("A_cumsum", "L", "decay_chunk"):
+            assert torch.equal(other[k], cache[k])
+
+
 def _graph(pkg, op):
     """The leaves, the output and an output gradient of one call of an operator with a recorded graph."""
     if op in ("mamba2", "operator", "gated", "mamba3"):
