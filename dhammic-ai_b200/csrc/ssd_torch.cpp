@@ -365,7 +365,8 @@ std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& 
         torch::autograd::set_history(out.y, node);
         torch::autograd::set_history(out.final_state, node);
     }
-    return {out.y, out.final_state, s.cum};
+    // (sums that came in leave without the graph that made them: they get no gradient here)
+    return {out.y, out.final_state, cached.defined() ? s.cum.detach() : s.cum};
 }
 
 // ---------------------------------------------------------------------------------------------------- norm and gate

@@ -351,6 +351,15 @@ def test_cache_can_be_pickled_and_copied(pkg, cabi):
             assert torch.equal(other[k], cache[k])
 
 
+def test_cached_sums_leave_without_their_graph(pkg, cabi):
+    """Sums that the caller made with a graph are values here: the cache that comes back does not carry the graph on."""
+    a = _op_args("operator")
+    decay = (-a["dt"]).requires_grad_(True)
+    cum = decay.view(2, 2, 64, 2).cumsum(2).permute(0, 3, 1, 2).contiguous()
+    _, _, cache = pkg.fused_ssd_scan(a["x"], decay, a["B"], a["C"], 64, None, {"A_cumsum": cum})
+    assert cum.requires_grad and not cache["A_cumsum"].requires_grad and torch.equal(cache["A_cumsum"], cum)
+
+
 def _graph(pkg, op):
     """The leaves, the output and an output gradient of one call of an operator with a recorded graph."""
     if op in ("mamba2", "operator", "gated", "mamba3"):
