@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import importlib.machinery
 import importlib.util
+import os
 from pathlib import Path
 
 import torch
@@ -12,6 +13,15 @@ from torch import Tensor
 from . import _cabi
 
 _ext = None
+check_status = os.environ.get("SSD_B200_CHECK_STATUS", "0") == "1"
+
+
+def set_check_status(flag: bool) -> None:
+    """The status check of both passes (see ``ssd_scan.set_check_status``), now or when the extension is loaded."""
+    global check_status
+    check_status = bool(flag)
+    if _ext is not None:
+        _ext.set_check_status(check_status)
 
 
 def load():
@@ -27,6 +37,7 @@ def load():
         spec = importlib.util.spec_from_file_location("ssd_torch", str(path), loader=loader)
         ext = importlib.util.module_from_spec(spec)
         loader.exec_module(ext)
+        ext.set_check_status(check_status)
         _ext = ext
     return _ext
 

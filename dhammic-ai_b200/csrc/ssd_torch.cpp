@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include <atomic>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -46,12 +47,14 @@ void check(int rc) {
     TORCH_CHECK(false, "ssd_b200 error ", rc, ": ", msg);
 }
 
-// Switches of the Python layer, passed with every call.
+// Switches of the Python layer that belong to a call.
 struct Options {
     int path;          // SSD_B200_PATH_*
     bool save_states;  // keep the forward's states for the backward
-    bool check_status; // synchronise after every call and report a bounded wait that ran out
 };
+// Synchronise after every call and report a bounded wait that ran out.  Read when a pass runs, so that the switch holds for the
+// backward of a forward that ran before it was set.
+std::atomic<bool> g_check_status{false};
 
 int dtype_code(const Tensor& t) {
     if (t.scalar_type() == at::kFloat) return SSD_B200_F32;
@@ -109,8 +112,8 @@ Tensor workspace(const ssd_b200_shape& s, int pass, const Tensor& like) {
     return bytes(n, like);
 }
 
-void check_status(const Options& o, const ssd_b200_shape& s, const Tensor& ws) {
-    if (o.check_status) check(ssd_b200_device_status(&s, ptr(ws), stream_of(ws)));
+void check_status(const ssd_b200_shape& s, const Tensor& ws) {
+    if (g_check_status.load(std::memory_order_relaxed)) check(ssd_b200_device_status(&s, ptr(ws), stream_of(ws)));
 }
 
 // The operators have reverse-mode derivatives only.  A tangent would be dropped without a word (the kernels see values), which the
@@ -169,7 +172,7 @@ ScanOut scan_forward(Scan& s, int64_t chunk, const Options& o, const Tensor& cum
     a.a_cumsum = ptr<float>(s.cum); a.cumsum_is_input = cum_in.defined(); a.workspace = ptr(ws); a.workspace_bytes = ws.numel();
     a.states = ptr(s.states); a.ysq = ptr<float>(ysq); a.skip = ptr<float>(s.skip);
     check(ssd_b200_fwd(&a, stream_of(s.x)));
-    check_status(o, s.shape, ws);
+    check_status(s.shape, ws);
     return out;
 }
 
@@ -177,7 +180,7 @@ struct ScanGrads {
     Tensor dx, dB, dC, da, ddt, dA_head, dD, dinit, dskip;
 };
 
-ScanGrads scan_backward(const Scan& s, const Options& o, const Tensor& dy, const Tensor& dfinal, bool cached) {
+ScanGrads scan_backward(const Scan& s, const Tensor& dy, const Tensor& dfinal, bool cached) {
     const int64_t b = s.x.size(0), T = s.x.size(1), h = s.x.size(2);
     const bool operator_form = s.a.defined(), mamba2 = !operator_form, scaled = operator_form && s.dt.defined();
     ScanGrads g;
@@ -200,7 +203,7 @@ ScanGrads scan_backward(const Scan& s, const Options& o, const Tensor& dy, const
     a.cumsum_is_input = cached; a.workspace = ptr(ws); a.workspace_bytes = ws.numel(); a.states = ptr(s.states);
     a.skip = ptr<float>(s.skip); a.dskip = ptr<float>(g.dskip);
     check(ssd_b200_bwd(&a, stream_of(s.x)));
-    check_status(o, s.shape, ws);
+    check_status(s.shape, ws);
     return g;
 }
 
@@ -247,7 +250,6 @@ struct SavingNode : Node {
 };
 struct ScanNode : SavingNode {
     SavedScan saved;
-    Options opt{};
     void release_saved() override { saved.release(); }
     Scan load() {
         return unpacked([&] { return saved.load(); });
@@ -262,10 +264,9 @@ std::shared_ptr<N> link_node(const Inputs&... inputs) {
     return node;
 }
 template <class N, class... Inputs>
-std::shared_ptr<N> new_node(const Scan& s, const Options& o, const Inputs&... inputs) {
+std::shared_ptr<N> new_node(const Scan& s, const Inputs&... inputs) {
     auto node = link_node<N>(inputs...);
     node->saved.save(s);
-    node->opt = o;
     return node;
 }
 
@@ -281,15 +282,15 @@ struct Mamba2Node : ScanNode {
         const Scan s = load();
         c10::cuda::CUDAGuard guard(s.x.device());
         const Tensor dy = grads[0].defined() ? dense_as(grads[0], s.x.scalar_type()) : at::zeros_like(s.x);
-        const ScanGrads g = scan_backward(s, opt, dy, dfinal_of(grads[1]), false);
+        const ScanGrads g = scan_backward(s, dy, dfinal_of(grads[1]), false);
         return {g.dx, cast(g.ddt, dt_type), cast(g.dA_head, A_type), g.dB, g.dC, cast(g.dD, D_type),
                 g.dinit.defined() ? g.dinit.view(init_shape) : Tensor()};
     }
 };
 
 std::tuple<Tensor, Tensor> mamba2(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Tensor& B, const Tensor& C, const OptTensor& D_,
-                                  int64_t chunk, const OptTensor& init_, int path, bool save_states, bool status) {
-    const Options o{path, save_states, status};
+                                  int64_t chunk, const OptTensor& init_, int path, bool save_states) {
+    const Options o{path, save_states};
     const Tensor D = get(D_), init = get(init_);
     refuse_tangents({&x, &dt, &A_head, &B, &C, &D, &init});
     check_inputs(x, B, C);
@@ -306,7 +307,7 @@ std::tuple<Tensor, Tensor> mamba2(const Tensor& x, const Tensor& dt, const Tenso
         out = scan_forward(s, chunk, o, {}, grad);
     }
     if (grad) {
-        auto node = new_node<Mamba2Node>(s, o, x, dt, A_head, B, C, D, init);
+        auto node = new_node<Mamba2Node>(s, x, dt, A_head, B, C, D, init);
         node->dt_type = dt.scalar_type();
         node->A_type = A_head.scalar_type();
         if (D.defined()) node->D_type = D.scalar_type();
@@ -328,15 +329,15 @@ struct OperatorNode : ScanNode {
         const Scan s = load();
         c10::cuda::CUDAGuard guard(s.x.device());
         const Tensor dy = grads[0].defined() ? dense_as(grads[0], s.x.scalar_type()) : at::zeros_like(s.x);
-        const ScanGrads g = scan_backward(s, opt, dy, dfinal_of(grads[1]), cached);
+        const ScanGrads g = scan_backward(s, dy, dfinal_of(grads[1]), cached);
         return {g.dx, cast(g.da, A_type), g.dB, g.dC, g.dinit.defined() ? cast(g.dinit.view(init_shape), init_type) : Tensor()};
     }
 };
 
 // (Y, final state in x's dtype, A_cumsum); `cum_in` is the A_cumsum of an earlier call (then A gets no gradient, as in the reference)
 std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk,
-                                                 const OptTensor& init_, const OptTensor& cum_in, int path, bool save_states, bool status) {
-    const Options o{path, save_states, status};
+                                                 const OptTensor& init_, const OptTensor& cum_in, int path, bool save_states) {
+    const Options o{path, save_states};
     const Tensor init = get(init_), cached = get(cum_in);
     refuse_tangents({&x, &A, &B, &C, &init, &cached});
     check_inputs(x, B, C);
@@ -355,7 +356,7 @@ std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& 
         out.final_state = cast(out.final_state, x.scalar_type());
     }
     if (grad) {
-        auto node = new_node<OperatorNode>(s, o, x, A, B, C, init);
+        auto node = new_node<OperatorNode>(s, x, A, B, C, init);
         node->A_type = A.scalar_type();
         node->cached = cum_in.has_value();
         if (init.defined()) {
@@ -452,7 +453,7 @@ struct GatedNode : ScanNode {
         c10::cuda::CUDAGuard guard(s.x.device());
         const Tensor dout = grads[0].defined() ? dense_as(grads[0], s.x.scalar_type()) : at::zeros_like(s.x);
         const NormGrads n = norm_backward(yv, wv, zv, dout, rv);
-        const ScanGrads g = scan_backward(s, opt, n.dx, dfinal_of(grads[1]), false);
+        const ScanGrads g = scan_backward(s, n.dx, dfinal_of(grads[1]), false);
         return {g.dx, cast(g.ddt, dt_type), cast(g.dA_head, A_type), g.dB, g.dC, cast(g.dD, D_type), cast(n.dz.view(z_shape), z_type),
                 cast(n.dw.view(w_shape), w_type), g.dinit.defined() ? g.dinit.view(init_shape) : Tensor()};
     }
@@ -460,8 +461,8 @@ struct GatedNode : ScanNode {
 
 std::tuple<Tensor, Tensor> mamba2_gated(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Tensor& B, const Tensor& C, const OptTensor& D_,
                                         const Tensor& z, const Tensor& weight, double eps, int64_t chunk, const OptTensor& init_, int path,
-                                        bool save_states, bool status) {
-    const Options o{path, save_states, status};
+                                        bool save_states) {
+    const Options o{path, save_states};
     const Tensor D = get(D_), init = get(init_);
     refuse_tangents({&x, &dt, &A_head, &B, &C, &D, &z, &weight, &init});
     check_inputs(x, B, C);
@@ -499,7 +500,7 @@ std::tuple<Tensor, Tensor> mamba2_gated(const Tensor& x, const Tensor& dt, const
             check(ssd_b200_rmsnorm_fwd(dtc, rows, Dn, static_cast<float>(eps), ptr(scan.y), ptr<float>(w), ptr(zc), ptr(out), ptr<float>(rstd), stream_of(x)));
     }
     if (grad) {
-        auto node = new_node<GatedNode>(s, o, x, dt, A_head, B, C, D, z, weight, init);
+        auto node = new_node<GatedNode>(s, x, dt, A_head, B, C, D, z, weight, init);
         node->y = SavedVariable(scan.y, false); node->z = SavedVariable(zc, false);
         node->w = SavedVariable(w, false); node->rstd = SavedVariable(rstd, false);
         node->dt_type = dt.scalar_type(); node->A_type = A_head.scalar_type();
@@ -536,7 +537,7 @@ struct Mamba3Node : ScanNode {
         c10::cuda::CUDAGuard guard(xv.device());
         const int64_t b = xv.size(0), T = xv.size(1), h = xv.size(2), n = Bv.size(3);
         const Tensor dy = grads[0].defined() ? dense_as(grads[0], xv.scalar_type()) : at::zeros_like(xv);
-        ScanGrads g = scan_backward(s, opt, dy, {}, false);
+        ScanGrads g = scan_backward(s, dy, {}, false);
         // fused: dx is complete; dw = <dX, x> and dyx = <dy, x> come from the scan's own row sums
         Tensor dx = g.dx, dxw, dw = g.ddt, dyx = g.dskip;
         if (!fused) {
@@ -564,8 +565,8 @@ struct Mamba3Node : ScanNode {
 };
 
 Tensor mamba3(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Tensor& B, const Tensor& C, const OptTensor& D_, const Tensor& raw_angles,
-              const Tensor& lam, int64_t chunk, int path, bool save_states, bool status) {
-    const Options o{path, save_states, status};
+              const Tensor& lam, int64_t chunk, int path, bool save_states) {
+    const Options o{path, save_states};
     const Tensor D = get(D_);
     refuse_tangents({&x, &dt, &A_head, &B, &C, &D, &raw_angles, &lam});
     check_inputs(x, B, C);
@@ -616,7 +617,7 @@ Tensor mamba3(const Tensor& x, const Tensor& dt, const Tensor& A_head, const Ten
                                        stream_of(x)));
     }
     if (grad) {
-        auto node = new_node<Mamba3Node>(s, o, x, dt, A_head, B, C, D, raw_angles, lam);
+        auto node = new_node<Mamba3Node>(s, x, dt, A_head, B, C, D, raw_angles, lam);
         node->block = block;
         node->x = SavedVariable(xc, false); node->dt = SavedVariable(dtc, false); node->lam = SavedVariable(lamc, false);
         node->A_head = SavedVariable(Ah, false); node->D = SavedVariable(Dc, false); node->B = SavedVariable(Bc, false);
@@ -759,6 +760,7 @@ PYBIND11_MODULE(ssd_torch, m) {
         }
     });
     const auto nogil = py::call_guard<py::gil_scoped_release>();
+    m.def("set_check_status", [](bool on) { g_check_status.store(on, std::memory_order_relaxed); });
     m.def("mamba2", &mamba2, nogil);
     m.def("operator_scan", &operator_scan, nogil);
     m.def("mamba2_gated", &mamba2_gated, nogil);

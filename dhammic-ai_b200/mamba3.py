@@ -33,4 +33,4 @@ from . import _native, ssd_scan as _op
 def ssd_mamba3(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: Tensor | None, raw_angles: Tensor,
                lam: Tensor, chunk_size: int) -> Tensor:
     """x (b,T,h,p); dt, lam (b,T,h) fp32; A_head, D (h); B, C (b,T,g,n); raw_angles (b,T,h,n/2).  Returns Y."""
-    return _native.call("mamba3", x, dt, A_head, B, C, D, raw_angles, lam, int(chunk_size), _op._FORCE_PATH, _op._SAVE_STATES, _op._CHECK_STATUS)
+    return _native.call("mamba3", x, dt, A_head, B, C, D, raw_angles, lam, int(chunk_size), _op._FORCE_PATH, _op._SAVE_STATES)

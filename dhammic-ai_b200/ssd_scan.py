@@ -39,7 +39,6 @@ from . import _cabi, _native
 
 _EAGER_CACHE = False
 _FORCE_PATH = _cabi.PATH_AUTO
-_CHECK_STATUS = os.environ.get("SSD_B200_CHECK_STATUS", "0") == "1"
 _SAVE_STATES = os.environ.get("SSD_B200_SAVE_STATES", "1") == "1"
 
 
@@ -54,12 +53,11 @@ def set_save_states(flag: bool) -> None:
 def set_check_status(flag: bool) -> None:
     """After every call, synchronise and raise if a kernel reported a bounded wait that ran out
     (debug / test use: it costs a stream synchronisation per call)."""
-    global _CHECK_STATUS
-    _CHECK_STATUS = bool(flag)
+    _native.set_check_status(flag)
 
 
 def _status(lib, shape, ws, dev) -> None:
-    if _CHECK_STATUS:
+    if _native.check_status:
         _cabi.check(lib.ssd_b200_device_status(C.byref(shape), _ptr(ws), _stream(dev)))
 
 
@@ -221,7 +219,7 @@ class FusedSSDScan:
               L_cache_in: Tensor | None, decay_chunk_cache_in: Tensor | None, A_cumsum_cache_in: Tensor | None):
         """(Y, final_state, L, decay_chunk, A_cumsum); L and decay_chunk are None unless the eager cache is on."""
         y, final, cum = _native.call("operator_scan", x, A, B, C_, int(chunk_size), initial_states, A_cumsum_cache_in,
-                                                     _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
+                                                     _FORCE_PATH, _SAVE_STATES)
         L = dc = None
         if _EAGER_CACHE:
             lazy = LazySSDCache(cum, _make_shape(x, _cabi.F32, B, int(chunk_size)), x.dtype)
@@ -265,7 +263,7 @@ def ssd_mamba2(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: T
     x (b,T,h,p) bf16/fp32; dt (b,T,h); A_head (h); B, C (b,T,g,n); D (h) or None;
     initial_states (b,h,p,n) or (b,1,h,p,n).  Returns (Y, final_state fp32 (b,h,p,n)).
     """
-    return _native.call("mamba2", x, dt, A_head, B, C, D, int(chunk_size), initial_states, _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
+    return _native.call("mamba2", x, dt, A_head, B, C, D, int(chunk_size), initial_states, _FORCE_PATH, _SAVE_STATES)
 
 
 def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor, D: Tensor | None, z: Tensor,
@@ -278,7 +276,7 @@ def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor
     initial_states.
     """
     return _native.call("mamba2_gated", x, dt, A_head, B, C, D, z, norm_weight, float(eps), int(chunk_size), initial_states,
-                                       _FORCE_PATH, _SAVE_STATES, _CHECK_STATUS)
+                                       _FORCE_PATH, _SAVE_STATES)
 
 
 def resolved_path_name(cfg) -> str:

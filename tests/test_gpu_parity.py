@@ -360,6 +360,22 @@ def test_cached_sums_leave_without_their_graph(pkg, cabi):
     assert cum.requires_grad and not cache["A_cumsum"].requires_grad and torch.equal(cache["A_cumsum"], cum)
 
 
+def test_status_check_holds_for_the_backward_of_earlier_forwards(pkg, cabi):
+    """set_check_status is read when a pass runs: a backward of a graph recorded before synchronises (as its forward would)."""
+    try:
+        pkg.set_check_status(False)
+        lv, out, g = _graph(pkg, "mamba2")
+        pkg.set_check_status(True)
+        torch.cuda.synchronize()
+        spin = torch.cuda.Event()
+        torch.cuda._sleep(200_000_000)  # about 0.1 s of waiting in front of the backward
+        spin.record()
+        torch.autograd.grad([out], lv, [g])
+        assert spin.query()
+    finally:
+        pkg.set_check_status(True)
+
+
 def _graph(pkg, op):
     """The leaves, the output and an output gradient of one call of an operator with a recorded graph."""
     if op in ("mamba2", "operator", "gated", "mamba3"):
