@@ -371,6 +371,8 @@ std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& 
 }
 
 // ---------------------------------------------------------------------------------------------------- norm and gate
+// Rows of `cols` values (of zero columns: none, which the C ABI refuses).
+int64_t rows_of(const Tensor& t, int64_t cols) { return cols ? t.numel() / cols : 0; }
 int64_t ws_floats(size_t n) { return static_cast<int64_t>(n); }
 
 struct NormGrads {
@@ -418,7 +420,7 @@ Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTenso
         xc = x.contiguous();
         w = f32(weight);
         if (z.defined()) zc = cast(z.contiguous(), x.scalar_type());
-        const int64_t rows = xc.numel() / D;
+        const int64_t rows = rows_of(xc, D);
         out = at::empty_like(xc);
         rstd = empty_f32({rows}, x);
         check(ssd_b200_rmsnorm_fwd(dtype_code(xc), rows, D, static_cast<float>(eps), ptr(xc), ptr<float>(w), ptr(zc), ptr(out), ptr<float>(rstd), stream_of(x)));
@@ -697,7 +699,7 @@ struct TrapezoidNode : SavingNode {
         at::NoGradGuard no_grad;
         const auto [d, l, bv, av] = unpacked([&] { return std::tuple(dt_raw.unpack(), lam_raw.unpack(), bias.unpack(), alog.unpack()); });
         c10::cuda::CUDAGuard guard(d.device());
-        const int64_t H = d.size(-1), rows = d.numel() / H;
+        const int64_t H = d.size(-1), rows = rows_of(d, H);
         Tensor g[4];
         for (int i = 0; i < 4; ++i) g[i] = grads[i].defined() ? cast(grads[i].contiguous(), d.scalar_type()) : at::zeros_like(d);
         const Tensor dd = at::empty_like(d), dl = at::empty_like(d), db = empty_f32({H}, d), da = empty_f32({H}, d);
@@ -731,7 +733,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> trapezoid(const Tensor& dt_raw, const
         bias = f32(cast(dt_bias.contiguous(), type));
         alog = f32(cast(A_log.contiguous(), type));
         for (Tensor& t : o) t = at::empty_like(d);
-        check(ssd_b200_trapezoid_fwd(dtype_code(d), d.numel() / H, H, ptr(d), ptr(l), ptr<float>(bias), ptr<float>(alog), ptr(o[0]), ptr(o[1]), ptr(o[2]),
+        check(ssd_b200_trapezoid_fwd(dtype_code(d), rows_of(d, H), H, ptr(d), ptr(l), ptr<float>(bias), ptr<float>(alog), ptr(o[0]), ptr(o[1]), ptr(o[2]),
                                      ptr(o[3]), stream_of(d)));
     }
     if (wants_grad({&dt_raw, &lam_raw, &dt_bias, &A_log})) {

@@ -267,3 +267,12 @@ def test_rmsnorm_backward_takes_any_workspace_address(pkg, cabi, D):
         res.append((dx, dw))
     for a, b in zip(*res):
         assert float((a - b).abs().max()) <= 2e-6 * float(b.abs().max())
+
+
+def test_tensors_without_columns_are_refused(pkg, cabi):
+    """An exception, not the end of the process (the number of rows is a quotient by the columns)."""
+    e = torch.empty(2, 3, 0, device=DEV)
+    w = torch.empty(0, device=DEV)
+    for call in (lambda: pkg.fused_rmsnorm(e, w, EPS), lambda: pkg.fused_gate_norm(e, e, w, EPS), lambda: pkg.fused_trapezoidal(e, e, w, w)):
+        with pytest.raises((ValueError, RuntimeError, ZeroDivisionError)):
+            call()
