@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
 // ------------------------------------------------------------------------------------------
 // The same from the per-position log-decay itself (dt * A_head, or `a` as given, fp32 or bf16), which is read once in the
 // caller's (b,T,h) layout through a shared-memory transpose and scanned inside each tile (warp per head, 32-lane segments
-// scanned side by side); also writes a_cumsum (b,h,c,l) in natural-log units.  Chunks of any length: where one
+// scanned side by side); also writes a_cumsum (b,h,c,l) in natural-log units, where one is wanted (a backward without
+// kept states runs this too, so that its per-position arrays have the forward's bits).  Chunks of any length: where one
 // ends inside the tile its sums come from a second, segmented scan of the same values (CUT), so that they carry no
 // rounding of the positions before the chunk; where a chunk began in an earlier tile, the block adds up the positions
 // between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
             } else {
                 c[s4] = v[s4] + before;
             }
-            if (tt < rows) cum[oc + tt] = c[s4];
+            if (cum && tt < rows) cum[oc + tt] = c[s4];
             const float w = v[s4] * 1.4426950408889634f;
             tcum[o + tt] = w;
             const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);

@@ -189,6 +189,19 @@ inline int launch_tile_cumsum(const Dims& d, const float* cum, const float* dt, 
     return 0;
 }
 
+// The same from the log-decays (`args` of a forward or a backward), and a_cumsum unless `cum` is null.
+template <class Args>
+inline int launch_cumsum_tile_fused(const Args* a, const Dims& d, float* cum, float* tcum, float* dtT, float* skipT, int* extreme, cudaStream_t st,
+                                    char* err, size_t errn) {
+    const int nt = tiles_of(d.T);
+    const dim3 g(nt, (d.h + 31) / 32, d.b);
+    const bool cut = d.l % LT != 0;  // a chunk ends inside a tile
+    SSD_LAUNCH(prof::K_CUMSUM, st, ((cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>)<<<g, 256, 0, st>>>(
+        a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, cum, tcum, dtT, a->skip, skipT, extreme, d.T, nt * LT, d.h, d.l)));
+    SSD_TC_CHECK("cumsum_tile_fused");
+    return 0;
+}
+
 // Cuts the walk of P into pieces where that pays and the workspace has the room, and summarises them.
 template <bool REV>
 inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace, size_t bytes, int* pieces, cudaStream_t st, char* err, size_t errn) {
@@ -234,11 +247,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     if (cudaMemsetAsync(status, 0, 8, st) != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "memset failed");
     if (!a->cumsum_is_input && !aux_valid && d.l <= kFusedChunkMax) {
         // the within-chunk cumulative sums, the tile-cumulative log2 copies, the transposes and the flag in one kernel
-        const dim3 g(nt, (d.h + 31) / 32, d.b);
-        const bool cut = d.l % LT != 0;  // a chunk ends inside a tile
-        SSD_LAUNCH(prof::K_CUMSUM, st, ((cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>)<<<g, 256, 0, st>>>(
-            a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, tcum, dtT, a->skip, skipT, extreme, d.T, Tp, d.h, d.l)));
-        SSD_TC_CHECK("cumsum_tile_fused");
+        if (int rc = launch_cumsum_tile_fused(a, d, a->a_cumsum, tcum, dtT, skipT, extreme, st, err, errn)) return rc;
     } else {
         if (!a->cumsum_is_input) {
             const size_t sm = (size_t)d.l * (d.h + 1) * 4;
@@ -320,8 +329,11 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         dtT = a->dt ? tcum + bht : nullptr;
         skipT = a->skip ? tcum + 2 * bht : nullptr;
         extreme = (int*)(tcum + 3 * bht);
-    } else if (int rc = launch_tile_cumsum(d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn)) {
-        return rc;
+    } else {  // as the forward made them: from the log-decays, or from the sums it was given
+        const bool decays = !a->cumsum_is_input && d.l <= kFusedChunkMax && (a->a || (a->dt && a->A_head));
+        if (int rc = decays ? launch_cumsum_tile_fused(a, d, nullptr, tcum, dtT, skipT, extreme, st, err, errn)
+                            : launch_tile_cumsum(d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn))
+            return rc;
     }
     if (int rc = set_walk_attrs(err, errn)) return rc;
     const uint64_t srows = (uint64_t)d.b * nt * d.h * DN;
