@@ -43,9 +43,10 @@ _SAVE_STATES = os.environ.get("SSD_B200_SAVE_STATES", "1") == "1"
 
 
 def set_save_states(flag: bool) -> None:
-    """Keep the per-tile recurrent states of the forward for the backward (default on: one bf16 buffer of
-    b*T*h*64 elements, the size of x at d_state 128) instead of recomputing them in the backward, which is
-    what the reference's input-only checkpointing corresponds to (src/kernels/ssd_scan.py:458)."""
+    """Keep the recurrent states of the forward for the backward (default on) instead of recomputing them in the backward,
+    which is what the reference's input-only checkpointing corresponds to (src/kernels/ssd_scan.py:458).  On the tensor-core
+    kernels that is one bf16 state per 128 positions (b*T*h*64 elements, the size of x), on the fp32 kernels one fp32 state
+    per chunk, and there only where it takes no more room than the chunk's x."""
     global _SAVE_STATES
     _SAVE_STATES = bool(flag)
 

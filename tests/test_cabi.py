@@ -89,6 +89,20 @@ def test_row_sums_of_squares_need_whole_tiles(cabi, T, refused):
     assert rc < 0 and (rc == cabi.EINVAL and "whole tiles" in cabi.last_error()) == refused
 
 
+def test_kept_states_take_no_more_room_than_x(cabi):
+    """What a forward holds for the backward on the SIMT path: at most x again and one state, nothing where a chunk's state is
+    larger than its x."""
+    lib = cabi.load()
+    for dtype, width in ((cabi.F32, 4), (cabi.BF16, 2)):
+        for n in (8, 16, 64, 128, 256):
+            for l in (16, 32, 64, 128):
+                s = _shape(cabi, dtype=dtype, path=cabi.PATH_SIMT, dstate=n, chunk=l)
+                x = s.batch * s.seqlen * s.nheads * s.headdim * width
+                got = lib.ssd_b200_states_bytes(C.byref(s))
+                assert got <= x + 256 + 4 * s.batch * s.nheads * s.headdim * n
+                assert (got > 0) == (n * 4 <= l * width)
+
+
 def test_operator_rejects_cpu_tensors(pkg, cabi):
     x = torch.zeros(1, 64, 2, 8)
     with pytest.raises(AssertionError):
