@@ -240,18 +240,95 @@ def test_fp32_head_splits_and_wide_states(pkg, cabi, oracle, b, T, h, p, n, g, l
     check_mamba2(pkg, oracle, cfg, TOL_FP32, init=True, dfinal=True, seed=99)
 
 
-def test_unaligned_inputs(pkg, cabi, oracle):
-    """Tensors that start between two 16-byte boundaries."""
-    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=192, nheads=2, ngroups=1, chunk=64)
+def _shifted(t):
+    """The same values on the GPU, starting one element behind a 16-byte boundary."""
+    out = torch.empty(t.numel() + 8, dtype=t.dtype, device=DEV)[1:t.numel() + 1].view(t.shape).copy_(t)
+    assert out.data_ptr() % 16 and out.is_contiguous()
+    return out
+
+
+@pytest.mark.parametrize("T", [256, 192])
+def test_unaligned_inputs(pkg, cabi, T):
+    """Tensors that start between two 16-byte boundaries, through the Python operators: copied to where the kernels want them."""
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=T, nheads=2, ngroups=1, chunk=64)
     inp = pkg.make_inputs(cfg, seed=5)
-    def shifted(t):
-        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
-        buf[1:] = t.to(DEV).flatten()
-        return buf[1:].view(t.shape)
-    got = pkg.ssd_mamba2(shifted(inp["x"]), inp["dt"].to(DEV), inp["A_head"].to(DEV), shifted(inp["B"]), shifted(inp["C"]),
+    got = pkg.ssd_mamba2(_shifted(inp["x"]), inp["dt"].to(DEV), inp["A_head"].to(DEV), _shifted(inp["B"]), _shifted(inp["C"]),
                          inp["D"].to(DEV), cfg.chunk)
     want = pkg.ssd_mamba2(*[inp[k].to(DEV) for k in ("x", "dt", "A_head", "B", "C", "D")], cfg.chunk)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def _cabi_passes(pkg, cabi, cfg, inp, shifted, path, ws_bytes=None):
+    """Forward and backward of the Mamba-2 form straight through the C ABI, the tensors named in `shifted` off the 16-byte
+    boundaries; returns (return codes, outputs)."""
+    import ctypes
+    lib, S = cabi.load(), pkg.ssd_scan
+    P, st = S._ptr, S._stream(torch.device(DEV))
+    b, T, h, p, n = cfg.batch, cfg.seqlen, cfg.nheads, cfg.headdim, cfg.d_state
+    def place(name, t):
+        return _shifted(t) if name in shifted else t.to(DEV).clone()
+    t = {k: place(k, inp[k]) for k in ("x", "B", "C", "dy")}
+    t.update({k: inp[k].to(DEV) for k in ("dt", "A_head", "D")})
+    o = {k: place(k, torch.zeros_like(inp[v])) for k, v in (("y", "x"), ("dx", "x"), ("dB", "B"), ("dC", "C"))}
+    o.update(final=torch.empty(b, h, p, n, device=DEV), cum=torch.zeros(b, h, T // cfg.chunk, cfg.chunk, device=DEV), ddt=torch.empty(b, T, h, device=DEV),
+             dA_head=torch.empty(h, device=DEV), dD=torch.empty(h, device=DEV))
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16 if cfg.dtype == "bf16" else cabi.F32, cabi.F32, path, b, T, h, p, n, cfg.ngroups, cfg.chunk)
+    rcs = []
+    for which in (cabi.PASS_FWD, cabi.PASS_BWD):
+        full = int(lib.ssd_b200_workspace_bytes(ctypes.byref(shape), which))
+        ws = torch.empty(full, dtype=torch.uint8, device=DEV)
+        nb = full if ws_bytes is None else ws_bytes[which]
+        if which == cabi.PASS_FWD:
+            a = cabi.FwdArgs(shape, P(t["x"]), None, P(t["dt"]), P(t["A_head"]), P(t["D"]), P(t["B"]), P(t["C"]), None, P(o["y"]), P(o["final"]),
+                             P(o["cum"]), 0, 0, P(ws), nb)
+            rcs.append(lib.ssd_b200_fwd(ctypes.byref(a), st))
+        else:
+            a = cabi.BwdArgs(shape, P(t["x"]), None, P(t["dt"]), P(t["A_head"]), P(t["D"]), P(t["B"]), P(t["C"]), None, P(o["cum"]), P(t["dy"]), None,
+                             P(o["dx"]), P(o["dB"]), P(o["dC"]), None, P(o["ddt"]), P(o["dA_head"]), P(o["dD"]), None, 0, 0, P(ws), nb)
+            rcs.append(lib.ssd_b200_bwd(ctypes.byref(a), st))
+        torch.cuda.synchronize()
+    return rcs, o
+
+
+@pytest.mark.parametrize("shifted", [("x",), ("B", "C"), ("y",), ("dy", "dx"), ("dB",), ("x", "B", "C", "y", "dy", "dx", "dB", "dC")])
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_unaligned_tensors_through_the_c_abi(pkg, cabi, dtype, shifted):
+    """The SIMT kernels take any address: the same bits as with aligned tensors.  The tensor-core kernels refuse on the host."""
+    cfg = replace(pkg.CONFIGS[2], dtype=dtype, batch=2, seqlen=192, nheads=4, ngroups=2, chunk=64)
+    inp = pkg.make_inputs(cfg, seed=6)
+    rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
+    rc1, got = _cabi_passes(pkg, cabi, cfg, inp, shifted, cabi.PATH_AUTO)
+    assert rc0 == rc1 == [0, 0]
+    for k in want:
+        assert torch.equal(want[k], got[k]), k
+    if dtype == "bf16":
+        whole = replace(cfg, seqlen=256)
+        rcs, _ = _cabi_passes(pkg, cabi, whole, pkg.make_inputs(whole, seed=6), shifted, cabi.PATH_AUTO)
+        refused = [bool({"x", "B", "C", "y"} & set(shifted)), bool({"x", "B", "C", "dy", "dx", "dB", "dC"} & set(shifted))]
+        assert [rc == cabi.EINVAL for rc in rcs] == refused
+
+
+def test_walk_in_one_piece_where_the_workspace_has_no_room(pkg, cabi):
+    """With less workspace than several pieces need, but enough for one, the walks run in one; with a byte less they are refused."""
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=4096, nheads=6, ngroups=2, chunk=128)
+    inp = pkg.make_inputs(cfg, seed=7)
+    lib = cabi.load()
+    import ctypes
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, 1, 4096, 6, 64, 128, 2, 128)
+    def up(v):
+        return (v + 255) // 256 * 256
+    nt, bht, state = 32, up(6 * 4096 * 4), up(6 * 64 * 128 * 4)
+    fwd = 256 + 3 * bht
+    bwd = fwd + 2 * up(6 * nt * 64 * 128 * 2) + 2 * state + 3 * bht + up(6 * nt * 32) + 2 * up(6 * nt * 4)
+    assert lib.ssd_b200_workspace_bytes(ctypes.byref(shape), cabi.PASS_FWD) > fwd
+    assert lib.ssd_b200_workspace_bytes(ctypes.byref(shape), cabi.PASS_BWD) > bwd
+    rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
+    rc1, got = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {cabi.PASS_FWD: fwd, cabi.PASS_BWD: bwd})
+    assert rc0 == rc1 == [0, 0]
+    for k in want:
+        assert rel_err(got[k], want[k]) < TOL_BF16, k
+    rc2, _ = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {cabi.PASS_FWD: fwd - 1, cabi.PASS_BWD: bwd - 1})
+    assert rc2 == [cabi.EWORKSPACE, cabi.EWORKSPACE]
 
 
 @pytest.mark.parametrize("h,p,n,g,l,T", [(3, 24, 12, 1, 32, 96), (4, 80, 40, 2, 48, 96), (6, 16, 72, 3, 100, 200),
@@ -569,7 +646,7 @@ def test_saved_states_equal_recomputed_states(pkg, cabi, chunk):
 
 
 @pytest.mark.parametrize("b,T,h,g,p,n,chunk", [(1, 4096, 6, 2, 64, 128, 128), (1, 3008, 30, 5, 64, 64, 64), (2, 6016, 4, 4, 48, 128, 64),
-                                               (1, 16384, 9, 1, 64, 128, 256)])
+                                               (1, 16384, 9, 1, 64, 128, 256), (1, 6016, 56, 8, 64, 128, 128)])
 def test_walks_in_pieces(pkg, cabi, oracle, tensor_cores, b, T, h, g, p, n, chunk):
     """Few (batch, head) pairs and a long sequence: the walks run in pieces side by side, seeded from summaries.  Several pieces, a
     short last piece, summaries in parts, states in and out, columns below the tile's; against the oracle, and bit for bit the same
