@@ -21,7 +21,7 @@ namespace prof {
 // Launch accounting and optional per-kernel CUDA-event timing (benchmark use, one host thread).
 const char* const kNames[K_COUNT] = {
     "chunk_cumsum", "chunk_state", "state_passing", "chunk_scan", "chunk_dstate", "state_passing_rev",
-    "bwd_row", "bwd_col", "decay_grad", "reduce_batch", "cache_L", "cache_decay_chunk", "state_prefix",
+    "chunk_bwd", "decay_grad", "reduce_batch", "cache_L", "cache_decay_chunk", "state_prefix",
     "tc_fwd_walk", "tc_bwd_state", "tc_bwd_walk", "tc_aux", "tc_summary", "tc_bwd_walk_alt", "tc_fwd_walk_alt", "exchange"};
 std::atomic<long long> g_launches{0};
 bool g_enabled = false;
@@ -278,7 +278,7 @@ int launch_chunk_bwd(ssd::simt::Params P, cudaStream_t st) {
     P.share_ws = chunk_bwd_smem(P.d, PT, false) > (PT * NTN == 1 ? 113 : 227) * 1024;
     const size_t sm = chunk_bwd_smem(P.d, PT, P.share_ws);
     if (int rc = set_smem<chunk_bwd_kernel<T, PT, NTN>>(sm, "chunk_bwd")) return rc;
-    SSD_LAUNCH(ssd::prof::K_BWD_COL, st, (chunk_bwd_kernel<T, PT, NTN><<<dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st>>>(P)));
+    SSD_LAUNCH(ssd::prof::K_CHUNK_BWD, st, (chunk_bwd_kernel<T, PT, NTN><<<dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st>>>(P)));
     CUDA_LAUNCH_CHECK("chunk_bwd");
     return 0;
 }

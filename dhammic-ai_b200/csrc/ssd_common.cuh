@@ -34,7 +34,7 @@ __device__ __forceinline__ size_t st_off(const Dims& d, int bb, int k, int hh) {
 namespace prof {
 // Kernel slots for launch accounting / optional per-kernel timing (definitions in ssd_b200_api.cu).
 enum Kernel {
-    K_CUMSUM = 0, K_CHUNK_STATE, K_STATE_PASS, K_CHUNK_SCAN, K_CHUNK_DSTATE, K_STATE_PASS_REV, K_BWD_ROW, K_BWD_COL,
+    K_CUMSUM = 0, K_CHUNK_STATE, K_STATE_PASS, K_CHUNK_SCAN, K_CHUNK_DSTATE, K_STATE_PASS_REV, K_CHUNK_BWD,
     K_DECAY, K_REDUCE, K_CACHE_L, K_CACHE_DC, K_PREFIX, K_TC_FWD, K_TC_BWD_STATE, K_TC_BWD, K_TC_AUX, K_TC_SUMMARY,
     K_TC_BWD_ALT, K_TC_FWD_ALT, K_EXCHANGE, K_COUNT
 };

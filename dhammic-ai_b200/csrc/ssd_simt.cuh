@@ -27,7 +27,7 @@
 // memory.  So a block of the forward and of the backward takes as few heads of a group as it needs to fill the chip (dB and dC of a
 // group are then summed over its blocks), the row and the column pass of the backward are one launch, states are kept from the forward,
 // and the products read shared memory 16 bytes at a time without bank conflicts.  Forward + backward of (2, 512, 8 heads, 64,
-// d_state 64, chunk 64): 665 us of kernels with one block per group and 4-byte reads, 62 us now.
+// d_state 64, chunk 64): 665 us of kernels with one block per group and 4-byte reads, 82 us now.
 //
 // The decay gradient is a small difference of large row and column sums; its rounding (about 1e-5 of dA_head) follows from the
 // order in which each element is summed.  That order is the same for any thread layout here: products run through k one by

@@ -77,6 +77,7 @@ inline Pieces pieces_of(const Dims& d, bool reverse) {
         const int pt = (nt + P - 1) / P, np = (nt + pt - 1) / pt;
         const int want = (int)std::max(1LL, std::min({(long long)pt, kPieceSms / (bh * (np - 1)), (long long)kMaxEntries / (np - 1)}));
         const int ps = (pt + want - 1) / want, parts = (pt + ps - 1) / ps;
+        if (reverse && nt - (np - 1) * pt <= (parts - 1) * ps) continue;  // the short last piece would have an empty part
         const double c = tile * pt + 0.8 * ps + 12.0 + 0.6 * parts * (np - 1);
         if (c < cost) {
             cost = c;

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     const int hh0 = blockIdx.x * NH, bb = blockIdx.y;
     const int gg = hh0 / P.hpg;
     const int part = (int)blockIdx.z % P.parts, piece = P.z0 + (int)blockIdx.z / P.parts;
-    const int k0 = piece * P.pt + part * P.ps, nt = max(0, min(min(P.ps, P.pt - part * P.ps), P.nt - k0));  // (the last piece can be short)
+    const int k0 = piece * P.pt + part * P.ps, nt = min(min(P.ps, P.pt - part * P.ps), P.nt - k0);  // at least one (see Pieces)
     // forward: tiles nt-1 .. 0 of the part; reverse: 0 .. nt-1
     auto tile_of = [&](int it) { return k0 + (REV ? it : nt - 1 - it); };
 
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         const float* tcum = P.tcum + bh * P.Tp;
         const float* dtT = (!REV && P.dtT) ? P.dtT + bh * P.Tp : nullptr;
         float run = 0.f;  // forward: log2-decay of the tiles after this one; reverse: of the tiles before it
-        const size_t o0 = (size_t)max(0, min(tile_of(0), P.nt - 1)) * LT;
+        const size_t o0 = (size_t)tile_of(0) * LT;
         float c_n = tcum[o0 + row];
         float S_n = tcum[o0 + LT - 1];
         float dt_n = dtT ? dtT[o0 + row] : 1.f;
@@ -161,15 +161,10 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         // `run` is now the total log2-decay of the piece
         const int last = nt - 1;
         uint32_t r[32];
-        if (nt > 0) {  // (block-uniform)
-            mbar_wait(&bar_m[last % NS], (last / NS) & 1, &failed);
-            tc_fence_after();
-            tmem_ld32(tm + lane_base(warp) + hs * 64 + hf * 32, r);
-            tmem_ld_wait();
-        } else {
-#pragma unroll
-            for (int q = 0; q < 32; ++q) r[q] = 0u;
-        }
+        mbar_wait(&bar_m[last % NS], (last / NS) & 1, &failed);
+        tc_fence_after();
+        tmem_ld32(tm + lane_base(warp) + hs * 64 + hf * 32, r);
+        tmem_ld_wait();
         const float dec = exp2f(run);
         float v[32];  // accumulator row = n, columns = p
         load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, v);

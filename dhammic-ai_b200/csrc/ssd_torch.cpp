@@ -1,6 +1,7 @@
 // Host path of the operators: argument checks, allocations, autograd nodes and the calls into the C ABI (include/ssd_b200.h), native
-// so that a call costs the CPU a few microseconds per launch.  (As Python autograd functions over ctypes the forward and
-// backward of one scan took the host about 200 us, more than the GPU needs for any call below some 300 MB.)
+// so that a call costs the CPU about 12 us per launch: forward + backward of one scan on the fp32 kernels, nine launches, take
+// the host 110 us.  (As Python autograd functions over ctypes about 200 us, more than the GPU needs for any call below some
+// 300 MB.)
 //
 // Every operator is one autograd node.  A forward runs without recording; when a gradient is wanted the node keeps its inputs
 // as saved variables (so that an input overwritten in place is noticed) and the buffers the kernels left for the backward.
@@ -373,7 +374,6 @@ std::tuple<Tensor, Tensor, Tensor> operator_scan(const Tensor& x, const Tensor& 
 // ---------------------------------------------------------------------------------------------------- norm and gate
 // Rows of `cols` values (of zero columns: none, which the C ABI refuses).
 int64_t rows_of(const Tensor& t, int64_t cols) { return cols ? t.numel() / cols : 0; }
-int64_t ws_floats(size_t n) { return static_cast<int64_t>(n); }
 
 struct NormGrads {
     Tensor dx, dz, dw;
@@ -381,7 +381,7 @@ struct NormGrads {
 NormGrads norm_backward(const Tensor& x, const Tensor& w, const Tensor& z, const Tensor& dout, const Tensor& rstd) {
     const int64_t D = w.numel(), rows = rstd.numel();
     NormGrads g{at::empty_like(x), z.defined() ? at::empty_like(z) : Tensor(), empty_f32({D}, x)};
-    const Tensor ws = empty_f32({ws_floats(ssd_b200_rmsnorm_ws_floats(rows, D))}, x);
+    const Tensor ws = empty_f32({static_cast<int64_t>(ssd_b200_rmsnorm_ws_floats(rows, D))}, x);
     check(ssd_b200_rmsnorm_bwd(dtype_code(x), rows, D, ptr(x), ptr<float>(w), ptr(z), ptr(dout), ptr<float>(rstd), ptr(g.dx), ptr(g.dz),
                                ptr<float>(g.dw), ptr<float>(ws), stream_of(x)));
     return g;
@@ -559,7 +559,7 @@ struct Mamba3Node : ScanNode {
         // a = dt A_head, with the two per-head sums, in one kernel on the (b,T,h) tensors
         const Tensor dlam = at::empty_like(dw), ddt = at::empty_like(dw), dAh = empty_f32({h}, xv);
         const Tensor dD = Dv.defined() ? empty_f32({h}, xv) : Tensor();
-        const Tensor ws = empty_f32({ws_floats(ssd_b200_m3_chain_ws_floats(&block))}, xv);
+        const Tensor ws = empty_f32({static_cast<int64_t>(ssd_b200_m3_chain_ws_floats(&block))}, xv);
         check(ssd_b200_m3_chain_bwd(&block, ptr<float>(dw), ptr<float>(dyx), ptr<float>(sd), ptr<float>(dtv), ptr<float>(lamv), ptr<float>(g.da),
                                     ptr<float>(Ah), ptr<float>(dlam), ptr<float>(ddt), ptr<float>(dAh), ptr<float>(dD), ptr<float>(ws), st));
         return {dx, cast(ddt, dt_type), cast(dAh, A_type), dB, dC, cast(dD, D_type), cast(dang, raw_type), cast(dlam, lam_type)};
@@ -703,7 +703,7 @@ struct TrapezoidNode : SavingNode {
         Tensor g[4];
         for (int i = 0; i < 4; ++i) g[i] = grads[i].defined() ? cast(grads[i].contiguous(), d.scalar_type()) : at::zeros_like(d);
         const Tensor dd = at::empty_like(d), dl = at::empty_like(d), db = empty_f32({H}, d), da = empty_f32({H}, d);
-        const Tensor ws = empty_f32({ws_floats(ssd_b200_trapezoid_ws_floats(rows, H))}, d);
+        const Tensor ws = empty_f32({static_cast<int64_t>(ssd_b200_trapezoid_ws_floats(rows, H))}, d);
         check(ssd_b200_trapezoid_bwd(dtype_code(d), rows, H, ptr(d), ptr(l), ptr<float>(bv), ptr<float>(av), ptr(g[0]), ptr(g[1]), ptr(g[2]), ptr(g[3]),
                                      ptr(dd), ptr(dl), ptr<float>(db), ptr<float>(da), ptr<float>(ws), stream_of(d)));
         return {dd, cast(dl, lam_type), cast(db, bias_type), cast(da, alog_type)};

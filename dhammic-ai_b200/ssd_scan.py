@@ -192,26 +192,6 @@ def _run_fwd(x, a, dt, A_head, D, B, Cm, chunk, init4, a_cumsum_in, want_states=
     return y, final, cum, shape, states
 
 
-def _run_bwd_scaled(shape, x, a, w, skip, B, Cm, cum, dY, states):
-    """Backward launcher of the scaled operator form (X = x * w, log-decay a, y += skip * x).  Returns
-    (dx, da, dw, dskip, dB, dC): dx complete, the three (b,T,h) gradients fp32."""
-    lib = _cabi.load()
-    dev = x.device
-    b, T, h, p = x.shape
-    with torch.cuda.device(dev):
-        dy = dY.contiguous().to(x.dtype)
-        dx, dB, dC = torch.empty_like(x), torch.empty_like(B), torch.empty_like(Cm)
-        da = torch.empty(b, T, h, dtype=torch.float32, device=dev)
-        dw, dskip = torch.empty_like(da), torch.empty_like(da)
-        ws = _workspace(lib, shape, _cabi.PASS_BWD, dev)
-        args = _cabi.BwdArgs(shape, _ptr(x), _ptr(a), _ptr(w), None, None, _ptr(B), _ptr(Cm), None, _ptr(cum), _ptr(dy),
-                             None, _ptr(dx), _ptr(dB), _ptr(dC), _ptr(da), _ptr(dw), None, None, None, 0, 0, _ptr(ws),
-                             ws.numel(), _ptr(states), _ptr(skip), _ptr(dskip))
-        _cabi.check(lib.ssd_b200_bwd(C.byref(args), _stream(dev)))
-        _status(lib, shape, ws, dev)
-    return dx, da, dw, dskip, dB, dC
-
-
 class FusedSSDScan:
     """Same call signature as the reference's FusedSSDScan (src/kernels/ssd_scan.py:441-465)."""
 

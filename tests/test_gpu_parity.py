@@ -911,8 +911,8 @@ def test_scaled_operator_form_matches_mamba2_form(pkg, cabi):
     """The scan's third calling form (log-decay a, input weight dt and skip coefficient all per position; what the
     one-scan Mamba-3 composition uses) against the Mamba-2 form with a = dt * A_head and skip = D on the same data:
     same y, dx, dB, dC, and  ddt = d weight + da * A_head,  dA_head = sum da * dt,  dD = sum dskip."""
-    import importlib
-    S = importlib.import_module("dhammic-ai_b200.ssd_scan")
+    import ctypes
+    S, lib, P = pkg.ssd_scan, cabi.load(), pkg.ssd_scan._ptr
     cfg = pkg.shrink(pkg.CONFIGS[2], 2, 512)
     inp = {k: v.to(DEV) for k, v in pkg.make_inputs(cfg).items()}
     want = mamba2_gpu(pkg, {k: v.cpu() for k, v in inp.items()}, cfg.chunk)
@@ -921,7 +921,12 @@ def test_scaled_operator_form_matches_mamba2_form(pkg, cabi):
     skip = inp["D"].expand(b, T, h).contiguous()
     y, final, cum, shape, states = S._run_fwd(inp["x"], a, inp["dt"], None, None, inp["B"], inp["C"], cfg.chunk, None, None,
                                              want_states=True, skip=skip)
-    dx, da, dw, dskip, dB, dC = S._run_bwd_scaled(shape, inp["x"], a, inp["dt"], skip, inp["B"], inp["C"], cum, inp["dy"], states)
+    dx, dB, dC = (torch.empty_like(inp[k]) for k in ("x", "B", "C"))
+    da, dw, dskip = (torch.empty(b, T, h, device=DEV) for _ in range(3))
+    ws = S._workspace(lib, shape, cabi.PASS_BWD, dx.device)
+    args = cabi.BwdArgs(shape, P(inp["x"]), P(a), P(inp["dt"]), None, None, P(inp["B"]), P(inp["C"]), None, P(cum), P(inp["dy"]), None, P(dx), P(dB), P(dC),
+                        P(da), P(dw), None, None, None, 0, 0, P(ws), ws.numel(), P(states), P(skip), P(dskip))
+    cabi.check(lib.ssd_b200_bwd(ctypes.byref(args), S._stream(dx.device)))
     torch.cuda.synchronize()
     got = {"y": y, "final_state": final, "dx": dx, "dB": dB, "dC": dC,
            "ddt": dw + da * inp["A_head"], "dA_head": (da * inp["dt"]).sum((0, 1)), "dD": dskip.sum((0, 1))}
