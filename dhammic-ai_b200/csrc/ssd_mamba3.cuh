@@ -268,22 +268,31 @@ template <class TA, int N>
 struct alignas(N * sizeof(TA)) AngleVec {
     TA v[N];
 };
+// N columns' angles of `rows` positions added to `s` one by one, sixteen loads ahead of the sum.
+template <class TA, int N>
+__device__ __forceinline__ void add_angles(const TA* __restrict__ p, int rows, int E, float (&s)[N]) {
+    constexpr int U = 16;
+    for (int i = 0; i < rows; i += U) {
+        AngleVec<TA, N> a[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) a[q] = *reinterpret_cast<const AngleVec<TA, N>*>(p + (size_t)min(i + q, rows - 1) * E);
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (i + q < rows)
+#pragma unroll
+                for (int c = 0; c < N; ++c) s[c] += to_f(a[q].v[c]);
+    }
+}
 template <class TA, int N>
 __global__ void __launch_bounds__(256) angle_segsum_kernel(const TA* __restrict__ raw, float* __restrict__ segsum, int Tlen, int E) {
     const int e = (blockIdx.y * 256 + threadIdx.x) * N;
     if (e >= E) return;
-    const int t0 = blockIdx.x * SEG, t1 = min(Tlen, t0 + SEG);
-    const TA* p = raw + ((size_t)blockIdx.z * Tlen + t0) * E + e;
-    AngleVec<float, N> s;
+    const int t0 = blockIdx.x * SEG;
+    float s[N];
 #pragma unroll
-    for (int q = 0; q < N; ++q) s.v[q] = 0.f;
-#pragma unroll 32
-    for (int t = t0; t < t1; ++t, p += E) {
-        const AngleVec<TA, N> a = *reinterpret_cast<const AngleVec<TA, N>*>(p);
-#pragma unroll
-        for (int q = 0; q < N; ++q) s.v[q] += to_f(a.v[q]);
-    }
-    store_angles<N>(segsum + ((size_t)blockIdx.z * gridDim.x + blockIdx.x) * E + e, s.v);
+    for (int q = 0; q < N; ++q) s[q] = 0.f;
+    add_angles<TA, N>(raw + ((size_t)blockIdx.z * Tlen + t0) * E + e, min(SEG, Tlen - t0), E, s);
+    store_angles<N>(segsum + ((size_t)blockIdx.z * gridDim.x + blockIdx.x) * E + e, s);
 }
 // In place: the sum of all segments before.
 __global__ void __launch_bounds__(64) angle_prefix_kernel(float* __restrict__ segsum, int nseg, int E) {
@@ -302,9 +311,10 @@ __global__ void __launch_bounds__(64) angle_prefix_kernel(float* __restrict__ se
         }
     }
 }
-// Whole segments per block from about four blocks per SM on.
+// Whole segments per block from six blocks per SM on: four are resident, and one and a half rounds of long blocks are no better
+// than several of short ones (620 blocks: 250 us, in short blocks 170; 2048 blocks: 721 against 773 us).
 inline bool rope_walks_segments(int b, int T, int E, int N) {
-    return (long long)b * ((T + SEG - 1) / SEG) * ((E / N + 255) / 256) >= 4 * 148;
+    return (long long)b * ((T + SEG - 1) / SEG) * ((E / N + 255) / 256) >= 6 * 148;
 }
 template <class T, class TA, int V, int WALK>
 __global__ void __launch_bounds__(256) rope_walk_fwd_kernel(const T* __restrict__ B, const T* __restrict__ C, const TA* __restrict__ raw,
@@ -321,15 +331,7 @@ __global__ void __launch_bounds__(256) rope_walk_fwd_kernel(const T* __restrict_
     const size_t a0 = bt * E + (size_t)unit * N, o0 = bt * h * n + (size_t)unit * V;
     float run[N];
     load_angles<N>(segsum + ((size_t)blockIdx.z * nseg + seg) * E + (size_t)unit * N, run);
-    if (WALK < SEG) {
-        const TA* p = raw + a0 - (size_t)(t0 - seg * SEG) * E;
-#pragma unroll 16
-        for (int t = seg * SEG; t < t0; ++t, p += E) {
-            const AngleVec<TA, N> a = *reinterpret_cast<const AngleVec<TA, N>*>(p);
-#pragma unroll
-            for (int q = 0; q < N; ++q) run[q] += to_f(a.v[q]);
-        }
-    }
+    if (WALK < SEG) add_angles<TA, N>(raw + a0 - (size_t)(t0 - seg * SEG) * E, t0 - seg * SEG, E, run);
 #pragma unroll 4
     for (int i = 0; i < t1 - t0; ++i) {
         const AngleVec<TA, N> a = *reinterpret_cast<const AngleVec<TA, N>*>(raw + a0 + (size_t)i * E);
