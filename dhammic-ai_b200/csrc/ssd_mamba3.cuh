@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(64) angle_prefix_kernel(float* __restrict__ se
     }
 }
 // Whole segments per block from six blocks per SM on: four are resident, and one and a half rounds of long blocks are no better
-// than several of short ones (620 blocks: 250 us, in short blocks 170; 2048 blocks: 721 against 773 us).
+// than several of short ones (620 blocks: 250 us, in short blocks 170).
 inline bool rope_walks_segments(int b, int T, int E, int N) {
     return (long long)b * ((T + SEG - 1) / SEG) * ((E / N + 255) / 256) >= 6 * 148;
 }

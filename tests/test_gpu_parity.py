@@ -718,10 +718,12 @@ def test_mamba3_variant(pkg, cabi, oracle, dtype, tol):
 
 
 @pytest.mark.parametrize("T,h,g,n,chunk,ang32,shift", [(64, 1, 1, 40, 64, False, 0), (128, 4, 4, 128, 128, False, 0), (448, 5, 1, 64, 64, True, 0),
-                                                       (1120, 12, 2, 104, 32, False, 1), (160, 600, 1, 64, 32, False, 0)])
+                                                       (1120, 12, 2, 104, 32, False, 1), (160, 600, 1, 64, 32, False, 0),
+                                                       (192, 3, 1, 42, 64, False, 0), (256, 2, 1, 10, 128, True, 0)])
 def test_mamba3_angles_edges(pkg, cabi, oracle, T, h, g, n, chunk, ang32, shift):
     """The running sum of the angles where it can go wrong: one block of positions and several, a last one that is not full,
-    columns that do not fill the blocks, angles in fp32 and at an odd address, enough columns for the one-pass reverse sum.
+    columns that do not fill the blocks, angles in fp32 and at an odd address (copied before the kernels see them), enough columns
+    for the one-pass reverse sum, state columns that are no whole vectors.
     Against the oracle's two-call composition."""
     gen = torch.Generator().manual_seed(T + h)
     def randn(*s):
