@@ -258,6 +258,21 @@ def test_unaligned_inputs(pkg, cabi, T):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+def test_segments_of_partial_tiles_take_unaligned_tensors(pkg, cabi):
+    """The segmented scan hands its tensors on as they are; segments that end inside a tile run on kernels that take any address."""
+    import importlib
+    split = importlib.import_module("dhammic-ai_b200.distributed")
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=384, nheads=2, ngroups=1, chunk=96)
+    inp = pkg.make_inputs(cfg, seed=8)
+    res = []
+    for place in (lambda t: t.to(DEV), _shifted):
+        lv = [(place(inp[k]) if k in ("x", "B", "C") else inp[k].to(DEV)).requires_grad_(True) for k in ("x", "dt", "A_head", "B", "C", "D")]
+        y, _ = split.ssd_mamba2_segmented(*lv, cfg.chunk, segments=2)
+        res.append([y.detach()] + list(torch.autograd.grad([y], lv, [place(inp["dy"])])))
+    for u, v in zip(*res):
+        assert torch.equal(u, v)
+
+
 def _cabi_passes(pkg, cabi, cfg, inp, shifted, path, ws_bytes=None):
     """Forward and backward of the Mamba-2 form straight through the C ABI, the tensors named in `shifted` off the 16-byte
     boundaries; returns (return codes, outputs)."""
