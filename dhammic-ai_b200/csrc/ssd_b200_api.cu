@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "ssd_simt.cuh"
+#include "ssd_mma.cuh"
 #include "ssd_tc_host.cuh"
 #include "ssd_mamba3.cuh"
 #include "ssd_elementwise.cuh"
@@ -180,12 +181,52 @@ SimtWs simt_ws(const ssd::Dims& d, int pass) {
 // The `states` buffer of the SIMT path: what a forward keeps for the backward of the same inputs, the state entering every chunk
 // and the final state, but only where a chunk's state takes no more room than its x, so that a layer holds at most as much again as
 // its x from forward to backward.  Two launches less in the backward: (2, 512, 8 heads, 64), d_state 64, chunk 64, fp32, a single
-// forward + backward 134 us against 145.  bf16 (4, 1984, 20 heads, 64) with the same chunk, where the states would be twice x: 929 us
-// with, 1016 us without.
+// forward + backward 134 us against 145.
 size_t simt_states_bytes(const ssd_b200_shape& s) {
     const ssd::Dims d = dims_of(s);
+    if (ssd::mma::supported(s.dtype, d.p, d.n)) return 0;  // these kernels walk the states again
     if ((size_t)d.n * 4 > (size_t)d.l * (s.dtype == SSD_B200_BF16 ? 2 : 4)) return 0;
     return align_up(simt_states_elems(d) * 4) + (size_t)d.b * d.h * d.p * d.n * 4;
+}
+
+// Workspace of the same calls on the tensor-core kernels of ssd_mma.cuh.
+int mma_splits(const ssd::Dims& d) {
+    const long long base = (long long)ssd::mma::tiles(d.T) * d.b * d.g;
+    int s = 1;
+    while (s < d.hpg && (base * s < 2 * 148 || d.hpg % s)) ++s;
+    return s;
+}
+struct MmaWs {
+    size_t H, sums, Q, final_state, carry, g_row, g_col, ddtx, dyx, dAh_part, dD_part, dB_part, dC_part, total;
+};
+MmaWs mma_ws(const ssd::Dims& d, int pass) {
+    MmaWs w{};
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        size_t o = off;
+        off += align_up(bytes);
+        return o;
+    };
+    const size_t pieces = (size_t)d.b * ssd::mma::tiles(d.T) * d.h * 3 * d.p * d.n * 2;
+    w.H = take(pieces);
+    w.sums = take((size_t)d.b * ssd::mma::tiles(d.T) * d.h * 2 * ssd::mma::MT * 4);
+    if (pass == SSD_B200_PASS_BWD) {
+        const size_t bht = (size_t)d.b * d.h * d.T * 4, splits = mma_splits(d);
+        const size_t bc = splits > 1 ? (size_t)d.b * d.T * d.g * splits * d.n * 4 : 0;
+        w.Q = take(pieces);
+        w.final_state = take((size_t)d.b * d.h * d.p * d.n * 4);
+        w.carry = take((size_t)d.b * ssd::mma::tiles(d.T) * d.h * 8 * 4);
+        w.g_row = take(bht);
+        w.g_col = take(bht);
+        w.ddtx = take(bht);
+        w.dyx = take(bht);
+        w.dAh_part = take((size_t)d.b * d.h * 4);
+        w.dD_part = take((size_t)d.b * d.h * 4);
+        w.dB_part = take(bc);
+        w.dC_part = take(bc);
+    }
+    w.total = off;
+    return w;
 }
 
 #define CUDA_LAUNCH_CHECK(what)                                                              \
@@ -243,6 +284,60 @@ int launch_chunk_scan(const ssd::simt::Params& P, cudaStream_t st) {
     return 0;
 }
 
+// ---- the tensor-core kernels of ssd_mma.cuh (bf16, the same precision)
+// With the workspace these kernels need; summaries of a piece of the sequence stay on the SIMT kernels.
+bool mma_runs(const ssd_b200_fwd_args* a, const ssd::Dims& d) {
+    return ssd::mma::supported(a->shape.dtype, d.p, d.n) && !(a->flags & SSD_B200_FWD_STATES_ONLY) &&
+           a->workspace_bytes >= mma_ws(d, SSD_B200_PASS_FWD).total;
+}
+bool mma_runs(const ssd_b200_bwd_args* a, const ssd::Dims& d) {
+    return ssd::mma::supported(a->shape.dtype, d.p, d.n) && !(a->flags & SSD_B200_BWD_DINIT_ONLY) &&
+           a->workspace_bytes >= mma_ws(d, SSD_B200_PASS_BWD).total;
+}
+template <class Args>
+ssd::mma::Params mma_params(const Args* a, const ssd::Dims& d) {
+    ssd::mma::Params P{};
+    P.d = d;
+    P.nt = ssd::mma::tiles(d.T);
+    P.splits = mma_splits(d);
+    P.x = (const __nv_bfloat16*)a->x; P.B = (const __nv_bfloat16*)a->B; P.C = (const __nv_bfloat16*)a->C;
+    P.cum = a->cumsum_is_input ? a->a_cumsum : nullptr; P.a = a->dt ? nullptr : a->a; P.a_is_bf16 = a->shape.a_dtype == SSD_B200_BF16;
+    P.dt = a->dt; P.A_head = a->A_head; P.D = a->D; P.init = a->init;
+    return P;
+}
+template <bool WIDE>
+int launch_mma_states(const ssd::mma::Params& P, int dirs, cudaStream_t st) {
+    using namespace ssd::mma;
+    if (int rc = set_smem<state_kernel<WIDE>>(StateCfg::SMEM, "mma_states")) return rc;
+    const dim3 g(P.d.h * ((P.d.n + kStateCols - 1) / kStateCols), P.d.b, dirs);
+    SSD_LAUNCH(dirs == 2 ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, state_kernel<WIDE><<<g, kStateThreads, StateCfg::SMEM, st>>>(P));
+    CUDA_LAUNCH_CHECK("mma_states");
+    return 0;
+}
+template <int NN, bool WIDE>
+int mma_fwd_launches(const ssd::mma::Params& P, cudaStream_t st) {
+    using namespace ssd::mma;
+    if (int rc = launch_mma_states<WIDE>(P, 1, st)) return rc;
+    const size_t sm = ScanCfg<NN>::SMEM;
+    if (int rc = set_smem<scan_kernel<NN, WIDE>>(sm, "mma_scan")) return rc;
+    SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, (scan_kernel<NN, WIDE><<<dim3(P.nt * P.d.b, P.d.g * P.splits), NTHR, sm, st>>>(P)));
+    CUDA_LAUNCH_CHECK("mma_scan");
+    return 0;
+}
+template <int NN, bool WIDE>
+int mma_bwd_launches(const ssd::mma::Params& P, cudaStream_t st) {
+    using namespace ssd::mma;
+    if (int rc = launch_mma_states<WIDE>(P, 2, st)) return rc;
+    const size_t sm = BwdCfg<NN>::SMEM;
+    if (int rc = set_smem<bwd_kernel<NN, WIDE>>(sm, "mma_bwd")) return rc;
+    SSD_LAUNCH(ssd::prof::K_CHUNK_BWD, st, (bwd_kernel<NN, WIDE><<<dim3(P.nt * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st>>>(P)));
+    CUDA_LAUNCH_CHECK("mma_bwd");
+    const size_t pairs = P.splits > 1 ? (size_t)P.d.b * P.d.T * P.d.g * P.d.n / 2 : 0;
+    SSD_LAUNCH(ssd::prof::K_DECAY, st, decay_kernel<WIDE><<<(unsigned)(P.d.b * P.d.h + (pairs + kDecayThreads - 1) / kDecayThreads), kDecayThreads, 0, st>>>(P));
+    CUDA_LAUNCH_CHECK("mma_decay");
+    return 0;
+}
+
 template <class T>
 int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
     using namespace ssd::simt;
@@ -250,7 +345,8 @@ int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
     Params P = simt_params(dims_of(a->shape));
     const ssd::Dims& d = P.d;
     SimtWs w = simt_ws(d, SSD_B200_PASS_FWD);
-    if (a->workspace_bytes < w.total) return fail(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
+    const bool mma = mma_runs(a, d);
+    if (!mma && a->workspace_bytes < w.total) return fail(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
     P.x = a->x; P.dt = a->dt; P.A_head = a->A_head; P.D = a->D; P.B = a->B; P.C = a->C;
     P.init = a->init; P.cum = a->a_cumsum; P.final_state = a->final_state; P.y = a->y;
     P.states = a->states ? (float*)a->states : (float*)((char*)a->workspace + w.states);
@@ -262,10 +358,19 @@ int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
             a->dt ? nullptr : a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, d.T, d.h, d.l));
         CUDA_LAUNCH_CHECK("chunk_cumsum");
     }
-    if (int rc = simt_chunk_states<T>(P, 0, st)) return rc;
+    if (!mma)
+        if (int rc = simt_chunk_states<T>(P, 0, st)) return rc;
     if (a->logdecay_total) {
         SSD_LAUNCH(ssd::prof::K_CUMSUM, st, logdecay_total_kernel<<<(d.b * d.h + 127) / 128, 128, 0, st>>>(a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
         CUDA_LAUNCH_CHECK("logdecay_total");
+    }
+    if (mma) {
+        ssd::mma::Params M = mma_params(a, d);
+        const MmaWs wm = mma_ws(d, SSD_B200_PASS_FWD);
+        M.H = (__nv_bfloat16*)((char*)a->workspace + wm.H); M.sums = (float*)((char*)a->workspace + wm.sums);
+        M.final_state = a->final_state; M.y = (__nv_bfloat16*)a->y;
+        if (any_unaligned({a->x, a->B, a->C, a->y})) return d.n <= 64 ? mma_fwd_launches<64, false>(M, st) : mma_fwd_launches<128, false>(M, st);
+        return d.n <= 64 ? mma_fwd_launches<64, true>(M, st) : mma_fwd_launches<128, true>(M, st);
     }
     if (a->flags & SSD_B200_FWD_STATES_ONLY) return 0;
     return d.p <= TS ? launch_chunk_scan<T, 1>(P, st) : launch_chunk_scan<T, 2>(P, st);
@@ -289,11 +394,41 @@ int dispatch_chunk_bwd(const ssd::simt::Params& P, cudaStream_t st) {
     return launch_chunk_bwd<T, PT, 4>(P, st);
 }
 
+// dA_head and dD: the sums over the batch.
+int simt_head_sums(const ssd_b200_bwd_args* a, const float* dAh_part, const float* dD_part, const ssd::Dims& d, cudaStream_t st) {
+    SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::simt::reduce_batch_kernel<<<dim3((d.h + 127) / 128, a->D ? 2 : 1), 128, 0, st>>>(
+        dAh_part, a->dA_head, dD_part, a->dD, d.b, d.h));
+    CUDA_LAUNCH_CHECK("reduce_batch");
+    return 0;
+}
+
+int mma_bwd(const ssd_b200_bwd_args* a, const ssd::Dims& d, cudaStream_t st) {
+    const MmaWs w = mma_ws(d, SSD_B200_PASS_BWD);
+    char* ws = (char*)a->workspace;
+    ssd::mma::Params M = mma_params(a, d);
+    M.dy = (const __nv_bfloat16*)a->dy; M.dfinal = a->dfinal; M.dinit = a->dinit;
+    M.H = (__nv_bfloat16*)(ws + w.H); M.sums = (float*)(ws + w.sums); M.Q = (__nv_bfloat16*)(ws + w.Q); M.final_state = (float*)(ws + w.final_state);
+    M.dx = (__nv_bfloat16*)a->dx; M.dB = (__nv_bfloat16*)a->dB; M.dC = (__nv_bfloat16*)a->dC;
+    M.g_row = (float*)(ws + w.g_row); M.g_col = (float*)(ws + w.g_col); M.ddtx = (float*)(ws + w.ddtx);
+    M.dyx = (a->dt && a->D) ? (float*)(ws + w.dyx) : nullptr;
+    if (M.splits > 1) {
+        M.dB_part = (float*)(ws + w.dB_part);
+        M.dC_part = (float*)(ws + w.dC_part);
+    }
+    M.carry = (float*)(ws + w.carry); M.da = a->cumsum_is_input ? nullptr : a->da; M.ddt = a->ddt; M.dAh_part = (float*)(ws + w.dAh_part); M.dD_part = (float*)(ws + w.dD_part);
+    int rc;
+    if (any_unaligned({a->x, a->B, a->C, a->dy, a->dx, a->dB, a->dC})) rc = d.n <= 64 ? mma_bwd_launches<64, false>(M, st) : mma_bwd_launches<128, false>(M, st);
+    else rc = d.n <= 64 ? mma_bwd_launches<64, true>(M, st) : mma_bwd_launches<128, true>(M, st);
+    if (rc) return rc;
+    return a->dt ? simt_head_sums(a, M.dAh_part, M.dD_part, d, st) : 0;
+}
+
 template <class T>
 int simt_bwd(const ssd_b200_bwd_args* a, cudaStream_t st) {
     using namespace ssd::simt;
     Params P = simt_params(dims_of(a->shape));
     const ssd::Dims& d = P.d;
+    if (mma_runs(a, d)) return mma_bwd(a, d, st);
     SimtWs w = simt_ws(d, SSD_B200_PASS_BWD);
     if (a->workspace_bytes < w.total) return fail(SSD_B200_EWORKSPACE, "workspace %zu < %zu", a->workspace_bytes, w.total);
     char* ws = (char*)a->workspace;
@@ -320,12 +455,7 @@ int simt_bwd(const ssd_b200_bwd_args* a, cudaStream_t st) {
     const size_t total = P.splits > 1 ? (size_t)d.b * d.T * d.g * d.n : 0;
     SSD_LAUNCH(ssd::prof::K_DECAY, st, decay_grad_kernel<T><<<(unsigned)(d.b * d.h + (total + NTHR - 1) / NTHR), NTHR, 0, st>>>(P));
     CUDA_LAUNCH_CHECK("decay_grad");
-    if (a->dt) {
-        SSD_LAUNCH(ssd::prof::K_REDUCE, st, reduce_batch_kernel<<<dim3((d.h + 127) / 128, a->D ? 2 : 1), 128, 0, st>>>(
-            P.dAh_part, a->dA_head, P.dD_part, a->dD, d.b, d.h));
-        CUDA_LAUNCH_CHECK("reduce_batch");
-    }
-    return 0;
+    return a->dt ? simt_head_sums(a, P.dAh_part, P.dD_part, d, st) : 0;
 }
 
 // 1 = operator form (a), 2 = Mamba-2 form (dt, A_head[, D]), 3 = scaled operator form (a and dt[, skip]); < 0 = error
@@ -610,7 +740,9 @@ size_t ssd_b200_workspace_bytes(const ssd_b200_shape* shape, int pass) {
     int path = resolve_path(*shape);
     if (path < 0) return 0;
     ssd::Dims d = dims_of(*shape);
-    return path == SSD_B200_PATH_TC ? ssd::tc::workspace_bytes(d, pass) : simt_ws(d, pass).total;
+    if (path == SSD_B200_PATH_TC) return ssd::tc::workspace_bytes(d, pass);
+    const size_t simt = simt_ws(d, pass).total;  // which is what a call needs; the tensor-core kernels run where there is room for them
+    return ssd::mma::supported(shape->dtype, d.p, d.n) ? std::max(simt, mma_ws(d, pass).total) : simt;
 }
 
 size_t ssd_b200_states_bytes(const ssd_b200_shape* shape) {
@@ -707,7 +839,7 @@ int ssd_b200_fwd_static_scratch(const ssd_b200_fwd_args* a, void* stream) {
     if (path < 0) return path;
     // (a tensor-core walk runs in one piece where the room for more is missing)
     const size_t need = path == SSD_B200_PATH_TC ? ssd::tc::ws_layout(dims_of(a->shape), SSD_B200_PASS_FWD).base
-                                                 : ssd_b200_workspace_bytes(&a->shape, SSD_B200_PASS_FWD);
+                                                 : simt_ws(dims_of(a->shape), SSD_B200_PASS_FWD).total;
     if (need > (size_t)SSD_B200_STATIC_SCRATCH_BYTES)
         return fail(SSD_B200_EWORKSPACE,
                     "this shape needs %zu bytes of scratch but the built-in array holds %u; use ssd_b200_fwd with a "

@@ -1,7 +1,7 @@
 // fp32-accumulate SIMT kernels for the SSD chunked scan, forward and backward.
 //
-// This is the full-precision path (fp32 storage, 1e-4 parity) and the path for shapes the
-// tensor-core kernels do not cover.  Everything is computed in fp32 whatever the storage type.
+// This is the full-precision path (fp32 storage, 1e-4 parity) and the path for shapes that neither the
+// tensor-core kernels nor those of ssd_mma.cuh cover.  Everything is computed in fp32 whatever the storage type.
 // The algorithm per (batch, head), chunk k, in-chunk positions i, j (l per chunk):
 //
 //   cum_i = sum_{m<=i} a_m          S_k = cum_{l-1}

@@ -212,6 +212,60 @@ def test_partial_tiles_keep_fp32_arithmetic(pkg, cabi, oracle, b, T, h, p, n, g,
         assert got[k].dtype == torch.float32 and rel_err(got[k], want[k].reshape(got[k].shape)) < TOL_FP32, k
 
 
+@pytest.mark.parametrize("b,T,h,p,n,g,l", [(1, 2, 1, 64, 64, 1, 1), (2, 63, 3, 64, 72, 3, 21), (1, 65, 4, 40, 128, 2, 65), (2, 192, 8, 64, 64, 1, 96),
+                                           (3, 330, 6, 56, 40, 2, 30), (8, 640, 5, 64, 64, 5, 32)])
+@pytest.mark.parametrize("form", ["mamba2", "operator"])
+def test_partial_tiles_products_of_pieces(pkg, cabi, oracle, form, b, T, h, p, n, g, l):
+    """The kernels for bf16 calls of partial tiles against the oracle in 64 bits: one position and one behind a tile, headdim and
+    d_state that end inside their panels, the heads of a group on one block and on several, log-decays in fp32 and bf16.  The
+    three bf16 pieces of an operand carry all of its 24 bits, so what is left is the rounding of fp32 sums of at most a few
+    thousand terms: 1e-5 of the largest value (two pieces would be 2^-16 off per term).  dA_head is a sum of b T signed terms
+    da dt, each right to 1e-6 of the largest, and some sqrt(b T) = 72 times smaller than their absolute sum: 1e-4."""
+    cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, headdim=p, d_state=n, ngroups=g, chunk=l)
+    inp = pkg.make_inputs(cfg, seed=31)
+    gen = torch.Generator().manual_seed(32)
+    init, dfinal = torch.randn(b, h, p, n, generator=gen) * 0.2, torch.randn(b, h, p, n, generator=gen)
+    if form == "mamba2":
+        got = mamba2_gpu(pkg, inp, l, init, dfinal)
+        want = oracle.mamba2_fwd_bwd(inp, l, torch.float64, init.unsqueeze(1), dfinal)
+        exact, rounded = ("final_state", "ddt", "dA_head", "dD", "dinit"), ("y", "dx", "dB", "dC")
+    else:
+        a = inp["dt"] * inp["A_head"]
+        if T % 2:
+            a = a.bfloat16()
+        got = run_operator(pkg, inp["x"], a, inp["B"], inp["C"], l, init.unsqueeze(1), inp["dy"], dfinal.bfloat16())
+        lv = [t.double().requires_grad_(True) for t in (inp["x"], a, inp["B"], inp["C"], init.unsqueeze(1))]
+        Y, fs, _ = oracle.ssd_chunked(lv[0], lv[1], oracle.expand_groups(lv[2], h), oracle.expand_groups(lv[3], h), l, lv[4])
+        want = dict(zip(("dx", "dA", "dB", "dC", "dinit"), torch.autograd.grad([Y, fs], lv, [inp["dy"].double(), dfinal.bfloat16().double()])), Y=Y, final=fs)
+        exact, rounded = (("dA",) if a.dtype == torch.float32 else ()) + ("dinit",), ("Y", "final", "dx", "dB", "dC")
+        cached = run_operator(pkg, inp["x"], a, inp["B"], inp["C"], l, init.unsqueeze(1), inp["dy"], dfinal.bfloat16(), {"A_cumsum": got["cache"]["A_cumsum"]})
+        assert cached["dA"] is None and rel_err(cached["dinit"], want["dinit"].reshape(got["dinit"].shape)) < 1e-5
+        for k in rounded:
+            assert rel_err(cached[k], want[k].detach().reshape(got[k].shape)) < 2 ** -8, k
+    for k in exact:
+        assert got[k].dtype == torch.float32 and rel_err(got[k], want[k].detach().reshape(got[k].shape)) < (1e-4 if k == "dA_head" else 1e-5), k
+    for k in rounded:  # one rounding to bf16
+        assert rel_err(got[k], want[k].detach().reshape(got[k].shape)) < 2 ** -8, k
+
+
+def test_partial_tiles_in_less_workspace(pkg, cabi):
+    """With the workspace of the fp32 multiply-add kernels only (fp32 states of 96-position chunks), these run."""
+    cfg = replace(pkg.CONFIGS[2], batch=2, seqlen=192, nheads=4, ngroups=2, chunk=96)
+    inp = pkg.make_inputs(cfg, seed=6)
+    state = 2 * 4 * 64 * 128 * 4  # of one chunk
+    def up(v):
+        return (v + 255) // 256 * 256
+    rows, parts = up(2 * 4 * 192 * 4), up(2 * 192 * 2 * 2 * 128 * 4)
+    ws = {cabi.PASS_FWD: 2 * state, cabi.PASS_BWD: 5 * state + 4 * rows + 2 * 256 + 2 * parts}
+    rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
+    rc1, got = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, ws)
+    assert rc0 == rc1 == [0, 0]
+    for k in want:
+        assert rel_err(got[k], want[k]) < (1e-5 if want[k].dtype == torch.float32 else 2 ** -7), k
+    rc2, _ = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {k: v - 1 for k, v in ws.items()})
+    assert rc2 == [cabi.EWORKSPACE, cabi.EWORKSPACE]
+
+
 def test_cached_call_takes_any_chunk(pkg, cabi):
     """With the sums given, nothing bounds the chunk (2048 positions of 32 heads are too many for the kernel that makes the sums,
     which is refused); same result as with chunks of 128."""
