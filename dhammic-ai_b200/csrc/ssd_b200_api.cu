@@ -150,6 +150,8 @@ int simt_splits(const ssd::Dims& d) {
 struct SimtWs {
     size_t states, final_state, dstates, g_row, g_col, ddtx, dyx, dAh_part, dD_part, dB_part, dC_part, total;
 };
+// Whether the calls of this shape run on the kernels of ssd_mma.cuh (SSD_B200_PATH_SIMT asks for those of ssd_simt.cuh).
+bool mma_shape(const ssd_b200_shape& s) { return s.path == SSD_B200_PATH_AUTO && ssd::mma::supported(s.dtype, (int)s.headdim, (int)s.dstate); }
 size_t simt_states_elems(const ssd::Dims& d) { return (size_t)d.b * d.c * d.h * d.p * d.n; }
 
 SimtWs simt_ws(const ssd::Dims& d, int pass) {
@@ -184,7 +186,7 @@ SimtWs simt_ws(const ssd::Dims& d, int pass) {
 // forward + backward 134 us against 145.
 size_t simt_states_bytes(const ssd_b200_shape& s) {
     const ssd::Dims d = dims_of(s);
-    if (ssd::mma::supported(s.dtype, d.p, d.n)) return 0;  // these kernels walk the states again
+    if (mma_shape(s)) return 0;  // these kernels walk the states again
     if ((size_t)d.n * 4 > (size_t)d.l * (s.dtype == SSD_B200_BF16 ? 2 : 4)) return 0;
     return align_up(simt_states_elems(d) * 4) + (size_t)d.b * d.h * d.p * d.n * 4;
 }
@@ -287,11 +289,11 @@ int launch_chunk_scan(const ssd::simt::Params& P, cudaStream_t st) {
 // ---- the tensor-core kernels of ssd_mma.cuh (bf16, the same precision)
 // With the workspace these kernels need; summaries of a piece of the sequence stay on the SIMT kernels.
 bool mma_runs(const ssd_b200_fwd_args* a, const ssd::Dims& d) {
-    return ssd::mma::supported(a->shape.dtype, d.p, d.n) && !(a->flags & SSD_B200_FWD_STATES_ONLY) &&
+    return mma_shape(a->shape) && !(a->flags & SSD_B200_FWD_STATES_ONLY) &&
            a->workspace_bytes >= mma_ws(d, SSD_B200_PASS_FWD).total;
 }
 bool mma_runs(const ssd_b200_bwd_args* a, const ssd::Dims& d) {
-    return ssd::mma::supported(a->shape.dtype, d.p, d.n) && !(a->flags & SSD_B200_BWD_DINIT_ONLY) &&
+    return mma_shape(a->shape) && !(a->flags & SSD_B200_BWD_DINIT_ONLY) &&
            a->workspace_bytes >= mma_ws(d, SSD_B200_PASS_BWD).total;
 }
 template <class Args>
@@ -742,7 +744,7 @@ size_t ssd_b200_workspace_bytes(const ssd_b200_shape* shape, int pass) {
     ssd::Dims d = dims_of(*shape);
     if (path == SSD_B200_PATH_TC) return ssd::tc::workspace_bytes(d, pass);
     const size_t simt = simt_ws(d, pass).total;  // which is what a call needs; the tensor-core kernels run where there is room for them
-    return ssd::mma::supported(shape->dtype, d.p, d.n) ? std::max(simt, mma_ws(d, pass).total) : simt;
+    return mma_shape(*shape) ? std::max(simt, mma_ws(d, pass).total) : simt;
 }
 
 size_t ssd_b200_states_bytes(const ssd_b200_shape* shape) {
