@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
                                                           float* __restrict__ tcum, float* __restrict__ dtT,
                                                           const float* __restrict__ skip, float* __restrict__ skipT,
                                                           int* __restrict__ extreme, int T, int Tp, int h, int l) {
+    dep_wait();
     __shared__ float sdt[LT][33];
     __shared__ float ssk[LT][33];
     const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
                                                                 float* __restrict__ dtT, const float* __restrict__ skip,
                                                                 float* __restrict__ skipT, int* __restrict__ extreme, int T, int Tp,
                                                                 int h, int l) {
+    dep_wait();
     __shared__ float sa[LT][33];
     __shared__ float sdt[LT][33];
     __shared__ float sbef[8][33];
@@ -214,6 +216,7 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) chunk_cumsum_kernel(const void* __restrict__ a, int a_is_bf16, const float* __restrict__ dt,
                                                            const float* __restrict__ A_head, float* __restrict__ cum, int T, int h, int l) {
+    dep_wait();
     extern __shared__ float sm[];
     const int k = blockIdx.x, bb = blockIdx.y;
     const int ldh = h + 1;
@@ -245,6 +248,7 @@ __global__ void __launch_bounds__(256) chunk_cumsum_kernel(const void* __restric
 
 // Total log-decay of every (batch, head) sequence from the within-chunk cumulative sums: sum of the chunks' last entries.
 __global__ void logdecay_total_kernel(const float* __restrict__ cum, float* __restrict__ out, int bh, int c, int l) {
+    dep_wait();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= bh) return;
     float s = 0.f;

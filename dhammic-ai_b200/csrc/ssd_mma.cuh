@@ -230,6 +230,7 @@ struct StateCfg {
 };
 template <bool WIDE>
 __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
+    dep_wait();
     using Cfg = StateCfg;
     extern __shared__ __align__(16) __nv_bfloat16 sh[];
     __nv_bfloat16* out = sh + Cfg::ST * Cfg::STAGE;          // [2][3][64][VP]
@@ -440,6 +441,7 @@ struct ScanCfg {
 };
 template <int NN, bool WIDE>
 __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) scan_kernel(Params P) {
+    dep_wait();
     extern __shared__ __align__(16) __nv_bfloat16 sh[];
     const Dims& d = P.d;
     const Where w = where(P);
@@ -579,6 +581,7 @@ __device__ __forceinline__ void rows_by_pieces(float (&o)[8][4], const uint32_t 
 
 template <int NN, bool WIDE>
 __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) bwd_kernel(Params P) {
+    dep_wait();
     extern __shared__ __align__(16) __nv_bfloat16 sh[];
     const Dims& d = P.d;
     const Where w = where(P);
@@ -825,6 +828,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 template <bool WIDE>
 __global__ void __launch_bounds__(kDecayThreads) decay_kernel(Params P) {
+    dep_wait();
     __shared__ float red[kDecayThreads / 32];
     const Dims& d = P.d;
     if ((int)blockIdx.x >= d.b * d.h) {

@@ -228,6 +228,7 @@ __device__ __forceinline__ float row_reduce16(float v) {
 // ------------------------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(NTHR) chunk_state_kernel(Params P, int mode) {
+    dep_wait_early();
     __shared__ __align__(16) float Us[TS * TS];
     __shared__ __align__(16) float Vs[TS * TS];
     __shared__ float w[TS];
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(NTHR) chunk_state_kernel(Params P, int mode) {
 // reverse : slot k <- Q_k = dH_{k+1},               dH_k   = exp(S_k) Q_k + local_k ; dinit = dH_0
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(NTHR) state_passing_kernel(Params P, int reverse) {
+    dep_wait_early();
     const Dims& d = P.d;
     const size_t pn = (size_t)d.p * d.n;
     const size_t e = (size_t)blockIdx.x * NTHR + threadIdx.x;
@@ -348,6 +350,7 @@ __device__ __forceinline__ void load_scalars(const Params& P, int bb, int hh, in
 // ------------------------------------------------------------------------------------------
 template <class T, int PT>
 __global__ void __launch_bounds__(NTHR) chunk_scan_kernel(Params P) {
+    dep_wait_early();
     extern __shared__ __align__(16) float sm[];
     const Dims& d = P.d;
     const Where w = where(P);
@@ -478,6 +481,7 @@ __device__ __forceinline__ void store_bc(const Params& P, const Where& w, int t0
 
 template <class T, int PT, int NTN>
 __global__ void __launch_bounds__(NTHR, PT * NTN == 1 ? 2 : 1) chunk_bwd_kernel(Params P) {
+    dep_wait_early();
     extern __shared__ __align__(16) float sm[];
     const Dims& d = P.d;
     const Where w = where(P);
@@ -742,6 +746,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ------------------------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(NTHR) decay_grad_kernel(Params P) {
+    dep_wait_early();
     __shared__ float red[NTHR / 32];
     __shared__ float wsum[NTHR / 32];
     const Dims& d = P.d;
@@ -837,6 +842,7 @@ __global__ void __launch_bounds__(NTHR) decay_grad_kernel(Params P) {
 
 // out[hh] = sum_b part[b,hh]   (fixed order: deterministic); dA_head, and dD by the blocks with blockIdx.y = 1
 __global__ void reduce_batch_kernel(const float* part, float* out, const float* part2, float* out2, int b, int h) {
+    dep_wait_early();
     int hh = blockIdx.x * blockDim.x + threadIdx.x;
     if (hh >= h) return;
     if (blockIdx.y) {

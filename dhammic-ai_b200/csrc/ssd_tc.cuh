@@ -74,6 +74,7 @@ struct DecayTileParams {
 };
 
 __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
+    dep_wait();
     __shared__ float sdt[LT][33];
     __shared__ float sout[LT][33];
     const int k = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
 // A second (part, out) pair, when given, is reduced by the blocks with blockIdx.y = 1 of the same launch.
 __global__ void __launch_bounds__(256) reduce_rows_kernel(const float* __restrict__ part, float* __restrict__ out, int rows, int h,
                                                           const float* __restrict__ part2 = nullptr, float* __restrict__ out2 = nullptr) {
+    dep_wait();
     __shared__ float red[8];
     const int hh = blockIdx.x;
     if (blockIdx.y) {

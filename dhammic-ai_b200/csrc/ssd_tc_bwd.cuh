@@ -72,6 +72,7 @@ static_assert(512 * kBwdRegsRow + 128 * kBwdRegsCtl <= kBwdThreads * kBwdRegsLau
 // out-of-line body this kernel loses registers to the call and spills).
 template <bool EXACT>
 __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constant__ BwdParams P) {
+    dep_wait();
     if ((P.extreme[0] != 0) != EXACT) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);

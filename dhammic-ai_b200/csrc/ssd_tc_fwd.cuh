@@ -60,6 +60,7 @@ __device__ __forceinline__ void store_quarter_row(uint8_t* panel, int row, int c
 
 template <bool EXACT>
 __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constant__ WalkParams P) {
+    dep_wait();
     if ((P.extreme[0] != 0) != EXACT) return;
     using Cfg = WalkCfg<0>;
     constexpr int NST = Cfg::NST;

@@ -50,6 +50,7 @@ struct SummaryParams {
 
 template <bool REV, int NH>
 __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const __grid_constant__ SummaryParams P) {
+    dep_wait();
     using Cfg = SumCfg<NH>;
     constexpr int NS = Cfg::STAGES;
     constexpr int CTLW = 8 * NH;  // control warp

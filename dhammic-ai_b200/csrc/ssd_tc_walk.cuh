@@ -89,6 +89,7 @@ struct WalkCfg {
 constexpr int kWalkThreads = 320;  // 8 row warps, the product-issue warp, the TMA warp
 
 __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __grid_constant__ WalkParams P) {
+    dep_wait();
     using Cfg = WalkCfg<1>;
     constexpr int NST = Cfg::NST;
     extern __shared__ uint8_t smem_raw[];

@@ -248,6 +248,44 @@ def test_partial_tiles_products_of_pieces(pkg, cabi, oracle, form, b, T, h, p, n
         assert rel_err(got[k], want[k].detach().reshape(got[k].shape)) < 2 ** -8, k
 
 
+@pytest.mark.parametrize("dtype,T,n,l", [("fp32", 192, 64, 64), ("bf16", 330, 64, 30), ("bf16", 2048, 128, 128)])
+def test_launch_order_eager_and_captured(pkg, cabi, dtype, T, n, l):
+    """Kernels are set up while the one before them runs: the same bits call after call, on inputs and memory that the calls before
+    have used, and from a captured graph, on the kernels of each path."""
+    cfg = replace(pkg.CONFIGS[2], dtype=dtype, batch=2, seqlen=T, nheads=6, ngroups=2, d_state=n, chunk=l)
+    inps = [{k: v.to(DEV) for k, v in pkg.make_inputs(cfg, seed=s).items()} for s in (41, 42)]
+    names = ("x", "dt", "A_head", "B", "C", "D")
+
+    def call(inp):
+        lv = [inp[k].detach().requires_grad_(True) for k in names]
+        y, fs = pkg.ssd_mamba2(*lv, l)
+        return [y.detach(), fs.detach()] + list(torch.autograd.grad([y], lv, [inp["dy"]]))
+
+    want = []
+    for inp in inps:
+        want.append([t.clone() for t in call(inp)])
+        torch.cuda.synchronize()
+    for i in range(20):  # back to back, in the memory of the call before
+        for inp, w in zip(inps, want):
+            for a, b in zip(call(inp), w):
+                assert torch.equal(a, b), i
+    static = {k: v.clone() for k, v in inps[0].items()}
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(static)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = call(static)
+    for inp, w in list(zip(inps, want)) * 3:
+        for k in static:
+            static[k].copy_(inp[k])
+        graph.replay()
+        for a, b in zip(outs, w):
+            assert torch.equal(a, b)
+
+
 def test_partial_tiles_in_less_workspace(pkg, cabi):
     """With the workspace of the fp32 multiply-add kernels only (fp32 states of 96-position chunks), these run."""
     cfg = replace(pkg.CONFIGS[2], batch=2, seqlen=192, nheads=4, ngroups=2, chunk=96)
