@@ -263,15 +263,15 @@ ssd::simt::Params simt_params(const ssd::Dims& d) {
 
 // Local states (mode 0) or local state gradients (mode 1) of every chunk, and the recurrence over the chunks.
 template <class T>
-int simt_chunk_states(const ssd::simt::Params& P, int mode, cudaStream_t st) {
+int simt_chunk_states(bool after, const ssd::simt::Params& P, int mode, cudaStream_t st) {
     using namespace ssd::simt;
     const ssd::Dims& d = P.d;
     const dim3 g(d.c * d.b, d.h, ((d.p + TS - 1) / TS) * ((d.n + TS - 1) / TS));
-    SSD_LAUNCH(mode ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, (ssd::launch_dep(chunk_state_kernel<T>, g, NTHR, 0, st, P, mode)));
+    SSD_LAUNCH(mode ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, (ssd::launch_dep(after, chunk_state_kernel<T>, g, NTHR, 0, st, P, mode)));
     CUDA_LAUNCH_CHECK("chunk_state");
     const size_t pn = (size_t)d.p * d.n;
     const dim3 gp((unsigned)((pn + NTHR - 1) / NTHR), d.h, d.b);
-    SSD_LAUNCH(mode ? ssd::prof::K_STATE_PASS_REV : ssd::prof::K_STATE_PASS, st, ssd::launch_dep(state_passing_kernel, gp, NTHR, 0, st, P, mode));
+    SSD_LAUNCH(mode ? ssd::prof::K_STATE_PASS_REV : ssd::prof::K_STATE_PASS, st, ssd::launch_dep(true, state_passing_kernel, gp, NTHR, 0, st, P, mode));
     CUDA_LAUNCH_CHECK("state_passing");
     return 0;
 }
@@ -281,7 +281,7 @@ int launch_chunk_scan(const ssd::simt::Params& P, cudaStream_t st) {
     using namespace ssd::simt;
     const size_t sm = chunk_scan_smem(P.d, PT);
     if (int rc = set_smem<chunk_scan_kernel<T, PT>>(sm, "chunk_scan")) return rc;
-    SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, (ssd::launch_dep(chunk_scan_kernel<T, PT>, dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits), NTHR, sm, st, P)));
+    SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, (ssd::launch_dep(true, chunk_scan_kernel<T, PT>, dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits), NTHR, sm, st, P)));
     CUDA_LAUNCH_CHECK("chunk_scan");
     return 0;
 }
@@ -308,34 +308,34 @@ ssd::mma::Params mma_params(const Args* a, const ssd::Dims& d) {
     return P;
 }
 template <bool WIDE>
-int launch_mma_states(const ssd::mma::Params& P, int dirs, cudaStream_t st) {
+int launch_mma_states(bool after, const ssd::mma::Params& P, int dirs, cudaStream_t st) {
     using namespace ssd::mma;
     if (int rc = set_smem<state_kernel<WIDE>>(StateCfg::SMEM, "mma_states")) return rc;
     const dim3 g(P.d.h * ((P.d.n + kStateCols - 1) / kStateCols), P.d.b, dirs);
-    SSD_LAUNCH(dirs == 2 ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, ssd::launch_dep(state_kernel<WIDE>, g, kStateThreads, StateCfg::SMEM, st, P));
+    SSD_LAUNCH(dirs == 2 ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, ssd::launch_dep(after, state_kernel<WIDE>, g, kStateThreads, StateCfg::SMEM, st, P));
     CUDA_LAUNCH_CHECK("mma_states");
     return 0;
 }
 template <int NN, bool WIDE>
 int mma_fwd_launches(const ssd::mma::Params& P, cudaStream_t st) {
     using namespace ssd::mma;
-    if (int rc = launch_mma_states<WIDE>(P, 1, st)) return rc;
+    if (int rc = launch_mma_states<WIDE>(!P.cum, P, 1, st)) return rc;
     const size_t sm = ScanCfg<NN>::SMEM;
     if (int rc = set_smem<scan_kernel<NN, WIDE>>(sm, "mma_scan")) return rc;
-    SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, (ssd::launch_dep(scan_kernel<NN, WIDE>, dim3(P.nt * P.d.b, P.d.g * P.splits), NTHR, sm, st, P)));
+    SSD_LAUNCH(ssd::prof::K_CHUNK_SCAN, st, (ssd::launch_dep(true, scan_kernel<NN, WIDE>, dim3(P.nt * P.d.b, P.d.g * P.splits), NTHR, sm, st, P)));
     CUDA_LAUNCH_CHECK("mma_scan");
     return 0;
 }
 template <int NN, bool WIDE>
 int mma_bwd_launches(const ssd::mma::Params& P, cudaStream_t st) {
     using namespace ssd::mma;
-    if (int rc = launch_mma_states<WIDE>(P, 2, st)) return rc;
+    if (int rc = launch_mma_states<WIDE>(false, P, 2, st)) return rc;
     const size_t sm = BwdCfg<NN>::SMEM;
     if (int rc = set_smem<bwd_kernel<NN, WIDE>>(sm, "mma_bwd")) return rc;
-    SSD_LAUNCH(ssd::prof::K_CHUNK_BWD, st, (ssd::launch_dep(bwd_kernel<NN, WIDE>, dim3(P.nt * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st, P)));
+    SSD_LAUNCH(ssd::prof::K_CHUNK_BWD, st, (ssd::launch_dep(true, bwd_kernel<NN, WIDE>, dim3(P.nt * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st, P)));
     CUDA_LAUNCH_CHECK("mma_bwd");
     const size_t pairs = P.splits > 1 ? (size_t)P.d.b * P.d.T * P.d.g * P.d.n / 2 : 0;
-    SSD_LAUNCH(ssd::prof::K_DECAY, st, ssd::launch_dep(decay_kernel<WIDE>, (unsigned)(P.d.b * P.d.h + (pairs + kDecayThreads - 1) / kDecayThreads), kDecayThreads, 0, st, P));
+    SSD_LAUNCH(ssd::prof::K_DECAY, st, ssd::launch_dep(true, decay_kernel<WIDE>, (unsigned)(P.d.b * P.d.h + (pairs + kDecayThreads - 1) / kDecayThreads), kDecayThreads, 0, st, P));
     CUDA_LAUNCH_CHECK("mma_decay");
     return 0;
 }
@@ -356,14 +356,14 @@ int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
     if (!a->cumsum_is_input) {
         const size_t sm = (size_t)d.l * (d.h + 1) * 4;
         if (int rc = set_smem<chunk_cumsum_kernel>(sm, "chunk_cumsum")) return rc;
-        SSD_LAUNCH(ssd::prof::K_CUMSUM, st, ssd::launch_dep(chunk_cumsum_kernel, dim3(d.c, d.b), NTHR, sm, st, 
+        SSD_LAUNCH(ssd::prof::K_CUMSUM, st, ssd::launch_dep(false, chunk_cumsum_kernel, dim3(d.c, d.b), NTHR, sm, st, 
             a->dt ? nullptr : a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, d.T, d.h, d.l));
         CUDA_LAUNCH_CHECK("chunk_cumsum");
     }
     if (!mma)
-        if (int rc = simt_chunk_states<T>(P, 0, st)) return rc;
+        if (int rc = simt_chunk_states<T>(!a->cumsum_is_input, P, 0, st)) return rc;
     if (a->logdecay_total) {
-        SSD_LAUNCH(ssd::prof::K_CUMSUM, st, ssd::launch_dep(logdecay_total_kernel, (d.b * d.h + 127) / 128, 128, 0, st, a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
+        SSD_LAUNCH(ssd::prof::K_CUMSUM, st, ssd::launch_dep(!a->cumsum_is_input || !mma, logdecay_total_kernel, (d.b * d.h + 127) / 128, 128, 0, st, a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
         CUDA_LAUNCH_CHECK("logdecay_total");
     }
     if (mma) {
@@ -385,7 +385,7 @@ int launch_chunk_bwd(ssd::simt::Params P, cudaStream_t st) {
     P.share_ws = chunk_bwd_smem(P.d, PT, false) > (PT * NTN == 1 ? 113 : 227) * 1024;
     const size_t sm = chunk_bwd_smem(P.d, PT, P.share_ws);
     if (int rc = set_smem<chunk_bwd_kernel<T, PT, NTN>>(sm, "chunk_bwd")) return rc;
-    SSD_LAUNCH(ssd::prof::K_CHUNK_BWD, st, (ssd::launch_dep(chunk_bwd_kernel<T, PT, NTN>, dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st, P)));
+    SSD_LAUNCH(ssd::prof::K_CHUNK_BWD, st, (ssd::launch_dep(true, chunk_bwd_kernel<T, PT, NTN>, dim3(P.lb * P.d.c * P.d.b, P.d.g * P.splits, 2), NTHR, sm, st, P)));
     CUDA_LAUNCH_CHECK("chunk_bwd");
     return 0;
 }
@@ -398,7 +398,7 @@ int dispatch_chunk_bwd(const ssd::simt::Params& P, cudaStream_t st) {
 
 // dA_head and dD: the sums over the batch.
 int simt_head_sums(const ssd_b200_bwd_args* a, const float* dAh_part, const float* dD_part, const ssd::Dims& d, cudaStream_t st) {
-    SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::launch_dep(ssd::simt::reduce_batch_kernel, dim3((d.h + 127) / 128, a->D ? 2 : 1), 128, 0, st, 
+    SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::launch_dep(true, ssd::simt::reduce_batch_kernel, dim3((d.h + 127) / 128, a->D ? 2 : 1), 128, 0, st, 
         dAh_part, a->dA_head, dD_part, a->dD, d.b, d.h));
     CUDA_LAUNCH_CHECK("reduce_batch");
     return 0;
@@ -450,12 +450,12 @@ int simt_bwd(const ssd_b200_bwd_args* a, cudaStream_t st) {
     }
     const bool dinit_only = (a->flags & SSD_B200_BWD_DINIT_ONLY) != 0;
     if (!dinit_only && !a->states)  // states entering each chunk and the final state, if the forward did not keep them
-        if (int rc = simt_chunk_states<T>(P, 0, st)) return rc;
-    if (int rc = simt_chunk_states<T>(P, 1, st)) return rc;  // local state gradients and the reverse recurrence
+        if (int rc = simt_chunk_states<T>(false, P, 0, st)) return rc;
+    if (int rc = simt_chunk_states<T>(!dinit_only && !a->states, P, 1, st)) return rc;  // local state gradients and the reverse recurrence
     if (dinit_only) return 0;
     if (int rc = d.p <= TS ? dispatch_chunk_bwd<T, 1>(P, st) : dispatch_chunk_bwd<T, 2>(P, st)) return rc;
     const size_t total = P.splits > 1 ? (size_t)d.b * d.T * d.g * d.n : 0;
-    SSD_LAUNCH(ssd::prof::K_DECAY, st, ssd::launch_dep(decay_grad_kernel<T>, (unsigned)(d.b * d.h + (total + NTHR - 1) / NTHR), NTHR, 0, st, P));
+    SSD_LAUNCH(ssd::prof::K_DECAY, st, ssd::launch_dep(true, decay_grad_kernel<T>, (unsigned)(d.b * d.h + (total + NTHR - 1) / NTHR), NTHR, 0, st, P));
     CUDA_LAUNCH_CHECK("decay_grad");
     return a->dt ? simt_head_sums(a, P.dAh_part, P.dD_part, d, st) : 0;
 }
@@ -625,7 +625,7 @@ int trapezoid_impl(bool backward, size_t M, int H, const void* dt_raw, const voi
         float* pb = part_ws;
         float* pa = part_ws + nblk * H;
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, trapezoid_bwd_kernel<T><<<(unsigned)nblk, 256, 0, st>>>((const T*)dt_raw, (const T*)lam_raw, dt_bias, A_log, (const T*)g[0], (const T*)g[1], (const T*)g[2], (const T*)g[3], (T*)out[0], (T*)out[1], pb, pa, M, H));
-        SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::launch_dep(ssd::tc::reduce_rows_kernel, dim3(H, 2), 256, 0, st, pb, d_dt_bias, (int)nblk, H, pa, d_A_log));
+        SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::launch_dep(true, ssd::tc::reduce_rows_kernel, dim3(H, 2), 256, 0, st, pb, d_dt_bias, (int)nblk, H, pa, d_A_log));
     }
     CUDA_LAUNCH_CHECK("trapezoid");
     return 0;
@@ -932,7 +932,7 @@ int ssd_b200_m3_chain_bwd(const ssd_b200_shape* shape, const float* dw, const fl
     float* pA = ws;
     float* pD = ws + nblk * d.h;
     SSD_LAUNCH(ssd::prof::K_TC_AUX, st, ssd::m3::chain_bwd_kernel<<<(unsigned)nblk, 256, 0, st>>>(dw, dyx, sdot, dt, lam, da, A_head, dlam, ddt, pA, pD, M, d.T, d.h, d.g));
-    SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::launch_dep(ssd::tc::reduce_rows_kernel, dim3(d.h, dD ? 2 : 1), 256, 0, st, pA, dA_head, (int)nblk, d.h, pD, dD));
+    SSD_LAUNCH(ssd::prof::K_REDUCE, st, ssd::launch_dep(true, ssd::tc::reduce_rows_kernel, dim3(d.h, dD ? 2 : 1), 256, 0, st, pA, dA_head, (int)nblk, d.h, pD, dD));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(SSD_B200_ECUDA, cudaGetErrorString(e));
     return SSD_B200_OK;

@@ -35,11 +35,12 @@ __device__ __forceinline__ size_t st_off(const Dims& d, int bb, int k, int hh) {
 // blocks wait in dep_wait() until that kernel is complete and its writes are visible.  Every thread of every kernel launched this way
 // calls dep_wait() before it touches global memory in any way, also where it has nothing to do: a kernel that could be complete
 // before the one ahead of it would hand the next one memory that is still being written.  With that, the order of
-// everything on the stream is what it is with plain launches; saved is the time from the end of one kernel to the first work of the
+// everything on the stream is what it is with plain launches.  `after`: what is on the stream directly before is a kernel of the same
+// pass; what follows a memset, or work of the caller's, is launched plainly.  Saved is the time from the end of one kernel to the first work of the
 // next: one slice of 512 positions and 24 heads 26.6 -> 22.5 us a call, one prompt of 16,384 positions 189.6 -> 183.5, a training
 // step of (8, 2048, 24 heads) 260.8 -> 248.0.
 template <class... K, class... A>
-inline void launch_dep(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline void launch_dep(bool after, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -49,7 +50,7 @@ inline void launch_dep(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem,
     c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = &at;
-    c.numAttrs = 1;
+    c.numAttrs = after ? 1 : 0;
     cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);  // (the caller looks at cudaGetLastError)
 }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

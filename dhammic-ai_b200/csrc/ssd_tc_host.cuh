@@ -181,11 +181,11 @@ inline int set_walk_attrs(char* err, size_t errn) {
     return 0;
 }
 
-inline int launch_tile_cumsum(const Dims& d, const float* cum, const float* dt, float* tcum, float* dtT, const float* skip,
+inline int launch_tile_cumsum(bool after, const Dims& d, const float* cum, const float* dt, float* tcum, float* dtT, const float* skip,
                               float* skipT, int* extreme, cudaStream_t st, char* err, size_t errn) {
     const int nt = tiles_of(d.T);
     dim3 g(nt, (d.h + 31) / 32, d.b);
-    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(tile_cumsum_kernel, g, 256, 0, st, cum, dt, tcum, dtT, skip, skipT, extreme, d.T, nt * LT, d.h, d.l));
+    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, tile_cumsum_kernel, g, 256, 0, st, cum, dt, tcum, dtT, skip, skipT, extreme, d.T, nt * LT, d.h, d.l));
     SSD_TC_CHECK("tile_cumsum");
     return 0;
 }
@@ -197,15 +197,15 @@ inline int launch_cumsum_tile_fused(const Args* a, const Dims& d, float* cum, fl
     const int nt = tiles_of(d.T);
     const dim3 g(nt, (d.h + 31) / 32, d.b);
     const bool cut = d.l % LT != 0;  // a chunk ends inside a tile
-    SSD_LAUNCH(prof::K_CUMSUM, st, (launch_dep((cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>), g, 256, 0, st, 
+    SSD_LAUNCH(prof::K_CUMSUM, st, (launch_dep(false, (cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>), g, 256, 0, st, 
         a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, cum, tcum, dtT, a->skip, skipT, extreme, d.T, nt * LT, d.h, d.l)));
     SSD_TC_CHECK("cumsum_tile_fused");
     return 0;
 }
 
-// Cuts the walk of P into pieces where that pays and the workspace has the room, and summarises them.
+// Cuts the walk of P into pieces where that pays and the workspace has the room, and summarises them.  `after`: see launch_dep.
 template <bool REV>
-inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace, size_t bytes, int* pieces, cudaStream_t st, char* err, size_t errn) {
+inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace, size_t bytes, int* pieces, bool* after, cudaStream_t st, char* err, size_t errn) {
     P.pt = P.nt;
     *pieces = 1;
     const Pieces pc = pieces_of(d, REV);
@@ -214,10 +214,11 @@ inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace
     S.mU = P.mU; S.mV = P.mV; S.tcum = P.tcum; S.dtT = P.dtT; S.out = (float*)((char*)workspace + w.piece_sum);
     S.logdecay = (float*)((char*)workspace + w.piece_decay); S.status = P.status; S.Tp = P.Tp; S.h = P.h; S.hpg = P.hpg; S.nt = P.nt;
     S.p = P.p; S.n = P.n; S.pt = pc.pt; S.ps = pc.ps; S.parts = pc.parts; S.z0 = REV ? 1 : 0;
-    SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(summary_kernel<REV, 1>, dim3(d.h, d.b, (pc.np - 1) * pc.parts), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
+    SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(*after, summary_kernel<REV, 1>, dim3(d.h, d.b, (pc.np - 1) * pc.parts), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
     SSD_TC_CHECK("tc_summary_pieces");
     P.pt = pc.pt; P.parts = pc.parts; P.piece_sum = S.out; P.piece_decay = S.logdecay;
     *pieces = pc.np;
+    *after = true;
     return 0;
 }
 
@@ -257,14 +258,15 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
             if (sm > 48 * 1024 &&
                 cudaFuncSetAttribute(chunk_cumsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
                 SSD_TC_FAIL(SSD_B200_ECUDA, "chunk_cumsum: set shared memory size failed");
-            SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(chunk_cumsum_kernel, dim3(d.c, d.b), 256, sm, st, 
+            SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(false, chunk_cumsum_kernel, dim3(d.c, d.b), 256, sm, st, 
                 a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, a->a_cumsum, d.T, d.h, d.l));
             SSD_TC_CHECK("chunk_cumsum");
         }
         if (!aux_valid)
-            if (int rc = launch_tile_cumsum(d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn)) return rc;
+            if (int rc = launch_tile_cumsum(!a->cumsum_is_input, d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn)) return rc;
     }
     if (int rc = set_walk_attrs(err, errn)) return rc;
+    bool after = !aux_valid;  // the cumulative sums are on the stream, or the memset of the status word
     WalkParams P{};
     P.skipT = skipT;
     P.extreme = extreme;
@@ -287,19 +289,19 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
         S.logdecay = a->logdecay_total; S.status = status; S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1;
         S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)  // two heads of a group per CTA share the group's panels
-            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(summary_kernel<false, 2>, dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
+            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(after, summary_kernel<false, 2>, dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
         else
-            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(summary_kernel<false, 1>, dim3(d.h, d.b), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
+            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(after, summary_kernel<false, 1>, dim3(d.h, d.b), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
         SSD_TC_CHECK("tc_summary_fwd");
         return 0;
     }
     int pieces;
-    if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, st, err, errn)) return rc;
-    SSD_LAUNCH(prof::K_TC_FWD, st, (launch_dep(fwd_walk_kernel<false>, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P)));
-    SSD_LAUNCH(prof::K_TC_FWD_ALT, st, (launch_dep(fwd_walk_kernel<true>, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P)));
+    if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
+    SSD_LAUNCH(prof::K_TC_FWD, st, (launch_dep(after, fwd_walk_kernel<false>, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P)));
+    SSD_LAUNCH(prof::K_TC_FWD_ALT, st, (launch_dep(true, fwd_walk_kernel<true>, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P)));
     SSD_TC_CHECK("tc_fwd_walk");
     if (a->logdecay_total) {
-        SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(logdecay_total_kernel, (d.b * d.h + 127) / 128, 128, 0, st, a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
+        SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(true, logdecay_total_kernel, (d.b * d.h + 127) / 128, 128, 0, st, a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
         SSD_TC_CHECK("logdecay_total");
     }
     return 0;
@@ -333,10 +335,11 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
     } else {  // as the forward made them: from the log-decays, or from the sums it was given
         const bool decays = !a->cumsum_is_input && d.l <= kFusedChunkMax && (a->a || (a->dt && a->A_head));
         if (int rc = decays ? launch_cumsum_tile_fused(a, d, nullptr, tcum, dtT, skipT, extreme, st, err, errn)
-                            : launch_tile_cumsum(d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn))
+                            : launch_tile_cumsum(false, d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn))
             return rc;
     }
     if (int rc = set_walk_attrs(err, errn)) return rc;
+    bool after = !a->states;  // the cumulative sums are on the stream, or the memset of the status word
     const uint64_t srows = (uint64_t)d.b * nt * d.h * DN;
     if (a->flags & SSD_B200_BWD_DINIT_ONLY) {  // d(initial state) of this piece for the given (or a zero) dfinal
         SummaryParams S{};
@@ -345,9 +348,9 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         S.tcum = tcum; S.dtT = nullptr; S.seed = a->dfinal; S.out = a->dinit; S.logdecay = nullptr; S.status = status;
         S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1; S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)
-            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(summary_kernel<true, 2>, dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
+            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(after, summary_kernel<true, 2>, dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
         else
-            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(summary_kernel<true, 1>, dim3(d.h, d.b), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
+            SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(after, summary_kernel<true, 1>, dim3(d.h, d.b), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
         SSD_TC_CHECK("tc_summary_rev");
         return 0;
     }
@@ -362,9 +365,10 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.tcum = tcum; P.dtT = dtT; P.D = nullptr; P.seed = a->init; P.out_state = fin; P.status = status;
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         int pieces;  // the same as the forward's: the states have the same bits
-        if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, st, err, errn)) return rc;
-        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (launch_dep(states_walk_kernel, dim3(d.h, d.b, pieces), kWalkThreads, WalkCfg<1>::SMEM, st, P)));
+        if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
+        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (launch_dep(after, states_walk_kernel, dim3(d.h, d.b, pieces), kWalkThreads, WalkCfg<1>::SMEM, st, P)));
         SSD_TC_CHECK("tc_bwd_state");
+        after = true;
     }
     {   // reverse walk: gradient of the state leaving every tile, and d(initial state)
         WalkParams P{};
@@ -372,13 +376,13 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.tcum = tcum; P.dtT = nullptr; P.D = nullptr; P.seed = a->dfinal; P.out_state = dinit; P.status = status;
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         int pieces;
-        if (int rc = split_walk<true>(P, d, w, ws, a->workspace_bytes, &pieces, st, err, errn)) return rc;
+        if (int rc = split_walk<true>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
         // two heads of a group per CTA: shared C panels, one N = 128 product per tile; but a tile then takes 1.7 us instead of
         // 1.5, so only where one head per CTA would not fit on the chip at once
         if (d.hpg % 2 == 0 && pieces == 1 && (long long)d.b * d.h > kPieceSms)
-            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(rev_walk_kernel<2>, dim3(d.h / 2, d.b), RevCfg<2>::THREADS, RevCfg<2>::SMEM, st, P));
+            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(after, rev_walk_kernel<2>, dim3(d.h / 2, d.b), RevCfg<2>::THREADS, RevCfg<2>::SMEM, st, P));
         else
-            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(rev_walk_kernel<1>, dim3(d.h, d.b, pieces), RevCfg<1>::THREADS, RevCfg<1>::SMEM, st, P));
+            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(after, rev_walk_kernel<1>, dim3(d.h, d.b, pieces), RevCfg<1>::THREADS, RevCfg<1>::SMEM, st, P));
         SSD_TC_CHECK("tc_bwd_dstate");
     }
     {
@@ -390,8 +394,8 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.items = nt * d.g * d.b;
         P.extreme = extreme;
         const dim3 grid(std::min(P.items, sm_count()));
-        SSD_LAUNCH(prof::K_TC_BWD, st, launch_dep(bwd_tile_kernel<false>, grid, kBwdThreads, kBwdSmem, st, P));
-        SSD_LAUNCH(prof::K_TC_BWD_ALT, st, launch_dep(bwd_tile_kernel<true>, grid, kBwdThreads, kBwdSmem, st, P));
+        SSD_LAUNCH(prof::K_TC_BWD, st, launch_dep(true, bwd_tile_kernel<false>, grid, kBwdThreads, kBwdSmem, st, P));
+        SSD_LAUNCH(prof::K_TC_BWD_ALT, st, launch_dep(true, bwd_tile_kernel<true>, grid, kBwdThreads, kBwdSmem, st, P));
         SSD_TC_CHECK("tc_bwd_walk");
     }
     {
@@ -402,10 +406,10 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.dskip = a->skip ? a->dskip : nullptr;
         P.dAh_part = (float*)(ws + w.dAh_part); P.dD_part = P.dyx ? (float*)(ws + w.dD_part) : nullptr;
         P.b = d.b; P.T = d.T; P.Tp = Tp; P.h = d.h; P.nt = nt;
-        SSD_LAUNCH(prof::K_DECAY, st, launch_dep(decay_tile_kernel, dim3(nt, (d.h + 31) / 32, d.b), 256, 0, st, P));
+        SSD_LAUNCH(prof::K_DECAY, st, launch_dep(true, decay_tile_kernel, dim3(nt, (d.h + 31) / 32, d.b), 256, 0, st, P));
         SSD_TC_CHECK("decay_grad");
         if (a->dt && a->A_head) {
-            SSD_LAUNCH(prof::K_REDUCE, st, launch_dep(reduce_rows_kernel, dim3(d.h, a->D ? 2 : 1), 256, 0, st, 
+            SSD_LAUNCH(prof::K_REDUCE, st, launch_dep(true, reduce_rows_kernel, dim3(d.h, a->D ? 2 : 1), 256, 0, st, 
                 P.dAh_part, a->dA_head, d.b * nt, d.h, P.dD_part, a->dD));
             SSD_TC_CHECK("reduce_batch");
         }
