@@ -541,7 +541,17 @@ int m3_fwd_impl(const ssd::Dims& d, const void* x, const float* dt, const float*
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_fwd_kernel<T, 2><<<dim3(d.T, d.b), 256, 0, st>>>((const T*)B, (const T*)C, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
     }
     const size_t grows = (size_t)d.b * d.T * d.g, rows = (size_t)d.b * d.T * d.h;
-    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, bc_dot_kernel<T><<<(unsigned)((grows + 7) / 8), 256, 0, st>>>((const T*)B, (const T*)C, sdot, d.n, grows));
+    {   // whole vectors where a row is 4, 8, 16 or 32 of them
+        constexpr int V = VecOf<T>::N;
+        const int tpr = d.n % V == 0 && !any_unaligned({B, C}) ? d.n / V : 0;
+        const T *b_ = (const T*)B, *c_ = (const T*)C;
+        auto blocks = [&](int t) { return (unsigned)((grows * t + 255) / 256); };
+        if (tpr == 4) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (bc_dot_kernel<T, V, 4><<<blocks(4), 256, 0, st>>>(b_, c_, sdot, d.n, grows)));
+        else if (tpr == 8) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (bc_dot_kernel<T, V, 8><<<blocks(8), 256, 0, st>>>(b_, c_, sdot, d.n, grows)));
+        else if (tpr == 16) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (bc_dot_kernel<T, V, 16><<<blocks(16), 256, 0, st>>>(b_, c_, sdot, d.n, grows)));
+        else if (tpr == 32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (bc_dot_kernel<T, V, 32><<<blocks(32), 256, 0, st>>>(b_, c_, sdot, d.n, grows)));
+        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (bc_dot_kernel<T, 1, 32><<<blocks(32), 256, 0, st>>>(b_, c_, sdot, d.n, grows)));
+    }
     if (xw) {
         M3_ROW_DISPATCH(!any_unaligned({x, xw}), xw_fwd_kernel, (const T*)x, dt, lam, A_head, (T*)xw, dA, d.T, d.h, d.p, rows);
     } else {  // the scan takes the weight and the skip coefficient per position: x is not touched here
