@@ -86,18 +86,28 @@ __device__ __forceinline__ uint32_t at_cr(uint32_t base, int pitch, int r0, int 
 // A (16 x 16) of a matrix stored [m][k]: at_rc, ldsm4.  Of one stored [k][m]: at_cr, ldsm4t.
 // B (16 x 16: two n tiles, registers {0,1} and {2,3}) of a matrix stored [n][k]: at_cr, ldsm4.  Of one stored [k][n]: at_rc, ldsm4t.
 
-// A pair of fp32 values as three pairs of bf16 pieces, cut and not rounded: hi + mid + lo is the value.  (The pieces of an infinite
-// value are not numbers: a result that would be infinite comes out as NaN.)
+// A pair of fp32 values as three pairs of bf16 pieces: hi + mid + lo is the value (below 2^-110 in magnitude to 2^-133).  A piece is cut
+// off the fp32 number before the value, and no further than the largest finite one: so each remainder of a value that is not zero is not
+// zero either and has the value's sign, and an infinite value is finite pieces and an infinite lo.  Sums of the three products
+// are then infinite where the product of the values is, on either side.  (Cut off the value itself, an infinite value left NaN as its
+// remainder, and a piece of zero made NaN of an infinite given operand.)  The conversion cuts and packs at once: against masking the bits
+// of each value, forward of (4, 1984, 20 heads, 64) 102.7 -> 100.6 us at d_state 64, forward and backward 300 -> 300; at d_state 128, where the
+// backward has no register left, 496 -> 503.
 __device__ __forceinline__ void cut8(float v0, float v1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const float2 minus = make_float2(-1.f, -1.f);
-    auto head = [](float2 v) { return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u)); };
-    auto pair = [](float2 v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); };
+    const float2 minus = make_float2(-1.f, -1.f), before = make_float2(0x1.fffffep-1f, 0x1.fffffep-1f);
+    auto head = [&](float2 v) {
+        uint32_t r;
+        v = ptx::mul2(v, before);
+        asm("cvt.rz.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v.y), "f"(v.x));
+        return r;
+    };
+    auto floats = [](uint32_t u) { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); };
     float2 v = make_float2(v0, v1);
-    hi = pair(v);
-    v = ptx::fma2(head(v), minus, v);
-    mid = pair(v);
-    v = ptx::fma2(head(v), minus, v);
-    lo = pair(v);
+    hi = head(v);
+    v = ptx::fma2(floats(hi), minus, v);
+    mid = head(v);
+    v = ptx::fma2(floats(mid), minus, v);
+    lo = __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632);
 }
 // The two accumulator tiles of 16 columns as the pieces of an A operand (k = those columns): f[0] = lo, f[1] = mid, f[2] = hi.
 __device__ __forceinline__ void cut_tiles(const float (&t0)[4], const float (&t1)[4], uint32_t (&f)[3][4]) {
@@ -690,6 +700,8 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) bwd_kernel(Params P) {
             }
             st0 = quad_sum(st0);
             st1 = quad_sum(st1);
+            if (r0 >= w.rows) st0 = 0.f;  // behind the end: no number where the state is infinite
+            if (r0 + 8 >= w.rows) st1 = 0.f;
             store_carry(st0 + st1, tile);
             sum0 = quad_sum(sum0) + st0;
             sum1 = quad_sum(sum1) + st1;
@@ -787,6 +799,8 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) bwd_kernel(Params P) {
             }
             st[0] = w0 * dt0 * quad_sum(st[0]);
             st[1] = w1 * dt1 * quad_sum(st[1]);
+            if (r0 >= w.rows) st[0] = 0.f;
+            if (r0 + 8 >= w.rows) st[1] = 0.f;
             store_carry(st[0] + st[1], tile);
             sum0 = quad_sum(sum0) + st[0];
             sum1 = quad_sum(sum1) + st[1];

@@ -248,6 +248,43 @@ def test_partial_tiles_products_of_pieces(pkg, cabi, oracle, form, b, T, h, p, n
         assert rel_err(got[k], want[k].detach().reshape(got[k].shape)) < 2 ** -8, k
 
 
+@pytest.mark.parametrize("case", ["state overflows", "gradient overflows", "x", "dy", "B", "C", "init", "dfinal"])
+@pytest.mark.parametrize("T,n", [(192, 64), (192, 128)])
+def test_partial_tiles_infinite_values(pkg, cabi, case, T, n):
+    """Infinite values among the inputs, and states and their gradients that leave the range of fp32: a result that is finite, or
+    infinite, with the fp32 multiply-adds of the SIMT path on the same tiles is finite, or the same infinity, here."""
+    b, h, g, p, l = 2, 4, 2, 64, min(T, 64)
+    gen = torch.Generator().manual_seed(3)
+    v = {"x": torch.randn(b, T, h, p, generator=gen), "dt": 0.05 * torch.rand(b, T, h, generator=gen) + 1e-3, "A_head": -torch.exp(torch.rand(h, generator=gen)),
+         "B": torch.randn(b, T, g, n, generator=gen) / n ** 0.5, "C": torch.randn(b, T, g, n, generator=gen) / n ** 0.5, "D": torch.randn(h, generator=gen),
+         "init": torch.randn(b, h, p, n, generator=gen), "dy": torch.randn(b, T, h, p, generator=gen), "dfinal": torch.randn(b, h, p, n, generator=gen)}
+    if case.endswith("overflows"):
+        v["A_head"] *= 1e-6
+        for k in ("x", "dy", "B", "C", "init", "dfinal"):  # (with both signs it would depend on the order of a sum which infinity comes first)
+            v[k].abs_()
+        k, m, t = ("x", "B", T // 3) if case.startswith("state") else ("dy", "C", T - 20)
+        v[k][:, t], v[m][:, t] = 3e38, 30.0
+    elif case in ("init", "dfinal"):
+        v[case][:, 1, 5, 7], v[case][0, 2, 3] = float("inf"), float("-inf")
+    else:
+        v[case][:, T // 2, 1, 5], v[case][1, T // 4, 0, 6] = float("inf"), float("-inf")
+    res = {}
+    for path in ("auto", "simt"):
+        pkg.set_kernel_path(path)
+        try:
+            lv = [v[k].to(DEV, torch.bfloat16 if k in "xBC" else None).requires_grad_(True) for k in ("x", "dt", "A_head", "B", "C", "D", "init")]
+            y, fs = pkg.ssd_mamba2(*lv[:6], l, lv[6])
+            res[path] = [y.detach(), fs.detach()] + list(torch.autograd.grad([y, fs], lv, [v["dy"].to(DEV, torch.bfloat16), v["dfinal"].to(DEV)]))
+        finally:
+            pkg.set_kernel_path("auto")
+    infinite = 0
+    for k, got, want in zip(("y", "final", "dx", "ddt", "dA_head", "dB", "dC", "dD", "dinit"), res["auto"], res["simt"]):
+        inf = torch.isinf(want)
+        infinite += int(inf.sum())
+        assert torch.equal(got[inf], want[inf]) and torch.isfinite(got[torch.isfinite(want)]).all(), k
+    assert infinite
+
+
 @pytest.mark.parametrize("dtype,T,n,l", [("fp32", 192, 64, 64), ("bf16", 330, 64, 30), ("bf16", 2048, 128, 128)])
 def test_launch_order_eager_and_captured(pkg, cabi, dtype, T, n, l):
     """Kernels are set up while the one before them runs: the same bits call after call, on inputs and memory that the calls before
