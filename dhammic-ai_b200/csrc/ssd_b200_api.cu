@@ -199,8 +199,11 @@ int mma_splits(const ssd::Dims& d) {
     return s;
 }
 struct MmaWs {
-    size_t H, sums, Q, final_state, carry, g_row, g_col, ddtx, dyx, dAh_part, dD_part, dB_part, dC_part, total;
+    size_t H, sums, part, part_logdecay, Q, final_state, carry, g_row, g_col, ddtx, dyx, dAh_part, dD_part, dB_part, dC_part, total;
 };
+// Column blocks of the walk over the states, and its tiles per piece in a pass (the backward walks in both directions).
+int mma_state_cols(const ssd::Dims& d) { return (d.n + ssd::mma::kStateCols - 1) / ssd::mma::kStateCols; }
+int mma_per(const ssd::Dims& d, int dirs) { return ssd::mma::piece_tiles(ssd::mma::tiles(d.T), (long long)d.b * d.h * mma_state_cols(d) * dirs); }
 MmaWs mma_ws(const ssd::Dims& d, int pass) {
     MmaWs w{};
     size_t off = 0;
@@ -212,6 +215,10 @@ MmaWs mma_ws(const ssd::Dims& d, int pass) {
     const size_t pieces = (size_t)d.b * ssd::mma::tiles(d.T) * d.h * 3 * d.p * d.n * 2;
     w.H = take(pieces);
     w.sums = take((size_t)d.b * ssd::mma::tiles(d.T) * d.h * 2 * ssd::mma::MT * 4);
+    const int dirs = pass == SSD_B200_PASS_BWD ? 2 : 1, per = mma_per(d, dirs);
+    const size_t sums = (size_t)dirs * d.b * d.h * mma_state_cols(d) * ((ssd::mma::tiles(d.T) - 1) / per);
+    w.part = take(sums * 2048 * 4);
+    w.part_logdecay = take(sums * 4);
     if (pass == SSD_B200_PASS_BWD) {
         const size_t bht = (size_t)d.b * d.h * d.T * 4, splits = mma_splits(d);
         const size_t bc = splits > 1 ? (size_t)d.b * d.T * d.g * splits * d.n * 4 : 0;
@@ -297,9 +304,13 @@ bool mma_runs(const ssd_b200_bwd_args* a, const ssd::Dims& d) {
            a->workspace_bytes >= mma_ws(d, SSD_B200_PASS_BWD).total;
 }
 template <class Args>
-ssd::mma::Params mma_params(const Args* a, const ssd::Dims& d) {
+ssd::mma::Params mma_params(const Args* a, const ssd::Dims& d, const MmaWs& w, int dirs) {
     ssd::mma::Params P{};
+    char* ws = (char*)a->workspace;
     P.d = d;
+    P.per = mma_per(d, dirs);
+    P.np = (ssd::mma::tiles(d.T) + P.per - 1) / P.per;
+    P.H = (__nv_bfloat16*)(ws + w.H); P.sums = (float*)(ws + w.sums); P.part = (float*)(ws + w.part); P.part_logdecay = (float*)(ws + w.part_logdecay);
     P.nt = ssd::mma::tiles(d.T);
     P.splits = mma_splits(d);
     P.x = (const __nv_bfloat16*)a->x; P.B = (const __nv_bfloat16*)a->B; P.C = (const __nv_bfloat16*)a->C;
@@ -310,9 +321,19 @@ ssd::mma::Params mma_params(const Args* a, const ssd::Dims& d) {
 template <bool WIDE>
 int launch_mma_states(bool after, const ssd::mma::Params& P, int dirs, cudaStream_t st) {
     using namespace ssd::mma;
-    if (int rc = set_smem<state_kernel<WIDE>>(StateCfg::SMEM, "mma_states")) return rc;
-    const dim3 g(P.d.h * ((P.d.n + kStateCols - 1) / kStateCols), P.d.b, dirs);
-    SSD_LAUNCH(dirs == 2 ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE, st, ssd::launch_dep(after, state_kernel<WIDE>, g, kStateThreads, StateCfg::SMEM, st, P));
+    const int rows = P.d.h * mma_state_cols(P.d), slot = dirs == 2 ? ssd::prof::K_CHUNK_DSTATE : ssd::prof::K_CHUNK_STATE;
+    if (P.np == 1) {
+        if (int rc = set_smem<state_kernel<WIDE, false>>(StateCfg::SMEM, "mma_states")) return rc;
+        SSD_LAUNCH(slot, st, (ssd::launch_dep(after, state_kernel<WIDE, false>, dim3(rows, P.d.b, dirs), kStateThreads, StateCfg::SMEM, st, P)));
+        CUDA_LAUNCH_CHECK("mma_states");
+        return 0;
+    }
+    if (int rc = set_smem<state_kernel<WIDE, true>>(StateCfg::SMEM, "mma_states")) return rc;
+    Params S = P;
+    S.summary = 1;
+    SSD_LAUNCH(slot, st, (ssd::launch_dep(after, state_kernel<WIDE, true>, dim3(rows * (P.np - 1), P.d.b, dirs), kStateThreads, StateCfg::SMEM, st, S)));
+    CUDA_LAUNCH_CHECK("mma_state_sums");
+    SSD_LAUNCH(slot, st, (ssd::launch_dep(true, state_kernel<WIDE, true>, dim3(rows * P.np, P.d.b, dirs), kStateThreads, StateCfg::SMEM, st, P)));
     CUDA_LAUNCH_CHECK("mma_states");
     return 0;
 }
@@ -367,9 +388,7 @@ int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
         CUDA_LAUNCH_CHECK("logdecay_total");
     }
     if (mma) {
-        ssd::mma::Params M = mma_params(a, d);
-        const MmaWs wm = mma_ws(d, SSD_B200_PASS_FWD);
-        M.H = (__nv_bfloat16*)((char*)a->workspace + wm.H); M.sums = (float*)((char*)a->workspace + wm.sums);
+        ssd::mma::Params M = mma_params(a, d, mma_ws(d, SSD_B200_PASS_FWD), 1);
         M.final_state = a->final_state; M.y = (__nv_bfloat16*)a->y;
         if (any_unaligned({a->x, a->B, a->C, a->y})) return d.n <= 64 ? mma_fwd_launches<64, false>(M, st) : mma_fwd_launches<128, false>(M, st);
         return d.n <= 64 ? mma_fwd_launches<64, true>(M, st) : mma_fwd_launches<128, true>(M, st);
@@ -407,9 +426,9 @@ int simt_head_sums(const ssd_b200_bwd_args* a, const float* dAh_part, const floa
 int mma_bwd(const ssd_b200_bwd_args* a, const ssd::Dims& d, cudaStream_t st) {
     const MmaWs w = mma_ws(d, SSD_B200_PASS_BWD);
     char* ws = (char*)a->workspace;
-    ssd::mma::Params M = mma_params(a, d);
+    ssd::mma::Params M = mma_params(a, d, w, 2);
     M.dy = (const __nv_bfloat16*)a->dy; M.dfinal = a->dfinal; M.dinit = a->dinit;
-    M.H = (__nv_bfloat16*)(ws + w.H); M.sums = (float*)(ws + w.sums); M.Q = (__nv_bfloat16*)(ws + w.Q); M.final_state = (float*)(ws + w.final_state);
+    M.Q = (__nv_bfloat16*)(ws + w.Q); M.final_state = (float*)(ws + w.final_state);
     M.dx = (__nv_bfloat16*)a->dx; M.dB = (__nv_bfloat16*)a->dB; M.dC = (__nv_bfloat16*)a->dC;
     M.g_row = (float*)(ws + w.g_row); M.g_col = (float*)(ws + w.g_col); M.ddtx = (float*)(ws + w.ddtx);
     M.dyx = (a->dt && a->D) ? (float*)(ws + w.dyx) : nullptr;

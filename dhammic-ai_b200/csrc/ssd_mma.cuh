@@ -24,6 +24,9 @@
 // from shared memory, 298 us in seven now (states 130, backward 109, scan 43, decay 11); d dt is 3.8e-7 off the exact one (5.8e-7),
 // dA_head 2.7e-6 (6.4e-6), the final state 2.6e-7 (2.7e-7).
 #pragma once
+#include <algorithm>
+#include <cmath>
+
 #include "ssd_common.cuh"
 #include "ssd_ptx.cuh"
 
@@ -47,6 +50,9 @@ struct Params {
     const float *dt, *A_head, *D, *init, *dfinal;
     __nv_bfloat16 *H, *Q;  // (b,nt,h,3,p,n): pieces of the state entering each tile, of the gradient of the state leaving it
     float* sums;           // (b,nt,h,2,64): sums of the log-decay within each tile, and dt (1 without dt, 0 behind the end)
+    int per, np;           // tiles of a piece of the walk over the states, pieces
+    int summary;           // the pieces' own sums are made, without a state before them: into part, for all but the last
+    float *part, *part_logdecay;  // (dir,b,h,n / 32,np - 1,4,128,4): fragments of a piece's sum, (dir,b,h,n / 32,np - 1): log-decay over it
     float *final_state, *dinit;
     __nv_bfloat16 *y, *dx, *dB, *dC;
     float *g_row, *g_col, *ddtx, *dyx;   // (b,h,T)
@@ -58,6 +64,18 @@ struct Params {
 // Which calls these kernels can run.
 inline bool supported(int dtype, int p, int n) { return dtype == 1 && p > 32 && p <= 64 && p % 8 == 0 && n > 32 && n <= 128 && n % 8 == 0; }
 inline int tiles(int T) { return (T + MT - 1) / MT; }
+// Tiles of a piece of the walk over the states, which has `blocks` blocks in one piece; nt for a walk in one piece.  As many pieces as the chip
+// holds blocks at a time (three an SM), but no more than sqrt(6 nt), where the sums of the pieces before a block cost what its own
+// steps do, and at least three, since every step but the last piece's is made twice.  Forward / forward and backward, us:
+//   63 tiles, 2 / 4 blocks    80 / 178 in one piece, 43 / 100 in 4, 23 / 60 in 16, 22 / 57 in 32, 25 / 66 in 96
+//   255 tiles, 32 / 64 blocks 350 / 885, 226 / 684 in 3, 186 / 612 in 4, 152 / 584 in 8, 149 / 556 in 12, 158 / 577 in 16, 178 / 649 in 64
+//   63 tiles, 64 / 128 blocks 107 / 304, 90 / 294 in 3, 82 / 291 in 4, 80 / 291 in 6, 84 / 301 in 16
+//   9 tiles, 2 / 4 blocks     20.6 / 47, 18.5 / 41 in 3, 16.5 / 39 in 5, 16.5 / 39 in 9
+// Fewer than seven tiles gain nothing.
+inline int piece_tiles(int nt, long long blocks) {
+    const int want = (int)std::min<long long>(3 * 148 / blocks, (long long)std::sqrt(6.0 * nt));
+    return nt < 7 || want < 3 ? nt : (nt + want - 1) / want;
+}
 
 // ---------------------------------------------------------------- fragments
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -229,6 +247,9 @@ __device__ __forceinline__ void tile_sums(float& c0, float& c1) {
 // Bound by the chain of its T / 64 steps, and within a step by shared memory and issue slots where an SM has two or three blocks.
 // 31 steps of (4, 1984, 20 heads), d_state 64: 75 us with 32 x 16 of the state per warp (the cut operand was then read back
 // by four warps) and 4-byte stores of the fragments (20 us of them).
+//
+// Where few blocks would walk far (pieces_of), the walk is cut into pieces that run side by side: a first launch makes each piece's own
+// sum, without a state before it, and in the second a block folds the sums of the pieces before its own into the state it starts from.
 // ------------------------------------------------------------------------------------------
 constexpr int kStateThreads = 160, kStateCols = 32;
 struct StateCfg {
@@ -238,7 +259,8 @@ struct StateCfg {
     static constexpr int OUT = 3 * MT * VP;          // elements: the pieces of the state on their way out
     static constexpr size_t SMEM = ((size_t)ST * STAGE + 2 * OUT) * 2 + (2 * MT + 4) * 4;
 };
-template <bool WIDE>
+// CUT: in pieces (a kernel of its own: with the bounds of a piece the walk of one piece took 2 % longer).
+template <bool WIDE, bool CUT>
 __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
     dep_wait();
     using Cfg = StateCfg;
@@ -248,21 +270,25 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
     float* dec = w + 2 * MT;
     const Dims& d = P.d;
     const int nb = (d.n + kStateCols - 1) / kStateCols;
-    const int hh = blockIdx.x / nb, col0 = (blockIdx.x % nb) * kStateCols, bb = blockIdx.y, dir = blockIdx.z;
+    const int piece = CUT ? blockIdx.x / (d.h * nb) : 0, hh = CUT ? blockIdx.x / nb % d.h : blockIdx.x / nb, col0 = (blockIdx.x % nb) * kStateCols, bb = blockIdx.y, dir = blockIdx.z;
     const int gg = hh / d.hpg, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    auto tile_of = [&](int it) { return dir ? P.nt - 1 - it : it; };
+    const bool summary = CUT && P.summary;
+    const int it0 = CUT ? piece * P.per : 0, steps = CUT ? min(P.per, P.nt - it0) : P.nt;
+    const size_t slot = ((((size_t)dir * d.b + bb) * d.h + hh) * nb + col0 / kStateCols) * (P.np - 1);  // of the first piece
+    auto tile_of = [&](int it) { return dir ? P.nt - 1 - it0 - it : it0 + it; };
     if (warp == 4) {  // the weights, and the arrays the other kernels read
         const bool given = P.a || P.cum;
         const float Ah = given ? 0.f : P.A_head[hh];
-        const bool keep = dir == 0 && col0 == 0;
+        const bool keep = dir == 0 && col0 == 0 && !summary;
+        float total = 0.f;
         Decay f0, f1;
         auto fetch = [&](int it) {
-            if (it >= P.nt) return;
+            if (it >= steps) return;
             f0 = fetch_decay(P, bb, hh, tile_of(it) * MT + lane);
             f1 = fetch_decay(P, bb, hh, tile_of(it) * MT + 32 + lane);
         };
         auto weights = [&](int it) {
-            if (it >= P.nt) return;
+            if (it >= steps) return;
             const int left = d.T - tile_of(it) * MT - lane;  // positions left from this lane's first
             const float d0 = left > 0 ? f0.dt : 0.f, d1 = left > 32 ? f1.dt : 0.f;
             float a0 = left > 0 ? (given ? f0.v : f0.dt * Ah) : 0.f, a1 = left > 32 ? (given ? f1.v : f1.dt * Ah) : 0.f;
@@ -273,6 +299,7 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
             o[lane] = dir ? exp_(a0) : exp_(S - a0) * d0;
             o[32 + lane] = dir ? exp_(a1) : exp_(S - a1) * d1;
             if (lane == 0) dec[it & 1] = exp_(S);
+            total += S;
             if (keep) {
                 float* k = P.sums + tile_off(d, P.nt, bb, tile_of(it), hh) * 2 * MT;
                 k[lane] = a0;
@@ -283,19 +310,20 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
         };
         fetch(0);
         weights(0);
-        for (int it = 0; it < P.nt; ++it) {
+        for (int it = 0; it < steps; ++it) {
             __syncthreads();
             weights(it + 1);
         }
+        if (summary && lane == 0) P.part_logdecay[slot + piece] = total;
         return;
     }
     const __nv_bfloat16* U = (dir ? P.dy : P.x) + ((size_t)bb * d.T * d.h + hh) * d.p;
     const __nv_bfloat16* V = (dir ? P.C : P.B) + ((size_t)bb * d.T * d.g + gg) * d.n + col0;
-    __nv_bfloat16* pieces = dir ? P.Q : P.H;
+    __nv_bfloat16* pieces = summary ? nullptr : dir ? P.Q : P.H;
     const uint32_t base = saddr(sh);
     auto stage = [&](int it) { return base + (it % Cfg::ST) * Cfg::STAGE * 2; };
     auto load = [&](int it) {  // one group of copies per tile, empty behind the last
-        if (it < P.nt) {
+        if (it < steps) {
             const int t0 = tile_of(it) * MT, rows = min(MT, d.T - t0);
             load_panel<64, WIDE>(stage(it), XP, U + (size_t)t0 * d.h * d.p, (size_t)d.h * d.p, rows, d.p);
             load_panel<kStateCols, WIDE>(stage(it) + kXPanel * 2, Cfg::VP, V + (size_t)t0 * d.g * d.n, (size_t)d.g * d.n, rows, d.n - col0);
@@ -305,7 +333,7 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
     load(0);
     load(1);
     float H[4][4];  // rows 16 q + g (+ 8), columns 2 t, 2 t + 1 of the warp's eight
-    const float* seed = dir ? P.dfinal : P.init;
+    const float* seed = summary ? nullptr : dir ? P.dfinal : P.init;
     const size_t bh = ((size_t)bb * d.h + hh) * d.p * d.n;
     const int nn0 = col0 + warp * 8 + 2 * t;
 #pragma unroll
@@ -314,6 +342,22 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
         for (int c = 0; c < 4; ++c) {
             const int pp = q * 16 + g + (c >> 1) * 8, nn = nn0 + (c & 1);
             H[q][c] = (seed && pp < d.p && nn < d.n) ? seed[bh + (size_t)pp * d.n + nn] : 0.f;
+        }
+    if (CUT && !summary)  // the pieces before this one
+#pragma unroll 4
+        for (int k = 0; k < piece; ++k) {
+            const float4* f = reinterpret_cast<const float4*>(P.part) + (slot + k) * 512 + threadIdx.x;
+            const float total = P.part_logdecay[slot + k], decay = exp_(total);
+            // (an infinite state lasts where only the decay over a whole piece is too small for a number)
+            auto step = [&](float h, float v) { return fmaf(isinf(h) && !isinf(total) ? 1.f : decay, h, v); };
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 v = f[q * 128];
+                H[q][0] = step(H[q][0], v.x);
+                H[q][1] = step(H[q][1], v.y);
+                H[q][2] = step(H[q][2], v.z);
+                H[q][3] = step(H[q][3], v.w);
+            }
         }
     auto stage_state = [&](int it) {  // the state before tile `it`, cut, on its way out
         uint32_t* o = reinterpret_cast<uint32_t*>(out + (it & 1) * Cfg::OUT + g * Cfg::VP + warp * 8 + 2 * t);
@@ -330,7 +374,7 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
             }
     };
     if (pieces) stage_state(0);
-    for (int it = 0; it < P.nt; ++it) {
+    for (int it = 0; it < steps; ++it) {
         cp_wait<1>();
         __syncthreads();  // there: the tile, its weights, the state before it.  Free: the stage of the last tile
         load(it + 2);
@@ -377,9 +421,15 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
         for (int q = 0; q < 4; ++q)
 #pragma unroll
             for (int c = 0; c < 4; ++c) H[q][c] = fmaf(decay, H[q][c], acc[q][c] + small[q][c]);
-        if (pieces && it + 1 < P.nt) stage_state(it + 1);
+        if (pieces && it + 1 < steps) stage_state(it + 1);
     }
-    if (float* o = dir ? P.dinit : P.final_state)
+    if (summary) {
+        float4* o = reinterpret_cast<float4*>(P.part) + (slot + piece) * 512 + threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[q * 128] = make_float4(H[q][0], H[q][1], H[q][2], H[q][3]);
+        return;
+    }
+    if (float* o = CUT && piece + 1 < P.np ? nullptr : dir ? P.dinit : P.final_state)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll

@@ -213,11 +213,13 @@ def test_partial_tiles_keep_fp32_arithmetic(pkg, cabi, oracle, b, T, h, p, n, g,
 
 
 @pytest.mark.parametrize("b,T,h,p,n,g,l", [(1, 2, 1, 64, 64, 1, 1), (2, 63, 3, 64, 72, 3, 21), (1, 65, 4, 40, 128, 2, 65), (2, 192, 8, 64, 64, 1, 96),
-                                           (3, 330, 6, 56, 40, 2, 30), (8, 640, 5, 64, 64, 5, 32)])
+                                           (3, 330, 6, 56, 40, 2, 30), (8, 640, 5, 64, 64, 5, 32), (1, 448, 1, 64, 64, 1, 32), (1, 1985, 2, 40, 72, 1, 397),
+                                           (2, 4090, 2, 64, 128, 1, 409)])
 @pytest.mark.parametrize("form", ["mamba2", "operator"])
 def test_partial_tiles_products_of_pieces(pkg, cabi, oracle, form, b, T, h, p, n, g, l):
     """The kernels for bf16 calls of partial tiles against the oracle in 64 bits: one position and one behind a tile, headdim and
-    d_state that end inside their panels, the heads of a group on one block and on several, log-decays in fp32 and bf16.  The
+    d_state that end inside their panels, the heads of a group on one block and on several, walks over the states in 1, 4 (the last
+    one shorter), 11 and 16 pieces, log-decays in fp32 and bf16.  The
     three bf16 pieces of an operand carry all of its 24 bits, so what is left is the rounding of fp32 sums of at most a few
     thousand terms: 1e-5 of the largest value (two pieces would be 2^-16 off per term).  dA_head is a sum of b T signed terms
     da dt, each right to 1e-6 of the largest, and some sqrt(b T) = 72 times smaller than their absolute sum: 1e-4."""
@@ -249,7 +251,7 @@ def test_partial_tiles_products_of_pieces(pkg, cabi, oracle, form, b, T, h, p, n
 
 
 @pytest.mark.parametrize("case", ["state overflows", "gradient overflows", "x", "dy", "B", "C", "init", "dfinal"])
-@pytest.mark.parametrize("T,n", [(192, 64), (192, 128), (40, 64)])
+@pytest.mark.parametrize("T,n", [(192, 64), (192, 128), (40, 64), (640, 64)])
 def test_partial_tiles_infinite_values(pkg, cabi, case, T, n):
     """Infinite values among the inputs, and states and their gradients that leave the range of fp32: a result that is finite, or
     infinite, with the fp32 multiply-adds of the SIMT path on the same tiles is finite, or the same infinity, here.  (An infinite value
@@ -286,7 +288,7 @@ def test_partial_tiles_infinite_values(pkg, cabi, case, T, n):
     assert infinite
 
 
-@pytest.mark.parametrize("dtype,T,n,l", [("fp32", 192, 64, 64), ("bf16", 330, 64, 30), ("bf16", 2048, 128, 128)])
+@pytest.mark.parametrize("dtype,T,n,l", [("fp32", 192, 64, 64), ("bf16", 330, 64, 30), ("bf16", 990, 64, 30), ("bf16", 2048, 128, 128)])
 def test_launch_order_eager_and_captured(pkg, cabi, dtype, T, n, l):
     """Kernels are set up while the one before them runs: the same bits call after call, on inputs and memory that the calls before
     have used, and from a captured graph, on the kernels of each path."""
