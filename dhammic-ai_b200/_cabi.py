@@ -17,7 +17,7 @@ FWD_AUX_VALID = 2
 BWD_DINIT_ONLY = 1
 
 EXPORTS = (
-    "ssd_b200_abi_version", "ssd_b200_last_error", "ssd_b200_workspace_bytes", "ssd_b200_states_bytes",
+    "ssd_b200_abi_version", "ssd_b200_last_error", "ssd_b200_workspace_bytes", "ssd_b200_workspace_min_bytes", "ssd_b200_states_bytes",
     "ssd_b200_resolve_path",
     "ssd_b200_fwd", "ssd_b200_bwd", "ssd_b200_materialize_cache", "ssd_b200_state_prefix_all", "ssd_b200_ipc_export", "ssd_b200_ipc_import", "ssd_b200_ipc_close", "ssd_b200_enable_peer_access", "ssd_b200_exchange_push", "ssd_b200_exchange_arrive",
     "ssd_b200_m3_prologue_fwd", "ssd_b200_m3_skip_fwd", "ssd_b200_m3_prologue_bwd", "ssd_b200_m3_chain_ws_floats", "ssd_b200_m3_chain_bwd", "ssd_b200_rope_fwd", "ssd_b200_rope_bwd",
@@ -73,6 +73,8 @@ def load() -> C.CDLL:
     lib.ssd_b200_last_error.restype = C.c_char_p
     lib.ssd_b200_workspace_bytes.restype = C.c_size_t
     lib.ssd_b200_workspace_bytes.argtypes = [C.POINTER(Shape), C.c_int]
+    lib.ssd_b200_workspace_min_bytes.restype = C.c_size_t
+    lib.ssd_b200_workspace_min_bytes.argtypes = [C.POINTER(Shape), C.c_int]
     lib.ssd_b200_states_bytes.restype = C.c_size_t
     lib.ssd_b200_states_bytes.argtypes = [C.POINTER(Shape)]
     lib.ssd_b200_resolve_path.restype = C.c_int

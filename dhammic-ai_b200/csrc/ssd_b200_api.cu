@@ -772,8 +772,17 @@ size_t ssd_b200_workspace_bytes(const ssd_b200_shape* shape, int pass) {
     if (path < 0) return 0;
     ssd::Dims d = dims_of(*shape);
     if (path == SSD_B200_PATH_TC) return ssd::tc::workspace_bytes(d, pass);
-    const size_t simt = simt_ws(d, pass).total;  // which is what a call needs; the tensor-core kernels run where there is room for them
+    const size_t simt = simt_ws(d, pass).total;  // the tensor-core kernels run where there is room for them
     return mma_shape(*shape) ? std::max(simt, mma_ws(d, pass).total) : simt;
+}
+
+size_t ssd_b200_workspace_min_bytes(const ssd_b200_shape* shape, int pass) {
+    if (check_shape(shape)) return 0;
+    if (pass != SSD_B200_PASS_FWD && pass != SSD_B200_PASS_BWD) return 0;
+    const int path = resolve_path(*shape);
+    if (path < 0) return 0;
+    const ssd::Dims d = dims_of(*shape);
+    return path == SSD_B200_PATH_TC ? ssd::tc::ws_layout(d, pass).base : simt_ws(d, pass).total;
 }
 
 size_t ssd_b200_states_bytes(const ssd_b200_shape* shape) {
@@ -868,9 +877,7 @@ int ssd_b200_fwd_static_scratch(const ssd_b200_fwd_args* a, void* stream) {
     if (int rc = check_shape(&a->shape)) return rc;
     int path = resolve_path(a->shape);
     if (path < 0) return path;
-    // (a tensor-core walk runs in one piece where the room for more is missing)
-    const size_t need = path == SSD_B200_PATH_TC ? ssd::tc::ws_layout(dims_of(a->shape), SSD_B200_PASS_FWD).base
-                                                 : simt_ws(dims_of(a->shape), SSD_B200_PASS_FWD).total;
+    const size_t need = ssd_b200_workspace_min_bytes(&a->shape, SSD_B200_PASS_FWD);
     if (need > (size_t)SSD_B200_STATIC_SCRATCH_BYTES)
         return fail(SSD_B200_EWORKSPACE,
                     "this shape needs %zu bytes of scratch but the built-in array holds %u; use ssd_b200_fwd with a "

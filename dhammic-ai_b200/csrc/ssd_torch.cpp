@@ -107,10 +107,16 @@ ssd_b200_shape make_shape(const Tensor& x, int a_dtype, const Tensor& B, int64_t
     return {SSD_B200_ABI_VERSION, dtype_code(x), a_dtype, path, x.size(0), x.size(1), x.size(2), x.size(3), B.size(3), B.size(2), chunk};
 }
 
+// The workspace of a call, or the least it runs with where the device has no room for the whole.
 Tensor workspace(const ssd_b200_shape& s, int pass, const Tensor& like) {
-    const size_t n = ssd_b200_workspace_bytes(&s, pass);
+    const size_t n = ssd_b200_workspace_bytes(&s, pass), least = ssd_b200_workspace_min_bytes(&s, pass);
     if (n == 0) check(ssd_b200_resolve_path(&s));
-    return bytes(n, like);
+    try {
+        return bytes(n, like);
+    } catch (const c10::OutOfMemoryError&) {
+        if (least >= n) throw;
+    }
+    return bytes(least, like);
 }
 
 void check_status(const ssd_b200_shape& s, const Tensor& ws) {

@@ -271,7 +271,7 @@ class CudaBackend:
             final = out_F if out_F is not None else torch.empty(b, h, p, n, dtype=torch.float32, device=dev)
             logp = out_logp if out_logp is not None else torch.empty(b, h, dtype=torch.float32, device=dev)
             cum = torch.empty(b, h, T // s.chunk, s.chunk, dtype=torch.float32, device=dev)
-            ws = _op._workspace(lib, shape, _cabi.PASS_FWD, dev)
+            ws = _op._workspace(lib, shape, _cabi.PASS_FWD, dev, summary=True)
             # the buffer the full pass keeps its per-tile states in: this pass already fills its per-position arrays
             nbytes = int(lib.ssd_b200_states_bytes(C.byref(shape)))
             states = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
@@ -297,7 +297,7 @@ class CudaBackend:
         shape = saved["shape"]
         with torch.cuda.device(dev):
             dinit = out if out is not None else torch.empty(b, h, p, s.B.shape[3], dtype=torch.float32, device=dev)
-            ws = _op._workspace(lib, shape, _cabi.PASS_BWD, dev)
+            ws = _op._workspace(lib, shape, _cabi.PASS_BWD, dev, summary=True)
             args = _cabi.BwdArgs(shape, None, None, None, None, None, None, _op._ptr(s.C), None, _op._ptr(saved["cum"]),
                                  _op._ptr(dy), _op._ptr(dfinal), None, None, None, None, None, None, None,
                                  _op._ptr(dinit), 0, _cabi.BWD_DINIT_ONLY, _op._ptr(ws), ws.numel(), _op._ptr(saved.get("states")))

@@ -99,11 +99,18 @@ def _make_shape(x: Tensor, a_dtype: int, B: Tensor, chunk: int) -> _cabi.Shape:
                        int(chunk))
 
 
-def _workspace(lib, shape: _cabi.Shape, which: int, dev) -> Tensor:
-    nbytes = lib.ssd_b200_workspace_bytes(C.byref(shape), which)
+def _workspace(lib, shape: _cabi.Shape, which: int, dev, summary: bool = False) -> Tensor:
+    """The workspace of a call, or the least it runs with: for a summary, and where the device has no room for the whole."""
+    least = int(lib.ssd_b200_workspace_min_bytes(C.byref(shape), which))
+    nbytes = least if summary else int(lib.ssd_b200_workspace_bytes(C.byref(shape), which))
     if nbytes == 0:
         _cabi.check(lib.ssd_b200_resolve_path(C.byref(shape)))
-    return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)
+    try:
+        return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        if least >= nbytes:
+            raise
+    return torch.empty(max(least, 256), dtype=torch.uint8, device=dev)
 
 
 class LazySSDCache(dict):

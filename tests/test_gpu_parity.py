@@ -348,6 +348,34 @@ def test_partial_tiles_in_less_workspace(pkg, cabi):
     assert rc2 == [cabi.EWORKSPACE, cabi.EWORKSPACE]
 
 
+def test_partial_tiles_where_memory_is_short(pkg, cabi):
+    """With chunks of 1000 positions the pieces of the states take 24 times the room of the fp32 states of the chunks.  A call that has
+    room for the latter only runs on the kernels that need no more."""
+    cfg = replace(pkg.CONFIGS[2], batch=4, seqlen=4000, nheads=20, ngroups=5, chunk=1000)
+    inp = {k: v.to(DEV) for k, v in pkg.make_inputs(cfg, seed=9).items()}
+
+    def call():
+        lv = [inp[k].detach().requires_grad_(True) for k in ("x", "dt", "A_head", "B", "C", "D")]
+        y, fs = pkg.ssd_mamba2(*lv, cfg.chunk)
+        return [y.detach(), fs.detach()] + list(torch.autograd.grad([y], lv, [inp["dy"]]))
+
+    want = call()
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, 4, 4000, 20, 64, 128, 5, 1000)
+    import ctypes
+    full, least = (int(f(ctypes.byref(shape), cabi.PASS_BWD)) for f in (cabi.load().ssd_b200_workspace_bytes, cabi.load().ssd_b200_workspace_min_bytes))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    room = least + 200 * 2 ** 20  # the outputs and the allocator's blocks
+    assert room < full
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        got = call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for k, a, b in zip(("y", "final", "dx", "ddt", "dA_head", "dB", "dC", "dD"), got, want):
+        assert rel_err(a, b) < (1e-4 if a.dtype == torch.float32 else 2 ** -7), k
+
+
 def test_cached_call_takes_any_chunk(pkg, cabi):
     """With the sums given, nothing bounds the chunk (2048 positions of 32 heads are too many for the kernel that makes the sums,
     which is refused); same result as with chunks of 128."""
