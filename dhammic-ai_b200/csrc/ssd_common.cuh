@@ -62,6 +62,20 @@ __device__ __forceinline__ void dep_wait_early() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Sum over a block of THREADS threads, valid in all of them; red: one float per warp.
+template <int THREADS>
+__device__ __forceinline__ float block_sum(float v, float* red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) s += red[w];
+    return s;
+}
+
 namespace prof {
 // Kernel slots for launch accounting / optional per-kernel timing (definitions in ssd_b200_api.cu).
 enum Kernel {

@@ -6,8 +6,9 @@
 // and the tensor cores add the exact products up in fp32, small pieces first.  Products of two given operands (C B^T, dY x^T) need one.
 //
 // Why mma.sync: the pieces are made in the registers that hold the accumulator of the product before (the fragment of D is the
-// fragment of A of the next product), so a masked score never leaves the registers.  On tcgen05 every piece would go back
-// through TMEM or shared memory: three panels per operand, which the shared memory of these kernels has no room for.
+// fragment of A of the next product), so a masked score never leaves the registers; on tcgen05 every piece would go through TMEM and a
+// barrier.  The rate of the products is not what bounds these kernels: the chain of the walk over the states is, and the latency of a head's
+// loads and fragments.
 //
 // Tiles are 64 positions whatever the caller's chunk (the recurrence does not depend on where chunks end); what lies behind the
 // end of a sequence is zero in shared memory.
@@ -78,7 +79,7 @@ inline int piece_tiles(int nt, long long blocks) {
 }
 
 // ---------------------------------------------------------------- fragments
-__device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+using ptx::smem_u32;
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
@@ -141,6 +142,7 @@ __device__ __forceinline__ void zero(float (&acc)[N][4]) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
 }
+// (As __expf, without the instructions that keep results below 2^-126.)
 __device__ __forceinline__ float exp_(float v) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v * 1.4426950408889634f));
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
     const __nv_bfloat16* U = (dir ? P.dy : P.x) + ((size_t)bb * d.T * d.h + hh) * d.p;
     const __nv_bfloat16* V = (dir ? P.C : P.B) + ((size_t)bb * d.T * d.g + gg) * d.n + col0;
     __nv_bfloat16* pieces = summary ? nullptr : dir ? P.Q : P.H;
-    const uint32_t base = saddr(sh);
+    const uint32_t base = smem_u32(sh);
     auto stage = [&](int it) { return base + (it % Cfg::ST) * Cfg::STAGE * 2; };
     auto load = [&](int it) {  // one group of copies per tile, empty behind the last
         if (it < steps) {
@@ -558,7 +560,7 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) scan_kernel(Params P) 
     __nv_bfloat16* xs = sh + 5 * kBPanel<NN>;
     float* cum = reinterpret_cast<float*>(xs + kXPanel);
     float* dts = cum + MT;
-    const uint32_t sC = saddr(sh), sB = sC + kBPanel<NN> * 2, sH = sB + kBPanel<NN> * 2, sX = saddr(xs);
+    const uint32_t sC = smem_u32(sh), sB = sC + kBPanel<NN> * 2, sH = sB + kBPanel<NN> * 2, sX = smem_u32(xs);
     const size_t bc = (((size_t)w.bb * d.T + w.t0) * d.g + w.gg) * d.n;
     load_panel<NN, WIDE>(sC, kBP<NN>, P.C + bc, (size_t)d.g * d.n, w.rows, d.n);
     load_panel<NN, WIDE>(sB, kBP<NN>, P.B + bc, (size_t)d.g * d.n, w.rows, d.n);
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) scan_kernel(Params P) 
         if (hl) __syncthreads();
         load_panel<64, WIDE>(sX, XP, P.x + xo, (size_t)d.h * d.p, w.rows, d.p);
         const size_t tile = tile_off(d, P.nt, w.bb, w.k, hh);
-        load_sums(saddr(cum), P, tile);
+        load_sums(smem_u32(cum), P, tile);
         load_pieces<NN>(sH, P.H + tile * 3 * d.p * d.n, d);
         cp_commit();
         cp_wait<0>();
@@ -706,7 +708,7 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) bwd_kernel(Params P) {
     __nv_bfloat16* ys = xs + kXPanel;
     float* cum = reinterpret_cast<float*>(ys + kXPanel);
     float* dts = cum + MT;
-    const uint32_t sOwn = saddr(sh), sOther = sOwn + kBPanel<NN> * 2, sW = sOther + kBPanel<NN> * 2, sX = saddr(xs), sY = saddr(ys);
+    const uint32_t sOwn = smem_u32(sh), sOther = sOwn + kBPanel<NN> * 2, sW = sOther + kBPanel<NN> * 2, sX = smem_u32(xs), sY = smem_u32(ys);
     const size_t bc = (((size_t)w.bb * d.T + w.t0) * d.g + w.gg) * d.n;
     load_panel<NN, WIDE>(sOwn, kBP<NN>, (row_pass ? P.C : P.B) + bc, (size_t)d.g * d.n, w.rows, d.n);
     load_panel<NN, WIDE>(sOther, kBP<NN>, (row_pass ? P.B : P.C) + bc, (size_t)d.g * d.n, w.rows, d.n);
@@ -737,7 +739,7 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) bwd_kernel(Params P) {
         load_panel<64, WIDE>(sX, XP, P.x + xo, (size_t)d.h * d.p, w.rows, d.p);
         load_panel<64, WIDE>(sY, XP, P.dy + xo, (size_t)d.h * d.p, w.rows, d.p);
         const size_t tile = tile_off(d, P.nt, w.bb, w.k, hh);
-        load_sums(saddr(cum), P, tile);
+        load_sums(smem_u32(cum), P, tile);
         cp_commit();
         load_pieces<NN>(sW, (row_pass ? P.H : P.Q) + tile * 3 * d.p * d.n, d);
         cp_commit();
@@ -939,17 +941,6 @@ __global__ void __launch_bounds__(NTHR, NN == 64 ? 3 : 2) bwd_kernel(Params P) {
 // 31 tiles.)  Four tiles a step, the next values on their way meanwhile.  The blocks behind them: dB and dC of a split group.
 // ------------------------------------------------------------------------------------------
 constexpr int kDecayThreads = 256;
-__device__ __forceinline__ float block_sum(float v, float* red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float s = 0.f;
-#pragma unroll
-    for (int w = 0; w < kDecayThreads / 32; ++w) s += red[w];
-    return s;
-}
 template <bool WIDE>
 __global__ void __launch_bounds__(kDecayThreads) decay_kernel(Params P) {
     dep_wait();
@@ -979,7 +970,7 @@ __global__ void __launch_bounds__(kDecayThreads) decay_kernel(Params P) {
         float v = 0.f;
 #pragma unroll 8
         for (size_t e = threadIdx.x; e < pn; e += kDecayThreads) v += P.dfinal[bh * pn + e] * P.final_state[bh * pn + e];
-        R = block_sum(v, red);
+        R = block_sum<kDecayThreads>(v, red);
     }
     const bool form2 = P.dt != nullptr;
     const float Ah = form2 ? P.A_head[hh] : 0.f;
@@ -1044,10 +1035,10 @@ __global__ void __launch_bounds__(kDecayThreads) decay_kernel(Params P) {
         }
     }
     if (form2) {
-        const float s = block_sum(dAh, red);
+        const float s = block_sum<kDecayThreads>(dAh, red);
         if (threadIdx.x == 0) P.dAh_part[bh] = s;
         if (P.dyx) {
-            const float sd = block_sum(yx, red);
+            const float sd = block_sum<kDecayThreads>(yx, red);
             if (threadIdx.x == 0) P.dD_part[bh] = sd;
         }
     }

@@ -725,18 +725,6 @@ __host__ inline size_t chunk_bwd_smem(const Dims& d, int pt, bool share_ws) {
     return ((size_t)2 * TS * ld_of(d.n) + 2 * TS * ld_of(d.p) + 2 * TS * TS + (size_t)(share_ws ? 0 : pt) * TS * TS + 4 * TS) * 4;
 }
 
-__device__ __forceinline__ float block_sum(float v, float* red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    float t = 0.f;
-    for (int w = 0; w < NTHR / 32; ++w) t += red[w];
-    return t;
-}
-
 // ------------------------------------------------------------------------------------------
 // What the backward's blocks left in parts.  Blocks [0, b h): the decay gradient of one (head, batch),
 // g = g_row - g_col (+ <dfinal, final> at T-1), d a_t = reverse inclusive cumsum of g over the whole sequence (tiles of 256
@@ -773,7 +761,7 @@ __global__ void __launch_bounds__(NTHR) decay_grad_kernel(Params P) {
         float v = 0.f;
 #pragma unroll 8
         for (size_t e = threadIdx.x; e < pn; e += NTHR) v += a[e] * f[e];
-        gfin = block_sum(v, red);
+        gfin = block_sum<NTHR>(v, red);
     }
     const size_t base = ((size_t)bb * d.h + hh) * d.T;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -831,10 +819,10 @@ __global__ void __launch_bounds__(NTHR) decay_grad_kernel(Params P) {
         }
     }
     if (form2) {
-        const float s = block_sum(dAh, red);
+        const float s = block_sum<NTHR>(dAh, red);
         if (threadIdx.x == 0) P.dAh_part[(size_t)bb * d.h + hh] = s;
         if (P.dyx) {
-            const float sd = block_sum(yx, red);
+            const float sd = block_sum<NTHR>(yx, red);
             if (threadIdx.x == 0) P.dD_part[(size_t)bb * d.h + hh] = sd;
         }
     }

@@ -214,16 +214,22 @@ def test_partial_tiles_keep_fp32_arithmetic(pkg, cabi, oracle, b, T, h, p, n, g,
 
 @pytest.mark.parametrize("b,T,h,p,n,g,l", [(1, 2, 1, 64, 64, 1, 1), (2, 63, 3, 64, 72, 3, 21), (1, 65, 4, 40, 128, 2, 65), (2, 192, 8, 64, 64, 1, 96),
                                            (3, 330, 6, 56, 40, 2, 30), (8, 640, 5, 64, 64, 5, 32), (1, 448, 1, 64, 64, 1, 32), (1, 1985, 2, 40, 72, 1, 397),
-                                           (2, 4090, 2, 64, 128, 1, 409)])
+                                           (2, 4090, 2, 64, 128, 1, 409),
+                                           (4, 1240, 20, 64, 64, 5, 40), (1, 3008, 30, 64, 64, 5, 47), (8, 1248, 4, 64, 128, 2, 48)])
 @pytest.mark.parametrize("form", ["mamba2", "operator"])
 def test_partial_tiles_products_of_pieces(pkg, cabi, oracle, form, b, T, h, p, n, g, l):
     """The kernels for bf16 calls of partial tiles against the oracle in 64 bits: one position and one behind a tile, headdim and
-    d_state that end inside their panels, the heads of a group on one block and on several, walks over the states in 1, 4 (the last
+    d_state that end inside their panels, one head per block and, in the last three, 4, 3 and 2 (on one block for the group, on two, on
+    one with d_state 128), walks over the states in 1, 4 (the last
     one shorter), 11 and 16 pieces, log-decays in fp32 and bf16.  The
     three bf16 pieces of an operand carry all of its 24 bits, so what is left is the rounding of fp32 sums of at most a few
     thousand terms: 1e-5 of the largest value (two pieces would be 2^-16 off per term).  dA_head is a sum of b T signed terms
     da dt, each right to 1e-6 of the largest, and some sqrt(b T) = 72 times smaller than their absolute sum: 1e-4."""
     cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, headdim=p, d_state=n, ngroups=g, chunk=l)
+    base, hpg, splits = (T + 63) // 64 * b * g, h // g, 1  # blocks that share a group, as the library counts them
+    while splits < hpg and (base * splits < 2 * 148 or hpg % splits):
+        splits += 1
+    assert hpg // splits == {1240: 4, 3008: 3, 1248: 2}.get(T, 1)
     inp = pkg.make_inputs(cfg, seed=31)
     gen = torch.Generator().manual_seed(32)
     init, dfinal = torch.randn(b, h, p, n, generator=gen) * 0.2, torch.randn(b, h, p, n, generator=gen)
@@ -338,14 +344,22 @@ def test_partial_tiles_in_less_workspace(pkg, cabi):
     def up(v):
         return (v + 255) // 256 * 256
     rows, parts = up(2 * 4 * 192 * 4), up(2 * 192 * 2 * 2 * 128 * 4)
+    import ctypes
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, 2, 192, 4, 64, 128, 2, 96)
     ws = {cabi.PASS_FWD: 2 * state, cabi.PASS_BWD: 5 * state + 4 * rows + 2 * 256 + 2 * parts}
-    rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
-    rc1, got = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, ws)
-    assert rc0 == rc1 == [0, 0]
+    lib, res = cabi.load(), []
+    for path, room in ((cabi.PATH_AUTO, None), (cabi.PATH_AUTO, ws), (cabi.PATH_SIMT, ws)):
+        before = cabi.launch_count()
+        res.append(_cabi_passes(pkg, cabi, cfg, inp, (), path, room) + (cabi.launch_count() - before,))
+    (rc0, want, n0), (rc1, got, n1), (rc2, simt, n2) = res
+    assert rc0 == rc1 == rc2 == [0, 0]
+    assert n0 < n1 == n2  # 3 + 4 launches against 4 + 7
     for k in want:
-        assert rel_err(got[k], want[k]) < (1e-5 if want[k].dtype == torch.float32 else 2 ** -7), k
-    rc2, _ = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {k: v - 1 for k, v in ws.items()})
-    assert rc2 == [cabi.EWORKSPACE, cabi.EWORKSPACE]
+        assert torch.equal(got[k], simt[k]) and rel_err(got[k], want[k]) < (1e-5 if want[k].dtype == torch.float32 else 2 ** -7), k
+    assert not torch.equal(want["ddt"], simt["ddt"])
+    assert [int(lib.ssd_b200_workspace_min_bytes(ctypes.byref(shape), k)) for k in sorted(ws)] == [ws[k] for k in sorted(ws)]
+    rc3, _ = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {k: v - 1 for k, v in ws.items()})
+    assert rc3 == [cabi.EWORKSPACE, cabi.EWORKSPACE]
 
 
 def test_partial_tiles_where_memory_is_short(pkg, cabi):
@@ -470,17 +484,18 @@ def _cabi_passes(pkg, cabi, cfg, inp, shifted, path, ws_bytes=None):
 
 
 @pytest.mark.parametrize("shifted", [("x",), ("B", "C"), ("y",), ("dy", "dx"), ("dB",), ("x", "B", "C", "y", "dy", "dx", "dB", "dC")])
-@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
-def test_unaligned_tensors_through_the_c_abi(pkg, cabi, dtype, shifted):
-    """The SIMT kernels take any address: the same bits as with aligned tensors.  The tensor-core kernels refuse on the host."""
-    cfg = replace(pkg.CONFIGS[2], dtype=dtype, batch=2, seqlen=192, nheads=4, ngroups=2, chunk=64)
+@pytest.mark.parametrize("dtype,n,g", [("bf16", 128, 2), ("bf16", 64, 4), ("bf16", 128, 4), ("fp32", 128, 2)])
+def test_unaligned_tensors_through_the_c_abi(pkg, cabi, dtype, n, g, shifted):
+    """The SIMT kernels and those for partial tiles (d_state 64 and 128, dB and dC from one block and from several) take any address: the same
+    bits as with aligned tensors.  The tcgen05 kernels refuse on the host."""
+    cfg = replace(pkg.CONFIGS[2], dtype=dtype, batch=2, seqlen=192, nheads=4, ngroups=g, d_state=n, chunk=64)
     inp = pkg.make_inputs(cfg, seed=6)
     rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
     rc1, got = _cabi_passes(pkg, cabi, cfg, inp, shifted, cabi.PATH_AUTO)
     assert rc0 == rc1 == [0, 0]
     for k in want:
         assert torch.equal(want[k], got[k]), k
-    if dtype == "bf16":
+    if dtype == "bf16" and n == 128:
         whole = replace(cfg, seqlen=256)
         rcs, _ = _cabi_passes(pkg, cabi, whole, pkg.make_inputs(whole, seed=6), shifted, cabi.PATH_AUTO)
         refused = [bool({"x", "B", "C", "y"} & set(shifted)), bool({"x", "B", "C", "dy", "dx", "dB", "dC"} & set(shifted))]
