@@ -55,8 +55,11 @@ inline void launch_dep(bool after, void (*kernel)(K...), dim3 grid, dim3 block, 
 }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Also lets the blocks of the kernel behind come to the SMs as soon as all of this one's have, instead of when they end.  For the SIMT
-// kernels, whose blocks are small and short: forward + backward of (2, 512, 8 heads, 64), d_state 64, fp32, 110 -> 103 us.  The kernels
-// with a block per SM lose by it (prefill 183.5 -> 197 us, (8, 2048, 24 heads) 248 -> 268).
+// kernels, whose blocks are small and short: forward + backward as a captured graph (called one by one they wait for the host and show
+// nothing), fp32, with dep_wait and with this: (2, 512, 8 heads, 32), d_state 8, 79.9 -> 73.8 us, (1, 1024, 4 heads, 32), d_state 16,
+// 53.3 -> 51.3, (1, 1984, 20 heads, 64), d_state 64, 299 -> 294.  Not ahead of the forward's scan, whose large blocks then come to SMs that
+// the state pass half fills: forward of (2, 512, 8 heads, 64), d_state 64, 26.7 -> 32.8.  The kernels with a block per SM lose by it
+// (prefill 183.5 -> 197 us, (8, 2048, 24 heads) 248 -> 268).
 __device__ __forceinline__ void dep_wait_early() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

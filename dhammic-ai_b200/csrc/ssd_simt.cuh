@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(NTHR) chunk_state_kernel(Params P, int mode) {
 // reverse : slot k <- Q_k = dH_{k+1},               dH_k   = exp(S_k) Q_k + local_k ; dinit = dH_0
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(NTHR) state_passing_kernel(Params P, int reverse) {
-    dep_wait_early();
+    if (reverse) dep_wait_early();
+    else dep_wait();  // blocks of the forward scan that come while this kernel's hold the SMs are spread unevenly
     const Dims& d = P.d;
     const size_t pn = (size_t)d.p * d.n;
     const size_t e = (size_t)blockIdx.x * NTHR + threadIdx.x;
