@@ -226,6 +226,9 @@ __device__ __forceinline__ Decay fetch_decay(const Params& P, int bb, int hh, in
     } else if (P.a) r.v = P.a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)P.a)[i]) : ((const float*)P.a)[i];
     return r;
 }
+// A log-decay as it enters the sums of a tile.  exp_ is zero below -87.4, so nothing passes a position of -90 either; lower values, down to a
+// type's lowest for a cut, would only take their bits from the sums of the positions behind, which may lie in other chunks of the caller's.
+__device__ __forceinline__ float cut_off(float a) { return a < -90.f ? -90.f : a; }
 // Inclusive sums over the 64 positions of a tile: lane l holds positions l and l + 32.  The whole warp.
 __device__ __forceinline__ void tile_sums(float& c0, float& c1) {
     const int lane = threadIdx.x & 31;
@@ -293,7 +296,7 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
             if (it >= steps) return;
             const int left = d.T - tile_of(it) * MT - lane;  // positions left from this lane's first
             const float d0 = left > 0 ? f0.dt : 0.f, d1 = left > 32 ? f1.dt : 0.f;
-            float a0 = left > 0 ? (given ? f0.v : f0.dt * Ah) : 0.f, a1 = left > 32 ? (given ? f1.v : f1.dt * Ah) : 0.f;
+            float a0 = left > 0 ? cut_off(given ? f0.v : f0.dt * Ah) : 0.f, a1 = left > 32 ? cut_off(given ? f1.v : f1.dt * Ah) : 0.f;
             fetch(it + 1);
             tile_sums(a0, a1);
             const float S = __shfl_sync(0xffffffffu, a1, 31);

@@ -294,6 +294,30 @@ def test_partial_tiles_infinite_values(pkg, cabi, case, T, n):
     assert infinite
 
 
+@pytest.mark.parametrize("low", [-1e4, -1e30, -3.38e38])
+@pytest.mark.parametrize("cached", [False, True])
+def test_partial_tiles_resets_at_chunk_ends(pkg, cabi, oracle, low, cached):
+    """Log-decays that cut the sequence off what lies before, down to the lowest values of bf16, at the last position of chunks of 16: the
+    positions behind keep their own decays, whatever the kernels' tiles are.  The oracle in 64 bits gets -1000, which is as much of a cut.
+    Two cuts a tile leave sums of up to 200, whose rounding of 2^-17 is what the factors between two positions are off by, twice: 2e-5."""
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=208, nheads=4, ngroups=2, d_state=64, chunk=16)
+    inp = pkg.make_inputs(cfg, seed=17)
+    res, a = [], inp["dt"] * inp["A_head"]
+    for v in (low, -1000.0):
+        a = a.clone()
+        a[:, [15, 31, 143, 159]] = v
+        res.append(a)
+    cache = None
+    if cached:
+        cache = {"A_cumsum": res[0].view(1, 13, 16, 4).cumsum(2).permute(0, 3, 1, 2).contiguous().to(DEV)}
+    got = run_operator(pkg, inp["x"], res[0], inp["B"], inp["C"], 16, None, inp["dy"], None, cache)
+    lv = [t.double().requires_grad_(True) for t in (inp["x"], res[1], inp["B"], inp["C"])]
+    Y, fs, _ = oracle.ssd_chunked(lv[0], lv[1], oracle.expand_groups(lv[2], 4), oracle.expand_groups(lv[3], 4), 16)
+    want = dict(zip(("dx", "dA", "dB", "dC"), torch.autograd.grad(Y, lv, inp["dy"].double())), Y=Y, final=fs)
+    for k in ("Y", "final", "dx", "dB", "dC") + (() if cached else ("dA",)):  # the others are rounded to bf16
+        assert rel_err(got[k], want[k].detach().reshape(got[k].shape)) < (2e-5 if k == "dA" else 2 ** -8), k
+
+
 @pytest.mark.parametrize("dtype,T,n,l", [("fp32", 192, 64, 64), ("bf16", 330, 64, 30), ("bf16", 990, 64, 30), ("bf16", 2048, 128, 128)])
 def test_launch_order_eager_and_captured(pkg, cabi, dtype, T, n, l):
     """Kernels are set up while the one before them runs: the same bits call after call, on inputs and memory that the calls before
