@@ -214,7 +214,7 @@ MmaWs mma_ws(const ssd::Dims& d, int pass) {
     };
     const size_t pieces = (size_t)d.b * ssd::mma::tiles(d.T) * d.h * 3 * d.p * d.n * 2;
     w.H = take(pieces);
-    w.sums = take((size_t)d.b * ssd::mma::tiles(d.T) * d.h * 2 * ssd::mma::MT * 4);
+    w.sums = take((size_t)d.b * ssd::mma::tiles(d.T) * d.h * 3 * ssd::mma::MT * 4);
     const int dirs = pass == SSD_B200_PASS_BWD ? 2 : 1, per = mma_per(d, dirs);
     const size_t sums = (size_t)dirs * d.b * d.h * mma_state_cols(d) * ((ssd::mma::tiles(d.T) - 1) / per);
     w.part = take(sums * 2048 * 4);

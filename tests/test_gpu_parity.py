@@ -294,6 +294,20 @@ def test_partial_tiles_infinite_values(pkg, cabi, case, T, n):
     assert infinite
 
 
+@pytest.mark.parametrize("l", [16, 32])
+def test_partial_tiles_fast_decay_in_short_chunks(pkg, cabi, oracle, l):
+    """Log-decays of -0.02 to -30: what is left of a position at the end of its tile is taken from the sum of the decays behind it, not from a
+    difference of sums of some hundreds (1e-5 of the state), also in the backward, where both have to agree."""
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=640, nheads=4, ngroups=1, d_state=64, chunk=l)
+    inp = pkg.make_inputs(cfg, seed=3)
+    inp["A_head"] = inp["A_head"] * 20
+    dfinal = torch.randn(1, 4, 64, 64, generator=torch.Generator().manual_seed(5))
+    got, want = mamba2_gpu(pkg, inp, l, None, dfinal), oracle.mamba2_fwd_bwd(inp, l, torch.float64, None, dfinal)
+    # 64 terms of a position's own sum, each right to 2^-24 of a sum below 20 (beyond that nothing is left): 1e-6
+    assert rel_err(got["final_state"], want["final_state"]) < 1e-6
+    assert rel_err(got["ddt"], want["ddt"]) < 1e-5
+
+
 @pytest.mark.parametrize("low", [-1e4, -1e30, -3.38e38])
 @pytest.mark.parametrize("cached", [False, True])
 def test_partial_tiles_resets_at_chunk_ends(pkg, cabi, oracle, low, cached):
