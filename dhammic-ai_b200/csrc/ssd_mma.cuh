@@ -374,9 +374,9 @@ __global__ void __launch_bounds__(kStateThreads, 3) state_kernel(Params P) {
 #pragma unroll 4
         for (int k = 0; k < piece; ++k) {
             const float4* f = reinterpret_cast<const float4*>(P.part) + (slot + k) * 512 + threadIdx.x;
-            const float total = P.part_logdecay[slot + k], decay = exp_(total);
-            // (an infinite state lasts where only the decay over a whole piece is too small for a number)
-            auto step = [&](float h, float v) { return fmaf(isinf(h) && !isinf(total) ? 1.f : decay, h, v); };
+            const float decay = exp_(P.part_logdecay[slot + k]);
+            // (an infinite state lasts, also where the decay over a whole piece is too small for a number)
+            auto step = [&](float h, float v) { return fmaf(isinf(h) ? 1.f : decay, h, v); };
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 v = f[q * 128];
