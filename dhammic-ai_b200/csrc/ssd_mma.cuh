@@ -15,15 +15,15 @@
 //
 //   state_kernel   one block per (batch, head, 32 columns of the state) walks the tiles with the state in registers and stores the state
 //                  entering every tile, already cut into its three pieces, and the within-tile sums of the log-decay; a second
-//                  set of blocks walks backwards with the state gradient.  One launch instead of a product per chunk and a
+//                  set of blocks walks backwards with the state gradient.  One launch, or two, instead of a product per chunk and a
 //                  pass over all of them.
 //   scan_kernel    y of one tile and the heads of a group (or a part of them)
 //   bwd_kernel     the row pass (dC, row sums) and the column pass (dx, dB, column sums) of one tile, as in chunk_bwd_kernel
 //   decay_kernel   the decay gradient of a (head, batch), and dB and dC of a group whose heads several blocks share
 //
 // Forward + backward of (4, 1984, 20 heads, 64), d_state 64, chunk 64: 990 us of kernels in eleven launches with fp32 multiply-adds
-// from shared memory, 298 us in seven now (states 130, backward 109, scan 43, decay 11); d dt is 3.8e-7 off the exact one (5.8e-7),
-// dA_head 2.7e-6 (6.4e-6), the final state 2.6e-7 (2.7e-7).
+// from shared memory, 303 us in seven now (states 131, backward 113, scan 42, decay 12); d dt is 4.0e-7 off the exact one (5.8e-7),
+// dA_head 2.9e-6 (4.2e-6), the final state 1.1e-7 (2.8e-7).  At d_state 128 503 us a call; the backward has 255 registers there and spills.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -271,7 +271,7 @@ __device__ __forceinline__ void tile_sums_behind(float& c0, float& c1) {
 // 31 steps of (4, 1984, 20 heads), d_state 64: 75 us with 32 x 16 of the state per warp (the cut operand was then read back
 // by four warps) and 4-byte stores of the fragments (20 us of them).
 //
-// Where few blocks would walk far (pieces_of), the walk is cut into pieces that run side by side: a first launch makes each piece's own
+// Where few blocks would walk far (piece_tiles), the walk is cut into pieces that run side by side: a first launch makes each piece's own
 // sum, without a state before it, and in the second a block folds the sums of the pieces before its own into the state it starts from.
 // ------------------------------------------------------------------------------------------
 constexpr int kStateThreads = 160, kStateCols = 32;

@@ -47,7 +47,7 @@ inline bool supported(int dtype, int p, int n) {
 // rounded to bf16 here and are fp32 in the kernels of ssd_mma.cuh and ssd_simt.cuh.  Calls that fill whole tiles take that rounding;
 // for others it is the caller's choice (SSD_B200_PATH_TC): the final state of 320 positions in chunks of 80 is 2.4e-3 off
 // the exact one on these kernels, 2.5e-7 in fp32 (and forward + backward of (4, 1984, 20 heads, 64), d_state 64, chunk 64
-// take 168 us here, 311 us there).
+// take 168 us here, 303 us there).
 inline bool whole_tiles(int T, int p, int n, int l) { return p == HP && n == DN && T % LT == 0 && (l % LT == 0 || LT % l == 0); }
 inline int tiles_of(int T) { return (T + LT - 1) / LT; }
 

@@ -45,8 +45,8 @@ _SAVE_STATES = os.environ.get("SSD_B200_SAVE_STATES", "1") == "1"
 def set_save_states(flag: bool) -> None:
     """Keep the recurrent states of the forward for the backward (default on) instead of recomputing them in the backward,
     which is what the reference's input-only checkpointing corresponds to (src/kernels/ssd_scan.py:458).  On the tensor-core
-    kernels that is one bf16 state per 128 positions (b*T*h*64 elements, the size of x), on the fp32 kernels one fp32 state
-    per chunk, and there only where it takes no more room than the chunk's x."""
+    kernels that is one bf16 state per 128 positions (b*T*h*64 elements, the size of x), on the fp32 multiply-adds one fp32 state
+    per chunk, and there only where it takes no more room than the chunk's x; the kernels for partial tiles keep none."""
     global _SAVE_STATES
     _SAVE_STATES = bool(flag)
 
@@ -69,10 +69,11 @@ def set_eager_cache(flag: bool) -> None:
 
 
 def set_kernel_path(path: str) -> None:
-    """'auto' (default), 'simt' (fp32 SIMT kernels) or 'tc' (tcgen05 kernels; raises if unsupported).  'auto' takes the tcgen05
-    kernels for bf16 calls that fill their tiles (headdim 64, d_state 128, whole tiles of 128 positions).  'tc' takes them for
-    others too (headdim above 32 and up to 64, d_state above 32 and up to 128, multiples of 8; any length and chunk), which is
-    faster, with the operands of the products rounded to bf16 where the fp32 kernels round nothing."""
+    """'auto' (default), 'simt' (fp32 multiply-adds) or 'tc' (tcgen05 kernels; raises if unsupported).  'auto' takes the tcgen05
+    kernels for bf16 calls that fill their tiles (headdim 64, d_state 128, whole tiles of 128 positions), runs other bf16 calls
+    (headdim above 32 and up to 64, d_state above 32 and up to 128, multiples of 8; any length and chunk) in fp32 arithmetic on
+    tensor-core kernels whose operands are cut into bf16 pieces, and the rest on fp32 multiply-adds.  'tc' takes the tcgen05 kernels
+    for those others too, which is faster, with the operands of the products rounded to bf16."""
     global _FORCE_PATH
     _FORCE_PATH = {"auto": _cabi.PATH_AUTO, "simt": _cabi.PATH_SIMT, "tc": _cabi.PATH_TC}[path]
 
@@ -268,7 +269,8 @@ def ssd_mamba2_gated(x: Tensor, dt: Tensor, A_head: Tensor, B: Tensor, C: Tensor
 
 
 def resolved_path_name(cfg) -> str:
-    """'simt' or 'tc': the kernels the library picks for a workload configuration under the current setting."""
+    """'tc' (the tcgen05 kernels) or 'simt' (everything in fp32 arithmetic, on multiply-adds or in bf16 pieces): what the library
+    picks for a workload configuration under the current setting."""
     lib = _cabi.load()
     shape = _cabi.Shape(_cabi.ABI_VERSION, _cabi.BF16 if cfg.dtype == "bf16" else _cabi.F32, _cabi.F32, _FORCE_PATH,
                         cfg.batch, cfg.seqlen, cfg.nheads, cfg.headdim, cfg.d_state, cfg.ngroups, cfg.chunk)
