@@ -9,14 +9,26 @@ namespace cum {
 constexpr int LT = 128;  // tile length
 
 // The decay mask of a 32-column block is the product of a per-row and a per-column factor taken relative to the
-// block's last column.  Below the diagonal both are <= 1.  Inside the diagonal block the row factor is
+// block's last column.  Below the diagonal both are <= 1.  Inside the diagonal block the row factor would be
 // 2^(decay from the row to the block end) >= 1 and the column factor its inverse scale; beyond this many log2
-// units across a block one of them would leave the fp32 range.  tile_cumsum_kernel raises a flag when any block
-// of the call exceeds it, and the kernels that build the mask carry two bodies: the factorised one, and one that
-// evaluates diagonal blocks entry by entry (one exp2 per entry); the flag selects the body on the device.
+// units across a block one of them would leave the fp32 range.  The forward evaluates diagonal blocks entry by entry (one exp2 per
+// entry); the backward, which is a seventh slower that way, has two instantiations, and the flags of the kernels below, one word per block,
+// select one on the device.
 constexpr float kMaskSafeLog2 = 100.f;
 constexpr int kFusedChunkMax = 1024;  // see cumsum_tile_fused_kernel
 
+// The block's word of the flags (null: not wanted), from the threads' own; every thread of the block calls this.
+__device__ __forceinline__ void raise_flag(int* extreme, int beyond) {
+    if (!extreme) return;
+    const int any = __syncthreads_or(beyond);
+    if (threadIdx.x == 0) extreme[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = any;
+}
+
+// The first block of a pass clears the status word (a memset of its own is a gap of 1.2 us and more on the stream, and what follows one is not
+// launched early).  What another block may write there comes at the earliest when a bounded wait of it runs out, a tenth of a second later.
+__device__ __forceinline__ void clear_status(int* status) {
+    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) *status = 0;
+}
 
 // ------------------------------------------------------------------------------------------
 // Per-position arrays of the tile kernels from a given a_cumsum: the tile-cumulative log2 decay, dt and the skip coefficient in
@@ -28,8 +40,10 @@ constexpr int kFusedChunkMax = 1024;  // see cumsum_tile_fused_kernel
 __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restrict__ cum, const float* __restrict__ dt,
                                                           float* __restrict__ tcum, float* __restrict__ dtT,
                                                           const float* __restrict__ skip, float* __restrict__ skipT,
-                                                          int* __restrict__ extreme, int T, int Tp, int h, int l) {
+                                                          int* __restrict__ extreme, int* __restrict__ status, int T, int Tp, int h, int l) {
     dep_wait();
+    clear_status(status);
+    int beyond = 0;
     __shared__ float sdt[LT][33];
     __shared__ float ssk[LT][33];
     const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
@@ -80,11 +94,12 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
             tcum[o + tt] = w;
             // decay across this 32-position block (lane 0 to lane 31)
             const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);
-            if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
+            if (!(span <= kMaskSafeLog2)) beyond = 1;
             if (dtT) dtT[o + tt] = sdt[tt][hl];
             if (skipT) skipT[o + tt] = ssk[tt][hl];
         }
     }
+    raise_flag(extreme, beyond);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -102,9 +117,11 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
                                                                 const float* __restrict__ dt, const float* __restrict__ A_head,
                                                                 float* __restrict__ cum, float* __restrict__ tcum,
                                                                 float* __restrict__ dtT, const float* __restrict__ skip,
-                                                                float* __restrict__ skipT, int* __restrict__ extreme, int T, int Tp,
-                                                                int h, int l) {
+                                                                float* __restrict__ skipT, int* __restrict__ extreme,
+                                                                int* __restrict__ status, int T, int Tp, int h, int l) {
     dep_wait();
+    clear_status(status);
+    int beyond = 0;
     __shared__ float sa[LT][33];
     __shared__ float sdt[LT][33];
     __shared__ float sbef[8][33];
@@ -187,7 +204,7 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
             const float w = v[s4] * 1.4426950408889634f;
             tcum[o + tt] = w;
             const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);
-            if (lane == 0 && !(span <= kMaskSafeLog2)) atomicOr(extreme, 1);
+            if (!(span <= kMaskSafeLog2)) beyond = 1;
             if (dtT) dtT[o + tt] = sdt[tt][hl];
         }
     }
@@ -206,6 +223,7 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
             for (int s4 = 0; s4 < LT / 32; ++s4) skipT[o + s4 * 32 + lane] = sa[s4 * 32 + lane][hl];
         }
     }
+    raise_flag(extreme, beyond);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -327,6 +327,13 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// 2^x in one instruction; what lies below 2^-126 comes out as zero.
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Packed fp32 pairs (sm_100): one instruction, two lanes.
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     unsigned long long d;

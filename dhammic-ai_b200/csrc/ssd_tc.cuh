@@ -242,9 +242,9 @@ struct WalkParams {
     CUtensorMap mY;   // y store (mode 0)
     CUtensorMap mS;   // state store: 2D [b*nt*h*128][64]
     int save_states;  // store the state entering every tile of the walk through mS
-    const int* extreme;  // see kMaskSafeLog2 (forward only)
     float* ysq;          // (b, T/128, h, 2, 128) per half row sum_p y^2 (forward only), or null
     int* status;
+    int zero_status;     // this kernel is the pass's first: it clears the status word
     int Tp, h, hpg, nt;  // Tp = nt * 128: stride of the per-position arrays
     int p, n;            // headdim and d_state of the tensors (at most 64 and 128)
     // Pieces of the sequence (blockIdx.z; see Pieces): tiles of a piece, and what the parts of each piece but the last

@@ -51,7 +51,8 @@ struct BwdParams {
     float* ddtx;                   // (b,h,T) sum_p dX * x
     float* dyx;                    // (b,h,T) sum_p dy * x
     float* gS;                     // (b,h,nt,8): the terms that act through S = cum[127] of the tile
-    const int* extreme;            // nonzero: the decay across some 32-position block is beyond the factorised mask
+    const int* extreme;            // `flags` words, any nonzero: the decay across some 32-position block is beyond the factorised mask
+    int flags;
     int* status;
     int Tp, h, hpg, nt, b;         // Tp = nt * 128: stride of the per-position arrays
     int n;                         // d_state (columns 64 .. of B, C, dB, dC exist only beyond 64)
@@ -67,13 +68,15 @@ constexpr int kBwdThreads = 640;  // 16 row warps + the control warp's warpgroup
 constexpr int kBwdRegsLaunch = 96, kBwdRegsRow = 104, kBwdRegsCtl = 64;
 static_assert(512 * kBwdRegsRow + 128 * kBwdRegsCtl <= kBwdThreads * kBwdRegsLaunch, "register trade exceeds the CTA's pool");
 
-// Two instantiations (EXACT: diagonal mask blocks entry by entry, see kMaskSafeLog2); both are launched and the
-// extreme-decay flag decides on the device which of the two does the work (kept as separate kernels: as an
-// out-of-line body this kernel loses registers to the call and spills).
+// Two instantiations (EXACT: diagonal mask blocks entry by entry, see kMaskSafeLog2; 1040 -> 1190 us at (16, 4096, 64 heads)); both are
+// launched and the extreme-decay flags decide on the device which of the two does the work.  (As two bodies of one kernel, chosen by a
+// branch at its top, they spill and the code misses the instruction cache: 1066 us, and 67 -> 75 for one of 8 items per SM.)
 template <bool EXACT>
 __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constant__ BwdParams P) {
     dep_wait();
-    if ((P.extreme[0] != 0) != EXACT) return;
+    int beyond = 0;
+    for (int i = threadIdx.x; i < P.flags; i += kBwdThreads) beyond |= P.extreme[i];
+    if ((__syncthreads_or(beyond) != 0) != EXACT) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* sC = sm;                  // 2 panels [pos][n]

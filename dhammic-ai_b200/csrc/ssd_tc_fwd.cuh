@@ -32,9 +32,10 @@
 // The per-half-row sums of y^2 keep their (b, T/128, h, 2, 128) layout: the odd quarter of each half leaves its partial
 // in shared memory, the even quarter adds its own and writes the sum after the block barrier at the top of the next tile.
 //
-// Two instantiations (EXACT: diagonal mask blocks entry by entry, see kMaskSafeLog2); both are launched and the flag
-// raised by the cumulative-sum kernel decides on the device which of the two does the work.  (As one kernel with two
-// out-of-line bodies the walk was a quarter slower: the call boundary costs it registers.)
+// The diagonal block of the mask is evaluated entry by entry (one exponential each, by one warp in ten), which holds for any log-decay; below it
+// the mask is the product of a row and a column factor, both at most 1.  (A second instantiation with factors in the diagonal block as well, and a
+// flag that chose between the two on the device, was no faster, 515 against 516 us at (16, 4096, 64 heads), and the idle one of the
+// two took 2.3 to 7 us a call.)
 #pragma once
 
 namespace ssd {
@@ -58,10 +59,9 @@ __device__ __forceinline__ void store_quarter_row(uint8_t* panel, int row, int c
     }
 }
 
-template <bool EXACT>
 __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constant__ WalkParams P) {
     dep_wait();
-    if ((P.extreme[0] != 0) != EXACT) return;
+    if (P.zero_status) clear_status(P.status);
     using Cfg = WalkCfg<0>;
     constexpr int NST = Cfg::NST;
     extern __shared__ uint8_t smem_raw[];
@@ -72,7 +72,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     uint8_t* sY = sH + PANEL;                              // y staging
     float* scum2 = reinterpret_cast<float*>(sY + PANEL);   // [2][128]
     float* sf = scum2 + 2 * LT;                            // [2][128] column factors dt_j 2^(cend - c_j)
-    float* sdtc = sf + 2 * LT;                             // [2][128] dt_j (EXACT instantiation only)
+    float* sdtc = sf + 2 * LT;                             // [2][128] dt_j
     float* sysq = sdtc + 2 * LT;                           // [2][2][128] partial sums of y^2 of the odd quarters
     __shared__ uint64_t bar_ld[2], bar_s, bar_u, bar_g, bar_mh, bar_m2, bar_h, bar_sr;
     __shared__ uint32_t tmem_slot;
@@ -251,7 +251,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             if (q == 0) {
                 scum2[buf * LT + row] = c_i;
                 sf[buf * LT + row] = dtv * exp2f(cend - c_i);
-                if (EXACT) sdtc[buf * LT + row] = dtv;
+                sdtc[buf * LT + row] = dtv;
             }
             mbar_wait(&bar_ld[s], (it / NST) & 1, &failed);
             named_barrier(1, 512);
@@ -293,35 +293,28 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 } else {
                     uint32_t r[32];
                     tmem_ld32(tm + (it & 1) * 128 + lanes + c0, r);
-                    // row factor relative to the block's last column: <= 1 below the diagonal block
-                    const float rf = exp2f(c_i - scum2[buf * LT + c0 + 31]);
-                    const float2* F2 = reinterpret_cast<const float2*>(sf + buf * LT + c0);
                     tmem_ld_wait();
                     const float2* S2 = reinterpret_cast<const float2*>(r);
-                    const float2 rf2 = make_float2(rf, rf);
-                    if (EXACT && diag) {
-                        // inside the diagonal block the two factors are 2^(+-decay across the block); this instantiation
-                        // runs when that leaves the fp32 range somewhere and evaluates the block entry by entry
+                    if (diag) {
                         const float2* C2 = reinterpret_cast<const float2*>(scum2 + buf * LT + c0);
                         const float2* T2 = reinterpret_cast<const float2*>(sdtc + buf * LT + c0);
 #pragma unroll
                         for (int q2 = 0; q2 < 16; ++q2) {
                             const float2 cj = C2[q2], tj = T2[q2];
                             float2 l;
-                            l.x = (c0 + 2 * q2 > row) ? 0.f : tj.x * exp2f(c_i - cj.x);
-                            l.y = (c0 + 2 * q2 + 1 > row) ? 0.f : tj.y * exp2f(c_i - cj.y);
+                            l.x = (c0 + 2 * q2 > row) ? 0.f : tj.x * ex2(c_i - cj.x);
+                            l.y = (c0 + 2 * q2 + 1 > row) ? 0.f : tj.y * ex2(c_i - cj.y);
                             const float2 v = mul2(S2[q2], l);
                             packed[q2] = pack_bf16(v.x, v.y);
                         }
                     } else {
+                        // row factor relative to the block's last column
+                        const float rf = exp2f(c_i - scum2[buf * LT + c0 + 31]);
+                        const float2* F2 = reinterpret_cast<const float2*>(sf + buf * LT + c0);
+                        const float2 rf2 = make_float2(rf, rf);
 #pragma unroll
                         for (int q2 = 0; q2 < 16; ++q2) {  // fp32 pairs: one instruction, two columns
-                            float2 l = mul2(rf2, F2[q2]);
-                            if (diag) {
-                                if (c0 + 2 * q2 > row) l.x = 0.f;
-                                if (c0 + 2 * q2 + 1 > row) l.y = 0.f;
-                            }
-                            const float2 v = mul2(S2[q2], l);
+                            const float2 v = mul2(S2[q2], mul2(rf2, F2[q2]));
                             packed[q2] = pack_bf16(v.x, v.y);
                         }
                     }

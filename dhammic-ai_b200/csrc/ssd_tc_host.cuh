@@ -25,32 +25,37 @@ inline EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2D bf16 tensor [rows][cols] (the saved states), box 64 columns x 128 rows, 128-byte swizzle.
-inline bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols) {
+// A bf16 tensor map with boxes of 128-byte rows, 128-byte swizzle.  The encoder belongs to the driver and wants a current context, which a
+// thread that has not called the runtime yet does not have (autograd's, where the map is the first thing that a backward asks for).
+inline bool encode_map(CUtensorMap* m, const void* base, cuuint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * 2};
-    cuuint32_t box[2] = {64, 128};
-    cuuint32_t es[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    auto encode = [&] {
+        return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaFree(nullptr) == cudaSuccess) r = encode();  // (the runtime makes the device's context current)
+    return r == CUDA_SUCCESS;
+}
+
+// 2D bf16 tensor [rows][cols] (the saved states), box 64 columns x 128 rows, 128-byte swizzle.
+inline bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols) {
+    const cuuint64_t dims[2] = {cols, rows};
+    const cuuint64_t strides[1] = {cols * 2};
+    const cuuint32_t box[2] = {64, 128};
+    return encode_map(m, base, 2, dims, strides, box);
 }
 
 // A (b, T, heads, inner) bf16 tensor as the tile kernels see it: boxes of 64 columns of one head x 128 positions of one
 // sequence.  Keeping the dimensions apart is what makes a box that reaches behind the end of a sequence, or behind a head's
 // last column, read zeros instead of the neighbour's values.
 inline bool make_map4(CUtensorMap* m, const void* base, const Dims& d, int heads, int inner) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return false;
-    cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)heads, (cuuint64_t)d.T, (cuuint64_t)d.b};
-    cuuint64_t strides[3] = {(cuuint64_t)inner * 2, (cuuint64_t)heads * inner * 2, (cuuint64_t)d.T * heads * inner * 2};
-    cuuint32_t box[4] = {64, 1, 128, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)heads, (cuuint64_t)d.T, (cuuint64_t)d.b};
+    const cuuint64_t strides[3] = {(cuuint64_t)inner * 2, (cuuint64_t)heads * inner * 2, (cuuint64_t)d.T * heads * inner * 2};
+    const cuuint32_t box[4] = {64, 1, 128, 1};
+    return encode_map(m, base, 4, dims, strides, box);
 }
 
 struct Ws {
@@ -86,6 +91,9 @@ inline Pieces pieces_of(const Dims& d, bool reverse) {
     }
     return best;
 }
+
+// Words of the extreme-decay flags: one per block of the cumulative sums.
+inline size_t flags_of(const Dims& d) { return (size_t)d.b * ((d.h + 31) / 32) * tiles_of(d.T); }
 
 inline Ws ws_layout(const Dims& d, int pass) {
     Ws w{};
@@ -132,10 +140,10 @@ inline Ws ws_layout(const Dims& d, int pass) {
 inline size_t workspace_bytes(const Dims& d, int pass) { return ws_layout(d, pass).total; }
 // The `states` buffer a forward call may fill for the backward call of the same inputs: the bf16 state entering
 // every tile, followed by the three (b,h,Tp) fp32 arrays the tile kernels read (tile-cumulative log2 decay, dt and
-// the per-position skip coefficient in (b,h,T) order) and the extreme-decay flag of tile_cumsum_kernel, so that the backward neither walks the states
+// the per-position skip coefficient in (b,h,T) order) and the extreme-decay flags, so that the backward neither walks the states
 // nor rebuilds those arrays.
 inline size_t tile_states_bytes(const Dims& d) { return (size_t)d.b * tiles_of(d.T) * d.h * DN * HP * 2; }
-inline size_t states_bytes(const Dims& d) { return tile_states_bytes(d) + 3 * ((size_t)d.b * d.h * tiles_of(d.T) * LT * 4) + 256; }
+inline size_t states_bytes(const Dims& d) { return tile_states_bytes(d) + 3 * ((size_t)d.b * d.h * tiles_of(d.T) * LT * 4) + flags_of(d) * 4; }
 
 #define SSD_TC_FAIL(code, ...)              \
     do {                                    \
@@ -165,8 +173,7 @@ inline int set_walk_attrs(char* err, size_t errn) {
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return 0;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(fwd_walk_kernel<false>, attr, (int)kFwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fwd_walk_kernel<true>, attr, (int)kFwdSmem);
+    cudaError_t e = cudaFuncSetAttribute(fwd_walk_kernel, attr, (int)kFwdSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(states_walk_kernel, attr, (int)WalkCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<1>, attr, (int)RevCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<2>, attr, (int)RevCfg<2>::SMEM);
@@ -182,23 +189,23 @@ inline int set_walk_attrs(char* err, size_t errn) {
 }
 
 inline int launch_tile_cumsum(bool after, const Dims& d, const float* cum, const float* dt, float* tcum, float* dtT, const float* skip,
-                              float* skipT, int* extreme, cudaStream_t st, char* err, size_t errn) {
+                              float* skipT, int* extreme, int* status, cudaStream_t st, char* err, size_t errn) {
     const int nt = tiles_of(d.T);
     dim3 g(nt, (d.h + 31) / 32, d.b);
-    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, tile_cumsum_kernel, g, 256, 0, st, cum, dt, tcum, dtT, skip, skipT, extreme, d.T, nt * LT, d.h, d.l));
+    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, tile_cumsum_kernel, g, 256, 0, st, cum, dt, tcum, dtT, skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l));
     SSD_TC_CHECK("tile_cumsum");
     return 0;
 }
 
 // The same from the log-decays (`args` of a forward or a backward), and a_cumsum unless `cum` is null.
 template <class Args>
-inline int launch_cumsum_tile_fused(const Args* a, const Dims& d, float* cum, float* tcum, float* dtT, float* skipT, int* extreme, cudaStream_t st,
+inline int launch_cumsum_tile_fused(const Args* a, const Dims& d, float* cum, float* tcum, float* dtT, float* skipT, int* extreme, int* status, cudaStream_t st,
                                     char* err, size_t errn) {
     const int nt = tiles_of(d.T);
     const dim3 g(nt, (d.h + 31) / 32, d.b);
     const bool cut = d.l % LT != 0;  // a chunk ends inside a tile
     SSD_LAUNCH(prof::K_CUMSUM, st, (launch_dep(false, (cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>), g, 256, 0, st, 
-        a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, cum, tcum, dtT, a->skip, skipT, extreme, d.T, nt * LT, d.h, d.l)));
+        a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, cum, tcum, dtT, a->skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l)));
     SSD_TC_CHECK("cumsum_tile_fused");
     return 0;
 }
@@ -212,13 +219,14 @@ inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace
     if (pc.np == 1 || bytes < w.total) return 0;
     SummaryParams S{};
     S.mU = P.mU; S.mV = P.mV; S.tcum = P.tcum; S.dtT = P.dtT; S.out = (float*)((char*)workspace + w.piece_sum);
-    S.logdecay = (float*)((char*)workspace + w.piece_decay); S.status = P.status; S.Tp = P.Tp; S.h = P.h; S.hpg = P.hpg; S.nt = P.nt;
+    S.logdecay = (float*)((char*)workspace + w.piece_decay); S.status = P.status; S.zero_status = P.zero_status; S.Tp = P.Tp; S.h = P.h; S.hpg = P.hpg; S.nt = P.nt;
     S.p = P.p; S.n = P.n; S.pt = pc.pt; S.ps = pc.ps; S.parts = pc.parts; S.z0 = REV ? 1 : 0;
     SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(*after, summary_kernel<REV, 1>, dim3(d.h, d.b, (pc.np - 1) * pc.parts), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
     SSD_TC_CHECK("tc_summary_pieces");
     P.pt = pc.pt; P.parts = pc.parts; P.piece_sum = S.out; P.piece_decay = S.logdecay;
     *pieces = pc.np;
     *after = true;
+    P.zero_status = 0;
     return 0;
 }
 
@@ -236,7 +244,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     float* tcum = (float*)(ws + w.tcum);
     float* dtT = a->dt ? (float*)(ws + w.dtT) : nullptr;
     float* skipT = a->skip ? (float*)(ws + w.skipT) : nullptr;
-    int* extreme = status + 1;  // raised by tile_cumsum_kernel (see kMaskSafeLog2)
+    int* extreme = nullptr;  // flags for the backward (see kMaskSafeLog2)
     const bool aux_valid = (a->flags & SSD_B200_FWD_AUX_VALID) != 0;
     if (aux_valid && !a->states) SSD_TC_FAIL(SSD_B200_EINVAL, "SSD_B200_FWD_AUX_VALID needs the `states` buffer that holds the arrays");
     if (a->states) {  // the per-position arrays live behind the tile states, kept for later calls on the same inputs
@@ -244,12 +252,10 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
         if (a->dt) dtT = tcum + bht;
         if (a->skip) skipT = tcum + 2 * bht;
         extreme = (int*)(tcum + 3 * bht);
-        if (!aux_valid && cudaMemsetAsync(extreme, 0, 4, st) != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "memset failed");
     }
-    if (cudaMemsetAsync(status, 0, 8, st) != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "memset failed");
     if (!a->cumsum_is_input && !aux_valid && d.l <= kFusedChunkMax) {
         // the within-chunk cumulative sums, the tile-cumulative log2 copies, the transposes and the flag in one kernel
-        if (int rc = launch_cumsum_tile_fused(a, d, a->a_cumsum, tcum, dtT, skipT, extreme, st, err, errn)) return rc;
+        if (int rc = launch_cumsum_tile_fused(a, d, a->a_cumsum, tcum, dtT, skipT, extreme, status, st, err, errn)) return rc;
     } else {
         if (!a->cumsum_is_input) {
             const size_t sm = (size_t)d.l * (d.h + 1) * 4;
@@ -263,13 +269,13 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
             SSD_TC_CHECK("chunk_cumsum");
         }
         if (!aux_valid)
-            if (int rc = launch_tile_cumsum(!a->cumsum_is_input, d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn)) return rc;
+            if (int rc = launch_tile_cumsum(!a->cumsum_is_input, d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, status, st, err, errn)) return rc;
     }
     if (int rc = set_walk_attrs(err, errn)) return rc;
-    bool after = !aux_valid;  // the cumulative sums are on the stream, or the memset of the status word
+    bool after = !aux_valid;  // the cumulative sums are on the stream (and have cleared the status word)
     WalkParams P{};
+    P.zero_status = aux_valid;
     P.skipT = skipT;
-    P.extreme = extreme;
     P.ysq = a->ysq;
     bool ok = make_map4(&P.mU, a->x, d, d.h, d.p) && make_map4(&P.mV, a->B, d, d.g, d.n) && make_map4(&P.mC, a->C, d, d.g, d.n) &&
               make_map4(&P.mY, states_only ? a->x : (const void*)a->y, d, d.h, d.p);
@@ -286,7 +292,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     if (states_only) {  // what this piece of the sequence adds to the state after it (plus the decayed seed)
         SummaryParams S{};
         S.mU = P.mU; S.mV = P.mV; S.tcum = tcum; S.dtT = dtT; S.seed = a->init; S.out = a->final_state;
-        S.logdecay = a->logdecay_total; S.status = status; S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1;
+        S.logdecay = a->logdecay_total; S.status = status; S.zero_status = aux_valid; S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1;
         S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)  // two heads of a group per CTA share the group's panels
             SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(after, summary_kernel<false, 2>, dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
@@ -297,8 +303,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     }
     int pieces;
     if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
-    SSD_LAUNCH(prof::K_TC_FWD, st, (launch_dep(after, fwd_walk_kernel<false>, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P)));
-    SSD_LAUNCH(prof::K_TC_FWD_ALT, st, (launch_dep(true, fwd_walk_kernel<true>, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P)));
+    SSD_LAUNCH(prof::K_TC_FWD, st, launch_dep(after, fwd_walk_kernel, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P));
     SSD_TC_CHECK("tc_fwd_walk");
     if (a->logdecay_total) {
         SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(true, logdecay_total_kernel, (d.b * d.h + 127) / 128, 128, 0, st, a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));
@@ -324,8 +329,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
     void* Qst = ws + w.Qst;
     float* fin = (float*)(ws + w.final_state);
     float* dinit = a->dinit ? a->dinit : (float*)(ws + w.dinit);
-    if (cudaMemsetAsync(status, 0, 8, st) != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "memset failed");
-    int* extreme = status + 1;
+    int* extreme = (int*)(ws + w.dAh_part);  // (written again behind the kernels that read the flags)
     float* skipT = a->skip ? (float*)(ws + w.skipT) : nullptr;
     if (a->states) {  // the forward left the arrays and the flag behind the tile states
         tcum = (float*)((uintptr_t)a->states + tile_states_bytes(d));
@@ -334,18 +338,18 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         extreme = (int*)(tcum + 3 * bht);
     } else {  // as the forward made them: from the log-decays, or from the sums it was given
         const bool decays = !a->cumsum_is_input && d.l <= kFusedChunkMax && (a->a || (a->dt && a->A_head));
-        if (int rc = decays ? launch_cumsum_tile_fused(a, d, nullptr, tcum, dtT, skipT, extreme, st, err, errn)
-                            : launch_tile_cumsum(false, d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, st, err, errn))
+        if (int rc = decays ? launch_cumsum_tile_fused(a, d, nullptr, tcum, dtT, skipT, extreme, status, st, err, errn)
+                            : launch_tile_cumsum(false, d, a->a_cumsum, a->dt, tcum, dtT, a->skip, skipT, extreme, status, st, err, errn))
             return rc;
     }
     if (int rc = set_walk_attrs(err, errn)) return rc;
-    bool after = !a->states;  // the cumulative sums are on the stream, or the memset of the status word
+    bool after = !a->states;  // the cumulative sums are on the stream (and have cleared the status word)
     const uint64_t srows = (uint64_t)d.b * nt * d.h * DN;
     if (a->flags & SSD_B200_BWD_DINIT_ONLY) {  // d(initial state) of this piece for the given (or a zero) dfinal
         SummaryParams S{};
         if (!(make_map4(&S.mU, a->dy, d, d.h, d.p) && make_map4(&S.mV, a->C, d, d.g, d.n)))
             SSD_TC_FAIL(SSD_B200_ECUDA, "tensor map encoding failed");
-        S.tcum = tcum; S.dtT = nullptr; S.seed = a->dfinal; S.out = a->dinit; S.logdecay = nullptr; S.status = status;
+        S.tcum = tcum; S.dtT = nullptr; S.seed = a->dfinal; S.out = a->dinit; S.logdecay = nullptr; S.status = status; S.zero_status = !after;
         S.Tp = Tp; S.h = d.h; S.hpg = d.hpg; S.nt = S.pt = S.ps = nt; S.parts = 1; S.p = d.p; S.n = d.n;
         if (d.hpg % 2 == 0)
             SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(after, summary_kernel<true, 2>, dim3(d.h / 2, d.b), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
@@ -373,7 +377,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
     {   // reverse walk: gradient of the state leaving every tile, and d(initial state)
         WalkParams P{};
         P.mU = mdY; P.mV = mC; P.mC = mC; P.mY = mdX; P.mS = mQ; P.save_states = 1;
-        P.tcum = tcum; P.dtT = nullptr; P.D = nullptr; P.seed = a->dfinal; P.out_state = dinit; P.status = status;
+        P.tcum = tcum; P.dtT = nullptr; P.D = nullptr; P.seed = a->dfinal; P.out_state = dinit; P.status = status; P.zero_status = !after;
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         int pieces;
         if (int rc = split_walk<true>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
@@ -393,6 +397,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.hpg = d.hpg; P.nt = nt; P.b = d.b; P.gS = (float*)(ws + w.gS);
         P.items = nt * d.g * d.b;
         P.extreme = extreme;
+        P.flags = (int)flags_of(d);
         const dim3 grid(std::min(P.items, sm_count()));
         SSD_LAUNCH(prof::K_TC_BWD, st, launch_dep(true, bwd_tile_kernel<false>, grid, kBwdThreads, kBwdSmem, st, P));
         SSD_LAUNCH(prof::K_TC_BWD_ALT, st, launch_dep(true, bwd_tile_kernel<true>, grid, kBwdThreads, kBwdSmem, st, P));

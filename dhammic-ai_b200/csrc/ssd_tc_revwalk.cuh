@@ -35,6 +35,7 @@ struct RevCfg {
 template <int NH>
 __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const __grid_constant__ WalkParams P) {
     dep_wait();
+    if (P.zero_status) clear_status(P.status);
     using Cfg = RevCfg<NH>;
     // no static shared memory: the dynamic region starts at the CTA's shared-memory base
     extern __shared__ __align__(1024) uint8_t smem_raw[];

@@ -42,6 +42,7 @@ struct SummaryParams {
     float* out;            // (z,b,h,p,n) fp32
     float* logdecay;       // (z,b,h) total log-decay of the part in natural-log units, or null
     int* status;
+    int zero_status;      // see WalkParams
     int Tp, h, hpg, nt;   // Tp = nt * 128: stride of the per-position arrays
     int p, n;
     int pt, ps, parts;    // tiles of a piece and of a part, parts per piece
@@ -51,6 +52,7 @@ struct SummaryParams {
 template <bool REV, int NH>
 __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const __grid_constant__ SummaryParams P) {
     dep_wait();
+    if (P.zero_status) clear_status(P.status);
     using Cfg = SumCfg<NH>;
     constexpr int NS = Cfg::STAGES;
     constexpr int CTLW = 8 * NH;  // control warp

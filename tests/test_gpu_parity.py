@@ -129,6 +129,28 @@ def check_mamba2(pkg, oracle, cfg, tol, init=False, dfinal=False, seed=None):
     return errs
 
 
+@pytest.mark.parametrize("b,T,h,at", [(1, 128, 4, (0, 0, 0)), (2, 384, 40, (1, 2, 39)), (3, 768, 36, (2, 5, 32)), (2, 1152, 66, (0, 8, 65))])
+@pytest.mark.parametrize("kept", [True, False])
+def test_fast_decay_in_one_block_of_the_flags(pkg, cabi, oracle, b, T, h, at, kept):
+    """A log-decay of -6 a position over 40 positions of one (batch, tile, head) only, that of a block of the cumulative sums at the
+    start, the end and inside the grid (heads in blocks of 32): 277 log2 units across a 32-column block, so the factorised mask of
+    the backward would leave the fp32 range there.  States kept by the forward or made again."""
+    bb, tile, head = at
+    cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, ngroups=2, chunk=128)
+    inp = pkg.make_inputs(cfg, seed=17)
+    inp["A_head"][head] = -60.0
+    inp["dt"][:, :, head] = 1e-3
+    inp["dt"][bb, tile * 128 + 50:tile * 128 + 90, head] = 0.1
+    pkg.set_save_states(kept)
+    try:
+        got = mamba2_gpu(pkg, inp, cfg.chunk)
+    finally:
+        pkg.set_save_states(True)
+    want = oracle.mamba2_fwd_bwd(inp, cfg.chunk, torch.float32)
+    bad = {k: rel_err(got[k], want[k].reshape(got[k].shape)) for k in got if not rel_err(got[k], want[k].reshape(got[k].shape)) < TOL_BF16}
+    assert not bad, bad
+
+
 def test_config0_fp32_full_size(pkg, cabi, oracle):
     check_mamba2(pkg, oracle, pkg.CONFIGS[0], TOL_FP32)
 
