@@ -63,32 +63,39 @@ struct Ws {
 };
 
 // The pieces that a walk over one sequence is cut into.  A walk has one CTA per (batch, head), which takes 2.15 us per tile forward
-// and 1.5 us in reverse; with few of them most SMs idle.  Pieces run side by side: every piece but the walk's last is first
-// summarised (0.8 us per tile, no chain, in parts that fill the chip), and a piece's CTA folds the summaries before its own into
-// its seed.  Only while all CTAs fit on the chip at once, and where the tiles taken off the chain outweigh the summary and its
-// launch (12 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.
+// and 1.5 us in reverse (1.75 for two heads of a group in one CTA); with few of them most SMs idle.  Pieces run side by side: every piece but the
+// walk's last is first summarised (0.8 us per tile, 1.2 for two heads of a group, no chain, in parts that fill the chip), and a piece's CTA
+// folds the summaries before its own into its seed.  Only while all CTAs fit on the chip at once, and where the tiles taken off the chain
+// outweigh the summary and its launch (12 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.
 // One prompt of 16,384 positions and 64 heads (128 tiles, two pieces): 282 us in one piece, 213 with one summary, 189 with two parts.
 struct Pieces {
     int pt, np, ps, parts;  // tiles of a piece, pieces, tiles of a summarised part, parts of a piece
+    int heads, sum_heads;   // of a group per CTA of the walk (reverse), of the summary
 };
 constexpr int kPieceSms = 148, kMaxEntries = 16;
 inline Pieces pieces_of(const Dims& d, bool reverse) {
     const int nt = tiles_of(d.T);
     const long long bh = (long long)d.b * d.h;
-    const double tile = reverse ? 1.5 : 2.15;
-    Pieces best{nt, 1, nt, 1};
-    double cost = 0.9 * tile * nt;
-    for (int P = 2; P <= kMaxEntries && P * bh <= kPieceSms && P <= nt; ++P) {
-        const int pt = (nt + P - 1) / P, np = (nt + pt - 1) / pt;
-        const int want = (int)std::max(1LL, std::min({(long long)pt, kPieceSms / (bh * (np - 1)), (long long)kMaxEntries / (np - 1)}));
-        const int ps = (pt + want - 1) / want, parts = (pt + ps - 1) / ps;
-        if (reverse && nt - (np - 1) * pt <= (parts - 1) * ps) continue;  // the short last piece would have an empty part
-        const double c = tile * pt + 0.8 * ps + 12.0 + 0.6 * parts * (np - 1);
-        if (c < cost) {
-            cost = c;
-            best = {pt, np, ps, parts};
-        }
-    }
+    const bool even = d.hpg % 2 == 0;
+    // in one piece: two heads per CTA (shared C panels, one N = 128 product per tile) only where one head per CTA would not fit on the chip at once
+    Pieces best{nt, 1, nt, 1, reverse && even && bh > kPieceSms ? 2 : 1, 1};
+    double cost = 0.9 * (reverse ? 1.5 : 2.15) * nt;
+    if (bh > kPieceSms) return best;
+    for (int heads = 1; heads <= (reverse && even ? 2 : 1); ++heads)
+        for (int P = 2; P <= kMaxEntries && P * bh <= kPieceSms * heads && P <= nt; ++P)
+            for (int sum_heads = 1; sum_heads <= (even ? 2 : 1); ++sum_heads) {
+                const int pt = (nt + P - 1) / P, np = (nt + pt - 1) / pt;
+                const long long ctas = bh / sum_heads * (np - 1);  // of the summary, for one part
+                const int want = (int)std::max(1LL, std::min({(long long)pt, kPieceSms / ctas, (long long)kMaxEntries / (np - 1)}));
+                const int ps = (pt + want - 1) / want, parts = (pt + ps - 1) / ps;
+                if (reverse && nt - (np - 1) * pt <= (parts - 1) * ps) continue;  // the short last piece would have an empty part
+                const double rounds = (double)((ctas * parts + kPieceSms - 1) / kPieceSms);
+                const double c = (!reverse ? 2.15 : heads == 2 ? 1.75 : 1.5) * pt + (sum_heads == 2 ? 1.2 : 0.8) * rounds * ps + 12.0 + 0.6 * parts * (np - 1);
+                if (c < cost) {
+                    cost = c;
+                    best = {pt, np, ps, parts, heads, sum_heads};
+                }
+            }
     return best;
 }
 
@@ -175,8 +182,10 @@ inline int set_walk_attrs(char* err, size_t errn) {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(fwd_walk_kernel, attr, (int)kFwdSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(states_walk_kernel, attr, (int)WalkCfg<1>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<1>, attr, (int)RevCfg<1>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<2>, attr, (int)RevCfg<2>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<1, false>, attr, (int)RevCfg<1>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<1, true>, attr, (int)RevCfg<1>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<2, false>, attr, (int)RevCfg<2>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<2, true>, attr, (int)RevCfg<2>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(summary_kernel<false, 1>, attr, (int)SumCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(summary_kernel<true, 1>, attr, (int)SumCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(summary_kernel<false, 2>, attr, (int)SumCfg<2>::SMEM);
@@ -221,7 +230,11 @@ inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace
     S.mU = P.mU; S.mV = P.mV; S.tcum = P.tcum; S.dtT = P.dtT; S.out = (float*)((char*)workspace + w.piece_sum);
     S.logdecay = (float*)((char*)workspace + w.piece_decay); S.status = P.status; S.zero_status = P.zero_status; S.Tp = P.Tp; S.h = P.h; S.hpg = P.hpg; S.nt = P.nt;
     S.p = P.p; S.n = P.n; S.pt = pc.pt; S.ps = pc.ps; S.parts = pc.parts; S.z0 = REV ? 1 : 0;
-    SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(*after, summary_kernel<REV, 1>, dim3(d.h, d.b, (pc.np - 1) * pc.parts), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
+    const int z = (pc.np - 1) * pc.parts;
+    if (pc.sum_heads == 2)
+        SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(*after, summary_kernel<REV, 2>, dim3(d.h / 2, d.b, z), SumCfg<2>::THREADS, SumCfg<2>::SMEM, st, S)));
+    else
+        SSD_LAUNCH(prof::K_TC_SUMMARY, st, (launch_dep(*after, summary_kernel<REV, 1>, dim3(d.h, d.b, z), SumCfg<1>::THREADS, SumCfg<1>::SMEM, st, S)));
     SSD_TC_CHECK("tc_summary_pieces");
     P.pt = pc.pt; P.parts = pc.parts; P.piece_sum = S.out; P.piece_decay = S.logdecay;
     *pieces = pc.np;
@@ -381,12 +394,11 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         int pieces;
         if (int rc = split_walk<true>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
-        // two heads of a group per CTA: shared C panels, one N = 128 product per tile; but a tile then takes 1.7 us instead of
-        // 1.5, so only where one head per CTA would not fit on the chip at once
-        if (d.hpg % 2 == 0 && pieces == 1 && (long long)d.b * d.h > kPieceSms)
-            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(after, rev_walk_kernel<2>, dim3(d.h / 2, d.b), RevCfg<2>::THREADS, RevCfg<2>::SMEM, st, P));
-        else
-            SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(after, rev_walk_kernel<1>, dim3(d.h, d.b, pieces), RevCfg<1>::THREADS, RevCfg<1>::SMEM, st, P));
+        const Pieces pc = pieces_of(d, true);
+        const bool cut = pieces > 1, two = pc.heads == 2 && pieces == pc.np;  // (in one piece for want of room: one head per CTA)
+        const auto kernel = two ? (cut ? rev_walk_kernel<2, true> : rev_walk_kernel<2, false>) : (cut ? rev_walk_kernel<1, true> : rev_walk_kernel<1, false>);
+        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, launch_dep(after, kernel, dim3(two ? d.h / 2 : d.h, d.b, pieces), two ? RevCfg<2>::THREADS : RevCfg<1>::THREADS,
+                                                        two ? RevCfg<2>::SMEM : RevCfg<1>::SMEM, st, P));
         SSD_TC_CHECK("tc_bwd_dstate");
     }
     {

@@ -1,6 +1,6 @@
 // Reverse tile walk of the backward pass (included by ssd_tc.cuh after ssd_tc_walk.cuh).
 //
-// One CTA walks the 128-position tiles of NH heads of one group (same batch entry; NH = 1: or of a piece of the sequence, where
+// One CTA walks the 128-position tiles of NH heads of one group (same batch entry; or of a piece of the sequence, where
 // a whole one per CTA would leave most of the chip idle) from the last tile to the first, with the gradient of each head's recurrent state Q (128 x 64, fp32) in the registers of that head's eight row
 // warps.  Per tile k and head it
 //   * stores Q as it leaves tile k (bf16, [n][p]) for the per-tile backward kernel,
@@ -32,7 +32,8 @@ struct RevCfg {
     static constexpr int THREADS = 256 * NH + 32;
 };
 
-template <int NH>
+// CUT: in pieces (two heads per CTA have no register to spare for the bounds of a piece: 241 us without them, 245 with, at (16, 4096, 64 heads)).
+template <int NH, bool CUT>
 __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const __grid_constant__ WalkParams P) {
     dep_wait();
     if (P.zero_status) clear_status(P.status);
@@ -57,8 +58,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
     constexpr int CTLW = 8 * NH;  // control warp
     const int hh0 = blockIdx.x * NH, bb = blockIdx.y;
     const int gg = hh0 / P.hpg;
-    // the piece's tiles; with two heads per CTA there is only ever one piece (and no register to spare)
-    const int k0 = NH == 1 ? (int)blockIdx.z * P.pt : 0, nt = NH == 1 ? min(P.pt, P.nt - k0) : P.nt;
+    const int k0 = CUT ? (int)blockIdx.z * P.pt : 0, nt = CUT ? min(P.pt, P.nt - k0) : P.nt;  // the piece's tiles
 
     if (tid == 0) {
         failed = 0;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
         const uint32_t lanes = lane_base(warp);
         uint8_t* sQ = sQ0 + (size_t)hs * PANEL;
         float H[32];  // state gradient row n = row, p in [hf*32, hf*32+32)
-        if (NH == 1) load_piece_row<true>(P, bh, row, hf * 32, H);
+        if (CUT) load_piece_row<true>(P, bh, row, hf * 32, H);
         else load_state_row(P.seed, bh, P.p, P.n, row, hf * 32, H);
         // Store the state gradient leaving tile nt-1-it: staged in the head's sQ panel, written by one TMA store of the
         // head's first thread, which waits until its previous store has read the panel; the first barrier (the head's

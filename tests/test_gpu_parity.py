@@ -562,6 +562,25 @@ def test_unaligned_tensors_through_the_c_abi(pkg, cabi, dtype, n, g, shifted):
         assert [rc == cabi.EINVAL for rc in rcs] == refused
 
 
+@pytest.mark.parametrize("b,T,h,g", [(1, 4096, 64, 2), (1, 4480, 64, 8), (2, 3968, 36, 3), (1, 8192, 148, 74)])
+def test_reverse_walk_in_pieces_of_two_heads(pkg, cabi, b, T, h, g):
+    """Sequences whose reverse walk is cut into pieces with two heads of a group per CTA (whole last pieces and short ones, two heads per group): the same
+    as in one piece, which is what a call with room for no more takes.  States and gradients are bf16 sums of the same terms in another order."""
+    cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, ngroups=g, chunk=128)
+    inp = pkg.make_inputs(cfg, seed=8)
+    def up(v):
+        return (v + 255) // 256 * 256
+    nt, bh = T // 128, b * h
+    bht, state = up(bh * T * 4), up(bh * 64 * 128 * 4)
+    fwd = 256 + 3 * bht
+    bwd = fwd + 2 * up(bh * nt * 64 * 128 * 2) + 2 * state + 3 * bht + up(bh * nt * 32) + 2 * up(bh * nt * 4)
+    rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {cabi.PASS_FWD: fwd, cabi.PASS_BWD: bwd})
+    rc1, got = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
+    assert rc0 == rc1 == [0, 0]
+    for k in want:
+        assert rel_err(got[k], want[k]) < TOL_BF16, k
+
+
 def test_walk_in_one_piece_where_the_workspace_has_no_room(pkg, cabi):
     """With less workspace than several pieces need, but enough for one, the walks run in one; with a byte less they are refused."""
     cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=4096, nheads=6, ngroups=2, chunk=128)

@@ -159,6 +159,28 @@ def test_sequence_parallel_passes_against_oracle(pkg, cabi, oracle):
     assert not bad, errs
 
 
+@pytest.mark.parametrize("dtype,init", [("bf16", torch.bfloat16), ("bf16", torch.float32), ("fp32", None)])
+def test_segmented_call_that_cuts_for_itself(pkg, cabi, dtype, init):
+    """segments = 0 is one call whose walks cut themselves: the results of segments that the caller names; what does not split is still refused."""
+    import importlib
+    D = importlib.import_module("dhammic-ai_b200.distributed")
+    cfg = replace(pkg.CONFIGS[2], dtype=dtype, batch=1, seqlen=8192, nheads=4, ngroups=2, chunk=128)
+    inp = pkg.make_inputs(cfg, seed=13)
+    i0 = None if init is None else (0.3 * torch.randn(1, 1, 4, 64, 128, generator=torch.Generator().manual_seed(3))).to(init)
+    res = []
+    for segments in (0, 4):
+        lv = [inp[k].to("cuda").requires_grad_(True) for k in ("x", "dt", "A_head", "B", "C", "D")]
+        il = None if i0 is None else i0.to("cuda").requires_grad_(True)
+        y, fs = D.ssd_mamba2_segmented(*lv, cfg.chunk, il, segments=segments)
+        ins = lv + ([] if il is None else [il])
+        res.append([y, fs, *torch.autograd.grad([y], ins, [inp["dy"].to("cuda")])])
+    tol = TOL_BF16 if dtype == "bf16" else 1e-4
+    for a, b in zip(*res):
+        assert a.shape == b.shape and a.dtype == b.dtype and rel_err(a.detach().float().cpu(), b.detach().float().cpu()) < tol
+    with pytest.raises(ValueError, match="segments of whole chunks"):
+        D.ssd_mamba2_segmented(*[inp[k].to("cuda") for k in ("x", "dt", "A_head", "B", "C", "D")], 8192)
+
+
 @pytest.mark.parametrize("per_step", [-4.0, -1.0])
 def test_tensor_core_path_fast_decay(pkg, cabi, oracle, per_step):
     """bf16, p 64, n 128 (the tcgen05 kernels) with a log-decay of `per_step` at every position: at -4 the decay
