@@ -629,8 +629,13 @@ int rope_op_impl(bool backward, long long BT, int H, int D, int aH, const void* 
                  void* out, float* dang, cudaStream_t st) {
     using namespace ssd::ew;
     constexpr int V = VecOf<T>::N;
-    const bool vec = D % V == 0 && !any_unaligned({x, dy, out});  // (the angles are read one by one)
-    if (!backward) {
+    const bool vec = D % V == 0 && !any_unaligned({x, dy, out});  // (angles shared by the heads are read one by one)
+    const size_t vecs = (size_t)BT * H * (D / V);
+    if (vec && aH == H && !any_unaligned({ang, dang}) && (vecs + 255) / 256 <= 0x7fffffffu) {
+        const unsigned nb = (unsigned)((vecs + 255) / 256);
+        if (!backward) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_flat_fwd_kernel<T, V><<<nb, 256, 0, st>>>((const T*)x, ang, (T*)out, vecs)));
+        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_flat_bwd_kernel<T, V><<<nb, 256, 0, st>>>((const T*)x, ang, (const T*)dy, (T*)out, dang, vecs)));
+    } else if (!backward) {
         if (vec) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_op_fwd_kernel<T, V><<<(unsigned)BT, 256, 0, st>>>((const T*)x, ang, (T*)out, H, D, aH)));
         else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_op_fwd_kernel<T, 2><<<(unsigned)BT, 256, 0, st>>>((const T*)x, ang, (T*)out, H, D, aH)));
     } else {

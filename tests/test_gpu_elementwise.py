@@ -213,6 +213,25 @@ def _shifted(t):
     return out
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1, 8), (1, 3, 5, 64), (2, 129, 3, 24), (1, 1000, 7, 40)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rope_angles_per_head_as_they_lie_in_memory(pkg, cabi, oracle, shape, dtype):
+    """Vectors that are no multiple of a block's 256, one vector in all, heads of three to sixteen vectors: values and gradients.  bf16 results are
+    one rounding off the fp32 ones of the same inputs (2^-8 of the value at most), angle gradients fp32 products."""
+    x, angles = _rope_inputs(*shape, dtype, seed=5, per_head=True)
+    g = torch.randn(*shape, generator=torch.Generator(device=DEV).manual_seed(6), device=DEV).to(dtype)
+    xr, ar = x.double().requires_grad_(True), angles.double().requires_grad_(True)
+    want = oracle.apply_rope(xr, ar)
+    want.backward(g.double())
+    xk, ak = x.clone().requires_grad_(True), angles.clone().requires_grad_(True)
+    y = pkg.fused_rope(xk, ak)
+    y.backward(g)
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    for got, ref in ((y, want), (xk.grad, xr.grad), (ak.grad, ar.grad)):
+        own = 2.0 ** -8 if got.dtype == torch.bfloat16 else ulp if got is ak.grad and ak.dtype == torch.bfloat16 else 0.0
+        assert ((got.double() - ref).abs() <= own * ref.abs() + 1e-5 * ref.abs().max()).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("who", ["x", "angles", "dy"])
 def test_rope_takes_any_address(pkg, cabi, dtype, who):
