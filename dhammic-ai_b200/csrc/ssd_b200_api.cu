@@ -600,7 +600,16 @@ int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* 
     const size_t rows = (size_t)d.b * d.T * d.h;
     if (dxw)  // otherwise the scan's backward has already produced dx, dw and dyx (scaled operator form)
         M3_ROW_DISPATCH(!any_unaligned({x, dy, dxw, dx}), xw_bwd_kernel, (const T*)x, (const T*)dy, (const T*)dxw, dt, lam, D, sdot, (T*)dx, dw, dyx, d.T, d.h, d.hpg, d.p, rows);
-    if (d.n % VecOf<T>::N == 0 && !any_unaligned({B, C, cum, dBr, dCr, dB, dC, dcum})) {
+    const bool aligned = !any_unaligned({B, C, cum, dBr, dCr, dB, dC, dcum});
+    const long long bt = (long long)d.b * d.T;
+    if (sizeof(T) == 2 && aligned && d.n % 64 == 0 && d.hpg % 4 == 0 && d.hpg <= 64 && bt * d.g * d.n < (1LL << 36)) {  // (and no more blocks than a grid has)
+        using bf = __nv_bfloat16;
+        const long long parts = ((long long)d.g * (d.n / 64) + kRingThreads / 32 - 1) / (kRingThreads / 32);
+        // sixteen positions a warp, fewer where that would be less than four rounds of the six blocks that an SM holds
+        const long long per = std::max(1LL, std::min(16LL, bt * parts / (4 * 6 * 148))), blocks = (bt + per - 1) / per * parts;
+
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_bwd_ring_kernel<<<(unsigned)blocks, kRingThreads, 0, st>>>((const bf*)B, (const bf*)C, cum, (const bf*)dBr, (const bf*)dCr, dyx, dt, lam, (bf*)dB, (bf*)dC, dcum, d.T, d.h, d.g, d.n, (unsigned)bt, (unsigned)per, (unsigned)parts)));
+    } else if (d.n % VecOf<T>::N == 0 && aligned) {
         const size_t items = (size_t)d.b * d.T * d.g * (d.n / VecOf<T>::N);
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_bwd_kernel<T, VecOf<T>::N><<<(unsigned)((items + 255) / 256), 256, 0, st>>>((const T*)B, (const T*)C, cum, (const T*)dBr, (const T*)dCr, dyx, dt, lam, (T*)dB, (T*)dC, dcum, d.T, d.h, d.g, d.n, items)));
     } else {

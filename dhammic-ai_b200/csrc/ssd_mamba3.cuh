@@ -423,6 +423,127 @@ __global__ void __launch_bounds__(256) rope_bwd_kernel(const T* __restrict__ B, 
     store_elems<T, V>(dC + ib, oc);
 }
 
+// The same where heads come in fours, at most 64 to a group, and columns in blocks of 64 (bf16): a warp takes four heads x eight vectors of columns
+// at a time, walks the heads of its group and then `per` positions; `parts` blocks share the warps of a position.  d theta is the cross product of
+// the unturned pair with the gradient turned back, which is wanted for dB and dC anyway; these are added over the four heads of a warp at the end
+// of a position, every lane keeping what it stores (12 shuffles for 64 sums).
+// HBM-bound.  Above, a thread waits for the loads of every head and for the three scalars of the diagonal term behind them, and finds its place by
+// divisions of 64-bit numbers: 4.6 TB/s, however the loop is unrolled.  Here the vectors come through a ring in shared memory, three stages, of which a
+// thread reads only what it copied itself (no barrier), the scalars a position ahead: 1050 -> 741 us at (16, 4096, 64 heads, 128 columns, 8
+// groups), 6.5 TB/s (860 with the scalars asked for where they are used).
+constexpr int kRingThreads = 128, kRingStages = 3;
+__global__ void __launch_bounds__(kRingThreads, 768 / kRingThreads) rope_bwd_ring_kernel(
+    const __nv_bfloat16* __restrict__ B, const __nv_bfloat16* __restrict__ C, const float* __restrict__ cum, const __nv_bfloat16* __restrict__ dBr,
+    const __nv_bfloat16* __restrict__ dCr, const float* __restrict__ dyx, const float* __restrict__ dt, const float* __restrict__ lam,
+    __nv_bfloat16* __restrict__ dB, __nv_bfloat16* __restrict__ dC, float* __restrict__ dcum, int Tlen, int h, int g, int n, unsigned rows, unsigned per, unsigned parts) {
+    using T = __nv_bfloat16;
+    constexpr int V = 8, STAGE = 5 * kRingThreads;
+    __shared__ __align__(16) uint4 ring[kRingStages * STAGE];  // a stage: dBr | dCr | angles | B | C
+    const unsigned hpg = h / g, strips = n / 64, w = blockIdx.x % parts * (kRingThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= g * strips) return;
+    const unsigned gg = w / strips, steps = hpg / 4;
+    const unsigned r0 = blockIdx.x / parts * per, R = min(per, rows - r0);
+    const unsigned j0 = ((w - gg * strips) * 8 + (lane & 7)) * V, h0 = gg * hpg + (lane >> 3);
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ring) + threadIdx.x * 16;
+    auto copy = [&](uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); };
+    unsigned fr = 0, fk = 0, fs = 0;  // what is fetched next: position, four heads, stage
+    auto fetch = [&] {                // one group of copies a step, empty behind the last
+        if (fr < R) {
+            const size_t o = ((size_t)(r0 + fr) * h + h0 + fk * 4) * n + j0;
+            const uint32_t d = mine + fs * (STAGE * 16);
+            copy(d, dBr + o);
+            copy(d + kRingThreads * 16, dCr + o);
+            copy(d + 2 * kRingThreads * 16, cum + o / 2);
+            if (fk == 0) {
+                const size_t ib = ((size_t)(r0 + fr) * g + gg) * n + j0;
+                copy(d + 3 * kRingThreads * 16, B + ib);
+                copy(d + 4 * kRingThreads * 16, C + ib);
+            }
+            if (++fk == steps) {
+                fk = 0;
+                ++fr;
+            }
+            if (++fs == kRingStages) fs = 0;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // (1 - lam), dt behind a position and <dy, x> at it, of this lane's heads of the group (at most two): a position ahead of their use
+    float lam_n[2], dt_n[2], yx_n[2];
+    auto fetch_diagonal = [&](unsigned r) {
+        const unsigned row = r0 + r;
+        const bool ok = r < R && (row + 1) % (unsigned)Tlen != 0;  // the last position of a sequence has none
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const bool on = ok && lane + 32 * i < hpg;
+            const size_t ih = (size_t)row * h + gg * hpg + lane + 32 * i;
+            lam_n[i] = on ? lam[ih + h] : 1.f;
+            dt_n[i] = on ? dt[ih + h] : 0.f;
+            yx_n[i] = on ? dyx[ih] : 0.f;
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < kRingStages - 1; ++i) fetch();
+    unsigned s = 0;
+    fetch_diagonal(0);
+    for (unsigned r = 0; r < R; ++r) {
+        float ds = 0.f;
+        float bv[V], cv[V], ab[V], ac[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) ab[q] = ac[q] = 0.f;
+        size_t o = ((size_t)(r0 + r) * h + h0) * n + j0;
+        for (unsigned k = 0; k < steps; ++k, o += 4 * n) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 2) : "memory");
+            const uint4* p = ring + s * STAGE + threadIdx.x;
+            const uint4 yb = p[0], yc = p[kRingThreads], ya = p[2 * kRingThreads];
+            if (k == 0) {
+                load_vec<T, V>(reinterpret_cast<const T*>(p + 3 * kRingThreads), bv);
+                load_vec<T, V>(reinterpret_cast<const T*>(p + 4 * kRingThreads), cv);
+                ds = -((1.f - lam_n[0]) * dt_n[0] * yx_n[0] + (1.f - lam_n[1]) * dt_n[1] * yx_n[1]);
+                fetch_diagonal(r + 1);
+            }
+            if (++s == kRingStages) s = 0;
+            fetch();
+            float db[V], dc[V], ang[V / 2], dth[V / 2];
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+                db[q] = to_f(reinterpret_cast<const T*>(&yb)[q]);
+                dc[q] = to_f(reinterpret_cast<const T*>(&yc)[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < V / 2; ++q) ang[q] = reinterpret_cast<const float*>(&ya)[q];
+#pragma unroll
+            for (int q = 0; q < V / 2; ++q) {
+                float sn, c;
+                sincos_reduced(ang[q], &sn, &c);
+                const float b1 = c * db[2 * q] + sn * db[2 * q + 1], b2 = c * db[2 * q + 1] - sn * db[2 * q];
+                const float c1 = c * dc[2 * q] + sn * dc[2 * q + 1], c2 = c * dc[2 * q + 1] - sn * dc[2 * q];
+                ab[2 * q] += b1;
+                ab[2 * q + 1] += b2;
+                ac[2 * q] += c1;
+                ac[2 * q + 1] += c2;
+                dth[q] = (bv[2 * q] * b2 - bv[2 * q + 1] * b1) + (cv[2 * q] * c2 - cv[2 * q + 1] * c1);
+            }
+            store_f32<V / 2>(dcum + o / 2, dth);
+        }
+#pragma unroll
+        for (int of = 16; of > 0; of >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, of);
+        // lanes 0-15 end with four columns of dB, 16-31 of dC
+        const bool up = lane & 16, odd = lane & 8;
+        float v[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) v[q] = (up ? ac[q] : ab[q]) + __shfl_xor_sync(0xffffffffu, up ? ab[q] : ac[q], 16);
+        uint2 out;
+        T* e = reinterpret_cast<T*>(&out);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float sum = (odd ? v[4 + q] : v[q]) + __shfl_xor_sync(0xffffffffu, odd ? v[q] : v[4 + q], 8);
+            const float lo = up ? bv[q] : cv[q], hi = up ? bv[4 + q] : cv[4 + q];
+            e[q] = from_f<T>(fmaf(ds, odd ? hi : lo, sum));
+        }
+        *reinterpret_cast<uint2*>((up ? dC : dB) + ((size_t)(r0 + r) * g + gg) * n + j0 + (odd ? 4 : 0)) = out;
+    }
+}
+
 // ------------------------------------------------------------------------------------------
 // Trapezoidal weights.  One warp per (position, head) (or per (position, group) for the dot): lanes over
 // headdim / d_state.

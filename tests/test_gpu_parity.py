@@ -1059,6 +1059,46 @@ def test_mamba3_angle_sums_do_not_depend_on_the_route(pkg, cabi, T, h, n, b, dty
     assert rel_err(res[0][0], want) < TOL_FP32
 
 
+@pytest.mark.parametrize("b,T,h,g,n", [(1, 1, 4, 1, 64), (2, 5, 64, 1, 64), (3, 37, 12, 1, 128), (2, 130, 24, 2, 64), (1, 300, 40, 1, 192), (16, 1100, 8, 2, 64),
+                                       (1, 1201, 64, 8, 128), (2, 33, 6, 2, 64), (1, 40, 68, 1, 64)])
+def test_mamba3_rotation_backward(pkg, cabi, b, T, h, g, n):
+    """Gradients of the rotation on their own: heads in fours through the ring in shared memory (a warp, several blocks and part of one per position; one to
+    sixteen positions a warp, sequences that end inside a block; up to 64 heads a group) and the kernel for everything else (the last two
+    shapes, and all shapes with angles off the 16-byte boundary), against 64 bits.  Angle gradients are fp32 sums of eight products: 1e-5 of
+    the largest; dB and dC end in bf16, half a unit in 2^-8 of the value."""
+    import ctypes
+    lib, S = cabi.load(), pkg.ssd_scan
+    gen = torch.Generator(device=DEV).manual_seed(T + h)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    B, C, dBr, dCr = (randn(*s).bfloat16() for s in ((b, T, g, n), (b, T, g, n), (b, T, h, n), (b, T, h, n)))
+    cum, dt, lam, dyx = 100.0 * randn(b, T, h, n // 2), torch.rand(b, T, h, generator=gen, device=DEV), torch.rand(b, T, h, generator=gen, device=DEV), randn(b, T, h)
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, b, T, h, 64, n, g, T)
+    def heads(v):  # (b,T,g,n) per head, as complex pairs
+        return torch.view_as_complex(v.double().view(b, T, g, n // 2, 2)).repeat_interleave(h // g, 2)
+    turn = torch.polar(torch.ones_like(cum, dtype=torch.float64), cum.double())
+    gb, gc = (torch.view_as_complex(v.double().view(b, T, h, n // 2, 2)) * turn.conj() for v in (dBr, dCr))
+    want_dth = (heads(B).conj() * gb + heads(C).conj() * gc).imag
+    u = torch.nn.functional.pad(((1 - lam) * dt).double()[:, 1:], (0, 0, 0, 1))
+    ds = -(u * dyx.double()).view(b, T, g, h // g).sum(-1, keepdim=True)
+    def group(v):
+        return torch.view_as_real(v.view(b, T, g, h // g, n // 2).sum(3)).reshape(b, T, g, n)
+    want_dB, want_dC = group(gb) + ds * C.double(), group(gc) + ds * B.double()
+    P = S._ptr
+    for shift in (0, 1):
+        cum_ = torch.empty(cum.numel() + shift, device=DEV)[shift:].view(cum.shape).copy_(cum)
+        dB, dC, dcum, dang = torch.empty_like(B), torch.empty_like(C), torch.empty_like(cum), torch.empty_like(cum)
+        sdot, dw = torch.zeros(b, T, g, device=DEV), torch.zeros(b, T, h, device=DEV)
+        seg = torch.empty(b * ((T + 127) // 128) * h * (n // 2), device=DEV)
+        cabi.check(lib.ssd_b200_m3_prologue_bwd(ctypes.byref(shape), None, None, P(dt), P(lam), None, P(B), P(C), P(cum_), P(sdot), None, P(dBr), P(dCr), None,
+                                                P(dw), P(dyx), P(dB), P(dC), P(dang), cabi.F32, P(dcum), P(seg), S._stream(torch.device(DEV))))
+        torch.cuda.synchronize()
+        assert rel_err(dcum, want_dth) < TOL_FP32
+        for got, want in ((dB, want_dB), (dC, want_dC)):
+            assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+        assert rel_err(dang, -dcum.double().flip(1).cumsum(1).flip(1)) < TOL_FP32
+
+
 @pytest.mark.parametrize("T", [600, 128])
 def test_mamba3_angle_gradient_does_not_depend_on_the_batch(pkg, cabi, T):
     """Many columns take the reverse sum of the angle gradients in one pass, few in two; the order of the sums, and so
