@@ -680,6 +680,23 @@ unsigned norm_blocks(size_t M, int rows_per_block, int most) {
     return (unsigned)std::min<size_t>(most, (M + rows_per_block - 1) / rows_per_block);
 }
 
+template <class T, int TPR, int NV, bool GATED>
+void launch_norm_bwd(unsigned nb, int threads, cudaStream_t st, const T* x, const float* w, const T* z, const T* dout, const float* rstd, T* dx, T* dz, float* part,
+                     size_t M, int D) {
+    using namespace ssd::ew;
+    constexpr size_t smem = NormBwd<T, TPR, NV>::SMEM;
+    if (smem > 48 * 1024) {  // opt in once per device and process
+        static std::atomic<unsigned long long> done{0};
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+        const unsigned long long bit = 1ull << (dev & 63);
+        if (!(done.load(std::memory_order_acquire) & bit) &&
+            cudaFuncSetAttribute(rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
+            done.fetch_or(bit, std::memory_order_release);
+    }
+    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<nb, threads, smem, st>>>(x, w, z, dout, rstd, dx, dz, part, M, D)));
+}
+
 // A warp per row up to 4 vectors a lane (512 fp32, 1024 bf16 columns), else the block; as few vectors a thread as the row needs.
 // `given`: the forward finds the rows' statistic in rstd.
 template <class T, bool GATED>
@@ -691,8 +708,7 @@ void launch_norm_rows(bool backward, size_t M, int D, float eps, const T* x, con
     do {                                                                                                                            \
         constexpr int threads = TPR < 256 ? 256 : TPR;                                                                              \
         if (backward)                                                                                                               \
-            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<nb, threads, 0, st>>>(                \
-                x, w, z, dout, rstd, out, dz, part, M, D)));                                                                        \
+            launch_norm_bwd<T, TPR, NV, GATED>(nb, threads, st, x, w, z, dout, rstd, out, dz, part, M, D);                           \
         else                                                                                                                        \
             SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_fwd_kernel<T, TPR, NV, GATED><<<nb, threads, 0, st>>>(                \
                 x, w, z, out, rstd, M, D, eps, given)));                                                                            \

@@ -180,7 +180,13 @@ __global__ void __launch_bounds__(128) rope_op_bwd_kernel(const T* __restrict__ 
 // already rounded to the working dtype (the reference casts them, src/kernels/trapezoidal.py:241-243).
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float softplus_f(float s) { return fmaxf(s, 0.f) + log1pf(__expf(-fabsf(s))); }
-__device__ __forceinline__ float sigmoid_f(float s) { return __fdividef(1.f, 1.f + __expf(-s)); }
+// (The exponential without the instructions that keep results below 2^-126: they are added to one.)
+__device__ __forceinline__ float sigmoid_f(float s) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(s * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+    return r;
+}
 
 template <class T>
 __global__ void __launch_bounds__(256) trapezoid_fwd_kernel(const T* __restrict__ dt_raw, const T* __restrict__ lam_raw,
@@ -288,7 +294,7 @@ __device__ __forceinline__ float silu_grad_f(float z) {
 
 // A row of D elements over TPR threads (a warp, or the block), NV 16-byte vectors each.  A block's row has one vector per thread: the
 // fewer registers a thread needs, the more warps hide the latency of the loads and of the gate's exponentials (with 256
-// threads and two vectors each the backward took 143 us at (16384, 4096), 133 us with 512 threads).
+// threads and two vectors each the backward took 143 us at (16384, 4096), 133 us with 512 threads, before the copies below).
 template <class T>
 __host__ __device__ inline bool rms_fits(int D) {
     return D % VecOf<T>::N == 0 && D <= 256 * 4 * VecOf<T>::N;
@@ -376,14 +382,26 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
     }
 }
 
+// Where a row is a block's, the vectors of the next two rows are on their way into shared memory by asynchronous copies, each thread reading what
+// it copied itself, and the gate's sigmoid is made once and kept: registers and the exponential's pipe are what the kernel is short of.
+// (16384, 4096) gated bf16: 139 us with one row ahead in registers and the sigmoid made twice, 122 now (5.5 TB/s).
+template <class T, int TPR, int NV>
+struct NormBwd {
+    static constexpr bool RING = TPR > 32 && NV == 1;
+    static constexpr int STAGES = 2, WEIGHTS = TPR * NV * VecOf<T>::N * 4;
+    static constexpr size_t SMEM = WEIGHTS + (RING ? (size_t)STAGES * 3 * TPR * 16 : 0);
+};
 template <class T, int TPR, int NV, bool GATED>
 __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR : 1) rmsnorm_rows_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const T* __restrict__ z,
                                                                const T* __restrict__ dout, const float* __restrict__ rstd, T* __restrict__ dx,
                                                                T* __restrict__ dz, float* __restrict__ part, size_t M, int D) {
     constexpr int V = VecOf<T>::N, RPB = TPR < 256 ? 256 / TPR : 1;
+    using Cfg = NormBwd<T, TPR, NV>;
+    constexpr bool RING = Cfg::RING;
+    extern __shared__ __align__(16) float sw[];  // the weights (in registers they would make the kernel spill), [STAGES][x, dout, z][TPR] vectors
+    const uint4* ring = reinterpret_cast<const uint4*>(sw + TPR * NV * V);
     __shared__ float red[2][32];
     const int sub = threadIdx.x % TPR;
-    __shared__ __align__(16) float sw[TPR * NV * V];  // (the weights in registers would make the kernel spill)
     for (int c = threadIdx.x; c < TPR * NV * V; c += TPR < 256 ? 256 : TPR) sw[c] = c < D ? w[c] : 0.f;
     __syncthreads();
     float dw[NV * V];
@@ -393,7 +411,23 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
     size_t row = (size_t)blockIdx.x * RPB + threadIdx.x / TPR;
     RowVecs<T, NV> xn, zn, gn;
     float rn = 0.f;
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ring) + sub * 16;
+    int fs = 0, s_ = 0;  // the stages that are fetched and read next
+    auto copy = [&](int i, const T* p) {  // zeros behind the row's last column
+        const int c = sub * V, ok = c < D ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mine + (fs * 3 + i) * (TPR * 16)), "l"(p + (ok ? c : 0)), "r"(ok) : "memory");
+    };
     auto fetch = [&](size_t r) {
+        if constexpr (RING) {  // one group a row, empty behind the last
+            if (r < M) {
+                copy(0, x + r * D);
+                copy(1, dout + r * D);
+                if (GATED) copy(2, z + r * D);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            fs ^= 1;
+            return;
+        }
         if (r >= M) return;
         xn.load(x + r * D, sub, TPR, D);
         gn.load(dout + r * D, sub, TPR, D);
@@ -401,11 +435,24 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
         rn = rstd[r];
     };
     fetch(row);
+    if (RING) {
+        fetch(row + step);
+        if (row < M) rn = rstd[row];
+    }
     for (int par = 0; row < M; row += step, par ^= 1) {
+        if constexpr (RING) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            const uint4* p = ring + s_ * (3 * TPR) + sub;
+            xn.v[0] = p[0];
+            gn.v[0] = p[TPR];
+            if (GATED) zn.v[0] = p[2 * TPR];
+            s_ ^= 1;
+        }
         const RowVecs<T, NV> xc = xn, zc = zn, gc = gn;
         const float r = rn;
-        fetch(row + step);
-        float s = 0.f;
+        if (!RING) fetch(row + step);
+        else if (row + step < M) rn = rstd[row + step];
+        float s = 0.f, sg[RING ? V : 1];
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             float wv[V];
@@ -413,12 +460,17 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
 #pragma unroll
             for (int q = 0; q < V; ++q) {
                 float dn = gc.at(i, q);
-                if (GATED) dn *= silu_f(zc.at(i, q));
+                if (GATED) {
+                    const float zv = zc.at(i, q), si = sigmoid_f(zv);
+                    dn *= zv * si;
+                    if (RING) sg[RING ? q : 0] = si;
+                }
                 const float t = xc.at(i, q) * dn;
                 s = fmaf(wv[q], t, s);
                 dw[i * V + q] = fmaf(r, t, dw[i * V + q]);
             }
         }
+        if (RING) fetch(row + 2 * step);  // into the stage of this row, whose values have all been used
         s = rms_sum<TPR>(s, red[par]);
         const float k = r * r * s / (float)D;
 #pragma unroll
@@ -432,7 +484,7 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
                 const float xv = xc.at(i, q), gv = gc.at(i, q), wq = wv[q];
                 float dn = gv;
                 if (GATED) {
-                    const float zv = zc.at(i, q), si = sigmoid_f(zv);
+                    const float zv = zc.at(i, q), si = RING ? sg[RING ? q : 0] : sigmoid_f(zv);
                     dn *= zv * si;
                     oz[q] = gv * (xv * r * wq) * (si * (1.f + zv * (1.f - si)));
                 }

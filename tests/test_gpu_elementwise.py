@@ -295,3 +295,26 @@ def test_tensors_without_columns_are_refused(pkg, cabi):
     for call in (lambda: pkg.fused_rmsnorm(e, w, EPS), lambda: pkg.fused_gate_norm(e, e, w, EPS), lambda: pkg.fused_trapezoidal(e, e, w, w)):
         with pytest.raises((ValueError, RuntimeError, ZeroDivisionError)):
             call()
+
+
+@pytest.mark.parametrize("M", [1, 3, 700])
+@pytest.mark.parametrize("D,dtype", [(1032, torch.bfloat16), (2048, torch.bfloat16), (2056, torch.bfloat16), (4096, torch.bfloat16), (4104, torch.bfloat16),
+                                     (8192, torch.bfloat16), (516, torch.float32), (1028, torch.float32), (4096, torch.float32)])
+def test_norm_rows_of_a_block(pkg, cabi, M, D, dtype):
+    """Backward of the norm, with and without a gate, where a row is a block's: fewer rows than are fetched ahead, one and many to a block, rows that do not
+    fill the block's 256, 512 or 1024 vectors, gates from -60 to 60.  Against 64 bits; bf16 results one rounding (2^-8) off, sums over a row
+    and over the rows fp32: 1e-5 of the largest value."""
+    gen = torch.Generator(device=DEV).manual_seed(D + M)
+    x, dout = (torch.randn(M, D, generator=gen, device=DEV).to(dtype) for _ in range(2))
+    z = (20.0 * torch.randn(M, D, generator=gen, device=DEV)).clamp(-60, 60).to(dtype)
+    w = 1.0 + 0.1 * torch.randn(D, generator=gen, device=DEV)
+    for gate in (z, None):
+        lv = [t.clone().requires_grad_(True) for t in ((x, gate, w) if gate is not None else (x, w))]
+        out = pkg.fused_gate_norm(*lv, 1e-6) if gate is not None else pkg.fused_rmsnorm(*lv, 1e-6)
+        got = torch.autograd.grad(out, lv, dout)
+        ref = [t.detach().double().requires_grad_(True) for t in lv]
+        y = ref[0] * torch.rsqrt(ref[0].square().mean(-1, keepdim=True) + 1e-6) * ref[-1]
+        want = torch.autograd.grad(y * torch.nn.functional.silu(ref[1]) if gate is not None else y, ref, dout.double())
+        for a, b in zip(got, want):
+            ulp = 2.0 ** -8 if a.dtype == torch.bfloat16 else 0.0
+            assert ((a.double() - b).abs() <= ulp * b.abs() + 1e-5 * b.abs().max()).all()
