@@ -14,6 +14,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
+#include <set>
+#include <utility>
 #include <initializer_list>
 #include <vector>
 
@@ -128,6 +131,18 @@ int resolve_path(const ssd_b200_shape& s) {
         return SSD_B200_PATH_TC;
     if (!simt_supported(s, &why)) return fail(SSD_B200_EUNSUPPORTED, "%s", why);
     return SSD_B200_PATH_SIMT;
+}
+
+// More than 48 KB of shared memory for a kernel: asked for once per device and process.
+template <class... A>
+void opt_in_smem(void (*kernel)(A...), int bytes) {
+    static std::mutex m;
+    static std::set<std::pair<const void*, int>> done;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+    const std::pair<const void*, int> key((const void*)kernel, dev);
+    std::lock_guard<std::mutex> lock(m);
+    if (!done.count(key) && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) done.insert(key);
 }
 
 bool any_unaligned(std::initializer_list<const void*> ps) {
@@ -551,10 +566,10 @@ int m3_fwd_impl(const ssd::Dims& d, const void* x, const float* dt, const float*
     } else {
         const dim3 gs(nseg, (E + 255) / 256, d.b);
         if (ang_f32) {  // angles keep their own precision whatever the storage type of x, B and C
-            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<float><<<gs, 256, 0, st>>>((const float*)ang, segsum, d.T, E));
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_segsum_kernel<float, false><<<gs, 256, 0, st>>>((const float*)ang, segsum, d.T, E)));
             SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, float><<<gs, 256, 0, st>>>((const float*)ang, segsum, cum, d.T, E, 0, -1.f)));
         } else {
-            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<T><<<gs, 256, 0, st>>>((const T*)ang, segsum, d.T, E));
+            SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_segsum_kernel<T, false><<<gs, 256, 0, st>>>((const T*)ang, segsum, d.T, E)));
             SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<T, float><<<gs, 256, 0, st>>>((const T*)ang, segsum, cum, d.T, E, 0, -1.f)));
         }
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_fwd_kernel<T, 2><<<dim3(d.T, d.b), 256, 0, st>>>((const T*)B, (const T*)C, cum, (T*)Br, (T*)Cr, d.T, d.h, d.g, d.n)));
@@ -590,6 +605,14 @@ int m3_skip_impl(const ssd::Dims& d, const void* y_scan, const void* x, const fl
     return 0;
 }
 
+template <class TO>
+void launch_scan_rev(dim3 grid, cudaStream_t st, const float* in, TO* out, int T, int E) {
+    using namespace ssd::m3;
+    constexpr int smem = kRevGroups * kRevRows * kRevThreads * 8;
+    opt_in_smem(scanT_rev_kernel<TO>, smem);
+    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_rev_kernel<TO><<<grid, kRevThreads, smem, st>>>(in, out, T, E, -1.f));
+}
+
 template <class T>
 int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* dt, const float* lam, const float* D,
                 const void* B, const void* C, const float* cum, const float* sdot, const void* dxw, const void* dBr,
@@ -617,13 +640,13 @@ int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* 
         SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rope_bwd_kernel<T, 2><<<(unsigned)((items + 255) / 256), 256, 0, st>>>((const T*)B, (const T*)C, cum, (const T*)dBr, (const T*)dCr, dyx, dt, lam, (T*)dB, (T*)dC, dcum, d.T, d.h, d.g, d.n, items)));
     }
     // d raw_angles[t] = - sum_{s >= t} d cum[s]
-    if ((long long)d.b * E >= kOnePassColumns) {
-        const dim3 go((E + 63) / 64, d.b);
-        if (ang_f32) SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_rev_kernel<float><<<go, 64, 0, st>>>(dcum, (float*)dang, d.T, E, -1.f));
-        else SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_rev_kernel<T><<<go, 64, 0, st>>>(dcum, (T*)dang, d.T, E, -1.f));
+    if ((long long)d.b * E >= kOnePassColumns && E % 2 == 0 && !(((uintptr_t)dcum | (uintptr_t)dang) & 7)) {
+        const dim3 go((E / 2 + kRevThreads - 1) / kRevThreads, d.b);
+        if (ang_f32) launch_scan_rev<float>(go, st, dcum, (float*)dang, d.T, E);
+        else launch_scan_rev<T>(go, st, dcum, (T*)dang, d.T, E);
     } else {
         const dim3 gs(nseg, (E + 255) / 256, d.b);
-        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_segsum_kernel<float><<<gs, 256, 0, st>>>(dcum, segsum, d.T, E));
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_segsum_kernel<float, true><<<gs, 256, 0, st>>>(dcum, segsum, d.T, E)));
         if (ang_f32)
             SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (scanT_apply_kernel<float, float><<<gs, 256, 0, st>>>(dcum, segsum, (float*)dang, d.T, E, 1, -1.f)));
         else
@@ -685,15 +708,7 @@ void launch_norm_bwd(unsigned nb, int threads, cudaStream_t st, const T* x, cons
                      size_t M, int D) {
     using namespace ssd::ew;
     constexpr size_t smem = NormBwd<T, TPR, NV>::SMEM;
-    if (smem > 48 * 1024) {  // opt in once per device and process
-        static std::atomic<unsigned long long> done{0};
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
-        const unsigned long long bit = 1ull << (dev & 63);
-        if (!(done.load(std::memory_order_acquire) & bit) &&
-            cudaFuncSetAttribute(rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
-            done.fetch_or(bit, std::memory_order_release);
-    }
+    if (smem > 48 * 1024) opt_in_smem(rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED>, (int)smem);
     SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<nb, threads, smem, st>>>(x, w, z, dout, rstd, dx, dz, part, M, D)));
 }
 

@@ -77,9 +77,9 @@ __device__ __forceinline__ void store_vec(T* p, const float (&f)[V]) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Scan along T of a (b, T, E) tensor.  Pass 1: per-segment sums.
+// Scan along T of a (b, T, E) tensor.  Pass 1: per-segment sums, each from its first position or (REV) from its last.
 // ------------------------------------------------------------------------------------------
-template <class T>
+template <class T, bool REV>
 __global__ void __launch_bounds__(256) scanT_segsum_kernel(const T* __restrict__ in, float* __restrict__ segsum, int Tlen,
                                                            int E) {
     const int seg = blockIdx.x, bb = blockIdx.z;
@@ -87,10 +87,11 @@ __global__ void __launch_bounds__(256) scanT_segsum_kernel(const T* __restrict__
     if (e >= E) return;
     const int nseg = gridDim.x;
     const int t0 = seg * SEG, t1 = min(Tlen, t0 + SEG);
-    const T* p = in + ((size_t)bb * Tlen + t0) * E + e;
+    const T* p = in + ((size_t)bb * Tlen + (REV ? t1 - 1 : t0)) * E + e;
+    const ptrdiff_t step = REV ? -(ptrdiff_t)E : E;
     float s = 0.f;
 #pragma unroll 8
-    for (int t = t0; t < t1; ++t, p += E) s += to_f(*p);  // eight loads in flight per thread
+    for (int t = t0; t < t1; ++t, p += step) s += to_f(*p);  // eight loads in flight per thread
     segsum[((size_t)bb * nseg + seg) * E + e] = s;
 }
 
@@ -126,50 +127,61 @@ __global__ void __launch_bounds__(256) scanT_apply_kernel(const TI* __restrict__
     }
 }
 
-// Both passes in one, from the last position to the first: a thread keeps one column's sum over the segments behind (their
-// sums added one by one, as scanT_apply_kernel does: same order, same bits) and holds a segment's values, half of them in
-// registers and half in shared memory, while it adds them up in one direction and walks them in the other.  Reads the input
-// once instead of twice: 325 + 174 us -> 346 us at (16, 4096, 64 x 64) fp32 -> bf16.  Needs enough columns to have the bytes in
-// flight (kOnePassColumns); blocks of 64 threads, so that they spread evenly over the SMs and all of them are resident there.
+// Both passes in one, from the last position to the first: a thread keeps two columns' sums over the segments behind (added one by one, as
+// scanT_apply_kernel does, each summed up from its end: same order, same bits) and walks the positions.  HBM-bound: the values come through a
+// ring in shared memory, 56 positions ahead, of which a thread reads only what it copied itself.  (16, 4096, 64 x 64)
+// fp32 -> bf16: 346 us with a segment at a time, half of it in registers, whose loads waited for its stores; 259 now (6.2 TB/s), 338 with 64 threads a
+// block.
+// Needs enough columns to have the bytes in flight (kOnePassColumns), an even number of them and 8-byte aligned tensors.
 constexpr int kOnePassColumns = 148 * 256;
+constexpr int kRevThreads = 128, kRevRows = 8, kRevGroups = 8;  // positions of a group of copies, groups
 template <class TO>
-__global__ void __launch_bounds__(64, 8) scanT_rev_kernel(const float* __restrict__ in, TO* __restrict__ out, int Tlen, int E, float sign) {
-    constexpr int U = SEG / 2;
-    __shared__ float hi[U][64];
-    const int e = blockIdx.x * 64 + threadIdx.x;
+__global__ void __launch_bounds__(kRevThreads) scanT_rev_kernel(const float* __restrict__ in, TO* __restrict__ out, int Tlen, int E, float sign) {
+    extern __shared__ __align__(16) float2 pos[];  // [kRevGroups][kRevRows][kRevThreads]
+    const int e = (blockIdx.x * kRevThreads + threadIdx.x) * 2;
     if (e >= E) return;
     const size_t base = (size_t)blockIdx.y * Tlen * E + e;
-    const uint32_t sh = (uint32_t)__cvta_generic_to_shared(&hi[0][threadIdx.x]);
-    float behind = 0.f;
-    for (int t0 = (Tlen - 1) / SEG * SEG; t0 >= 0; t0 -= SEG) {
-        const int rows = min(SEG, Tlen - t0);
-        const float* p = in + base + (size_t)t0 * E;
-#pragma unroll 16
-        for (int q = 0; q < U; ++q) {  // zeros behind the end
-            const int ok = U + q < rows ? 4 : 0;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sh + q * 256), "l"(p + (size_t)(ok ? U + q : 0) * E), "r"(ok) : "memory");
-        }
-        float lo[U];
+    const float* p = in + base;
+    TO* o = out + base;
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(pos) + threadIdx.x * 8;
+    const int last = (Tlen - 1) / kRevRows;
+    auto fetch = [&](int g) {  // group g of the sequence (zeros behind the end); one group of copies, empty before the start
+        if (g >= 0) {
 #pragma unroll
-        for (int q = 0; q < U; ++q) lo[q] = q < rows ? p[(size_t)q * E] : 0.f;
-        asm volatile("cp.async.wait_all;" ::: "memory");  // (a thread reads only what it copied itself)
-        float s = 0.f, run = behind;
-#pragma unroll
-        for (int q = 0; q < U; ++q) s += lo[q];
-#pragma unroll 16
-        for (int q = 0; q < U; ++q) s += hi[q][threadIdx.x];
-        TO* o = out + base + (size_t)t0 * E;
-#pragma unroll 16
-        for (int q = U - 1; q >= 0; --q) {
-            run += hi[q][threadIdx.x];
-            if (U + q < rows) o[(size_t)(U + q) * E] = from_f<TO>(sign * run);
+            for (int q = 0; q < kRevRows; ++q) {
+                const int t = g * kRevRows + q, ok = t < Tlen ? 8 : 0;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(mine + ((g % kRevGroups) * kRevRows + q) * (kRevThreads * 8)), "l"(p + (size_t)(ok ? t : 0) * E), "r"(ok) : "memory");
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int q = U - 1; q >= 0; --q) {
-            run += lo[q];
-            if (q < rows) o[(size_t)q * E] = from_f<TO>(sign * run);
+    for (int i = 0; i < kRevGroups - 1; ++i) fetch(last - i);
+    float2 behind = make_float2(0.f, 0.f), run = behind, s = behind;
+    for (int g = last; g >= 0; --g) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRevGroups - 2) : "memory");
+        float2 v[kRevRows];
+#pragma unroll
+        for (int q = 0; q < kRevRows; ++q) v[q] = pos[((g % kRevGroups) * kRevRows + q) * kRevThreads + threadIdx.x];
+        fetch(g - (kRevGroups - 1));  // where the group before this one was
+#pragma unroll
+        for (int q = kRevRows - 1; q >= 0; --q) {
+            const int t = g * kRevRows + q;
+            run.x += v[q].x;
+            run.y += v[q].y;
+            s.x += v[q].x;
+            s.y += v[q].y;
+            if (t < Tlen) {
+                if constexpr (sizeof(TO) == 2) *reinterpret_cast<__nv_bfloat162*>(o + (size_t)t * E) = __floats2bfloat162_rn(sign * run.x, sign * run.y);
+                else *reinterpret_cast<float2*>(o + (size_t)t * E) = make_float2(sign * run.x, sign * run.y);
+            }
         }
-        behind += s;
+        if (g % (SEG / kRevRows) == 0) {  // the segment's first positions
+            behind.x += s.x;
+            behind.y += s.y;
+            run = behind;
+            s = make_float2(0.f, 0.f);
+        }
     }
 }
 
