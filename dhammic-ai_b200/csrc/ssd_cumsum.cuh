@@ -15,13 +15,15 @@ constexpr int LT = 128;  // tile length
 // entry); the backward, which is a seventh slower that way, has two instantiations, and the flags of the kernels below, one word per block,
 // select one on the device.
 constexpr float kMaskSafeLog2 = 100.f;
+constexpr int kFewCumsumBlocks = 512;
 constexpr int kFusedChunkMax = 1024;  // see cumsum_tile_fused_kernel
 
-// The block's word of the flags (null: not wanted), from the threads' own; every thread of the block calls this.
-__device__ __forceinline__ void raise_flag(int* extreme, int beyond) {
+// The block's words of the flags (one per tile and eight heads; null: not wanted), from the threads' own; every thread of the block calls this.
+template <int HB>
+__device__ __forceinline__ void raise_flag(int* extreme, int beyond, int h) {
     if (!extreme) return;
-    const int any = __syncthreads_or(beyond);
-    if (threadIdx.x == 0) extreme[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = any;
+    const int any = __syncthreads_or(beyond), words = (h + 7) / 8, w = blockIdx.y * (HB / 8) + threadIdx.x;
+    if (threadIdx.x < HB / 8 && w < words) extreme[((size_t)blockIdx.z * words + w) * gridDim.x + blockIdx.x] = any;
 }
 
 // The first block of a pass clears the status word (a memset of its own is a gap of 1.2 us and more on the stream, and what follows one is not
@@ -33,10 +35,11 @@ __device__ __forceinline__ void clear_status(int* status) {
 // ------------------------------------------------------------------------------------------
 // Per-position arrays of the tile kernels from a given a_cumsum: the tile-cumulative log2 decay, dt and the skip coefficient in
 // (b,h,Tp) order, Tp = T rounded up to whole tiles (behind the end of the sequence the decay stays at its last value and
-// dt and skip are zero).  One block per (tile, 32 heads, batch): dt arrives in the caller's (b,T,h) order and goes
+// dt and skip are zero).  One block per (tile, HB heads, batch; kFewCumsumBlocks): dt arrives in the caller's (b,T,h) order and goes
 // through a shared-memory transpose, so reads and writes are both 128-byte rows.  Chunks of any length: the cumulative
 // decay from the tile's start is a difference inside the tile's first chunk plus the totals of the chunks that end in
 // the tile.
+template <int HB>
 __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restrict__ cum, const float* __restrict__ dt,
                                                           float* __restrict__ tcum, float* __restrict__ dtT,
                                                           const float* __restrict__ skip, float* __restrict__ skipT,
@@ -44,38 +47,40 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
     dep_wait();
     clear_status(status);
     int beyond = 0;
-    __shared__ float sdt[LT][33];
-    __shared__ float ssk[LT][33];
+    constexpr int R = 256 / HB;  // rows that the block's threads read at a time
+    __shared__ float sdt[LT][HB + 1];
+    __shared__ float ssk[LT][HB + 1];
     const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = hg * 32;
+    const int h0 = hg * HB, rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
     const int t0 = kt * LT, rows = min(LT, T - t0);
-    const bool head_ok = h0 + lane < h;
+    const bool head_ok = h0 + hcol < h;
     if (dt) {
 #pragma unroll
-        for (int t = warp; t < LT; t += 8)
-            sdt[t][lane] = (head_ok && t < rows) ? dt[((size_t)bb * T + t0 + t) * h + h0 + lane] : 0.f;
+        for (int t = rl; t < LT; t += R)
+            sdt[t][hcol] = (head_ok && t < rows) ? dt[((size_t)bb * T + t0 + t) * h + h0 + hcol] : 0.f;
     }
     if (skip) {  // per-position skip coefficient of the scaled operator form, same transpose
 #pragma unroll
-        for (int t = warp; t < LT; t += 8)
-            ssk[t][lane] = (head_ok && t < rows) ? skip[((size_t)bb * T + t0 + t) * h + h0 + lane] : 0.f;
+        for (int t = rl; t < LT; t += R)
+            ssk[t][hcol] = (head_ok && t < rows) ? skip[((size_t)bb * T + t0 + t) * h + h0 + hcol] : 0.f;
     }
     __syncthreads();
     const int k0 = t0 / l, i0 = t0 - k0 * l;  // chunk of the tile's first position, position in it
     const bool one = i0 + rows <= l;           // the whole tile lies in that chunk
-    float v[4][4], before[4];
+    constexpr int NH = HB / 8;  // heads of a warp
+    float v[NH][4], before[NH];
 #pragma unroll
-    for (int i4 = 0; i4 < 4; ++i4) {  // every load of the warp's four heads is issued before any of them is used
-        const int hh = h0 + warp * 4 + i4;
+    for (int i4 = 0; i4 < NH; ++i4) {  // every load of the warp's heads is issued before any of them is used
+        const int hh = h0 + warp * NH + i4;
         const float* cu = cum + ((size_t)bb * h + hh) * T;  // (b,h,c,l): position t of the sequence at t
         before[i4] = (hh < h && i0 > 0) ? cu[t0 - 1] : 0.f;
 #pragma unroll
         for (int s4 = 0; s4 < 4; ++s4) v[i4][s4] = hh < h ? cu[t0 + min(s4 * 32 + lane, rows - 1)] : 0.f;
     }
 #pragma unroll
-    for (int i4 = 0; i4 < 4; ++i4) {
-        const int hl = warp * 4 + i4, hh = h0 + hl;
+    for (int i4 = 0; i4 < NH; ++i4) {
+        const int hl = warp * NH + i4, hh = h0 + hl;
         if (hh >= h) break;  // warp-uniform
         const float* cu = cum + ((size_t)bb * h + hh) * T;
         const size_t o = ((size_t)bb * h + hh) * Tp + t0;
@@ -99,7 +104,7 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
             if (skipT) skipT[o + tt] = ssk[tt][hl];
         }
     }
-    raise_flag(extreme, beyond);
+    raise_flag<HB>(extreme, beyond, h);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -112,7 +117,10 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
 // between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
 // kernels this replaces: 28 -> 7 us at (8, 2048, 24) with chunks of 64).  The skip array is transposed in a second round
 // through the panel of the log-decay.
-template <bool CUT>
+// HB heads to a block: 32, whose reads are whole 128-byte rows, or 8 where blocks of 32 would be too few to fill the chip: a block then has a
+// quarter of the loads and one head a warp instead of four (kFewCumsumBlocks): 4 blocks of 32 heads 4.9 us, in blocks of 8 3.2; 256 blocks 7.6 / 6.6, 1024
+// 15.4 / 16.8.
+template <bool CUT, int HB>
 __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __restrict__ a, int a_is_bf16,
                                                                 const float* __restrict__ dt, const float* __restrict__ A_head,
                                                                 float* __restrict__ cum, float* __restrict__ tcum,
@@ -122,45 +130,46 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
     dep_wait();
     clear_status(status);
     int beyond = 0;
-    __shared__ float sa[LT][33];
-    __shared__ float sdt[LT][33];
-    __shared__ float sbef[8][33];
+    constexpr int R = 256 / HB;  // rows that the block's threads read at a time
+    __shared__ float sa[LT][HB + 1];
+    __shared__ float sdt[LT][HB + 1];
+    __shared__ float sbef[8][HB + 1];
     const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = hg * 32;
+    const int h0 = hg * HB, rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
     const int t0 = kt * LT, rows = min(LT, T - t0);
-    const bool head_ok = h0 + lane < h;
-    const float Ah = (!a && head_ok) ? A_head[h0 + lane] : 0.f;
+    const bool head_ok = h0 + hcol < h;
+    const float Ah = (!a && head_ok) ? A_head[h0 + hcol] : 0.f;
     auto log_decay = [&](size_t i, float d) {
         if (!a) return d * Ah;
         return a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[i]) : ((const float*)a)[i];
     };
     const size_t row0 = (size_t)bb * T;
 #pragma unroll
-    for (int t = warp; t < LT; t += 8) {
-        const size_t i = (row0 + t0 + t) * h + h0 + lane;
+    for (int t = rl; t < LT; t += R) {
+        const size_t i = (row0 + t0 + t) * h + h0 + hcol;
         float d = 0.f, av = 0.f;
         if (head_ok && t < rows) {
             if (dt) d = dt[i];
             av = log_decay(i, d);
         }
-        sa[t][lane] = av;
-        sdt[t][lane] = d;
+        sa[t][hcol] = av;
+        sdt[t][hcol] = d;
     }
     const int i0 = t0 % l;  // positions of the tile's first chunk that lie in earlier tiles
-    if (i0) {
+    if (i0 && rl < 8) {  // (eight sums whatever HB, so that they have the same bits)
         float s = 0.f;
 #pragma unroll 8
-        for (int t = warp; t < i0; t += 8) {
-            const size_t i = (row0 + t0 - i0 + t) * h + h0 + lane;
+        for (int t = rl; t < i0; t += 8) {
+            const size_t i = (row0 + t0 - i0 + t) * h + h0 + hcol;
             if (head_ok) s += log_decay(i, dt && !a ? dt[i] : 0.f);
         }
-        sbef[warp][lane] = s;
+        sbef[rl][hcol] = s;
     }
     __syncthreads();
 #pragma unroll
-    for (int i4 = 0; i4 < 4; ++i4) {
-        const int hl = warp * 4 + i4, hh = h0 + hl;
+    for (int i4 = 0; i4 < HB / 8; ++i4) {
+        const int hl = warp * (HB / 8) + i4, hh = h0 + hl;
         if (hh >= h) break;  // warp-uniform
         const size_t o = ((size_t)bb * h + hh) * Tp + t0, oc = ((size_t)bb * h + hh) * T + t0;
         float before = 0.f;
@@ -211,19 +220,19 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
     if (skip) {
         __syncthreads();
 #pragma unroll
-        for (int t = warp; t < LT; t += 8)
-            sa[t][lane] = (head_ok && t < rows) ? skip[(row0 + t0 + t) * h + h0 + lane] : 0.f;
+        for (int t = rl; t < LT; t += R)
+            sa[t][hcol] = (head_ok && t < rows) ? skip[(row0 + t0 + t) * h + h0 + hcol] : 0.f;
         __syncthreads();
 #pragma unroll
-        for (int i4 = 0; i4 < 4; ++i4) {
-            const int hl = warp * 4 + i4, hh = h0 + hl;
+        for (int i4 = 0; i4 < HB / 8; ++i4) {
+            const int hl = warp * (HB / 8) + i4, hh = h0 + hl;
             if (hh >= h) break;
             const size_t o = ((size_t)bb * h + hh) * Tp + t0;
 #pragma unroll
             for (int s4 = 0; s4 < LT / 32; ++s4) skipT[o + s4 * 32 + lane] = sa[s4 * 32 + lane][hl];
         }
     }
-    raise_flag(extreme, beyond);
+    raise_flag<HB>(extreme, beyond, h);
 }
 
 // ------------------------------------------------------------------------------------------

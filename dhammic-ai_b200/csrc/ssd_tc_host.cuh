@@ -99,8 +99,8 @@ inline Pieces pieces_of(const Dims& d, bool reverse) {
     return best;
 }
 
-// Words of the extreme-decay flags: one per block of the cumulative sums.
-inline size_t flags_of(const Dims& d) { return (size_t)d.b * ((d.h + 31) / 32) * tiles_of(d.T); }
+// Words of the extreme-decay flags: one per tile and eight heads.
+inline size_t flags_of(const Dims& d) { return (size_t)d.b * ((d.h + 7) / 8) * tiles_of(d.T); }
 
 inline Ws ws_layout(const Dims& d, int pass) {
     Ws w{};
@@ -197,11 +197,14 @@ inline int set_walk_attrs(char* err, size_t errn) {
     return 0;
 }
 
+inline bool few_cumsum_blocks(const Dims& d) { return (long long)tiles_of(d.T) * ((d.h + 31) / 32) * d.b < kFewCumsumBlocks; }
+
 inline int launch_tile_cumsum(bool after, const Dims& d, const float* cum, const float* dt, float* tcum, float* dtT, const float* skip,
                               float* skipT, int* extreme, int* status, cudaStream_t st, char* err, size_t errn) {
     const int nt = tiles_of(d.T);
-    dim3 g(nt, (d.h + 31) / 32, d.b);
-    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, tile_cumsum_kernel, g, 256, 0, st, cum, dt, tcum, dtT, skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l));
+    const bool few = few_cumsum_blocks(d);
+    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, few ? tile_cumsum_kernel<8> : tile_cumsum_kernel<32>, dim3(nt, few ? (d.h + 7) / 8 : (d.h + 31) / 32, d.b), 256, 0, st, cum,
+                                              dt, tcum, dtT, skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l));
     SSD_TC_CHECK("tile_cumsum");
     return 0;
 }
@@ -211,10 +214,11 @@ template <class Args>
 inline int launch_cumsum_tile_fused(const Args* a, const Dims& d, float* cum, float* tcum, float* dtT, float* skipT, int* extreme, int* status, cudaStream_t st,
                                     char* err, size_t errn) {
     const int nt = tiles_of(d.T);
-    const dim3 g(nt, (d.h + 31) / 32, d.b);
-    const bool cut = d.l % LT != 0;  // a chunk ends inside a tile
-    SSD_LAUNCH(prof::K_CUMSUM, st, (launch_dep(false, (cut ? cumsum_tile_fused_kernel<true> : cumsum_tile_fused_kernel<false>), g, 256, 0, st, 
-        a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, cum, tcum, dtT, a->skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l)));
+    const bool few = few_cumsum_blocks(d), cut = d.l % LT != 0;  // cut: a chunk ends inside a tile
+    const auto kernel = few ? (cut ? cumsum_tile_fused_kernel<true, 8> : cumsum_tile_fused_kernel<false, 8>)
+                            : (cut ? cumsum_tile_fused_kernel<true, 32> : cumsum_tile_fused_kernel<false, 32>);
+    SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(false, kernel, dim3(nt, few ? (d.h + 7) / 8 : (d.h + 31) / 32, d.b), 256, 0, st,
+        a->a, a->shape.a_dtype == SSD_B200_BF16, a->dt, a->A_head, cum, tcum, dtT, a->skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l));
     SSD_TC_CHECK("cumsum_tile_fused");
     return 0;
 }
