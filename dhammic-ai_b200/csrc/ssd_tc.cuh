@@ -52,7 +52,7 @@ inline bool whole_tiles(int T, int p, int n, int l) { return p == HP && n == DN 
 inline int tiles_of(int T) { return (T + LT - 1) / LT; }
 
 // ------------------------------------------------------------------------------------------
-// Decay gradient of the tensor-core backward, one block per (128-tile, 32 heads, batch).
+// Decay gradient of the tensor-core backward, one block per (128-tile, HB heads, batch; see kFewCumsumBlocks).
 // Inputs in (b,h,T) layout (coalesced along t): the per-row gradients g w.r.t. the tile-cumulative
 // log-decay, ddtx = sum_p dX x, dyx = sum_p dy x, and gS, the terms that act through the tile's last row.  Within a tile
 //   dA[t] = sum_{t' >= t} g[t']      (a suffix sum, four 32-lane segments per warp and head)
@@ -73,26 +73,28 @@ struct DecayTileParams {
     int b, T, Tp, h, nt;  // Tp = nt * 128: stride of g, ddtx and dyx
 };
 
+template <int HB>
 __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
     dep_wait();
-    __shared__ float sdt[LT][33];
-    __shared__ float sout[LT][33];
+    constexpr int R = 256 / HB, NH = HB / 8;  // rows that the block's threads move at a time, heads of a warp
+    __shared__ float sdt[LT][HB + 1];
+    __shared__ float sout[LT][HB + 1];
     const int k = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = hg * 32;
-    const bool head_ok = h0 + lane < P.h;
+    const int h0 = hg * HB, rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
+    const bool head_ok = h0 + hcol < P.h;
     const int rows = min(LT, P.T - k * LT);
     if (P.dt) {
 #pragma unroll
-        for (int t = warp; t < LT; t += 8)
-            sdt[t][lane] = (head_ok && t < rows) ? P.dt[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + lane] : 0.f;
+        for (int t = rl; t < LT; t += R)
+            sdt[t][hcol] = (head_ok && t < rows) ? P.dt[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + hcol] : 0.f;
     }
-    // every load of the warp's four heads is issued before any of them is used
+    // every load of the warp's heads is issued before any of them is used
     const bool scaled = P.dt && !P.A_head;  // scaled operator form: three per-position outputs
-    float va[4][4], dxa[4][4], yxp[4][4], gsa[4];
+    float va[NH][4], dxa[NH][4], yxp[NH][4], gsa[NH];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int hh = h0 + warp * 4 + i;
+    for (int i = 0; i < NH; ++i) {
+        const int hh = h0 + warp * NH + i;
         gsa[i] = 0.f;
 #pragma unroll
         for (int s4 = 0; s4 < 4; ++s4) va[i][s4] = dxa[i][s4] = yxp[i][s4] = 0.f;
@@ -111,8 +113,8 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int hl = warp * 4 + i, hh = h0 + hl;
+    for (int i = 0; i < NH; ++i) {
+        const int hl = warp * NH + i, hh = h0 + hl;
         if (hh >= P.h) break;  // warp-uniform
         float v[4];
 #pragma unroll
@@ -170,8 +172,8 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
         if (!out) continue;  // block-uniform
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int hl = warp * 4 + i, hh = h0 + hl;
+        for (int i = 0; i < NH; ++i) {
+            const int hl = warp * NH + i, hh = h0 + hl;
             if (hh >= P.h) break;
             const float Ah = (P.A_head && pass == 0) ? P.A_head[hh] : 0.f;
 #pragma unroll
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
         __syncthreads();
         if (head_ok) {
 #pragma unroll
-            for (int t = warp; t < rows; t += 8) out[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + lane] = sout[t][lane];
+            for (int t = rl; t < rows; t += R) out[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + hcol] = sout[t][hcol];
         }
     }
 }

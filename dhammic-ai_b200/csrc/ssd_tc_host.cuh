@@ -427,7 +427,8 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.dskip = a->skip ? a->dskip : nullptr;
         P.dAh_part = (float*)(ws + w.dAh_part); P.dD_part = P.dyx ? (float*)(ws + w.dD_part) : nullptr;
         P.b = d.b; P.T = d.T; P.Tp = Tp; P.h = d.h; P.nt = nt;
-        SSD_LAUNCH(prof::K_DECAY, st, launch_dep(true, decay_tile_kernel, dim3(nt, (d.h + 31) / 32, d.b), 256, 0, st, P));
+        const bool few = few_cumsum_blocks(d);
+        SSD_LAUNCH(prof::K_DECAY, st, launch_dep(true, few ? decay_tile_kernel<8> : decay_tile_kernel<32>, dim3(nt, few ? (d.h + 7) / 8 : (d.h + 31) / 32, d.b), 256, 0, st, P));
         SSD_TC_CHECK("decay_grad");
         if (a->dt && a->A_head) {
             SSD_LAUNCH(prof::K_REDUCE, st, launch_dep(true, reduce_rows_kernel, dim3(d.h, a->D ? 2 : 1), 256, 0, st, 
