@@ -1059,6 +1059,29 @@ def test_mamba3_angle_sums_do_not_depend_on_the_route(pkg, cabi, T, h, n, b, dty
     assert rel_err(res[0][0], want) < TOL_FP32
 
 
+@pytest.mark.parametrize("h,chunk", [(3, 64), (9, 256), (33, 128)])
+def test_cumulative_sums_in_blocks_of_eight_and_of_32_heads(pkg, cabi, h, chunk):
+    """512 blocks of 32 heads and more against a batch entry alone, whose blocks have eight: the sums have the same bits, also where a chunk
+    begins in an earlier tile, and the decay gradients, taken from both kinds of blocks, agree (the walks are cut differently)."""
+    b, T = 16, 4096
+    gen = torch.Generator(device=DEV).manual_seed(h)
+    x, B, C, dy = (torch.randn(b, T, *s, generator=gen, device=DEV).bfloat16() for s in ((h, 64), (1, 128), (1, 128), (h, 64)))
+    B, C = B / 128 ** 0.5, C / 128 ** 0.5
+    A = -0.2 * torch.rand(b, T, h, generator=gen, device=DEV)
+    def run(part):
+        lv = [t[part].contiguous().requires_grad_(True) for t in (x, A, B, C)]
+        y, _, cache = pkg.fused_ssd_scan(*lv, chunk)
+        again = pkg.fused_ssd_scan(*lv, chunk, None, cache)[0]  # from the given sums
+        return cache["A_cumsum"], y, again, *torch.autograd.grad(y, lv, dy[part])[:2]
+    whole = run(slice(None))
+    for i in (0, b - 1):
+        alone = run(slice(i, i + 1))
+        assert torch.equal(alone[0], whole[0][i:i + 1])
+        assert torch.equal(whole[1], whole[2]) or rel_err(whole[1], whole[2]) < TOL_BF16
+        for u, v in zip(alone[1:], whole[1:]):
+            assert rel_err(u, v[i:i + 1]) < TOL_BF16
+
+
 @pytest.mark.parametrize("b,T,h,g,n", [(1, 1, 4, 1, 64), (2, 5, 64, 1, 64), (3, 37, 12, 1, 128), (2, 130, 24, 2, 64), (1, 300, 40, 1, 192), (16, 1100, 8, 2, 64),
                                        (1, 1201, 64, 8, 128), (2, 33, 6, 2, 64), (1, 40, 68, 1, 64)])
 def test_mamba3_rotation_backward(pkg, cabi, b, T, h, g, n):
