@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
 
 // Where a row is a block's, the vectors of the next two rows are on their way into shared memory by asynchronous copies, each thread reading what
 // it copied itself, and the gate's sigmoid is made once and kept: registers and the exponential's pipe are what the kernel is short of.
-// (16384, 4096) gated bf16: 139 us with one row ahead in registers and the sigmoid made twice, 122 now (5.5 TB/s).
+// (16384, 4096) gated bf16: 139 us with one row ahead in registers and the sigmoid made twice, 111 now (6.0 TB/s; 120 before values were widened
+// as to_f does).
 template <class T, int TPR, int NV>
 struct NormBwd {
     static constexpr bool RING = TPR > 32 && NV == 1;

@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(256) rope_fwd_kernel(const T* __restrict__ B, 
 // sums of the segments before (angle_segsum_kernel, angle_prefix_kernel) and runs through its segment one by one: the order, and
 // the bits, of scanT_segsum_kernel and scanT_apply_kernel.  Where whole segments are too few blocks (rope_walks_segments), blocks of
 // 32 positions first add up what lies before them in the segment.
-// HBM-bound: at (16, 4096, 64 heads, 64 pairs) 138 + 333 + 531 us with a kernel for each step, 87 + 5 + 722 us now.
+// HBM-bound: at (16, 4096, 64 heads, 64 pairs) 138 + 333 + 531 us with a kernel for each step, 87 + 5 + 690 us now.
 // Needs whole vectors (n a multiple of V, 16-byte aligned angles).
 template <class TA, int N>
 struct alignas(N * sizeof(TA)) AngleVec {
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(256) rope_bwd_kernel(const T* __restrict__ B, 
 // HBM-bound.  Above, a thread waits for the loads of every head and for the three scalars of the diagonal term behind them, and finds its place by
 // divisions of 64-bit numbers: 4.6 TB/s, however the loop is unrolled.  Here the vectors come through a ring in shared memory, three stages, of which a
 // thread reads only what it copied itself (no barrier), the scalars a position ahead: 1050 -> 741 us at (16, 4096, 64 heads, 128 columns, 8
-// groups), 6.5 TB/s (860 with the scalars asked for where they are used).
+// groups), 6.5 TB/s (860 with the scalars asked for where they are used; 720 since values are widened as to_f does).
 constexpr int kRingThreads = 128, kRingStages = 3;
 __global__ void __launch_bounds__(kRingThreads, 768 / kRingThreads) rope_bwd_ring_kernel(
     const __nv_bfloat16* __restrict__ B, const __nv_bfloat16* __restrict__ C, const float* __restrict__ cum, const __nv_bfloat16* __restrict__ dBr,

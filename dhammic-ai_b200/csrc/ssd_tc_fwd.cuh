@@ -32,7 +32,7 @@
 // The per-half-row sums of y^2 keep their (b, T/128, h, 2, 128) layout: the odd quarter of each half leaves its partial
 // in shared memory, the even quarter adds its own and writes the sum after the block barrier at the top of the next tile.
 //
-// The diagonal block of the mask is evaluated entry by entry (one exponential each, by one warp in ten), which holds for any log-decay; below it
+// The diagonal block of the mask is evaluated entry by entry (one exponential each, by four of the ten warps that have a block to mask), which holds for any log-decay; below it
 // the mask is the product of a row and a column factor, both at most 1.  (A second instantiation with factors in the diagonal block as well, and a
 // flag that chose between the two on the device, was no faster, 515 against 516 us at (16, 4096, 64 heads), and the idle one of the
 // two took 2.3 to 7 us a call.)
