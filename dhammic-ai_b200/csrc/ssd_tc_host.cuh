@@ -67,12 +67,15 @@ struct Ws {
 // walk's last is first summarised (0.8 us per tile, 1.2 for two heads of a group, no chain, in parts that fill the chip), and a piece's CTA
 // folds the summaries before its own into its seed.  Only while all CTAs fit on the chip at once, and where the tiles taken off the chain
 // outweigh the summary and its launch (12 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.
+// No walk is cut from kWholeWalks pairs on, although reverse walks of up to 148 pairs with two heads per CTA would still gain by it ((1, 24576, 80 heads) forward and
+// backward 1,157 us cut, 1,197 whole; (2, 16384, 64) 1,017, 1,019): a cut changes the order of the state gradient's sums, and a call of
+// that many pairs has the same bits alone as a micro-batch of a larger one.
 // One prompt of 16,384 positions and 64 heads (128 tiles, two pieces): 282 us in one piece, 213 with one summary, 189 with two parts.
 struct Pieces {
     int pt, np, ps, parts;  // tiles of a piece, pieces, tiles of a summarised part, parts of a piece
     int heads, sum_heads;   // of a group per CTA of the walk (reverse), of the summary
 };
-constexpr int kPieceSms = 148, kMaxEntries = 16;
+constexpr int kPieceSms = 148, kMaxEntries = 16, kWholeWalks = 75;
 inline Pieces pieces_of(const Dims& d, bool reverse) {
     const int nt = tiles_of(d.T);
     const long long bh = (long long)d.b * d.h;
@@ -80,7 +83,7 @@ inline Pieces pieces_of(const Dims& d, bool reverse) {
     // in one piece: two heads per CTA (shared C panels, one N = 128 product per tile) only where one head per CTA would not fit on the chip at once
     Pieces best{nt, 1, nt, 1, reverse && even && bh > kPieceSms ? 2 : 1, 1};
     double cost = 0.9 * (reverse ? 1.5 : 2.15) * nt;
-    if (bh > kPieceSms) return best;
+    if (bh >= kWholeWalks) return best;
     for (int heads = 1; heads <= (reverse && even ? 2 : 1); ++heads)
         for (int P = 2; P <= kMaxEntries && P * bh <= kPieceSms * heads && P <= nt; ++P)
             for (int sum_heads = 1; sum_heads <= (even ? 2 : 1); ++sum_heads) {

@@ -581,6 +581,26 @@ def test_reverse_walk_in_pieces_of_two_heads(pkg, cabi, b, T, h, g):
         assert rel_err(got[k], want[k]) < TOL_BF16, k
 
 
+@pytest.mark.parametrize("T,h,g", [(6144, 96, 2), (12288, 128, 8), (24576, 76, 1)])
+def test_gradients_of_many_heads_do_not_depend_on_the_batch(pkg, cabi, T, h, g):
+    """One batch entry of 75 to 148 (batch, head) pairs alone, and the same entry in a batch of two: outputs and gradients have the same bits, so a call
+    may be cut into micro-batches (with fewer pairs the walks are cut into pieces, and with them the sums)."""
+    cfg = replace(pkg.CONFIGS[2], batch=2, seqlen=T, nheads=h, ngroups=g, chunk=128)
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    x, B, C, dy = (randn(2, T, *s).bfloat16() for s in ((h, 64), (g, 128), (g, 128), (h, 64)))
+    dt, A, D = 0.05 * torch.rand(2, T, h, generator=gen, device=DEV), -torch.rand(h, generator=gen, device=DEV), randn(h)
+    def run(part):
+        lv = [t.requires_grad_(True) for t in (x[part].clone(), dt[part].clone(), A.clone(), B[part].clone() / 128 ** 0.5, C[part].clone(), D.clone())]
+        y, fs = pkg.ssd_mamba2(*lv, cfg.chunk)
+        return [y, fs, *(v for i, v in enumerate(torch.autograd.grad(y, lv, dy[part])) if i not in (2, 5))]
+    whole = run(slice(None))
+    for i in range(2):
+        for name, u, v in zip(("y", "final", "dx", "ddt", "dB", "dC"), run(slice(i, i + 1)), whole):
+            assert torch.equal(u, v[i:i + 1]), name
+
+
 def test_walk_in_one_piece_where_the_workspace_has_no_room(pkg, cabi):
     """With less workspace than several pieces need, but enough for one, the walks run in one; with a byte less they are refused."""
     cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=4096, nheads=6, ngroups=2, chunk=128)
