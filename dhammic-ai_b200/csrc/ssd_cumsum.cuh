@@ -117,11 +117,20 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
 // between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
 // kernels this replaces: 28 -> 7 us at (8, 2048, 24) with chunks of 64).  The skip array is transposed in a second round
 // through the panel of the log-decay.
+// A thread's values of every `step`-th row, zeros from row `rows` on: a loop of its own, so that every load is issued before a value is used.  (Left to the
+// compiler in one loop with the stores to shared memory, the loads went out one after the other or all at once as the rest of the kernel had it: 104 us or 123 at
+// (4, 131072, 64 heads), 94 so.)
+template <int N, class TV>
+__device__ __forceinline__ void load_column(float (&v)[N], const TV* p, int step, int rows, int h) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = q * step < rows ? to_f(p[(size_t)q * step * h]) : 0.f;
+}
+
 // HB heads to a block: 32, whose reads are whole 128-byte rows, or 8 where blocks of 32 would be too few to fill the chip: a block then has a
 // quarter of the loads and one head a warp instead of four (kFewCumsumBlocks): 4 blocks of 32 heads 4.9 us, in blocks of 8 3.2; 256 blocks 7.6 / 6.6, 1024
 // 15.4 / 16.8.
 template <bool CUT, int HB>
-__global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __restrict__ a, int a_is_bf16,
+__global__ void __launch_bounds__(256, CUT ? 4 : 5) cumsum_tile_fused_kernel(const void* __restrict__ a, int a_is_bf16,
                                                                 const float* __restrict__ dt, const float* __restrict__ A_head,
                                                                 float* __restrict__ cum, float* __restrict__ tcum,
                                                                 float* __restrict__ dtT, const float* __restrict__ skip,
@@ -140,21 +149,23 @@ __global__ void __launch_bounds__(256) cumsum_tile_fused_kernel(const void* __re
     const int t0 = kt * LT, rows = min(LT, T - t0);
     const bool head_ok = h0 + hcol < h;
     const float Ah = (!a && head_ok) ? A_head[h0 + hcol] : 0.f;
-    auto log_decay = [&](size_t i, float d) {
-        if (!a) return d * Ah;
-        return a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[i]) : ((const float*)a)[i];
-    };
+    auto given = [&](size_t i) { return a_is_bf16 ? __bfloat162float(((const __nv_bfloat16*)a)[i]) : ((const float*)a)[i]; };
+    auto log_decay = [&](size_t i, float d) { return a ? given(i) : d * Ah; };
     const size_t row0 = (size_t)bb * T;
+    constexpr int N = LT / R;
+    float dv[N], av[N];
+    const size_t first = (row0 + t0 + rl) * h + h0 + hcol;
+    const int mine = head_ok ? rows - rl : 0;
+    if (a) {
+        if (a_is_bf16) load_column(av, (const __nv_bfloat16*)a + first, R, mine, h);
+        else load_column(av, (const float*)a + first, R, mine, h);
+    }
+    if (dt) load_column(dv, dt + first, R, mine, h);
 #pragma unroll
-    for (int t = rl; t < LT; t += R) {
-        const size_t i = (row0 + t0 + t) * h + h0 + hcol;
-        float d = 0.f, av = 0.f;
-        if (head_ok && t < rows) {
-            if (dt) d = dt[i];
-            av = log_decay(i, d);
-        }
-        sa[t][hcol] = av;
-        sdt[t][hcol] = d;
+    for (int q = 0; q < N; ++q) {
+        const int t = rl + q * R;
+        sa[t][hcol] = a ? av[q] : q * R < mine ? dv[q] * Ah : 0.f;
+        if (dt) sdt[t][hcol] = dv[q];
     }
     const int i0 = t0 % l;  // positions of the tile's first chunk that lie in earlier tiles
     if (i0 && rl < 8) {  // (eight sums whatever HB, so that they have the same bits)
