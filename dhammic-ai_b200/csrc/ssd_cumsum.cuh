@@ -15,7 +15,11 @@ constexpr int LT = 128;  // tile length
 // entry); the backward, which is a seventh slower that way, has two instantiations, and the flags of the kernels below, one word per block,
 // select one on the device.
 constexpr float kMaskSafeLog2 = 100.f;
-constexpr int kFewCumsumBlocks = 512;
+// Heads to a block of cumsum_tile_fused_kernel: 32, whose reads are whole 128-byte rows, or eight, a quarter of the loads and one head a warp instead of four, where
+// blocks of eight are few (nine to an SM) or blocks of 32 are half empty (cumsum_blocks_of_eight).  Blocks of 32 / of eight, us, each after a
+// write of 256 MB: 4 blocks of 32 heads, 24 of them heads, 8.2 / 6.4; 256, all heads, 10.2 / 10.3; 384 12.3 / 12.3; 512 14.3 / 14.4; 1024 18.4 / 22.5; 1024 with
+// 8 heads each 14.4 / 10.2, with 16 14.6 / 14.4, with 24 17.4 / 17.8; log-decays given in bf16: 256, all heads, 12.3 / 10.2, 1024 20.5 / 22.5.
+constexpr int kFewCumsumBlocks = 9 * 148;
 constexpr int kFusedChunkMax = 1024;  // see cumsum_tile_fused_kernel
 
 // The block's words of the flags (one per tile and eight heads; null: not wanted), from the threads' own; every thread of the block calls this.
@@ -35,11 +39,11 @@ __device__ __forceinline__ void clear_status(int* status) {
 // ------------------------------------------------------------------------------------------
 // Per-position arrays of the tile kernels from a given a_cumsum: the tile-cumulative log2 decay, dt and the skip coefficient in
 // (b,h,Tp) order, Tp = T rounded up to whole tiles (behind the end of the sequence the decay stays at its last value and
-// dt and skip are zero).  One block per (tile, HB heads, batch; kFewCumsumBlocks): dt arrives in the caller's (b,T,h) order and goes
-// through a shared-memory transpose, so reads and writes are both 128-byte rows.  Chunks of any length: the cumulative
+// dt and skip are zero).  One block per (tile, eight heads, batch), a head a warp: dt arrives in the caller's (b,T,h) order and goes
+// through a shared-memory transpose: reads of 32 bytes, writes of 128-byte rows.  (Blocks of 32 heads, four a warp, behind a call on the same inputs with chunks
+// of 64: 12.4 us against 4.0 at (8, 2048, 32 heads), 23.5 / 15.7 at (16, 4096, 64), 59 / 55 at (4, 65536, 64), 105 / 108 at (4, 131072, 64).)  Chunks of any length: the cumulative
 // decay from the tile's start is a difference inside the tile's first chunk plus the totals of the chunks that end in
 // the tile.
-template <int HB>
 __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restrict__ cum, const float* __restrict__ dt,
                                                           float* __restrict__ tcum, float* __restrict__ dtT,
                                                           const float* __restrict__ skip, float* __restrict__ skipT,
@@ -47,51 +51,43 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
     dep_wait();
     clear_status(status);
     int beyond = 0;
-    constexpr int R = 256 / HB;  // rows that the block's threads read at a time
+    constexpr int HB = 8, R = 256 / HB;  // heads of a block, rows that its threads read at a time
     __shared__ float sdt[LT][HB + 1];
     __shared__ float ssk[LT][HB + 1];
-    const int kt = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
+    const int kt = blockIdx.x, h0 = blockIdx.y * HB, bb = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = hg * HB, rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
+    const int rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
     const int t0 = kt * LT, rows = min(LT, T - t0);
-    const bool head_ok = h0 + hcol < h;
+    const bool col_ok = h0 + hcol < h;
     if (dt) {
 #pragma unroll
         for (int t = rl; t < LT; t += R)
-            sdt[t][hcol] = (head_ok && t < rows) ? dt[((size_t)bb * T + t0 + t) * h + h0 + hcol] : 0.f;
+            sdt[t][hcol] = (col_ok && t < rows) ? dt[((size_t)bb * T + t0 + t) * h + h0 + hcol] : 0.f;
     }
     if (skip) {  // per-position skip coefficient of the scaled operator form, same transpose
 #pragma unroll
         for (int t = rl; t < LT; t += R)
-            ssk[t][hcol] = (head_ok && t < rows) ? skip[((size_t)bb * T + t0 + t) * h + h0 + hcol] : 0.f;
+            ssk[t][hcol] = (col_ok && t < rows) ? skip[((size_t)bb * T + t0 + t) * h + h0 + hcol] : 0.f;
     }
     __syncthreads();
-    const int k0 = t0 / l, i0 = t0 - k0 * l;  // chunk of the tile's first position, position in it
-    const bool one = i0 + rows <= l;           // the whole tile lies in that chunk
-    constexpr int NH = HB / 8;  // heads of a warp
-    float v[NH][4], before[NH];
-#pragma unroll
-    for (int i4 = 0; i4 < NH; ++i4) {  // every load of the warp's heads is issued before any of them is used
-        const int hh = h0 + warp * NH + i4;
+    const int hh = h0 + warp;
+    if (hh < h) {  // warp-uniform
+        const int k0 = t0 / l, i0 = t0 - k0 * l;  // chunk of the tile's first position, position in it
+        const bool one = i0 + rows <= l;           // the whole tile lies in that chunk
         const float* cu = cum + ((size_t)bb * h + hh) * T;  // (b,h,c,l): position t of the sequence at t
-        before[i4] = (hh < h && i0 > 0) ? cu[t0 - 1] : 0.f;
+        const float before = i0 > 0 ? cu[t0 - 1] : 0.f;
+        float v[4];
 #pragma unroll
-        for (int s4 = 0; s4 < 4; ++s4) v[i4][s4] = hh < h ? cu[t0 + min(s4 * 32 + lane, rows - 1)] : 0.f;
-    }
-#pragma unroll
-    for (int i4 = 0; i4 < NH; ++i4) {
-        const int hl = warp * NH + i4, hh = h0 + hl;
-        if (hh >= h) break;  // warp-uniform
-        const float* cu = cum + ((size_t)bb * h + hh) * T;
+        for (int s4 = 0; s4 < 4; ++s4) v[s4] = cu[t0 + min(s4 * 32 + lane, rows - 1)];
         const size_t o = ((size_t)bb * h + hh) * Tp + t0;
 #pragma unroll
         for (int s4 = 0; s4 < 4; ++s4) {
             const int tt = s4 * 32 + lane;
-            float w = v[i4][s4] - before[i4];
+            float w = v[s4] - before;
             if (!one) {
                 const int k = (t0 + min(tt, rows - 1)) / l;
                 if (k != k0) {
-                    w = v[i4][s4] + (cu[(size_t)(k0 + 1) * l - 1] - before[i4]);
+                    w = v[s4] + (cu[(size_t)(k0 + 1) * l - 1] - before);
                     for (int kk = k0 + 1; kk < k; ++kk) w += cu[(size_t)(kk + 1) * l - 1];
                 }
             }
@@ -100,8 +96,8 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
             // decay across this 32-position block (lane 0 to lane 31)
             const float span = __shfl_sync(0xffffffffu, w, 0) - __shfl_sync(0xffffffffu, w, 31);
             if (!(span <= kMaskSafeLog2)) beyond = 1;
-            if (dtT) dtT[o + tt] = sdt[tt][hl];
-            if (skipT) skipT[o + tt] = ssk[tt][hl];
+            if (dtT) dtT[o + tt] = sdt[tt][warp];
+            if (skipT) skipT[o + tt] = ssk[tt][warp];
         }
     }
     raise_flag<HB>(extreme, beyond, h);

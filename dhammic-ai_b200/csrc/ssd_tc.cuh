@@ -52,7 +52,8 @@ inline bool whole_tiles(int T, int p, int n, int l) { return p == HP && n == DN 
 inline int tiles_of(int T) { return (T + LT - 1) / LT; }
 
 // ------------------------------------------------------------------------------------------
-// Decay gradient of the tensor-core backward, one block per (128-tile, HB heads, batch; see kFewCumsumBlocks).
+// Decay gradient of the tensor-core backward, one block per (128-tile, eight heads, batch): a head a warp and 32 registers.  (Blocks
+// of 32 heads, four a warp, need 128: 18.5 us against 14.4 for 384 of them, 27.5 / 20.8 at (16, 4096, 64 heads), 176 / 145 at (4, 131072, 64).)
 // Inputs in (b,h,T) layout (coalesced along t): the per-row gradients g w.r.t. the tile-cumulative
 // log-decay, ddtx = sum_p dX x, dyx = sum_p dy x, and gS, the terms that act through the tile's last row.  Within a tile
 //   dA[t] = sum_{t' >= t} g[t']      (a suffix sum, four 32-lane segments per warp and head)
@@ -73,58 +74,46 @@ struct DecayTileParams {
     int b, T, Tp, h, nt;  // Tp = nt * 128: stride of g, ddtx and dyx
 };
 
-template <int HB>
 __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
     dep_wait();
-    constexpr int R = 256 / HB, NH = HB / 8;  // rows that the block's threads move at a time, heads of a warp
+    constexpr int HB = 8, R = 256 / HB;  // heads of a block, rows that its threads move at a time
     __shared__ float sdt[LT][HB + 1];
     __shared__ float sout[LT][HB + 1];
-    const int k = blockIdx.x, hg = blockIdx.y, bb = blockIdx.z;
+    const int k = blockIdx.x, bb = blockIdx.z, h0 = blockIdx.y * HB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = hg * HB, rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
-    const bool head_ok = h0 + hcol < P.h;
+    const int rl = threadIdx.x / HB, hcol = threadIdx.x % HB;
+    const bool col_ok = h0 + hcol < P.h;
     const int rows = min(LT, P.T - k * LT);
     if (P.dt) {
 #pragma unroll
         for (int t = rl; t < LT; t += R)
-            sdt[t][hcol] = (head_ok && t < rows) ? P.dt[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + hcol] : 0.f;
+            sdt[t][hcol] = (col_ok && t < rows) ? P.dt[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + hcol] : 0.f;
     }
-    // every load of the warp's heads is issued before any of them is used
+    // every load of the warp's head is issued before any of them is used
     const bool scaled = P.dt && !P.A_head;  // scaled operator form: three per-position outputs
-    float va[NH][4], dxa[NH][4], yxp[NH][4], gsa[NH];
+    const int hh = h0 + warp;
+    const bool on = hh < P.h;  // warp-uniform
+    float v[4], dxa[4], yxp[4], gs = 0.f;
 #pragma unroll
-    for (int i = 0; i < NH; ++i) {
-        const int hh = h0 + warp * NH + i;
-        gsa[i] = 0.f;
+    for (int s4 = 0; s4 < 4; ++s4) v[s4] = dxa[s4] = yxp[s4] = 0.f;
+    if (on) {
+        const size_t base = ((size_t)bb * P.h + hh) * P.Tp + (size_t)k * LT;
 #pragma unroll
-        for (int s4 = 0; s4 < 4; ++s4) va[i][s4] = dxa[i][s4] = yxp[i][s4] = 0.f;
-        if (hh < P.h) {
-            const size_t base = ((size_t)bb * P.h + hh) * P.Tp + (size_t)k * LT;
-#pragma unroll
-            for (int s4 = 0; s4 < 4; ++s4) {
-                const int t = s4 * 32 + lane;
-                va[i][s4] = P.g[base + t];
-                dxa[i][s4] = P.ddtx[base + t];
-                if (P.dyx) yxp[i][s4] = P.dyx[base + t];
-            }
-            if (lane < 8)  // the eight terms that act through the tile's last row, one per lane
-                gsa[i] = P.gS[((((size_t)bb * P.h + hh) * P.nt) + k) * 8 + lane];
+        for (int s4 = 0; s4 < 4; ++s4) {
+            const int t = s4 * 32 + lane;
+            v[s4] = P.g[base + t];
+            dxa[s4] = P.ddtx[base + t];
+            if (P.dyx) yxp[s4] = P.dyx[base + t];
         }
+        if (lane < 8)  // the eight terms that act through the tile's last row, one per lane
+            gs = P.gS[((((size_t)bb * P.h + hh) * P.nt) + k) * 8 + lane];
     }
     __syncthreads();
+    if (on) {
+        // fixed-order sum of the eight terms (the other lanes hold zero), result in every lane
 #pragma unroll
-    for (int i = 0; i < NH; ++i) {
-        const int hl = warp * NH + i, hh = h0 + hl;
-        if (hh >= P.h) break;  // warp-uniform
-        float v[4];
-#pragma unroll
-        for (int s4 = 0; s4 < 4; ++s4) v[s4] = va[i][s4];
-        {
-            float gs = gsa[i];  // fixed-order sum of the eight terms (the other lanes hold zero), result in every lane
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
-            if (lane == 31) v[3] += gs;
-        }
+        for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
+        if (lane == 31) v[3] += gs;
         // suffix sums: inside each 32-lane segment by shuffles, then the totals of the later segments
         float tot[4];
 #pragma unroll
@@ -140,15 +129,13 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
         }
         v[2] += tot[3];
         v[1] += tot[3] + tot[2];
-        v[0] += (tot[3] + tot[2]) + tot[1];
-#pragma unroll
-        for (int s4 = 0; s4 < 4; ++s4) va[i][s4] = v[s4];  // d a[t] of this head and tile
+        v[0] += (tot[3] + tot[2]) + tot[1];  // v: d a[t] of this head and tile
         if (P.dt && !scaled) {
             float dAh = 0.f, yx = 0.f;
 #pragma unroll
             for (int s4 = 0; s4 < 4; ++s4) {
-                dAh += v[s4] * sdt[s4 * 32 + lane][hl];
-                yx += yxp[i][s4];
+                dAh += v[s4] * sdt[s4 * 32 + lane][warp];
+                yx += yxp[s4];
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -171,22 +158,19 @@ __global__ void __launch_bounds__(256) decay_tile_kernel(DecayTileParams P) {
         else out = scaled ? P.dskip : nullptr;
         if (!out) continue;  // block-uniform
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < NH; ++i) {
-            const int hl = warp * NH + i, hh = h0 + hl;
-            if (hh >= P.h) break;
+        if (on) {
             const float Ah = (P.A_head && pass == 0) ? P.A_head[hh] : 0.f;
 #pragma unroll
             for (int s4 = 0; s4 < 4; ++s4) {
                 float val;
-                if (pass == 0) val = P.dt ? dxa[i][s4] + va[i][s4] * Ah : va[i][s4];
-                else if (pass == 1) val = va[i][s4];
-                else val = yxp[i][s4];
-                sout[s4 * 32 + lane][hl] = val;
+                if (pass == 0) val = P.dt ? dxa[s4] + v[s4] * Ah : v[s4];
+                else if (pass == 1) val = v[s4];
+                else val = yxp[s4];
+                sout[s4 * 32 + lane][warp] = val;
             }
         }
         __syncthreads();
-        if (head_ok) {
+        if (col_ok) {
 #pragma unroll
             for (int t = rl; t < rows; t += R) out[((size_t)bb * P.T + (size_t)k * LT + t) * P.h + h0 + hcol] = sout[t][hcol];
         }

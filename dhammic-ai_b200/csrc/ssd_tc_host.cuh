@@ -200,14 +200,16 @@ inline int set_walk_attrs(char* err, size_t errn) {
     return 0;
 }
 
-inline bool few_cumsum_blocks(const Dims& d) { return (long long)tiles_of(d.T) * ((d.h + 31) / 32) * d.b < kFewCumsumBlocks; }
+inline bool cumsum_blocks_of_eight(const Dims& d) {  // see kFewCumsumBlocks
+    const int eights = (d.h + 7) / 8;
+    return (long long)tiles_of(d.T) * eights * d.b <= kFewCumsumBlocks || eights <= 2 * ((d.h + 31) / 32);
+}
 
 inline int launch_tile_cumsum(bool after, const Dims& d, const float* cum, const float* dt, float* tcum, float* dtT, const float* skip,
                               float* skipT, int* extreme, int* status, cudaStream_t st, char* err, size_t errn) {
     const int nt = tiles_of(d.T);
-    const bool few = few_cumsum_blocks(d);
-    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, few ? tile_cumsum_kernel<8> : tile_cumsum_kernel<32>, dim3(nt, few ? (d.h + 7) / 8 : (d.h + 31) / 32, d.b), 256, 0, st, cum,
-                                              dt, tcum, dtT, skip, skipT, extreme, status, d.T, nt * LT, d.h, d.l));
+    SSD_LAUNCH(prof::K_TC_AUX, st, launch_dep(after, tile_cumsum_kernel, dim3(nt, (d.h + 7) / 8, d.b), 256, 0, st, cum, dt, tcum, dtT, skip, skipT, extreme, status, d.T,
+                                              nt * LT, d.h, d.l));
     SSD_TC_CHECK("tile_cumsum");
     return 0;
 }
@@ -217,7 +219,7 @@ template <class Args>
 inline int launch_cumsum_tile_fused(const Args* a, const Dims& d, float* cum, float* tcum, float* dtT, float* skipT, int* extreme, int* status, cudaStream_t st,
                                     char* err, size_t errn) {
     const int nt = tiles_of(d.T);
-    const bool few = few_cumsum_blocks(d), cut = d.l % LT != 0;  // cut: a chunk ends inside a tile
+    const bool few = cumsum_blocks_of_eight(d), cut = d.l % LT != 0;  // cut: a chunk ends inside a tile
     const auto kernel = few ? (cut ? cumsum_tile_fused_kernel<true, 8> : cumsum_tile_fused_kernel<false, 8>)
                             : (cut ? cumsum_tile_fused_kernel<true, 32> : cumsum_tile_fused_kernel<false, 32>);
     SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(false, kernel, dim3(nt, few ? (d.h + 7) / 8 : (d.h + 31) / 32, d.b), 256, 0, st,
@@ -430,8 +432,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.dskip = a->skip ? a->dskip : nullptr;
         P.dAh_part = (float*)(ws + w.dAh_part); P.dD_part = P.dyx ? (float*)(ws + w.dD_part) : nullptr;
         P.b = d.b; P.T = d.T; P.Tp = Tp; P.h = d.h; P.nt = nt;
-        const bool few = few_cumsum_blocks(d);
-        SSD_LAUNCH(prof::K_DECAY, st, launch_dep(true, few ? decay_tile_kernel<8> : decay_tile_kernel<32>, dim3(nt, few ? (d.h + 7) / 8 : (d.h + 31) / 32, d.b), 256, 0, st, P));
+        SSD_LAUNCH(prof::K_DECAY, st, launch_dep(true, decay_tile_kernel, dim3(nt, (d.h + 7) / 8, d.b), 256, 0, st, P));
         SSD_TC_CHECK("decay_grad");
         if (a->dt && a->A_head) {
             SSD_LAUNCH(prof::K_REDUCE, st, launch_dep(true, reduce_rows_kernel, dim3(d.h, a->D ? 2 : 1), 256, 0, st, 

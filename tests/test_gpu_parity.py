@@ -133,7 +133,7 @@ def check_mamba2(pkg, oracle, cfg, tol, init=False, dfinal=False, seed=None):
 @pytest.mark.parametrize("kept", [True, False])
 def test_fast_decay_in_one_block_of_the_flags(pkg, cabi, oracle, b, T, h, at, kept):
     """A log-decay of -6 a position over 40 positions of one (batch, tile, head) only, that of a block of the cumulative sums at the
-    start, the end and inside the grid (heads in blocks of 32): 277 log2 units across a 32-column block, so the factorised mask of
+    start, the end and inside the grid (heads in blocks of eight): 277 log2 units across a 32-column block, so the factorised mask of
     the backward would leave the fp32 range there.  States kept by the forward or made again."""
     bb, tile, head = at
     cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, ngroups=2, chunk=128)
@@ -148,6 +148,47 @@ def test_fast_decay_in_one_block_of_the_flags(pkg, cabi, oracle, b, T, h, at, ke
         pkg.set_save_states(True)
     want = oracle.mamba2_fwd_bwd(inp, cfg.chunk, torch.float32)
     bad = {k: rel_err(got[k], want[k].reshape(got[k].shape)) for k in got if not rel_err(got[k], want[k].reshape(got[k].shape)) < TOL_BF16}
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("h,at", [(33, (0, 0, 0)), (33, (15, 31, 32)), (36, (7, 13, 31)), (64, (3, 30, 40))])
+@pytest.mark.parametrize("sums", ["kept", "made again", "given"])
+def test_fast_decay_in_one_block_of_32_heads(pkg, cabi, oracle, h, at, sums):
+    """The same in calls whose cumulative sums take heads in blocks of 32, where one block writes four flag words, the last one of a ragged head count fewer;
+    sums from the log-decays, kept for the backward or made again by it, and given by an earlier call.  Only the batch entry with the stretch is compared."""
+    bb, tile, head = at
+    b, T, g = 16, 4096, 1
+    cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=T, nheads=h, ngroups=g, chunk=64)
+    gen = torch.Generator(device=DEV).manual_seed(h + tile)
+    x, dy = (torch.randn(b, T, h, 64, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    B, C = (torch.randn(b, T, g, 128, generator=gen, device=DEV).div_(128 ** 0.5).bfloat16() for _ in range(2))
+    dt, A = 0.1 * torch.rand(b, T, h, generator=gen, device=DEV), -torch.rand(h, generator=gen, device=DEV)
+    A[head] = -60.0
+    dt[:, :, head] = 1e-3
+    dt[bb, tile * 128 + 50:tile * 128 + 90, head] = 0.1
+    own = {"x": x[bb:bb + 1], "dt": dt[bb:bb + 1], "A_head": A, "B": B[bb:bb + 1], "C": C[bb:bb + 1], "D": torch.zeros(h), "dy": dy[bb:bb + 1]}
+    if sums == "given":
+        xs, a = (x.float() * dt.unsqueeze(-1)).bfloat16(), dt * A
+        cache = pkg.fused_ssd_scan(xs[bb:bb + 1], a[bb:bb + 1], B[bb:bb + 1], C[bb:bb + 1], cfg.chunk)[2]
+        full = {"A_cumsum": torch.zeros(b, h, T // cfg.chunk, cfg.chunk, device=DEV)}
+        full["A_cumsum"][bb] = cache["A_cumsum"][0]
+        lv = [t.requires_grad_(True) for t in (xs, B, C)]
+        y = pkg.fused_ssd_scan(lv[0], a, lv[1], lv[2], cfg.chunk, None, full)[0]
+        got = dict(zip(("dx", "dB", "dC"), torch.autograd.grad(y, lv, dy)), y=y)
+        lo = [t[bb:bb + 1].detach().float().cpu().requires_grad_(True) for t in (xs, B, C)]
+        yo = oracle.ssd_chunked(lo[0], a[bb:bb + 1].cpu(), lo[1].expand(-1, -1, h, -1), lo[2].expand(-1, -1, h, -1), cfg.chunk)[0]
+        want = dict(zip(("dx", "dB", "dC"), torch.autograd.grad(yo, lo, dy[bb:bb + 1].float().cpu())), y=yo.detach())
+    else:
+        lv = [t.requires_grad_(True) for t in (x, dt, B, C)]
+        pkg.set_save_states(sums == "kept")
+        try:
+            y = pkg.ssd_mamba2(lv[0], lv[1], A, lv[2], lv[3], None, cfg.chunk)[0]
+            got = dict(zip(("dx", "ddt", "dB", "dC"), torch.autograd.grad(y, lv, dy)), y=y)
+        finally:
+            pkg.set_save_states(True)
+        full = oracle.mamba2_fwd_bwd({k: v.detach().cpu() for k, v in own.items()}, cfg.chunk, torch.float32)
+        want = {k: full[k] for k in got}
+    bad = {k: rel_err(got[k][bb:bb + 1], want[k]) for k in got if not rel_err(got[k][bb:bb + 1], want[k]) < TOL_BF16}
     assert not bad, bad
 
 
