@@ -278,6 +278,50 @@ def test_segmented_scan_inside_one_gpu(pkg, cabi, idx, segments, tol):
     assert D.pick_segments(1, 64, 131072) == 8 and D.pick_segments(16, 64, 4096) == 1
 
 
+@pytest.mark.parametrize("dtype,b,T,h,p,n,g,l,grads,cut", [
+    # the tcgen05 kernels: up to four pairs, with gradients from 131,072 positions on
+    ("bf16", 1, 131072, 4, 64, 128, 4, 128, True, True), ("bf16", 2, 131072, 2, 64, 128, 1, 128, True, True), ("bf16", 1, 65536, 1, 64, 128, 1, 128, True, False),
+    ("bf16", 1, 131072, 5, 64, 128, 1, 128, True, False), ("bf16", 1, 98304, 2, 64, 128, 1, 128, False, True), ("bf16", 1, 98304, 2, 64, 128, 1, 128, True, False),
+    # partial tiles: with gradients only
+    ("bf16", 1, 65536, 3, 64, 64, 1, 64, True, True), ("bf16", 1, 65536, 4, 64, 64, 1, 64, True, False), ("bf16", 1, 131072, 1, 64, 64, 1, 64, False, False),
+    # fp32, and bf16 with a headdim that the kernels for partial tiles do not take
+    ("fp32", 1, 32768, 2, 64, 16, 1, 64, True, True), ("fp32", 1, 32768, 1, 64, 16, 1, 64, True, False), ("bf16", 1, 131072, 4, 16, 8, 1, 64, True, True),
+    ("fp32", 1, 65536, 2, 64, 16, 1, 64, False, True), ("fp32", 1, 65536, 2, 64, 16, 1, 128, False, False), ("fp32", 1, 131072, 8, 64, 16, 1, 64, True, False)])
+def test_which_segmented_calls_are_one_call(pkg, cabi, monkeypatch, dtype, b, T, h, p, n, g, l, grads, cut):
+    """segments = 0: one call, or segments where a few heads of a very long sequence would each walk alone."""
+    D = importlib.import_module("dhammic-ai_b200.distributed")
+    took = []
+    monkeypatch.setattr(D._op, "ssd_mamba2", lambda *a, **k: took.append("one"))
+    monkeypatch.setattr(D, "ssd_mamba2_sequence_parallel", lambda *a, **k: took.append(k["segments"]))
+    def of(*shape):
+        return torch.empty((), dtype=torch.bfloat16 if dtype == "bf16" else torch.float32).expand(*shape)
+    A = torch.zeros(h, requires_grad=grads)
+    D.ssd_mamba2_segmented(of(b, T, h, p), of(b, T, h), A, of(b, T, g, n), of(b, T, g, n), None, l)
+    with torch.no_grad():
+        D.ssd_mamba2_segmented(of(b, T, h, p), of(b, T, h), A, of(b, T, g, n), of(b, T, g, n), None, l, segments=4)
+    assert took == [0 if cut else "one", 4]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,T,n,l", [("fp32", 32768, 16, 64), ("bf16", 131072, 128, 128), ("bf16", 65536, 64, 64)])
+def test_segments_of_a_few_heads_of_a_long_sequence(pkg, cabi, dtype, T, n, l):
+    """Two heads of a long sequence without a number of segments: the segments that the shape wants, bit for bit, with an initial state and without D."""
+    D = importlib.import_module("dhammic-ai_b200.distributed")
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    store = torch.bfloat16 if dtype == "bf16" else torch.float32
+    x, dy = (torch.randn(1, T, 2, 64, generator=gen, device="cuda").to(store) for _ in range(2))
+    B, C = (torch.randn(1, T, 1, n, generator=gen, device="cuda").div_(n ** 0.5).to(store) for _ in range(2))
+    dt, A = 0.05 * torch.rand(1, T, 2, generator=gen, device="cuda"), torch.tensor([-0.3, -2.0], device="cuda")
+    init = torch.randn(1, 2, 64, n, generator=gen, device="cuda")
+    res = []
+    for segments in (0, D.pick_segments(1, 2, T)):
+        lv = [t.clone().requires_grad_(True) for t in (x, dt, A, B, C, init)]
+        y, fs = D.ssd_mamba2_segmented(*lv[:5], None, l, lv[5], segments=segments)
+        res.append([y, fs, *torch.autograd.grad(y, lv, dy)])
+    for u, v in zip(*res):
+        assert torch.equal(u, v)
+
+
 # ---------------------------------------------------------------------------------------------------------
 # failures made on the host: no GPU is involved, nothing hangs
 # ---------------------------------------------------------------------------------------------------------
