@@ -16,6 +16,7 @@
 #include <atomic>
 #include <mutex>
 #include <set>
+#include <type_traits>
 #include <utility>
 #include <initializer_list>
 #include <vector>
@@ -703,13 +704,33 @@ unsigned norm_blocks(size_t M, int rows_per_block, int most) {
     return (unsigned)std::min<size_t>(most, (M + rows_per_block - 1) / rows_per_block);
 }
 
+// Whether the backward of rows that are a block's takes them through the ring (NormBwd).  Gated bf16 rows always do (0.80 to 0.99 of the time without, at any
+// length), and so do fp32 rows without a gate (0.90 to 1.00); the others by what was measured, us without / with the ring:
+//   fp32 with a gate: not where the row fills the block's vectors (rows of a power of two, whose streams meet in the same DRAM banks the more
+//     the further ahead they are read).  (16384, 2048) 109.7 / 120.6, (16384, 4096) 206.9 / 218.8, (16384, 1024) 63.8 / 66.0, but (16384, 1536) 90.9 / 85.2, (16384, 3072) 170 / 161
+//   bf16 without a gate: where few threads have no vector and a block walks many rows.  (16384, 4096) 84.6 / 82.7, (16384, 8192) 163.6 / 157.9, but
+//     (16384, 2088) 68.5 / 71.4, (2048, 4096) 21.4 / 21.8, (2048, 2048) 17.0 / 17.8
+template <class T>
+bool norm_bwd_ring(int vecs, int threads, size_t M, unsigned blocks) {
+    return sizeof(T) == 2 ? vecs * 8 >= threads * 7 && M >= (size_t)blocks * 16 : vecs < threads;
+}
+
+template <class T, int TPR, int NV, bool GATED, bool RING>
+void launch_norm_bwd_as(unsigned nb, int threads, cudaStream_t st, const T* x, const float* w, const T* z, const T* dout, const float* rstd, T* dx, T* dz, float* part,
+                        size_t M, int D) {
+    using namespace ssd::ew;
+    constexpr size_t smem = NormBwd<T, TPR, NV, RING>::SMEM;
+    if (smem > 48 * 1024) opt_in_smem(rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED, RING>, (int)smem);
+    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED, RING><<<nb, threads, smem, st>>>(x, w, z, dout, rstd, dx, dz, part, M, D)));
+}
 template <class T, int TPR, int NV, bool GATED>
 void launch_norm_bwd(unsigned nb, int threads, cudaStream_t st, const T* x, const float* w, const T* z, const T* dout, const float* rstd, T* dx, T* dz, float* part,
                      size_t M, int D) {
-    using namespace ssd::ew;
-    constexpr size_t smem = NormBwd<T, TPR, NV>::SMEM;
-    if (smem > 48 * 1024) opt_in_smem(rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED>, (int)smem);
-    SSD_LAUNCH(ssd::prof::K_TC_AUX, st, (rmsnorm_rows_bwd_kernel<T, TPR, NV, GATED><<<nb, threads, smem, st>>>(x, w, z, dout, rstd, dx, dz, part, M, D)));
+    auto as = [&](auto ring) { launch_norm_bwd_as<T, TPR, NV, GATED, ring.value>(nb, threads, st, x, w, z, dout, rstd, dx, dz, part, M, D); };
+    if constexpr (TPR == 32) as(std::false_type());
+    else if constexpr (GATED == (sizeof(T) == 2)) as(std::true_type());
+    else if (norm_bwd_ring<T>(D / ssd::ew::VecOf<T>::N, threads, M, nb)) as(std::true_type());
+    else as(std::false_type());
 }
 
 // A warp per row up to 4 vectors a lane (512 fp32, 1024 bf16 columns), else the block; as few vectors a thread as the row needs.

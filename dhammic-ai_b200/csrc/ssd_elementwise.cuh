@@ -382,23 +382,21 @@ __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR :
     }
 }
 
-// Where a row is a block's, the vectors of the next two rows are on their way into shared memory by asynchronous copies, each thread reading what
+// RING, where a row is a block's: the vectors of the next two rows are on their way into shared memory by asynchronous copies, each thread reading what
 // it copied itself, and the gate's sigmoid is made once and kept: registers and the exponential's pipe are what the kernel is short of.
-// (16384, 4096) gated bf16: 139 us with one row ahead in registers and the sigmoid made twice, 111 now (6.0 TB/s; 120 before values were widened
-// as to_f does).
-template <class T, int TPR, int NV>
+// (16384, 4096) gated bf16: 139 us with one row ahead in registers and the sigmoid made twice, 111 so (6.0 TB/s; 120 before values were widened
+// as to_f does).  norm_bwd_ring has the rows that do better without.
+template <class T, int TPR, int NV, bool RING>
 struct NormBwd {
-    static constexpr bool RING = TPR > 32 && NV == 1;
+    static_assert(!RING || (TPR > 32 && NV == 1), "a ring of one vector a thread");
     static constexpr int STAGES = 2, WEIGHTS = TPR * NV * VecOf<T>::N * 4;
     static constexpr size_t SMEM = WEIGHTS + (RING ? (size_t)STAGES * 3 * TPR * 16 : 0);
 };
-template <class T, int TPR, int NV, bool GATED>
+template <class T, int TPR, int NV, bool GATED, bool RING>
 __global__ void __launch_bounds__(TPR < 256 ? 256 : TPR, TPR > 32 ? 1024 / TPR : 1) rmsnorm_rows_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const T* __restrict__ z,
                                                                const T* __restrict__ dout, const float* __restrict__ rstd, T* __restrict__ dx,
                                                                T* __restrict__ dz, float* __restrict__ part, size_t M, int D) {
     constexpr int V = VecOf<T>::N, RPB = TPR < 256 ? 256 / TPR : 1;
-    using Cfg = NormBwd<T, TPR, NV>;
-    constexpr bool RING = Cfg::RING;
     extern __shared__ __align__(16) float sw[];  // the weights (in registers they would make the kernel spill), [STAGES][x, dout, z][TPR] vectors
     const uint4* ring = reinterpret_cast<const uint4*>(sw + TPR * NV * V);
     __shared__ float red[2][32];

@@ -297,13 +297,7 @@ def test_tensors_without_columns_are_refused(pkg, cabi):
             call()
 
 
-@pytest.mark.parametrize("M", [1, 3, 700])
-@pytest.mark.parametrize("D,dtype", [(1032, torch.bfloat16), (2048, torch.bfloat16), (2056, torch.bfloat16), (4096, torch.bfloat16), (4104, torch.bfloat16),
-                                     (8192, torch.bfloat16), (516, torch.float32), (1028, torch.float32), (4096, torch.float32)])
-def test_norm_rows_of_a_block(pkg, cabi, M, D, dtype):
-    """Backward of the norm, with and without a gate, where a row is a block's: fewer rows than are fetched ahead, one and many to a block, rows that do not
-    fill the block's 256, 512 or 1024 vectors, gates from -60 to 60.  Against 64 bits; bf16 results one rounding (2^-8) off, sums over a row
-    and over the rows fp32: 1e-5 of the largest value."""
+def _norm_rows(pkg, M, D, dtype):
     gen = torch.Generator(device=DEV).manual_seed(D + M)
     x, dout = (torch.randn(M, D, generator=gen, device=DEV).to(dtype) for _ in range(2))
     z = (20.0 * torch.randn(M, D, generator=gen, device=DEV)).clamp(-60, 60).to(dtype)
@@ -318,3 +312,22 @@ def test_norm_rows_of_a_block(pkg, cabi, M, D, dtype):
         for a, b in zip(got, want):
             ulp = 2.0 ** -8 if a.dtype == torch.bfloat16 else 0.0
             assert ((a.double() - b).abs() <= ulp * b.abs() + 1e-5 * b.abs().max()).all()
+
+
+@pytest.mark.parametrize("M", [1, 3, 700])
+@pytest.mark.parametrize("D,dtype", [(1032, torch.bfloat16), (2048, torch.bfloat16), (2056, torch.bfloat16), (4096, torch.bfloat16), (4104, torch.bfloat16),
+                                     (8192, torch.bfloat16), (516, torch.float32), (1028, torch.float32), (4096, torch.float32)])
+def test_norm_rows_of_a_block(pkg, cabi, M, D, dtype):
+    """Backward of the norm, with and without a gate, where a row is a block's: fewer rows than are fetched ahead, one and many to a block, rows that do not
+    fill the block's 256, 512 or 1024 vectors, gates from -60 to 60.  Against 64 bits; bf16 results one rounding (2^-8) off, sums over a row
+    and over the rows fp32: 1e-5 of the largest value."""
+    _norm_rows(pkg, M, D, dtype)
+
+
+@pytest.mark.parametrize("M,D,dtype", [(9472, 2048, torch.bfloat16), (9471, 2048, torch.bfloat16), (9600, 1792, torch.bfloat16), (9600, 1784, torch.bfloat16),
+                                       (4800, 4096, torch.bfloat16), (2400, 8192, torch.bfloat16), (700, 1024, torch.float32), (700, 2048, torch.float32),
+                                       (700, 2044, torch.float32), (700, 1536, torch.float32)])
+def test_norm_rows_with_and_without_the_ring(pkg, cabi, M, D, dtype):
+    """The same on both sides of the lines between rows that come through the ring and rows that do not: bf16 without a gate from 16 rows a block and seven
+    eighths of its vectors on, fp32 with a gate unless the row fills them."""
+    _norm_rows(pkg, M, D, dtype)
