@@ -26,7 +26,8 @@ inline EncodeTiledFn encode_fn() {
 }
 
 // A bf16 tensor map with boxes of 128-byte rows, 128-byte swizzle.  The encoder belongs to the driver and wants a current context, which a
-// thread that has not called the runtime yet does not have (autograd's, where the map is the first thing that a backward asks for).
+// thread that has not called the runtime yet does not have (autograd's, where the map is the first thing that a backward asks for).  Setting the
+// device that is set makes its context current, and is allowed while a stream is captured.
 inline bool encode_map(CUtensorMap* m, const void* base, cuuint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
@@ -36,7 +37,8 @@ inline bool encode_map(CUtensorMap* m, const void* base, cuuint32_t rank, const 
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     };
     CUresult r = encode();
-    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaFree(nullptr) == cudaSuccess) r = encode();  // (the runtime makes the device's context current)
+    int dev = 0;
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
     return r == CUDA_SUCCESS;
 }
 

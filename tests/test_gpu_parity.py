@@ -642,6 +642,52 @@ def test_gradients_of_many_heads_do_not_depend_on_the_batch(pkg, cabi, T, h, g):
             assert torch.equal(u, v[i:i + 1]), name
 
 
+_FIRST_BACKWARD = """
+import sys
+sys.path.insert(0, {root!r})
+import importlib, torch
+pkg = importlib.import_module("dhammic-ai_b200")
+cfg = pkg.shrink(pkg.CONFIGS[2], 1, 256)
+inp = pkg.make_inputs(cfg)
+names = ("x", "dt", "A_head", "B", "C", "D")
+lv = [inp[k].cuda().requires_grad_(True) for k in names]
+dy = inp["dy"].cuda()
+side = torch.cuda.Stream()
+torch.cuda.synchronize()
+with torch.cuda.stream(side):  # (a backward runs on its forward's stream)
+    y, _ = pkg.ssd_mamba2(*lv, cfg.chunk)
+    room = [torch.empty(64 << 20, dtype=torch.uint8, device="cuda")] + [torch.empty(512, device="cuda") for _ in range(600)]
+    del room
+torch.cuda.synchronize()
+if {capture}:
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        first = torch.autograd.grad([y], lv, [dy], retain_graph=True)
+    graph.replay()
+else:
+    with torch.cuda.stream(side):
+        first = torch.autograd.grad([y], lv, [dy], retain_graph=True)
+torch.cuda.synchronize()
+with torch.cuda.stream(side):
+    again = torch.autograd.grad([y], lv, [dy])
+torch.cuda.synchronize()
+assert all(torch.equal(u, v) for u, v in zip(first, again))
+print("same")
+"""
+
+
+@pytest.mark.parametrize("capture", [False, True])
+def test_first_backward_of_a_process(pkg, cabi, capture):
+    """The first backward, on an autograd thread that has not called the runtime yet and needs a context for its tensor maps: with room in the allocator, so that no
+    allocation binds one before, and inside a capture, where what binds it must be allowed.  In a process of its own, since only the first is of interest."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    code = _FIRST_BACKWARD.format(root=str(Path(__file__).resolve().parents[1]), capture=capture)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]
+
+
 def test_walk_in_one_piece_where_the_workspace_has_no_room(pkg, cabi):
     """With less workspace than several pieces need, but enough for one, the walks run in one; with a byte less they are refused."""
     cfg = replace(pkg.CONFIGS[2], batch=1, seqlen=4096, nheads=6, ngroups=2, chunk=128)
