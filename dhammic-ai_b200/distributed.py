@@ -544,39 +544,25 @@ def ssd_mamba2_sequence_parallel(x: Tensor, dt: Tensor, A_head: Tensor, B: Tenso
     return _SeqSplitSSD.apply(x, dt, A_head, B, C, D, int(chunk_size), initial_state, S, comm, backend)
 
 
-def _segments_pay(x: Tensor, B: Tensor, chunk_size: int, grads: bool) -> bool:
-    """Whether a call that leaves the number of segments open is better made as segments than as one call.
-
-    One call wins from five (batch, head) pairs on, whatever the length.  With fewer, what a head does alone grows with the sequence:
-    the last piece of its walk (the tcgen05 kernels cut it sixteen times at most), the sums over the positions of a head in the
-    backward of the fp32 and the partial-tile kernels, the recurrence over the chunks of the fp32 ones.  Segments cost the host 130 us
-    forward and 400 with gradients.  One call / segments, us, one sequence:
-      tcgen05, forward    65,536 x 4 heads 115 / 123    98,304 x 4 165 / 137      131,072 x 5 213 / 224
-               gradients  98,304 x 2 366 / 394          131,072 x 4 609 / 570     131,072 x 5 671 / 690
-      partial, forward    131,072 x 2 159 / 314         262,144 x 1 196 / 324
-      tiles    gradients  49,152 x 2 400 / 396          65,536 x 2 522 / 458      131,072 x 3 1,229 / 1,202     131,072 x 4 1,466 / 1,479
-      fp32,    forward    65,536 x 1 183 / 156, in chunks of 128 169 / 177        65,536 x 2 207 / 190 (d_state 16), 285 / 289 (64)
-               gradients  24,576 x 2 412 / 407          32,768 x 1 366 / 399, x 2 546 / 500    65,536 x 4 1,439 / 1,282 (16), 1,738 / 1,707 (64)
-                          98,304 x 6 2,921 / 2,830 (16), 3,466 / 3,679 (64)"""
+def _one_call(x: Tensor, B: Tensor, chunk_size: int, grads: bool) -> bool:
+    """Whether a call that leaves the number of segments open is made as one call: on the tcgen05 kernels, whose sums end at a tile's or a piece's end
+    either way.  The fp32 and the partial-tile kernels would be faster so as well (0.4 to 0.9 of the time from five (batch, head) pairs on), but sum up the decay's
+    gradients over a head's whole sequence: (1, 16384, 8 heads, 64), d_state 64, fp32, dA_head 7.0e-5 off against 5.1e-6 as segments,
+    ddt 1.4e-6 / 4.7e-7; 16 heads in bf16 5.0e-5 / 2.9e-6 and 6.4e-7 / 3.4e-7.
+    Up to four pairs of a very long sequence are faster as segments: the walks cut themselves sixteen times at most.  Segments cost the
+    host 130 us forward and 400 with gradients.  One call / segments, us:
+      forward    65,536 positions x 4 heads 115 / 123     98,304 x 4 165 / 137     131,072 x 5 213 / 224
+      gradients  98,304 x 2 366 / 394                     131,072 x 4 609 / 570    131,072 x 5 671 / 690"""
     b, T, h, p = x.shape
-    pairs = b * h
-    if pairs > 4:
-        return False
-    n = B.shape[3]
     shape = _op._make_shape(x, _cabi.F32, B, int(chunk_size))
-    path = _cabi.load().ssd_b200_resolve_path(C.byref(shape))
-    if path == _cabi.PATH_TC:
-        return T >= (131072 if grads else 98304)
-    if shape.path == _cabi.PATH_AUTO and x.dtype == torch.bfloat16 and 32 < p <= 64 and 32 < n <= 128 and p % 8 == 0 and n % 8 == 0:  # partial tiles
-        return grads and pairs <= 3 and T >= 65536
-    if grads:
-        return T >= 32768 and pairs * T >= 49152
-    return T // int(chunk_size) >= max(768, 512 * pairs) and pairs <= 3
+    if _cabi.load().ssd_b200_resolve_path(C.byref(shape)) != _cabi.PATH_TC:
+        return False
+    return b * h > 4 or T < (131072 if grads else 98304)
 
 
 def ssd_mamba2_segmented(x, dt, A_head, B, C, D, chunk_size, initial_state=None, segments: int = 0, backend=None):
-    """ssd_mamba2 with the sequence cut into `segments` pieces inside this GPU (0 = as the kernels cut it themselves, or into
-    as many as the shape wants where that is faster: a few heads of a very long sequence).
+    """ssd_mamba2 with the sequence cut into `segments` pieces inside this GPU (0 = as the kernels cut it themselves where that is faster
+    and as exact, see `_one_call`, or into as many as the shape wants).
 
     One call cuts its walks where the chip would idle and sums up only the pieces whose sum is read, in each direction as many as that
     direction wants; segments that the caller chooses are summed up whole in both.  Forward and backward, one call against eight or
@@ -585,7 +571,7 @@ def ssd_mamba2_segmented(x, dt, A_head, B, C, D, chunk_size, initial_state=None,
     if segments <= 0 and backend is None:
         _segments(segments, b, h, T, chunk_size)  # (a length that does not split is refused either way)
         ins = (x, dt, A_head, B, C, D, initial_state)
-        if not _segments_pay(x, B, chunk_size, torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ins)):
+        if _one_call(x, B, chunk_size, torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ins)):
             init = None if initial_state is None else initial_state.reshape(b, h, p, B.shape[3])
             return _op.ssd_mamba2(x, dt, A_head, B, C, D, int(chunk_size), init)
     return ssd_mamba2_sequence_parallel(x, dt, A_head, B, C, D, chunk_size, initial_state, comm=LoopbackComm(),

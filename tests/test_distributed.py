@@ -282,13 +282,12 @@ def test_segmented_scan_inside_one_gpu(pkg, cabi, idx, segments, tol):
     # the tcgen05 kernels: up to four pairs, with gradients from 131,072 positions on
     ("bf16", 1, 131072, 4, 64, 128, 4, 128, True, True), ("bf16", 2, 131072, 2, 64, 128, 1, 128, True, True), ("bf16", 1, 65536, 1, 64, 128, 1, 128, True, False),
     ("bf16", 1, 131072, 5, 64, 128, 1, 128, True, False), ("bf16", 1, 98304, 2, 64, 128, 1, 128, False, True), ("bf16", 1, 98304, 2, 64, 128, 1, 128, True, False),
-    # partial tiles: with gradients only
-    ("bf16", 1, 65536, 3, 64, 64, 1, 64, True, True), ("bf16", 1, 65536, 4, 64, 64, 1, 64, True, False), ("bf16", 1, 131072, 1, 64, 64, 1, 64, False, False),
-    # fp32, and bf16 with a headdim that the kernels for partial tiles do not take
-    ("fp32", 1, 32768, 2, 64, 16, 1, 64, True, True), ("fp32", 1, 32768, 1, 64, 16, 1, 64, True, False), ("bf16", 1, 131072, 4, 16, 8, 1, 64, True, True),
-    ("fp32", 1, 65536, 2, 64, 16, 1, 64, False, True), ("fp32", 1, 65536, 2, 64, 16, 1, 128, False, False), ("fp32", 1, 131072, 8, 64, 16, 1, 64, True, False)])
+    ("bf16", 1, 16384, 64, 64, 128, 8, 128, False, False),
+    # the kernels that sum up over a head's whole sequence: always
+    ("bf16", 1, 65536, 4, 64, 64, 1, 64, True, True), ("bf16", 1, 16384, 64, 64, 128, 1, 32, False, False), ("bf16", 2, 30720, 32, 64, 128, 1, 96, True, True),
+    ("fp32", 1, 16384, 8, 64, 64, 1, 64, True, True), ("fp32", 1, 16384, 8, 64, 64, 1, 64, False, True), ("bf16", 1, 16384, 32, 16, 8, 1, 64, True, True)])
 def test_which_segmented_calls_are_one_call(pkg, cabi, monkeypatch, dtype, b, T, h, p, n, g, l, grads, cut):
-    """segments = 0: one call, or segments where a few heads of a very long sequence would each walk alone."""
+    """segments = 0: one call on the tcgen05 kernels, segments on the others and where a few heads of a very long sequence would each walk alone."""
     D = importlib.import_module("dhammic-ai_b200.distributed")
     took = []
     monkeypatch.setattr(D._op, "ssd_mamba2", lambda *a, **k: took.append("one"))
@@ -320,6 +319,31 @@ def test_segments_of_a_few_heads_of_a_long_sequence(pkg, cabi, dtype, T, n, l):
         res.append([y, fs, *torch.autograd.grad(y, lv, dy)])
     for u, v in zip(*res):
         assert torch.equal(u, v)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,h", [("fp32", 4), ("bf16", 8)])
+def test_segmented_sums_do_not_run_over_the_whole_sequence(pkg, cabi, oracle, dtype, h):
+    """Decay gradients of a long sequence on the kernels that sum up over a call's whole sequence, without a number of segments, against 64 bits.  A running
+    sum over 16,384 positions is 5e-5 (dA_head) and 6e-7 to 1.4e-6 (ddt) off, sums over a segment 3e-6 to 5e-6 and 3e-7 to 5e-7; the bounds lie between."""
+    D = importlib.import_module("dhammic-ai_b200.distributed")
+    T, n, l = 16384, 64, 64
+    store = torch.bfloat16 if dtype == "bf16" else torch.float32
+    gen = torch.Generator(device="cuda").manual_seed(h)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device="cuda")
+    x, dy = randn(1, T, h, 64).to(store), randn(1, T, h, 64).to(store)
+    B, C = ((randn(1, T, 1, n) / n ** 0.5).to(store) for _ in range(2))
+    dt = torch.nn.functional.softplus(0.5 * randn(1, T, h) - 3.9).clamp_(1e-3, 0.1)
+    A = -torch.exp(2.77 * torch.rand(h, generator=gen, device="cuda"))
+    def grads(leaves, fn):
+        lv = [t.requires_grad_(True) for t in leaves]
+        return torch.autograd.grad(fn(*lv), lv[1:3], dy.to(lv[0].dtype))
+    got = grads([t.clone() for t in (x, dt, A, B, C)], lambda *v: D.ssd_mamba2_segmented(*v, None, l)[0])
+    want = grads([t.double() for t in (x, dt, A, B, C)], lambda x, dt, A, B, C: oracle.ssd_chunked(
+        x * dt.unsqueeze(-1), dt * A, B.expand(-1, -1, h, -1), C.expand(-1, -1, h, -1), l)[0])
+    off = [float((u.double() - v).norm() / v.norm()) for u, v in zip(got, want)]
+    assert off[0] < (6e-7 if dtype == "fp32" else 4.5e-7) and off[1] < 1.5e-5, off
 
 
 # ---------------------------------------------------------------------------------------------------------
