@@ -706,8 +706,8 @@ unsigned norm_blocks(size_t M, int rows_per_block, int most) {
 
 // Whether the backward of rows that are a block's takes them through the ring (NormBwd).  Gated bf16 rows always do (0.80 to 0.99 of the time without, at any
 // length), and so do fp32 rows without a gate (0.90 to 1.00); the others by what was measured, us without / with the ring:
-//   fp32 with a gate: not where the row fills the block's vectors (rows of a power of two, whose streams meet in the same DRAM banks the more
-//     the further ahead they are read).  (16384, 2048) 109.7 / 120.6, (16384, 4096) 206.9 / 218.8, (16384, 1024) 63.8 / 66.0, but (16384, 1536) 90.9 / 85.2, (16384, 3072) 170 / 161
+//   fp32 with a gate: not where the row fills the block's vectors (rows of a power of two; why further ahead is
+//     slower there was not found).  (16384, 2048) 109.7 / 120.6, (16384, 4096) 206.9 / 218.8, (16384, 1024) 63.8 / 66.0, but (16384, 1536) 90.9 / 85.2, (16384, 3072) 170 / 161
 //   bf16 without a gate: where few threads have no vector and a block walks many rows.  (16384, 4096) 84.6 / 82.7, (16384, 8192) 163.6 / 157.9, but
 //     (16384, 2088) 68.5 / 71.4, (2048, 4096) 21.4 / 21.8, (2048, 2048) 17.0 / 17.8
 template <class T>

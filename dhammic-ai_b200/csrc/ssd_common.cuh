@@ -14,7 +14,9 @@ struct Dims {
 __device__ __forceinline__ float to_f(float v) { return v; }
 // A bf16 value as fp32 by a mixed-precision addition (sm_100), which takes either half of a register as it is and runs at the rate of an fp32 one
 // (1.1 cycles a warp), where the shift or mask that makes an fp32 number of a half takes two, on the pipe that the conversions to bf16 need.  For the
-// element-wise kernels (gated norm's backward of (16384, 4096) 120 -> 111 us, rotation with the running angle 723 -> 696 at (16, 4096, 64 heads)); the
+// element-wise kernels (gated norm's backward of (16384, 4096) 120 -> 111 us, rotation with the running angle 723 -> 696 at (16, 4096, 64 heads), the rotation's
+// backward of pairs that are no whole vectors, (4, 2048, 24, 66), 57.6 -> 47.4 although it spills 20 bytes, its forward 30.2 both ways), and where the fp32
+// multiply-add kernels read bf16 rows that are no whole vectors (no difference: 970 -> 970 us forward and backward of (4, 1984, 20, 64), d_state 64); the
 // tile kernels, which wait for latencies, lose 1 % by it and keep shifts and masks.
 __device__ __forceinline__ float to_f(__nv_bfloat16 v) {
     float r;

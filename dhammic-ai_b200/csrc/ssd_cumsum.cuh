@@ -31,7 +31,8 @@ __device__ __forceinline__ void raise_flag(int* extreme, int beyond, int h) {
 }
 
 // The first block of a pass clears the status word (a memset of its own is a gap of 1.2 us and more on the stream, and what follows one is not
-// launched early).  What another block may write there comes at the earliest when a bounded wait of it runs out, a tenth of a second later.
+// launched early).  What may be written there in the same kernel: what a block finds wrong at its start, which every block does and so this one too, behind its
+// clearing; and that a bounded wait ran out, a tenth of a second later.
 __device__ __forceinline__ void clear_status(int* status) {
     if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) *status = 0;
 }

@@ -278,7 +278,7 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
         extreme = (int*)(tcum + 3 * bht);
     }
     if (!a->cumsum_is_input && !aux_valid && d.l <= kFusedChunkMax) {
-        // the within-chunk cumulative sums, the tile-cumulative log2 copies, the transposes and the flag in one kernel
+        // the within-chunk cumulative sums, the tile-cumulative log2 copies, the transposes and the flags in one kernel
         if (int rc = launch_cumsum_tile_fused(a, d, a->a_cumsum, tcum, dtT, skipT, extreme, status, st, err, errn)) return rc;
     } else {
         if (!a->cumsum_is_input) {
@@ -355,7 +355,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
     float* dinit = a->dinit ? a->dinit : (float*)(ws + w.dinit);
     int* extreme = (int*)(ws + w.dAh_part);  // (written again behind the kernels that read the flags)
     float* skipT = a->skip ? (float*)(ws + w.skipT) : nullptr;
-    if (a->states) {  // the forward left the arrays and the flag behind the tile states
+    if (a->states) {  // the forward left the arrays and the flags behind the tile states
         tcum = (float*)((uintptr_t)a->states + tile_states_bytes(d));
         dtT = a->dt ? tcum + bht : nullptr;
         skipT = a->skip ? tcum + 2 * bht : nullptr;

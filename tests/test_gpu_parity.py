@@ -603,10 +603,12 @@ def test_unaligned_tensors_through_the_c_abi(pkg, cabi, dtype, n, g, shifted):
         assert [rc == cabi.EINVAL for rc in rcs] == refused
 
 
-@pytest.mark.parametrize("b,T,h,g", [(1, 4096, 64, 2), (1, 4480, 64, 8), (2, 3968, 36, 3), (1, 8192, 148, 74)])
+@pytest.mark.parametrize("b,T,h,g", [(1, 4096, 64, 2), (1, 4480, 64, 8), (2, 3968, 36, 3), (1, 4096, 64, 32)])
 def test_reverse_walk_in_pieces_of_two_heads(pkg, cabi, b, T, h, g):
     """Sequences whose reverse walk is cut into pieces with two heads of a group per CTA (whole last pieces and short ones, two heads per group): the same
-    as in one piece, which is what a call with room for no more takes.  States and gradients are bf16 sums of the same terms in another order."""
+    as in one piece, which is what a call with room for no more takes.  States and gradients are bf16 sums of the same terms in another order.  The
+    summaries launched say what was cut: the forward's walk, the same walk in the backward, and the reverse one."""
+    import ctypes
     cfg = replace(pkg.CONFIGS[2], batch=b, seqlen=T, nheads=h, ngroups=g, chunk=128)
     inp = pkg.make_inputs(cfg, seed=8)
     def up(v):
@@ -615,9 +617,18 @@ def test_reverse_walk_in_pieces_of_two_heads(pkg, cabi, b, T, h, g):
     bht, state = up(bh * T * 4), up(bh * 64 * 128 * 4)
     fwd = 256 + 3 * bht
     bwd = fwd + 2 * up(bh * nt * 64 * 128 * 2) + 2 * state + 3 * bht + up(bh * nt * 32) + 2 * up(bh * nt * 4)
-    rc0, want = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, {cabi.PASS_FWD: fwd, cabi.PASS_BWD: bwd})
-    rc1, got = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO)
-    assert rc0 == rc1 == [0, 0]
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, b, T, h, 64, 128, g, 128)
+    assert cabi.load().ssd_b200_workspace_bytes(ctypes.byref(shape), cabi.PASS_BWD) > bwd
+    def passes(*room):
+        cabi.profile_enable(True)
+        try:
+            rcs, out = _cabi_passes(pkg, cabi, cfg, inp, (), cabi.PATH_AUTO, *room)
+            return rcs, out, cabi.profile_read().get("tc_summary", (0.0, 0))[1]
+        finally:
+            cabi.profile_enable(False)
+    rc0, want, whole = passes({cabi.PASS_FWD: fwd, cabi.PASS_BWD: bwd})
+    rc1, got, cut = passes()
+    assert rc0 == rc1 == [0, 0] and (whole, cut) == (0, 3)
     for k in want:
         assert rel_err(got[k], want[k]) < TOL_BF16, k
 
@@ -1166,10 +1177,10 @@ def test_mamba3_angle_sums_do_not_depend_on_the_route(pkg, cabi, T, h, n, b, dty
     assert rel_err(res[0][0], want) < TOL_FP32
 
 
-@pytest.mark.parametrize("h,chunk", [(3, 64), (9, 256), (33, 128)])
+@pytest.mark.parametrize("h,chunk", [(3, 64), (9, 256), (17, 64), (24, 256), (33, 128)])
 def test_cumulative_sums_in_blocks_of_eight_and_of_32_heads(pkg, cabi, h, chunk):
-    """512 blocks of 32 heads and more against a batch entry alone, whose blocks have eight: the sums have the same bits, also where a chunk
-    begins in an earlier tile, and the decay gradients, taken from both kinds of blocks, agree (the walks are cut differently)."""
+    """512 tiles in blocks of 32 heads (of eight where half of 32 would be none) against a batch entry alone, whose blocks have eight: the sums have the same bits, also
+    where a chunk begins in an earlier tile, and the decay gradients agree (the walks are cut differently)."""
     b, T = 16, 4096
     gen = torch.Generator(device=DEV).manual_seed(h)
     x, B, C, dy = (torch.randn(b, T, *s, generator=gen, device=DEV).bfloat16() for s in ((h, 64), (1, 128), (1, 128), (h, 64)))
@@ -1246,6 +1257,38 @@ def test_mamba3_angle_gradient_does_not_depend_on_the_batch(pkg, cabi, T):
         return y.detach(), torch.autograd.grad([y], [part[6]], [dy[:k]])[0]
     (y0, d0), (y1, d1) = dang(b), dang(1)
     assert torch.equal(y0[:1], y1) and torch.equal(d0[:1], d1)
+
+
+@pytest.mark.parametrize("T", [1, 7, 9, 55, 57, 129, 601])
+@pytest.mark.parametrize("ang32", [True, False])
+@pytest.mark.parametrize("h,n,b", [(19, 20, 200), (19, 10, 400)])
+def test_mamba3_reverse_sum_at_its_edges(pkg, cabi, T, ang32, h, n, b):
+    """The reverse sum of the angle gradients in one pass: lengths that are no multiple of the eight positions fetched together, fewer than the 56 fetched
+    ahead, ends inside a segment; columns that fill part of a block; and an odd number of columns, which takes two passes.  The same bits as a
+    batch entry alone, whose columns are too few for one pass, and fp32 sums of up to 601 terms against 64 bits (bf16: one rounding)."""
+    import ctypes
+    lib, S = cabi.load(), pkg.ssd_scan
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    B, C, dBr, dCr = (randn(b, T, k, n).bfloat16() for k in (1, 1, h, h))
+    cum, dt, lam, dyx = randn(b, T, h, n // 2), torch.rand(b, T, h, generator=gen, device=DEV), torch.rand(b, T, h, generator=gen, device=DEV), randn(b, T, h)
+    P = S._ptr
+    def run(k):
+        ins = [t[:k].contiguous() for t in (dt, lam, B, C, cum, dBr, dCr, dyx)]
+        shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, k, T, h, 64, n, 1, T)
+        dB, dC, dcum = torch.empty_like(ins[2]), torch.empty_like(ins[3]), torch.empty_like(ins[4])
+        dang = torch.empty(k, T, h, n // 2, dtype=torch.float32 if ang32 else torch.bfloat16, device=DEV)
+        sdot, dw, seg = torch.zeros(k, T, 1, device=DEV), torch.zeros(k, T, h, device=DEV), torch.empty(k * ((T + 127) // 128) * h * (n // 2), device=DEV)
+        cabi.check(lib.ssd_b200_m3_prologue_bwd(ctypes.byref(shape), None, None, P(ins[0]), P(ins[1]), None, P(ins[2]), P(ins[3]), P(ins[4]), P(sdot), None, P(ins[5]),
+                                                P(ins[6]), None, P(dw), P(ins[7]), P(dB), P(dC), P(dang), cabi.F32 if ang32 else cabi.BF16, P(dcum), P(seg),
+                                                S._stream(torch.device(DEV))))
+        torch.cuda.synchronize()
+        return dcum, dang
+    (dcum, dang), (_, alone) = run(b), run(1)
+    assert torch.equal(dang[:1], alone)
+    want = -dcum.double().flip(1).cumsum(1).flip(1)
+    assert ((dang.double() - want).abs() <= (0.0 if ang32 else 2.0 ** -8) * want.abs() + 1e-5 * want.abs().max()).all()
 
 
 def test_mamba3_against_reference_fixture(pkg, cabi):
