@@ -545,19 +545,30 @@ def ssd_mamba2_sequence_parallel(x: Tensor, dt: Tensor, A_head: Tensor, B: Tenso
 
 
 def _one_call(x: Tensor, B: Tensor, chunk_size: int, grads: bool) -> bool:
-    """Whether a call that leaves the number of segments open is made as one call: on the tcgen05 kernels, whose sums end at a tile's or a piece's end
-    either way.  The fp32 and the partial-tile kernels would be faster so as well (0.4 to 0.9 of the time from five (batch, head) pairs on), but sum up the decay's
-    gradients over a head's whole sequence: (1, 16384, 8 heads, 64), d_state 64, fp32, dA_head 7.0e-5 off against 5.1e-6 as segments,
-    ddt 1.4e-6 / 4.7e-7; 16 heads in bf16 5.0e-5 / 2.9e-6 and 6.4e-7 / 3.4e-7.
-    Up to four pairs of a very long sequence are faster as segments: the walks cut themselves sixteen times at most.  Segments cost the
-    host 130 us forward and 400 with gradients.  One call / segments, us:
-      forward    65,536 positions x 4 heads 115 / 123     98,304 x 4 165 / 137     131,072 x 5 213 / 224
-      gradients  98,304 x 2 366 / 394                     131,072 x 4 609 / 570    131,072 x 5 671 / 690"""
+    """Whether a call that leaves the number of segments open is made as one call.
+
+    With gradients only on the tcgen05 kernels, whose sums end at a tile's or a piece's end either way.  The fp32 and the partial-tile kernels would be faster so
+    as well (0.4 to 0.9 of the time from five (batch, head) pairs on), but sum up the decay's gradients over a head's whole sequence: (1, 16384, 8 heads, 64),
+    d_state 64, fp32, dA_head 7.0e-5 off against 5.1e-6 as segments, ddt 1.4e-6 / 4.7e-7; 16 heads in bf16 5.0e-5 / 2.9e-6 and 6.4e-7 / 3.4e-7.  Outputs and final
+    state are as exact in one call (the fp32 state 3.1e-7 off either way, that of partial tiles 1.5e-7 against 3.1e-7).
+    A few pairs of a very long sequence are faster as segments: the walks of the tcgen05 kernels cut themselves sixteen times at most, the fp32 kernels take the chunks
+    of a head one after the other.  Segments cost the host 130 us forward and 400 with gradients.  One call / segments, us:
+      tcgen05, forward    65,536 positions x 4 heads 115 / 123     98,304 x 4 165 / 137     131,072 x 5 213 / 224
+               gradients  98,304 x 2 366 / 394                     131,072 x 4 609 / 570    131,072 x 5 671 / 690
+      partial tiles, forward   131,072 x 2 159 / 314               262,144 x 1 196 / 324
+      fp32, forward       65,536 x 1 183 / 156, in chunks of 128 169 / 177     65,536 x 2 207 / 190 (d_state 16), 285 / 289 (64)     98,304 x 4 538 / 542"""
     b, T, h, p = x.shape
-    shape = _op._make_shape(x, _cabi.F32, B, int(chunk_size))
-    if _cabi.load().ssd_b200_resolve_path(C.byref(shape)) != _cabi.PATH_TC:
+    pairs = b * h
+    if pairs > 4 and not grads:
+        return True
+    n, shape = B.shape[3], _op._make_shape(x, _cabi.F32, B, int(chunk_size))
+    if _cabi.load().ssd_b200_resolve_path(C.byref(shape)) == _cabi.PATH_TC:
+        return pairs > 4 or T < (131072 if grads else 98304)
+    if grads:
         return False
-    return b * h > 4 or T < (131072 if grads else 98304)
+    if shape.path == _cabi.PATH_AUTO and x.dtype == torch.bfloat16 and 32 < p <= 64 and 32 < n <= 128 and p % 8 == 0 and n % 8 == 0:  # partial tiles
+        return True
+    return pairs > 3 or T // int(chunk_size) < max(768, 512 * pairs)
 
 
 def ssd_mamba2_segmented(x, dt, A_head, B, C, D, chunk_size, initial_state=None, segments: int = 0, backend=None):
