@@ -105,15 +105,6 @@ __global__ void __launch_bounds__(256) tile_cumsum_kernel(const float* __restric
 }
 
 // ------------------------------------------------------------------------------------------
-// The same from the per-position log-decay itself (dt * A_head, or `a` as given, fp32 or bf16), which is read once in the
-// caller's (b,T,h) layout through a shared-memory transpose and scanned inside each tile (warp per head, 32-lane segments
-// scanned side by side); also writes a_cumsum (b,h,c,l) in natural-log units, where one is wanted (a backward without
-// kept states runs this too, so that its per-position arrays have the forward's bits).  Chunks of any length: where one
-// ends inside the tile its sums come from a second, segmented scan of the same values (CUT), so that they carry no
-// rounding of the positions before the chunk; where a chunk began in an earlier tile, the block adds up the positions
-// between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
-// kernels this replaces: 28 -> 7 us at (8, 2048, 24) with chunks of 64).  The skip array is transposed in a second round
-// through the panel of the log-decay.
 // A thread's values of every `step`-th row, zeros from row `rows` on: a loop of its own, so that every load is issued before a value is used.  (Left to the
 // compiler in one loop with the stores to shared memory, the loads went out one after the other or all at once as the rest of the kernel had it: 104 us or 123 at
 // (4, 131072, 64 heads), 94 so.)
@@ -123,9 +114,17 @@ __device__ __forceinline__ void load_column(float (&v)[N], const TV* p, int step
     for (int q = 0; q < N; ++q) v[q] = q * step < rows ? to_f(p[(size_t)q * step * h]) : 0.f;
 }
 
-// HB heads to a block: 32, whose reads are whole 128-byte rows, or 8 where blocks of 32 would be too few to fill the chip: a block then has a
-// quarter of the loads and one head a warp instead of four (kFewCumsumBlocks): 4 blocks of 32 heads 4.9 us, in blocks of 8 3.2; 256 blocks 7.6 / 6.6, 1024
-// 15.4 / 16.8.
+// The same from the per-position log-decay itself (dt * A_head, or `a` as given, fp32 or bf16), which is read once in the
+// caller's (b,T,h) layout through a shared-memory transpose and scanned inside each tile (warp per head, 32-lane segments
+// scanned side by side); also writes a_cumsum (b,h,c,l) in natural-log units, where one is wanted (a backward without
+// kept states runs this too, so that its per-position arrays have the forward's bits).  Chunks of any length: where one
+// ends inside the tile its sums come from a second, segmented scan of the same values (CUT), so that they carry no
+// rounding of the positions before the chunk; where a chunk began in an earlier tile, the block adds up the positions
+// between (kFusedChunkMax bounds that second read, at most the chunk, against a launch and a pass over a_cumsum for the two
+// kernels this replaces: 28 -> 7 us at (8, 2048, 24) with chunks of 64).  The skip array is transposed in a second round
+// through the panel of the log-decay.
+// HB heads to a block: see kFewCumsumBlocks.  Registers for five blocks on an SM, four with CUT: with six the loads no longer fit at once (92 -> 102 us at
+// (4, 131072, 64 heads)), with CUT five are 121 us and four 117.
 template <bool CUT, int HB>
 __global__ void __launch_bounds__(256, CUT ? 4 : 5) cumsum_tile_fused_kernel(const void* __restrict__ a, int a_is_bf16,
                                                                 const float* __restrict__ dt, const float* __restrict__ A_head,

@@ -4,7 +4,8 @@
 y, dx, ddt, dB, dC (and dA_head, dD) into pinned host buffers.  The batch is cut into micro-batches and three
 CUDA streams overlap the host->device copies of micro-batch i+1, the kernels of micro-batch i and the
 device->host copies of micro-batch i-1, so that a step costs about max(copy-in, compute, copy-out) instead
-of their sum.  Batch entries are independent scans, so slicing the batch changes no result; the per-head
+of their sum.  Batch entries are independent scans, so slicing the batch changes no result (micro-batches of 75
+(batch, head) pairs and more give the bits of the whole batch; walks of fewer are cut into pieces, whose sums round differently); the per-head
 gradients dA_head and dD are summed over the micro-batches on the device.
 
 This is the end-to-end path ``bench.py`` times (``e2e``): it goes through the public operator
