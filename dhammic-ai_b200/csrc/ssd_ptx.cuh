@@ -86,8 +86,11 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait.  Returns false (and leaves *failed set) when the limit is reached or when another
 // wait of this block has already given up, so a broken pipeline drains quickly instead of spinning.
+// Not unrolled: left to itself the compiler writes four polls for every wait, and the tile kernels, whose warps run some ten loops at once, no
+// longer fit the instruction cache.
 constexpr uint32_t kSpinLimit = 4u << 20;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = kSpinLimit) {
+#pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 1023u) == 1023u && *failed) return false;
@@ -98,6 +101,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 
 // The same for phases that other threads complete with mbarrier.arrive: polls without suspending.
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = 16u * kSpinLimit) {
+#pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_test_wait(bar, parity)) return true;
         if ((i & 4095u) == 4095u && *failed) return false;
@@ -127,6 +131,12 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(col), "r"(head), "r"(pos), "r"(batch)
         : "memory");
 }
+// `bytes` of contiguous memory, both addresses and the size multiples of 16.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
 // The store of such a box; what lies outside the tensor is not written.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* smem_src, int col, int head, int pos, int batch) {
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map),
@@ -139,8 +149,9 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
                  : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_read() {  // smem source may be reused
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+template <int N = 0>
+__device__ __forceinline__ void tma_store_wait_read() {  // smem source of all but the last N groups may be reused
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Four bytes global -> shared without a register in between (generic proxy); wait_all covers the caller's own copies.

@@ -4,38 +4,49 @@
 // (64 x 128, fp32) in registers; more than one piece where (batch, head) pairs alone leave most of the chip idle (Pieces,
 // ssd_tc_host.cuh).  Per tile k (V = B, U = x, C of the tile; H = state entering it; S_k = its total log2-decay):
 //   S  = C V^T                     issued one tile ahead into a double-buffered TMEM accumulator
+//   Hl = V^T (d dt o U)            the tile's contribution to the state, one tile ahead; the weighted copy of U is made by the rows
 //   Yo = C H^T                     the entering state's part of the output
-//   Hl = V^T (d dt o U)            the tile's contribution to the state; the weighted copy of U is made by the rows
 //   G' = S o L o dt  (bf16 pairs, written back to TMEM by the rows),  Yd = G' U   (A operand from TMEM)
 //   y  = e o Yo + Yd + skip o x,   H <- 2^{S_k} H + Hl
 // 16 row warps: thread = (row, column quarter).  A quarter is one 32-column block of the causal mask (active iff
-// quarter <= row block), 16 columns of every 64-wide accumulator and 16 values of the row's state.  (With two threads per
-// row every per-tile step of a row thread was twice as long; the per-tile chain weighted copy -> mask -> Yd -> output is
-// what bounds the kernel.)  A control warpgroup holds the lane that issues every tcgen05.mma and, in another warp, the
-// lane that issues every TMA copy: the issuing lane of a product is held about as long as the product runs, so it
-// does nothing else.  The kernel starts at 96 registers per thread; the control warpgroup gives registers back and the
-// row warps take them (setmaxnreg).  Loads are double-buffered (80 KB per tile: the group's B and C panels and the
-// head's x); the state update runs as soon as Hl is done, while Yd still runs.
+// quarter <= row block), 16 columns of every 64-wide accumulator and 16 values of the row's state.  Four control warps: one lane of each issues
+// copies or products.  The kernel starts at 96 registers per thread; the control warpgroup gives registers back and the
+// row warps take them (setmaxnreg).
 //
-// Shared memory: 2 stages of [V panels 0,1 | U | C panels 0,1] | weighted U | state (bf16 [n][p]) | y staging |
-// per-column arrays.  TMEM: S double-buffered [0,256), G' [256,320), Yd [320,384), Yo [384,448), Hl [448,512).
+// What bounds it is the chain of a tile's steps and, with every SM busy, the clock, which falls from 1.9 to 1.6 GHz.  A tile's chain is
+// mask -> state update, beside Yd -> output; everything else runs ahead:
+//   * x has a ring of its own, three tiles deep; its weighted copy for tile k+1 is made while Yd of tile k runs, so that Hl and Yo of a tile are done
+//     when its mask is.  B and C, whose last reader Yo runs early in their tile, have two stages that are refilled from there on.
+//   * A lane that waits has to let the products it has issued drain first (some 300 cycles), so products that wait for different things are
+//     issued by different warps; and an mbarrier arrive reaches a polling lane some 300 cycles later, a hardware barrier 30, so the row warps
+//     hand over by bar.arrive.
+//   * All loops that run at once (16 row warps, four control warps) have to fit the instruction cache: with the waits
+//     unrolled by the compiler the pipeline above was slower than one without any of this, 315 us against 286 for 148 walks of 128 tiles.
+// (16, 4096, 64 heads, 8 groups): 520 -> 427 us, 512 -> 389 without kept states; (8, 2048, 24) 85 -> 64; one walk of 128 tiles to every other SM
+// 280 -> 184.  Tried and slower: the state on eight warps and mask and output on the other eight (500 us: the masks of the rows 96-127 take two
+// warps 1,500 cycles and four 1,000); Yd in two halves as the masks complete (its lane drains in between).
 //
-// mbarriers (phase = tile parity unless noted):
-//   bar_ld[s]  TMA bytes of stage s landed                        (phase = (tile / 2) & 1)
-//   bar_s      S of the tile is in TMEM                           (products -> row warps)
-//   bar_u      weighted rows written, one arrival per warp         (row warps -> products)
-//   bar_g      masked operand written, one arrival per warp        (row warps -> products)
-//   bar_mh     Yo and Hl of the tile have completed               (products -> row warps)
-//   bar_m2     every product of the tile has completed            (products -> row warps, TMA lane: stage free)
-//   bar_h      accumulators read, new state written, one per warp (row warps -> products, TMA lane)
-//   bar_sr     the stores of the tile before have read sH / sY    (TMA lane -> products)
+// Shared memory: 2 stages of [V panels 0,1 | C panels 0,1] | x ring, y staged in place | weighted x | state (bf16 [n][p]) |
+// per-position scalars of the ring's tiles, copied with x | column factors | barriers.  TMEM: S double-buffered [0,256), G' [256,320), Yd [320,384),
+// Yo [384,448), Hl [448,512).
+//
+// mbarriers (s = tile & 1, phase = (tile / 2) & 1 unless noted):
+//   bar_vc[s]  B and C of the tile landed
+//   bar_mh[s]  Hl and Yo of the tile have completed, the store of its entering state has read sH, x of the next tile landed (-> row warps,
+//              loads of B and C)
+//   bar_m2     Yd of the tile and S of the next have completed     (-> row warps; phase = tile parity)
+//   bar_s0, bar_x0   S and x of the first tile
+// Named barriers (row warps arrive, control warps wait):
+//   kBarU   weighted rows of a tile and the state entering it written, Hl and Yo of the tile before read (-> Hl, Yo, store of the state)
+//   kBarG   masked operand written                                  (-> Yd)
+//   kBarH   y staged over x, the tile's x and scalars no longer used (-> store of y, next load into the slot; two by tile parity: the row warps
+//           may arrive once more before the store's warp has seen the last one)
 // The per-half-row sums of y^2 keep their (b, T/128, h, 2, 128) layout: the odd quarter of each half leaves its partial
-// in shared memory, the even quarter adds its own and writes the sum after the block barrier at the top of the next tile.
+// in shared memory, the even quarter adds its own and writes the sum during the next tile.
 //
 // The diagonal block of the mask is evaluated entry by entry (one exponential each, by four of the ten warps that have a block to mask), which holds for any log-decay; below it
 // the mask is the product of a row and a column factor, both at most 1.  (A second instantiation with factors in the diagonal block as well, and a
-// flag that chose between the two on the device, was no faster, 515 against 516 us at (16, 4096, 64 heads), and the idle one of the
-// two took 2.3 to 7 us a call.)
+// flag that chose between the two on the device, was no faster, and the idle one of the two took 2.3 to 7 us a call.)
 #pragma once
 
 namespace ssd {
@@ -44,7 +55,14 @@ namespace tc {
 constexpr int kFwdThreads = 640;
 constexpr int kFwdRegsLaunch = 96, kFwdRegsRow = 104, kFwdRegsCtl = 64;
 static_assert(512 * kFwdRegsRow + 128 * kFwdRegsCtl <= kFwdThreads * kFwdRegsLaunch, "register trade exceeds the CTA's pool");
-constexpr size_t kFwdSmem = WalkCfg<0>::SMEM + 4 * LT * 4;  // + partial sums of y^2 [2][2][128]
+constexpr uint32_t kFwdStageBytes = 4 * PANEL;  // V panels 0,1 | C panels 0,1
+constexpr int kFwdStages = 2, kFwdRing = 3;
+// stages | x ring (y staged in place) | weighted x, state | per ring slot: cumulative decay, dt, skip coefficient [128] each | column factors of
+// each row warp [16][32] | partial sums of y^2 [2][2][128] | barriers
+constexpr size_t kFwdSmem = kFwdStages * (size_t)kFwdStageBytes + (kFwdRing + 2) * (size_t)PANEL + (3 * kFwdRing + 4 + 4) * LT * 4 + 192;
+// named barriers: all row warps arrive, one or three control warps wait
+constexpr int kBarG = 1, kBarU = 2, kBarH = 3 /* and 4 */, kBarRows = 5;
+static_assert(kFwdSmem <= 227 * 1024, "more shared memory than a CTA can have");
 
 // 16 fp32 values of (row, quarter) as two 16-byte chunks of a 128-byte-swizzled [row][64] bf16 panel
 __device__ __forceinline__ void store_quarter_row(uint8_t* panel, int row, int chunk0, const float (&v)[16]) {
@@ -62,23 +80,26 @@ __device__ __forceinline__ void store_quarter_row(uint8_t* panel, int row, int c
 __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constant__ WalkParams P) {
     dep_wait();
     if (P.zero_status) clear_status(P.status);
-    using Cfg = WalkCfg<0>;
-    constexpr int NST = Cfg::NST;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* sStage = sm;                                  // per stage: V panels 0,1 | U | C panels 0,1
-    uint8_t* sUd = sStage + (size_t)NST * Cfg::STAGE_BYTES;  // weighted copy of U
+    // no static shared memory: the dynamic region starts at the CTA's shared-memory base
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* sStage = smem_raw;                            // per stage: V panels 0,1 | C panels 0,1
+    uint8_t* sRing = sStage + kFwdStages * kFwdStageBytes; // x; y is staged over it
+    uint8_t* sUd = sRing + kFwdRing * PANEL;               // weighted copy of x
     uint8_t* sH = sUd + PANEL;                             // state, bf16, [n][p]
-    uint8_t* sY = sH + PANEL;                              // y staging
-    float* scum2 = reinterpret_cast<float*>(sY + PANEL);   // [2][128]
-    float* sf = scum2 + 2 * LT;                            // [2][128] column factors dt_j 2^(cend - c_j)
-    float* sdtc = sf + 2 * LT;                             // [2][128] dt_j
-    float* sysq = sdtc + 2 * LT;                           // [2][2][128] partial sums of y^2 of the odd quarters
-    __shared__ uint64_t bar_ld[2], bar_s, bar_u, bar_g, bar_mh, bar_m2, bar_h, bar_sr;
-    __shared__ uint32_t tmem_slot;
-    __shared__ int failed, rows_nt;
+    float* scum = reinterpret_cast<float*>(sH + PANEL);    // [ring][3][128] tile-cumulative log2-decay, dt, skip coefficient
+    float* sf = scum + 3 * kFwdRing * LT;                  // [16][32] column factors dt_j 2^(cend - c_j) of each row warp's block
+    float* sysq = sf + 4 * LT;                             // [2][2][128] partial sums of y^2 of the odd quarters
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sysq + 4 * LT);
+    uint64_t *bar_vc = bars, *bar_mh = bars + 2, *bar_m2 = bars + 4, *bar_s0 = bars + 5, *bar_x0 = bars + 6;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 7);
+    int& failed = *reinterpret_cast<int*>(bars + 8);
+    int& rows_nt = *reinterpret_cast<int*>(bars + 9);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (smem_u32(smem_raw) & 1023u) {  // the swizzled panels need a 1024-byte aligned base: report instead of computing garbage
+        if (tid == 0) atomicExch(P.status, 2);
+        return;
+    }
     const int hh = blockIdx.x, bb = blockIdx.y;
     const int gg = hh / P.hpg;
     const size_t bh = (size_t)bb * P.h + hh;
@@ -87,15 +108,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     if (tid == 0) {
         failed = 0;
         rows_nt = nt;
-        mbar_init(&bar_ld[0], 1);
-        mbar_init(&bar_ld[1], 1);
-        mbar_init(&bar_s, 1);
-        mbar_init(&bar_u, 16);
-        mbar_init(&bar_g, 16);
-        mbar_init(&bar_mh, 1);
-        mbar_init(&bar_m2, 1);
-        mbar_init(&bar_h, 16);
-        mbar_init(&bar_sr, 1);
+        for (int i = 0; i < 7; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 4 : i == 4 ? 2 : 1);  // mh: Hl, Yo, the store of the state, the next tile's x; m2: Yd, the next S
         mbar_fence_init();
     }
     if (warp == 16) {
@@ -106,6 +119,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     // state row of this thread: n = row, p in [16 q, 16 q + 16)
     float H[16];
     if (warp < 16) {
+        for (int i = tid; i < kFwdRing * LT; i += 512) scum[(3 * (i / LT) + 1) * LT + i % LT] = 1.f;  // (without dt)
         load_piece_row<false>(P, bh, row, q * 16, H);
         store_quarter_row(sH, row, q * 2, H);
         fence_async_smem();
@@ -116,104 +130,140 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     const uint32_t tm = tmem_slot;
     // S double-buffered [0,256), masked operand (bf16 pairs) [256,320), Yd [320,384), Yo [384,448), Hl [448,512)
     const uint32_t tG = tm + 256, tYd = tm + 320, tYo = tm + 384, tHl = tm + 448;
-    auto state_row = [&](int it) {  // row of tile `it` of this walk in the [b*nt*h*128][64] state tensor
-        return (int)((((size_t)bb * P.nt + k0 + it) * P.h + hh) * DN);
-    };
-
     if (warp >= 16) {
         setmaxnreg_dec<kFwdRegsCtl>();
-        if (warp == 16 && lane == 0) {
-            // ------------------------------------------------------------------ product lane: every tcgen05.mma
-            const uint32_t hMN = desc_lo(smem_u32(sH), PANEL), udMN = desc_lo(smem_u32(sUd), PANEL);
-            const uint32_t stK = desc_lo(smem_u32(sStage), 16), stMN = desc_lo(smem_u32(sStage), PANEL);
-            constexpr uint32_t PU = PANEL >> 4, SU = Cfg::STAGE_BYTES >> 4;  // panel and stage pitch in 16-byte units
-            auto offK = [](int kk) { return (uint32_t)(((kk >> 2) * (int)PANEL + (kk & 3) * 32) >> 4); };
-            auto offMN = [](int kk) { return (uint32_t)(kk * 128); };
-            auto fresh = [](uint32_t v) {  // keeps the descriptors from being hoisted out of the tile loop (64 registers here)
-                asm volatile("" : "+r"(v));
-                return v;
-            };
-            auto issue_S = [&](int it) {  // S = C B^T of tile `it` into TMEM buffer it & 1
-                const uint32_t vK = fresh(stK + (uint32_t)(it % NST) * SU), cK = vK + 3 * PU, tS = tm + (it & 1) * 128;
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk) mma_ss_lo(tS, cK + offK(kk), vK + offK(kk), kIdescS, kk > 0);
-                mma_commit(&bar_s);
-            };
+        const uint32_t stK = desc_lo(smem_u32(sStage), 16), stMN = desc_lo(smem_u32(sStage), PANEL);
+        constexpr uint32_t PU = PANEL >> 4, SU = kFwdStageBytes >> 4;  // panel and stage pitch in 16-byte units
+        auto offK = [](int kk) { return (uint32_t)(((kk >> 2) * (int)PANEL + (kk & 3) * 32) >> 4); };
+        auto offMN = [](int kk) { return (uint32_t)(kk * 128); };
+        auto fresh = [](uint32_t v) {  // keeps the descriptors from being hoisted out of the tile loop (64 registers here)
+            asm volatile("" : "+r"(v));
+            return v;
+        };
+        auto load_vc = [&](int it) {
+            uint8_t* st = sStage + (size_t)(it & 1) * kFwdStageBytes;
+            uint64_t* bar = &bar_vc[it & 1];
+            mbar_expect_tx(bar, kFwdStageBytes);
+            const int pos = (k0 + it) * LT;
+            tma_load_4d(st, &P.mV, bar, 0, gg, pos, bb);
+            tma_load_4d(st + PANEL, &P.mV, bar, 64, gg, pos, bb);
+            tma_load_4d(st + 2 * PANEL, &P.mC, bar, 0, gg, pos, bb);
+            tma_load_4d(st + 3 * PANEL, &P.mC, bar, 64, gg, pos, bb);
+        };
+        if (warp == 16) {
+            // ------------------------------------------------------------------ products: Yd
+            const uint32_t xMN = desc_lo(smem_u32(sRing), PANEL);
+            int r = 0;  // it % 3
             for (int it = 0; it < nt; ++it) {
-                const int s = it % NST;
-                const uint32_t ph = it & 1;
-                mbar_wait(&bar_ld[s], (it / NST) & 1, &failed);
-                const uint32_t vMN = fresh(stMN + (uint32_t)s * SU), uMN = vMN + 2 * PU, cK = fresh(stK + (uint32_t)s * SU + 3 * PU);
-                const uint32_t hMN_ = fresh(hMN), udMN_ = fresh(udMN);
-                if (it == 0) {
+                __syncwarp();
+                named_barrier(kBarG, 544);
+                if (lane == 0) {
                     tc_fence_after();
-                    issue_S(0);
+                    const uint32_t uMN = fresh(xMN + (uint32_t)r * PU);
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk)  // Yd = G' x : A in TMEM (K = j), B = x [j][p] MN-major
+                        mma_ts_lo(tYd, tG + kk * 8, uMN + offMN(kk), kIdescKM, kk > 0);
+                    mma_commit(bar_m2);
                 }
-                if (it > 0) mbar_wait_spin(&bar_h, (it - 1) & 1, &failed);  // new state in sH, accumulators free
-                tc_fence_after();
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)  // Yo = C H^T : A = C K-major, B = the running state in sH, [n][p] MN-major
-                    mma_ss_lo(tYo, cK + offK(kk), hMN_ + offMN(kk), kIdescKM, kk > 0);
-                mbar_wait_spin(&bar_u, ph, &failed);
-                tc_fence_after();
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)  // Hl = V^T Ud : both MN-major, K = position
-                    mma_ss_lo(tHl, vMN + offMN(kk), udMN_ + offMN(kk), kIdescMM, kk > 0);
-                // the rows rewrite sH after bar_mh and sY after bar_m2: the stores of the tile before must have read them
-                mbar_wait_spin(&bar_sr, ph, &failed);
-                mma_commit(&bar_mh);  // Yo and Hl done: the state update may start while Yd runs
-                mbar_wait_spin(&bar_g, ph, &failed);
-                tc_fence_after();
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)  // Yd = G' x : A in TMEM (K = j), B = x [j][p] MN-major
-                    mma_ts_lo(tYd, tG + kk * 8, uMN + offMN(kk), kIdescKM, kk > 0);
-                mma_commit(&bar_m2);
-                if (it + 1 < nt) {
-                    mbar_wait(&bar_ld[(it + 1) % NST], ((it + 1) / NST) & 1, &failed);
-                    tc_fence_after();
-                    issue_S(it + 1);
-                }
+                if (++r == kFwdRing) r = 0;
             }
-        } else if (warp == 17 && lane == 0) {
-            // ------------------------------------------------------------------ TMA lane: every load and store
-            prefetch_tmap(&P.mU);
-            prefetch_tmap(&P.mV);
-            prefetch_tmap(&P.mC);
-            auto issue_loads = [&](int it) {
-                const int s = it % NST;
-                uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
-                mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                const int pos = (k0 + it) * LT;
-                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
-                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
-                tma_load_4d(st + 2 * PANEL, &P.mU, &bar_ld[s], 0, hh, pos, bb);
-                tma_load_4d(st + 3 * PANEL, &P.mC, &bar_ld[s], 0, gg, pos, bb);
-                tma_load_4d(st + 4 * PANEL, &P.mC, &bar_ld[s], 64, gg, pos, bb);
+        } else if (warp == 17) {
+            // ------------------------------------------------------------------ TMA: x, every store
+            const size_t t0 = bh * P.Tp + (size_t)k0 * LT;
+            auto load_x = [&](int it) {  // and the tile's per-position scalars
+                const int r = it % kFwdRing;
+                uint64_t* bar = it > 0 ? &bar_mh[(it - 1) & 1] : bar_x0;
+                mbar_expect_tx(bar, PANEL + LT * 4 * (1 + (P.dtT != nullptr) + (P.skipT != nullptr)));
+                tma_load_4d(sRing + r * PANEL, &P.mU, bar, 0, hh, (k0 + it) * LT, bb);
+                float* sc = scum + r * 3 * LT;
+                const size_t o = t0 + (size_t)it * LT;
+                bulk_load(sc, P.tcum + o, LT * 4, bar);
+                if (P.dtT) bulk_load(sc + LT, P.dtT + o, LT * 4, bar);
+                if (P.skipT) bulk_load(sc + 2 * LT, P.skipT + o, LT * 4, bar);
             };
-            for (int it = 0; it < NST - 1 && it < nt; ++it) issue_loads(it);
-            if (P.save_states) {  // the seed is the state entering the first tile
-                tma_store_2d(&P.mS, sH, 0, state_row(0));
+            auto store_y = [&](int it) {
+                tma_store_4d(&P.mY, sRing + (it % kFwdRing) * PANEL, 0, hh, (k0 + it) * LT, bb);
                 tma_store_commit();
+            };
+            if (lane == 0) {
+                prefetch_tmap(&P.mU);
+                for (int it = 0; it < kFwdRing && it < nt; ++it) load_x(it);
             }
             for (int it = 0; it < nt; ++it) {
-                if (it + NST - 1 < nt) {
-                    // the stage of tile it-1 is free once every product of that tile has completed
-                    if (it > 0) mbar_wait(&bar_m2, (it - 1) & 1, &failed);
-                    issue_loads(it + NST - 1);
-                }
-                if (it > 0) {
-                    mbar_wait_spin(&bar_h, (it - 1) & 1, &failed);  // new state in sH, y staged
-                    tma_store_4d(&P.mY, sY, 0, hh, (k0 + it - 1) * LT, bb);
-                    if (P.save_states) tma_store_2d(&P.mS, sH, 0, state_row(it));
+                __syncwarp();
+                named_barrier(kBarU, 608);  // the entering state is in sH
+                if (lane == 0 && P.save_states) {
+                    tma_store_2d(&P.mS, sH, 0, (int)((((size_t)bb * P.nt + k0 + it) * P.h + hh) * DN));
                     tma_store_commit();
                 }
-                tma_store_wait_read();
-                mbar_arrive(&bar_sr);  // sH and sY may be rewritten
+                if (it > 0) {
+                    __syncwarp();
+                    named_barrier(kBarH + ((it - 1) & 1), 544);  // y of the tile before staged
+                    if (lane == 0) store_y(it - 1);
+                }
+                if (lane == 0) {
+                    if (it > 0) tma_store_wait_read<1>();
+                    else tma_store_wait_read();
+                    mbar_arrive(&bar_mh[it & 1]);  // the store has read sH
+                    if (it + 1 == nt) mbar_arrive(&bar_mh[it & 1]);  // (no x behind it)
+                    if (it > 0 && it + 2 < nt) {
+                        tma_store_wait_read();  // y
+                        load_x(it + 2);
+                    }
+                }
             }
-            mbar_wait_spin(&bar_h, (nt - 1) & 1, &failed);
-            tma_store_4d(&P.mY, sY, 0, hh, (k0 + nt - 1) * LT, bb);
-            tma_store_commit();
-            tma_store_wait_all();
+            __syncwarp();
+            named_barrier(kBarH + ((nt - 1) & 1), 544);
+            if (lane == 0) {
+                store_y(nt - 1);
+                tma_store_wait_all();
+            }
+        } else {
+            // ------------------------------------------------------------------ products: Hl and S in one warp, Yo and the loads of B and C in another
+            const bool hl = warp == 18;
+            const uint32_t udMN = desc_lo(smem_u32(sUd), PANEL), hMN = desc_lo(smem_u32(sH), PANEL);
+            auto issue_S = [&](int it) {  // S = C B^T of tile `it` into TMEM buffer it & 1, which the rows have masked two tiles before
+                mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &failed);
+                tc_fence_after();
+                const uint32_t vK = fresh(stK + (uint32_t)(it & 1) * SU), cK = vK + 2 * PU, tS = tm + (it & 1) * 128;
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk) mma_ss_lo(tS, cK + offK(kk), vK + offK(kk), kIdescS, kk > 0);
+                mma_commit(it > 0 ? bar_m2 : bar_s0);
+            };
+            if (!hl && lane == 0) {
+                prefetch_tmap(&P.mV);
+                prefetch_tmap(&P.mC);
+                load_vc(0);
+                if (nt > 1) load_vc(1);
+            }
+            if (hl && lane == 0) issue_S(0);
+            for (int it = 0; it < nt; ++it) {
+                if (!hl && lane == 0) mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &failed);
+                __syncwarp();
+                named_barrier(kBarU, 608);  // weighted rows and entering state written, Hl and Yo of the tile before read
+                if (lane == 0) {
+                    tc_fence_after();
+                    if (hl) {
+                        const uint32_t vMN = fresh(stMN + (uint32_t)(it & 1) * SU), udMN_ = fresh(udMN);
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)  // Hl = V^T Ud : both MN-major, K = position
+                            mma_ss_lo(tHl, vMN + offMN(kk), udMN_ + offMN(kk), kIdescMM, kk > 0);
+                    } else {
+                        const uint32_t cK = fresh(stK + (uint32_t)(it & 1) * SU + 2 * PU), hMN_ = fresh(hMN);
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)  // Yo = C H^T : A = C K-major, B = the running state in sH, [n][p] MN-major
+                            mma_ss_lo(tYo, cK + offK(kk), hMN_ + offMN(kk), kIdescKM, kk > 0);
+                    }
+                    mma_commit(&bar_mh[it & 1]);
+                    if (hl) {
+                        if (it + 1 < nt) issue_S(it + 1);
+                        else mbar_arrive(bar_m2);  // (no S behind it)
+                    } else if (it + 2 < nt) {
+                        mbar_wait(&bar_mh[it & 1], (it >> 1) & 1, &failed);  // Hl and Yo (and S) of the tile, the readers of its stage, have completed
+                        load_vc(it + 2);
+                    }
+                }
+            }
         }
         __syncwarp();
     } else {
@@ -222,130 +272,155 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         const volatile int& rnt = rows_nt;  // in shared memory: the row warps have no register left for it
         const int rb = row >> 5;  // row block, warp-uniform
         const bool active = q <= rb, diag = q == rb;
-        const size_t t0 = bh * P.Tp + (size_t)k0 * LT;
-        const float* tcum = P.tcum + t0;
-        const float* dtT = P.dtT ? P.dtT + t0 : nullptr;
         const uint32_t lanes = lane_base(warp);
         const float Dhead = P.D ? P.D[hh] : 0.f;
-        const float* skipT = P.skipT ? P.skipT + t0 : nullptr;  // per-position skip instead of D
         const bool has_skip = P.D || P.skipT;
         const int c0 = q * 32;  // this thread's 32 columns of S
-        // per-tile scalars are fetched one tile ahead
-        float c_n = tcum[row];
-        float cend_n = tcum[row | 31];
-        float dt_n = dtT ? dtT[row] : 1.f;
-        float sk_n = skipT ? skipT[row] : Dhead;
+        float* wsf = sf + warp * 32;
+        float c_i, Sk;      // of the tile that `weigh` has prepared
+        uint32_t xw[8];     // its weighted x: this thread's quarter row
+        // What a tile needs of x and the scalars before its own turn: the weighted copy, the column factors of this warp's block.
+        auto weigh = [&](int r) {
+            const float* sc = scum + r * 3 * LT;
+            c_i = sc[row];
+            Sk = sc[LT - 1];
+            // the row weight as a bf16 pair: one packed multiply per two elements (the product is rounded to
+            // bf16 for the MMA anyway; rounding the weight first costs at most one more ulp of bf16)
+            const __nv_bfloat162 w2 = __float2bfloat162_rn(exp2f(Sk - c_i) * sc[LT + row]);
+            const uint8_t* sU = sRing + r * PANEL;
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+                const uint4 v = *reinterpret_cast<const uint4*>(sU + sw128(row, q * 2 + ch));
+                const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    __nv_bfloat162 p = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&u[j]), w2);
+                    xw[ch * 4 + j] = *reinterpret_cast<uint32_t*>(&p);
+                }
+            }
+        };
+        float rf = 0.f;  // row factor of this warp's block, relative to the block's last column
+        auto factors = [&](int r) {
+            if (active && !diag) {
+                const float* sc = scum + r * 3 * LT;
+                const float cend = sc[c0 + 31];
+                wsf[lane] = sc[LT + c0 + lane] * exp2f(cend - sc[c0 + lane]);
+                rf = exp2f(c_i - cend);
+            }
+        };
+        auto put_weighted = [&]() {
+            *reinterpret_cast<uint4*>(sUd + sw128(row, q * 2)) = make_uint4(xw[0], xw[1], xw[2], xw[3]);
+            *reinterpret_cast<uint4*>(sUd + sw128(row, q * 2 + 1)) = make_uint4(xw[4], xw[5], xw[6], xw[7]);
+            tc_fence_before();
+            fence_async_smem();
+            __syncwarp();
+            named_arrive(kBarU, 608);
+        };
         float ysq_own = 0.f;  // even quarters: own partial of the tile before
+        mbar_wait(bar_x0, 0, &failed);
+        weigh(0);
+        put_weighted();
+        factors(0);
+        mbar_wait(bar_s0, 0, &failed);
+        tc_fence_after();
+        int ring = 0;  // it % 3
 
         for (int it = 0; it < rnt; ++it) {
-            const int s = it % NST, buf = it & 1;
             const uint32_t ph = it & 1;
-            const float c_i = c_n, cend = cend_n, dtv = dt_n, Dh = sk_n;
-            if (it + 1 < rnt) {
-                const size_t o = (size_t)(it + 1) * LT;
-                c_n = tcum[o + row];
-                cend_n = tcum[o + (row | 31)];
-                dt_n = dtT ? dtT[o + row] : 1.f;
-                if (skipT) sk_n = skipT[o + row];
-            }
-            if (q == 0) {
-                scum2[buf * LT + row] = c_i;
-                sf[buf * LT + row] = dtv * exp2f(cend - c_i);
-                sdtc[buf * LT + row] = dtv;
-            }
-            mbar_wait(&bar_ld[s], (it / NST) & 1, &failed);
-            named_barrier(1, 512);
-            if (P.ysq && it > 0 && !(q & 1))  // the sum of the half row of the tile before: own quarter + the odd one's
-                P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
-                    ysq_own + sysq[(((it - 1) & 1) * 2 + (q >> 1)) * LT + row];
-
-            const float Sk = scum2[buf * LT + LT - 1];
-            uint8_t* sU = sStage + (size_t)s * Cfg::STAGE_BYTES + 2 * PANEL;
-            // this thread's quarter row of U: keep x for the skip term, write the weighted copy
-            uint32_t xrow[8];
-            {
-                // the row weight as a bf16 pair: one packed multiply per two elements (the product is rounded to
-                // bf16 for the MMA anyway; rounding the weight first costs at most one more ulp of bf16)
-                const __nv_bfloat162 w2 = __float2bfloat162_rn(exp2f(Sk - c_i) * dtv);
+            const float e = exp2f(c_i), dec = exp2f(Sk);
+            const float* sc = scum + ring * 3 * LT;
+            const uint32_t tS = tm + (it & 1) * 128 + lanes + c0;
+            if (diag) {  // entry by entry
+                const float4* C4 = reinterpret_cast<const float4*>(sc + c0);
+                const float4* T4 = reinterpret_cast<const float4*>(sc + LT + c0);
 #pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint4 v = *reinterpret_cast<const uint4*>(sU + sw128(row, q * 2 + ch));
-                    uint32_t* u = reinterpret_cast<uint32_t*>(&v);
+                for (int sub = 0; sub < 2; ++sub) {
+                    uint32_t r[16], packed[8];
+                    tmem_ld16(tS + sub * 16, r);
+                    float2 l[8];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        xrow[ch * 4 + j] = u[j];
-                        __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&u[j]), w2);
-                        u[j] = *reinterpret_cast<uint32_t*>(&r);
+                    for (int q4 = 0; q4 < 4; ++q4) {
+                        const int j = sub * 16 + 4 * q4;
+                        const float4 cj = C4[sub * 4 + q4], tj = T4[sub * 4 + q4];
+                        l[2 * q4].x = (j > lane) ? 0.f : tj.x * ex2(c_i - cj.x);
+                        l[2 * q4].y = (j + 1 > lane) ? 0.f : tj.y * ex2(c_i - cj.y);
+                        l[2 * q4 + 1].x = (j + 2 > lane) ? 0.f : tj.z * ex2(c_i - cj.z);
+                        l[2 * q4 + 1].y = (j + 3 > lane) ? 0.f : tj.w * ex2(c_i - cj.w);
                     }
-                    *reinterpret_cast<uint4*>(sUd + sw128(row, q * 2 + ch)) = v;
-                }
-            }
-            fence_async_smem();
-            mbar_arrive_warp(&bar_u);
-
-            mbar_wait(&bar_s, ph, &failed);
-            tc_fence_after();
-            {
-                uint32_t packed[16];
-                if (!active) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) packed[j] = 0u;
-                } else {
-                    uint32_t r[32];
-                    tmem_ld32(tm + (it & 1) * 128 + lanes + c0, r);
                     tmem_ld_wait();
                     const float2* S2 = reinterpret_cast<const float2*>(r);
-                    if (diag) {
-                        const float2* C2 = reinterpret_cast<const float2*>(scum2 + buf * LT + c0);
-                        const float2* T2 = reinterpret_cast<const float2*>(sdtc + buf * LT + c0);
 #pragma unroll
-                        for (int q2 = 0; q2 < 16; ++q2) {
-                            const float2 cj = C2[q2], tj = T2[q2];
-                            float2 l;
-                            l.x = (c0 + 2 * q2 > row) ? 0.f : tj.x * ex2(c_i - cj.x);
-                            l.y = (c0 + 2 * q2 + 1 > row) ? 0.f : tj.y * ex2(c_i - cj.y);
-                            const float2 v = mul2(S2[q2], l);
-                            packed[q2] = pack_bf16(v.x, v.y);
-                        }
-                    } else {
-                        // row factor relative to the block's last column
-                        const float rf = exp2f(c_i - scum2[buf * LT + c0 + 31]);
-                        const float2* F2 = reinterpret_cast<const float2*>(sf + buf * LT + c0);
-                        const float2 rf2 = make_float2(rf, rf);
-#pragma unroll
-                        for (int q2 = 0; q2 < 16; ++q2) {  // fp32 pairs: one instruction, two columns
-                            const float2 v = mul2(S2[q2], mul2(rf2, F2[q2]));
-                            packed[q2] = pack_bf16(v.x, v.y);
-                        }
+                    for (int q2 = 0; q2 < 8; ++q2) {
+                        const float2 v = mul2(S2[q2], l[q2]);
+                        packed[q2] = pack_bf16(v.x, v.y);
                     }
+                    tmem_st8(tG + lanes + q * 16 + sub * 8, packed);
                 }
+                tmem_st_wait();
+            } else if (active) {
+                uint32_t r[32], packed[16];
+                tmem_ld32(tS, r);
+                __syncwarp();  // the warp's column factors
+                const float2 rf2 = make_float2(rf, rf);
+                const float4* F4 = reinterpret_cast<const float4*>(wsf);
+                tmem_ld_wait();
+                const float2* S2 = reinterpret_cast<const float2*>(r);
+#pragma unroll
+                for (int q4 = 0; q4 < 8; ++q4) {  // fp32 pairs: one instruction, two columns
+                    const float4 f = F4[q4];
+                    const float2 v = mul2(S2[2 * q4], mul2(rf2, make_float2(f.x, f.y))), w = mul2(S2[2 * q4 + 1], mul2(rf2, make_float2(f.z, f.w)));
+                    packed[2 * q4] = pack_bf16(v.x, v.y);
+                    packed[2 * q4 + 1] = pack_bf16(w.x, w.y);
+                }
+                tmem_st16(tG + lanes + q * 16, packed);
+                tmem_st_wait();
+            } else if (it == 0) {  // above the diagonal G' is zero in every tile: written once
+                uint32_t packed[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) packed[j] = 0u;
                 tmem_st16(tG + lanes + q * 16, packed);
                 tmem_st_wait();
             }
             tc_fence_before();
-            mbar_arrive_warp(&bar_g);
+            __syncwarp();
+            named_arrive(kBarG, 544);
 
-            // the state update needs Hl only, which completes before Yd: it runs while the rows would wait for Yd
-            mbar_wait(&bar_mh, ph, &failed);
+            // while Yd runs: what the next tile needs early, and the state update
+            uint8_t* sU = sRing + ring * PANEL;
+            const float Dh = P.skipT ? sc[2 * LT + row] : Dhead;
+            if (++ring == kFwdRing) ring = 0;
+            mbar_wait(&bar_mh[ph], (it >> 1) & 1, &failed);  // Hl and Yo have completed, so sH and sUd are free; the next tile's x is there
             tc_fence_after();
+            if (P.ysq && it > 0 && !(q & 1))  // the sum of the half row of the tile before: own quarter + the odd one's (written before this tile's mask)
+                P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
+                    ysq_own + sysq[(((it - 1) & 1) * 2 + (q >> 1)) * LT + row];
+            uint32_t o[16];
             {
                 uint32_t r[16];
                 tmem_ld16(tHl + lanes + q * 16, r);
-                const float dec = exp2f(Sk);
+                tmem_ld16(tYo + lanes + q * 16, o);
+                if (it + 1 < rnt) weigh(ring);
                 tmem_ld_wait();
                 float2* H2 = reinterpret_cast<float2*>(H);
                 const float2 d2 = make_float2(dec, dec);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) H2[j] = fma2(d2, H2[j], reinterpret_cast<const float2*>(r)[j]);
-                store_quarter_row(sH, row, q * 2, H);
             }
-            mbar_wait(&bar_m2, ph, &failed);
-            tc_fence_after();
+            if (it + 1 < rnt) {
+                store_quarter_row(sH, row, q * 2, H);
+                put_weighted();
+                factors(ring);
+            }
             {
-                uint32_t a[16], o[16];
+                uint32_t a[16], xrow[8];
+#pragma unroll
+                for (int ch = 0; ch < 2; ++ch) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(sU + sw128(row, q * 2 + ch));
+                    xrow[ch * 4 + 0] = v.x; xrow[ch * 4 + 1] = v.y; xrow[ch * 4 + 2] = v.z; xrow[ch * 4 + 3] = v.w;
+                }
+                mbar_wait(bar_m2, ph, &failed);
+                tc_fence_after();
                 tmem_ld16(tYd + lanes + q * 16, a);
-                tmem_ld16(tYo + lanes + q * 16, o);
-                const float e = exp2f(c_i);
                 tmem_ld_wait();
                 float y[16];
                 const float2* A2 = reinterpret_cast<const float2*>(a);
@@ -358,7 +433,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     if (has_skip) v = fma2(D2, __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&xrow[j])), v);
                     Y2[j] = v;
                 }
-                store_quarter_row(sY, row, q * 2, y);
+                store_quarter_row(sU, row, q * 2, y);  // over this thread's own values of x, which Yd has read
                 if (P.ysq) {  // sum of squares of this quarter row, for the norm over all heads that follows the scan
                     float2 s2 = make_float2(0.f, 0.f);
 #pragma unroll
@@ -369,10 +444,11 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             }
             tc_fence_before();
             fence_async_smem();
-            mbar_arrive_warp(&bar_h);
+            __syncwarp();
+            named_arrive(kBarH + ph, 544);
         }
         if (P.ysq) {
-            named_barrier(1, 512);
+            named_barrier(kBarRows, 512);
             if (!(q & 1))
                 P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (rnt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((rnt - 1) & 1) * 2 + (q >> 1)) * LT + row];

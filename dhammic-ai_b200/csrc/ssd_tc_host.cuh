@@ -186,7 +186,7 @@ inline int set_walk_attrs(char* err, size_t errn) {
     if (done.load(std::memory_order_acquire) & bit) return 0;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(fwd_walk_kernel, attr, (int)kFwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(states_walk_kernel, attr, (int)WalkCfg<1>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(states_walk_kernel, attr, (int)WalkCfg::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<1, false>, attr, (int)RevCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<1, true>, attr, (int)RevCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(rev_walk_kernel<2, false>, attr, (int)RevCfg<2>::SMEM);
@@ -394,7 +394,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.Tp = Tp; P.h = d.h; P.hpg = d.hpg; P.nt = nt; P.p = d.p; P.n = d.n;
         int pieces;  // the same as the forward's: the states have the same bits
         if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
-        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (launch_dep(after, states_walk_kernel, dim3(d.h, d.b, pieces), kWalkThreads, WalkCfg<1>::SMEM, st, P)));
+        SSD_LAUNCH(prof::K_TC_BWD_STATE, st, (launch_dep(after, states_walk_kernel, dim3(d.h, d.b, pieces), kWalkThreads, WalkCfg::SMEM, st, P)));
         SSD_TC_CHECK("tc_bwd_state");
         after = true;
     }

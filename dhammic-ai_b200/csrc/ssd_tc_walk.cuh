@@ -9,7 +9,7 @@
 //              so it does nothing else);
 //   warp 9     one lane issues every TMA load and store.
 // The forward itself is fwd_walk_kernel (ssd_tc_fwd.cuh), the reverse walk of the backward rev_walk_kernel
-// (ssd_tc_revwalk.cuh); WalkCfg<0> below is the shared-memory layout of the forward.
+// (ssd_tc_revwalk.cuh).
 //
 // mbarriers (phase = tile parity unless noted):
 //   bar_ld[s]  TMA bytes of stage s landed                        (phase = (tile / NST) & 1)
@@ -24,6 +24,11 @@ namespace tc {
 
 __device__ __forceinline__ void named_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+
+// Counts the calling warp in without waiting.
+__device__ __forceinline__ void named_arrive(int id, int nthreads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
 // Write 32 fp32 values as bf16 into chunks [chunk0, chunk0+4) of this row of a swizzled panel.
@@ -77,20 +82,17 @@ __device__ __forceinline__ void store_state_row(float* base, size_t bh, int p, i
         if (p == HP || p0 + q < p) o[(size_t)q * n] = H[q];
 }
 
-template <int MODE>
 struct WalkCfg {
-    static constexpr int NST = (MODE == 1) ? 3 : 2;              // load stages
-    static constexpr int STAGE_PANELS = (MODE == 0) ? 5 : 3;                   // V(2) U(1) [C(2)]
-    static constexpr uint32_t STAGE_BYTES = STAGE_PANELS * PANEL;
-    // stages | sUd | sH | sY (mode 0) | scum2[2][128] sf[2][128] sdtc[2][128] | alignment slack
-    static constexpr size_t SMEM = (size_t)NST * STAGE_BYTES + 2 * PANEL + (MODE == 0 ? PANEL : 0) + 6 * LT * 4 + 1024;
+    static constexpr int NST = 3;                      // load stages
+    static constexpr uint32_t STAGE_BYTES = 3 * PANEL;  // V panels 0,1 | U
+    static constexpr size_t SMEM = (size_t)NST * STAGE_BYTES + 2 * PANEL + 1024;  // stages | sUd | sH | alignment slack
 };
 
 constexpr int kWalkThreads = 320;  // 8 row warps, the product-issue warp, the TMA warp
 
 __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __grid_constant__ WalkParams P) {
     dep_wait();
-    using Cfg = WalkCfg<1>;
+    using Cfg = WalkCfg;
     constexpr int NST = Cfg::NST;
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment by an offset on the __shared__ array itself, so that every access below stays a
