@@ -59,56 +59,38 @@ __device__ __forceinline__ uint32_t mbar_arrive_if_token(uint64_t* bar, bool pre
         : "memory");
     return lo;
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Non-blocking test of a phase (mbarrier.try_wait may suspend the thread for a system-chosen time when the phase is
-// still open; measured here: a waiter that polled just before the last arrive of OTHER THREADS saw the phase about
-// 0.75 us late, while completions by tcgen05.commit or TMA bytes woke it at once).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait.  Returns false (and leaves *failed set) when the limit is reached or when another
-// wait of this block has already given up, so a broken pipeline drains quickly instead of spinning.
-// Not unrolled: left to itself the compiler writes four polls for every wait, and the tile kernels, whose warps run some ten loops at once, no
-// longer fit the instruction cache.
+// Bounded waits: they give up when the limit is reached or when another wait of this block has given up (*failed, in shared memory, is set
+// then), so a broken pipeline drains quickly instead of spinning.  Written out because their size counts: left to the compiler a wait is four polls
+// and 50 instructions, and the tile kernels, whose warps run some ten loops at once, no longer fit the instruction cache.
 constexpr uint32_t kSpinLimit = 4u << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = kSpinLimit) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < limit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *failed) return false;
-    }
-    *failed = 1;
-    return false;
+#define SSD_MBAR_WAIT(poll)                                                                 \
+    asm volatile(                                                                           \
+        "{\n\t.reg .pred p;\n\t.reg .b32 n, f;\n\t"                                         \
+        "mov.b32 n, %3;\n"                                                                  \
+        "WAIT:\n\t"                                                                         \
+        "mbarrier." poll ".parity.shared::cta.b64 p, [%0], %1;\n\t"                         \
+        "@p bra DONE;\n\t"                                                                  \
+        "ld.volatile.shared.b32 f, [%2];\n\t"                                               \
+        "setp.ne.b32 p, f, 0;\n\t"                                                          \
+        "@p bra DONE;\n\t"                                                                  \
+        "add.s32 n, n, -1;\n\t"                                                             \
+        "setp.ne.b32 p, n, 0;\n\t"                                                          \
+        "@p bra WAIT;\n\t"                                                                  \
+        "mov.b32 f, 1;\n\t"                                                                 \
+        "st.volatile.shared.b32 [%2], f;\n"                                                 \
+        "DONE:\n\t}"                                                                        \
+        ::"r"(smem_u32(bar)), "r"(parity), "r"(smem_u32((const void*)failed)), "r"(limit)   \
+        : "memory")
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = kSpinLimit) {
+    SSD_MBAR_WAIT("try_wait");
 }
-
-// The same for phases that other threads complete with mbarrier.arrive: polls without suspending.
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = 16u * kSpinLimit) {
-#pragma unroll 1
-    for (uint32_t i = 0; i < limit; ++i) {
-        if (mbar_test_wait(bar, parity)) return true;
-        if ((i & 4095u) == 4095u && *failed) return false;
-    }
-    *failed = 1;
-    return false;
+// The same for phases that other threads complete with mbarrier.arrive: polls without suspending.  (try_wait may suspend the thread for a
+// system-chosen time while the phase is open; a waiter that polled just before the last arrive of OTHER THREADS saw the phase about
+// 0.75 us late, while completions by tcgen05.commit or TMA bytes woke it at once.)
+__device__ __forceinline__ void mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = 16u * kSpinLimit) {
+    SSD_MBAR_WAIT("test_wait");
 }
+#undef SSD_MBAR_WAIT
 
 // ---------------------------------------------------------------- proxy fences
 __device__ __forceinline__ void fence_async_smem() {  // generic-proxy smem writes -> visible to TMA / tcgen05
@@ -130,6 +112,13 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(col), "r"(head), "r"(pos), "r"(batch)
         : "memory");
+}
+// Such a box into the L2 only.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int col, int head, int pos, int batch) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(col), "r"(head), "r"(pos), "r"(batch) : "memory");
 }
 // `bytes` of contiguous memory, both addresses and the size multiples of 16.
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

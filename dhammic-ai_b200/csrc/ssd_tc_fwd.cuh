@@ -119,7 +119,8 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     // state row of this thread: n = row, p in [16 q, 16 q + 16)
     float H[16];
     if (warp < 16) {
-        for (int i = tid; i < kFwdRing * LT; i += 512) scum[(3 * (i / LT) + 1) * LT + i % LT] = 1.f;  // (without dt)
+        if (!P.dtT)
+            for (int i = tid; i < kFwdRing * LT; i += 512) scum[(3 * (i / LT) + 1) * LT + i % LT] = 1.f;
         load_piece_row<false>(P, bh, row, q * 16, H);
         store_quarter_row(sH, row, q * 2, H);
         fence_async_smem();
@@ -154,6 +155,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             // ------------------------------------------------------------------ products: Yd
             const uint32_t xMN = desc_lo(smem_u32(sRing), PANEL);
             int r = 0;  // it % 3
+#pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 __syncwarp();
                 named_barrier(kBarG, 544);
@@ -189,6 +191,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 prefetch_tmap(&P.mU);
                 for (int it = 0; it < kFwdRing && it < nt; ++it) load_x(it);
             }
+#pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 __syncwarp();
                 named_barrier(kBarU, 608);  // the entering state is in sH
@@ -237,6 +240,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 if (nt > 1) load_vc(1);
             }
             if (hl && lane == 0) issue_S(0);
+#pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 if (!hl && lane == 0) mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &failed);
                 __syncwarp();
@@ -325,6 +329,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         tc_fence_after();
         int ring = 0;  // it % 3
 
+#pragma unroll 1
         for (int it = 0; it < rnt; ++it) {
             const uint32_t ph = it & 1;
             const float e = exp2f(c_i), dec = exp2f(Sk);
