@@ -7,7 +7,7 @@
 //
 // Neither is a recurrence: every tile adds one product to the same accumulator, so the kernel is a plain stream.
 // One CTA per (batch entry, NH heads of a group): TMA loads (stages of the group's B or C panels + the x or dy panel of each
-// head), eight warps per head scale the rows of their 64-wide panel in place, one lane issues eight tcgen05.mma per tile
+// head), eight warps per head scale the rows of their 64-wide panel in place, one lane of another warp issues eight tcgen05.mma per tile
 // (N = 64 NH: the heads' panels side by side) that all accumulate into one TMEM accumulator, read once at the end.  With
 // NH = 2 (heads per group even) the group's panels, two thirds of what a one-head CTA pulls in per tile, are fetched once
 // for two heads; what one SM can pull in is what bounds this kernel.  The weights are <= 1 (dt aside), so nothing
@@ -17,9 +17,11 @@
 // A given seed (initial state, or final-state gradient) enters as  exp(total log-decay) * seed.  blockIdx.z =
 // (piece of `pt` tiles, part of `ps` tiles), each with its own out and logdecay (blockIdx.z, b, h, ...): the pieces of one
 // sequence that the walks run side by side.
-// mbarriers, per stage s (phase (it / stages) & 1): bar_ld[s] TMA bytes landed; bar_u[s] rows scaled, one arrival per
-// warp; bar_m[s] the products of the stage completed (the stage may be reloaded; the last one also releases the
-// accumulator to the row warps).
+// mbarriers, per stage s (phase = turn of the stages): bar_ld[s] TMA bytes landed; bar_m[s] the products of the stage completed (the stage may be
+// reloaded; the last one also releases the accumulator to the row warps).  Hardware barrier kSumBarU + s: rows scaled (row warps arrive, the
+// products' warp waits; one per stage, since the row warps may be as many tiles ahead of the products as there are stages).
+// Products and copies are issued by different warps, so that a stage is asked for again when its products are done and not a tile
+// later: 64 heads of 131,072 positions, half of them forward 160 -> 130 us, three quarters of them in reverse 289 -> 211.
 #pragma once
 
 namespace ssd {
@@ -30,7 +32,7 @@ struct SumCfg {
     static constexpr int STAGES = NH == 1 ? 4 : 3;
     static constexpr uint32_t STAGE_BYTES = (2 + NH) * PANEL;  // V panels 0,1 | U of each head
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
-    static constexpr int THREADS = 256 * NH + 32;
+    static constexpr int THREADS = 256 * NH + 64;
 };
 
 struct SummaryParams {
@@ -49,16 +51,18 @@ struct SummaryParams {
     int z0;               // piece of the blocks with blockIdx.z = 0
 };
 
+constexpr int kSumBarU = 1;  // one per stage
 template <bool REV, int NH>
 __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const __grid_constant__ SummaryParams P) {
     dep_wait();
     if (P.zero_status) clear_status(P.status);
     using Cfg = SumCfg<NH>;
     constexpr int NS = Cfg::STAGES;
-    constexpr int CTLW = 8 * NH;  // control warp
+    constexpr int MMAW = 8 * NH, TMAW = MMAW + 1;  // control warps
+    constexpr int BAR = 256 * NH + 32;             // row warps and the products' warp
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sStage = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    __shared__ uint64_t bar_ld[4], bar_u[4], bar_m[4];
+    __shared__ uint64_t bar_ld[4], bar_m[4];
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
 
@@ -74,12 +78,11 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         failed = 0;
         for (int s = 0; s < NS; ++s) {
             mbar_init(&bar_ld[s], 1);
-            mbar_init(&bar_u[s], 8 * NH);
             mbar_init(&bar_m[s], 1);
         }
         mbar_fence_init();
     }
-    if (warp == CTLW) {
+    if (warp == MMAW) {
         tmem_alloc(&tmem_slot, 64 * NH);
         tmem_relinquish();
     }
@@ -88,34 +91,43 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     tc_fence_after();
     const uint32_t tm = tmem_slot;  // accumulator row = n, columns [64 hs, 64 hs + 64) = p of head hs
 
-    if (warp == CTLW) {
+    if (warp == MMAW) {
+        const uint32_t stMN = desc_lo(smem_u32(sStage), PANEL);
+        int s = 0;
+#pragma unroll 1
+        for (int it = 0; it < nt; ++it) {
+            __syncwarp();
+            named_barrier(kSumBarU + s, BAR);
+            if (lane == 0) {
+                tc_fence_after();
+                uint32_t v = stMN + (uint32_t)s * (Cfg::STAGE_BYTES >> 4);
+                asm volatile("" : "+r"(v));
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)  // acc[n][p of every head] += V^T Uw : both MN-major, K = position
+                    mma_ss_lo(tm, v + kk * 128, v + (2 * PANEL >> 4) + kk * 128, NH == 2 ? kIdescMM128 : kIdescMM, it > 0 || kk > 0);
+                mma_commit(&bar_m[s]);
+            }
+            if (++s == NS) s = 0;
+        }
+    } else if (warp == TMAW) {
         if (lane == 0) {
             prefetch_tmap(&P.mU);
             prefetch_tmap(&P.mV);
-            auto issue_loads = [&](int it) {
-                const int s = it % NS;
+            int s = 0;
+            uint32_t ph = 1;  // (the first turn waits for nothing)
+#pragma unroll 1
+            for (int it = 0; it < nt; ++it) {
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
                 const int pos = tile_of(it) * LT;
+                mbar_wait(&bar_m[s], ph, &failed);  // the products of the stage's tile before are done
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
-                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
-                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
 #pragma unroll
                 for (int hs = 0; hs < NH; ++hs) tma_load_4d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], 0, hh0 + hs, pos, bb);
-            };
-            for (int it = 0; it < NS && it < nt; ++it) issue_loads(it);
-            for (int it = 0; it < nt; ++it) {
-                const int s = it % NS;
-                const uint32_t st = smem_u32(sStage + (size_t)s * Cfg::STAGE_BYTES);
-                mbar_wait(&bar_u[s], (it / NS) & 1, &failed);
-                tc_fence_after();
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)  // acc[n][p of every head] += V^T Uw : both MN-major, K = position
-                    mma_ss(tm, smem_desc(st + kk * 2048, PANEL, 1024), smem_desc(st + 2 * PANEL + kk * 2048, PANEL, 1024),
-                           NH == 2 ? kIdescMM128 : kIdescMM, it > 0 || kk > 0);
-                mma_commit(&bar_m[s]);
-                if (it >= 1 && it - 1 + NS < nt) {  // the stage of the tile before is free once its products are done
-                    mbar_wait(&bar_m[(it - 1) % NS], ((it - 1) / NS) & 1, &failed);
-                    issue_loads(it - 1 + NS);
+                tma_load_4d(st, &P.mV, &bar_ld[s], 0, gg, pos, bb);
+                tma_load_4d(st + PANEL, &P.mV, &bar_ld[s], 64, gg, pos, bb);
+                if (++s == NS) {
+                    s = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -132,8 +144,10 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         float c_n = tcum[o0 + row];
         float S_n = tcum[o0 + LT - 1];
         float dt_n = dtT ? dtT[o0 + row] : 1.f;
+        int s = 0;
+        uint32_t ph = 0;
+#pragma unroll 1
         for (int it = 0; it < nt; ++it) {
-            const int s = it % NS;
             const float c_i = c_n, Sk = S_n, dtv = dt_n;
             if (it + 1 < nt) {
                 const size_t o = (size_t)tile_of(it + 1) * LT;
@@ -143,7 +157,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
             }
             const float w = REV ? exp2f(run + c_i) : dtv * exp2f(run + (Sk - c_i));
             run += Sk;
-            mbar_wait(&bar_ld[s], (it / NS) & 1, &failed);
+            mbar_wait(&bar_ld[s], ph, &failed);
             uint8_t* sU = sStage + (size_t)s * Cfg::STAGE_BYTES + (2 + hs) * PANEL;
             const __nv_bfloat162 w2 = __float2bfloat162_rn(w);
 #pragma unroll
@@ -159,7 +173,12 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
                 *p = v;
             }
             fence_async_smem();
-            mbar_arrive_warp(&bar_u[s]);
+            __syncwarp();
+            named_arrive(kSumBarU + s, BAR);
+            if (++s == NS) {
+                s = 0;
+                ph ^= 1;
+            }
         }
         // `run` is now the total log2-decay of the piece
         const int last = nt - 1;
@@ -180,7 +199,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     tc_fence_before();
     __syncthreads();
     if (tid == 0 && failed) atomicExch(P.status, 1);
-    if (warp == CTLW) tmem_dealloc(tm, 64 * NH);
+    if (warp == MMAW) tmem_dealloc(tm, 64 * NH);
 }
 
 }  // namespace tc
