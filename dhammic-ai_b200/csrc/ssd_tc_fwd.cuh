@@ -61,7 +61,8 @@ constexpr int kFwdStages = 2, kFwdRing = 3;
 // each row warp [16][32] | partial sums of y^2 [2][2][128] | barriers
 constexpr size_t kFwdSmem = kFwdStages * (size_t)kFwdStageBytes + (kFwdRing + 2) * (size_t)PANEL + (3 * kFwdRing + 4 + 4) * LT * 4 + 192;
 // named barriers: all row warps arrive, one or three control warps wait
-constexpr int kBarG = 1, kBarU = 2, kBarH = 3 /* and 4 */, kBarRows = 5;
+constexpr int kBarG = 1, kBarU = 2, kBarH = 3 /* and 4 */, kBarRows = 5, kBarLead = 6, kBarLeadU = 7 /* and 8 */;
+constexpr int kLeadStages = 4;  // of [V panels 0,1 | x], over everything in front of the state
 static_assert(kFwdSmem <= 227 * 1024, "more shared memory than a CTA can have");
 
 // 16 fp32 values of (row, quarter) as two 16-byte chunks of a 128-byte-swizzled [row][64] bf16 panel
@@ -90,25 +91,33 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     float* sf = scum + 3 * kFwdRing * LT;                  // [16][32] column factors dt_j 2^(cend - c_j) of each row warp's block
     float* sysq = sf + 4 * LT;                             // [2][2][128] partial sums of y^2 of the odd quarters
     uint64_t* bars = reinterpret_cast<uint64_t*>(sysq + 4 * LT);
-    uint64_t *bar_vc = bars, *bar_mh = bars + 2, *bar_m2 = bars + 4, *bar_s0 = bars + 5, *bar_x0 = bars + 6;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 7);
-    int& failed = *reinterpret_cast<int*>(bars + 8);
-    int& rows_nt = *reinterpret_cast<int*>(bars + 9);
+    uint64_t *bar_vc = bars, *bar_mh = bars + 2, *bar_m2 = bars + 4, *bar_s0 = bars + 5, *bar_x0 = bars + 6, *lead_ld = bars + 7, *lead_m = bars + 11;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 15);
+    int& failed = *reinterpret_cast<int*>(bars + 16);
+    int& rows_nt = *reinterpret_cast<int*>(bars + 17);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (smem_u32(smem_raw) & 1023u) {  // the swizzled panels need a 1024-byte aligned base: report instead of computing garbage
         if (tid == 0) atomicExch(P.status, 2);
         return;
     }
-    const int hh = blockIdx.x, bb = blockIdx.y;
+    int hh = blockIdx.x, bb = blockIdx.y;
+    int k0 = blockIdx.z * P.pt, nt = min(P.pt, P.nt - k0);  // the piece's tiles
+    int lead = 0;                                           // tiles before them whose states this CTA walks for itself
+    if (P.self.np > 1) {  // one-dimensional grid: whole walks, then pieces that find their own way (SelfCut)
+        const int r = blockIdx.x - P.self.whole, pair = r < 0 ? (int)blockIdx.x : P.self.whole + r / P.self.np, z = r < 0 ? 0 : r % P.self.np;
+        hh = pair % P.h;
+        bb = pair / P.h;
+        k0 = lead = r < 0 ? 0 : P.self.cut[z];
+        nt = (r < 0 ? P.nt : P.self.cut[z + 1]) - k0;
+    }
     const int gg = hh / P.hpg;
     const size_t bh = (size_t)bb * P.h + hh;
-    const int k0 = blockIdx.z * P.pt, nt = min(P.pt, P.nt - k0);  // the piece's tiles
 
     if (tid == 0) {
         failed = 0;
         rows_nt = nt;
-        for (int i = 0; i < 7; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 4 : i == 4 ? 2 : 1);  // mh: Hl, Yo, the store of the state, the next tile's x; m2: Yd, the next S
+        for (int i = 0; i < 15; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 4 : i == 4 ? 2 : 1);  // mh: Hl, Yo, the store of the state, the next tile's x; m2: Yd, the next S
         mbar_fence_init();
     }
     if (warp == 16) {
@@ -122,8 +131,6 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         if (!P.dtT)
             for (int i = tid; i < kFwdRing * LT; i += 512) scum[(3 * (i / LT) + 1) * LT + i % LT] = 1.f;
         load_piece_row<false>(P, bh, row, q * 16, H);
-        store_quarter_row(sH, row, q * 2, H);
-        fence_async_smem();
     }
     tc_fence_before();
     __syncthreads();
@@ -187,10 +194,33 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 tma_store_4d(&P.mY, sRing + (it % kFwdRing) * PANEL, 0, hh, (k0 + it) * LT, bb);
                 tma_store_commit();
             };
-            if (lane == 0) {
-                prefetch_tmap(&P.mU);
-                for (int it = 0; it < kFwdRing && it < nt; ++it) load_x(it);
+            if (lane == 0) prefetch_tmap(&P.mU);
+            if (lead > 0) {
+                if (lane == 0) {
+                    for (int it = 0; it < 2 && it < nt; ++it) {  // what the piece itself starts with comes to the L2 meanwhile
+                        const int pos = (k0 + it) * LT;
+                        tma_prefetch_4d(&P.mU, 0, hh, pos, bb);
+                        for (int c = 0; c < 128; c += 64) {
+                            tma_prefetch_4d(&P.mV, c, gg, pos, bb);
+                            tma_prefetch_4d(&P.mC, c, gg, pos, bb);
+                        }
+                    }
+#pragma unroll 1
+                    for (int it = 0; it < lead; ++it) {
+                        const int s = it % kLeadStages, pos = it * LT;
+                        uint8_t* st = smem_raw + s * 3 * PANEL;
+                        if (it >= kLeadStages) mbar_wait(&lead_m[s], (it / kLeadStages - 1) & 1, &failed);  // the stage's product before is done
+                        mbar_expect_tx(&lead_ld[s], 3 * PANEL);
+                        tma_load_4d(st + 2 * PANEL, &P.mU, &lead_ld[s], 0, hh, pos, bb);
+                        tma_load_4d(st, &P.mV, &lead_ld[s], 0, gg, pos, bb);
+                        tma_load_4d(st + PANEL, &P.mV, &lead_ld[s], 64, gg, pos, bb);
+                    }
+                }
+                __syncwarp();
+                named_barrier(kBarLead, 576);
             }
+            if (lane == 0)
+                for (int it = 0; it < kFwdRing && it < nt; ++it) load_x(it);
 #pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 __syncwarp();
@@ -233,6 +263,22 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 for (int kk = 0; kk < 8; ++kk) mma_ss_lo(tS, cK + offK(kk), vK + offK(kk), kIdescS, kk > 0);
                 mma_commit(it > 0 ? bar_m2 : bar_s0);
             };
+            if (!hl && lead > 0) named_barrier(kBarLead, 576);
+            if (hl) {
+#pragma unroll 1
+                for (int it = 0; it < lead; ++it) {
+                    __syncwarp();
+                    named_barrier(kBarLeadU + (it & 1), 544);
+                    if (lane == 0) {
+                        tc_fence_after();
+                        const uint32_t st = fresh(stMN + (uint32_t)(it % kLeadStages) * 3 * PU);
+#pragma unroll 2
+                        for (int kk = 0; kk < 8; ++kk)  // V^T [d dt o x]
+                            mma_ss_lo(tYo + (it & 1) * 64, st + offMN(kk), st + 2 * PU + offMN(kk), kIdescMM, kk > 0);
+                        mma_commit(&lead_m[it % kLeadStages]);
+                    }
+                }
+            }
             if (!hl && lane == 0) {
                 prefetch_tmap(&P.mV);
                 prefetch_tmap(&P.mC);
@@ -281,7 +327,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         const bool has_skip = P.D || P.skipT;
         const int c0 = q * 32;  // this thread's 32 columns of S
         float* wsf = sf + warp * 32;
-        float c_i, Sk;      // of the tile that `weigh` has prepared
+        float c_i, Sk = 0.f;  // of the tile that `weigh` has prepared
         uint32_t xw[8];     // its weighted x: this thread's quarter row
         // What a tile needs of x and the scalars before its own turn: the weighted copy, the column factors of this warp's block.
         auto weigh = [&](int r) {
@@ -321,6 +367,59 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             named_arrive(kBarU, 608);
         };
         float ysq_own = 0.f;  // even quarters: own partial of the tile before
+        if (lead > 0) {
+            // the states of the tiles before the piece, as the walk itself makes them: weighted rows in place, one tile ahead of the product, whose
+            // accumulator alternates between the columns of Yo and Hl
+            const float *tc = P.tcum + bh * P.Tp, *dt = P.dtT ? P.dtT + bh * P.Tp : nullptr;
+            float c = tc[row], S = tc[LT - 1], d = dt ? dt[row] : 1.f;
+#pragma unroll 1
+            for (int it = -1; it < lead; ++it) {
+                const float dec = exp2f(it < 0 ? 0.f : Sk);
+                if (it + 1 < lead) {
+                    const int s = (it + 1) % kLeadStages;
+                    mbar_wait(&lead_ld[s], ((it + 1) / kLeadStages) & 1, &failed);
+                    uint8_t* sU = smem_raw + (s * 3 + 2) * PANEL;
+                    const __nv_bfloat162 w2 = __float2bfloat162_rn(exp2f(S - c) * d);
+#pragma unroll
+                    for (int ch = 0; ch < 2; ++ch) {
+                        uint4* p4 = reinterpret_cast<uint4*>(sU + sw128(row, q * 2 + ch));
+                        uint4 v = *p4;
+                        uint32_t* u = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            __nv_bfloat162 p = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&u[j]), w2);
+                            u[j] = *reinterpret_cast<uint32_t*>(&p);
+                        }
+                        *p4 = v;
+                    }
+                    Sk = S;
+                    tc_fence_before();
+                    fence_async_smem();
+                    __syncwarp();
+                    named_arrive(kBarLeadU + ((it + 1) & 1), 544);
+                    if (it + 2 < lead) {
+                        const int o = (it + 2) * LT;
+                        c = tc[o + row];
+                        S = tc[o + LT - 1];
+                        d = dt ? dt[o + row] : 1.f;
+                    }
+                }
+                if (it >= 0) {
+                    mbar_wait(&lead_m[it % kLeadStages], (it / kLeadStages) & 1, &failed);
+                    tc_fence_after();
+                    uint32_t r[16];
+                    tmem_ld16(tYo + (it & 1) * 64 + lanes + q * 16, r);
+                    tmem_ld_wait();
+                    float2* H2 = reinterpret_cast<float2*>(H);
+                    const float2 d2 = make_float2(dec, dec);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) H2[j] = fma2(d2, H2[j], reinterpret_cast<const float2*>(r)[j]);
+                }
+            }
+            __syncwarp();
+            named_arrive(kBarLead, 576);  // the panels are free
+        }
+        store_quarter_row(sH, row, q * 2, H);
         mbar_wait(bar_x0, 0, &failed);
         weigh(0);
         put_weighted();
@@ -397,7 +496,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             mbar_wait(&bar_mh[ph], (it >> 1) & 1, &failed);  // Hl and Yo have completed, so sH and sUd are free; the next tile's x is there
             tc_fence_after();
             if (P.ysq && it > 0 && !(q & 1))  // the sum of the half row of the tile before: own quarter + the odd one's (written before this tile's mask)
-                P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
+                P.ysq[((((size_t)bb * P.nt + k0 + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((it - 1) & 1) * 2 + (q >> 1)) * LT + row];
             uint32_t o[16];
             {
@@ -455,10 +554,10 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         if (P.ysq) {
             named_barrier(kBarRows, 512);
             if (!(q & 1))
-                P.ysq[((((size_t)bb * P.nt + blockIdx.z * P.pt + (rnt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
+                P.ysq[((((size_t)bb * P.nt + k0 + (rnt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((rnt - 1) & 1) * 2 + (q >> 1)) * LT + row];
         }
-        if (blockIdx.z * P.pt + rnt == P.nt) store_state_row(P.out_state, bh, P.p, P.n, row, q * 16, H);
+        if (k0 + rnt == P.nt) store_state_row(P.out_state, bh, P.p, P.n, row, q * 16, H);
     }
     tc_fence_before();
     __syncthreads();

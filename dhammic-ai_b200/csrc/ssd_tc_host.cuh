@@ -1,6 +1,8 @@
 // Host side of the tensor-core path: tensor maps, workspace layout and launches.
 #pragma once
 #include <atomic>
+#include <climits>
+#include <cmath>
 #include <cstdio>
 
 #include "../../include/ssd_b200.h"
@@ -64,27 +66,57 @@ struct Ws {
     size_t status, tcum, dtT, skipT, Hst, Qst, final_state, dinit, g, ddtx, dyx, gS, dAh_part, dD_part, piece_sum, piece_decay, base, total;
 };
 
-// The pieces that a walk over one sequence is cut into.  A walk has one CTA per (batch, head), which takes 2.15 us per tile forward
-// and 1.5 us in reverse (1.75 for two heads of a group in one CTA); with few of them most SMs idle.  Pieces run side by side: every piece but the
-// walk's last is first summarised (0.8 us per tile, 1.2 for two heads of a group, no chain, in parts that fill the chip), and a piece's CTA
+constexpr int kPieceSms = 148, kMaxEntries = 16, kWholeWalks = 75;  // SMs; see Pieces
+// The forward walks of a call's last round over the SMs (of all its pairs, where there are no more pairs than SMs), where they leave at least half the SMs idle and
+// no walk is summarised (Pieces): as many CTAs a walk as there are SMs for, up to four, each of which walks the states before its own tiles for itself.  These
+// take 0.8 us a tile and the piece's own 1.5, so pieces shrink by a constant factor.  Only where that saves a tenth of the walk.
+// 44 walks of 16 tiles behind 148 whole ones 57 -> 53 us, 64 walks of 16 tiles 32.5 -> 29, 24 walks of four tiles 10.4 -> 9.6.
+constexpr double kTileUs = 1.5, kLeadUs = 0.8;
+inline SelfCut self_cut(const Dims& d) {
+    const int nt = tiles_of(d.T);
+    const long long bh = (long long)d.b * d.h, rest = bh % kPieceSms;
+    SelfCut best{(int)bh, 1, {0, nt}};
+    if (rest == 0 || bh > INT_MAX / 4) return best;
+    const double f = 1.0 - kLeadUs / kTileUs;
+    double cost = 0.9 * kTileUs * nt;
+    for (int np = 2; np <= 4 && np * rest <= kPieceSms && np <= nt; ++np) {
+        SelfCut c{(int)(bh - rest), np, {0}};
+        double len = nt * (1.0 - f) / (1.0 - std::pow(f, np)), at = 0, longest = 0;
+        bool ok = true;
+        for (int z = 0; z < np; ++z, len *= f) {
+            at += len;
+            c.cut[z + 1] = z + 1 == np ? nt : (int)(at + 0.5);
+            ok = ok && c.cut[z + 1] > c.cut[z];
+            longest = std::max(longest, kTileUs * (c.cut[z + 1] - c.cut[z]) + (z ? kLeadUs * c.cut[z] + 0.7 : 0.0));
+        }
+        if (ok && longest < cost) {
+            cost = longest;
+            best = c;
+        }
+    }
+    return best;
+}
+
+// The pieces that a walk over one sequence is cut into.  A walk has one CTA per (batch, head), which takes 1.5 us per tile forward
+// and 1.1 us in reverse (1.3 for two heads of a group in one CTA); with few of them most SMs idle.  Pieces run side by side: every piece but the
+// walk's last is first summarised (0.7 us per tile, 1.05 for two heads of a group, no chain, in parts that fill the chip), and a piece's CTA
 // folds the summaries before its own into its seed.  Only while all CTAs fit on the chip at once, and where the tiles taken off the chain
-// outweigh the summary and its launch (12 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.
+// outweigh the summary and its launch (10 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.
 // No walk is cut from kWholeWalks pairs on, although reverse walks of up to 148 pairs with two heads per CTA would still gain by it ((1, 24576, 80 heads) forward and
 // backward 1,157 us cut, 1,197 whole; (2, 16384, 64) 1,017, 1,019): a cut changes the order of the state gradient's sums, and a call of
 // that many pairs has the same bits alone as a micro-batch of a larger one.
-// One prompt of 16,384 positions and 64 heads (128 tiles, two pieces): 282 us in one piece, 213 with one summary, 189 with two parts.
+// One prompt of 16,384 positions and 64 heads (128 tiles): 184 us in one piece, 126 in two, 141 in two that find their own way (self_cut).
 struct Pieces {
     int pt, np, ps, parts;  // tiles of a piece, pieces, tiles of a summarised part, parts of a piece
     int heads, sum_heads;   // of a group per CTA of the walk (reverse), of the summary
 };
-constexpr int kPieceSms = 148, kMaxEntries = 16, kWholeWalks = 75;
 inline Pieces pieces_of(const Dims& d, bool reverse) {
     const int nt = tiles_of(d.T);
     const long long bh = (long long)d.b * d.h;
     const bool even = d.hpg % 2 == 0;
     // in one piece: two heads per CTA (shared C panels, one N = 128 product per tile) only where one head per CTA would not fit on the chip at once
     Pieces best{nt, 1, nt, 1, reverse && even && bh > kPieceSms ? 2 : 1, 1};
-    double cost = 0.9 * (reverse ? 1.5 : 2.15) * nt;
+    double cost = 0.9 * (reverse ? 1.1 : kTileUs) * nt;
     if (bh >= kWholeWalks) return best;
     for (int heads = 1; heads <= (reverse && even ? 2 : 1); ++heads)
         for (int P = 2; P <= kMaxEntries && P * bh <= kPieceSms * heads && P <= nt; ++P)
@@ -95,7 +127,7 @@ inline Pieces pieces_of(const Dims& d, bool reverse) {
                 const int ps = (pt + want - 1) / want, parts = (pt + ps - 1) / ps;
                 if (reverse && nt - (np - 1) * pt <= (parts - 1) * ps) continue;  // the short last piece would have an empty part
                 const double rounds = (double)((ctas * parts + kPieceSms - 1) / kPieceSms);
-                const double c = (!reverse ? 2.15 : heads == 2 ? 1.75 : 1.5) * pt + (sum_heads == 2 ? 1.2 : 0.8) * rounds * ps + 12.0 + 0.6 * parts * (np - 1);
+                const double c = (!reverse ? kTileUs : heads == 2 ? 1.3 : 1.1) * pt + (sum_heads == 2 ? 1.05 : 0.7) * rounds * ps + 10.0 + 0.6 * parts * (np - 1);
                 if (c < cost) {
                     cost = c;
                     best = {pt, np, ps, parts, heads, sum_heads};
@@ -327,7 +359,12 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     }
     int pieces;
     if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
-    SSD_LAUNCH(prof::K_TC_FWD, st, launch_dep(after, fwd_walk_kernel, dim3(d.h, d.b, pieces), kFwdThreads, kFwdSmem, st, P));
+    dim3 grid(d.h, d.b, pieces);
+    if (pieces == 1) {
+        P.self = self_cut(d);
+        if (P.self.np > 1) grid = dim3((unsigned)(P.self.whole + (d.b * d.h - P.self.whole) * P.self.np));
+    }
+    SSD_LAUNCH(prof::K_TC_FWD, st, launch_dep(after, fwd_walk_kernel, grid, kFwdThreads, kFwdSmem, st, P));
     SSD_TC_CHECK("tc_fwd_walk");
     if (a->logdecay_total) {
         SSD_LAUNCH(prof::K_CUMSUM, st, launch_dep(true, logdecay_total_kernel, (d.b * d.h + 127) / 128, 128, 0, st, a->a_cumsum, a->logdecay_total, d.b * d.h, d.c, d.l));

@@ -653,6 +653,32 @@ def test_gradients_of_many_heads_do_not_depend_on_the_batch(pkg, cabi, T, h, g):
             assert torch.equal(u, v[i:i + 1]), name
 
 
+@pytest.mark.parametrize("tiles", [1, 2, 3, 4, 6, 9, 12])
+@pytest.mark.parametrize("h,g,few,many", [(1, 1, 1, 80), (3, 1, 2, 27), (6, 2, 4, 14), (3, 1, 56, 28)])
+def test_walks_that_find_their_own_way(pkg, cabi, tiles, h, g, few, many):
+    """Forward walks that leave most SMs idle (all of a call's, or those behind the last full round of 148) are cut, and every CTA makes the states before its tiles
+    for itself: outputs, states and the norm's statistic have the bits of whole walks, which calls of 75 to 148 pairs take.  Lengths from
+    one tile to the longest whose walks are not summarised instead; with and without per-position arrays and kept states."""
+    T, n = 128 * tiles, max(few, many)
+    gen = torch.Generator(device=DEV).manual_seed(tiles)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    x, z, B, C = (randn(n, T, *s).bfloat16() for s in ((h, 64), (h * 64,), (g, 128), (g, 128)))
+    dt, A, D, w = 0.05 * torch.rand(n, T, h, generator=gen, device=DEV), -torch.rand(h, generator=gen, device=DEV), randn(h), randn(h * 64)
+    init = randn(n, h, 64, 128)
+    def run(b):
+        xb, zb, Bb, Cb, dtb, ib = (t[:b].contiguous() for t in (x, z, B / 128 ** 0.5, C, dt, init))
+        out = [*pkg.ssd_mamba2(xb, dtb, A, Bb, Cb, D, 128, ib), *pkg.ssd_mamba2_gated(xb, dtb, A, Bb, Cb, None, zb, w, 1e-6, 128),
+               *pkg.fused_ssd_scan(xb, (dtb * A), Bb, Cb, 128)[:2]]
+        leaf = xb.clone().requires_grad_(True)  # with the states kept for the backward
+        y, fs = pkg.ssd_mamba2(leaf, dtb, A, Bb, Cb, D, 128, ib)
+        return out + [y.detach(), fs.detach(), torch.autograd.grad(y, leaf, xb)[0]]
+    m = min(few, many)
+    for i, (u, v) in enumerate(zip(run(few), run(many))):
+        # (the gradient of few pairs takes another reverse walk, and the states are what the walks left)
+        assert torch.equal(u[:m], v[:m]) if i < 8 else rel_err(u[:m].float(), v[:m].float()) < TOL_BF16, i
+
+
 _FIRST_BACKWARD = """
 import sys
 sys.path.insert(0, {root!r})
