@@ -12,8 +12,7 @@ constexpr int LT = 128;  // tile length
 // block's last column.  Below the diagonal both are <= 1.  Inside the diagonal block the row factor would be
 // 2^(decay from the row to the block end) >= 1 and the column factor its inverse scale; beyond this many log2
 // units across a block one of them would leave the fp32 range.  The forward evaluates diagonal blocks entry by entry (one exp2 per
-// entry); the backward, which is a seventh slower that way, has two instantiations, and the flags of the kernels below, one word per block,
-// select one on the device.
+// entry); the backward, which is 2 % slower that way, does where the flags of the kernels below, one word per block, ask for it.
 constexpr float kMaskSafeLog2 = 100.f;
 // Heads to a block of cumsum_tile_fused_kernel: 32, whose reads are whole 128-byte rows, or eight, a quarter of the loads and one head a warp instead of four, where
 // blocks of eight are few (nine to an SM) or blocks of 32 are half empty (cumsum_blocks_of_eight).  Blocks of 32 / of eight, us, each after a

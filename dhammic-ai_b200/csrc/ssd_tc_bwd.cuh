@@ -36,6 +36,7 @@
 // be, nor a division in one: the text shrank from 90 to 54 KB, instruction cache misses to a fifth (880 -> 815); less work in the row warps between mask and
 // epilogue gives nothing more.  All together 1,050 -> 817 us, (8, 2048, 24 heads, one group) 116 -> 97, one head per group (16, 4096, 64) 1,690 -> 1,387.
 #pragma once
+#include <type_traits>
 
 namespace ssd {
 namespace tc {
@@ -73,16 +74,15 @@ constexpr int kBwdThreads = 640;  // 16 row warps + the control warpgroup (regis
 constexpr int kBwdRegsLaunch = 96, kBwdRegsRow = 112, kBwdRegsCtl = 32;
 static_assert(512 * kBwdRegsRow + 128 * kBwdRegsCtl <= kBwdThreads * kBwdRegsLaunch, "register trade exceeds the CTA's pool");
 
-// Two instantiations (EXACT: diagonal mask blocks entry by entry, see kMaskSafeLog2; 1040 -> 1190 us at (16, 4096, 64 heads)); both are
-// launched and the extreme-decay flags decide on the device which of the two does the work.  (As two bodies of one kernel, chosen by a
-// branch at its top, they spill and the code misses the instruction cache: 1066 us, and 67 -> 75 for one of 8 items per SM.)  Every CTA of both reads all the
-// words, one for 128 positions of eight heads: the idle one takes 3.1 us for 384 of them, 4.5 for 4,096, 6.5 for 65,536, of a step of 234, 1,850 and 15,600.
-template <bool EXACT>
+// Where the extreme-decay flags (one word for 128 positions of eight heads) say that the decay across some 32-position block is beyond the factorised mask,
+// the diagonal blocks are evaluated entry by entry (kMaskSafeLog2), which costs
+// 806 -> 825 us at (16, 4096, 64 heads).  (As an instantiation of its own, both launched and one of the two returning at once, every backward paid 2.7 to
+// 3.9 us for the idle one.)
 __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constant__ BwdParams P) {
     dep_wait();
     int beyond = 0;
     for (int i = threadIdx.x; i < P.flags; i += kBwdThreads) beyond |= P.extreme[i];
-    if ((__syncthreads_or(beyond) != 0) != EXACT) return;
+    const bool exact = __syncthreads_or(beyond) != 0;
     // no static shared memory: the dynamic region starts at the CTA's shared-memory base
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* sC = smem_raw;            // 2 panels [pos][n]
@@ -447,6 +447,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             tc_fence_after();
             float2 rowacc2 = make_float2(0.f, 0.f);
             if (active) {
+                auto mask = [&](auto entries) {  // (two bodies: as a question in the loop 878 us instead of 814)
                 const float2 rf2 = make_float2(rf, rf);
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
@@ -469,7 +470,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                         const float4 f4 = F4[q2 / 2], t4 = T4[q2 / 2];
                         const float2 F = q2 & 1 ? make_float2(f4.z, f4.w) : make_float2(f4.x, f4.y), T = q2 & 1 ? make_float2(t4.z, t4.w) : make_float2(t4.x, t4.y);
                         float2 l;
-                        if (EXACT && diag) {  // see the forward walk: the diagonal block entry by entry
+                        if (decltype(entries)::value) {  // see the forward walk: the diagonal block entry by entry
                             const float2 cj = C2[q2];
                             l.x = exp2f(c_i - cj.x);
                             l.y = exp2f(c_i - cj.y);
@@ -490,6 +491,9 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                     *reinterpret_cast<uint4*>(sGq + sw128(row, gch + sub * 2)) = make_uint4(gp[0], gp[1], gp[2], gp[3]);
                     *reinterpret_cast<uint4*>(sGq + sw128(row, gch + sub * 2 + 1)) = make_uint4(gp[4], gp[5], gp[6], gp[7]);
                 }
+                };
+                if (exact && diag) mask(std::true_type{});
+                else mask(std::false_type{});
             } else {
                 if (hl == 0) {
                     // above the diagonal G is zero for every head: written once (the G panels are staging only after the loop)

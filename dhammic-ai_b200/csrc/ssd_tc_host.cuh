@@ -227,8 +227,7 @@ inline int set_walk_attrs(char* err, size_t errn) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(summary_kernel<true, 1>, attr, (int)SumCfg<1>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(summary_kernel<false, 2>, attr, (int)SumCfg<2>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(summary_kernel<true, 2>, attr, (int)SumCfg<2>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_tile_kernel<false>, attr, (int)kBwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_tile_kernel<true>, attr, (int)kBwdSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_tile_kernel, attr, (int)kBwdSmem);
     if (e != cudaSuccess) SSD_TC_FAIL(SSD_B200_ECUDA, "set shared memory size: %s", cudaGetErrorString(e));
     done.fetch_or(bit, std::memory_order_release);
     return 0;
@@ -459,8 +458,7 @@ inline int backward(const ssd_b200_bwd_args* a, const Dims& d, cudaStream_t st, 
         P.extreme = extreme;
         P.flags = (int)flags_of(d);
         const dim3 grid(std::min(P.items, sm_count()));
-        SSD_LAUNCH(prof::K_TC_BWD, st, launch_dep(true, bwd_tile_kernel<false>, grid, kBwdThreads, kBwdSmem, st, P));
-        SSD_LAUNCH(prof::K_TC_BWD_ALT, st, launch_dep(true, bwd_tile_kernel<true>, grid, kBwdThreads, kBwdSmem, st, P));
+        SSD_LAUNCH(prof::K_TC_BWD, st, launch_dep(true, bwd_tile_kernel, grid, kBwdThreads, kBwdSmem, st, P));
         SSD_TC_CHECK("tc_bwd_walk");
     }
     {
