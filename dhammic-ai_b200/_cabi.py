@@ -20,7 +20,7 @@ EXPORTS = (
     "ssd_b200_abi_version", "ssd_b200_last_error", "ssd_b200_workspace_bytes", "ssd_b200_workspace_min_bytes", "ssd_b200_states_bytes",
     "ssd_b200_resolve_path",
     "ssd_b200_fwd", "ssd_b200_bwd", "ssd_b200_materialize_cache", "ssd_b200_state_prefix_all", "ssd_b200_ipc_export", "ssd_b200_ipc_import", "ssd_b200_ipc_close", "ssd_b200_enable_peer_access", "ssd_b200_exchange_push", "ssd_b200_exchange_arrive",
-    "ssd_b200_m3_prologue_fwd", "ssd_b200_m3_skip_fwd", "ssd_b200_m3_prologue_bwd", "ssd_b200_m3_chain_ws_floats", "ssd_b200_m3_chain_bwd", "ssd_b200_rope_fwd", "ssd_b200_rope_bwd",
+    "ssd_b200_m3_prologue_fwd", "ssd_b200_m3_skip_fwd", "ssd_b200_m3_prologue_bwd", "ssd_b200_m3_dcum_ws_floats", "ssd_b200_m3_chain_ws_floats", "ssd_b200_m3_chain_bwd", "ssd_b200_rope_fwd", "ssd_b200_rope_bwd",
     "ssd_b200_trapezoid_ws_floats", "ssd_b200_trapezoid_fwd", "ssd_b200_trapezoid_bwd",
     "ssd_b200_rmsnorm_ws_floats", "ssd_b200_rmsnorm_fwd", "ssd_b200_rmsnorm_fwd_presummed", "ssd_b200_rmsnorm_bwd", "ssd_b200_fwd_static_scratch", "ssd_b200_static_scratch_bytes", "ssd_b200_device_status", "ssd_b200_selftest_bounded_wait",
     "ssd_b200_launch_count", "ssd_b200_profile_enable", "ssd_b200_profile_kernels", "ssd_b200_profile_kernel_name",
@@ -125,6 +125,8 @@ def load() -> C.CDLL:
     lib.ssd_b200_m3_skip_fwd.argtypes = [C.POINTER(Shape)] + [C.c_void_p] * 8
     lib.ssd_b200_m3_prologue_bwd.restype = C.c_int
     lib.ssd_b200_m3_prologue_bwd.argtypes = [C.POINTER(Shape)] + [C.c_void_p] * 18 + [C.c_int32] + [C.c_void_p] * 3
+    lib.ssd_b200_m3_dcum_ws_floats.restype = C.c_size_t
+    lib.ssd_b200_m3_dcum_ws_floats.argtypes = [C.POINTER(Shape)] + [C.c_void_p] * 5
     lib.ssd_b200_m3_chain_ws_floats.restype = C.c_size_t
     lib.ssd_b200_m3_chain_ws_floats.argtypes = [C.POINTER(Shape)]
     lib.ssd_b200_m3_chain_bwd.restype = C.c_int

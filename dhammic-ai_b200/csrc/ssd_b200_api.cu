@@ -614,6 +614,37 @@ void launch_scan_rev(dim3 grid, cudaStream_t st, const float* in, TO* out, int T
     SSD_LAUNCH(ssd::prof::K_TC_AUX, st, scanT_rev_kernel<TO><<<grid, kRevThreads, smem, st>>>(in, out, T, E, -1.f));
 }
 
+// Whether dB, dC and the angle gradients come from one kernel (rope_bwd_sum_kernel), and the blocks of its clusters; 0 if not.
+int m3_ranks(const ssd::Dims& d, bool bf16, std::initializer_list<const void*> tensors) {
+    return bf16 && d.n % 64 == 0 && (d.hpg == 4 || d.hpg == 8) && !any_unaligned(tensors) ? ssd::m3::sum_ranks((long long)d.b * d.g * (d.n / 64), d.T) : 0;
+}
+template <class TA>
+void m3_angle_gradient(const ssd::Dims& d, const void* B, const void* C, const float* cum, const void* dBr, const void* dCr, const float* dyx, const float* dt,
+                       const float* lam, void* dB, void* dC, TA* dang, cudaStream_t st) {
+    using namespace ssd::m3;
+    using bf = __nv_bfloat16;
+    const int chains = d.b * d.g * (d.n / 64), ranks = sum_ranks(chains, d.T);
+    auto launch = [&](auto steps) {
+        using Cfg = SumCfg<decltype(steps)::value>;
+        auto kernel = rope_bwd_sum_kernel<TA, decltype(steps)::value>;
+        opt_in_smem(kernel, Cfg::smem(8));
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = ranks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3(chains * ranks);
+        c.blockDim = dim3(kSumThreads);
+        c.dynamicSmemBytes = Cfg::smem(ranks);
+        c.stream = st;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        SSD_LAUNCH(ssd::prof::K_TC_AUX, st, cudaLaunchKernelEx(&c, kernel, (const bf*)B, (const bf*)C, cum, (const bf*)dBr, (const bf*)dCr, dyx, dt, lam, (bf*)dB, (bf*)dC, dang, d.T, d.h, d.g, d.n, ranks));
+    };
+    if (d.hpg == 8) launch(std::integral_constant<int, 2>{});
+    else launch(std::integral_constant<int, 1>{});
+}
+
 template <class T>
 int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* dt, const float* lam, const float* D,
                 const void* B, const void* C, const float* cum, const float* sdot, const void* dxw, const void* dBr,
@@ -626,6 +657,14 @@ int m3_bwd_impl(const ssd::Dims& d, const void* x, const void* dy, const float* 
         M3_ROW_DISPATCH(!any_unaligned({x, dy, dxw, dx}), xw_bwd_kernel, (const T*)x, (const T*)dy, (const T*)dxw, dt, lam, D, sdot, (T*)dx, dw, dyx, d.T, d.h, d.hpg, d.p, rows);
     const bool aligned = !any_unaligned({B, C, cum, dBr, dCr, dB, dC, dcum});
     const long long bt = (long long)d.b * d.T;
+    if (!dcum) {
+        if constexpr (sizeof(T) == 2) {
+            if (ang_f32) m3_angle_gradient<float>(d, B, C, cum, dBr, dCr, dyx, dt, lam, dB, dC, (float*)dang, st);
+            else m3_angle_gradient<T>(d, B, C, cum, dBr, dCr, dyx, dt, lam, dB, dC, (T*)dang, st);
+        }
+        CUDA_LAUNCH_CHECK("mamba3 prologue backward");
+        return 0;
+    }
     if (sizeof(T) == 2 && aligned && d.n % 64 == 0 && d.hpg % 4 == 0 && d.hpg <= 64 && bt * d.g * d.n < (1LL << 36)) {  // (and no more blocks than a grid has)
         using bf = __nv_bfloat16;
         const long long parts = ((long long)d.g * (d.n / 64) + kRingThreads / 32 - 1) / (kRingThreads / 32);
@@ -1040,14 +1079,20 @@ int ssd_b200_m3_chain_bwd(const ssd_b200_shape* shape, const float* dw, const fl
     return SSD_B200_OK;
 }
 
+size_t ssd_b200_m3_dcum_ws_floats(const ssd_b200_shape* shape, const void* B, const void* C, const float* cum, const void* dBr, const void* dCr) {
+    if (!shape || check_shape(shape)) return 0;
+    return m3_ranks(dims_of(*shape), shape->dtype == SSD_B200_BF16, {B, C, cum, dBr, dCr}) ? 0 : (size_t)shape->batch * shape->seqlen * shape->nheads * (shape->dstate / 2);
+}
+
 int ssd_b200_m3_prologue_bwd(const ssd_b200_shape* shape, const void* x, const void* dy, const float* dt, const float* lam,
                              const float* D, const void* B, const void* C, const float* cum, const float* sdot,
                              const void* dxw, const void* dBr, const void* dCr, void* dx, float* dw, float* dyx, void* dB,
                              void* dC, void* d_raw_angles, int32_t angles_dtype, float* dcum_ws, float* segsum_ws,
                              void* stream) {
     if (int rc = check_shape(shape)) return rc;
-    if (!dt || !lam || !B || !C || !cum || !sdot || !dBr || !dCr || !dw || !dyx || !dB || !dC || !d_raw_angles || !dcum_ws ||
-        !segsum_ws)
+    if (!dt || !lam || !B || !C || !cum || !sdot || !dBr || !dCr || !dw || !dyx || !dB || !dC || !d_raw_angles || !segsum_ws)
+        return fail(SSD_B200_EINVAL, "null pointer");
+    if (!dcum_ws && !m3_ranks(dims_of(*shape), shape->dtype == SSD_B200_BF16, {B, C, cum, dBr, dCr, dB, dC, d_raw_angles}))
         return fail(SSD_B200_EINVAL, "null pointer");
     if (dxw && (!x || !dy || !dx)) return fail(SSD_B200_EINVAL, "with dxw given, x, dy and dx are needed");
     if (angles_dtype != SSD_B200_F32 && angles_dtype != shape->dtype) return fail(SSD_B200_EINVAL, "d_raw_angles must be fp32 or in the storage dtype");

@@ -21,12 +21,15 @@
 // All of them are HBM-bound streaming kernels; the scans along T are two-pass (per-segment sums, then a
 // segment-local scan seeded by the prefix of the earlier segments).
 #pragma once
+#include <type_traits>
+
 #include "ssd_common.cuh"
 
 namespace ssd {
 namespace m3 {
 
 constexpr int SEG = 128;  // positions per scan segment
+constexpr int kRun = 8, kHalf = SEG / 2;  // positions of a run and of half a segment, of which a reverse sum is made up
 
 // 16-byte vector access: V elements of T (8 bf16 or 4 fp32) per thread, or V = 1 for shapes that do not divide.
 template <class T> struct VecOf { static constexpr int N = 16 / sizeof(T); };
@@ -77,7 +80,12 @@ __device__ __forceinline__ void store_vec(T* p, const float (&f)[V]) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Scan along T of a (b, T, E) tensor.  Pass 1: per-segment sums, each from its first position or (REV) from its last.
+// Scan along T of a (b, T, E) tensor.  Pass 1: per-segment sums, each from its first position.
+//
+// Sums from the end (of the angle gradients) are made up in one order whichever kernel makes them, so that their bits do not depend on the batch:
+// runs of eight positions, each added from its first; halves of a segment from their last run to the first; a segment is the second half plus
+// the first; segments from the last to the first.  A position's sum is that of the segments behind (and the second half, in the first), the
+// runs behind in its half, and the positions of its run from the last to its own, one by one.
 // ------------------------------------------------------------------------------------------
 template <class T, bool REV>
 __global__ void __launch_bounds__(256) scanT_segsum_kernel(const T* __restrict__ in, float* __restrict__ segsum, int Tlen,
@@ -87,11 +95,22 @@ __global__ void __launch_bounds__(256) scanT_segsum_kernel(const T* __restrict__
     if (e >= E) return;
     const int nseg = gridDim.x;
     const int t0 = seg * SEG, t1 = min(Tlen, t0 + SEG);
-    const T* p = in + ((size_t)bb * Tlen + (REV ? t1 - 1 : t0)) * E + e;
-    const ptrdiff_t step = REV ? -(ptrdiff_t)E : E;
+    if (REV) {
+        float half[2] = {0.f, 0.f};
+        for (int r = (t1 - 1) / kRun; r >= t0 / kRun; --r) {
+            const float* p = reinterpret_cast<const float*>(in) + ((size_t)bb * Tlen + r * kRun) * E + e;
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < kRun; ++q) s += r * kRun + q < t1 ? p[(size_t)q * E] : 0.f;
+            (r * kRun % SEG < kHalf ? half[0] : half[1]) += s;
+        }
+        segsum[((size_t)bb * nseg + seg) * E + e] = half[1] + half[0];
+        return;
+    }
+    const T* p = in + ((size_t)bb * Tlen + t0) * E + e;
     float s = 0.f;
 #pragma unroll 8
-    for (int t = t0; t < t1; ++t, p += step) s += to_f(*p);  // eight loads in flight per thread
+    for (int t = t0; t < t1; ++t, p += E) s += to_f(*p);  // eight loads in flight per thread
     segsum[((size_t)bb * nseg + seg) * E + e] = s;
 }
 
@@ -118,23 +137,38 @@ __global__ void __launch_bounds__(256) scanT_apply_kernel(const TI* __restrict__
             out[o] = from_f<TO>(sign * run);
         }
     } else {
-#pragma unroll 8
-        for (int t = t1 - 1; t >= t0; --t) {
-            const size_t o = ((size_t)bb * Tlen + t) * E + e;
-            run += to_f(in[o]);
-            out[o] = from_f<TO>(sign * run);
+        const float behind = run;
+        float half = 0.f;
+        for (int r = (t1 - 1) / kRun; r >= t0 / kRun; --r) {
+            if ((r + 1) * kRun % SEG == kHalf) {  // the first half's last run
+                run = behind + half;
+                half = 0.f;
+            }
+            const size_t o = ((size_t)bb * Tlen + r * kRun) * E + e;
+            float v[kRun], s = 0.f, sum = run;
+#pragma unroll
+            for (int q = 0; q < kRun; ++q) v[q] = r * kRun + q < t1 ? to_f(in[o + (size_t)q * E]) : 0.f;
+#pragma unroll
+            for (int q = 0; q < kRun; ++q) s += v[q];
+#pragma unroll
+            for (int q = kRun - 1; q >= 0; --q) {
+                sum += v[q];
+                if (r * kRun + q < t1) out[o + (size_t)q * E] = from_f<TO>(sign * sum);
+            }
+            run += s;
+            half += s;
         }
     }
 }
 
-// Both passes in one, from the last position to the first: a thread keeps two columns' sums over the segments behind (added one by one, as
-// scanT_apply_kernel does, each summed up from its end: same order, same bits) and walks the positions.  HBM-bound: the values come through a
+// Both passes in one, from the last position to the first: a thread keeps two columns' sums over the segments behind
+// and walks the positions.  HBM-bound: the values come through a
 // ring in shared memory, 56 positions ahead, of which a thread reads only what it copied itself.  (16, 4096, 64 x 64)
 // fp32 -> bf16: 346 us with a segment at a time, half of it in registers, whose loads waited for its stores; 259 now (6.2 TB/s), 338 with 64 threads a
 // block.
 // Needs enough columns to have the bytes in flight (kOnePassColumns), an even number of them and 8-byte aligned tensors.
 constexpr int kOnePassColumns = 148 * 256;
-constexpr int kRevThreads = 128, kRevRows = 8, kRevGroups = 8;  // positions of a group of copies, groups
+constexpr int kRevThreads = 128, kRevRows = kRun, kRevGroups = 8;  // positions of a group of copies, groups
 template <class TO>
 __global__ void __launch_bounds__(kRevThreads) scanT_rev_kernel(const float* __restrict__ in, TO* __restrict__ out, int Tlen, int E, float sign) {
     extern __shared__ __align__(16) float2 pos[];  // [kRevGroups][kRevRows][kRevThreads]
@@ -157,29 +191,40 @@ __global__ void __launch_bounds__(kRevThreads) scanT_rev_kernel(const float* __r
     };
 #pragma unroll
     for (int i = 0; i < kRevGroups - 1; ++i) fetch(last - i);
-    float2 behind = make_float2(0.f, 0.f), run = behind, s = behind;
+    float2 behind = make_float2(0.f, 0.f), run = behind, s = behind, upper = behind;
     for (int g = last; g >= 0; --g) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kRevGroups - 2) : "memory");
         float2 v[kRevRows];
 #pragma unroll
         for (int q = 0; q < kRevRows; ++q) v[q] = pos[((g % kRevGroups) * kRevRows + q) * kRevThreads + threadIdx.x];
         fetch(g - (kRevGroups - 1));  // where the group before this one was
+        float2 all = make_float2(0.f, 0.f), sum = run;
+#pragma unroll
+        for (int q = 0; q < kRevRows; ++q) {
+            all.x += v[q].x;
+            all.y += v[q].y;
+        }
 #pragma unroll
         for (int q = kRevRows - 1; q >= 0; --q) {
             const int t = g * kRevRows + q;
-            run.x += v[q].x;
-            run.y += v[q].y;
-            s.x += v[q].x;
-            s.y += v[q].y;
+            sum.x += v[q].x;
+            sum.y += v[q].y;
             if (t < Tlen) {
-                if constexpr (sizeof(TO) == 2) *reinterpret_cast<__nv_bfloat162*>(o + (size_t)t * E) = __floats2bfloat162_rn(sign * run.x, sign * run.y);
-                else *reinterpret_cast<float2*>(o + (size_t)t * E) = make_float2(sign * run.x, sign * run.y);
+                if constexpr (sizeof(TO) == 2) *reinterpret_cast<__nv_bfloat162*>(o + (size_t)t * E) = __floats2bfloat162_rn(sign * sum.x, sign * sum.y);
+                else *reinterpret_cast<float2*>(o + (size_t)t * E) = make_float2(sign * sum.x, sign * sum.y);
             }
         }
-        if (g % (SEG / kRevRows) == 0) {  // the segment's first positions
-            behind.x += s.x;
-            behind.y += s.y;
-            run = behind;
+        run = make_float2(run.x + all.x, run.y + all.y);
+        s = make_float2(s.x + all.x, s.y + all.y);
+        if (g % (kHalf / kRevRows) == 0) {  // the first positions of half a segment
+            if (g % (SEG / kRevRows)) {
+                upper = s;
+                run = make_float2(behind.x + s.x, behind.y + s.y);
+            } else {
+                behind = make_float2(behind.x + (upper.x + s.x), behind.y + (upper.y + s.y));
+                upper = make_float2(0.f, 0.f);
+                run = behind;
+            }
             s = make_float2(0.f, 0.f);
         }
     }
@@ -554,6 +599,240 @@ __global__ void __launch_bounds__(kRingThreads, 768 / kRingThreads) rope_bwd_rin
         }
         *reinterpret_cast<uint2*>((up ? dC : dB) + ((size_t)(r0 + r) * g + gg) * n + j0 + (odd ? 4 : 0)) = out;
     }
+}
+
+// The same with the sum over the positions behind, for groups of 4 STEPS heads: the angles' gradient itself, without the gradient of their running
+// sums in memory.  A cluster of `ranks` blocks walks a strip of 64 columns of a group from the end of its sequence: a block takes half a segment, each
+// warp a run of eight positions, first to last through the ring, and keeps what it makes in shared memory.  Then the runs' sums go up to the halves' and
+// segments', in the order of scanT_rev_kernel (same bits), and the warp comes back over its run with the sum behind it.  A lane reads the
+// B and C of its columns as other lanes copied them (once per warp); everything else it reads it copied itself.
+//
+// Two blocks of eight warps an SM (114 KB: 64 kept, 36 the ring).  Written and read again, the gradient of the sums was 8 of 20 bytes per angle.  bf16 angles,
+// 64 heads, 8 groups, 128 columns, ring and reverse sums -> this: (16, 4096) 983 -> 801 us, (8, 2048) 318 -> 226, (2, 4096) 171 -> 127, (4, 256) 36 -> 17.  What
+// binds it now is issue and the latency of the ring, not HBM (4.7 TB/s): with the places in memory worked out by 64-bit products at each
+// step 857, with prefetches into L2 four positions ahead 1024.
+constexpr int kSumWarps = 8, kSumThreads = 32 * kSumWarps;
+static_assert(kSumWarps * kRun == kHalf, "a block walks half a segment at a time");
+template <int STEPS>
+struct SumCfg {
+    static constexpr int STAGE = 3 * kSumThreads;            // 16-byte units: dBr | dCr | angles
+    static constexpr int BCS = STEPS == 1 ? 3 : 2;           // positions whose B and C are there or on their way
+    static constexpr int RING = kRingStages * STAGE, BC = kSumWarps * BCS * 16, KEPT = kSumWarps * kRun * STEPS * 32, TOT = kSumWarps * STEPS * 32, HALF = STEPS * 32;
+    static constexpr int smem(int ranks) { return (RING + BC + KEPT + TOT + (ranks > 1 ? HALF : 0)) * 16; }
+};
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_peer(const float4* p, unsigned rank) {
+    uint32_t a;
+    float4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+template <class TA, int STEPS>
+__global__ void __launch_bounds__(kSumThreads, 2) rope_bwd_sum_kernel(
+    const __nv_bfloat16* __restrict__ B, const __nv_bfloat16* __restrict__ C, const float* __restrict__ cum, const __nv_bfloat16* __restrict__ dBr,
+    const __nv_bfloat16* __restrict__ dCr, const float* __restrict__ dyx, const float* __restrict__ dt, const float* __restrict__ lam,
+    __nv_bfloat16* __restrict__ dB, __nv_bfloat16* __restrict__ dC, TA* __restrict__ dang, int Tlen, int h, int g, int n, int ranks) {
+    using T = __nv_bfloat16;
+    using Cfg = SumCfg<STEPS>;
+    constexpr int V = 8, HPG = 4 * STEPS;
+    extern __shared__ __align__(16) uint4 sum_sh[];
+    uint4* ring = sum_sh;
+    uint4* bc = ring + Cfg::RING;                                  // [warp][position][B 8 | C 8]
+    float4* kept = reinterpret_cast<float4*>(bc + Cfg::BC);        // [warp][position of the run][four heads][lane]
+    float4* tot = kept + Cfg::KEPT;                                // [warp][four heads][lane]: sum of the run, then of all behind it
+    float4* half = tot + Cfg::TOT;                                 // [four heads][lane]: the block's, for the others of its cluster
+    const int strips = n / 64, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % ranks, chain = blockIdx.x / ranks, strip = chain % strips, gg = chain / strips % g, bb = chain / strips / g;
+    const int j0 = (strip * 8 + (lane & 7)) * V, h0 = gg * HPG + (lane >> 3);
+    const size_t seq = (size_t)bb * Tlen;
+    const int bands = (Tlen + ranks * kHalf - 1) / (ranks * kHalf);
+    auto first = [&](int band) { return ((band * ranks + rank) * kSumWarps + w) * kRun; };
+    auto length = [&](int band) { return max(0, min(kRun, Tlen - first(band))); };
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ring) + threadIdx.x * 16, my_bc = (uint32_t)__cvta_generic_to_shared(bc) + (w * Cfg::BCS * 16 + lane) * 16;
+    auto copy = [&](uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); };
+    // what is fetched next: positions left in the run, runs left, stage, place of B and C, byte offsets in dBr (dCr, angles) and B (C)
+    const int last = length(bands - 1) ? bands - 1 : bands - 2;
+    const size_t row_y = (size_t)h * n * 2, row_b = (size_t)g * n * 2;
+    const uint32_t step_y = 4 * n * 2;
+    const char* bc_of = reinterpret_cast<const char*>(lane < 8 ? B : C);
+    int f_left = last >= 0 ? length(last) : 0, f_runs = last;
+    size_t f_y = ((seq + (last >= 0 ? first(last) : 0)) * h + h0) * n * 2 + j0 * 2, f_b = ((seq + (last >= 0 ? first(last) : 0)) * g + gg) * n * 2 + j0 * 2;
+    size_t run_y = f_y, run_b = f_b;                                           // its run's first position
+    const size_t turn_y = row_y * ranks * kHalf, turn_b = row_b * ranks * kHalf;  // to the run before
+    uint32_t f_stage = mine, f_place = my_bc;
+    auto fetch = [&](auto k) {  // one group of copies a step, empty behind the last
+        constexpr int K = decltype(k)::value;
+        if (f_left > 0) {
+            const size_t o = f_y + K * step_y;
+            copy(f_stage, reinterpret_cast<const char*>(dBr) + o);
+            copy(f_stage + kSumThreads * 16, reinterpret_cast<const char*>(dCr) + o);
+            copy(f_stage + 2 * kSumThreads * 16, reinterpret_cast<const char*>(cum) + o);
+            if (K == 0 && lane < 16) copy(f_place, bc_of + f_b);
+            if (K == STEPS - 1) {
+                f_y += row_y;
+                f_b += row_b;
+                f_place = f_place == my_bc + (Cfg::BCS - 1) * 256 ? my_bc : f_place + 256;
+                if (--f_left == 0 && f_runs-- > 0) {
+                    f_left = kRun;
+                    f_y = run_y -= turn_y;
+                    f_b = run_b -= turn_b;
+                }
+            }
+            f_stage = f_stage == mine + (kRingStages - 1) * Cfg::STAGE * 16 ? mine : f_stage + Cfg::STAGE * 16;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float lam_n = 1.f, dt_n = 0.f, yx_n = 0.f;  // as in rope_bwd_ring_kernel, of the next position
+    auto fetch_diagonal = [&](int t) {
+        const bool on = t >= 0 && t + 1 < Tlen && lane < HPG;
+        const size_t ih = (seq + t) * h + gg * HPG + lane;
+        lam_n = on ? lam[ih + h] : 1.f;
+        dt_n = on ? dt[ih + h] : 0.f;
+        yx_n = on ? dyx[ih] : 0.f;
+    };
+    if (last >= 0) fetch_diagonal(first(last));
+    static_assert(kRingStages == 3, "two steps ahead: the same four heads of the next position, or the position after that");
+    fetch(std::integral_constant<int, 0>{});
+    fetch(std::integral_constant<int, STEPS - 1>{});
+    float4 behind = make_float4(0.f, 0.f, 0.f, 0.f), upper = behind;  // sums of the segments behind, of this one's upper half
+    int s = 0, cp = 0;
+    const size_t row_out = (size_t)h * (n / 2) * sizeof(TA);
+#pragma unroll 1
+    for (int band = bands - 1; band >= 0; --band) {
+        const int R = length(band), t0 = first(band);
+        float4 sum[STEPS];
+#pragma unroll
+        for (int k = 0; k < STEPS; ++k) sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        char* to = reinterpret_cast<char*>(lane & 16 ? dC : dB) + ((seq + t0) * g + gg) * n * 2 + j0 * 2 + (lane & 8);
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+            float ds = 0.f, bv[V], cv[V], ab[V], ac[V];
+#pragma unroll
+            for (int q = 0; q < V; ++q) ab[q] = ac[q] = 0.f;
+            auto step = [&](auto kc) {
+                constexpr int k = decltype(kc)::value;
+                asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 2) : "memory");
+                const uint4* p = ring + s * Cfg::STAGE + threadIdx.x;
+                const uint4 yb = p[0], yc = p[kSumThreads], ya = p[2 * kSumThreads];
+                if (k == 0) {
+                    __syncwarp();  // B and C came with other lanes' copies; and all are through with the position before
+                    const uint4* q = bc + (w * Cfg::BCS + cp) * 16 + (lane & 7);
+                    load_vec<T, V>(reinterpret_cast<const T*>(q), bv);
+                    load_vec<T, V>(reinterpret_cast<const T*>(q + 8), cv);
+                    if (++cp == Cfg::BCS) cp = 0;
+                    ds = -(1.f - lam_n) * dt_n * yx_n;
+                    fetch_diagonal(r + 1 < R ? t0 + r + 1 : band ? first(band - 1) : -1);
+                }
+                if (++s == kRingStages) s = 0;
+                fetch(kc);
+                float db[V], dc[V], dth[V / 2];
+#pragma unroll
+                for (int q = 0; q < V; ++q) {
+                    db[q] = to_f(reinterpret_cast<const T*>(&yb)[q]);
+                    dc[q] = to_f(reinterpret_cast<const T*>(&yc)[q]);
+                }
+#pragma unroll
+                for (int q = 0; q < V / 2; ++q) {
+                    float sn, c;
+                    sincos_reduced(reinterpret_cast<const float*>(&ya)[q], &sn, &c);
+                    const float b1 = c * db[2 * q] + sn * db[2 * q + 1], b2 = c * db[2 * q + 1] - sn * db[2 * q];
+                    const float c1 = c * dc[2 * q] + sn * dc[2 * q + 1], c2 = c * dc[2 * q + 1] - sn * dc[2 * q];
+                    ab[2 * q] += b1;
+                    ab[2 * q + 1] += b2;
+                    ac[2 * q] += c1;
+                    ac[2 * q + 1] += c2;
+                    dth[q] = (bv[2 * q] * b2 - bv[2 * q + 1] * b1) + (cv[2 * q] * c2 - cv[2 * q + 1] * c1);
+                }
+                const float4 v = make_float4(dth[0], dth[1], dth[2], dth[3]);
+                kept[((w * kRun + r) * STEPS + k) * 32 + lane] = v;
+                sum[k] = add4(sum[k], v);
+            };
+            step(std::integral_constant<int, 0>{});
+            if constexpr (STEPS == 2) step(std::integral_constant<int, 1>{});
+#pragma unroll
+            for (int of = 16; of > 0; of >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, of);
+            const bool up = lane & 16, odd = lane & 8;  // lanes 0-15 end with four columns of dB, 16-31 of dC
+            float v[V];
+#pragma unroll
+            for (int q = 0; q < V; ++q) v[q] = (up ? ac[q] : ab[q]) + __shfl_xor_sync(0xffffffffu, up ? ab[q] : ac[q], 16);
+            uint2 out;
+            T* e = reinterpret_cast<T*>(&out);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float all = (odd ? v[4 + q] : v[q]) + __shfl_xor_sync(0xffffffffu, odd ? v[q] : v[4 + q], 8);
+                const float lo = up ? bv[q] : cv[q], hi = up ? bv[4 + q] : cv[4 + q];
+                e[q] = from_f<T>(fmaf(ds, odd ? hi : lo, all));
+            }
+            *reinterpret_cast<uint2*>(to) = out;
+            to += row_b;
+        }
+#pragma unroll
+        for (int k = 0; k < STEPS; ++k) tot[(w * STEPS + k) * 32 + lane] = sum[k];
+        __syncthreads();
+        float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool adds = threadIdx.x < STEPS * 32;  // thread (four heads, lane)
+        if (adds) {
+#pragma unroll
+            for (int i = kSumWarps - 1; i >= 0; --i) own = add4(own, tot[i * STEPS * 32 + threadIdx.x]);
+            if (ranks > 1) half[threadIdx.x] = own;
+        }
+        if (ranks > 1) cluster_sync();
+        if (adds) {
+            float4 run = behind;
+            for (int j = ranks - 1; j >= 0; --j) {
+                const bool second = (band * ranks + j) & 1;  // half of its segment
+                if (j == rank) run = second ? behind : add4(behind, upper);
+                const float4 v = j == rank ? own : ld_peer(half + threadIdx.x, j);
+                if (second) {
+                    upper = v;
+                } else {
+                    behind = add4(behind, add4(upper, v));
+                    upper = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+#pragma unroll
+            for (int i = kSumWarps - 1; i >= 0; --i) {
+                float4* p = tot + i * STEPS * 32 + threadIdx.x;
+                const float4 v = *p;
+                *p = run;
+                run = add4(run, v);
+            }
+        }
+        if (ranks > 1) cluster_sync();
+        else __syncthreads();
+#pragma unroll
+        for (int k = 0; k < STEPS; ++k) {
+            float4 run = tot[(w * STEPS + k) * 32 + lane];
+            char* e = reinterpret_cast<char*>(dang + ((seq + t0 + R - 1) * h + h0 + 4 * k) * (n / 2) + j0 / 2);
+            for (int r = R - 1; r >= 0; --r, e -= row_out) {
+                run = add4(run, kept[((w * kRun + r) * STEPS + k) * 32 + lane]);
+                if constexpr (sizeof(TA) == 2) {
+                    uint2 u;
+                    T* x = reinterpret_cast<T*>(&u);
+                    x[0] = from_f<T>(-run.x); x[1] = from_f<T>(-run.y); x[2] = from_f<T>(-run.z); x[3] = from_f<T>(-run.w);
+                    *reinterpret_cast<uint2*>(e) = u;
+                } else {
+                    *reinterpret_cast<float4*>(e) = make_float4(-run.x, -run.y, -run.z, -run.w);
+                }
+            }
+        }
+    }
+}
+// Blocks of a cluster: what leaves least of the last round of blocks (two an SM) empty, a cluster's barriers at 4 % a block.  (8, 2048), 128 strips: 294 us
+// with one, 226 with two, 237 with four, 250 with eight; (12, 3072), 192 strips: 572, 569, 518, 545; (6, 2048), 96: 281, 215, 202, 190.  0 where
+// even eight leave the chip too empty: (2, 4096), 32 strips, 127 us against 171 of the ring and the sums behind it, (1, 4096), 16 strips, 114 against 96.
+inline int sum_ranks(long long chains, int T) {
+    int best = 0;
+    double least = 0;
+    for (int c = 1; c <= 8 && (c == 1 || c * kHalf <= T); c *= 2) {
+        const double t = (double)((chains * c + 2 * 148 - 1) / (2 * 148)) / c * (1 + 0.04 * (c > 1) * c);
+        if (!best || t < least) { best = c; least = t; }
+    }
+    return chains * best >= 200 ? best : 0;
 }
 
 // ------------------------------------------------------------------------------------------

@@ -556,7 +556,8 @@ struct Mamba3Node : ScanNode {
         }
         const Tensor dB = at::empty_like(Bv), dC = at::empty_like(Cv);
         const Tensor dang = at::empty({b, T, h, n / 2}, xv.options().dtype(ang_type));
-        const Tensor dcum = empty_f32({b, T, h, n / 2}, xv), seg = empty_f32({b * ((T + 127) / 128) * h * (n / 2)}, xv);
+        const Tensor dcum = ssd_b200_m3_dcum_ws_floats(&block, ptr(Bv), ptr(Cv), ptr<float>(cumv), ptr(g.dB), ptr(g.dC)) ? empty_f32({b, T, h, n / 2}, xv) : Tensor();
+        const Tensor seg = empty_f32({b * ((T + 127) / 128) * h * (n / 2)}, xv);
         void* st = stream_of(xv);
         check(ssd_b200_m3_prologue_bwd(&block, ptr(xv), ptr(dy), ptr<float>(dtv), ptr<float>(lamv), ptr<float>(Dv), ptr(Bv), ptr(Cv), ptr<float>(cumv),
                                        ptr<float>(sd), ptr(dxw), ptr(g.dB), ptr(g.dC), ptr(dx), ptr<float>(dw), ptr<float>(dyx), ptr(dB), ptr(dC),

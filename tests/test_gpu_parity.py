@@ -1266,6 +1266,41 @@ def test_mamba3_rotation_backward(pkg, cabi, b, T, h, g, n):
         assert rel_err(dang, -dcum.double().flip(1).cumsum(1).flip(1)) < TOL_FP32
 
 
+@pytest.mark.parametrize("b,T,h,g,n", [(26, 1, 64, 8, 64), (52, 7, 16, 4, 64), (26, 65, 16, 4, 128), (25, 129, 16, 4, 64), (13, 257, 32, 4, 64), (13, 600, 8, 2, 64),
+                                       (12, 300, 64, 8, 128), (16, 1100, 8, 2, 64)])
+@pytest.mark.parametrize("ang32", [True, False])
+def test_mamba3_rotation_backward_with_its_sum(pkg, cabi, b, T, h, g, n, ang32):
+    """Rotation undone and angle gradients summed in one kernel, in clusters of one to eight blocks, groups of four and eight heads, lengths that end inside a
+    run, half a segment and a cluster's band: the bits of the two steps on their own (with room for what lies between them), also of a
+    batch entry alone; and those against 64 bits, as above."""
+    import ctypes
+    lib, S = cabi.load(), pkg.ssd_scan
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    P = S._ptr
+    B, C, dBr, dCr = (randn(*s).bfloat16() for s in ((b, T, g, n), (b, T, g, n), (b, T, h, n), (b, T, h, n)))
+    cum, dt, lam, dyx = 30.0 * randn(b, T, h, n // 2), torch.rand(b, T, h, generator=gen, device=DEV), torch.rand(b, T, h, generator=gen, device=DEV), randn(b, T, h)
+    def run(k, apart):
+        ins = [t[:k].contiguous() for t in (dt, lam, B, C, cum, dBr, dCr, dyx)]
+        shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16, cabi.F32, cabi.PATH_AUTO, k, T, h, 64, n, g, T)
+        if not apart:
+            assert lib.ssd_b200_m3_dcum_ws_floats(ctypes.byref(shape), P(ins[2]), P(ins[3]), P(ins[4]), P(ins[5]), P(ins[6])) == 0
+        dB, dC, dcum = torch.empty_like(ins[2]), torch.empty_like(ins[3]), torch.empty_like(ins[4]) if apart else None
+        dang = torch.empty(k, T, h, n // 2, dtype=torch.float32 if ang32 else torch.bfloat16, device=DEV)
+        sdot, dw, seg = torch.zeros(k, T, g, device=DEV), torch.zeros(k, T, h, device=DEV), torch.empty(k * ((T + 127) // 128) * h * (n // 2), device=DEV)
+        cabi.check(lib.ssd_b200_m3_prologue_bwd(ctypes.byref(shape), None, None, P(ins[0]), P(ins[1]), None, P(ins[2]), P(ins[3]), P(ins[4]), P(sdot), None, P(ins[5]),
+                                                P(ins[6]), None, P(dw), P(ins[7]), P(dB), P(dC), P(dang), cabi.F32 if ang32 else cabi.BF16,
+                                                P(dcum) if apart else None, P(seg), S._stream(torch.device(DEV))))
+        torch.cuda.synchronize()
+        return dB, dC, dang, dcum
+    one, two, alone = run(b, False), run(b, True), run(1, True)
+    for u, v, w in zip(one[:3], two[:3], alone[:3]):
+        assert torch.equal(u, v) and torch.equal(u[:1], w)
+    want = -two[3].double().flip(1).cumsum(1).flip(1)
+    assert ((one[2].double() - want).abs() <= (0.0 if ang32 else 2.0 ** -8) * want.abs() + 1e-5 * want.abs().max()).all()
+
+
 @pytest.mark.parametrize("T", [600, 128])
 def test_mamba3_angle_gradient_does_not_depend_on_the_batch(pkg, cabi, T):
     """Many columns take the reverse sum of the angle gradients in one pass, few in two; the order of the sums, and so
