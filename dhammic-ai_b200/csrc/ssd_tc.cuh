@@ -21,8 +21,8 @@
 //        dG = dY X^T, dS = dG o L, dX = G^T dY + diag(d) B Q^T, dC += dS B + diag(e) dY H,
 //        dB += dS^T C + diag(d) X Q, and the per-position decay-gradient terms.
 //
-// TMEM lane = tile row; every epilogue is one thread per row (tcgen05.ld 32x32b).  In the walk and the tile kernels one
-// lane of a warp of its own issues the products and one lane of another warp the TMA copies.
+// TMEM lane = tile row (tcgen05.ld 32x32b); the epilogues are the work of row warps, two or four threads to a row.  Products and TMA copies are issued by
+// one lane each of other warps: products that wait for different things by different ones (fwd_walk_kernel, bwd_tile_kernel).
 #pragma once
 #include "ssd_common.cuh"
 #include "ssd_cumsum.cuh"
@@ -47,7 +47,7 @@ inline bool supported(int dtype, int p, int n) {
 // rounded to bf16 here and are fp32 in the kernels of ssd_mma.cuh and ssd_simt.cuh.  Calls that fill whole tiles take that rounding;
 // for others it is the caller's choice (SSD_B200_PATH_TC): the final state of 320 positions in chunks of 80 is 2.4e-3 off
 // the exact one on these kernels, 2.5e-7 in fp32 (and forward + backward of (4, 1984, 20 heads, 64), d_state 64, chunk 64
-// take 168 us here, 303 us there).
+// take 125 us here, 303 us there).
 inline bool whole_tiles(int T, int p, int n, int l) { return p == HP && n == DN && T % LT == 0 && (l % LT == 0 || LT % l == 0); }
 inline int tiles_of(int T) { return (T + LT - 1) / LT; }
 
