@@ -34,8 +34,12 @@
 //   bar_vc[s]  B and C of the tile landed
 //   bar_mh[s]  Hl and Yo of the tile have completed, the store of its entering state has read sH, x of the next tile landed (-> row warps,
 //              loads of B and C)
-//   bar_m2     Yd of the tile and S of the next have completed     (-> row warps; phase = tile parity)
+//   bar_m2[s]  Yd of the tile and S of the next have completed     (-> row warps)
 //   bar_s0, bar_x0   S and x of the first tile
+// Where several warps arrive at an mbarrier, none of them may arrive for a later tile before the others have for this one, or the phase completes without what it
+// stands for.  bar_mh and bar_m2 are two each for that: a warp's next arrival at the same one is two tiles later, behind a hardware barrier that the row
+// warps reach only when they have seen this phase complete.  bar_m2 of tile k: they wait for it ahead of kBarU of tile k + 2 (ahead of Hl, S and the last
+// tile's arrival) and of kBarG (ahead of Yd), but behind kBarU of tile k + 1.  bar_mh of tile k: they wait for it ahead of kBarU of tile k + 1.
 // Named barriers (row warps arrive, control warps wait):
 //   kBarU   weighted rows of a tile and the state entering it written, Hl and Yo of the tile before read (-> Hl, Yo, store of the state)
 //   kBarG   masked operand written                                  (-> Yd)
@@ -91,10 +95,10 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     float* sf = scum + 3 * kFwdRing * LT;                  // [16][32] column factors dt_j 2^(cend - c_j) of each row warp's block
     float* sysq = sf + 4 * LT;                             // [2][2][128] partial sums of y^2 of the odd quarters
     uint64_t* bars = reinterpret_cast<uint64_t*>(sysq + 4 * LT);
-    uint64_t *bar_vc = bars, *bar_mh = bars + 2, *bar_m2 = bars + 4, *bar_s0 = bars + 5, *bar_x0 = bars + 6, *lead_ld = bars + 7, *lead_m = bars + 11;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 15);
-    int& failed = *reinterpret_cast<int*>(bars + 16);
-    int& rows_nt = *reinterpret_cast<int*>(bars + 17);
+    uint64_t *bar_vc = bars, *bar_mh = bars + 2, *bar_m2 = bars + 4, *bar_s0 = bars + 6, *bar_x0 = bars + 7, *lead_ld = bars + 8, *lead_m = bars + 12;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 16);
+    int& failed = *reinterpret_cast<int*>(bars + 17);
+    int& rows_nt = *reinterpret_cast<int*>(bars + 18);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (smem_u32(smem_raw) & 1023u) {  // the swizzled panels need a 1024-byte aligned base: report instead of computing garbage
@@ -117,7 +121,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     if (tid == 0) {
         failed = 0;
         rows_nt = nt;
-        for (int i = 0; i < 15; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 4 : i == 4 ? 2 : 1);  // mh: Hl, Yo, the store of the state, the next tile's x; m2: Yd, the next S
+        for (int i = 0; i < 16; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 4 : i == 4 || i == 5 ? 2 : 1);  // mh: Hl, Yo, the store of the state, the next tile's x; m2: Yd, the next S
         mbar_fence_init();
     }
     if (warp == 16) {
@@ -172,7 +176,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)  // Yd = G' x : A in TMEM (K = j), B = x [j][p] MN-major
                         mma_ts_lo(tYd, tG + kk * 8, uMN + offMN(kk), kIdescKM, kk > 0);
-                    mma_commit(bar_m2);
+                    mma_commit(&bar_m2[it & 1]);
                 }
                 if (++r == kFwdRing) r = 0;
             }
@@ -261,7 +265,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 const uint32_t vK = fresh(stK + (uint32_t)(it & 1) * SU), cK = vK + 2 * PU, tS = tm + (it & 1) * 128;
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) mma_ss_lo(tS, cK + offK(kk), vK + offK(kk), kIdescS, kk > 0);
-                mma_commit(it > 0 ? bar_m2 : bar_s0);
+                mma_commit(it > 0 ? &bar_m2[(it - 1) & 1] : bar_s0);
             };
             if (!hl && lead > 0) named_barrier(kBarLead, 576);
             if (hl) {
@@ -307,7 +311,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     mma_commit(&bar_mh[it & 1]);
                     if (hl) {
                         if (it + 1 < nt) issue_S(it + 1);
-                        else mbar_arrive(bar_m2);  // (no S behind it)
+                        else mbar_arrive(&bar_m2[it & 1]);  // (no S behind it)
                     } else if (it + 2 < nt) {
                         mbar_wait(&bar_mh[it & 1], (it >> 1) & 1, &failed);  // Hl and Yo (and S) of the tile, the readers of its stage, have completed
                         load_vc(it + 2);
@@ -522,7 +526,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     const uint4 v = *reinterpret_cast<const uint4*>(sU + sw128(row, q * 2 + ch));
                     xrow[ch * 4 + 0] = v.x; xrow[ch * 4 + 1] = v.y; xrow[ch * 4 + 2] = v.z; xrow[ch * 4 + 3] = v.w;
                 }
-                mbar_wait(bar_m2, ph, &failed);
+                mbar_wait(&bar_m2[ph], (it >> 1) & 1, &failed);
                 tc_fence_after();
                 tmem_ld16(tYd + lanes + q * 16, a);
                 tmem_ld_wait();
