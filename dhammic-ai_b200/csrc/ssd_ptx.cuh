@@ -2,8 +2,8 @@
 // (cp.async.bulk.tensor, no cluster multicast anywhere), tcgen05 MMA / TMEM, and the
 // shared-memory / instruction descriptors of tcgen05.mma.
 //
-// Every wait is bounded: a wait that runs out sets a flag the caller turns into an error status
-// (no trap, no endless spin).
+// Every wait for an mbarrier is bounded: one that runs out clears a word of the block (`alive`), on which all others give up too, and which the block turns into
+// an error status at its end (no trap, no endless spin).  Hardware barriers know no limit; until_taken keeps them from waiting for good in such a block.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -59,8 +59,8 @@ __device__ __forceinline__ uint32_t mbar_arrive_if_token(uint64_t* bar, bool pre
         : "memory");
     return lo;
 }
-// Bounded waits: they give up when the limit is reached or when another wait of this block has given up (*failed, in shared memory, is set
-// then), so a broken pipeline drains quickly instead of spinning.  Written out because their size counts: left to the compiler a wait is four polls
+// Bounded waits: they give up when the limit is reached or when another wait of this block has given up (*alive, in shared memory and above zero until
+// then, is zero), so a broken pipeline drains quickly instead of spinning.  Written out because their size counts: left to the compiler a wait is four polls
 // and 50 instructions, and the tile kernels, whose warps run some ten loops at once, no longer fit the instruction cache.
 constexpr uint32_t kSpinLimit = 4u << 20;
 #define SSD_MBAR_WAIT(poll)                                                                 \
@@ -71,26 +71,35 @@ constexpr uint32_t kSpinLimit = 4u << 20;
         "mbarrier." poll ".parity.shared::cta.b64 p, [%0], %1;\n\t"                         \
         "@p bra DONE;\n\t"                                                                  \
         "ld.volatile.shared.b32 f, [%2];\n\t"                                               \
-        "setp.ne.b32 p, f, 0;\n\t"                                                          \
+        "setp.le.s32 p, f, 0;\n\t"                                                          \
         "@p bra DONE;\n\t"                                                                  \
         "add.s32 n, n, -1;\n\t"                                                             \
         "setp.ne.b32 p, n, 0;\n\t"                                                          \
         "@p bra WAIT;\n\t"                                                                  \
-        "mov.b32 f, 1;\n\t"                                                                 \
+        "mov.b32 f, 0;\n\t"                                                                 \
         "st.volatile.shared.b32 [%2], f;\n"                                                 \
         "DONE:\n\t}"                                                                        \
-        ::"r"(smem_u32(bar)), "r"(parity), "r"(smem_u32((const void*)failed)), "r"(limit)   \
+        ::"r"(smem_u32(bar)), "r"(parity), "r"(smem_u32((const void*)alive)), "r"(limit)    \
         : "memory")
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = kSpinLimit) {
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* alive, uint32_t limit = kSpinLimit) {
     SSD_MBAR_WAIT("try_wait");
 }
 // The same for phases that other threads complete with mbarrier.arrive: polls without suspending.  (try_wait may suspend the thread for a
 // system-chosen time while the phase is open; a waiter that polled just before the last arrive of OTHER THREADS saw the phase about
 // 0.75 us late, while completions by tcgen05.commit or TMA bytes woke it at once.)
-__device__ __forceinline__ void mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* failed, uint32_t limit = 16u * kSpinLimit) {
+__device__ __forceinline__ void mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* alive, uint32_t limit = 16u * kSpinLimit) {
     SSD_MBAR_WAIT("test_wait");
 }
 #undef SSD_MBAR_WAIT
+__device__ __forceinline__ bool gave_up(const volatile int* alive) { return *alive <= 0; }
+// The end of a block, every thread's: what it reports; and where a wait gave up, a millisecond in which copies that are still on their way land before its
+// shared memory is another block's.
+__device__ __forceinline__ void end_of_waits(const volatile int* alive, int* status) {
+    if (!gave_up(alive)) return;
+    if (threadIdx.x == 0) atomicExch(status, 1);
+#pragma unroll 1
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+}
 
 // ---------------------------------------------------------------- proxy fences
 __device__ __forceinline__ void fence_async_smem() {  // generic-proxy smem writes -> visible to TMA / tcgen05
@@ -163,6 +172,40 @@ __device__ __forceinline__ void setmaxnreg_inc() {
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// Hand-over by a hardware barrier: the warps that make something are counted in without waiting, the few that go on with it wait in named_bar_sync.
+// A maker must not be counted twice in one turn of a barrier.  The waits between two hand-overs see to that, since they stand for what the takers do behind
+// their barrier, until one gives up: then they stand for nothing.  So the takers keep count of the turns that are over, and every maker looks once a round,
+// behind the wait that its next hand-overs rely on, whether a wait has given up (nothing had then, in the whole block, if not), and if so waits until those
+// turns are over.  A block whose warps reach its barriers in one order, each warp some of them, comes to its end with this whatever wait runs out: the
+// first barrier in that order that is not over lacks only warps that no later one holds back.
+__device__ __forceinline__ void hand_over(int id, int count) {
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+// taken: the takers' counts, four words, of which each says how many rounds may begin, and which start where the makers' first round needs them (what is not
+// used at kTakenAll).  Bounded all the same.
+constexpr int kTakenAll = 0x7fffffff;
+__device__ __forceinline__ void until_taken(int late, const int4* taken, int round) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b32 n, a, b, c, d;\n\t"
+        "setp.eq.s32 p, %0, 0;\n\t"
+        "@p bra DONE;\n\t"
+        "mov.b32 n, %3;\n"
+        "AGAIN:\n\t"
+        "ld.volatile.shared.v4.b32 {a, b, c, d}, [%1];\n\t"
+        "min.s32 a, a, b;\n\t"
+        "min.s32 c, c, d;\n\t"
+        "min.s32 a, a, c;\n\t"
+        "setp.gt.s32 p, a, %2;\n\t"
+        "@p bra DONE;\n\t"
+        "add.s32 n, n, -1;\n\t"
+        "setp.ne.b32 p, n, 0;\n\t"
+        "@p bra AGAIN;\n"
+        "DONE:\n\t}"
+        ::"r"(late), "r"(smem_u32(taken)), "r"(round), "r"(16u * kSpinLimit)
+        : "memory");
+}
+__device__ __forceinline__ void set_taken(int* count, int rounds) { *(volatile int*)count = rounds; }
 
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

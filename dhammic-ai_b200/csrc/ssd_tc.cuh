@@ -202,16 +202,16 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const float* __restric
 // gives up, records it in the status word exactly as the tile kernels do, and returns.  The context stays usable.
 __global__ void __launch_bounds__(32) bounded_wait_selftest_kernel(int* status, int polls) {
     __shared__ uint64_t bar;
-    __shared__ int failed;
+    __shared__ int alive;
     if (threadIdx.x == 0) {
-        failed = 0;
+        alive = 1;
         mbar_init(&bar, 1);
         mbar_fence_init();
     }
     __syncwarp();
-    mbar_wait(&bar, 0, &failed, (uint32_t)polls);
+    mbar_wait(&bar, 0, &alive, (uint32_t)polls);
     __syncwarp();
-    if (threadIdx.x == 0 && failed) atomicExch(status, 1);
+    if (threadIdx.x == 0 && gave_up(&alive)) atomicExch(status, 1);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -66,8 +66,9 @@ struct BwdParams {
 // [2][3][4][128] | warp partials [2][16] | barriers
 constexpr size_t kBwdSmem = 13 * PANEL + 6 * LT * 4 + 4 * LT * 4 + 24 * LT * 4 + 128 + 192;
 static_assert(kBwdSmem <= 227 * 1024, "more shared memory than a CTA can have");
-// named barriers: all row warps arrive, control warps wait (kBwdBarE: three of them, the others one); among row warps: the rows 96-127, all
-constexpr int kBwdBarA = 1, kBwdBarB = 2, kBwdBarE = 3, kBwdBarC = 4, kBwdBarG1 = 5, kBwdBarG2 = 6, kBwdBarLow = 7, kBwdBarRows = 8, kBwdBarQ = 9;
+// named barriers: all row warps arrive, control warps wait (kBwdBarE: three of them, the others one; kBwdBarA, B and C are two by head parity: see until_taken);
+// among row warps: the rows 96-127, all; kBwdBarQ: warp 16 arrives, 18 waits
+constexpr int kBwdBarA = 1 /* and 2 */, kBwdBarB = 3 /* and 4 */, kBwdBarC = 5 /* and 6 */, kBwdBarE = 7, kBwdBarG1 = 8, kBwdBarG2 = 9, kBwdBarLow = 10, kBwdBarRows = 11, kBwdBarQ = 12;
 constexpr int kBwdThreads = 640;  // 16 row warps + the control warpgroup (registers are budgeted per warpgroup)
 // Registers per thread: at launch, and after the two warpgroup kinds have traded (setmaxnreg.inc waits for the pool, so the
 // sum after the trade must not exceed what the CTA was launched with)
@@ -103,7 +104,9 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
     uint64_t *bar_cb = bars, *bar_xy = bars + 1, *bar_hq = bars + 3, *bar_m2y = bars + 4, *bar_m2b = bars + 5, *bar_m3 = bars + 6, *bar_sr2 = bars + 7,
              *bar_m1 = bars + 8, *bar_m2 = bars + 9;
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 10);
-    int& failed = *reinterpret_cast<int*>(bars + 11);
+    int& alive = *reinterpret_cast<int*>(bars + 11);
+    // see until_taken: .x kBwdBarA, .y kBwdBarB, kBwdBarQ and (with an item's last head) kBwdBarG1, .z kBwdBarE, kBwdBarC and (likewise) kBwdBarG2
+    int4& taken = *reinterpret_cast<int4*>(bars + 12);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (smem_u32(smem_raw) & 1023u) {  // the swizzled panels need a 1024-byte aligned base: report instead of computing garbage
@@ -134,7 +137,8 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
     };
 
     if (tid == 0) {
-        failed = 0;
+        alive = 1;
+        taken = make_int4(0, 1, 1, kTakenAll);
         for (int i = 0; i < 10; ++i) mbar_init(&bars[i], i < 8 ? 1 : 2);
         mbar_fence_init();
     }
@@ -176,7 +180,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         const uint32_t hMN = desc_lo(smem_u32(sH), PANEL), qMN = desc_lo(smem_u32(sQ), PANEL);
         const uint32_t xyK = desc_lo(smem_u32(sXY), 16);  // x of buffer 0; dy +PANEL, buffer 1 +2 PANEL (in 16-byte units)
         auto issue_dG = [&](uint32_t hcur) {  // dG = dY x^T (K = p) of the head with running index hcur
-            mbar_wait(&bar_xy[hcur & 1], (hcur >> 1) & 1, &failed);  // prefetched during the head before
+            mbar_wait(&bar_xy[hcur & 1], (hcur >> 1) & 1, &alive);  // prefetched during the head before
             tc_fence_after();
             const uint32_t x0 = fresh(xyK + 2 * PU * (hcur & 1)), y0 = x0 + PU;
 #pragma unroll
@@ -190,12 +194,12 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             for (int hl = 0; hl < hpg; ++hl, ++hcur) {
                 const uint32_t ph = hcur & 1;
                 if (lane == 0) {
-                    if (hcur > 0) mbar_wait(bar_m2b, ph ^ 1, &failed);  // dYe of the head before is read
+                    if (hcur > 0) mbar_wait(bar_m2b, ph ^ 1, &alive);  // dYe of the head before is read
                     issue_dG(hcur);  // over its Yo and dYe
-                    mbar_wait(bar_hq, ph, &failed);  // H and Q of this head have landed
+                    mbar_wait(bar_hq, ph, &alive);  // H and Q of this head have landed
                 }
                 __syncwarp();
-                named_bar_sync(kBwdBarA, 544);  // G complete, S and dG read by every row
+                named_bar_sync(kBwdBarA + ph, 544);  // G complete, S and dG read by every row
                 if (lane == 0) {
                     tc_fence_after();
                     const uint32_t yMN = fresh(xyK + 2 * PU * ph) + PU + ((PANEL >> 4) << 16) - (1u << 16);  // dy of this head, MN-major
@@ -211,9 +215,10 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                     for (int kk = 0; kk < 8; ++kk)  // dX2 = B Q^T : A = B K-major (K = n), B = Q^T [n][p] MN-major
                         mma_ss_lo(tX2, bK_ + offK(kk), qMN_ + offMN(kk), kIdescKM, kk > 0);
                     mma_commit(bar_m2);  // ... and goes on with dX1 and dX2
+                    set_taken(&taken.x, hcur + 1);
+                    until_taken(gave_up(&alive), &taken, hcur);
                 }
-                __syncwarp();
-                named_arrive(kBwdBarQ, 64);
+                hand_over(kBwdBarQ, 64);
                 named_bar_sync(kBwdBarE, 608);  // every row has read Yo, dX1 and dX2
             }
         }
@@ -252,7 +257,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             // between two items (and before the first, behind the last)
             const bool on = item < P.items;
             if (lane == 0) {
-                if (ic > 0) mbar_wait(bar_m3, (ic - 1) & 1, &failed);
+                if (ic > 0) mbar_wait(bar_m3, (ic - 1) & 1, &alive);
                 // C, B, H, Q are free: the item's loads go out before the group terms of the one before are stored
                 if (on) {
                     mbar_expect_tx(bar_cb, 4 * PANEL);
@@ -275,6 +280,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                         tma_store_4d(&P.mdB, sdBst + PANEL, 64, done.gg, done.k * LT, done.bb);
                     }
                     tma_store_commit();
+                    set_taken(&taken.z, hcur + 1);
                     tma_store_wait_read();  // shared memory must outlive the reads only (the writes complete with the kernel)
                     mbar_arrive(bar_sr2);
                 }
@@ -302,7 +308,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                 __syncwarp();
                 named_bar_sync(kBwdBarE, 608);
                 if (lane == 0) {
-                    mbar_wait(bar_m2b, hcur & 1, &failed);
+                    mbar_wait(bar_m2b, hcur & 1, &alive);
                     const bool last = hl + 1 == hpg;
                     if (!last) load_hq(done, hl + 1);
                     // x / dy of the head after the next; with the last head, of the next item's first into the buffer of the head before this one (this head's
@@ -310,10 +316,11 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                     if (last ? more : hl + 2 < hpg) load_xy(last ? at : done, last ? 0 : hl + 2, last ? hcur + 1 : hcur);
                 }
                 __syncwarp();
-                named_bar_sync(kBwdBarC, 544);  // dx staged
+                named_bar_sync(kBwdBarC + (hcur & 1), 544);  // dx staged
                 if (lane == 0) {
                     tma_store_4d(&P.mdX, sdX, 0, done.gg * hpg + hl, done.k * LT, done.bb);
                     tma_store_commit();
+                    if (hl + 1 < hpg) set_taken(&taken.z, hcur + 2);
                     tma_store_wait_read();
                     mbar_arrive(bar_m2);  // the dx staging panel may be rewritten
                 }
@@ -330,9 +337,9 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
 #pragma unroll 1
             for (int hl = 0; hl < hpg; ++hl, ++hcur) {
                 const uint32_t ph = hcur & 1;
-                if (lane == 0) mbar_wait(bar_hq, ph, &failed);
+                if (lane == 0) mbar_wait(bar_hq, ph, &alive);
                 __syncwarp();
-                named_bar_sync(kBwdBarB, 544);  // Xd, dYe complete
+                named_bar_sync(kBwdBarB + ph, 544);  // Xd, dYe complete
                 named_bar_sync(kBwdBarQ, 64);   // the products of the epilogue are ahead in the queue
                 if (lane == 0) {
                     tc_fence_after();
@@ -344,6 +351,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                     for (int kk = 0; kk < 4; ++kk)  // dB += Xd Q : A = Xd K-major (in place of x), B = Q^T [n][p] K-major
                         mma_ss_lo(tdB, x0 + 2 * kk, qK_ + 2 * kk, kIdescKK128, hl > 0 || kk > 0);
                     mma_commit(bar_m2b);  // releases H, Q, Xd and the dYe columns
+                    if (hl + 1 < hpg) set_taken(&taken.y, hcur + 2);
                 }
             }
             __syncwarp();
@@ -358,6 +366,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                 for (int kk = 0; kk < 8; ++kk)  // dB += dS^T C : A = dS MN-major (M = j, K = i), B = C [i][n] MN-major
                     mma_ss_lo<true>(tdB, hMN_ + offMN(kk), cMN_ + offMN(kk), kIdescMM128);
                 mma_commit(bar_m3);
+                set_taken(&taken.y, hcur + 1);
             }
         }
     } else {
@@ -366,7 +375,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         uint32_t hcur = 0, ic = 0;
 #pragma unroll 1
         for (int item = item0; item < P.items; item += (int)gridDim.x, ++ic) {
-            if (lane == 0) mbar_wait(bar_cb, ic & 1, &failed);  // (loaded behind the group terms of the item before)
+            if (lane == 0) mbar_wait(bar_cb, ic & 1, &alive);  // (loaded behind the group terms of the item before)
 #pragma unroll 1
             for (int hl = 0; hl < hpg; ++hl, ++hcur) {
                 if (lane == 0) {
@@ -377,7 +386,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                         mma_ss_lo(tS, c + offK(kk), b + offK(kk), kIdescKK128, kk > 0);  // the rows finish its epilogue
                     // of an item's first head announced when the stores of dC and dB have read their staging panels: the rows overwrite the G panels
                     // right after bar_m1
-                    if (hl == 0 && ic > 0) mbar_wait_spin(bar_sr2, (ic - 1) & 1, &failed);
+                    if (hl == 0 && ic > 0) mbar_wait_spin(bar_sr2, (ic - 1) & 1, &alive);
                     mma_commit(bar_m1);
                 }
                 __syncwarp();
@@ -396,18 +405,13 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
     const bool active = qc <= rb, diag = qc == rb;
     const uint32_t lanes = lane_base(warp);
     float* wsf = sf + warp * 32;
-    // every lane has fenced its own writes; the warp meets and is counted in
-    auto warp_arrive = [&](int id, int count) {
-        __syncwarp();
-        named_arrive(id, count);
-    };
     // G panel and 16-byte chunk of this thread's two 16-column steps
     uint8_t* sGq = sG + (qc >> 1) * PANEL;
     const int gch = (qc & 1) * 4;
     // Before a head's S and dG are there: its x, dy and scalars have landed; the column factors of this warp's block.
     auto enter = [&](uint32_t hcur) {
         const int xb = hcur & 1;
-        mbar_wait(&bar_xy[xb], (hcur >> 1) & 1, &failed);
+        mbar_wait(&bar_xy[xb], (hcur >> 1) & 1, &alive);
         const float* sc = scal + xb * 3 * LT;
         if (active) wsf[lane] = exp2f(sc[qc * 32 + 31] - sc[qc * 32 + lane]);
         __syncwarp();
@@ -443,7 +447,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             uint8_t* sdY = sX + PANEL;
             const float c_i = sc[row];
             const float rf = active ? exp2f(c_i - sc[qc * 32 + 31]) : 0.f;
-            mbar_wait(bar_m1, ph, &failed);
+            mbar_wait(bar_m1, ph, &alive);
             tc_fence_after();
             float2 rowacc2 = make_float2(0.f, 0.f);
             if (active) {
@@ -506,7 +510,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             // (A) this thread's part of G is complete and its S / dG entries are read: Yo, dX1, dX2 are issued
             tc_fence_before();
             fence_async_smem();
-            warp_arrive(kBwdBarA, 544);
+            hand_over(kBwdBarA + ph, 544);
             // dYe goes where the last column quarter of dG was: the rows 96-127 wait for their quarter-3 warp to have read it
             if (rb == 3) named_bar_sync(kBwdBarLow, 128);
             const float Sk = sc[LT - 1], dtv = sc[LT + row], Dh = P.skipT ? sc[2 * LT + row] : Dhead;
@@ -538,7 +542,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             // products pair up chunk by chunk whatever the swizzle: 1024 chunks of 16 bytes.
             float qh_acc = 0.f;
             if (!active) {
-                mbar_wait(bar_hq, ph, &failed);
+                mbar_wait(bar_hq, ph, &alive);
                 float2 q2 = make_float2(0.f, 0.f);
 #pragma unroll 2
                 for (int c = (rb * (5 - rb) / 2 + qc - 1) * 32 + lane; c < 1024; c += 192) {  // rb 0: qc 1..3, rb 1: 2, 3, rb 2: 3
@@ -556,7 +560,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             // (B) Xd, dYe complete: dC, dB are issued
             tc_fence_before();
             fence_async_smem();
-            warp_arrive(kBwdBarB, 544);
+            hand_over(kBwdBarB + ph, 544);
             float ddt_acc, st_acc, yo_acc, dyx;
             {
                 uint32_t yr[8];
@@ -565,8 +569,9 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                     uint4 u = *reinterpret_cast<const uint4*>(sdY + sw128(row, qc * 2 + ch));
                     yr[ch * 4 + 0] = u.x; yr[ch * 4 + 1] = u.y; yr[ch * 4 + 2] = u.z; yr[ch * 4 + 3] = u.w;
                 }
+                until_taken(gave_up(&alive), &taken, (int)hcur);  // (what was waited for has A, B, E before this head's behind it, C before the last head's, and G1, G2)
                 // e_i <dY_i, Yo_i> over this thread's 16 columns (Yo = C H^T is the first product of the group)
-                mbar_wait(bar_m2y, ph, &failed);
+                mbar_wait(bar_m2y, ph, &alive);
                 tc_fence_after();
                 {
                     uint32_t o[16];
@@ -580,7 +585,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                     yo_acc = ei * (r2.x + r2.y);
                 }
                 if (hcur > 0) emit(hcur - 1);  // while dX1 and dX2 run (its partials were written before Yo was issued)
-                mbar_wait(bar_m2, ph, &failed);
+                mbar_wait(bar_m2, ph, &alive);
                 tc_fence_after();
                 // fp32 pairs throughout: e = dX1 + d dX2, dx = dt e + D dy, and the row sums <e, x>, <dX2, x>, <dy, x>
                 float2 ddt2 = make_float2(0.f, 0.f), st2 = make_float2(0.f, 0.f), yx2 = make_float2(0.f, 0.f);
@@ -591,7 +596,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                 tmem_ld_wait();
                 // (E) Yo, dX1 and dX2 are in registers: the accumulators of this head may be overwritten
                 tc_fence_before();
-                warp_arrive(kBwdBarE, 608);
+                hand_over(kBwdBarE, 608);
                 const float2* A2 = reinterpret_cast<const float2*>(a);
                 const float2* S2 = reinterpret_cast<const float2*>(b2);
                 uint32_t dxp[8];
@@ -614,7 +619,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
             }
             // (C) dx staged: the TMA warp stores it
             fence_async_smem();
-            warp_arrive(kBwdBarC, 544);
+            hand_over(kBwdBarC + ph, 544);
             {
                 // gradient w.r.t. the tile-cumulative log-decay of this row, one partial per quarter, summed during the
                 // next head; the terms that act through S = cum[127] (state weights d_j, and the decay of the entering
@@ -633,7 +638,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         // ---- group terms: stage sum_h dS as bf16 [i][j] (panel = column half) in the H / Q panels for the two
         // closing products
         const uint32_t hlast = hc + hpg - 1;
-        mbar_wait(bar_m2b, hlast & 1, &failed);  // the last head's products have read H, Q, Xd / dY
+        mbar_wait(bar_m2b, hlast & 1, &alive);  // the last head's products have read H, Q, Xd / dY
         {
             float v[32];
 #pragma unroll
@@ -645,8 +650,8 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         }
         tc_fence_before();
         fence_async_smem();
-        warp_arrive(kBwdBarG1, 544);
-        mbar_wait(bar_m3, ic & 1, &failed);
+        hand_over(kBwdBarG1, 544);
+        mbar_wait(bar_m3, ic & 1, &alive);
         tc_fence_after();
         uint8_t* sdBst = sXY + (2 * (hlast & 1)) * PANEL;  // dB staging: the last head's x / dy buffer
         {
@@ -664,7 +669,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
         }
         tc_fence_before();
         fence_async_smem();
-        warp_arrive(kBwdBarG2, 544);  // dC, dB staged and read out of TMEM: the TMA warp stores them
+        hand_over(kBwdBarG2, 544);  // dC, dB staged and read out of TMEM: the TMA warp stores them
         hc += hpg;
         ic += 1;
         item += (int)gridDim.x;
@@ -676,7 +681,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
   }
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && failed) atomicExch(P.status, 1);
+    end_of_waits(&alive, P.status);
     if (warp == 1) tmem_dealloc(tm, 512);
 }
 

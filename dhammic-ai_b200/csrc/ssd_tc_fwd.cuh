@@ -42,7 +42,7 @@
 // tile's arrival) and of kBarG (ahead of Yd), but behind kBarU of tile k + 1.  bar_mh of tile k: they wait for it ahead of kBarU of tile k + 1.
 // Named barriers (row warps arrive, control warps wait):
 //   kBarU   weighted rows of a tile and the state entering it written, Hl and Yo of the tile before read (-> Hl, Yo, store of the state)
-//   kBarG   masked operand written                                  (-> Yd)
+//   kBarG   masked operand written                                  (-> Yd; two by tile parity: see until_taken)
 //   kBarH   y staged over x, the tile's x and scalars no longer used (-> store of y, next load into the slot; two by tile parity: the row warps
 //           may arrive once more before the store's warp has seen the last one)
 // The per-half-row sums of y^2 keep their (b, T/128, h, 2, 128) layout: the odd quarter of each half leaves its partial
@@ -65,7 +65,7 @@ constexpr int kFwdStages = 2, kFwdRing = 3;
 // each row warp [16][32] | partial sums of y^2 [2][2][128] | barriers
 constexpr size_t kFwdSmem = kFwdStages * (size_t)kFwdStageBytes + (kFwdRing + 2) * (size_t)PANEL + (3 * kFwdRing + 4 + 4) * LT * 4 + 192;
 // named barriers: all row warps arrive, one or three control warps wait
-constexpr int kBarG = 1, kBarU = 2, kBarH = 3 /* and 4 */, kBarRows = 5, kBarLead = 6, kBarLeadU = 7 /* and 8 */;
+constexpr int kBarG = 1 /* and 2 */, kBarU = 3, kBarH = 4 /* and 5 */, kBarRows = 6, kBarLead = 7, kBarLeadU = 8 /* and 9 */;
 constexpr int kLeadStages = 4;  // of [V panels 0,1 | x], over everything in front of the state
 static_assert(kFwdSmem <= 227 * 1024, "more shared memory than a CTA can have");
 
@@ -97,8 +97,10 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     uint64_t* bars = reinterpret_cast<uint64_t*>(sysq + 4 * LT);
     uint64_t *bar_vc = bars, *bar_mh = bars + 2, *bar_m2 = bars + 4, *bar_s0 = bars + 6, *bar_x0 = bars + 7, *lead_ld = bars + 8, *lead_m = bars + 12;
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 16);
-    int& failed = *reinterpret_cast<int*>(bars + 17);
-    int& rows_nt = *reinterpret_cast<int*>(bars + 18);
+    int& alive = *reinterpret_cast<int*>(bars + 17);
+    int& rows_nt = *reinterpret_cast<int*>(bars + 18);  // (`alive` is the same until a wait gives up)
+    // see until_taken: .x kBarG, .y kBarU and kBarH; kBarLeadU
+    int4 &taken = *reinterpret_cast<int4*>(bars + 20), &taken_lead = *reinterpret_cast<int4*>(bars + 22);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (smem_u32(smem_raw) & 1023u) {  // the swizzled panels need a 1024-byte aligned base: report instead of computing garbage
@@ -119,7 +121,9 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     const size_t bh = (size_t)bb * P.h + hh;
 
     if (tid == 0) {
-        failed = 0;
+        alive = nt;
+        taken = make_int4(1, 0, kTakenAll, kTakenAll);
+        taken_lead = make_int4(0, kTakenAll, kTakenAll, kTakenAll);
         rows_nt = nt;
         for (int i = 0; i < 16; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 4 : i == 4 || i == 5 ? 2 : 1);  // mh: Hl, Yo, the store of the state, the next tile's x; m2: Yd, the next S
         mbar_fence_init();
@@ -169,7 +173,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
 #pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 __syncwarp();
-                named_barrier(kBarG, 544);
+                named_barrier(kBarG + (it & 1), 544);
                 if (lane == 0) {
                     tc_fence_after();
                     const uint32_t uMN = fresh(xMN + (uint32_t)r * PU);
@@ -177,6 +181,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     for (int kk = 0; kk < 8; ++kk)  // Yd = G' x : A in TMEM (K = j), B = x [j][p] MN-major
                         mma_ts_lo(tYd, tG + kk * 8, uMN + offMN(kk), kIdescKM, kk > 0);
                     mma_commit(&bar_m2[it & 1]);
+                    set_taken(&taken.x, it + 2);
                 }
                 if (++r == kFwdRing) r = 0;
             }
@@ -213,7 +218,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     for (int it = 0; it < lead; ++it) {
                         const int s = it % kLeadStages, pos = it * LT;
                         uint8_t* st = smem_raw + s * 3 * PANEL;
-                        if (it >= kLeadStages) mbar_wait(&lead_m[s], (it / kLeadStages - 1) & 1, &failed);  // the stage's product before is done
+                        if (it >= kLeadStages) mbar_wait(&lead_m[s], (it / kLeadStages - 1) & 1, &alive);  // the stage's product before is done
                         mbar_expect_tx(&lead_ld[s], 3 * PANEL);
                         tma_load_4d(st + 2 * PANEL, &P.mU, &lead_ld[s], 0, hh, pos, bb);
                         tma_load_4d(st, &P.mV, &lead_ld[s], 0, gg, pos, bb);
@@ -239,6 +244,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     if (lane == 0) store_y(it - 1);
                 }
                 if (lane == 0) {
+                    set_taken(&taken.y, it + 1);
                     if (it > 0) tma_store_wait_read<1>();
                     else tma_store_wait_read();
                     mbar_arrive(&bar_mh[it & 1]);  // the store has read sH
@@ -260,7 +266,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             const bool hl = warp == 18;
             const uint32_t udMN = desc_lo(smem_u32(sUd), PANEL), hMN = desc_lo(smem_u32(sH), PANEL);
             auto issue_S = [&](int it) {  // S = C B^T of tile `it` into TMEM buffer it & 1, which the rows have masked two tiles before
-                mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &failed);
+                mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &alive);
                 tc_fence_after();
                 const uint32_t vK = fresh(stK + (uint32_t)(it & 1) * SU), cK = vK + 2 * PU, tS = tm + (it & 1) * 128;
 #pragma unroll
@@ -280,6 +286,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                         for (int kk = 0; kk < 8; ++kk)  // V^T [d dt o x]
                             mma_ss_lo(tYo + (it & 1) * 64, st + offMN(kk), st + 2 * PU + offMN(kk), kIdescMM, kk > 0);
                         mma_commit(&lead_m[it % kLeadStages]);
+                        set_taken(&taken_lead.x, it + 1);
                     }
                 }
             }
@@ -292,7 +299,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             if (hl && lane == 0) issue_S(0);
 #pragma unroll 1
             for (int it = 0; it < nt; ++it) {
-                if (!hl && lane == 0) mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &failed);
+                if (!hl && lane == 0) mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &alive);
                 __syncwarp();
                 named_barrier(kBarU, 608);  // weighted rows and entering state written, Hl and Yo of the tile before read
                 if (lane == 0) {
@@ -313,7 +320,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                         if (it + 1 < nt) issue_S(it + 1);
                         else mbar_arrive(&bar_m2[it & 1]);  // (no S behind it)
                     } else if (it + 2 < nt) {
-                        mbar_wait(&bar_mh[it & 1], (it >> 1) & 1, &failed);  // Hl and Yo (and S) of the tile, the readers of its stage, have completed
+                        mbar_wait(&bar_mh[it & 1], (it >> 1) & 1, &alive);  // Hl and Yo (and S) of the tile, the readers of its stage, have completed
                         load_vc(it + 2);
                     }
                 }
@@ -323,7 +330,6 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     } else {
         // ------------------------------------------------------------------ row warps: thread = (row, column quarter)
         setmaxnreg_inc<kFwdRegsRow>();
-        const volatile int& rnt = rows_nt;  // in shared memory: the row warps have no register left for it
         const int rb = row >> 5;  // row block, warp-uniform
         const bool active = q <= rb, diag = q == rb;
         const uint32_t lanes = lane_base(warp);
@@ -367,8 +373,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             *reinterpret_cast<uint4*>(sUd + sw128(row, q * 2 + 1)) = make_uint4(xw[4], xw[5], xw[6], xw[7]);
             tc_fence_before();
             fence_async_smem();
-            __syncwarp();
-            named_arrive(kBarU, 608);
+            hand_over(kBarU, 608);
         };
         float ysq_own = 0.f;  // even quarters: own partial of the tile before
         if (lead > 0) {
@@ -381,7 +386,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 const float dec = exp2f(it < 0 ? 0.f : Sk);
                 if (it + 1 < lead) {
                     const int s = (it + 1) % kLeadStages;
-                    mbar_wait(&lead_ld[s], ((it + 1) / kLeadStages) & 1, &failed);
+                    mbar_wait(&lead_ld[s], ((it + 1) / kLeadStages) & 1, &alive);
                     uint8_t* sU = smem_raw + (s * 3 + 2) * PANEL;
                     const __nv_bfloat162 w2 = __float2bfloat162_rn(exp2f(S - c) * d);
 #pragma unroll
@@ -399,8 +404,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     Sk = S;
                     tc_fence_before();
                     fence_async_smem();
-                    __syncwarp();
-                    named_arrive(kBarLeadU + ((it + 1) & 1), 544);
+                    hand_over(kBarLeadU + ((it + 1) & 1), 544);
                     if (it + 2 < lead) {
                         const int o = (it + 2) * LT;
                         c = tc[o + row];
@@ -409,7 +413,8 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     }
                 }
                 if (it >= 0) {
-                    mbar_wait(&lead_m[it % kLeadStages], (it / kLeadStages) & 1, &failed);
+                    mbar_wait(&lead_m[it % kLeadStages], (it / kLeadStages) & 1, &alive);
+                    until_taken(gave_up(&alive), &taken_lead, it);
                     tc_fence_after();
                     uint32_t r[16];
                     tmem_ld16(tYo + (it & 1) * 64 + lanes + q * 16, r);
@@ -420,20 +425,19 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     for (int j = 0; j < 8; ++j) H2[j] = fma2(d2, H2[j], reinterpret_cast<const float2*>(r)[j]);
                 }
             }
-            __syncwarp();
-            named_arrive(kBarLead, 576);  // the panels are free
+            hand_over(kBarLead, 576);  // the panels are free
         }
         store_quarter_row(sH, row, q * 2, H);
-        mbar_wait(bar_x0, 0, &failed);
+        mbar_wait(bar_x0, 0, &alive);
         weigh(0);
         put_weighted();
         factors(0);
-        mbar_wait(bar_s0, 0, &failed);
+        mbar_wait(bar_s0, 0, &alive);
         tc_fence_after();
         int ring = 0;  // it % 3
 
 #pragma unroll 1
-        for (int it = 0; it < rnt; ++it) {
+        for (int it = 0;;) {
             const uint32_t ph = it & 1;
             const float e = exp2f(c_i), dec = exp2f(Sk);
             const float* sc = scum + ring * 3 * LT;
@@ -490,19 +494,19 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 tmem_st_wait();
             }
             tc_fence_before();
-            __syncwarp();
-            named_arrive(kBarG, 544);
+            hand_over(kBarG + ph, 544);
 
             // while Yd runs: what the next tile needs early, and the state update
             uint8_t* sU = sRing + ring * PANEL;
             const float Dh = P.skipT ? sc[2 * LT + row] : Dhead;
             if (++ring == kFwdRing) ring = 0;
-            mbar_wait(&bar_mh[ph], (it >> 1) & 1, &failed);  // Hl and Yo have completed, so sH and sUd are free; the next tile's x is there
+            mbar_wait(&bar_mh[ph], (it >> 1) & 1, &alive);  // Hl and Yo have completed, so sH and sUd are free; the next tile's x is there
             tc_fence_after();
             if (P.ysq && it > 0 && !(q & 1))  // the sum of the half row of the tile before: own quarter + the odd one's (written before this tile's mask)
                 P.ysq[((((size_t)bb * P.nt + k0 + (it - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((it - 1) & 1) * 2 + (q >> 1)) * LT + row];
             uint32_t o[16];
+            const int rnt = *(const volatile int*)&alive;  // tiles of the walk (the row warps have no register left for it), or zero
             {
                 uint32_t r[16];
                 tmem_ld16(tHl + lanes + q * 16, r);
@@ -518,6 +522,9 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 store_quarter_row(sH, row, q * 2, H);
                 put_weighted();
                 factors(ring);
+            } else if (rnt <= 0) {
+                until_taken(1, &taken, it);  // U of this tile, H and G of the one before are behind what was waited for
+                if (it + 1 < rows_nt) hand_over(kBarU, 608);
             }
             {
                 uint32_t a[16], xrow[8];
@@ -526,7 +533,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     const uint4 v = *reinterpret_cast<const uint4*>(sU + sw128(row, q * 2 + ch));
                     xrow[ch * 4 + 0] = v.x; xrow[ch * 4 + 1] = v.y; xrow[ch * 4 + 2] = v.z; xrow[ch * 4 + 3] = v.w;
                 }
-                mbar_wait(&bar_m2[ph], (it >> 1) & 1, &failed);
+                mbar_wait(&bar_m2[ph], (it >> 1) & 1, &alive);
                 tc_fence_after();
                 tmem_ld16(tYd + lanes + q * 16, a);
                 tmem_ld_wait();
@@ -552,9 +559,10 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             }
             tc_fence_before();
             fence_async_smem();
-            __syncwarp();
-            named_arrive(kBarH + ph, 544);
+            hand_over(kBarH + ph, 544);
+            if (++it >= *(const volatile int*)&alive && it >= rows_nt) break;
         }
+        const int rnt = rows_nt;
         if (P.ysq) {
             named_barrier(kBarRows, 512);
             if (!(q & 1))
@@ -565,7 +573,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
     }
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && failed) atomicExch(P.status, 1);
+    end_of_waits(&alive, P.status);
     if (warp == 16) tmem_dealloc(tm, 512);
 }
 

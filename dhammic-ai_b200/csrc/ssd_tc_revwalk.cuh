@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
     uint64_t* bar_u = bars + 3;       // [NU]
     uint64_t* bar_m = bars + 7;       // [2]
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 9);
-    int& failed = *reinterpret_cast<int*>(bars + 10);
+    int& alive = *reinterpret_cast<int*>(bars + 10);
+    int4& taken = *reinterpret_cast<int4*>(bars + 12);  // see until_taken: .x kRevBarU, .y kRevBarQ
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (smem_u32(smem_raw) & 1023u) {  // the swizzled panels need a 1024-byte aligned base: report instead of computing garbage
@@ -73,7 +74,8 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
     const int k0 = CUT ? (int)blockIdx.z * P.pt : 0, nt = CUT ? min(P.pt, P.nt - k0) : P.nt;  // the piece's tiles
 
     if (tid == 0) {
-        failed = 0;
+        alive = nt;  // until a wait gives up
+        taken = make_int4(0, 0, kTakenAll, kTakenAll);
         for (int i = 0; i < 9; ++i) mbar_init(&bars[i], i < 7 ? 1 : 2);
         mbar_fence_init();
     }
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
 #pragma unroll 1
         for (int it = 0; it < nt; ++it) {
             const int b = it & 1;
-            if (lane == 0) mbar_wait(&bar_c[sc], cph, &failed);
+            if (lane == 0) mbar_wait(&bar_c[sc], cph, &alive);
             __syncwarp();
             named_barrier(kRevBarU + b, BAR);
             if (lane == 0) {
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
                 for (int kk = 0; kk < 8; ++kk)  // Hl = C^T [e . dY of each head] : both MN-major, K = position, N = 64 NH
                     mma_ss_lo(tm + b * 64 * NH, v + kk * 128, u + kk * 128, NH == 2 ? kIdescMM128 : kIdescMM, kk > 0);
                 mma_commit(&bar_m[b]);
+                set_taken(&taken.x, it + 1);
             }
             if (++sc == NC) {
                 sc = 0;
@@ -147,9 +150,10 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
                 for (int hs = 0; hs < NH; ++hs)
                     tma_store_2d(&P.mS, sQ0 + ((it & 1) * NH + hs) * PANEL, 0, (int)((((size_t)bb * P.nt + k0 + (nt - 1 - it)) * P.h + hh0 + hs) * DN));
                 tma_store_commit();
+                set_taken(&taken.y, it + 1);
                 tma_store_wait_read<1>();
                 mbar_arrive(&bar_m[it & 1]);  // the other panels may be rewritten
-                mbar_wait(&bar_m[it & 1], (it >> 1) & 1, &failed);  // the MMA of the tile is done
+                mbar_wait(&bar_m[it & 1], (it >> 1) & 1, &alive);  // the MMA of the tile is done
                 if (it + NC < nt) load_c(it + NC);
                 if (it + NU < nt) load_u(it + NU);
             }
@@ -178,7 +182,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
         for (int it = -1; it < nt; ++it) {
             // weighted copy of this thread's half row of dY of tile it + 1, in place
             if (it + 1 < nt) {
-                mbar_wait(&bar_u[s], lph, &failed);
+                mbar_wait(&bar_u[s], lph, &alive);
                 uint8_t* sU = sU0 + (size_t)(s * NH + hs) * PANEL;
                 const __nv_bfloat162 w2 = __float2bfloat162_rn(exp2f(it < 0 ? c0 : c1));
 #pragma unroll
@@ -195,8 +199,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
                 }
                 tc_fence_before();
                 fence_async_smem();
-                __syncwarp();
-                named_arrive(kRevBarU + ((it + 1) & 1), BAR);
+                hand_over(kRevBarU + ((it + 1) & 1), BAR);
                 if (++s == NU) {
                     s = 0;
                     lph ^= 1;
@@ -209,7 +212,8 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
                     c1 = tcum[row - (it + 2) * LT];
                     S1 = tcum[LT - 1 - (it + 2) * LT];
                 }
-                mbar_wait(&bar_m[it & 1], (it >> 1) & 1, &failed);
+                mbar_wait(&bar_m[it & 1], (it >> 1) & 1, &alive);
+                const int live = *(const volatile int*)&alive;
                 tc_fence_after();
                 uint32_t r[32];
                 tmem_ld32(tm + (it & 1) * 64 * NH + hs * 64 + lanes + hf * 32, r);
@@ -218,18 +222,20 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
                 const float2 d2 = make_float2(dec, dec);
 #pragma unroll
                 for (int q = 0; q < 16; ++q) H2[q] = fma2(d2, H2[q], reinterpret_cast<const float2*>(r)[q]);
-                if (it + 1 == nt) break;
+                if (it + 1 >= live) {
+                    if (it + 1 == nt) break;
+                    until_taken(1, &taken, it);  // U and Q of the tile are behind what was waited for
+                }
             }
             store_half_row(sQ + ((it + 1) & 1) * NH * PANEL, row, hf * 4, H);  // (the store of two tiles before has read it: bar_m)
             fence_async_smem();
-            __syncwarp();
-            named_arrive(kRevBarQ, BAR);
+            hand_over(kRevBarQ, BAR);
         }
         if (k0 == 0) store_state_row(P.out_state, bh, P.p, P.n, row, hf * 32, H);
     }
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && failed) atomicExch(P.status, 1);
+    end_of_waits(&alive, P.status);
     if (warp == MMAW) tmem_dealloc(tm, 128 * NH);
 }
 

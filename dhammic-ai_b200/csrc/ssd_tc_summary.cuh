@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     uint8_t* sStage = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     __shared__ uint64_t bar_ld[4], bar_m[4];
     __shared__ uint32_t tmem_slot;
-    __shared__ int failed;
+    __shared__ int alive;
+    __shared__ int4 taken;  // see until_taken: .x kSumBarU
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hh0 = blockIdx.x * NH, bb = blockIdx.y;
@@ -75,7 +76,8 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     auto tile_of = [&](int it) { return k0 + (REV ? it : nt - 1 - it); };
 
     if (tid == 0) {
-        failed = 0;
+        alive = 1;
+        taken = make_int4(NS, kTakenAll, kTakenAll, kTakenAll);
         for (int s = 0; s < NS; ++s) {
             mbar_init(&bar_ld[s], 1);
             mbar_init(&bar_m[s], 1);
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
                 for (int kk = 0; kk < 8; ++kk)  // acc[n][p of every head] += V^T Uw : both MN-major, K = position
                     mma_ss_lo(tm, v + kk * 128, v + (2 * PANEL >> 4) + kk * 128, NH == 2 ? kIdescMM128 : kIdescMM, it > 0 || kk > 0);
                 mma_commit(&bar_m[s]);
+                set_taken(&taken.x, it + 1 + NS);
             }
             if (++s == NS) s = 0;
         }
@@ -119,7 +122,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
             for (int it = 0; it < nt; ++it) {
                 uint8_t* st = sStage + (size_t)s * Cfg::STAGE_BYTES;
                 const int pos = tile_of(it) * LT;
-                mbar_wait(&bar_m[s], ph, &failed);  // the products of the stage's tile before are done
+                mbar_wait(&bar_m[s], ph, &alive);  // the products of the stage's tile before are done
                 mbar_expect_tx(&bar_ld[s], Cfg::STAGE_BYTES);
 #pragma unroll
                 for (int hs = 0; hs < NH; ++hs) tma_load_4d(st + (2 + hs) * PANEL, &P.mU, &bar_ld[s], 0, hh0 + hs, pos, bb);
@@ -157,7 +160,8 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
             }
             const float w = REV ? exp2f(run + c_i) : dtv * exp2f(run + (Sk - c_i));
             run += Sk;
-            mbar_wait(&bar_ld[s], ph, &failed);
+            mbar_wait(&bar_ld[s], ph, &alive);
+            const int late = gave_up(&alive);
             uint8_t* sU = sStage + (size_t)s * Cfg::STAGE_BYTES + (2 + hs) * PANEL;
             const __nv_bfloat162 w2 = __float2bfloat162_rn(w);
 #pragma unroll
@@ -173,8 +177,8 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
                 *p = v;
             }
             fence_async_smem();
-            __syncwarp();
-            named_arrive(kSumBarU + s, BAR);
+            until_taken(late, &taken, it);
+            hand_over(kSumBarU + s, BAR);
             if (++s == NS) {
                 s = 0;
                 ph ^= 1;
@@ -183,7 +187,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
         // `run` is now the total log2-decay of the piece
         const int last = nt - 1;
         uint32_t r[32];
-        mbar_wait(&bar_m[last % NS], (last / NS) & 1, &failed);
+        mbar_wait(&bar_m[last % NS], (last / NS) & 1, &alive);
         tc_fence_after();
         tmem_ld32(tm + lane_base(warp) + hs * 64 + hf * 32, r);
         tmem_ld_wait();
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
     }
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && failed) atomicExch(P.status, 1);
+    end_of_waits(&alive, P.status);
     if (warp == MMAW) tmem_dealloc(tm, 64 * NH);
 }
 

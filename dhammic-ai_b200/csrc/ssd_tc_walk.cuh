@@ -26,11 +26,6 @@ __device__ __forceinline__ void named_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Counts the calling warp in without waiting.
-__device__ __forceinline__ void named_arrive(int id, int nthreads) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
 // Write 32 fp32 values as bf16 into chunks [chunk0, chunk0+4) of this row of a swizzled panel.
 __device__ __forceinline__ void store_half_row(uint8_t* panel, int row, int chunk0, const float (&v)[32]) {
 #pragma unroll
@@ -103,7 +98,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     uint8_t* sH = sUd + PANEL;                             // state, bf16, [n][p]
     __shared__ uint64_t bar_ld[3], bar_u, bar_m2, bar_h, bar_sr;
     __shared__ uint32_t tmem_slot;
-    __shared__ int failed;
+    __shared__ int alive;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hh = blockIdx.x, bb = blockIdx.y;
@@ -112,7 +107,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     const int k0 = blockIdx.z * P.pt, nt = min(P.pt, P.nt - k0);  // the piece's tiles
 
     if (tid == 0) {
-        failed = 0;
+        alive = 1;
         for (int s = 0; s < NST; ++s) mbar_init(&bar_ld[s], 1);
         mbar_init(&bar_u, 8);
         mbar_init(&bar_m2, 1);
@@ -147,15 +142,15 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
             for (int it = 0; it < nt; ++it) {
                 const uint32_t ph = it & 1;
                 const uint32_t vMN = stMN + (uint32_t)(it % NST) * SU;
-                mbar_wait(&bar_ld[it % NST], (it / NST) & 1, &failed);
-                if (it > 0) mbar_wait_spin(&bar_h, (it - 1) & 1, &failed);  // accumulator read
-                mbar_wait_spin(&bar_u, ph, &failed);
+                mbar_wait(&bar_ld[it % NST], (it / NST) & 1, &alive);
+                if (it > 0) mbar_wait_spin(&bar_h, (it - 1) & 1, &alive);  // accumulator read
+                mbar_wait_spin(&bar_u, ph, &alive);
                 tc_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)  // Hl = V^T Ud : both MN-major, K = position
                     mma_ss_lo(tHl, vMN + kk * 128, udMN + kk * 128, kIdescMM, kk > 0);
                 // the rows rewrite sH after bar_m2: the store of the tile before must have read it
-                mbar_wait_spin(&bar_sr, ph, &failed);
+                mbar_wait_spin(&bar_sr, ph, &alive);
                 mma_commit(&bar_m2);
             }
         }
@@ -180,11 +175,11 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
             for (int it = 0; it < nt; ++it) {
                 if (it + NST - 1 < nt) {
                     // the stage of tile it-1 is free once the product of that tile has completed
-                    if (it > 0) mbar_wait(&bar_m2, (it - 1) & 1, &failed);
+                    if (it > 0) mbar_wait(&bar_m2, (it - 1) & 1, &alive);
                     issue_loads(it + NST - 1);
                 }
                 if (it > 0) {
-                    mbar_wait_spin(&bar_h, (it - 1) & 1, &failed);  // new state in sH
+                    mbar_wait_spin(&bar_h, (it - 1) & 1, &alive);  // new state in sH
                     tma_store_2d(&P.mS, sH, 0, state_row(it));
                     tma_store_commit();
                 }
@@ -212,7 +207,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
                 S_n = tcum[o + LT - 1];
                 dt_n = dtT ? dtT[o + row] : 1.f;
             }
-            mbar_wait(&bar_ld[s], (it / NST) & 1, &failed);
+            mbar_wait(&bar_ld[s], (it / NST) & 1, &alive);
             {
                 // (sUd is free: this thread waited for the product of the tile before, its only reader, before the state update)
                 // this thread's half row of U, weighted by d_j dt_j as a bf16 pair (one packed multiply per two elements)
@@ -232,7 +227,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
             }
             fence_async_smem();
             mbar_arrive_warp(&bar_u);
-            mbar_wait(&bar_m2, ph, &failed);
+            mbar_wait(&bar_m2, ph, &alive);
             tc_fence_after();
             {
                 uint32_t r[32];
@@ -254,7 +249,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) states_walk_kernel(const __gr
     }
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && failed) atomicExch(P.status, 1);
+    end_of_waits(&alive, P.status);
     if (warp == 8) tmem_dealloc(tHl, 64);
 }
 

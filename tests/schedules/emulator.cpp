@@ -34,14 +34,14 @@ namespace emu {
 constexpr int kPanel = 16384, kStack = 96 * 1024;
 struct Mbar { int count = 0, pending = 0; long long bytes = 0; uint32_t phase = 0; };
 struct HwBar { int expected = 0, arrived = 0; uint32_t turn = 0; uint32_t warps = 0; };
-enum Why { kReady, kMbar, kHw, kWarp, kStores, kDone };
+enum Why { kReady, kMbar, kHw, kWarp, kStores, kPoll, kDone };
 struct Fiber {
     ucontext_t ctx;
     Why why = kReady;
     const void* bar = nullptr;
     uint32_t parity = 0, turn = 0;
-    volatile int* failed = nullptr;
-    int stores = 0;
+    volatile int* alive = nullptr;
+    int stores = 0;  // groups that may still read; what the counts have to pass
     bool expired = false;
 };
 struct Agent { double at; int kind; int index; };  // kind 0: warp, 1: products of a thread, 2: copy
@@ -85,12 +85,12 @@ inline void arrive(const void* p) {
     --b.pending;
     settle(b);
 }
-inline void wait(const void* p, uint32_t parity, volatile int* failed) {
+inline void wait(const void* p, uint32_t parity, volatile int* alive) {
     Fiber& f = S.fibers[S.current];
     pause();
-    f.why = kMbar; f.bar = p; f.parity = parity; f.failed = failed; f.expired = false;
+    f.why = kMbar; f.bar = p; f.parity = parity; f.alive = alive; f.expired = false;
     leave();
-    if (f.expired) *failed = 1;
+    if (f.expired) *alive = 0;
 }
 // Every lane of the warp; `last` runs in the last of them to come.
 inline void warp_meet(const std::function<void()>& last = {}) {
@@ -127,12 +127,21 @@ inline void hw_arrive(int id, int count) {
     pause();
     warp_meet([&] { count_in(id, count); });
 }
+inline void poll(const void* counts, int more_than) {
+    Fiber& f = S.fibers[S.current];
+    f.why = kPoll; f.bar = counts; f.stores = more_than;
+    leave();
+}
 inline bool can_go(Fiber& f, int i) {
     switch (f.why) {
         case kReady: return true;
-        case kMbar: return f.expired || mbar(f.bar).phase != f.parity || *f.failed;
+        case kMbar: return f.expired || mbar(f.bar).phase != f.parity || *f.alive <= 0;
         case kHw: return ((const HwBar*)f.bar)->turn != f.turn;
         case kWarp: return S.warp_bar[i / 32].turn != f.turn;
+        case kPoll: {
+            const volatile int* t = (const volatile int*)f.bar;
+            return min(min(t[0], t[1]), min(t[2], t[3])) > f.stores;
+        }
         case kStores: {
             int open = 0;
             auto& g = S.groups[i];
@@ -290,8 +299,8 @@ inline void mbar_expect_tx(uint64_t* b, uint32_t n) {
     emu::arrive(b);
 }
 constexpr uint32_t kSpinLimit = 1;
-inline void mbar_wait(uint64_t* b, uint32_t ph, volatile int* failed, uint32_t = 0) { emu::wait(b, ph, failed); }
-inline void mbar_wait_spin(uint64_t* b, uint32_t ph, volatile int* failed, uint32_t = 0) { emu::wait(b, ph, failed); }
+inline void mbar_wait(uint64_t* b, uint32_t ph, volatile int* alive, uint32_t = 0) { emu::wait(b, ph, alive); }
+inline void mbar_wait_spin(uint64_t* b, uint32_t ph, volatile int* alive, uint32_t = 0) { emu::wait(b, ph, alive); }
 inline void fence_async_smem() { emu::pause(); }
 inline void tc_fence_before() { emu::pause(); }
 inline void tc_fence_after() {}
@@ -342,6 +351,16 @@ template <int R> inline void setmaxnreg_inc() {}
 inline void bar_sync(int id, int n) { emu::hw_sync(id, n); }
 inline void bar_arrive(int id, int n) { emu::hw_arrive(id, n); }
 inline void named_bar_sync(int id, int n) { emu::hw_sync(id, n); }
+inline bool gave_up(const volatile int* alive) {
+    const int a = *alive;
+    emu::pause();
+    return a <= 0;
+}
+inline void end_of_waits(const volatile int* alive, int* status) { if (gave_up(alive) && threadIdx.x == 0) *status = 1; }
+inline void hand_over(int id, int n) { emu::hw_arrive(id, n); }
+constexpr int kTakenAll = 0x7fffffff;
+inline void until_taken(int late, const int4* taken, int round) { if (late) emu::poll(&taken->x, round); }
+inline void set_taken(int* count, int rounds) { *(volatile int*)count = rounds; emu::pause(); }
 inline void prefetch_tmap(const CUtensorMap*) {}
 inline void tmem_alloc(uint32_t* p, uint32_t) { *p = 0; }
 inline void tmem_relinquish() {}

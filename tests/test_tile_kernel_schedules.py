@@ -1,9 +1,10 @@
 """The tile kernels' own source on the CPU (schedules/emulator.cpp), every warp, copy and group of products in random order: what the source does not order shows as
 other bits, a barrier that a warp reaches twice in one turn is counted, and a block in which a wait runs out still comes to its end."""
 import ctypes as C
-import math
+import importlib
 import re
 import subprocess
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ import torch
 from conftest import ROOT
 
 CSRC = ROOT / "dhammic-ai_b200" / "csrc"
-CUDA = "/usr/local/cuda/include"
+CUDA = Path(importlib.import_module("dhammic-ai_b200.build")._nvcc()).resolve().parent.parent / "include"
 _PTR = ("x", "B", "C", "y", "dy", "dx", "dB", "dC", "states", "dstates", "tcum", "dtT", "skipT", "D", "seed", "out_state", "ysq", "g_", "ddtx", "dyx", "gS", "status", "extreme")
 
 
@@ -105,6 +106,19 @@ def test_any_order_gives_the_same_bits(emulator, kernel, more, shape):
         assert (call.args.hung, call.args.overruns, call.args.underflows) == (0, 0, 0), schedule
         for k, v in want.items():
             assert np.array_equal(v.view(np.uint8), got[k].view(np.uint8)), (schedule, k)
+
+
+@pytest.mark.parametrize("kernel,more,shape", CASES, ids=IDS)
+def test_a_wait_that_runs_out_ends_the_block(emulator, kernel, more, shape):
+    """Waits given up at random, or because a copy never lands: the block reports it and comes to its end, and no warp is counted twice in one turn of a barrier."""
+    call, f, expiries = Call(**shape), getattr(emulator, kernel), 0
+    for schedule in range(1, 25):
+        how = dict(expire=1) if schedule % 2 else dict(lose_copy=schedule // 2 - 1)
+        got = call.run(f, *more, schedule=schedule, **how)
+        assert (call.args.hung, call.args.overruns) == (0, 0), schedule
+        assert int(got["status"][0]) == int(call.args.expiries > 0), schedule
+        expiries += call.args.expiries
+    assert expiries > 0
 
 
 def test_emulated_walk_is_the_scan(emulator):
