@@ -70,7 +70,8 @@ constexpr int kPieceSms = 148, kMaxEntries = 16, kWholeWalks = 75;  // SMs; see 
 // The forward walks of a call's last round over the SMs (of all its pairs, where there are no more pairs than SMs), where they leave at least half the SMs idle and
 // no walk is summarised (Pieces): as many CTAs a walk as there are SMs for, up to four, each of which walks the states before its own tiles for itself.  These
 // take 0.8 us a tile and the piece's own 1.5, so pieces shrink by a constant factor.  Only where that saves a tenth of the walk.
-// 44 walks of 16 tiles behind 148 whole ones 57 -> 53 us, 64 walks of 16 tiles 32.5 -> 29, 24 walks of four tiles 10.4 -> 9.6.
+// Whole -> cut, us: 44 walks behind 148 whole ones, of 4 tiles 22.8 -> 22.5, 16 tiles 58.3 -> 52.8, 64 tiles 195 -> 172, 256 tiles 742 -> 657; 72 of 16 tiles behind 148
+// 60.0 -> 56.2, 4 of 256 739 -> 605; all of a call's: 24 of 2 tiles 8.1 -> 8.0, 4 tiles 10.7 -> 10.0, 8 tiles 16.2 -> 12.8, 64 of 4 tiles 11.8 -> 11.4, 16 tiles 29.0 -> 23.4.
 constexpr double kTileUs = 1.5, kLeadUs = 0.8;
 inline SelfCut self_cut(const Dims& d) {
     const int nt = tiles_of(d.T);

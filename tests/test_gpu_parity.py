@@ -679,6 +679,29 @@ def test_walks_that_find_their_own_way(pkg, cabi, tiles, h, g, few, many):
         assert torch.equal(u[:m], v[:m]) if i < 8 else rel_err(u[:m].float(), v[:m].float()) < TOL_BF16, i
 
 
+@pytest.mark.parametrize("tiles", [2, 5, 12, 40])
+@pytest.mark.parametrize("h,g,batch", [(3, 1, 56), (24, 1, 8), (4, 2, 40)])
+def test_walks_behind_a_full_round(pkg, cabi, tiles, h, g, batch):
+    """Of 160 to 192 forward walks those behind the first 148 are cut (in up to four pieces); the last entries of the batch, on both sides of that line, have the bits
+    that they have in a call of their own, of 75 and more walks, which are whole."""
+    T, n = 128 * tiles, -(-75 // h)
+    assert batch * h > 148 and (batch - n) * h < 148
+    gen = torch.Generator(device=DEV).manual_seed(tiles)
+    def randn(*s):
+        return torch.randn(*s, generator=gen, device=DEV)
+    x, z, B, C = (randn(batch, T, *s).bfloat16() for s in ((h, 64), (h * 64,), (g, 128), (g, 128)))
+    dt, A, D, w = 0.05 * torch.rand(batch, T, h, generator=gen, device=DEV), -torch.rand(h, generator=gen, device=DEV), randn(h), randn(h * 64)
+    init = randn(batch, h, 64, 128)
+    def run(first):
+        xb, zb, Bb, Cb, dtb, ib = (t[first:].contiguous() for t in (x, z, B / 128 ** 0.5, C, dt, init))
+        leaf = xb.clone().requires_grad_(True)  # with the states kept for the backward
+        y, fs = pkg.ssd_mamba2(leaf, dtb, A, Bb, Cb, D, 128, ib)
+        return [*pkg.ssd_mamba2(xb, dtb, A, Bb, Cb, D, 128, ib), *pkg.ssd_mamba2_gated(xb, dtb, A, Bb, Cb, None, zb, w, 1e-6, 128),
+                *pkg.fused_ssd_scan(xb, dtb * A, Bb, Cb, 128)[:2], y.detach(), fs.detach(), torch.autograd.grad(y, leaf, xb)[0]]
+    for i, (u, v) in enumerate(zip(run(0), run(batch - n))):
+        assert torch.equal(u[batch - n:], v), i
+
+
 _FIRST_BACKWARD = """
 import sys
 sys.path.insert(0, {root!r})

@@ -121,6 +121,14 @@ def test_a_wait_that_runs_out_ends_the_block(emulator, kernel, more, shape):
     assert expiries > 0
 
 
+@pytest.mark.parametrize("tiles,h,whole,cut", [(4, 1, 0, (0, 2, 4)), (7, 2, 1, (0, 4, 7)), (8, 3, 1, (0, 3, 6, 8)), (9, 2, 0, (0, 3, 5, 7, 9))])
+def test_cut_walks_have_the_bits_of_whole_ones(emulator, tiles, h, whole, cut):
+    shape = dict(T=128 * tiles - 50, h=h, g=1)
+    want, got = (Call(**shape, **kw).run(emulator.forward, schedule=3) for kw in ({}, dict(whole=whole, cut=cut)))
+    for k in ("y", "states", "out_state", "ysq"):
+        assert np.array_equal(want[k].view(np.uint8), got[k].view(np.uint8)), k
+
+
 def test_emulated_walk_is_the_scan(emulator):
     """Against the recurrence in 64 bits, whose operands the kernel rounds to bf16."""
     call = Call(T=300, h=2, g=1)
