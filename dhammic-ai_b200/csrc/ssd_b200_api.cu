@@ -406,6 +406,10 @@ int simt_fwd(const ssd_b200_fwd_args* a, cudaStream_t st) {
     if (mma) {
         ssd::mma::Params M = mma_params(a, d, mma_ws(d, SSD_B200_PASS_FWD), 1);
         M.final_state = a->final_state; M.y = (__nv_bfloat16*)a->y;
+        if (ssd::overlap(a->init, a->final_state, (size_t)d.b * d.h * d.p * d.n * 4)) {
+            M.per = M.nt;
+            M.np = 1;
+        }
         if (any_unaligned({a->x, a->B, a->C, a->y})) return d.n <= 64 ? mma_fwd_launches<64, false>(M, st) : mma_fwd_launches<128, false>(M, st);
         return d.n <= 64 ? mma_fwd_launches<64, true>(M, st) : mma_fwd_launches<128, true>(M, st);
     }

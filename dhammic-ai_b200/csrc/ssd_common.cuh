@@ -75,6 +75,10 @@ __device__ __forceinline__ void dep_wait_early() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Whether two buffers of so many bytes share memory.  A state that is updated in place (init and final_state the same buffer) must be read before it is
+// written, and only a walk that one block takes from end to end sees to that.
+inline bool overlap(const void* a, const void* b, size_t bytes) { return a && b && (const char*)a < (const char*)b + bytes && (const char*)b < (const char*)a + bytes; }
+
 // Sum over a block of THREADS threads, valid in all of them; red: one float per warp.
 template <int THREADS>
 __device__ __forceinline__ float block_sum(float v, float* red) {

@@ -268,7 +268,7 @@ inline int split_walk(WalkParams& P, const Dims& d, const Ws& w, void* workspace
     P.pt = P.nt;
     *pieces = 1;
     const Pieces pc = pieces_of(d, REV);
-    if (pc.np == 1 || bytes < w.total) return 0;
+    if (pc.np == 1 || bytes < w.total || overlap(P.seed, P.out_state, (size_t)d.b * d.h * d.p * d.n * 4)) return 0;
     SummaryParams S{};
     S.mU = P.mU; S.mV = P.mV; S.tcum = P.tcum; S.dtT = P.dtT; S.out = (float*)((char*)workspace + w.piece_sum);
     S.logdecay = (float*)((char*)workspace + w.piece_decay); S.status = P.status; S.zero_status = P.zero_status; S.Tp = P.Tp; S.h = P.h; S.hpg = P.hpg; S.nt = P.nt;
@@ -360,7 +360,8 @@ inline int forward(const ssd_b200_fwd_args* a, const Dims& d, cudaStream_t st, c
     int pieces;
     if (int rc = split_walk<false>(P, d, w, ws, a->workspace_bytes, &pieces, &after, st, err, errn)) return rc;
     dim3 grid(d.h, d.b, pieces);
-    if (pieces == 1) {
+    // (x is read again by the pieces behind, so it must not be written to either)
+    if (pieces == 1 && !overlap(a->init, a->final_state, (size_t)d.b * d.h * d.p * d.n * 4) && !overlap(a->x, a->y, (size_t)d.b * d.T * d.h * d.p * 2)) {
         P.self = self_cut(d);
         if (P.self.np > 1) grid = dim3((unsigned)(P.self.whole + (d.b * d.h - P.self.whole) * P.self.np));
     }

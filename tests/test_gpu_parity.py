@@ -771,6 +771,33 @@ def test_walk_in_one_piece_where_the_workspace_has_no_room(pkg, cabi):
     assert rc2 == [cabi.EWORKSPACE, cabi.EWORKSPACE]
 
 
+@pytest.mark.parametrize("dtype,b,T,h,n,g", [("bf16", 1, 512, 24, 128, 1), ("bf16", 1, 1024, 64, 128, 8), ("bf16", 8, 512, 24, 128, 1), ("bf16", 1, 8192, 8, 128, 2),
+                                             ("bf16", 1, 4032, 4, 64, 1), ("bf16", 1, 4032, 4, 128, 1), ("fp32", 2, 256, 8, 64, 1)])
+def test_state_updated_in_place(pkg, cabi, dtype, b, T, h, n, g):
+    """init and final_state in one buffer: the results of two.  Walks that are cut where the two are apart (by themselves, summarised, those of partial tiles, behind a
+    full round) and whole ones.  On the tcgen05 kernels the bits are those of a call with room for one piece."""
+    cfg = replace(pkg.CONFIGS[2], dtype=dtype, batch=b, seqlen=T, nheads=h, ngroups=g, d_state=n, chunk=64)
+    inp = {k: v.to(DEV) for k, v in pkg.make_inputs(cfg, seed=6).items()}
+    import ctypes
+    lib, S = cabi.load(), pkg.ssd_scan
+    P, st = S._ptr, S._stream(torch.device(DEV))
+    shape = cabi.Shape(cabi.ABI_VERSION, cabi.BF16 if dtype == "bf16" else cabi.F32, cabi.F32, cabi.PATH_AUTO, b, T, h, 64, n, g, 64)
+    tc = lib.ssd_b200_resolve_path(ctypes.byref(shape)) == cabi.PATH_TC
+    room = {f: int(getattr(lib, f"ssd_b200_workspace_{f}")(ctypes.byref(shape), cabi.PASS_FWD)) for f in ("bytes", "min_bytes")}
+    ws, init = torch.empty(room["bytes"], dtype=torch.uint8, device=DEV), torch.randn(b, h, 64, n, device=DEV)
+    def run(in_place, nb):
+        state, y, cum = init.clone(), torch.empty_like(inp["x"]), torch.empty(b, h, T // 64, 64, device=DEV)
+        final = state if in_place else torch.empty_like(init)
+        a = cabi.FwdArgs(shape, P(inp["x"]), None, P(inp["dt"]), P(inp["A_head"]), P(inp["D"]), P(inp["B"]), P(inp["C"]), P(state), P(y), P(final), P(cum), 0, 0, P(ws), nb)
+        cabi.check(lib.ssd_b200_fwd(ctypes.byref(a), st))
+        torch.cuda.synchronize()
+        return y, final
+    want = run(False, room["min_bytes" if tc else "bytes"])
+    for _ in range(8):
+        for u, v in zip(run(True, room["bytes"]), want):
+            assert torch.equal(u, v) if tc else rel_err(u.float(), v.float()) < (1e-5 if u.dtype == torch.float32 else 2 ** -7)
+
+
 @pytest.mark.parametrize("h,p,n,g,l,T", [(3, 24, 12, 1, 32, 96), (4, 80, 40, 2, 48, 96), (6, 16, 72, 3, 100, 200),
                                          (2, 128, 130, 1, 64, 64), (2, 8, 8, 2, 16, 16)])
 def test_ragged_shapes_fp32(pkg, cabi, oracle, h, p, n, g, l, T):
