@@ -43,22 +43,6 @@ __device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
     __syncwarp();
     mbar_arrive_if(bar, (threadIdx.x & 31) == 0);
 }
-// The same, returning the low word of the state token of the arriving thread (0 elsewhere): arithmetic made to depend
-// on it cannot be scheduled ahead of the arrive (an arrive without consumers is otherwise sunk past any amount of
-// register-only work, and the waiter sees the phase that much later).
-__device__ __forceinline__ uint32_t mbar_arrive_if_token(uint64_t* bar, bool pred) {
-    uint32_t lo;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 st;\n\t.reg .b32 hi;\n\t"
-        "setp.ne.b32 p, %2, 0;\n\t"
-        "mov.b64 st, 0;\n\t"
-        "@p mbarrier.arrive.shared::cta.b64 st, [%1];\n\t"
-        "mov.b64 {%0, hi}, st;\n\t}"
-        : "=r"(lo)
-        : "r"(smem_u32(bar)), "r"((uint32_t)pred)
-        : "memory");
-    return lo;
-}
 // Bounded waits: they give up when the limit is reached or when another wait of this block has given up (*alive, in shared memory and above zero until
 // then, is zero), so a broken pipeline drains quickly instead of spinning.  Written out because their size counts: left to the compiler a wait is four polls
 // and 50 instructions, and the tile kernels, whose warps run some ten loops at once, no longer fit the instruction cache.
@@ -152,11 +136,6 @@ __device__ __forceinline__ void tma_store_wait_read() {  // smem source of all b
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-// Four bytes global -> shared without a register in between (generic proxy); wait_all covers the caller's own copies.
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Per-thread register budget of the calling warpgroup (4 consecutive warps, all of which must execute it): release
 // registers to the pool / take them from it.  The kernel needs a compile-time register cap (__maxnreg__).
 template <int R>
@@ -234,14 +213,10 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 // K-major operand (the 64 contiguous elements run along K): stride offset = 1024 (eight rows); the
 // leading offset is unused.  MN-major operand (the 64 contiguous elements run along M or N, rows are
 // K): stride offset = 1024 (eight K rows), leading offset = distance between 64-wide MN panels.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
+// The high word is the same for every operand of these kernels; an issuing thread derives the low word of each K step with one integer add.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+    return ((saddr >> 4) & 0x3FFFu) | ((lbo_bytes >> 4) << 16);
 }
 // Instruction descriptor, kind::f16, bf16 x bf16 -> fp32, dense.
 //   [4,6) D format (1 = f32)  [7,10) A format (1 = bf16)  [10,13) B format (1 = bf16)
@@ -251,33 +226,7 @@ __host__ __device__ constexpr uint32_t instr_desc(int M, int N, bool a_mn_major,
            ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       bool accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]; A holds bf16 pairs packed in 32-bit TMEM columns.
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                       bool accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-        : "memory");
-}
-// The same products from the low words of the operand descriptors (address and leading offset); the high word
-// (stride offset 1024, version, SWIZZLE_128B) is the same for every operand of these kernels.  An issuing thread
-// derives the descriptor of each K step with one integer add.
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
-    return ((saddr >> 4) & 0x3FFFu) | ((lbo_bytes >> 4) << 16);
-}
+// D[tmem] (+)= A[smem] * B[smem], operands by the low words of their descriptors; issued by ONE thread.
 template <bool ACC>
 __device__ __forceinline__ void mma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
     asm volatile(
@@ -299,6 +248,7 @@ __device__ __forceinline__ void mma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32
         ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"((uint32_t)accumulate), "r"(kDescHi)
         : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem]; A holds bf16 pairs packed in 32-bit TMEM columns.
 __device__ __forceinline__ void mma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, bool accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
@@ -337,24 +287,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t& r0, uint32_t& r1) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st1(uint32_t taddr, uint32_t r0) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%1], {%0};" ::"r"(r0), "r"(taddr) : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-        "%29,%30,%31};"
-        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-          "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-          "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
-        : "memory");
-}
 // x16: 16 consecutive 32-bit columns.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(

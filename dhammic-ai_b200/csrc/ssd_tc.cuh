@@ -249,44 +249,13 @@ struct WalkParams {
     SelfCut self;  // forward walk, np > 1: one-dimensional grid
 };
 
-constexpr uint32_t kIdescS = instr_desc(128, 128, false, false);    // K-major x K-major, N = 128
 constexpr uint32_t kIdescKM = instr_desc(128, 64, false, true);     // A K-major, B MN-major, N = 64
 constexpr uint32_t kIdescMM = instr_desc(128, 64, true, true);      // both MN-major, N = 64
-constexpr uint32_t kIdescKK128 = instr_desc(128, 128, false, false);
+constexpr uint32_t kIdescKK128 = instr_desc(128, 128, false, false); // K-major x K-major, N = 128
 constexpr uint32_t kIdescKM128 = instr_desc(128, 128, false, true);  // A K-major, B MN-major, N = 128
 constexpr uint32_t kIdescMM128 = instr_desc(128, 128, true, true);   // both MN-major, N = 128
-constexpr uint32_t kIdescKK64 = instr_desc(128, 64, false, false);
 
 __device__ __forceinline__ uint32_t lane_base(int warp) { return ((uint32_t)((warp & 3) * 32)) << 16; }
-
-// Scale one 128-byte row of bf16 (8 chunks of 16 bytes) by w while copying src -> dst (both swizzled).
-__device__ __forceinline__ void scale_row(const uint8_t* src, uint8_t* dst, int row, float w) {
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-        uint4 v = *reinterpret_cast<const uint4*>(src + sw128(row, ch));
-        uint32_t* u = reinterpret_cast<uint32_t*>(&v);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            __nv_bfloat162 bv = *reinterpret_cast<__nv_bfloat162*>(&u[q]);
-            float2 f = __bfloat1622float2(bv);
-            u[q] = pack_bf16(f.x * w, f.y * w);
-        }
-        *reinterpret_cast<uint4*>(dst + sw128(row, ch)) = v;
-    }
-}
-
-// Write 32 fp32 values (columns c0 .. c0+31 of this thread's row) as bf16 into a swizzled panel.
-__device__ __forceinline__ void store_row32(uint8_t* panel, int row, int col0_in_panel, const float (&v)[32]) {
-#pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-        uint4 o;
-        o.x = pack_bf16(v[ch * 8 + 0], v[ch * 8 + 1]);
-        o.y = pack_bf16(v[ch * 8 + 2], v[ch * 8 + 3]);
-        o.z = pack_bf16(v[ch * 8 + 4], v[ch * 8 + 5]);
-        o.w = pack_bf16(v[ch * 8 + 6], v[ch * 8 + 7]);
-        *reinterpret_cast<uint4*>(panel + sw128(row, col0_in_panel / 8 + ch)) = o;
-    }
-}
 
 }  // namespace tc
 }  // namespace ssd

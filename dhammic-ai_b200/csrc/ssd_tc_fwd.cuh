@@ -173,7 +173,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
 #pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 __syncwarp();
-                named_barrier(kBarG + (it & 1), 544);
+                named_bar_sync(kBarG + (it & 1), 544);
                 if (lane == 0) {
                     tc_fence_after();
                     const uint32_t uMN = fresh(xMN + (uint32_t)r * PU);
@@ -226,21 +226,21 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                     }
                 }
                 __syncwarp();
-                named_barrier(kBarLead, 576);
+                named_bar_sync(kBarLead, 576);
             }
             if (lane == 0)
                 for (int it = 0; it < kFwdRing && it < nt; ++it) load_x(it);
 #pragma unroll 1
             for (int it = 0; it < nt; ++it) {
                 __syncwarp();
-                named_barrier(kBarU, 608);  // the entering state is in sH
+                named_bar_sync(kBarU, 608);  // the entering state is in sH
                 if (lane == 0 && P.save_states) {
                     tma_store_2d(&P.mS, sH, 0, (int)((((size_t)bb * P.nt + k0 + it) * P.h + hh) * DN));
                     tma_store_commit();
                 }
                 if (it > 0) {
                     __syncwarp();
-                    named_barrier(kBarH + ((it - 1) & 1), 544);  // y of the tile before staged
+                    named_bar_sync(kBarH + ((it - 1) & 1), 544);  // y of the tile before staged
                     if (lane == 0) store_y(it - 1);
                 }
                 if (lane == 0) {
@@ -256,7 +256,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 }
             }
             __syncwarp();
-            named_barrier(kBarH + ((nt - 1) & 1), 544);
+            named_bar_sync(kBarH + ((nt - 1) & 1), 544);
             if (lane == 0) {
                 store_y(nt - 1);
                 tma_store_wait_all();
@@ -270,15 +270,15 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
                 tc_fence_after();
                 const uint32_t vK = fresh(stK + (uint32_t)(it & 1) * SU), cK = vK + 2 * PU, tS = tm + (it & 1) * 128;
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) mma_ss_lo(tS, cK + offK(kk), vK + offK(kk), kIdescS, kk > 0);
+                for (int kk = 0; kk < 8; ++kk) mma_ss_lo(tS, cK + offK(kk), vK + offK(kk), kIdescKK128, kk > 0);
                 mma_commit(it > 0 ? &bar_m2[(it - 1) & 1] : bar_s0);
             };
-            if (!hl && lead > 0) named_barrier(kBarLead, 576);
+            if (!hl && lead > 0) named_bar_sync(kBarLead, 576);
             if (hl) {
 #pragma unroll 1
                 for (int it = 0; it < lead; ++it) {
                     __syncwarp();
-                    named_barrier(kBarLeadU + (it & 1), 544);
+                    named_bar_sync(kBarLeadU + (it & 1), 544);
                     if (lane == 0) {
                         tc_fence_after();
                         const uint32_t st = fresh(stMN + (uint32_t)(it % kLeadStages) * 3 * PU);
@@ -301,7 +301,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
             for (int it = 0; it < nt; ++it) {
                 if (!hl && lane == 0) mbar_wait(&bar_vc[it & 1], (it >> 1) & 1, &alive);
                 __syncwarp();
-                named_barrier(kBarU, 608);  // weighted rows and entering state written, Hl and Yo of the tile before read
+                named_bar_sync(kBarU, 608);  // weighted rows and entering state written, Hl and Yo of the tile before read
                 if (lane == 0) {
                     tc_fence_after();
                     if (hl) {
@@ -564,7 +564,7 @@ __global__ void __maxnreg__(kFwdRegsLaunch) fwd_walk_kernel(const __grid_constan
         }
         const int rnt = rows_nt;
         if (P.ysq) {
-            named_barrier(kBarRows, 512);
+            named_bar_sync(kBarRows, 512);
             if (!(q & 1))
                 P.ysq[((((size_t)bb * P.nt + k0 + (rnt - 1)) * P.h + hh) * 2 + (q >> 1)) * LT + row] =
                     ysq_own + sysq[(((rnt - 1) & 1) * 2 + (q >> 1)) * LT + row];

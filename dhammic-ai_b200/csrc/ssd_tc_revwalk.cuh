@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
             const int b = it & 1;
             if (lane == 0) mbar_wait(&bar_c[sc], cph, &alive);
             __syncwarp();
-            named_barrier(kRevBarU + b, BAR);
+            named_bar_sync(kRevBarU + b, BAR);
             if (lane == 0) {
                 tc_fence_after();
                 uint32_t v = cMN + (uint32_t)sc * (2 * PANEL >> 4), u = uMN + (uint32_t)su * (NH * PANEL >> 4);
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(RevCfg<NH>::THREADS, 1) rev_walk_kernel(const 
 #pragma unroll 1
         for (int it = 0; it < nt; ++it) {
             __syncwarp();
-            named_barrier(kRevBarQ, BAR);  // the state gradient leaving tile nt-1-it is staged
+            named_bar_sync(kRevBarQ, BAR);  // the state gradient leaving tile nt-1-it is staged
             if (lane == 0) {
 #pragma unroll
                 for (int hs = 0; hs < NH; ++hs)

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(SumCfg<NH>::THREADS, 1) summary_kernel(const _
 #pragma unroll 1
         for (int it = 0; it < nt; ++it) {
             __syncwarp();
-            named_barrier(kSumBarU + s, BAR);
+            named_bar_sync(kSumBarU + s, BAR);
             if (lane == 0) {
                 tc_fence_after();
                 uint32_t v = stMN + (uint32_t)s * (Cfg::STAGE_BYTES >> 4);

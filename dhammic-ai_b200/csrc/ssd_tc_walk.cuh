@@ -22,10 +22,6 @@
 namespace ssd {
 namespace tc {
 
-__device__ __forceinline__ void named_barrier(int id, int nthreads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
 // Write 32 fp32 values as bf16 into chunks [chunk0, chunk0+4) of this row of a swizzled panel.
 __device__ __forceinline__ void store_half_row(uint8_t* panel, int row, int chunk0, const float (&v)[32]) {
 #pragma unroll

@@ -292,7 +292,6 @@ inline uint32_t smem_u32(const void* p) { return (uint32_t)((const uint8_t*)p - 
 inline void mbar_init(uint64_t* b, uint32_t n) { auto& m = emu::mbar(b); m = emu::Mbar{}; m.count = m.pending = (int)n; }
 inline void mbar_fence_init() {}
 inline void mbar_arrive(uint64_t* b) { emu::pause(); emu::arrive(b); }
-inline void mbar_arrive_if(uint64_t* b, bool p) { if (p) emu::arrive(b); }
 inline void mbar_arrive_warp(uint64_t* b) { emu::pause(); emu::warp_meet([&] { emu::arrive(b); }); }
 inline void mbar_expect_tx(uint64_t* b, uint32_t n) {
     emu::mbar(b).bytes += n;
@@ -348,8 +347,6 @@ template <int N = 0> inline void tma_store_wait_read() {
 inline void tma_store_wait_all() { tma_store_wait_read<0>(); }
 template <int R> inline void setmaxnreg_dec() {}
 template <int R> inline void setmaxnreg_inc() {}
-inline void bar_sync(int id, int n) { emu::hw_sync(id, n); }
-inline void bar_arrive(int id, int n) { emu::hw_arrive(id, n); }
 inline void named_bar_sync(int id, int n) { emu::hw_sync(id, n); }
 inline bool gave_up(const volatile int* alive) {
     const int a = *alive;
@@ -407,7 +404,6 @@ template <int N> inline void tmem_put(uint32_t a, const uint32_t (&r)[N]) {
 }
 inline void tmem_ld32(uint32_t a, uint32_t (&r)[32]) { tmem_get(a, r); }
 inline void tmem_ld16(uint32_t a, uint32_t (&r)[16]) { tmem_get(a, r); }
-inline void tmem_st32(uint32_t a, const uint32_t (&r)[32]) { tmem_put(a, r); }
 inline void tmem_st16(uint32_t a, const uint32_t (&r)[16]) { tmem_put(a, r); }
 inline void tmem_st8(uint32_t a, const uint32_t (&r)[8]) { tmem_put(a, r); }
 inline void tmem_ld_wait() {}

@@ -2,7 +2,6 @@
 other bits, a barrier that a warp reaches twice in one turn is counted, and a block in which a wait runs out still comes to its end."""
 import ctypes as C
 import importlib
-import re
 import subprocess
 from pathlib import Path
 
@@ -26,9 +25,7 @@ class Args(C.Structure):
 def emulator(tmp_path_factory):
     out = tmp_path_factory.mktemp("schedules")
     for f in CSRC.glob("ssd_tc*.cuh"):
-        text = f.read_text().replace("extern __shared__", "extern")
-        text = re.sub(r'asm volatile\("bar\.(sync|arrive) %0, %1;" ::"r"\((\w+)\), "r"\((\w+)\) : "memory"\);', r"bar_\1(\2, \3);", text)
-        (out / f.name).write_text(text)
+        (out / f.name).write_text(f.read_text().replace("extern __shared__", "extern"))
     for name in ("ssd_common.cuh", "ssd_cumsum.cuh", "ssd_ptx.cuh"):  # the emulator's own
         (out / name).write_text("#pragma once\n")
     lib = out / "emulator.so"
