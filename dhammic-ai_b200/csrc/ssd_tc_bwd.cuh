@@ -34,7 +34,7 @@
 // warps (a waiting lane drains its queue; with one lane 1,050 us at (16, 4096, 64 heads, 8 groups), 907 with three) and dC / dB behind the products that the row
 // epilogue waits for (838 -> 825); hardware barriers for what the row warps hand over (see the forward walk); no loop unrolled that is not meant to
 // be, nor a division in one: the text shrank from 90 to 54 KB, instruction cache misses to a fifth (880 -> 815); less work in the row warps between mask and
-// epilogue gives nothing more.  All together 1,050 -> 817 us, (8, 2048, 24 heads, one group) 116 -> 97, one head per group (16, 4096, 64) 1,690 -> 1,387.
+// epilogue gives nothing more.  All together 1,050 -> 807 us, (8, 2048, 24 heads, one group) 116 -> 89, one head per group (16, 4096, 64) 1,690 -> 1,397.
 #pragma once
 #include <type_traits>
 
@@ -296,7 +296,7 @@ __global__ void __maxnreg__(kBwdRegsLaunch) bwd_tile_kernel(const __grid_constan
                 // the panels) and every row has taken its dy values (they do before they arrive at kBwdBarE)
                 if (lane == 0 && hl + 1 == hpg && more) {
                     // The next item's panels have room only when this item's products are complete: into the L2 meanwhile.  One head per group:
-                    // 1,459 -> 1,387 us at (16, 4096, 64 heads), 383 -> 366 at a batch of four; eight heads 825 -> 817.
+                    // 72 us of 1,459 at (16, 4096, 64 heads), 17 of 383 at a batch of four; with eight heads 8 of 825.
                     const int srow = ((at.bb * P.nt + at.k) * P.h + at.gg * hpg) * DN;
                     tma_prefetch_4d(&P.mC, 0, at.gg, at.k * LT, at.bb);
                     tma_prefetch_4d(&P.mC, 64, at.gg, at.k * LT, at.bb);

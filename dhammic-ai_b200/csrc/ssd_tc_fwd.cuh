@@ -22,7 +22,7 @@
 //     hand over by bar.arrive.
 //   * All loops that run at once (16 row warps, four control warps) have to fit the instruction cache: with the waits
 //     unrolled by the compiler the pipeline above was slower than one without any of this, 315 us against 286 for 148 walks of 128 tiles.
-// (16, 4096, 64 heads, 8 groups): 520 -> 427 us, 512 -> 389 without kept states; (8, 2048, 24) 85 -> 64; one walk of 128 tiles to every other SM
+// (16, 4096, 64 heads, 8 groups): 520 -> 424 us, 512 -> 384 without kept states; (8, 2048, 24) 85 -> 58, and 53 with the last walks cut; one walk of 128 tiles to every other SM
 // 280 -> 184.  Tried and slower: the state on eight warps and mask and output on the other eight (500 us: the masks of the rows 96-127 take two
 // warps 1,500 cycles and four 1,000); Yd in two halves as the masks complete (its lane drains in between).
 //

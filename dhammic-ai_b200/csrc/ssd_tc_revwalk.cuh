@@ -13,8 +13,8 @@
 // With NH = 2 the two heads share the C panels of a stage and one N = 128 product per tile
 // (C^T [e dY_a | e dY_b]); their register chains are independent and run side by side on different warps.
 // What bounds it: the row warps' steps of a tile where SMs are few (1.1 us, 1.28 for two heads), memory where all are busy: (16, 4096, 64 heads, 8 groups)
-// 229 us, 4.8 TB/s (246 with copies and products on one lane, a block barrier on either side of every staged tile and log-decays asked for where they are
-// used), one head per group 350 us, 6.1 TB/s (366).
+// 215 us, 5.0 TB/s (246 with copies and products on one lane, a block barrier on either side of every staged tile and log-decays asked for where they are
+// used), one head per group 335 us, 6.4 TB/s (366).
 //
 // Threads: head hs = tid / 256 owns warps 8 hs .. 8 hs + 7 (thread = row, column half); one lane of the next warp issues the products, one of the
 // last all copies.  The row warps hand over by hardware barriers and wait for mbarriers only (see the forward walk); a tile's log-decays are

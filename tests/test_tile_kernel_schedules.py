@@ -12,7 +12,6 @@ import torch
 from conftest import ROOT
 
 CSRC = ROOT / "dhammic-ai_b200" / "csrc"
-CUDA = Path(importlib.import_module("dhammic-ai_b200.build")._nvcc()).resolve().parent.parent / "include"
 _PTR = ("x", "B", "C", "y", "dy", "dx", "dB", "dC", "states", "dstates", "tcum", "dtT", "skipT", "D", "seed", "out_state", "ysq", "g_", "ddtx", "dyx", "gS", "status", "extreme")
 
 
@@ -28,8 +27,9 @@ def emulator(tmp_path_factory):
         (out / f.name).write_text(f.read_text().replace("extern __shared__", "extern"))
     for name in ("ssd_common.cuh", "ssd_cumsum.cuh", "ssd_ptx.cuh"):  # the emulator's own
         (out / name).write_text("#pragma once\n")
+    cuda = Path(importlib.import_module("dhammic-ai_b200.build")._nvcc()).resolve().parent.parent / "include"
     lib = out / "emulator.so"
-    subprocess.run(["g++", "-O2", "-fno-strict-aliasing", "-std=c++17", "-fPIC", "-shared", "-w", f"-I{CUDA}", f"-I{out}", str(ROOT / "tests" / "schedules" / "emulator.cpp"), "-o", str(lib)], check=True)
+    subprocess.run(["g++", "-O2", "-fno-strict-aliasing", "-std=c++17", "-fPIC", "-shared", "-w", f"-I{cuda}", f"-I{out}", str(ROOT / "tests" / "schedules" / "emulator.cpp"), "-o", str(lib)], check=True)
     return C.CDLL(str(lib))
 
 
