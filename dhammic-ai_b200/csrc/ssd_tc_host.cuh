@@ -98,8 +98,8 @@ inline SelfCut self_cut(const Dims& d) {
     return best;
 }
 
-// The pieces that a walk over one sequence is cut into.  A walk has one CTA per (batch, head), which takes 1.5 us per tile forward
-// and 1.1 us in reverse (1.3 for two heads of a group in one CTA); with few of them most SMs idle.  Pieces run side by side: every piece but the
+// The pieces that a walk over one sequence is cut into.  A walk has one CTA per (batch, head), which is reckoned with 1.5 us per tile forward
+// and 1.1 us in reverse (1.3 for two heads of a group in one CTA; 1.4, 0.97 and 1.22 with 80 CTAs); with few of them most SMs idle.  Pieces run side by side: every piece but the
 // walk's last is first summarised (0.7 us per tile, 1.05 for two heads of a group, no chain, in parts that fill the chip), and a piece's CTA
 // folds the summaries before its own into its seed.  Only while all CTAs fit on the chip at once, and where the tiles taken off the chain
 // outweigh the summary and its launch (10 us) by a tenth.  A function of the shape alone: the workspace's size follows from it.

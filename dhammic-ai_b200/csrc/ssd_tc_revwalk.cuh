@@ -12,7 +12,7 @@
 // k+1 while the MMA of tile k runs.  The weighted rows e_i * dY[i,:] are written in place over the loaded dY panel.
 // With NH = 2 the two heads share the C panels of a stage and one N = 128 product per tile
 // (C^T [e dY_a | e dY_b]); their register chains are independent and run side by side on different warps.
-// What bounds it: the row warps' steps of a tile where SMs are few (1.1 us, 1.28 for two heads), memory where all are busy: (16, 4096, 64 heads, 8 groups)
+// What bounds it: the row warps' steps of a tile where SMs are few (0.7 us with two blocks on the chip, 0.97 with 80, 1.22 for two heads), memory where all are busy: (16, 4096, 64 heads, 8 groups)
 // 215 us, 5.0 TB/s (246 with copies and products on one lane, a block barrier on either side of every staged tile and log-decays asked for where they are
 // used), one head per group 335 us, 6.4 TB/s (366).
 //
