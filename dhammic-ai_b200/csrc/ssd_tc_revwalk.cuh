@@ -36,7 +36,7 @@ constexpr int kRevBarQ = 1, kRevBarU = 2 /* and 3 */;
 template <int NH>
 struct RevCfg {
     // dY is weighted a tile before its product, C wanted for the product only.  The state gradients are staged in two panels a head: with one
-    // its store was part of every tile's chain (1.4 us a tile of two heads, 1.28 now).
+    // its store was part of every tile's chain (1.4 us a tile of two heads, 1.28 with two).
     static constexpr int C_STAGES = NH == 1 ? 3 : 2, U_STAGES = NH == 1 ? 4 : 3;
     static constexpr size_t SMEM = (size_t)(2 * C_STAGES + NH * U_STAGES + 2 * NH) * PANEL + 128;  // C (2 panels) | dY | sQ | barriers
     static constexpr int THREADS = 256 * NH + 64;
